@@ -11,6 +11,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
@@ -51,14 +52,17 @@ def build(force: bool = False, verbose: bool = False) -> str:
     nvcc = find_nvcc()
     os.makedirs(LIB_DIR, exist_ok=True)
     objs = []
+    cmds = []
     for src in sources():
         obj = os.path.join(LIB_DIR, os.path.basename(src)[:-3] + ".o")
         cmd = [nvcc, *NVCC_FLAGS, "-c", src, "-o", obj]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
             print(" ".join(cmd), flush=True)
-        subprocess.run(cmd, check=True)
+        cmds.append(cmd)
         objs.append(obj)
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:     # one nvcc per source
+        list(pool.map(lambda cmd: subprocess.run(cmd, check=True), cmds))
     tmp = LIB_PATH + ".tmp"
     # the link step names the same architecture, so nvcc does not fall back to (and warn about) its default one
     subprocess.run([nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", tmp, *objs], check=True)

@@ -14,9 +14,17 @@ from ._build import LIB_PATH
 
 _P, _I, _LL, _F = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
 
+class LayerParams(ctypes.Structure):
+    """``fm_layer_params`` of the header."""
+    _fields_ = [("ln1_weight", _P), ("ln1_bias", _P), ("w_qkv", _P), ("w_o", _P), ("attn_scale", _P), ("ln2_weight", _P),
+                ("ln2_bias", _P), ("w_fc1", _P), ("w_fc2", _P), ("mlp_scale", _P), ("ln1_eps", _F), ("ln2_eps", _F),
+                ("scale", _F), ("window", _I), ("stream_dtype", _I), ("value_dtype", _I), ("ffn", _I)]
+
+
 #: name -> argtypes, in header order.  tests/test_host_logic.py checks this table against the header.
 SIGNATURES: dict[str, list] = {
     "fm_abi_version": [],
+    "fm_layer_forward": [ctypes.POINTER(LayerParams), _P, _P, _P, _LL, _P, _P, _LL, _I, _I, _P, _P, _I, _I, _P, _P],
     "fm_qkv_rope_bf16": [_P, _P, _P, _P, _LL, _P, _P, _P, _I, _I, _I, _P, _P],
     "fm_out_proj_f16": [_P, _P, _P, _P, _P, _LL, _I, _P, _P],
     "fm_linear_f16": [_P, _P, _P, _P, _P, _LL, _I, _I, _I, _I, _I, _P, _P],
@@ -80,5 +88,6 @@ def check(rc: int, what: str) -> None:
         kind = {-1: "rejected geometry", -2: "grid too large", -3: "misaligned pointer",
                 -4: "cuTensorMapEncodeTiled unavailable",
                 -5: "more frames than the built-in workspace holds",
+                -7: "workspace too small",
                 -6: "clip length outside the fused kernel's range (128 < T <= 256)"}.get(rc, "CUDA error" if rc > 0 else "error")
         raise RuntimeError(f"{what} failed with status {rc} ({kind})")

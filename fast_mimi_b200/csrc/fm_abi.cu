@@ -36,10 +36,31 @@ int encode_tiled(CUtensorMap* map, CUtensorMapDataType dtype, uint32_t rank, voi
   return static_cast<int>(r);
 }
 
+int encode_rows_16bit(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols) {
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {cols * 2};
+  const cuuint32_t box[2] = {box_cols, box_rows};
+  const cuuint32_t estr[2] = {1, 1};
+  return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                      CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+int sm_count() {
+  constexpr int kMaxDev = 64;
+  static int known[kMaxDev];           // written with the same value by whoever asks first
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+  if (dev < kMaxDev && known[dev] > 0) return known[dev];
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (sms <= 0) sms = 1;
+  if (dev < kMaxDev) known[dev] = sms;
+  return sms;
+}
+
 int ensure_dynamic_smem(const void* kernel, int bytes) {
   // cudaFuncSetAttribute is per device; remember the largest size granted to each (kernel, device) pair
   // and ask again only for more.
-  constexpr int kMaxDev = 64, kMaxKern = 32;
+  constexpr int kMaxDev = 64, kMaxKern = 128;
   static std::mutex mu;
   static const void* kerns[kMaxKern];
   static int granted[kMaxKern][kMaxDev];

@@ -439,10 +439,45 @@ __device__ __forceinline__ void st_global_v8(void* p, const uint32_t* w) {
                : "memory");
 }
 
+// Programmatic dependent launch.  A kernel of a chain waits here for the kernel in front of it (completed, its writes
+// visible); without the launch attribute both are no-ops.  What comes BEFORE the wait may only read what no kernel of
+// the chain writes (weights).
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The status word of the chain was already non-zero when this kernel began: it does nothing, but still waits for the
+// kernel in front, so that its own end means that everything before it has ended too.
+__device__ __forceinline__ bool chain_stopped(const int* status) {
+  if (status == nullptr || *reinterpret_cast<const volatile int*>(status) == 0) return false;
+  griddep_wait();
+  return true;
+}
+// Lets the next kernel of the chain start its own prologue once every block of this grid has said so (or exited).
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// Exact-form GELU  0.5 x (1 + erf(x / sqrt 2))  with erf from the rational approximation
+//   erf(z) = 1 - (1 + a1 z + ... + a6 z^6)^-16,  z >= 0,  |error| <= 3e-7   (Abramowitz & Stegun 7.1.28)
+// instead of erff(): 15 issue slots and one reciprocal per value, no branch.  The epilogue is arithmetic-bound
+// with erff() (about 40 slots per value); the approximation error is far below the rounding of the result
+// to 16 bit.  Large |z| overflows the power to +inf, whose reciprocal is 0, i.e. erf = 1.
+__device__ __forceinline__ float gelu_erf(float x) {
+  const float z = fabsf(x) * 0.70710678118654752f;
+  float t = fmaf(z, 0.0000430638f, 0.0002765672f);
+  t = fmaf(z, t, 0.0001520143f);
+  t = fmaf(z, t, 0.0092705272f);
+  t = fmaf(z, t, 0.0422820123f);
+  t = fmaf(z, t, 0.0705230784f);
+  t = fmaf(z, t, 1.0f);
+  t *= t; t *= t; t *= t; t *= t;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(t));
+  const float e = copysignf(1.0f - r, x);
+  const float hx = 0.5f * x;
+  return fmaf(hx, e, hx);
 }
 
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {

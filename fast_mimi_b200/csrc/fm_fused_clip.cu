@@ -33,6 +33,7 @@
 #include "fm_attn_tile.cuh"
 #include "fm_common.cuh"
 #include "fm_kernels.h"
+#include "fm_launch.h"
 
 namespace fm {
 
@@ -193,6 +194,8 @@ attn_fused_clip_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();            // both CTAs' barriers exist before anything signals across the pair
+  griddep_launch();
+  if (warp != kIssueWarp0) griddep_wait();   // x may come from the kernel in front; the W loads need not wait for it
   tc_fence_after_sync();
   const uint32_t tmem_base = sh->tmem_base;
   CtaCtl* ctl = &sh->ctl;
@@ -514,9 +517,11 @@ attn_fused_clip_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
   }
 }
 
+bool use_fused_clip(int B) { return B > 0; }
+
 int launch_attn_fused_clip(const void* x, const void* w_qkv, const float* cos, const float* sin, long long cos_bstride,
                            void* out, int B, int T, int window, float scale, int dtype_flags, int* status,
-                           cudaStream_t st) {
+                           cudaStream_t st, int dependent) {
   using namespace fused;
   if (T <= kTile || T > 2 * kTile || B <= 0 || window <= 0 || cos == nullptr || sin == nullptr) return -1;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w_qkv) | reinterpret_cast<uintptr_t>(out) |
@@ -542,10 +547,7 @@ int launch_attn_fused_clip(const void* x, const void* w_qkv, const float* cos, c
                                 CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != 0) return rc;
   }
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int max_pairs = sms / 2 > 0 ? sms / 2 : 1;
+  const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
   const int n_pairs = B < max_pairs ? B : max_pairs;
   // dtype_flags bit 0: v, P and the output are FP16 (else BF16); bit 1: x and w_qkv hold FP16 (else BF16).
   const int in_fmt = (dtype_flags & 2) ? 0 : 1;
@@ -553,9 +555,8 @@ int launch_attn_fused_clip(const void* x, const void* w_qkv, const float* cos, c
   auto kern = (dtype_flags & 1) ? attn_fused_clip_kernel<__half> : attn_fused_clip_kernel<__nv_bfloat16>;
   const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
   if (rc != 0) return rc;
-  kern<<<2 * n_pairs, kThreads, kSmemBytes, st>>>(tmap_x, tmap_w, cos, sin, cos_bstride, static_cast<uint16_t*>(out), B, T,
-                                                 window, scale * 1.4426950408889634f, idesc_proj, status);
-  return static_cast<int>(cudaGetLastError());
+  return launch_kernel(kern, dim3(2 * n_pairs), kThreads, kSmemBytes, st, 1, dependent, tmap_x, tmap_w, cos, sin, cos_bstride,
+                       static_cast<uint16_t*>(out), B, T, window, scale * 1.4426950408889634f, idesc_proj, status);
 }
 
 }  // namespace fm

@@ -1,4 +1,8 @@
 // Internal launcher declarations shared by the .cu files of the library.
+//
+// `dependent`: the launch may start before the kernel in front of it has finished (programmatic dependent launch).  Only
+// for kernels launched behind one another by one entry point: the first kernel of such a chain reads nothing before its
+// wait, so what the later ones read early (weights, rows already in a ring) was complete before the chain began.
 #pragma once
 
 #include <cuda.h>
@@ -35,6 +39,10 @@ struct QkvEpilogueArgs {
 int encode_tiled(CUtensorMap* map, CUtensorMapDataType dtype, uint32_t rank, void* base, const cuuint64_t* dims,
                  const cuuint64_t* strides, const cuuint32_t* box, const cuuint32_t* elem_strides,
                  CUtensorMapSwizzle swizzle);
+// [rows, cols] row-major 16-bit matrix, boxes of box_rows x box_cols, 128-byte swizzle.
+int encode_rows_16bit(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols);
+// Multiprocessors of the current device.
+int sm_count();
 // Opt a kernel into `bytes` of dynamic shared memory once per (kernel, device).
 int ensure_dynamic_smem(const void* kernel, int bytes);
 
@@ -45,7 +53,7 @@ int launch_band_attn_fp32(const float* q, const float* k, const float* v, float*
                           int Tq, int Tk, int q_off, int k_off, int window, float scale,
                           const long long* strides, cudaStream_t st);
 int launch_qkv_rope_gemm(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep, int M, int dtype_flags,
-                         int* status, cudaStream_t st);
+                         int* status, cudaStream_t st, int dependent = 0);
 // y[M,512] = resid + out_scale * (a[M,512] * w[512,512]^T): the attention output projection with the layer
 // scale and the residual add of the reference's transformer layer folded into the epilogue.
 int launch_out_proj_gemm(const void* a, const void* w, void* y, const float* out_scale, const void* resid, int M,
@@ -53,10 +61,16 @@ int launch_out_proj_gemm(const void* a, const void* w, void* y, const float* out
 // y[M,N] = resid + scale * act(a[M,K] * w[N,K]^T); in_dtype 0 BF16 / 1 FP16; out_dtype 0 BF16 / 1 FP16 / 2 FP32
 // (type of y and resid); gelu 1 = exact GELU.  N a multiple of 256, K a multiple of 64.
 int launch_linear_gemm(const void* a, const void* w, void* y, const float* scale, const void* resid, int M, int N,
-                       int K, int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st);
+                       int K, int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent = 0);
+// The same two products for few rows (fm_linear_small.cu): 128 x 64 tiles, K split over a cluster.
+bool few_row_tiles(int M, int N);
+int launch_linear_small(const void* a, const void* w, void* y, const float* scale, const void* resid, int M, int N, int K,
+                        int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent);
+int launch_qkv_small(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status,
+                     cudaStream_t st, int dependent);
 // LayerNorm over 512 channels; x_dtype 0 BF16 / 1 FP16 / 2 FP32, y_dtype 0 BF16 / 1 FP16.
 int launch_layernorm512(const void* x, int x_dtype, const float* weight, const float* bias, float eps, void* y,
-                        int y_dtype, long long rows, cudaStream_t st);
+                        int y_dtype, long long rows, cudaStream_t st, int dependent = 0);
 // Residual vector quantisation (fm_rvq.cu): candidate selection + exact FP32 decision for one layer, FP16 copy of
 // the residual, ordered FP32 decode.
 int launch_rvq_select(const void* scores, int scores_fp16, const float* e_sq, const float* codebook, float* resid, void* resid16,
@@ -81,24 +95,31 @@ int launch_rvq_to_half(const float* x, void* y, long long rows, cudaStream_t st)
 int launch_rvq_decode(const long long* codes, const float* codebooks, float* out, long long rows, int n_layers,
                       int n_codes, int* bad_code, cudaStream_t st);
 int launch_band_attn_prefill(const void* q, const void* k, const void* v, void* out, int B, int T, int window,
-                             float scale, int value_is_fp16, int* status, cudaStream_t st);
+                             float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent = 0);
 // Queries [B, Tq, 512] against keys / values [B, Tk, 512], Tk >= Tq: the last Tq key rows are the queries' own
 // frames, the Tk - Tq rows before them are older (cached) frames.
 int launch_band_attn_chunk(const void* q, const void* k, const void* v, void* out, int B, int Tq, int Tk, int window,
-                           float scale, int value_is_fp16, int* status, cudaStream_t st);
+                           float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent = 0);
 // KV ring <-> frame-major tensors for multi-frame cached calls (fm_ring.cu).
 int launch_ring_linearize(const void* ring_k, const void* ring_v, const void* k_new, const void* v_new, void* k_lin,
-                          void* v_lin, int S, int T, int delta, int past, int slots, cudaStream_t st);
+                          void* v_lin, int S, int T, int delta, int past, int slots, cudaStream_t st, int dependent = 0);
 int launch_ring_append(const void* k_new, const void* v_new, void* ring_k, void* ring_v, int S, int T, int past,
-                       int slots, cudaStream_t st);
+                       int slots, cudaStream_t st, int dependent = 0);
+// T <= 8 new frames per stream over its ring (at most 256 slots), ring update included (fm_stream_attn.cu).
+// out_dtype: 2 = FP32, anything else = the value type.
+int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k, void* ring_v, void* out, int S, int T,
+                       int past, int slots, int window, float scale, int value_is_fp16, int out_dtype, int* status,
+                       cudaStream_t st, int dependent = 0);
 // Projection + RoPE + banded attention in one kernel for 128 < T <= 256 (fm_fused_clip.cu): q, k, v stay on chip.
 int launch_attn_fused_clip(const void* x, const void* w_qkv, const float* cos, const float* sin, long long cos_bstride,
                            void* out, int B, int T, int window, float scale, int dtype_flags, int* status,
-                           cudaStream_t st);
+                           cudaStream_t st, int dependent = 0);
+// Whether whole clips take the one-kernel form (fm_fused_clip.cu) rather than projection + attention.
+bool use_fused_clip(int B);
 int launch_band_attn_clip(const void* q, const void* k, const void* v, void* out, int B, int T, int window,
-                          float scale, int value_is_fp16, int* status, cudaStream_t st);
+                          float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent = 0);
 int launch_band_attn_long(const void* q, const void* k, const void* v, void* out, int B, int T, int window,
-                          float scale, int value_is_fp16, int* status, cudaStream_t st);
+                          float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent = 0);
 int launch_ring_decode_attn(const void* q, const void* ring_k, const void* ring_v, float* out,
                             const int* stream_pos, int pos_base, int S, int ring_slots, float scale,
                             int value_is_fp16, int* status, cudaStream_t st);

@@ -12,6 +12,7 @@
 
 #include "fm_common.cuh"
 #include "fm_kernels.h"
+#include "fm_launch.h"
 
 namespace fm {
 
@@ -22,11 +23,11 @@ constexpr int kWarpsPerBlock = 8;
 template <int kIn>
 __device__ __forceinline__ void load4(const void* base, long long elem, float (&v)[4]) {
   if constexpr (kIn == 2) {
-    const float4 f = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(base) + elem));
+    const float4 f = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(base) + elem));
     v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
   } else {
     using T16 = typename std::conditional<kIn == 1, __half, __nv_bfloat16>::type;
-    const uint2 u = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(base) + elem));
+    const uint2 u = __ldcg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(base) + elem));
     const float2 a = Pack16<T16>::unpack(u.x), b = Pack16<T16>::unpack(u.y);
     v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
   }
@@ -40,6 +41,10 @@ layernorm512_kernel(const void* __restrict__ x, const float* __restrict__ weight
                     float eps, void* __restrict__ y, long long rows) {
   using namespace ln;
   using TOut = typename std::conditional<kOut == 1, __half, __nv_bfloat16>::type;
+  // This kernel opens a layer's chain of dependent launches: it lets the next kernel start only after its own wait, so
+  // whatever that one reads ahead of ITS wait (weights) was complete before the chain began.
+  griddep_wait();
+  griddep_launch();
   const int lane = threadIdx.x & 31;
   const long long warp0 = static_cast<long long>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
   const long long stride = static_cast<long long>(gridDim.x) * kWarpsPerBlock;
@@ -86,7 +91,7 @@ layernorm512_kernel(const void* __restrict__ x, const float* __restrict__ weight
 }
 
 int launch_layernorm512(const void* x, int x_dtype, const float* weight, const float* bias, float eps, void* y,
-                        int y_dtype, long long rows, cudaStream_t st) {
+                        int y_dtype, long long rows, cudaStream_t st, int dependent) {
   using namespace ln;
   if (rows < 0 || x_dtype < 0 || x_dtype > 2 || y_dtype < 0 || y_dtype > 1) return -1;
   if (rows == 0) return 0;
@@ -94,18 +99,15 @@ int launch_layernorm512(const void* x, int x_dtype, const float* weight, const f
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(weight) |
        reinterpret_cast<uintptr_t>(bias)) & 15u)
     return -3;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long want = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  const long long cap = static_cast<long long>(sms > 0 ? sms : 1) * 8;    // 8 resident blocks of 256 threads per SM
+  const long long cap = static_cast<long long>(sm_count()) * 8;    // 8 resident blocks of 256 threads per SM
   const int grid = static_cast<int>(want < cap ? want : cap);
   using Kern = void (*)(const void*, const float*, const float*, float, void*, long long);
   static const Kern table[3][2] = {{layernorm512_kernel<0, 0>, layernorm512_kernel<0, 1>},
                                    {layernorm512_kernel<1, 0>, layernorm512_kernel<1, 1>},
                                    {layernorm512_kernel<2, 0>, layernorm512_kernel<2, 1>}};
-  table[x_dtype][y_dtype]<<<grid, kWarpsPerBlock * 32, 0, st>>>(x, weight, bias, eps, y, rows);
-  return static_cast<int>(cudaGetLastError());
+  return launch_kernel(table[x_dtype][y_dtype], dim3(grid), kWarpsPerBlock * 32, 0, st, 1, dependent, x, weight, bias, eps, y,
+                       rows);
 }
 
 }  // namespace fm

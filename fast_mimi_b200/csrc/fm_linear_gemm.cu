@@ -28,6 +28,7 @@
 
 #include "fm_common.cuh"
 #include "fm_kernels.h"
+#include "fm_launch.h"
 
 namespace fm {
 
@@ -63,26 +64,6 @@ struct Barriers {
 };
 static_assert(sizeof(Barriers) <= 256, "barrier block too large");
 
-// Exact-form GELU  0.5 x (1 + erf(x / sqrt 2))  with erf from the rational approximation
-//   erf(z) = 1 - (1 + a1 z + ... + a6 z^6)^-16,  z >= 0,  |error| <= 3e-7   (Abramowitz & Stegun 7.1.28)
-// instead of erff(): 15 issue slots and one reciprocal per value, no branch.  The epilogue is arithmetic-bound
-// with erff() (about 40 slots per value); the approximation error is far below the rounding of the result
-// to 16 bit.  Large |z| overflows the power to +inf, whose reciprocal is 0, i.e. erf = 1.
-__device__ __forceinline__ float gelu_erf(float x) {
-  const float z = fabsf(x) * 0.70710678118654752f;
-  float t = fmaf(z, 0.0000430638f, 0.0002765672f);
-  t = fmaf(z, t, 0.0001520143f);
-  t = fmaf(z, t, 0.0092705272f);
-  t = fmaf(z, t, 0.0422820123f);
-  t = fmaf(z, t, 0.0705230784f);
-  t = fmaf(z, t, 1.0f);
-  t *= t; t *= t; t *= t; t *= t;
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(t));
-  const float e = copysignf(1.0f - r, x);
-  const float hx = 0.5f * x;
-  return fmaf(hx, e, hx);
-}
 }  // namespace lin
 
 struct LinearArgs {
@@ -143,6 +124,8 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();
+  griddep_launch();
+  if (warp != kEpiWarps) griddep_wait();   // the residual may come from the kernel in front (the producer waits below)
   tc_fence_after_sync();
   const uint32_t tmem_base = bars->tmem_base;
   CtaCtl* ctl = &bars->ctl;
@@ -159,16 +142,27 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
       tma_prefetch_desc(&tmap_w);
       int stage = 0;
       uint32_t phase = 0;
+      // The W slices of the first stages do not depend on the kernel in front: they are requested before the wait.
+      const int ahead = u_count > 0 ? (k_chunks < kStages ? k_chunks : kStages) : 0;
+      for (int kc = 0; kc < ahead; ++kc) {
+        if (leader) mbar_arrive_expect_tx(&bars->full[kc], 2 * kStageBytes);
+        tma_load_2d_pair(smem_stage + kc * kStageBytes + kABytes, &tmap_w, &bars->full[kc], kc * kBlockK,
+                         (pair % n_tiles) * kBlockN + static_cast<int>(rank) * kHalfN);
+      }
+      griddep_wait();
       for (int i = 0; i < u_count; ++i) {
         const int u = pair + i * n_pairs, row_tile = u / n_tiles, ntile = u % n_tiles;
         const int m0 = (2 * row_tile + static_cast<int>(rank)) * kBlockM;
         const int n0 = ntile * kBlockN + static_cast<int>(rank) * kHalfN;
         for (int kc = 0; kc < k_chunks; ++kc) {
-          mbar_wait(&bars->empty[stage], phase ^ 1u, ctl, status, kErrWaitConsumer);
-          if (leader) mbar_arrive_expect_tx(&bars->full[stage], 2 * kStageBytes);
+          const bool early = i == 0 && kc < ahead;
+          if (!early) {
+            mbar_wait(&bars->empty[stage], phase ^ 1u, ctl, status, kErrWaitConsumer);
+            if (leader) mbar_arrive_expect_tx(&bars->full[stage], 2 * kStageBytes);
+          }
           uint8_t* dst = smem_stage + stage * kStageBytes;
           tma_load_2d_pair(dst, &tmap_a, &bars->full[stage], kc * kBlockK, m0);
-          tma_load_2d_pair(dst + kABytes, &tmap_w, &bars->full[stage], kc * kBlockK, n0);
+          if (!early) tma_load_2d_pair(dst + kABytes, &tmap_w, &bars->full[stage], kc * kBlockK, n0);
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
       }
@@ -279,7 +273,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             const float4* r4 = reinterpret_cast<const float4*>(static_cast<const float*>(args.resid) + row * args.N + col0);
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-              const float4 r = __ldg(r4 + j);
+              const float4 r = r4[j];
               v[4 * j] += r.x; v[4 * j + 1] += r.y; v[4 * j + 2] += r.z; v[4 * j + 3] += r.w;
             }
           } else {
@@ -287,7 +281,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             const uint4* r4 = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(args.resid) + row * args.N + col0);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-              const uint4 r = __ldg(r4 + j);
+              const uint4 r = r4[j];
               const uint32_t w4[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
@@ -359,7 +353,7 @@ static int encode_2d(CUtensorMap* map, CUtensorMapDataType type, int elem_bytes,
 }
 
 int launch_linear_gemm(const void* a, const void* w, void* y, const float* scale, const void* resid, int M, int N,
-                       int K, int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st) {
+                       int K, int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent) {
   using namespace lin;
   if (M < 0 || N <= 0 || K <= 0 || N % kBlockN != 0 || K % kBlockK != 0) return -1;
   if (in_dtype < 0 || in_dtype > 1 || out_dtype < 0 || out_dtype > 3) return -1;
@@ -369,6 +363,8 @@ int launch_linear_gemm(const void* a, const void* w, void* y, const float* scale
   if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y) |
        reinterpret_cast<uintptr_t>(scale) | reinterpret_cast<uintptr_t>(resid)) & 15u)
     return -3;
+  if (out_dtype != 3 && few_row_tiles(M, N))
+    return launch_linear_small(a, w, y, scale, resid, M, N, K, in_dtype, out_dtype, gelu, status, st, dependent);
   CUtensorMap tmap_a, tmap_w, tmap_y;
   const CUtensorMapDataType t16 = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;   // any 16-bit element type moves alike
   int rc = encode_2d(&tmap_a, t16, 2, a, static_cast<uint64_t>(M), static_cast<uint64_t>(K), kBlockM, kBlockK);
@@ -385,10 +381,7 @@ int launch_linear_gemm(const void* a, const void* w, void* y, const float* scale
   const int m_tiles = (M + kBlockM - 1) / kBlockM;
   const int pair_tiles = (m_tiles + 1) / 2;
   const int total_units = pair_tiles * (N / kBlockN);
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int max_pairs = sms / 2 > 0 ? sms / 2 : 1;
+  const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
   const int n_pairs = total_units < max_pairs ? total_units : max_pairs;
   const int fmt = in_dtype == 1 ? 0 : 1;   // tcgen05 kind::f16 operand format: 0 = F16, 1 = BF16
   const uint32_t idesc = umma_idesc_f16(2 * kBlockM, kBlockN, fmt, fmt, 0, 0);
@@ -406,8 +399,8 @@ int launch_linear_gemm(const void* a, const void* w, void* y, const float* scale
   const int threads = wide ? Shape<true>::kThreads : Shape<false>::kThreads;
   rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes);
   if (rc != 0) return rc;
-  kern<<<2 * n_pairs, threads, smem_bytes, st>>>(tmap_a, tmap_w, tmap_y, args, total_units, idesc, status);
-  return static_cast<int>(cudaGetLastError());
+  return launch_kernel(kern, dim3(2 * n_pairs), threads, smem_bytes, st, 1, dependent, tmap_a, tmap_w, tmap_y, args, total_units,
+                       idesc, status);
 }
 
 }  // namespace fm

@@ -1,0 +1,335 @@
+// Linear layers and the QKV projection for few rows (sm_100a): y = residual + scale * act(a W^T), or q | k | v with
+// RoPE, for calls whose rows fill only a few 128-row tiles (one clip, one frame of up to a few hundred streams).
+//
+// What bounds such a call is latency and the number of SMs that pull weights out of L2, not arithmetic: the pair
+// kernels (fm_linear_gemm.cu, fm_qkv_gemm.cu) cut the output into 256 x 256 tiles, so that 125 rows x 512 outputs at
+// K = 2048 occupied 4 of 148 SMs, each walking 32 K-chunks one after the other (33 us; here 5 us).  Here a block owns
+// 128 rows x 64 outputs (one attention head) and a SLICE of K: the blocks of a thread-block cluster share one output
+// tile and split K between them, so the same layer runs on 64 SMs with four chunks each.  The partial sums meet in
+// distributed shared memory: row r of the tile belongs to cluster rank r % S, every block writes its FP32 partials of
+// that row straight into the owner's shared memory, one cluster barrier, and the owner adds them in rank order (the
+// result does not depend on timing), applies the epilogue and stores whole 64-byte segments.
+//
+// Weights do not depend on the kernel in front, so in a chain of dependent launches the W slices of the first stages
+// are requested before the wait for that kernel and arrive while it still runs.  About 105 KB of shared memory and 64
+// tensor-memory columns per block leave room for the next kernel's blocks on the same SM, which is what makes that
+// overlap possible.
+//
+// Warps 0-3: accumulator rows out of tensor memory.  Warp 4: TMA.  Warp 5: MMA.  All six finish the owned rows.
+#include <type_traits>
+
+#include "fm_common.cuh"
+#include "fm_kernels.h"
+#include "fm_launch.h"
+
+namespace fm {
+
+namespace small {
+constexpr int kBlockM = 128;
+constexpr int kBlockN = 64;
+constexpr int kBlockK = 64;
+constexpr int kStages = 3;
+constexpr int kABytes = kBlockM * kBlockK * 2;     // 16 KB
+constexpr int kBBytes = kBlockN * kBlockK * 2;     // 8 KB
+constexpr int kStageBytes = kABytes + kBBytes;
+constexpr int kRedBytes = kBlockM * kBlockN * 4;   // S sources x (128 / S) rows x 64 FP32
+constexpr int kThreads = 192;
+constexpr int kTmemCols = 64;
+constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kRedBytes + 128;
+
+struct Barriers {
+  uint64_t full[kStages];
+  uint64_t empty[kStages];
+  uint64_t acc_full;
+  uint32_t tmem_base;
+  CtaCtl ctl;
+};
+static_assert(sizeof(Barriers) <= 128, "barrier block too large");
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, float a, float b, float c, float d) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+// 16-byte piece `c` (0..15) of row `r` of the reduction buffer; the low three bits are permuted by the row so that
+// eight lanes with consecutive rows (writing) or consecutive pieces (reading) touch eight different bank groups.
+__device__ __forceinline__ uint32_t red_offset(uint32_t r, uint32_t c) { return r * 256u + ((c ^ (r & 7u)) << 4); }
+}  // namespace small
+
+struct SmallArgs {
+  const float* scale;     // [N] or null
+  const void* resid;      // [M, N] in the output's type or null
+  void* y;                // [M, N]
+  int M, N, chunks;       // chunks: K / 64 / S, this block's share
+  int split;              // S, blocks per cluster
+  int gelu;
+  QkvEpilogueArgs qkv;    // kOut 3
+};
+
+// kOut: 0 = BF16, 1 = FP16, 2 = FP32 output and residual; 3 = q | k | v with RoPE (VT: type of v)
+template <int kOut, typename VT>
+__global__ void __launch_bounds__(small::kThreads)
+linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
+                    const __grid_constant__ SmallArgs args, uint32_t idesc, int* status) {
+  using namespace small;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* red = smem + kStages * kStageBytes;
+  Barriers* bars = reinterpret_cast<Barriers*>(red + kRedBytes);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int split = args.split;
+  const int rank = split > 1 ? static_cast<int>(cluster_cta_rank()) : 0;
+  const int ntile = static_cast<int>(blockIdx.x) / split;
+  const int n0 = ntile * kBlockN;
+  const int m0 = static_cast<int>(blockIdx.y) * kBlockM;
+  const int chunk0 = rank * args.chunks;
+
+  // read early: a status set before this chain began stops every kernel of it (the stores are left out)
+  const bool skip = status != nullptr && *reinterpret_cast<volatile int*>(status) != 0;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(&bars->full[i], 1);
+      mbar_init(&bars->empty[i], 1);
+    }
+    mbar_init(&bars->acc_full, 1);
+    bars->ctl.abort = 0;
+    fence_mbar_init();
+  }
+  if (warp == 5) {
+    tmem_alloc(&bars->tmem_base, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  if (split > 1) cluster_arrive();        // "this block runs": its shared memory may be written from now on
+  griddep_launch();
+  const uint32_t tmem_base = bars->tmem_base;
+  CtaCtl* ctl = &bars->ctl;
+
+  if (warp == 4) {
+    if (lane == 0) {
+      tma_prefetch_desc(&tmap_a);
+      const int ahead = args.chunks < kStages ? args.chunks : kStages;
+      for (int i = 0; i < ahead; ++i) {
+        mbar_arrive_expect_tx(&bars->full[i], kStageBytes);
+        tma_load_2d(smem + i * kStageBytes + kABytes, &tmap_w, &bars->full[i], (chunk0 + i) * kBlockK, n0);
+      }
+      griddep_wait();
+      for (int i = 0; i < ahead; ++i)
+        tma_load_2d(smem + i * kStageBytes, &tmap_a, &bars->full[i], (chunk0 + i) * kBlockK, m0);
+      for (int i = ahead; i < args.chunks; ++i) {
+        const int st = i % kStages;
+        mbar_wait(&bars->empty[st], (static_cast<uint32_t>(i / kStages) & 1u) ^ 1u, ctl, status, kErrWaitConsumer);
+        mbar_arrive_expect_tx(&bars->full[st], kStageBytes);
+        tma_load_2d(smem + st * kStageBytes + kABytes, &tmap_w, &bars->full[st], (chunk0 + i) * kBlockK, n0);
+        tma_load_2d(smem + st * kStageBytes, &tmap_a, &bars->full[st], (chunk0 + i) * kBlockK, m0);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 5) {
+    const bool one = elect_one();
+    for (int i = 0; i < args.chunks; ++i) {
+      const int st = i % kStages;
+      mbar_wait(&bars->full[st], static_cast<uint32_t>(i / kStages) & 1u, ctl, status, kErrWaitTma);
+      tc_fence_after_sync();
+      const uint32_t base = smem_u32(smem + st * kStageBytes);
+      const uint64_t a_desc = umma_desc_sw128(base);
+      const uint64_t b_desc = umma_desc_sw128(base + kABytes);
+#pragma unroll
+      for (int ks = 0; ks < kBlockK / 16; ++ks)
+        if (one) tc_mma_ss(tmem_base, a_desc + 2u * ks, b_desc + 2u * ks, idesc, (i | ks) != 0 ? 1u : 0u);
+      if (one) tc_commit(&bars->empty[st]);
+    }
+    if (one) tc_commit(&bars->acc_full);
+    __syncwarp();
+  } else {
+    mbar_wait(&bars->acc_full, 0, ctl, status, kErrWaitMma);
+    tc_fence_after_sync();
+  }
+  griddep_wait();                          // residual and outputs belong to the chain
+  if (split > 1) cluster_wait();           // every block of the cluster runs
+  const int log_s = 31 - __clz(split);
+  if (warp < 4) {
+    const int row = warp * 32 + lane;
+    const int owner = row & (split - 1), slot = rank * (kBlockM >> log_s) + (row >> log_s);
+    uint32_t red_addr = smem_u32(red);
+    if (split > 1) red_addr = map_to_cta(red_addr, static_cast<uint32_t>(owner));
+    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t v[32];
+      tmem_ld32(t_row + h * 32, v);
+      tmem_ld_wait();
+      if (m0 + row < args.M) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          st_cluster_v4(red_addr + red_offset(slot, h * 8 + c), __uint_as_float(v[4 * c]), __uint_as_float(v[4 * c + 1]),
+                        __uint_as_float(v[4 * c + 2]), __uint_as_float(v[4 * c + 3]));
+      }
+    }
+    tc_fence_before_sync();
+  }
+  if (split > 1) {
+    cluster_arrive();
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
+
+  // The rows this block owns: rank, rank + S, ... of the tile; eight threads per row, columns 4j.. and 32 + 4j...
+  const int valid = args.M - m0 < kBlockM ? args.M - m0 : kBlockM;
+  const int n_own = skip ? 0 : (valid - rank + split - 1) >> log_s;
+  for (int item = static_cast<int>(threadIdx.x); item < n_own * 8; item += kThreads) {
+    const int local = item >> 3, j = item & 7;
+    const long long row = m0 + (local << log_s) + rank;
+    float lo[4] = {0.f, 0.f, 0.f, 0.f}, hi[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int s = 0; s < split; ++s) {
+      const uint32_t r = s * (kBlockM >> log_s) + local;
+      const float4 a = *reinterpret_cast<const float4*>(red + red_offset(r, j));
+      const float4 b = *reinterpret_cast<const float4*>(red + red_offset(r, j + 8));
+      lo[0] += a.x; lo[1] += a.y; lo[2] += a.z; lo[3] += a.w;
+      hi[0] += b.x; hi[1] += b.y; hi[2] += b.z; hi[3] += b.w;
+    }
+    if constexpr (kOut == 3) {
+      const QkvEpilogueArgs& ep = args.qkv;
+      const int seg = ntile >> 3, head = ntile & 7;
+      const int clip = static_cast<int>(row / ep.T), t = static_cast<int>(row % ep.T);
+      uint2 plo, phi;
+      if (seg < 2) {
+        const long long at = clip * ep.cos_bstride + static_cast<long long>(t) * 64 + 4 * j;
+        const float4 c4 = *reinterpret_cast<const float4*>(ep.cos + at), s4 = *reinterpret_cast<const float4*>(ep.sin + at);
+        const float c[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
+        float o_lo[4], o_hi[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          o_lo[e] = lo[e] * c[e] - hi[e] * sn[e];
+          o_hi[e] = hi[e] * c[e] + lo[e] * sn[e];
+        }
+        plo = make_uint2(Pack16<__nv_bfloat16>::pack(o_lo[0], o_lo[1]), Pack16<__nv_bfloat16>::pack(o_lo[2], o_lo[3]));
+        phi = make_uint2(Pack16<__nv_bfloat16>::pack(o_hi[0], o_hi[1]), Pack16<__nv_bfloat16>::pack(o_hi[2], o_hi[3]));
+      } else {
+        plo = make_uint2(Pack16<VT>::pack(lo[0], lo[1]), Pack16<VT>::pack(lo[2], lo[3]));
+        phi = make_uint2(Pack16<VT>::pack(hi[0], hi[1]), Pack16<VT>::pack(hi[2], hi[3]));
+      }
+      uint16_t* lin = seg == 0 ? ep.q : (seg == 1 ? ep.k : ep.v);
+      if (lin != nullptr) {
+        uint16_t* dst = lin + row * 512 + head * 64 + 4 * j;
+        *reinterpret_cast<uint2*>(dst) = plo;
+        *reinterpret_cast<uint2*>(dst + 32) = phi;
+      }
+      uint16_t* ring = seg == 1 ? ep.ring_k : (seg == 2 ? ep.ring_v : nullptr);
+      if (ring != nullptr) {
+        const int pos = ep.pos_base + (ep.clip_pos != nullptr ? ep.clip_pos[clip] : 0) + t;
+        if (pos < 0) {                     // would index another stream's ring: recorded, not written
+          if (status != nullptr) atomicMax(status, static_cast<int>(kErrBounds));
+        } else if (t >= ep.T - ep.ring_slots) {
+          uint16_t* dst = ring + ((static_cast<long long>(clip) * 8 + head) * ep.ring_slots + pos % ep.ring_slots) * 64 + 4 * j;
+          *reinterpret_cast<uint2*>(dst) = plo;
+          *reinterpret_cast<uint2*>(dst + 32) = phi;
+        }
+      }
+    } else {
+      const long long at = row * args.N + n0 + 4 * j;
+      float* part[2] = {lo, hi};
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float* v = part[h];
+        if (args.gelu) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[e] = gelu_erf(v[e]);
+        }
+        if (args.scale != nullptr) {
+          const float4 s = __ldg(reinterpret_cast<const float4*>(args.scale + n0 + 32 * h + 4 * j));
+          v[0] *= s.x; v[1] *= s.y; v[2] *= s.z; v[3] *= s.w;
+        }
+        if constexpr (kOut == 2) {
+          if (args.resid != nullptr) {
+            const float4 r = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(args.resid) + at + 32 * h));
+            v[0] += r.x; v[1] += r.y; v[2] += r.z; v[3] += r.w;
+          }
+          *reinterpret_cast<float4*>(static_cast<float*>(args.y) + at + 32 * h) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+          using T16 = typename std::conditional<kOut == 1, __half, __nv_bfloat16>::type;
+          if (args.resid != nullptr) {
+            const uint2 r = __ldcg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(args.resid) + at + 32 * h));
+            const float2 a = Pack16<T16>::unpack(r.x), b = Pack16<T16>::unpack(r.y);
+            v[0] += a.x; v[1] += a.y; v[2] += b.x; v[3] += b.y;
+          }
+          *reinterpret_cast<uint2*>(static_cast<uint16_t*>(args.y) + at + 32 * h) =
+              make_uint2(Pack16<T16>::pack(v[0], v[1]), Pack16<T16>::pack(v[2], v[3]));
+        }
+      }
+    }
+  }
+
+  __syncthreads();
+  if (ctl->abort) __nanosleep(20000);   // copies that may still be in flight get time to land
+  if (warp == 5) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, kTmemCols);
+  }
+}
+
+// Two blocks fit an SM, so up to two 128 x 64 tiles per SM the grid runs in one wave and a tile's latency is all there is.
+// Beyond that the blocks re-read activations and weights too often for what they save, and the 256 x 256 tiles of the
+// pair kernels are faster: at K = 512, N = 2048 1024 rows (256 tiles) take 9.1 us here and 10.9 us there, 1500 rows (384
+// tiles) 13.9 against 10.9; at K = 2048, N = 512 3678 rows (232 tiles) 17.1 against 22.1, 5000 rows (320) 27.5 against 22.5.
+bool few_row_tiles(int M, int N) {
+  return static_cast<long long>((M + small::kBlockM - 1) / small::kBlockM) * (N / small::kBlockN) <= 2ll * sm_count();
+}
+
+// Blocks per cluster: as many as keep the grid within one block per SM and divide the K chunks.
+static int choose_split(int tiles, int k_chunks) {
+  int s = 8;
+  while (s > 1 && (k_chunks % s != 0 || tiles * s > sm_count())) s >>= 1;
+  return s;
+}
+
+template <int kOut, typename VT>
+static int launch_small(const void* a, const void* w, SmallArgs& args, int K, int in_dtype, int* status,
+                        cudaStream_t st, int dependent) {
+  using namespace small;
+  CUtensorMap tmap_a, tmap_w;
+  int rc = encode_rows_16bit(&tmap_a, a, static_cast<uint64_t>(args.M), static_cast<uint64_t>(K), kBlockM, kBlockK);
+  if (rc != 0) return rc;
+  rc = encode_rows_16bit(&tmap_w, w, static_cast<uint64_t>(args.N), static_cast<uint64_t>(K), kBlockN, kBlockK);
+  if (rc != 0) return rc;
+  const int m_tiles = (args.M + kBlockM - 1) / kBlockM, n_tiles = args.N / kBlockN;
+  args.split = choose_split(m_tiles * n_tiles, K / kBlockK);
+  args.chunks = K / kBlockK / args.split;
+  const int fmt = in_dtype == 1 ? 0 : 1;
+  const uint32_t idesc = umma_idesc_f16(kBlockM, kBlockN, fmt, fmt, 0, 0);
+  auto kern = linear_small_kernel<kOut, VT>;
+  rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
+  if (rc != 0) return rc;
+  return launch_kernel(kern, dim3(n_tiles * args.split, m_tiles), kThreads, kSmemBytes, st, args.split, dependent, tmap_a,
+                       tmap_w, args, idesc, status);
+}
+
+int launch_linear_small(const void* a, const void* w, void* y, const float* scale, const void* resid, int M, int N, int K,
+                        int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent) {
+  SmallArgs args = {};
+  args.scale = scale;
+  args.resid = resid;
+  args.y = y;
+  args.M = M;
+  args.N = N;
+  args.gelu = gelu;
+  if (out_dtype == 2) return launch_small<2, __half>(a, w, args, K, in_dtype, status, st, dependent);
+  if (out_dtype == 1) return launch_small<1, __half>(a, w, args, K, in_dtype, status, st, dependent);
+  return launch_small<0, __half>(a, w, args, K, in_dtype, status, st, dependent);
+}
+
+int launch_qkv_small(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status,
+                     cudaStream_t st, int dependent) {
+  SmallArgs args = {};
+  args.M = M;
+  args.N = 1536;
+  args.qkv = ep;
+  const int in_dtype = (dtype_flags & 2) ? 1 : 0;
+  if (dtype_flags & 1) return launch_small<3, __half>(x, w_qkv, args, 512, in_dtype, status, st, dependent);
+  return launch_small<3, __nv_bfloat16>(x, w_qkv, args, 512, in_dtype, status, st, dependent);
+}
+
+}  // namespace fm

@@ -20,6 +20,7 @@
 // key axis, key row j of Tk = delta + Tq is visible iff  i + delta - W < j <= i + delta.
 #include "fm_common.cuh"
 #include "fm_kernels.h"
+#include "fm_launch.h"
 
 namespace fm {
 
@@ -54,7 +55,7 @@ band_attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
                          const __grid_constant__ CUtensorMap tmap_v, uint16_t* __restrict__ out, int T, int Tk,
                          int delta, int window, float scale_log2e, int* status) {
   using namespace fmha;
-  if (status != nullptr && *reinterpret_cast<volatile int*>(status) != 0) return;
+  if (chain_stopped(status)) return;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -95,6 +96,8 @@ band_attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  griddep_launch();
+  griddep_wait();                       // q, k, v may come from the kernel in front
   const uint32_t tmem_base = bars->tmem_base;
   const uint32_t tmem_s = tmem_base;
   const uint32_t tmem_o = tmem_base + 128;
@@ -296,7 +299,7 @@ static int encode_clip_tile(CUtensorMap* map, const void* base, int B, int T, CU
 }
 
 static int launch_general(const void* q, const void* k, const void* v, void* out, int B, int T, int Tk, int delta,
-                          int window, float scale, int value_is_fp16, int* status, cudaStream_t st) {
+                          int window, float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent) {
   using namespace fmha;
   if (B > 65535) return -1;
   CUtensorMap tq, tk, tv;
@@ -311,24 +314,23 @@ static int launch_general(const void* q, const void* k, const void* v, void* out
   if (rc != 0) return rc;
   dim3 grid((T + kTile - 1) / kTile, 8, B);
   const float scale_log2e = scale * 1.4426950408889634f;
-  kern<<<grid, kThreads, kSmemBytes, st>>>(tq, tk, tv, static_cast<uint16_t*>(out), T, Tk, delta, window, scale_log2e,
-                                          status);
-  return static_cast<int>(cudaGetLastError());
+  return launch_kernel(kern, grid, kThreads, kSmemBytes, st, 1, dependent, tq, tk, tv, static_cast<uint16_t*>(out), T, Tk, delta,
+                       window, scale_log2e, status);
 }
 
 int launch_band_attn_chunk(const void* q, const void* k, const void* v, void* out, int B, int Tq, int Tk, int window,
-                           float scale, int value_is_fp16, int* status, cudaStream_t st) {
+                           float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent) {
   if (B <= 0 || Tq <= 0) return (B == 0 || Tq == 0) ? 0 : -1;
   if (window <= 0 || Tk < Tq) return -1;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
        reinterpret_cast<uintptr_t>(out)) & 15u)
     return -3;
-  if (Tk == Tq) return launch_band_attn_prefill(q, k, v, out, B, Tq, window, scale, value_is_fp16, status, st);
-  return launch_general(q, k, v, out, B, Tq, Tk, Tk - Tq, window, scale, value_is_fp16, status, st);
+  if (Tk == Tq) return launch_band_attn_prefill(q, k, v, out, B, Tq, window, scale, value_is_fp16, status, st, dependent);
+  return launch_general(q, k, v, out, B, Tq, Tk, Tk - Tq, window, scale, value_is_fp16, status, st, dependent);
 }
 
 int launch_band_attn_prefill(const void* q, const void* k, const void* v, void* out, int B, int T, int window,
-                             float scale, int value_is_fp16, int* status, cudaStream_t st) {
+                             float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent) {
   using namespace fmha;
   if (B <= 0 || T <= 0) return (B == 0 || T == 0) ? 0 : -1;
   if (window <= 0 || B > 65535) return -1;
@@ -337,11 +339,11 @@ int launch_band_attn_prefill(const void* q, const void* k, const void* v, void* 
     return -3;
   // Clips that fit two 128-frame tiles take the whole-clip kernel (one CTA per (clip, head) item).
   if (T > kTile && T <= 2 * kTile && B <= (1 << 27))
-    return launch_band_attn_clip(q, k, v, out, B, T, window, scale, value_is_fp16, status, st);
+    return launch_band_attn_clip(q, k, v, out, B, T, window, scale, value_is_fp16, status, st, dependent);
   // Longer clips whose window spans exactly three key tiles per query tile take the run-walking kernel.
   if (T > 2 * kTile && window > kTile + 1 && window <= 2 * kTile + 1 && B <= (1 << 27))
-    return launch_band_attn_long(q, k, v, out, B, T, window, scale, value_is_fp16, status, st);
-  return launch_general(q, k, v, out, B, T, T, 0, window, scale, value_is_fp16, status, st);
+    return launch_band_attn_long(q, k, v, out, B, T, window, scale, value_is_fp16, status, st, dependent);
+  return launch_general(q, k, v, out, B, T, T, 0, window, scale, value_is_fp16, status, st, dependent);
 }
 
 }  // namespace fm

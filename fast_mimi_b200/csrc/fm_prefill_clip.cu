@@ -22,6 +22,7 @@
 #include "fm_attn_tile.cuh"
 #include "fm_common.cuh"
 #include "fm_kernels.h"
+#include "fm_launch.h"
 
 namespace fm {
 
@@ -70,7 +71,7 @@ band_attn_clip_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
                       float scale_log2e, int* status) {
   using namespace clip;
   using namespace attn_tile;
-  if (status != nullptr && *reinterpret_cast<volatile int*>(status) != 0) return;
+  if (chain_stopped(status)) return;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -108,6 +109,8 @@ band_attn_clip_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  griddep_launch();
+  griddep_wait();                       // q, k, v may come from the kernel in front
   const uint32_t tmem_base = sh->tmem_base;
   CtaCtl* ctl = &sh->ctl;
   const int n_local = (n_items - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
@@ -302,7 +305,7 @@ static int encode_clip_map(CUtensorMap* map, const void* base, int B, int T, uin
 }
 
 int launch_band_attn_clip(const void* q, const void* k, const void* v, void* out, int B, int T, int window, float scale,
-                          int value_is_fp16, int* status, cudaStream_t st) {
+                          int value_is_fp16, int* status, cudaStream_t st, int dependent) {
   using namespace clip;
   if (T <= kTile || T > 2 * kTile || B <= 0 || window <= 0) return -1;
   CUtensorMap tq, tq32, tk, tv, tout;
@@ -315,14 +318,10 @@ int launch_band_attn_clip(const void* q, const void* k, const void* v, void* out
   auto kern = value_is_fp16 ? band_attn_clip_kernel<__half> : band_attn_clip_kernel<__nv_bfloat16>;
   rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
   if (rc != 0) return rc;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int n_items = B * 8;
-  const int grid = n_items < sms ? n_items : sms;
-  kern<<<grid, kThreads, kSmemBytes, st>>>(tq, tq32, tk, tv, tout, n_items, T, window, scale * 1.4426950408889634f,
-                                          status);
-  return static_cast<int>(cudaGetLastError());
+  const int grid = n_items < sm_count() ? n_items : sm_count();
+  return launch_kernel(kern, dim3(grid), kThreads, kSmemBytes, st, 1, dependent, tq, tq32, tk, tv, tout, n_items, T, window,
+                       scale * 1.4426950408889634f, status);
 }
 
 }  // namespace fm

@@ -21,6 +21,7 @@
 #include "fm_attn_tile.cuh"
 #include "fm_common.cuh"
 #include "fm_kernels.h"
+#include "fm_launch.h"
 
 namespace fm {
 
@@ -98,7 +99,7 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
                       int* status) {
   using namespace longclip;
   using namespace attn_tile;
-  if (status != nullptr && *reinterpret_cast<volatile int*>(status) != 0) return;
+  if (chain_stopped(status)) return;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -137,6 +138,8 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  griddep_launch();
+  griddep_wait();                       // q, k, v may come from the kernel in front
   const uint32_t tmem_base = sh->tmem_base;
   CtaCtl* ctl = &sh->ctl;
 
@@ -342,7 +345,7 @@ static int encode_long_map(CUtensorMap* map, const void* base, int B, int T, uin
 }
 
 int launch_band_attn_long(const void* q, const void* k, const void* v, void* out, int B, int T, int window, float scale,
-                          int value_is_fp16, int* status, cudaStream_t st) {
+                          int value_is_fp16, int* status, cudaStream_t st, int dependent) {
   using namespace longclip;
   // three key tiles per query tile: the window must reach into tile t-2 and not beyond it
   if (T <= 2 * kTile || B <= 0 || window <= kTile + 1 || window > 2 * kTile + 1) return -1;
@@ -355,10 +358,7 @@ int launch_band_attn_long(const void* q, const void* k, const void* v, void* out
   auto kern = value_is_fp16 ? band_attn_long_kernel<__half> : band_attn_long_kernel<__nv_bfloat16>;
   rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
   if (rc != 0) return rc;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (sms <= 0) sms = 1;
+  const int sms = sm_count();
   // Runs: whole (clip, head) sequences when there are enough of them to occupy the SMs, else segments of
   // each sequence (a segment re-reads the two K / V tiles in front of it).
   const int n_tiles = (T + kTile - 1) / kTile;
@@ -372,9 +372,8 @@ int launch_band_attn_long(const void* q, const void* k, const void* v, void* out
   if (n_runs_ll > 0x7fffffffLL) return -1;
   const int n_runs = static_cast<int>(n_runs_ll);
   const int grid = n_runs < sms ? n_runs : sms;
-  kern<<<grid, kThreads, kSmemBytes, st>>>(tq, tk, tv, tout, n_runs, n_seg, seg_tiles, n_tiles, T, window,
-                                          scale * 1.4426950408889634f, status);
-  return static_cast<int>(cudaGetLastError());
+  return launch_kernel(kern, dim3(grid), kThreads, kSmemBytes, st, 1, dependent, tq, tk, tv, tout, n_runs, n_seg, seg_tiles,
+                       n_tiles, T, window, scale * 1.4426950408889634f, status);
 }
 
 }  // namespace fm

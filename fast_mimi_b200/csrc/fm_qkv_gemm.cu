@@ -21,6 +21,7 @@
 // x producer.
 #include "fm_common.cuh"
 #include "fm_kernels.h"
+#include "fm_launch.h"
 
 namespace fm {
 
@@ -105,6 +106,8 @@ qkv_rope_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();            // both CTAs' barriers exist before anything signals across the pair
+  griddep_launch();
+  if (warp != kEpiWarps) griddep_wait();   // x may come from the kernel in front; the W loads need not wait for it
   tc_fence_after_sync();
   const uint32_t tmem_base = bars->tmem_base;
   CtaCtl* ctl = &bars->ctl;
@@ -307,7 +310,7 @@ qkv_rope_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
             if (ep.resid != nullptr && row_ok) {
               // this frame's 32 + 32 bytes of the residual: whole sectors, read once
               const uint4* r_lo = reinterpret_cast<const uint4*>(ep.resid + row * 512 + head * 64 + piece * 16);
-              const uint4 r[4] = {__ldg(r_lo), __ldg(r_lo + 1), __ldg(r_lo + 4), __ldg(r_lo + 5)};
+              const uint4 r[4] = {r_lo[0], r_lo[1], r_lo[4], r_lo[5]};
               const uint32_t* rw = reinterpret_cast<const uint32_t*>(r);
 #pragma unroll
               for (int d = 0; d < 16; d += 2) {
@@ -363,43 +366,30 @@ qkv_rope_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
   }
 }
 
-static int encode_2d_16bit(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
-                           uint32_t box_cols) {
-  const cuuint64_t dims[2] = {cols, rows};
-  const cuuint64_t strides[1] = {cols * 2};
-  const cuuint32_t box[2] = {box_cols, box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                      CU_TENSOR_MAP_SWIZZLE_128B);
-}
-
 static int launch_gemm(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep, int M, int dtype_flags,
-                       int* status, cudaStream_t st) {
+                       int* status, cudaStream_t st, int dependent) {
   using namespace gemm;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w_qkv) | reinterpret_cast<uintptr_t>(ep.q) |
        reinterpret_cast<uintptr_t>(ep.k) | reinterpret_cast<uintptr_t>(ep.v) | reinterpret_cast<uintptr_t>(ep.ring_k) |
        reinterpret_cast<uintptr_t>(ep.ring_v)) & 15u)
     return -3;
   CUtensorMap tmap_x, tmap_w, tmap_q, tmap_k, tmap_v;
-  int rc = encode_2d_16bit(&tmap_x, x, static_cast<uint64_t>(M), kHidden, kBlockM, kBlockK);
+  int rc = encode_rows_16bit(&tmap_x, x, static_cast<uint64_t>(M), kHidden, kBlockM, kBlockK);
   if (rc != 0) return rc;
-  rc = encode_2d_16bit(&tmap_w, w_qkv, static_cast<uint64_t>(ep.n_tiles) * kBlockN, kHidden, kHalfN, kBlockK);
+  rc = encode_rows_16bit(&tmap_w, w_qkv, static_cast<uint64_t>(ep.n_tiles) * kBlockN, kHidden, kHalfN, kBlockK);
   if (rc != 0) return rc;
   // Output maps (16-bit elements whatever the float format); a missing output reuses x as a placeholder
   // that the kernel never stores through.
-  rc = encode_2d_16bit(&tmap_q, ep.q != nullptr ? ep.q : x, static_cast<uint64_t>(M), 512, 32, 64);
+  rc = encode_rows_16bit(&tmap_q, ep.q != nullptr ? ep.q : x, static_cast<uint64_t>(M), 512, 32, 64);
   if (rc != 0) return rc;
-  rc = encode_2d_16bit(&tmap_k, ep.k != nullptr ? ep.k : x, static_cast<uint64_t>(M), 512, 32, 64);
+  rc = encode_rows_16bit(&tmap_k, ep.k != nullptr ? ep.k : x, static_cast<uint64_t>(M), 512, 32, 64);
   if (rc != 0) return rc;
-  rc = encode_2d_16bit(&tmap_v, ep.v != nullptr ? ep.v : x, static_cast<uint64_t>(M), 512, 32, 64);
+  rc = encode_rows_16bit(&tmap_v, ep.v != nullptr ? ep.v : x, static_cast<uint64_t>(M), 512, 32, 64);
   if (rc != 0) return rc;
   const int m_tiles = (M + kBlockM - 1) / kBlockM;
   const int pair_tiles = (m_tiles + 1) / 2;          // an odd last tile gets a partner that works on padding
   const int total_units = pair_tiles * ep.n_tiles;            // (pair of frame tiles, 256-wide output tile)
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int max_pairs = sms / 2 > 0 ? sms / 2 : 1;   // persistent: one CTA per SM, CTAs in pairs
+  const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;   // persistent: one CTA per SM, CTAs in pairs
   const int n_pairs = total_units < max_pairs ? total_units : max_pairs;
   // dtype_flags bit 0: v is written as FP16 (else BF16); bit 1: x and w_qkv hold FP16 (else BF16).
   const int in_fmt = (dtype_flags & 2) ? 0 : 1;   // tcgen05 kind::f16 operand format: 0 = F16, 1 = BF16
@@ -407,13 +397,12 @@ static int launch_gemm(const void* x, const void* w_qkv, const QkvEpilogueArgs& 
   auto kern = (dtype_flags & 1) ? qkv_rope_gemm_kernel<__half> : qkv_rope_gemm_kernel<__nv_bfloat16>;
   rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
   if (rc != 0) return rc;
-  kern<<<2 * n_pairs, kThreads, kSmemBytes, st>>>(tmap_x, tmap_w, tmap_q, tmap_k, tmap_v, ep, M, total_units, idesc,
-                                                      status);
-  return static_cast<int>(cudaGetLastError());
+  return launch_kernel(kern, dim3(2 * n_pairs), kThreads, kSmemBytes, st, 1, dependent, tmap_x, tmap_w, tmap_q, tmap_k, tmap_v,
+                       ep, M, total_units, idesc, status);
 }
 
 int launch_qkv_rope_gemm(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep_in, int M, int dtype_flags,
-                         int* status, cudaStream_t st) {
+                         int* status, cudaStream_t st, int dependent) {
   if (M <= 0) return M == 0 ? 0 : -1;
   if (ep_in.T <= 0 || ep_in.cos == nullptr || ep_in.sin == nullptr) return -1;
   QkvEpilogueArgs ep = ep_in;
@@ -421,7 +410,14 @@ int launch_qkv_rope_gemm(const void* x, const void* w_qkv, const QkvEpilogueArgs
   ep.seg_base = 0;
   ep.out_scale = nullptr;
   ep.resid = nullptr;
-  return launch_gemm(x, w_qkv, ep, M, dtype_flags, status, st);
+  if (few_row_tiles(M, 1536)) {
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w_qkv) | reinterpret_cast<uintptr_t>(ep.q) |
+         reinterpret_cast<uintptr_t>(ep.k) | reinterpret_cast<uintptr_t>(ep.v) | reinterpret_cast<uintptr_t>(ep.ring_k) |
+         reinterpret_cast<uintptr_t>(ep.ring_v)) & 15u)
+      return -3;
+    return launch_qkv_small(x, w_qkv, ep, M, dtype_flags, status, st, dependent);
+  }
+  return launch_gemm(x, w_qkv, ep, M, dtype_flags, status, st, dependent);
 }
 
 int launch_out_proj_gemm(const void* a, const void* w, void* y, const float* out_scale, const void* resid, int M,
@@ -437,7 +433,7 @@ int launch_out_proj_gemm(const void* a, const void* w, void* y, const float* out
   ep.seg_base = 2;
   ep.out_scale = out_scale;
   ep.resid = static_cast<const uint16_t*>(resid);
-  return launch_gemm(a, w, ep, M, dtype_flags, status, st);
+  return launch_gemm(a, w, ep, M, dtype_flags, status, st, 0);
 }
 
 }  // namespace fm

@@ -10,6 +10,7 @@
 // Linearising BEFORE appending matters: a long chunk overwrites slots that its own first rows still attend to.
 #include "fm_common.cuh"
 #include "fm_kernels.h"
+#include "fm_launch.h"
 
 namespace fm {
 
@@ -18,6 +19,8 @@ __global__ void __launch_bounds__(256)
 ring_linearize_kernel(const uint4* __restrict__ ring_k, const uint4* __restrict__ ring_v, const uint4* __restrict__ k_new,
                       const uint4* __restrict__ v_new, uint4* __restrict__ k_lin, uint4* __restrict__ v_lin, int S, int T,
                       int delta, int past, int slots) {
+  griddep_launch();
+  griddep_wait();
   const int Tk = delta + T;
   const long long total = static_cast<long long>(S) * Tk * 64;      // 64 pieces per frame (8 heads x 8)
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -30,12 +33,12 @@ ring_linearize_kernel(const uint4* __restrict__ ring_k, const uint4* __restrict_
     if (j < delta) {
       const int slot = (past - delta + j) % slots;
       const long long src = ((s * 8 + (piece >> 3)) * slots + slot) * 8 + (piece & 7);
-      kv = ring_k[src];
-      vv = ring_v[src];
+      kv = __ldcg(ring_k + src);
+      vv = __ldcg(ring_v + src);
     } else {
       const long long src = (s * T + (j - delta)) * 64 + piece;
-      kv = k_new[src];
-      vv = v_new[src];
+      kv = __ldcg(k_new + src);
+      vv = __ldcg(v_new + src);
     }
     k_lin[i] = kv;
     v_lin[i] = vv;
@@ -45,6 +48,8 @@ ring_linearize_kernel(const uint4* __restrict__ ring_k, const uint4* __restrict_
 __global__ void __launch_bounds__(256)
 ring_append_kernel(const uint4* __restrict__ k_new, const uint4* __restrict__ v_new, uint4* __restrict__ ring_k,
                    uint4* __restrict__ ring_v, int S, int T, int t_first, int past, int slots) {
+  griddep_launch();
+  griddep_wait();
   const int n_t = T - t_first;                                      // rows t_first .. T-1 survive in the ring
   const long long total = static_cast<long long>(S) * n_t * 64;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -56,36 +61,32 @@ ring_append_kernel(const uint4* __restrict__ k_new, const uint4* __restrict__ v_
     const int slot = (past + t) % slots;
     const long long src = (s * T + t) * 64 + piece;
     const long long dst = ((s * 8 + (piece >> 3)) * slots + slot) * 8 + (piece & 7);
-    ring_k[dst] = k_new[src];
-    ring_v[dst] = v_new[src];
+    ring_k[dst] = __ldcg(k_new + src);
+    ring_v[dst] = __ldcg(v_new + src);
   }
 }
 
 static int copy_grid(long long pieces) {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long want = (pieces + 255) / 256;
-  const long long cap = static_cast<long long>(sms > 0 ? sms : 1) * 8;
+  const long long cap = static_cast<long long>(sm_count()) * 8;
   return static_cast<int>(want < cap ? (want > 0 ? want : 1) : cap);
 }
 
 int launch_ring_linearize(const void* ring_k, const void* ring_v, const void* k_new, const void* v_new, void* k_lin,
-                          void* v_lin, int S, int T, int delta, int past, int slots, cudaStream_t st) {
+                          void* v_lin, int S, int T, int delta, int past, int slots, cudaStream_t st, int dependent) {
   if (S <= 0 || T <= 0) return (S == 0 || T == 0) ? 0 : -1;
   if (slots <= 0 || delta < 0 || delta > past || delta >= slots + 1) return -1;
   if ((reinterpret_cast<uintptr_t>(ring_k) | reinterpret_cast<uintptr_t>(ring_v) | reinterpret_cast<uintptr_t>(k_new) |
        reinterpret_cast<uintptr_t>(v_new) | reinterpret_cast<uintptr_t>(k_lin) | reinterpret_cast<uintptr_t>(v_lin)) & 15u)
     return -3;
   const long long pieces = static_cast<long long>(S) * (delta + T) * 64;
-  ring_linearize_kernel<<<copy_grid(pieces), 256, 0, st>>>(
+  return launch_kernel(ring_linearize_kernel, dim3(copy_grid(pieces)), 256, 0, st, 1, dependent,
       static_cast<const uint4*>(ring_k), static_cast<const uint4*>(ring_v), static_cast<const uint4*>(k_new),
       static_cast<const uint4*>(v_new), static_cast<uint4*>(k_lin), static_cast<uint4*>(v_lin), S, T, delta, past, slots);
-  return static_cast<int>(cudaGetLastError());
 }
 
 int launch_ring_append(const void* k_new, const void* v_new, void* ring_k, void* ring_v, int S, int T, int past,
-                       int slots, cudaStream_t st) {
+                       int slots, cudaStream_t st, int dependent) {
   if (S <= 0 || T <= 0) return (S == 0 || T == 0) ? 0 : -1;
   if (slots <= 0 || past < 0) return -1;
   if ((reinterpret_cast<uintptr_t>(ring_k) | reinterpret_cast<uintptr_t>(ring_v) | reinterpret_cast<uintptr_t>(k_new) |
@@ -93,10 +94,9 @@ int launch_ring_append(const void* k_new, const void* v_new, void* ring_k, void*
     return -3;
   const int t_first = T > slots ? T - slots : 0;
   const long long pieces = static_cast<long long>(S) * (T - t_first) * 64;
-  ring_append_kernel<<<copy_grid(pieces), 256, 0, st>>>(static_cast<const uint4*>(k_new), static_cast<const uint4*>(v_new),
-                                                        static_cast<uint4*>(ring_k), static_cast<uint4*>(ring_v), S, T,
-                                                        t_first, past, slots);
-  return static_cast<int>(cudaGetLastError());
+  return launch_kernel(ring_append_kernel, dim3(copy_grid(pieces)), 256, 0, st, 1, dependent, static_cast<const uint4*>(k_new),
+                       static_cast<const uint4*>(v_new), static_cast<uint4*>(ring_k), static_cast<uint4*>(ring_v), S, T, t_first,
+                       past, slots);
 }
 
 }  // namespace fm

@@ -1,0 +1,365 @@
+// Attention of a few new frames per live stream over the stream's KV ring, and the ring's update, in one kernel
+// (sm_100a).  T <= 8 new frames at positions past .. past + T - 1; q, k, v of the new frames come from the projection
+// kernel as [S, T, 512], the ring [S, 8, slots, 64] holds position p in slot p % slots.
+//
+//   out[s, t, h, :] = softmax_p( scale * q . k_p ) v_p     over past + t - W < p <= past + t
+//   ring slot (past + t) % slots <- new row t
+//
+// Covers the reference's cached attention of one or a few frames (MimiKVCache.update's concat-and-crop,
+// src/fast_mimi/model.py:450-471, then SDPA with the band of src/fast_mimi/model.py:2194-2205).
+//
+// HBM-bound once there are more (stream, head) items than SMs, latency-bound below that.  An item is 2 x slots x 128
+// bytes of ring; a persistent block streams items through shared memory (one TMA box each for K and V, 128-byte swizzle,
+// up to three items in flight) and two groups of four warps take them in turn.  What limited the earlier forms was not
+// the copy but the arithmetic around it: a dot product per lane, its conversions and shuffles cost 6400 warp instructions
+// per item, half of the SM's issue slots at full bandwidth.  Here each warp multiplies its 64 slots with mma.sync
+// (m16n8k16, queries as rows, FP32 accumulation): about 600 instructions per item, the same for one query as for eight,
+// so a call of up to eight frames costs the ring's bytes once.  Probabilities stay FP32-grade: they enter P V as the sum
+// of two 16-bit parts.  (tcgen05 would need 128 rows and tensor-memory round trips for at most 8 queries.)
+//
+// Rows that are already in the ring do not depend on the projection, so in a chain of dependent launches the first items
+// are requested before the wait for it.  A block has an item's ring rows in shared memory before it stores that item's
+// new rows, and no other block touches its (stream, head): the ring is updated in place.
+#include <type_traits>
+
+#include "fm_common.cuh"
+#include "fm_kernels.h"
+#include "fm_launch.h"
+
+namespace fm {
+
+namespace stream {
+constexpr int kGroups = 2, kGroupWarps = 4;
+constexpr int kThreads = (kGroups * kGroupWarps + 1) * 32;
+constexpr int kMaxStages = 3;
+constexpr int kMaxT = 8;
+constexpr int kTileBytes = 256 * 128;                 // K or V of an item, padded to 256 slots
+constexpr int kStageBytes = 2 * kTileBytes;
+constexpr int kNewBytes = 2 * 16 * 128;               // new K and V rows of a group's item, padded to 16
+constexpr int kMergeBytes = kGroupWarps * kMaxT * 64 * 4;
+struct Ctl {
+  uint64_t full[kMaxStages];
+  uint64_t empty[kMaxStages];
+  CtaCtl ctl;
+  float m[kGroups][kGroupWarps][kMaxT];
+  float l[kGroups][kGroupWarps][kMaxT];
+};
+constexpr int smem_bytes(int stages) {
+  return 1024 + stages * kStageBytes + kGroups * (kNewBytes + kMergeBytes) + static_cast<int>(sizeof(Ctl));
+}
+static_assert(smem_bytes(kMaxStages) <= 232448, "exceeds the 227 KB a block may use");
+
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// c (rows 0-7 of the 16 x 8 tile; rows 8-15 carry no query) += a[16 x 16] b[16 x 8]
+template <typename T>
+__device__ __forceinline__ void mma_rows8(float (&c)[2], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
+  float z0 = 0.f, z1 = 0.f;
+  if constexpr (std::is_same<T, __half>::value)
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(z0), "+f"(z1) : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
+  else
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(z0), "+f"(z1) : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
+}
+// x, y as hi + lo, both parts of type T
+template <typename T>
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& lo) {
+  hi = Pack16<T>::pack(x, y);
+  const float2 b = Pack16<T>::unpack(hi);
+  lo = Pack16<T>::pack(x - b.x, y - b.y);
+}
+}  // namespace stream
+
+struct StreamArgs {
+  const uint16_t *q, *k, *v;     // [S, T, 512]
+  uint16_t *ring_k, *ring_v;     // [S, 8, slots, 64]
+  void* out;                     // [S, T, 512]
+  int n_items, T, past, delta, slots, window;
+  int n_loaded;                  // ring rows per item that the tensor maps' boxes cover: min(past, slots)
+  int stages;
+  float scale_log2e;
+};
+
+// VT: value type of the ring and v; OT: type of the result
+template <typename VT, typename OT>
+__global__ void __launch_bounds__(stream::kThreads, 1)
+stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+                   const __grid_constant__ StreamArgs a, int* status) {
+  using namespace stream;
+  if (chain_stopped(status)) return;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem_new = smem + a.stages * kStageBytes;
+  float* smem_merge = reinterpret_cast<float*>(smem_new + kGroups * kNewBytes);
+  Ctl* c = reinterpret_cast<Ctl*>(smem_new + kGroups * (kNewBytes + kMergeBytes));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < a.stages; ++i) {
+      mbar_init(&c->full[i], 1);
+      mbar_init(&c->empty[i], kGroupWarps);
+    }
+    c->ctl.abort = 0;
+    fence_mbar_init();
+  }
+  // Slots past the loaded ones and rows past the new ones are never written: zeros, so that a probability of zero times
+  // what lies there is zero.
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  for (int i = threadIdx.x; i < a.stages * 2 * (256 - a.n_loaded) * 8; i += kThreads) {
+    const int per = (256 - a.n_loaded) * 8, tile = i / per, piece = i % per;
+    *reinterpret_cast<uint4*>(smem + tile * kTileBytes + a.n_loaded * 128 + piece * 16) = zero;
+  }
+  for (int i = threadIdx.x; i < kGroups * kNewBytes / 16; i += kThreads) *reinterpret_cast<uint4*>(smem_new + i * 16) = zero;
+  fence_proxy_async_smem();
+  __syncthreads();
+  griddep_launch();
+  CtaCtl* ctl = &c->ctl;
+
+  if (warp == kGroups * kGroupWarps) {
+    if (lane == 0) {
+      if (a.n_loaded > 0) {
+        tma_prefetch_desc(&tmap_k);
+        tma_prefetch_desc(&tmap_v);
+        int n = 0;
+        for (int item = blockIdx.x; item < a.n_items; item += gridDim.x, ++n) {
+          const int st = n % a.stages;
+          mbar_wait(&c->empty[st], (static_cast<uint32_t>(n / a.stages) & 1u) ^ 1u, ctl, status, kErrWaitConsumer);
+          mbar_arrive_expect_tx(&c->full[st], 2u * static_cast<uint32_t>(a.n_loaded) * 128u);
+          tma_load_2d(smem + st * kStageBytes, &tmap_k, &c->full[st], 0, item * a.slots);
+          tma_load_2d(smem + st * kStageBytes + kTileBytes, &tmap_v, &c->full[st], 0, item * a.slots);
+        }
+      }
+      griddep_wait();
+    }
+  } else {
+    griddep_wait();
+    const int cg = warp / kGroupWarps, gw = warp % kGroupWarps, gt = threadIdx.x - cg * kGroupWarps * 32;
+    const int g = lane >> 2, cpair = (lane & 3) * 2;     // mma fragments: query row g; columns cpair, cpair + 1
+    uint8_t* new_k = smem_new + cg * kNewBytes;
+    uint8_t* new_v = new_k + kNewBytes / 2;
+    float* merge = smem_merge + cg * (kMergeBytes / 4);
+    const int first = a.slots > 0 ? (a.past - a.delta) % a.slots : 0;     // slot of the oldest visible row
+    int n = cg;
+    for (long long item = blockIdx.x + static_cast<long long>(cg) * gridDim.x; item < a.n_items;
+         item += static_cast<long long>(kGroups) * gridDim.x, n += kGroups) {
+      const int st = n % a.stages;
+      const int s = static_cast<int>(item >> 3), h = static_cast<int>(item & 7);
+      const size_t new0 = static_cast<size_t>(s) * a.T * 512 + h * 64;
+      // the queries, straight into fragments: 4 K-steps x {columns cpair.., cpair + 8..} of row g
+      uint32_t qa[4][2];
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          qa[ks][e] = g < a.T ? __ldcg(reinterpret_cast<const uint32_t*>(a.q + new0 + static_cast<size_t>(g) * 512 + ks * 16 + e * 8 + cpair)) : 0u;
+      }
+      // the new rows: the group's last warp stages them (row = lane / 2.., 16-byte pieces)
+      uint4 nk[2], nv[2];
+      const int n_pieces = a.T * 8;
+      if (gw == kGroupWarps - 1) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int piece = lane + 32 * e;
+          if (piece < n_pieces) {
+            const size_t at = new0 + static_cast<size_t>(piece >> 3) * 512 + (piece & 7) * 8;
+            nk[e] = __ldcg(reinterpret_cast<const uint4*>(a.k + at));
+            nv[e] = __ldcg(reinterpret_cast<const uint4*>(a.v + at));
+          }
+        }
+      }
+      if (a.n_loaded > 0) mbar_wait(&c->full[st], static_cast<uint32_t>(n / a.stages) & 1u, ctl, status, kErrWaitTma);
+      uint8_t* tile_k = smem + st * kStageBytes;
+      uint8_t* tile_v = tile_k + kTileBytes;
+      if (gw == kGroupWarps - 1) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int piece = lane + 32 * e, t = piece >> 3;
+          if (piece < n_pieces) {
+            *reinterpret_cast<uint4*>(new_k + sw128_offset(t, piece & 7)) = nk[e];
+            *reinterpret_cast<uint4*>(new_v + sw128_offset(t, piece & 7)) = nv[e];
+            if (t >= a.T - a.slots) {                    // of two rows for one slot the newer stays
+              const size_t at = (static_cast<size_t>(item) * a.slots + (a.past + t) % a.slots) * 64 + (piece & 7) * 8;
+              *reinterpret_cast<uint4*>(a.ring_k + at) = nk[e];
+              *reinterpret_cast<uint4*>(a.ring_v + at) = nv[e];
+            }
+          }
+        }
+        __syncwarp();
+      }
+      // Row number of slot j: its distance from the oldest visible row; rows >= delta are no longer visible to anyone.
+      // What such a slot of V holds must not reach the sums through 0 * x.
+      const int slot0 = gw * 64;
+      {
+        bool any = false;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int j = slot0 + lane + 32 * e;
+          int r = j - first;
+          if (r < 0) r += a.slots;
+          if (j < a.n_loaded && r >= a.delta) {
+            any = true;
+#pragma unroll
+            for (int p = 0; p < 8; ++p) *reinterpret_cast<uint4*>(tile_v + j * 128 + p * 16) = zero;
+          }
+        }
+        if (__any_sync(0xffffffffu, any)) {
+          fence_proxy_async_smem();                      // before the stage's next TMA load
+          __syncwarp();
+        }
+      }
+
+      // ---- scores of this warp's eight (nine: with the new rows) 8-key tiles
+      const int n_tiles = a.n_loaded > slot0 ? (a.n_loaded - slot0 + 7) >> 3 : 0;     // of eight
+      float sc[10][2];
+      float m = -INFINITY;
+      const int lo = a.delta + g - a.window + 1, hi = a.delta + g;                    // visible rows of query g
+#pragma unroll
+      for (int nt = 0; nt < 10; ++nt) {
+        sc[nt][0] = sc[nt][1] = -INFINITY;
+        const bool fresh = nt >= 8;
+        if (fresh ? (gw == kGroupWarps - 1 && nt == 8) : nt < n_tiles) {              // the same for the whole warp
+          // x4: keys lane % 8 of the tile, dimensions 8 (lane / 8) .. of the first, then of the second half
+          const int key = fresh ? (lane & 7) : slot0 + nt * 8 + (lane & 7);
+          const uint32_t base = smem_u32(fresh ? new_k : tile_k);
+          uint32_t b01[4], b23[4];
+          ldmatrix4(b01, base + sw128_offset(key, lane >> 3));
+          ldmatrix4(b23, base + sw128_offset(key, 4 + (lane >> 3)));
+          float acc[2] = {0.f, 0.f};
+          mma_rows8<__nv_bfloat16>(acc, qa[0][0], qa[0][1], b01[0], b01[1]);
+          mma_rows8<__nv_bfloat16>(acc, qa[1][0], qa[1][1], b01[2], b01[3]);
+          mma_rows8<__nv_bfloat16>(acc, qa[2][0], qa[2][1], b23[0], b23[1]);
+          mma_rows8<__nv_bfloat16>(acc, qa[3][0], qa[3][1], b23[2], b23[3]);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            int r;
+            if (fresh) {
+              r = a.delta + cpair + e;
+            } else {
+              const int j = slot0 + nt * 8 + cpair + e;
+              r = j - first;
+              if (r < 0) r += a.slots;
+              if (j >= a.n_loaded || r >= a.delta) r = -1 << 20;
+            }
+            if (r >= lo && r <= hi && r >= 0) sc[nt][e] = acc[e] * a.scale_log2e;
+            m = fmaxf(m, sc[nt][e]);
+          }
+        }
+      }
+      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+      const float m_use = m == -INFINITY ? 0.f : m;
+      float l = 0.f;
+#pragma unroll
+      for (int nt = 0; nt < 10; ++nt) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          sc[nt][e] = ex2_approx(sc[nt][e] - m_use);
+          l += sc[nt][e];
+        }
+      }
+      l += __shfl_xor_sync(0xffffffffu, l, 1);
+      l += __shfl_xor_sync(0xffffffffu, l, 2);
+
+      // ---- O = P V, 16 keys per step
+      float o[8][2];
+#pragma unroll
+      for (int d = 0; d < 8; ++d) o[d][0] = o[d][1] = 0.f;
+#pragma unroll
+      for (int ks = 0; ks < 5; ++ks) {
+        const bool fresh = ks == 4;
+        if (fresh ? gw == kGroupWarps - 1 : 2 * ks < n_tiles) {
+          uint32_t h0, l0, h1, l1;
+          split_pair<VT>(sc[2 * ks][0], sc[2 * ks][1], h0, l0);
+          split_pair<VT>(sc[2 * ks + 1][0], sc[2 * ks + 1][1], h1, l1);
+          const int key = (fresh ? 0 : slot0 + ks * 16) + (lane & 15);
+          const uint32_t base = smem_u32(fresh ? new_v : tile_v);
+#pragma unroll
+          for (int dp = 0; dp < 4; ++dp) {               // 16 dimensions: two 8-wide column tiles
+            uint32_t b[4];
+            ldmatrix4_trans(b, base + sw128_offset(key, dp * 2 + (lane >> 4)));
+            mma_rows8<VT>(o[2 * dp], h0, h1, b[0], b[1]);
+            mma_rows8<VT>(o[2 * dp], l0, l1, b[0], b[1]);
+            mma_rows8<VT>(o[2 * dp + 1], h0, h1, b[2], b[3]);
+            mma_rows8<VT>(o[2 * dp + 1], l0, l1, b[2], b[3]);
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&c->empty[st]);         // this warp's reads of the stage are done
+
+      // ---- four-way merge
+      if (g < a.T) {
+#pragma unroll
+        for (int d = 0; d < 8; ++d)
+          *reinterpret_cast<float2*>(merge + (gw * kMaxT + g) * 64 + d * 8 + cpair) = make_float2(o[d][0], o[d][1]);
+        if ((lane & 3) == 0) {
+          c->m[cg][gw][g] = m;
+          c->l[cg][gw][g] = l;
+        }
+      }
+      named_bar_sync(1 + cg, kGroupWarps * 32);
+      for (int i = gt; i < a.T * 64; i += kGroupWarps * 32) {
+        const int t = i >> 6, d = i & 63;
+        float mx = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < kGroupWarps; ++w) mx = fmaxf(mx, c->m[cg][w][t]);
+        float num = 0.f, den = 0.f;
+#pragma unroll
+        for (int w = 0; w < kGroupWarps; ++w) {
+          const float f = ex2_approx(c->m[cg][w][t] - mx);            // 0 for a warp that saw no row
+          num = fmaf(f, merge[(w * kMaxT + t) * 64 + d], num);
+          den = fmaf(f, c->l[cg][w][t], den);
+        }
+        const size_t at = new0 + static_cast<size_t>(t) * 512 + d;
+        const float y = num / den;
+        if constexpr (std::is_same<OT, float>::value) static_cast<float*>(a.out)[at] = y;
+        else if constexpr (std::is_same<OT, __half>::value) static_cast<__half*>(a.out)[at] = __float2half_rn(y);
+        else static_cast<__nv_bfloat16*>(a.out)[at] = __float2bfloat16_rn(y);
+      }
+      named_bar_sync(1 + cg, kGroupWarps * 32);          // the merge buffer and the new rows' tiles are free again
+    }
+  }
+  __syncthreads();
+  if (ctl->abort) __nanosleep(20000);
+}
+
+int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k, void* ring_v, void* out, int S, int T,
+                       int past, int slots, int window, float scale, int value_is_fp16, int out_dtype, int* status,
+                       cudaStream_t st, int dependent) {
+  using namespace stream;
+  if (S <= 0 || T <= 0) return (S == 0 || T == 0) ? 0 : -1;
+  if (past < 0 || window <= 0 || slots < window || slots > 256 || T > kMaxT || S > (1 << 19)) return -1;
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
+       reinterpret_cast<uintptr_t>(ring_k) | reinterpret_cast<uintptr_t>(ring_v) | reinterpret_cast<uintptr_t>(out)) & 15u)
+    return -3;
+  const int delta = past < window - 1 ? past : window - 1;
+  const int n_loaded = past < slots ? past : slots;
+  CUtensorMap tk = {}, tv = {};
+  if (n_loaded > 0) {
+    int rc = encode_rows_16bit(&tk, ring_k, static_cast<uint64_t>(S) * 8 * slots, 64, static_cast<uint32_t>(n_loaded), 64);
+    if (rc == 0) rc = encode_rows_16bit(&tv, ring_v, static_cast<uint64_t>(S) * 8 * slots, 64, static_cast<uint32_t>(n_loaded), 64);
+    if (rc != 0) return rc;
+  }
+  const int n_items = S * 8, sms = sm_count();
+  int stages = (n_items + sms - 1) / sms;               // one item per block: one stage, and room for other blocks
+  if (stages > kMaxStages) stages = kMaxStages;
+  StreamArgs a = {static_cast<const uint16_t*>(q), static_cast<const uint16_t*>(k), static_cast<const uint16_t*>(v),
+                  static_cast<uint16_t*>(ring_k), static_cast<uint16_t*>(ring_v), out, n_items, T, past, delta, slots, window,
+                  n_loaded, stages, scale * 1.4426950408889634f};
+  using Kern = void (*)(CUtensorMap, CUtensorMap, StreamArgs, int*);
+  Kern kern;
+  if (value_is_fp16) kern = out_dtype == 2 ? stream_attn_kernel<__half, float> : stream_attn_kernel<__half, __half>;
+  else kern = out_dtype == 2 ? stream_attn_kernel<__nv_bfloat16, float> : stream_attn_kernel<__nv_bfloat16, __nv_bfloat16>;
+  const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes(stages));
+  if (rc != 0) return rc;
+  return launch_kernel(kern, dim3(n_items < sms ? n_items : sms), kThreads, smem_bytes(stages), st, 1, dependent, tk, tv, a, status);
+}
+
+}  // namespace fm

@@ -5,8 +5,8 @@
 (``self_attn``, ``mlp.fc1``, ``mlp.fc2``, ``input_layernorm``, ``post_attention_layernorm``,
 ``self_attn_layer_scale.scale``, ``mlp_layer_scale.scale``), so state dicts are interchangeable.
 
-The whole layer runs on this package's kernels, six launches for a call without cache on clips of 129-256 frames
-(seven for other lengths, where projection + RoPE and the attention are two kernels):
+The whole layer runs on this package's kernels, behind one native call (``ops.layer_forward``) that issues them as a
+chain of dependent launches:
 
     LayerNorm -> QKV projection + RoPE + banded attention -> o_proj + layer scale + residual
               -> LayerNorm -> fc1 + GELU -> fc2 + layer scale + residual
@@ -22,8 +22,9 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from . import ops
+from . import _native, ops
 from .attention import MimiAttentionB200
+from .kv_ring import MimiKVRing
 
 
 class _LayerScale(nn.Module):
@@ -64,6 +65,29 @@ class _Cast16:
         return hit[1]
 
 
+class _LayerPlan:
+    """What one native layer call needs besides its activations: the 16-bit weights, FP32 LayerNorm parameters and layer
+    scales, and the struct that points at them."""
+
+    def __init__(self, layer: "MimiTransformerLayerB200", x: torch.Tensor, ps: tuple, key: list) -> None:
+        attn = layer.self_attn
+        ops._need(x.dtype in ops._OUT_CODES, "x must be bfloat16, float16 or float32")
+        ffn = ps[9].shape[0]
+        ops._need(tuple(ps[9].shape) == (ffn, 512) and tuple(ps[10].shape) == (512, ffn) and ffn % 256 == 0,
+                  "the MLP must be 512 -> n -> 512 with n a multiple of 256")
+        tc = attn._tc_input_dtype(x)
+        f32 = lambda p: p.detach().float().contiguous()       # no copy for FP32 parameters
+        self.key = key
+        self.keep = (f32(ps[0]), f32(ps[1]), attn.packed_qkv_weight(tc), attn.out_weight(attn.value_dtype), f32(ps[6]),
+                     f32(ps[7]), f32(ps[8]), layer._cast.get("fc1", ps[9], tc), layer._cast.get("fc2", ps[10], tc), f32(ps[11]))
+        for t in self.keep:
+            ops._need(t.is_cuda, "the layer's parameters must be on a CUDA device")
+        self.params = _native.LayerParams(*(t.data_ptr() for t in self.keep), layer.input_layernorm.eps,
+                                          layer.post_attention_layernorm.eps, attn.scaling, attn.sliding_window,
+                                          ops._OUT_CODES[x.dtype],
+                                          ops._VALUE_CODES[attn.value_dtype] | (2 if tc == torch.float16 else 0), ffn)
+
+
 class MimiTransformerLayerB200(nn.Module):
     def __init__(self, hidden_size: int = 512, intermediate_size: int = 2048, num_heads: int = 8, head_dim: int = 64,
                  sliding_window: int = 250, layer_idx: int = 0, norm_eps: float = 1e-5,
@@ -76,6 +100,7 @@ class MimiTransformerLayerB200(nn.Module):
         self.self_attn_layer_scale = _LayerScale(hidden_size, layer_scale_initial_scale)
         self.mlp_layer_scale = _LayerScale(hidden_size, layer_scale_initial_scale)
         self._cast = _Cast16()
+        self._plan: _LayerPlan | None = None
 
     @classmethod
     def from_reference(cls, layer: nn.Module, value_dtype: torch.dtype = torch.float16) -> "MimiTransformerLayerB200":
@@ -92,6 +117,38 @@ class MimiTransformerLayerB200(nn.Module):
         new.mlp_layer_scale = layer.mlp_layer_scale
         return new
 
+    def _parameters_in_use(self) -> tuple:
+        """The layer's parameters, looked up in the modules' own tables (an attribute access per level costs more host
+        time than a launch)."""
+        m = self._modules
+        try:
+            a, mlp = m["self_attn"]._modules, m["mlp"]._modules
+            ln1, ln2 = m["input_layernorm"]._parameters, m["post_attention_layernorm"]._parameters
+            return (ln1["weight"], ln1["bias"], a["q_proj"]._parameters["weight"], a["k_proj"]._parameters["weight"],
+                    a["v_proj"]._parameters["weight"], a["o_proj"]._parameters["weight"],
+                    m["self_attn_layer_scale"]._parameters["scale"], ln2["weight"], ln2["bias"],
+                    mlp["fc1"]._parameters["weight"], mlp["fc2"]._parameters["weight"], m["mlp_layer_scale"]._parameters["scale"])
+        except KeyError:         # a parameter that is computed (parametrised weights and the like)
+            at, ln1, ln2 = self.self_attn, self.input_layernorm, self.post_attention_layernorm
+            return (ln1.weight, ln1.bias, at.q_proj.weight, at.k_proj.weight, at.v_proj.weight, at.o_proj.weight,
+                    self.self_attn_layer_scale.scale, ln2.weight, ln2.bias, self.mlp.fc1.weight, self.mlp.fc2.weight,
+                    self.mlp_layer_scale.scale)
+
+    def _native_plan(self, x: torch.Tensor) -> "_LayerPlan":
+        """The parameter block of the native call for activations like ``x``; rebuilt when a parameter was replaced or
+        written to, or when an option it depends on changed."""
+        attn = self.self_attn
+        ps = self._parameters_in_use()
+        key = [x.dtype, x.device, attn.sliding_window, attn.scaling, attn.value_dtype, attn.input_dtype,
+               self.input_layernorm.eps, self.post_attention_layernorm.eps]
+        for p in ps:
+            key.append(p.data_ptr())
+            key.append(p._version)
+        plan = self._plan
+        if plan is None or plan.key != key:
+            plan = self._plan = _LayerPlan(self, x, ps, key)
+        return plan
+
     def forward(self, hidden_states: torch.Tensor, attention_mask: torch.Tensor | None, past_key_values,
                 position_embeddings: tuple[torch.Tensor, torch.Tensor], output_attentions: bool = False,
                 canonical_window_mask: bool = False) -> tuple[torch.Tensor, torch.Tensor | None]:
@@ -105,19 +162,30 @@ class MimiTransformerLayerB200(nn.Module):
             raise RuntimeError("the fused layer expects bias-free projections, as in Mimi's checkpoints")
         attn = self.self_attn
         x = hidden_states.contiguous()
+        cache = past_key_values
+        if cache is None or isinstance(cache, MimiKVRing):
+            cos, sin = position_embeddings
+            if cos.dtype != torch.float32 or sin.dtype != torch.float32:
+                cos, sin = cos.to(torch.float32), sin.to(torch.float32)
+            plan = self._native_plan(x)
+            window, ring, past = attn.sliding_window, None, 0
+            if cache is not None:
+                ops._need(cache.num_streams == x.shape[0], "cache was created for a different number of streams")
+                ops._need(cache.sliding_window == window, "cache window differs from the module's")
+                ring, past = cache.layer_rings(attn.layer_idx), cache.get_seq_length(attn.layer_idx)
+            out = ops.layer_forward(plan.params, x, cos.contiguous(), sin.contiguous(), value_dtype=attn.value_dtype, ring=ring,
+                                    past=past, window=window)
+            if cache is not None:
+                cache.advance(attn.layer_idx, x.shape[1])
+            return out, None
+        # a cache object of another kind: the kernels one by one around its own update
         stream_dtype = x.dtype
         tc = attn._tc_input_dtype(x)
         cos, sin = (t.to(torch.float32).contiguous() for t in position_embeddings)
         ln1, ln2 = self.input_layernorm, self.post_attention_layernorm
         f32 = lambda p: p.detach().float().contiguous()       # no copy for FP32 parameters
         h = ops.layer_norm(x, f32(ln1.weight), f32(ln1.bias), eps=ln1.eps, out_dtype=tc)
-        if past_key_values is None:
-            core = ops.attention_prefill(h, attn.packed_qkv_weight(tc), cos, sin, window=attn.sliding_window,
-                                         scale=attn.scaling, value_dtype=attn.value_dtype)
-        else:
-            core = attn._forward_tc(h, past_key_values, cos, sin)      # ring decode (FP32 result) or chunk path
-            if core.dtype not in ops._VALUE_CODES:
-                core = core.to(attn.value_dtype)
+        core = attn._forward_tc(h, past_key_values, cos, sin)
         x1 = ops.linear(core, attn.out_weight(core.dtype), scale=f32(self.self_attn_layer_scale.scale), residual=x,
                         out_dtype=stream_dtype)
         h2 = ops.layer_norm(x1, f32(ln2.weight), f32(ln2.bias), eps=ln2.eps, out_dtype=tc)

@@ -15,7 +15,8 @@ _VALUE_CODES = {torch.bfloat16: 0, torch.float16: 1}
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device (the raw handle, without building a ``torch.cuda.Stream``)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _need(cond: bool, msg: str) -> None:
@@ -64,6 +65,9 @@ def default_status(device) -> torch.Tensor:
     """The per-device status word used when a call does not pass its own.  Once a kernel has recorded
     a bounded-wait timeout in it, later kernels given the same word return at once; check it with
     ``read_status(default_status(dev))`` and clear it with ``.zero_()``."""
+    st = _default_status.get(device)
+    if st is not None:
+        return st
     dev = torch.device(device)
     if dev.index is None:
         dev = torch.device("cuda", torch.cuda.current_device())
@@ -191,6 +195,35 @@ def linear(a, w, *, scale=None, residual=None, activation=None, out_dtype=None, 
                            1 if a.dtype == torch.float16 else 0, _OUT_CODES[out_dtype],
                            1 if activation == "gelu" else 0, _status_ptr(status, a), _stream())
     _native.check(rc, "fm_linear_f16")
+    return out
+
+
+def layer_forward(params, x, cos, sin, *, value_dtype, ring=None, past=0, window=250, out=None, status=None):
+    """One whole transformer layer in a single native call.  ``params``: a filled ``_native.LayerParams``; ``x [B,T,512]``
+    in the residual stream's type, ``cos, sin [1 or B, T, 64]``; ``ring``: ``None`` or this layer's ``(ring_k, ring_v)``
+    with ``past`` frames seen.  The intermediate tensors live in one workspace."""
+    B, T, C = x.shape
+    _need(x.is_cuda and x.is_contiguous() and C == HIDDEN and x.dtype in _OUT_CODES, "x must be contiguous CUDA [B, T, 512]")
+    bstride = _check_tables(cos, sin, B, T)
+    rows = B * T
+    size = rows * (2048 + HIDDEN * x.element_size() + max(2 * params.ffn, 3072)) + 4096
+    ring_k = ring_v = None
+    slots = 0
+    if ring is not None:
+        k, v = ring
+        _need(k.is_cuda and k.dtype == torch.bfloat16 and k.is_contiguous() and k.dim() == 4 and k.shape[0] == B
+              and k.shape[1] == HEADS and k.shape[3] == HEAD_DIM, "ring_k must be contiguous bf16 [B, 8, slots, 64]")
+        _need(v.is_cuda and v.dtype == value_dtype and v.is_contiguous() and v.shape == k.shape, "ring_v must match ring_k")
+        slots = k.shape[2]
+        ring_k, ring_v = k.data_ptr(), v.data_ptr()
+        size += 2048 * B * (min(past, window - 1) + T)
+    workspace = torch.empty(size, dtype=torch.uint8, device=x.device)
+    if out is None:
+        out = torch.empty_like(x)
+    rc = _native.load().fm_layer_forward(params, x.data_ptr(), out.data_ptr(), workspace.data_ptr(), size, cos.data_ptr(),
+                                         sin.data_ptr(), bstride, B, T, ring_k, ring_v, past, slots,
+                                         _status_ptr(status, x), _stream())
+    _native.check(rc, "fm_layer_forward")
     return out
 
 

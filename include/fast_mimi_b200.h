@@ -28,6 +28,43 @@ extern "C" {
 
 int fm_abi_version(void);
 
+/* One whole transformer layer of Mimi (512 channels, MLP of `ffn`, a multiple of 256) as one call: LayerNorm, projections with RoPE, banded
+ * attention, output projection, LayerNorm, MLP, layer scales and residual adds; the reference's
+ * MimiTransformerLayer.forward (src/fast_mimi/model.py:2026-2061).
+ *   params      host struct of device pointers; matrices are row-major [out, in] and 16 bit: w_qkv, w_fc1, w_fc2 in
+ *               BF16 / FP16 by bit 1 of value_dtype, w_o in the value type (bit 0); LayerNorm parameters and layer
+ *               scales FP32 (the scales may be NULL)
+ *   x, y        [B, T, 512] in stream_dtype (0 BF16, 1 FP16, 2 FP32), y != x
+ *   workspace   256-byte aligned device memory, at least  B*T*(2048 + 512*elem + max(2*ffn, 3072)) + 2*1024*B*(min(past, window-1) + T)
+ *               + 4096 bytes (elem: bytes per value of x; the second term for cached calls only); -7 if too small
+ *   ring_k/v    NULL for a call without cache; else this layer's ring [B, 8, ring_slots, 64] (K BF16, V value type) with
+ *               `past` frames seen: the T new frames attend to it and to themselves, then enter it
+ *   cos, sin    [1 or B, T, 64] FP32 of the new frames' positions
+ * The launches form a chain of programmatically dependent kernels on `stream`. */
+typedef struct fm_layer_params {
+  const float* ln1_weight;
+  const float* ln1_bias;
+  const void* w_qkv;
+  const void* w_o;
+  const float* attn_scale;
+  const float* ln2_weight;
+  const float* ln2_bias;
+  const void* w_fc1;
+  const void* w_fc2;
+  const float* mlp_scale;
+  float ln1_eps;
+  float ln2_eps;
+  float scale;
+  int window;
+  int stream_dtype;
+  int value_dtype;
+  int ffn;
+} fm_layer_params;
+
+int fm_layer_forward(const fm_layer_params* params, const void* x, void* y, void* workspace, long long workspace_bytes,
+                     const float* cos, const float* sin, long long cos_bstride, int B, int T, void* ring_k, void* ring_v,
+                     int past, int ring_slots, int* status, void* stream);
+
 /* Self-test of the bounded device waits every kernel of this library uses (no counterpart in the reference, whose
  * kernels do not wait on one another): a one-thread kernel waits, with a limit of limit_us microseconds (at most
  * 100 000), on a barrier that nothing arrives on.  The wait gives up, code 103 lands in *status and the kernel

@@ -1,0 +1,93 @@
+"""The kernels that calls with few rows take: the split-K linear and projection (128 x 64 tiles, K shared out over a
+cluster), the streaming attention that reads and updates the ring in one pass, and the layer entry point that chains
+them, vs plain FP32 products and the CPU oracle."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from oracle import mimi_attention_oracle as O
+from test_gpu_layer_blocks import ROUND, _layer_params
+
+pytestmark = pytest.mark.gpu
+
+
+# rows: one, either side of a tile's edge, two tiles; shapes: every split (8, 4, 2, 1 blocks per cluster) that K and the
+# number of tiles lead to, a K that only divides by two, the first size past the rule's edge (two tiles per SM)
+@pytest.mark.parametrize("rows", [1, 127, 128, 129, 256, 1100])
+@pytest.mark.parametrize("shape", [(512, 512), (2048, 512), (512, 2048), (128, 256), (64, 1536)])
+def test_linear_with_few_rows(rows, shape):
+    import fast_mimi_b200 as fm
+    K, N = shape
+    g = torch.Generator(device="cuda").manual_seed(rows * 31 + K)
+    a = torch.randn(rows, K, device="cuda", generator=g).half()
+    w = (torch.randn(N, K, device="cuda", generator=g) / K ** 0.5).half()
+    s = torch.rand(N, device="cuda", generator=g) + 0.2
+    acc = a.double() @ w.double().T
+    for out_dtype in (torch.float32, torch.float16):
+        r = torch.randn(rows, N, device="cuda", generator=g).to(out_dtype)
+        got = fm.ops.linear(a, w, scale=s, residual=r, out_dtype=out_dtype)
+        assert O.rel_l2(got.double(), r.double() + s * acc) < max(ROUND[out_dtype], 2e-5)
+        got = fm.ops.linear(a, w, activation="gelu", out_dtype=out_dtype)
+        assert O.rel_l2(got.double(), torch.nn.functional.gelu(acc)) < max(ROUND[out_dtype], 2e-5)
+    fm.check_status()
+
+
+@pytest.mark.parametrize("B,T", [(1, 1), (1, 127), (3, 43), (2, 128), (5, 100)])
+def test_projection_with_few_rows(B, T):
+    import fast_mimi_b200 as fm
+    g = torch.Generator().manual_seed(B * 1000 + T)
+    x = torch.randn(B, T, 512, generator=g).bfloat16()
+    w = (torch.randn(1536, 512, generator=g) * 0.04).bfloat16()
+    pos = torch.randint(0, 3000, (B, T), generator=g)                      # a table per clip
+    cos, sin = fm.rope_tables(pos)
+    q, k, v = O.qkv_project(x.float(), *w.float().chunk(3, 0))              # [B, 8, T, 64]
+    c, s = cos[:, None], sin[:, None]
+    rot = lambda t: t * c + O.rotate_half(t) * s
+    frames = lambda t: t.transpose(1, 2).reshape(B, T, 512)
+    for value_dtype in (torch.float16, torch.bfloat16):
+        got = fm.ops.qkv_rope(x.cuda(), w.cuda(), cos.cuda(), sin.cuda(), value_dtype=value_dtype)
+        for y, ref, dt in zip(got, (rot(q), rot(k), v), (torch.bfloat16, torch.bfloat16, value_dtype)):
+            assert O.rel_l2(y.float().cpu(), frames(ref)) < ROUND[dt]
+    fm.check_status()
+
+
+@pytest.mark.parametrize("window", [250, 100, 3])
+@pytest.mark.parametrize("streams", [1, 5])
+def test_layer_on_live_streams_matches_the_oracle(streams, window):
+    """A session of calls of 1 .. 7 frames (the streaming kernel), longer ones (the tensor-core path) and one beyond the
+    window, over rings that fill up and wrap; every call against the oracle's layer on its own cache.  Bar as for the
+    layer without a cache: 2e-3 on what the layer adds to its input."""
+    import fast_mimi_b200 as fm
+    p = _layer_params(70 + window)
+    layer = fm.MimiTransformerLayerB200(sliding_window=window).cuda()
+    layer.load_state_dict(p, strict=True)
+    ring, cache = fm.MimiKVRing(1, streams, window), O.KVCacheOracle(window=window)
+    g = torch.Generator().manual_seed(window)
+    past = 0
+    for T in (1, 1, 2, 7, 60, 1, 8, 7, 200, 3, 1, 7, 260, 1, 2):
+        x = torch.randn(streams, T, 512, generator=g)
+        cos, sin = fm.rope_tables(torch.arange(past, past + T)[None])
+        got, _ = layer(x.cuda(), None, ring, (cos.cuda(), sin.cuda()))
+        want = O.transformer_layer(x, p, cache=cache, window=window)
+        assert O.rel_l2(got.cpu() - x, want - x) < 2e-3, (T, past)
+        past += T
+    fm.check_status()
+
+
+def test_layer_follows_its_parameters():
+    """The layer's parameter block is rebuilt when a parameter is written to, replaced, or the options change."""
+    import fast_mimi_b200 as fm
+    layer = fm.MimiTransformerLayerB200().cuda()
+    x = torch.randn(1, 20, 512, device="cuda")
+    cs = fm.rope_tables(torch.arange(20, device="cuda")[None])
+    run = lambda: layer(x, None, None, cs)[0]
+    for p in (_layer_params(1), _layer_params(2)):
+        layer.load_state_dict(p)
+        assert O.rel_l2(run().cpu() - x.cpu(), O.transformer_layer(x.cpu(), p) - x.cpu()) < 2e-3
+    before = run()
+    layer.mlp.fc2 = torch.nn.Linear(2048, 512, bias=False).cuda()
+    assert not torch.equal(run(), before)
+    before = run()
+    layer.self_attn.sliding_window = 4
+    assert not torch.equal(run(), before)
