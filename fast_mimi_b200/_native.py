@@ -7,10 +7,14 @@ call time and there is no fallback: a missing library raises.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import threading
 
-from ._build import LIB_PATH
+import torch  # noqa: F401  (the extension module links against its libraries)
+
+from ._build import BIND_PATH, LIB_PATH
 
 _P, _I, _LL, _F = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
 
@@ -18,7 +22,7 @@ class LayerParams(ctypes.Structure):
     """``fm_layer_params`` of the header."""
     _fields_ = [("ln1_weight", _P), ("ln1_bias", _P), ("w_qkv", _P), ("w_o", _P), ("attn_scale", _P), ("ln2_weight", _P),
                 ("ln2_bias", _P), ("w_fc1", _P), ("w_fc2", _P), ("mlp_scale", _P), ("ln1_eps", _F), ("ln2_eps", _F),
-                ("scale", _F), ("window", _I), ("stream_dtype", _I), ("value_dtype", _I), ("ffn", _I)]
+                ("scale", _F), ("window", _I), ("stream_dtype", _I), ("value_dtype", _I), ("ffn", _I), ("weights_settled", _I)]
 
 
 #: name -> argtypes, in header order.  tests/test_host_logic.py checks this table against the header.
@@ -79,6 +83,25 @@ def load() -> ctypes.CDLL:
                 fn.restype = _I
             _lib = lib
     return _lib
+
+
+_bind = None
+
+
+def bind():
+    """The extension module with the per-call host work (``csrc/bind``), loaded once."""
+    global _bind
+    if _bind is None:
+        load()
+        with _lock:
+            if _bind is None:
+                if not os.path.exists(BIND_PATH):
+                    raise NativeLibraryMissing(f"{BIND_PATH} is missing: build it with `python -m fast_mimi_b200._build`")
+                loader = importlib.machinery.ExtensionFileLoader("_fm_bind", BIND_PATH)
+                module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fm_bind", loader))
+                loader.exec_module(module)
+                _bind = module
+    return _bind
 
 
 def check(rc: int, what: str) -> None:

@@ -64,6 +64,13 @@ int launch_linear_gemm(const void* a, const void* w, void* y, const float* scale
                        int K, int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent = 0);
 // The same two products for few rows (fm_linear_small.cu): 128 x 64 tiles, K split over a cluster.
 bool few_row_tiles(int M, int N);
+// LayerNorm folded into the product behind it (fm_ln_linear.cu), for up to 256 rows: the chain-opening QKV projection and
+// gelu(LayerNorm(x) W^T).
+bool few_rows_with_norm(int M);
+int launch_ln_qkv(const void* x, int x_dtype, const float* weight, const float* bias, float eps, const void* w_qkv,
+                  const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status, cudaStream_t st, int dependent);
+int launch_ln_linear_gelu(const void* x, int x_dtype, const float* weight, const float* bias, float eps, const void* w, void* y,
+                          int M, int N, int tc_fp16, int* status, cudaStream_t st, int dependent);
 int launch_linear_small(const void* a, const void* w, void* y, const float* scale, const void* resid, int M, int N, int K,
                         int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent);
 int launch_qkv_small(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status,

@@ -69,9 +69,13 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
   const int value_fp16 = p.value_dtype & 1;
   const int tc = (p.value_dtype & 2) ? 1 : 0;                    // 16-bit type of the products' operands: 0 BF16, 1 FP16
 
-  int rc = launch_layernorm512(x, p.stream_dtype, p.ln1_weight, p.ln1_bias, p.ln1_eps, b.h, tc, rows, st, 1);
-  if (rc != 0) return rc;
-  if (whole_clip && use_fused_clip(B)) {
+  const bool norm_inside = few_rows_with_norm(rows);
+  int rc = 0;
+  if (!norm_inside) {
+    rc = launch_layernorm512(x, p.stream_dtype, p.ln1_weight, p.ln1_bias, p.ln1_eps, b.h, tc, rows, st, 1);
+    if (rc != 0) return rc;
+  }
+  if (whole_clip && !norm_inside && use_fused_clip(B)) {
     rc = launch_attn_fused_clip(b.h, p.w_qkv, cos, sin, cos_bstride, b.core, B, T, p.window, p.scale, p.value_dtype, status, st, 1);
   } else {
     QkvEpilogueArgs ep = {};
@@ -83,7 +87,11 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
     ep.cos_bstride = cos_bstride;
     ep.T = T;
     ep.ring_slots = 1;
-    rc = launch_qkv_rope_gemm(b.h, p.w_qkv, ep, rows, p.value_dtype, status, st, 1);
+    // The kernel that opens the chain may ask for W_qkv ahead of its wait only if W_qkv cannot be the work of the kernel
+    // in front: not on the first call after the caller has (re)made it.
+    rc = norm_inside ? launch_ln_qkv(x, p.stream_dtype, p.ln1_weight, p.ln1_bias, p.ln1_eps, p.w_qkv, ep, rows, p.value_dtype,
+                                     status, st, p.weights_settled)
+                     : launch_qkv_rope_gemm(b.h, p.w_qkv, ep, rows, p.value_dtype, status, st, 1);
     if (rc != 0) return rc;
     if (!cached) {
       rc = launch_band_attn_prefill(b.q, b.k, b.v, b.core, B, T, p.window, p.scale, value_fp16, status, st, 1);
@@ -105,9 +113,14 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
   if (rc != 0) return rc;
   rc = launch_linear_gemm(b.core, p.w_o, b.x1, p.attn_scale, x, rows, 512, 512, value_fp16, p.stream_dtype, 0, status, st, 1);
   if (rc != 0) return rc;
-  rc = launch_layernorm512(b.x1, p.stream_dtype, p.ln2_weight, p.ln2_bias, p.ln2_eps, b.h, tc, rows, st, 1);
-  if (rc != 0) return rc;
-  rc = launch_linear_gemm(b.h, p.w_fc1, b.g, nullptr, nullptr, rows, p.ffn, 512, tc, tc, 1, status, st, 1);
+  if (norm_inside) {
+    rc = launch_ln_linear_gelu(b.x1, p.stream_dtype, p.ln2_weight, p.ln2_bias, p.ln2_eps, p.w_fc1, b.g, rows, p.ffn, tc, status,
+                               st, 1);
+  } else {
+    rc = launch_layernorm512(b.x1, p.stream_dtype, p.ln2_weight, p.ln2_bias, p.ln2_eps, b.h, tc, rows, st, 1);
+    if (rc != 0) return rc;
+    rc = launch_linear_gemm(b.h, p.w_fc1, b.g, nullptr, nullptr, rows, p.ffn, 512, tc, tc, 1, status, st, 1);
+  }
   if (rc != 0) return rc;
   return launch_linear_gemm(b.g, p.w_fc2, y, p.mlp_scale, b.x1, rows, 512, p.ffn, tc, p.stream_dtype, 0, status, st, 1);
 }

@@ -16,11 +16,8 @@
 // overlap possible.
 //
 // Warps 0-3: accumulator rows out of tensor memory.  Warp 4: TMA.  Warp 5: MMA.  All six finish the owned rows.
-#include <type_traits>
-
-#include "fm_common.cuh"
-#include "fm_kernels.h"
 #include "fm_launch.h"
+#include "fm_small_tile.cuh"
 
 namespace fm {
 
@@ -51,20 +48,7 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 __device__ __forceinline__ void st_cluster_v4(uint32_t addr, float a, float b, float c, float d) {
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
-// 16-byte piece `c` (0..15) of row `r` of the reduction buffer; the low three bits are permuted by the row so that
-// eight lanes with consecutive rows (writing) or consecutive pieces (reading) touch eight different bank groups.
-__device__ __forceinline__ uint32_t red_offset(uint32_t r, uint32_t c) { return r * 256u + ((c ^ (r & 7u)) << 4); }
 }  // namespace small
-
-struct SmallArgs {
-  const float* scale;     // [N] or null
-  const void* resid;      // [M, N] in the output's type or null
-  void* y;                // [M, N]
-  int M, N, chunks;       // chunks: K / 64 / S, this block's share
-  int split;              // S, blocks per cluster
-  int gelu;
-  QkvEpilogueArgs qkv;    // kOut 3
-};
 
 // kOut: 0 = BF16, 1 = FP16, 2 = FP32 output and residual; 3 = q | k | v with RoPE (VT: type of v)
 template <int kOut, typename VT>
@@ -143,13 +127,21 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
     if (one) tc_commit(&bars->acc_full);
     __syncwarp();
-  } else {
+  }
+  griddep_wait();                          // residual and outputs belong to the chain
+  // The rows this block owns: rank, rank + S, ... of the tile; eight threads per row, columns 4j.. and 32 + 4j...
+  const int log_s = 31 - __clz(split);
+  const int valid = args.M - m0 < kBlockM ? args.M - m0 : kBlockM;
+  const int n_items = skip ? 0 : ((valid - rank + split - 1) >> log_s) * 8;
+  auto item_row = [&](int item) { return m0 + ((item >> 3) << log_s) + rank; };
+  PieceOperands ops;
+  int item = static_cast<int>(threadIdx.x);
+  if (item < n_items) load_operands<kOut>(args, item_row(item), ntile, item & 7, ops);
+  if (warp < 4) {
     mbar_wait(&bars->acc_full, 0, ctl, status, kErrWaitMma);
     tc_fence_after_sync();
   }
-  griddep_wait();                          // residual and outputs belong to the chain
   if (split > 1) cluster_wait();           // every block of the cluster runs
-  const int log_s = 31 - __clz(split);
   if (warp < 4) {
     const int row = warp * 32 + lane;
     const int owner = row & (split - 1), slot = rank * (kBlockM >> log_s) + (row >> log_s);
@@ -177,12 +169,8 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     __syncthreads();
   }
 
-  // The rows this block owns: rank, rank + S, ... of the tile; eight threads per row, columns 4j.. and 32 + 4j...
-  const int valid = args.M - m0 < kBlockM ? args.M - m0 : kBlockM;
-  const int n_own = skip ? 0 : (valid - rank + split - 1) >> log_s;
-  for (int item = static_cast<int>(threadIdx.x); item < n_own * 8; item += kThreads) {
+  for (; item < n_items; item += kThreads) {
     const int local = item >> 3, j = item & 7;
-    const long long row = m0 + (local << log_s) + rank;
     float lo[4] = {0.f, 0.f, 0.f, 0.f}, hi[4] = {0.f, 0.f, 0.f, 0.f};
     for (int s = 0; s < split; ++s) {
       const uint32_t r = s * (kBlockM >> log_s) + local;
@@ -191,76 +179,9 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       lo[0] += a.x; lo[1] += a.y; lo[2] += a.z; lo[3] += a.w;
       hi[0] += b.x; hi[1] += b.y; hi[2] += b.z; hi[3] += b.w;
     }
-    if constexpr (kOut == 3) {
-      const QkvEpilogueArgs& ep = args.qkv;
-      const int seg = ntile >> 3, head = ntile & 7;
-      const int clip = static_cast<int>(row / ep.T), t = static_cast<int>(row % ep.T);
-      uint2 plo, phi;
-      if (seg < 2) {
-        const long long at = clip * ep.cos_bstride + static_cast<long long>(t) * 64 + 4 * j;
-        const float4 c4 = *reinterpret_cast<const float4*>(ep.cos + at), s4 = *reinterpret_cast<const float4*>(ep.sin + at);
-        const float c[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
-        float o_lo[4], o_hi[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          o_lo[e] = lo[e] * c[e] - hi[e] * sn[e];
-          o_hi[e] = hi[e] * c[e] + lo[e] * sn[e];
-        }
-        plo = make_uint2(Pack16<__nv_bfloat16>::pack(o_lo[0], o_lo[1]), Pack16<__nv_bfloat16>::pack(o_lo[2], o_lo[3]));
-        phi = make_uint2(Pack16<__nv_bfloat16>::pack(o_hi[0], o_hi[1]), Pack16<__nv_bfloat16>::pack(o_hi[2], o_hi[3]));
-      } else {
-        plo = make_uint2(Pack16<VT>::pack(lo[0], lo[1]), Pack16<VT>::pack(lo[2], lo[3]));
-        phi = make_uint2(Pack16<VT>::pack(hi[0], hi[1]), Pack16<VT>::pack(hi[2], hi[3]));
-      }
-      uint16_t* lin = seg == 0 ? ep.q : (seg == 1 ? ep.k : ep.v);
-      if (lin != nullptr) {
-        uint16_t* dst = lin + row * 512 + head * 64 + 4 * j;
-        *reinterpret_cast<uint2*>(dst) = plo;
-        *reinterpret_cast<uint2*>(dst + 32) = phi;
-      }
-      uint16_t* ring = seg == 1 ? ep.ring_k : (seg == 2 ? ep.ring_v : nullptr);
-      if (ring != nullptr) {
-        const int pos = ep.pos_base + (ep.clip_pos != nullptr ? ep.clip_pos[clip] : 0) + t;
-        if (pos < 0) {                     // would index another stream's ring: recorded, not written
-          if (status != nullptr) atomicMax(status, static_cast<int>(kErrBounds));
-        } else if (t >= ep.T - ep.ring_slots) {
-          uint16_t* dst = ring + ((static_cast<long long>(clip) * 8 + head) * ep.ring_slots + pos % ep.ring_slots) * 64 + 4 * j;
-          *reinterpret_cast<uint2*>(dst) = plo;
-          *reinterpret_cast<uint2*>(dst + 32) = phi;
-        }
-      }
-    } else {
-      const long long at = row * args.N + n0 + 4 * j;
-      float* part[2] = {lo, hi};
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float* v = part[h];
-        if (args.gelu) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) v[e] = gelu_erf(v[e]);
-        }
-        if (args.scale != nullptr) {
-          const float4 s = __ldg(reinterpret_cast<const float4*>(args.scale + n0 + 32 * h + 4 * j));
-          v[0] *= s.x; v[1] *= s.y; v[2] *= s.z; v[3] *= s.w;
-        }
-        if constexpr (kOut == 2) {
-          if (args.resid != nullptr) {
-            const float4 r = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(args.resid) + at + 32 * h));
-            v[0] += r.x; v[1] += r.y; v[2] += r.z; v[3] += r.w;
-          }
-          *reinterpret_cast<float4*>(static_cast<float*>(args.y) + at + 32 * h) = make_float4(v[0], v[1], v[2], v[3]);
-        } else {
-          using T16 = typename std::conditional<kOut == 1, __half, __nv_bfloat16>::type;
-          if (args.resid != nullptr) {
-            const uint2 r = __ldcg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(args.resid) + at + 32 * h));
-            const float2 a = Pack16<T16>::unpack(r.x), b = Pack16<T16>::unpack(r.y);
-            v[0] += a.x; v[1] += a.y; v[2] += b.x; v[3] += b.y;
-          }
-          *reinterpret_cast<uint2*>(static_cast<uint16_t*>(args.y) + at + 32 * h) =
-              make_uint2(Pack16<T16>::pack(v[0], v[1]), Pack16<T16>::pack(v[2], v[3]));
-        }
-      }
-    }
+    const PieceOperands now = ops;
+    if (item + kThreads < n_items) load_operands<kOut>(args, item_row(item + kThreads), ntile, (item + kThreads) & 7, ops);
+    finish_piece<kOut, VT>(args, lo, hi, now, item_row(item), ntile, j, status);
   }
 
   __syncthreads();

@@ -1,0 +1,135 @@
+// What the few-row product kernels share (fm_linear_small.cu, fm_ln_linear.cu): arguments, the layout of an FP32 tile of
+// 64 columns in shared memory, and the epilogue of one piece of a finished row.
+#pragma once
+
+#include <type_traits>
+
+#include "fm_common.cuh"
+#include "fm_kernels.h"
+
+namespace fm {
+
+namespace small {
+// 16-byte piece `c` (0..15) of row `r` of the reduction buffer; the low three bits are permuted by the row so that
+// eight lanes with consecutive rows (writing) or consecutive pieces (reading) touch eight different bank groups.
+__device__ __forceinline__ uint32_t red_offset(uint32_t r, uint32_t c) { return r * 256u + ((c ^ (r & 7u)) << 4); }
+}  // namespace small
+
+struct SmallArgs {
+  const float* scale;     // [N] or null
+  const void* resid;      // [M, N] in the output's type or null
+  void* y;                // [M, N]
+  int M, N, chunks;       // chunks: K / 64 / S, this block's share
+  int split;              // S, blocks per cluster
+  int gelu;
+  QkvEpilogueArgs qkv;    // kOut 3
+};
+
+// What the epilogue of eight values of row `row` of output tile `ntile` (64 columns, one attention head) reads besides the
+// product: columns 4j .. 4j + 3 ([0]) and 32 + 4j .. ([1]), the two halves of RoPE pairs.  Asked for before the product
+// is complete, so that its latency does not follow the reduction's.
+// kOut: 0 = BF16, 1 = FP16, 2 = FP32 output and residual; 3 = q | k | v with RoPE.
+struct PieceOperands {
+  float4 a[2];            // residual, or cos and sin
+  float4 s[2];            // per-channel scale
+};
+
+template <int kOut>
+__device__ __forceinline__ void load_operands(const SmallArgs& args, int row, int ntile, int j, PieceOperands& p) {
+  if constexpr (kOut == 3) {
+    if (ntile < 16) {     // q and k
+      const QkvEpilogueArgs& ep = args.qkv;
+      const int clip = row / ep.T, t = row - clip * ep.T;
+      const long long at = clip * ep.cos_bstride + static_cast<long long>(t) * 64 + 4 * j;
+      p.a[0] = *reinterpret_cast<const float4*>(ep.cos + at);
+      p.a[1] = *reinterpret_cast<const float4*>(ep.sin + at);
+    }
+  } else {
+    const int col = ntile * 64 + 4 * j;
+    const long long at = static_cast<long long>(row) * args.N + col;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      p.s[h] = args.scale != nullptr ? __ldg(reinterpret_cast<const float4*>(args.scale + col + 32 * h)) : make_float4(1.f, 1.f, 1.f, 1.f);
+      p.a[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (args.resid != nullptr) {
+        if constexpr (kOut == 2) {
+          p.a[h] = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(args.resid) + at + 32 * h));
+        } else {
+          using T16 = typename std::conditional<kOut == 1, __half, __nv_bfloat16>::type;
+          const uint2 r = __ldcg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(args.resid) + at + 32 * h));
+          const float2 x = Pack16<T16>::unpack(r.x), y = Pack16<T16>::unpack(r.y);
+          p.a[h] = make_float4(x.x, x.y, y.x, y.y);
+        }
+      }
+    }
+  }
+}
+
+// The epilogue itself: lo and hi are the product's columns 4j .. and 32 + 4j ..
+template <int kOut, typename VT>
+__device__ __forceinline__ void finish_piece(const SmallArgs& args, float (&lo)[4], float (&hi)[4], const PieceOperands& p,
+                                             int row, int ntile, int j, int* status) {
+  if constexpr (kOut == 3) {
+    const QkvEpilogueArgs& ep = args.qkv;
+    const int seg = ntile >> 3, head = ntile & 7;
+    uint2 plo, phi;
+    if (seg < 2) {
+      const float c[4] = {p.a[0].x, p.a[0].y, p.a[0].z, p.a[0].w}, sn[4] = {p.a[1].x, p.a[1].y, p.a[1].z, p.a[1].w};
+      float o_lo[4], o_hi[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        o_lo[e] = lo[e] * c[e] - hi[e] * sn[e];
+        o_hi[e] = hi[e] * c[e] + lo[e] * sn[e];
+      }
+      plo = make_uint2(Pack16<__nv_bfloat16>::pack(o_lo[0], o_lo[1]), Pack16<__nv_bfloat16>::pack(o_lo[2], o_lo[3]));
+      phi = make_uint2(Pack16<__nv_bfloat16>::pack(o_hi[0], o_hi[1]), Pack16<__nv_bfloat16>::pack(o_hi[2], o_hi[3]));
+    } else {
+      plo = make_uint2(Pack16<VT>::pack(lo[0], lo[1]), Pack16<VT>::pack(lo[2], lo[3]));
+      phi = make_uint2(Pack16<VT>::pack(hi[0], hi[1]), Pack16<VT>::pack(hi[2], hi[3]));
+    }
+    uint16_t* lin = seg == 0 ? ep.q : (seg == 1 ? ep.k : ep.v);
+    if (lin != nullptr) {
+      uint16_t* dst = lin + static_cast<long long>(row) * 512 + head * 64 + 4 * j;
+      *reinterpret_cast<uint2*>(dst) = plo;
+      *reinterpret_cast<uint2*>(dst + 32) = phi;
+    }
+    uint16_t* ring = seg == 1 ? ep.ring_k : (seg == 2 ? ep.ring_v : nullptr);
+    if (ring != nullptr) {
+      const int clip = row / ep.T, t = row - clip * ep.T;
+      const int pos = ep.pos_base + (ep.clip_pos != nullptr ? ep.clip_pos[clip] : 0) + t;
+      if (pos < 0) {                     // would index another stream's ring: recorded, not written
+        if (status != nullptr) atomicMax(status, static_cast<int>(kErrBounds));
+      } else if (t >= ep.T - ep.ring_slots) {
+        uint16_t* dst = ring + ((static_cast<long long>(clip) * 8 + head) * ep.ring_slots + pos % ep.ring_slots) * 64 + 4 * j;
+        *reinterpret_cast<uint2*>(dst) = plo;
+        *reinterpret_cast<uint2*>(dst + 32) = phi;
+      }
+    }
+  } else {
+    const long long at = static_cast<long long>(row) * args.N + ntile * 64 + 4 * j;
+    float* part[2] = {lo, hi};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float* v = part[h];
+      if (args.gelu) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = gelu_erf(v[e]);
+      }
+      if (args.scale != nullptr) {
+        v[0] *= p.s[h].x; v[1] *= p.s[h].y; v[2] *= p.s[h].z; v[3] *= p.s[h].w;
+      }
+      if (args.resid != nullptr) {
+        v[0] += p.a[h].x; v[1] += p.a[h].y; v[2] += p.a[h].z; v[3] += p.a[h].w;
+      }
+      if constexpr (kOut == 2) {
+        *reinterpret_cast<float4*>(static_cast<float*>(args.y) + at + 32 * h) = make_float4(v[0], v[1], v[2], v[3]);
+      } else {
+        using T16 = typename std::conditional<kOut == 1, __half, __nv_bfloat16>::type;
+        *reinterpret_cast<uint2*>(static_cast<uint16_t*>(args.y) + at + 32 * h) =
+            make_uint2(Pack16<T16>::pack(v[0], v[1]), Pack16<T16>::pack(v[2], v[3]));
+      }
+    }
+  }
+}
+
+}  // namespace fm

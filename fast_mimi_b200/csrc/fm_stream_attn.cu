@@ -146,34 +146,50 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
     uint8_t* new_v = new_k + kNewBytes / 2;
     float* merge = smem_merge + cg * (kMergeBytes / 4);
     const int first = a.slots > 0 ? (a.past - a.delta) % a.slots : 0;     // slot of the oldest visible row
-    int n = cg;
-    for (long long item = blockIdx.x + static_cast<long long>(cg) * gridDim.x; item < a.n_items;
-         item += static_cast<long long>(kGroups) * gridDim.x, n += kGroups) {
-      const int st = n % a.stages;
-      const int s = static_cast<int>(item >> 3), h = static_cast<int>(item & 7);
-      const size_t new0 = static_cast<size_t>(s) * a.T * 512 + h * 64;
-      // the queries, straight into fragments: 4 K-steps x {columns cpair.., cpair + 8..} of row g
-      uint32_t qa[4][2];
+    // An item's queries, straight into fragments (4 K-steps x {columns cpair.., cpair + 8..} of row g), and for the
+    // group's last warp the new rows (16-byte pieces): asked for one item ahead, so that their latency passes behind the
+    // item in hand.
+    const int n_pieces = a.T * 8;
+    uint32_t q_next[4][2];
+    uint4 k_next[2], v_next[2];
+    auto fetch = [&](long long item) {
+      const size_t new0 = static_cast<size_t>(item >> 3) * a.T * 512 + static_cast<int>(item & 7) * 64;
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
 #pragma unroll
         for (int e = 0; e < 2; ++e)
-          qa[ks][e] = g < a.T ? __ldcg(reinterpret_cast<const uint32_t*>(a.q + new0 + static_cast<size_t>(g) * 512 + ks * 16 + e * 8 + cpair)) : 0u;
+          q_next[ks][e] = g < a.T ? __ldcg(reinterpret_cast<const uint32_t*>(a.q + new0 + static_cast<size_t>(g) * 512 + ks * 16 + e * 8 + cpair)) : 0u;
       }
-      // the new rows: the group's last warp stages them (row = lane / 2.., 16-byte pieces)
-      uint4 nk[2], nv[2];
-      const int n_pieces = a.T * 8;
       if (gw == kGroupWarps - 1) {
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int piece = lane + 32 * e;
           if (piece < n_pieces) {
             const size_t at = new0 + static_cast<size_t>(piece >> 3) * 512 + (piece & 7) * 8;
-            nk[e] = __ldcg(reinterpret_cast<const uint4*>(a.k + at));
-            nv[e] = __ldcg(reinterpret_cast<const uint4*>(a.v + at));
+            k_next[e] = __ldcg(reinterpret_cast<const uint4*>(a.k + at));
+            v_next[e] = __ldcg(reinterpret_cast<const uint4*>(a.v + at));
           }
         }
       }
+    };
+    auto take = [&](uint32_t (&qa)[4][2], uint4 (&nk)[2], uint4 (&nv)[2]) {
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) { qa[ks][0] = q_next[ks][0]; qa[ks][1] = q_next[ks][1]; }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) { nk[e] = k_next[e]; nv[e] = v_next[e]; }
+    };
+    int n = cg;
+    if (blockIdx.x + static_cast<long long>(cg) * gridDim.x < a.n_items) fetch(blockIdx.x + static_cast<long long>(cg) * gridDim.x);
+    for (long long item = blockIdx.x + static_cast<long long>(cg) * gridDim.x; item < a.n_items;
+         item += static_cast<long long>(kGroups) * gridDim.x, n += kGroups) {
+      const int st = n % a.stages;
+      const int s = static_cast<int>(item >> 3), h = static_cast<int>(item & 7);
+      const size_t new0 = static_cast<size_t>(s) * a.T * 512 + h * 64;
+      uint32_t qa[4][2];
+      uint4 nk[2], nv[2];
+      take(qa, nk, nv);
+      if (item + static_cast<long long>(kGroups) * gridDim.x < a.n_items)
+        fetch(item + static_cast<long long>(kGroups) * gridDim.x);
       if (a.n_loaded > 0) mbar_wait(&c->full[st], static_cast<uint32_t>(n / a.stages) & 1u, ctl, status, kErrWaitTma);
       uint8_t* tile_k = smem + st * kStageBytes;
       uint8_t* tile_v = tile_k + kTileBytes;

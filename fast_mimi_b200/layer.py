@@ -18,6 +18,8 @@ several; LayerNorms, projections and the MLP are the same kernels.
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
@@ -65,29 +67,6 @@ class _Cast16:
         return hit[1]
 
 
-class _LayerPlan:
-    """What one native layer call needs besides its activations: the 16-bit weights, FP32 LayerNorm parameters and layer
-    scales, and the struct that points at them."""
-
-    def __init__(self, layer: "MimiTransformerLayerB200", x: torch.Tensor, ps: tuple, key: list) -> None:
-        attn = layer.self_attn
-        ops._need(x.dtype in ops._OUT_CODES, "x must be bfloat16, float16 or float32")
-        ffn = ps[9].shape[0]
-        ops._need(tuple(ps[9].shape) == (ffn, 512) and tuple(ps[10].shape) == (512, ffn) and ffn % 256 == 0,
-                  "the MLP must be 512 -> n -> 512 with n a multiple of 256")
-        tc = attn._tc_input_dtype(x)
-        f32 = lambda p: p.detach().float().contiguous()       # no copy for FP32 parameters
-        self.key = key
-        self.keep = (f32(ps[0]), f32(ps[1]), attn.packed_qkv_weight(tc), attn.out_weight(attn.value_dtype), f32(ps[6]),
-                     f32(ps[7]), f32(ps[8]), layer._cast.get("fc1", ps[9], tc), layer._cast.get("fc2", ps[10], tc), f32(ps[11]))
-        for t in self.keep:
-            ops._need(t.is_cuda, "the layer's parameters must be on a CUDA device")
-        self.params = _native.LayerParams(*(t.data_ptr() for t in self.keep), layer.input_layernorm.eps,
-                                          layer.post_attention_layernorm.eps, attn.scaling, attn.sliding_window,
-                                          ops._OUT_CODES[x.dtype],
-                                          ops._VALUE_CODES[attn.value_dtype] | (2 if tc == torch.float16 else 0), ffn)
-
-
 class MimiTransformerLayerB200(nn.Module):
     def __init__(self, hidden_size: int = 512, intermediate_size: int = 2048, num_heads: int = 8, head_dim: int = 64,
                  sliding_window: int = 250, layer_idx: int = 0, norm_eps: float = 1e-5,
@@ -100,7 +79,7 @@ class MimiTransformerLayerB200(nn.Module):
         self.self_attn_layer_scale = _LayerScale(hidden_size, layer_scale_initial_scale)
         self.mlp_layer_scale = _LayerScale(hidden_size, layer_scale_initial_scale)
         self._cast = _Cast16()
-        self._plan: _LayerPlan | None = None
+        self._plan = None
 
     @classmethod
     def from_reference(cls, layer: nn.Module, value_dtype: torch.dtype = torch.float16) -> "MimiTransformerLayerB200":
@@ -117,37 +96,59 @@ class MimiTransformerLayerB200(nn.Module):
         new.mlp_layer_scale = layer.mlp_layer_scale
         return new
 
-    def _parameters_in_use(self) -> tuple:
-        """The layer's parameters, looked up in the modules' own tables (an attribute access per level costs more host
-        time than a launch)."""
-        m = self._modules
-        try:
-            a, mlp = m["self_attn"]._modules, m["mlp"]._modules
-            ln1, ln2 = m["input_layernorm"]._parameters, m["post_attention_layernorm"]._parameters
-            return (ln1["weight"], ln1["bias"], a["q_proj"]._parameters["weight"], a["k_proj"]._parameters["weight"],
-                    a["v_proj"]._parameters["weight"], a["o_proj"]._parameters["weight"],
-                    m["self_attn_layer_scale"]._parameters["scale"], ln2["weight"], ln2["bias"],
-                    mlp["fc1"]._parameters["weight"], mlp["fc2"]._parameters["weight"], m["mlp_layer_scale"]._parameters["scale"])
-        except KeyError:         # a parameter that is computed (parametrised weights and the like)
-            at, ln1, ln2 = self.self_attn, self.input_layernorm, self.post_attention_layernorm
-            return (ln1.weight, ln1.bias, at.q_proj.weight, at.k_proj.weight, at.v_proj.weight, at.o_proj.weight,
-                    self.self_attn_layer_scale.scale, ln2.weight, ln2.bias, self.mlp.fc1.weight, self.mlp.fc2.weight,
-                    self.mlp_layer_scale.scale)
+    def __getstate__(self) -> dict:
+        return {**self.__dict__, "_plan": None}         # device addresses: rebuilt by the copy's first call
 
-    def _native_plan(self, x: torch.Tensor) -> "_LayerPlan":
-        """The parameter block of the native call for activations like ``x``; rebuilt when a parameter was replaced or
-        written to, or when an option it depends on changed."""
+    def _native_plan(self, x: torch.Tensor):
+        """The parameter block of the native call for activations like ``x`` (16-bit weights, FP32 LayerNorm parameters and
+        layer scales) and, where every parameter is an entry of its module, the plan that notices when one of them, a
+        submodule or an option changes."""
+        attn, mlp, ln1, ln2 = self.self_attn, self.mlp, self.input_layernorm, self.post_attention_layernorm
+        ops._need(x.dtype in ops._OUT_CODES, "x must be bfloat16, float16 or float32")
+        if mlp.fc1.bias is not None or attn.o_proj.bias is not None:
+            raise RuntimeError("the fused layer expects bias-free projections, as in Mimi's checkpoints")
+        fc1, fc2 = mlp.fc1.weight, mlp.fc2.weight
+        ffn = fc1.shape[0]
+        ops._need(tuple(fc1.shape) == (ffn, 512) and tuple(fc2.shape) == (512, ffn) and ffn % 256 == 0,
+                  "the MLP must be 512 -> n -> 512 with n a multiple of 256")
+        tc = attn._tc_input_dtype(x)
+        f32 = lambda p: p.detach().float().contiguous()       # no copy for FP32 parameters
+        keep = (f32(ln1.weight), f32(ln1.bias), attn.packed_qkv_weight(tc), attn.out_weight(attn.value_dtype),
+                f32(self.self_attn_layer_scale.scale), f32(ln2.weight), f32(ln2.bias), self._cast.get("fc1", fc1, tc),
+                self._cast.get("fc2", fc2, tc), f32(self.mlp_layer_scale.scale))
+        for t in keep:
+            ops._need(t.is_cuda, "the layer's parameters must be on a CUDA device")
+        params = _native.LayerParams(*(t.data_ptr() for t in keep), ln1.eps, ln2.eps, attn.scaling, attn.sliding_window,
+                                     ops._OUT_CODES[x.dtype],
+                                     ops._VALUE_CODES[attn.value_dtype] | (2 if tc == torch.float16 else 0), ffn, 0)
+        watches = [(self._modules, n) for n in ("self_attn", "mlp", "input_layernorm", "post_attention_layernorm",
+                                                "self_attn_layer_scale", "mlp_layer_scale")]
+        watches += [(attn._modules, n) for n in ("q_proj", "k_proj", "v_proj", "o_proj")]
+        watches += [(mlp._modules, "fc1"), (mlp._modules, "fc2")]
+        watches += [(m._parameters, "weight") for m in (ln1, ln2, attn.q_proj, attn.k_proj, attn.v_proj, attn.o_proj, mlp.fc1, mlp.fc2)]
+        watches += [(m._parameters, "bias") for m in (ln1, ln2, attn.o_proj, mlp.fc1)]
+        watches += [(m._parameters, "scale") for m in (self.self_attn_layer_scale, self.mlp_layer_scale)]
+        watches += [(attn.__dict__, n) for n in ("sliding_window", "scaling", "value_dtype", "input_dtype")]
+        watches += [(ln1.__dict__, "eps"), (ln2.__dict__, "eps")]
+        try:
+            like_value = torch.empty(0, dtype=attn.value_dtype)
+            self._plan = _native.bind().LayerPlan(watches, keep, ctypes.addressof(params), ops.default_status(x.device), x, like_value)
+        except KeyError:            # a computed parameter (parametrised weights and the like): nothing to watch
+            self._plan = None
+        return params, keep
+
+    def _forward_checked(self, x, cos, sin, ring_k, ring_v, past) -> torch.Tensor:
+        """The call with everything looked at: arguments of other types or layouts, changed parameters, errors."""
         attn = self.self_attn
-        ps = self._parameters_in_use()
-        key = [x.dtype, x.device, attn.sliding_window, attn.scaling, attn.value_dtype, attn.input_dtype,
-               self.input_layernorm.eps, self.post_attention_layernorm.eps]
-        for p in ps:
-            key.append(p.data_ptr())
-            key.append(p._version)
-        plan = self._plan
-        if plan is None or plan.key != key:
-            plan = self._plan = _LayerPlan(self, x, ps, key)
-        return plan
+        x = x.contiguous()
+        cos, sin = cos.to(torch.float32).contiguous(), sin.to(torch.float32).contiguous()
+        params, keep = self._native_plan(x)
+        if self._plan is not None:
+            y = _native.bind().layer_forward(self._plan, x, cos, sin, ring_k, ring_v, past)
+            if isinstance(y, torch.Tensor):
+                return y
+        return ops.layer_forward(params, x, cos, sin, value_dtype=attn.value_dtype,
+                                 ring=None if ring_k is None else (ring_k, ring_v), past=past, window=attn.sliding_window)
 
     def forward(self, hidden_states: torch.Tensor, attention_mask: torch.Tensor | None, past_key_values,
                 position_embeddings: tuple[torch.Tensor, torch.Tensor], output_attentions: bool = False,
@@ -158,26 +159,31 @@ class MimiTransformerLayerB200(nn.Module):
             raise RuntimeError("MimiTransformerLayerB200 runs on a CUDA device only; there is no CPU path")
         if attention_mask is not None and attention_mask.dim() != 4:
             raise RuntimeError("key-padding masks are not supported; pass None or the 4-D causal band mask")
+        cache = past_key_values
+        if cache is None or isinstance(cache, MimiKVRing):
+            ring_k = ring_v = None
+            past = 0
+            if cache is not None:
+                attn = self.self_attn
+                ops._need(cache.num_streams == hidden_states.shape[0], "cache was created for a different number of streams")
+                ops._need(cache.sliding_window == attn.sliding_window, "cache window differs from the module's")
+                ring_k, ring_v = cache.layer_rings(attn.layer_idx)
+                past = cache.get_seq_length(attn.layer_idx)
+            cos, sin = position_embeddings
+            out = None
+            if self._plan is not None:
+                out = _native.bind().layer_forward(self._plan, hidden_states, cos, sin, ring_k, ring_v, past)
+            if out is None:
+                out = self._forward_checked(hidden_states, cos, sin, ring_k, ring_v, past)
+            elif type(out) is int:
+                _native.check(out, "fm_layer_forward")
+            if cache is not None:
+                cache.advance(attn.layer_idx, hidden_states.shape[1])
+            return out, None
         if self.mlp.fc1.bias is not None or self.self_attn.o_proj.bias is not None:
             raise RuntimeError("the fused layer expects bias-free projections, as in Mimi's checkpoints")
         attn = self.self_attn
         x = hidden_states.contiguous()
-        cache = past_key_values
-        if cache is None or isinstance(cache, MimiKVRing):
-            cos, sin = position_embeddings
-            if cos.dtype != torch.float32 or sin.dtype != torch.float32:
-                cos, sin = cos.to(torch.float32), sin.to(torch.float32)
-            plan = self._native_plan(x)
-            window, ring, past = attn.sliding_window, None, 0
-            if cache is not None:
-                ops._need(cache.num_streams == x.shape[0], "cache was created for a different number of streams")
-                ops._need(cache.sliding_window == window, "cache window differs from the module's")
-                ring, past = cache.layer_rings(attn.layer_idx), cache.get_seq_length(attn.layer_idx)
-            out = ops.layer_forward(plan.params, x, cos.contiguous(), sin.contiguous(), value_dtype=attn.value_dtype, ring=ring,
-                                    past=past, window=window)
-            if cache is not None:
-                cache.advance(attn.layer_idx, x.shape[1])
-            return out, None
         # a cache object of another kind: the kernels one by one around its own update
         stream_dtype = x.dtype
         tc = attn._tc_input_dtype(x)

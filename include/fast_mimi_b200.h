@@ -34,6 +34,8 @@ int fm_abi_version(void);
  *   params      host struct of device pointers; matrices are row-major [out, in] and 16 bit: w_qkv, w_fc1, w_fc2 in
  *               BF16 / FP16 by bit 1 of value_dtype, w_o in the value type (bit 0); LayerNorm parameters and layer
  *               scales FP32 (the scales may be NULL)
+ *               weights_settled: 0 on the first call after any of them was written on this stream (the call then starts
+ *               only when everything in front of it has ended), 1 afterwards
  *   x, y        [B, T, 512] in stream_dtype (0 BF16, 1 FP16, 2 FP32), y != x
  *   workspace   256-byte aligned device memory, at least  B*T*(2048 + 512*elem + max(2*ffn, 3072)) + 2*1024*B*(min(past, window-1) + T)
  *               + 4096 bytes (elem: bytes per value of x; the second term for cached calls only); -7 if too small
@@ -59,6 +61,7 @@ typedef struct fm_layer_params {
   int stream_dtype;
   int value_dtype;
   int ffn;
+  int weights_settled;
 } fm_layer_params;
 
 int fm_layer_forward(const fm_layer_params* params, const void* x, void* y, void* workspace, long long workspace_bytes,
