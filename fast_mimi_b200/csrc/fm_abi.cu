@@ -117,7 +117,9 @@ static int prefill_two_kernels(const void* x, const void* w_qkv, const float* co
                                int value_dtype, int* status, void* stream) {
   int rc = fm_qkv_rope_bf16(x, w_qkv, cos, sin, cos_bstride, q_ws, k_ws, v_ws, B, T, value_dtype, status, stream);
   if (rc != 0) return rc;
-  return fm_band_attn_prefill_bf16(q_ws, k_ws, v_ws, out, B, T, window, scale, value_dtype & 1, status, stream);
+  // the attention kernel may set itself up while the projection still runs
+  return fm::launch_band_attn_prefill(q_ws, k_ws, v_ws, out, B, T, window, scale, value_dtype & 1, status,
+                                      static_cast<cudaStream_t>(stream), 1);
 }
 
 int fm_attention_prefill_bf16(const void* x, const void* w_qkv, const float* cos, const float* sin,

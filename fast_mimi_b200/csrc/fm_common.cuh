@@ -459,25 +459,57 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
-// Exact-form GELU  0.5 x (1 + erf(x / sqrt 2))  with erf from the rational approximation
-//   erf(z) = 1 - (1 + a1 z + ... + a6 z^6)^-16,  z >= 0,  |error| <= 3e-7   (Abramowitz & Stegun 7.1.28)
-// instead of erff(): 15 issue slots and one reciprocal per value, no branch.  The epilogue is arithmetic-bound
-// with erff() (about 40 slots per value); the approximation error is far below the rounding of the result
-// to 16 bit.  Large |z| overflows the power to +inf, whose reciprocal is 0, i.e. erf = 1.
-__device__ __forceinline__ float gelu_erf(float x) {
-  const float z = fabsf(x) * 0.70710678118654752f;
-  float t = fmaf(z, 0.0000430638f, 0.0002765672f);
-  t = fmaf(z, t, 0.0001520143f);
-  t = fmaf(z, t, 0.0092705272f);
-  t = fmaf(z, t, 0.0422820123f);
-  t = fmaf(z, t, 0.0705230784f);
-  t = fmaf(z, t, 1.0f);
-  t *= t; t *= t; t *= t; t *= t;
+// Two FP32 values in a 64-bit register pair: one issue slot for both (add / mul / fma .rn.f32x2).
+__device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 f2_unpack(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
   float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(t));
-  const float e = copysignf(1.0f - r, x);
-  const float hx = 0.5f * x;
-  return fmaf(hx, e, hx);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Exact-form GELU  0.5 x (1 + erf(x / sqrt 2))  of two values, with erf from the rational approximation
+//   erf(z) = 1 - (1 + a1 z + ... + a6 z^6)^-16,  z >= 0,  |error| <= 3e-7   (Abramowitz & Stegun 7.1.28)
+// which makes it  max(x, 0) - 0.5 |x| r  with r = (...)^-16 and the powers of 1 / sqrt 2 folded into the coefficients:
+// nine issue slots per value in packed arithmetic (17 before with scalar FMAs, about 40 with erff()), one of them the
+// reciprocal.  The epilogue of fc1 is bound by these slots, not by the tensor core; the approximation error is far below
+// the rounding of the result to 16 bit.  Large |x| overflows the power to +inf, whose reciprocal is 0, i.e. erf = 1.
+__device__ __forceinline__ void gelu_erf2(float& x0, float& x1) {
+  constexpr float kS = 0.70710678118654752f;
+  constexpr float a1 = 0.0705230784f * kS, a2 = 0.0422820123f * kS * kS, a3 = 0.0092705272f * kS * kS * kS;
+  constexpr float a4 = 0.0001520143f * kS * kS * kS * kS, a5 = 0.0002765672f * kS * kS * kS * kS * kS;
+  constexpr float a6 = 0.0000430638f * kS * kS * kS * kS * kS * kS;
+  const unsigned long long z = f2_pack(fabsf(x0), fabsf(x1));
+  unsigned long long t = f2_fma(z, f2_pack(a6, a6), f2_pack(a5, a5));
+  t = f2_fma(z, t, f2_pack(a4, a4));
+  t = f2_fma(z, t, f2_pack(a3, a3));
+  t = f2_fma(z, t, f2_pack(a2, a2));
+  t = f2_fma(z, t, f2_pack(a1, a1));
+  t = f2_fma(z, t, f2_pack(1.f, 1.f));
+  t = f2_mul(t, t); t = f2_mul(t, t); t = f2_mul(t, t); t = f2_mul(t, t);
+  const float2 p = f2_unpack(t);
+  const unsigned long long r = f2_pack(rcp_approx(p.x), rcp_approx(p.y));
+  const float2 y = f2_unpack(f2_fma(f2_mul(z, f2_pack(-0.5f, -0.5f)), r, f2_pack(fmaxf(x0, 0.f), fmaxf(x1, 0.f))));
+  x0 = y.x;
+  x1 = y.y;
 }
 
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {

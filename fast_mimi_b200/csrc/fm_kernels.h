@@ -64,9 +64,9 @@ int launch_linear_gemm(const void* a, const void* w, void* y, const float* scale
                        int K, int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent = 0);
 // The same two products for few rows (fm_linear_small.cu): 128 x 64 tiles, K split over a cluster.
 bool few_row_tiles(int M, int N);
-// LayerNorm folded into the product behind it (fm_ln_linear.cu), for up to 256 rows: the chain-opening QKV projection and
+// LayerNorm folded into the product behind it (fm_ln_linear.cu) while one wave of blocks holds the rows: the chain-opening QKV projection and
 // gelu(LayerNorm(x) W^T).
-bool few_rows_with_norm(int M);
+bool few_rows_with_norm(int M, int N);
 int launch_ln_qkv(const void* x, int x_dtype, const float* weight, const float* bias, float eps, const void* w_qkv,
                   const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status, cudaStream_t st, int dependent);
 int launch_ln_linear_gelu(const void* x, int x_dtype, const float* weight, const float* bias, float eps, const void* w, void* y,
@@ -117,12 +117,18 @@ int launch_ring_append(const void* k_new, const void* v_new, void* ring_k, void*
 int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k, void* ring_v, void* out, int S, int T,
                        int past, int slots, int window, float scale, int value_is_fp16, int out_dtype, int* status,
                        cudaStream_t st, int dependent = 0);
+// Attention for few query tiles (fm_few_attn.cu): at most two 64-query blocks per SM.  ring_k null: clips; else T new frames
+// per stream on top of the ring, which the kernel also updates where one block has a whole (stream, head).
+bool few_attn_tiles(int S, int T);
+bool few_attn_updates_ring(int T);
+int launch_few_attn(const void* q, const void* k, const void* v, void* ring_k, void* ring_v, void* out, int S, int T, int past,
+                    int slots, int window, float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent = 0);
 // Projection + RoPE + banded attention in one kernel for 128 < T <= 256 (fm_fused_clip.cu): q, k, v stay on chip.
 int launch_attn_fused_clip(const void* x, const void* w_qkv, const float* cos, const float* sin, long long cos_bstride,
                            void* out, int B, int T, int window, float scale, int dtype_flags, int* status,
                            cudaStream_t st, int dependent = 0);
 // Whether whole clips take the one-kernel form (fm_fused_clip.cu) rather than projection + attention.
-bool use_fused_clip(int B);
+bool use_fused_clip(int B, int T);
 int launch_band_attn_clip(const void* q, const void* k, const void* v, void* out, int B, int T, int window,
                           float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent = 0);
 int launch_band_attn_long(const void* q, const void* k, const void* v, void* out, int B, int T, int window,

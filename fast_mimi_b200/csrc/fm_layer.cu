@@ -69,13 +69,14 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
   const int value_fp16 = p.value_dtype & 1;
   const int tc = (p.value_dtype & 2) ? 1 : 0;                    // 16-bit type of the products' operands: 0 BF16, 1 FP16
 
-  const bool norm_inside = few_rows_with_norm(rows);
+  const bool norm1_inside = few_rows_with_norm(rows, 1536), norm2_inside = few_rows_with_norm(rows, p.ffn);
   int rc = 0;
-  if (!norm_inside) {
+  if (!norm1_inside) {
     rc = launch_layernorm512(x, p.stream_dtype, p.ln1_weight, p.ln1_bias, p.ln1_eps, b.h, tc, rows, st, 1);
     if (rc != 0) return rc;
   }
-  if (whole_clip && !norm_inside && use_fused_clip(B)) {
+  const bool few_tiles = !few && few_attn_tiles(B, T) && (!cached || slots <= 256);
+  if (whole_clip && !few_tiles && use_fused_clip(B, T)) {
     rc = launch_attn_fused_clip(b.h, p.w_qkv, cos, sin, cos_bstride, b.core, B, T, p.window, p.scale, p.value_dtype, status, st, 1);
   } else {
     QkvEpilogueArgs ep = {};
@@ -89,11 +90,14 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
     ep.ring_slots = 1;
     // The kernel that opens the chain may ask for W_qkv ahead of its wait only if W_qkv cannot be the work of the kernel
     // in front: not on the first call after the caller has (re)made it.
-    rc = norm_inside ? launch_ln_qkv(x, p.stream_dtype, p.ln1_weight, p.ln1_bias, p.ln1_eps, p.w_qkv, ep, rows, p.value_dtype,
-                                     status, st, p.weights_settled)
-                     : launch_qkv_rope_gemm(b.h, p.w_qkv, ep, rows, p.value_dtype, status, st, 1);
+    rc = norm1_inside ? launch_ln_qkv(x, p.stream_dtype, p.ln1_weight, p.ln1_bias, p.ln1_eps, p.w_qkv, ep, rows, p.value_dtype,
+                                      status, st, p.weights_settled)
+                      : launch_qkv_rope_gemm(b.h, p.w_qkv, ep, rows, p.value_dtype, status, st, 1);
     if (rc != 0) return rc;
-    if (!cached) {
+    if (few_tiles) {
+      rc = launch_few_attn(b.q, b.k, b.v, ring_k, ring_v, b.core, B, T, past, slots, p.window, p.scale, value_fp16, status, st, 1);
+      if (rc == 0 && cached && !few_attn_updates_ring(T)) rc = launch_ring_append(b.k, b.v, ring_k, ring_v, B, T, past, slots, st, 1);
+    } else if (!cached) {
       rc = launch_band_attn_prefill(b.q, b.k, b.v, b.core, B, T, p.window, p.scale, value_fp16, status, st, 1);
     } else if (few) {
       rc = launch_stream_attn(b.q, b.k, b.v, ring_k, ring_v, b.core, B, T, past, slots, p.window, p.scale, value_fp16, 0,
@@ -113,7 +117,7 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
   if (rc != 0) return rc;
   rc = launch_linear_gemm(b.core, p.w_o, b.x1, p.attn_scale, x, rows, 512, 512, value_fp16, p.stream_dtype, 0, status, st, 1);
   if (rc != 0) return rc;
-  if (norm_inside) {
+  if (norm2_inside) {
     rc = launch_ln_linear_gelu(b.x1, p.stream_dtype, p.ln2_weight, p.ln2_bias, p.ln2_eps, p.w_fc1, b.g, rows, p.ffn, tc, status,
                                st, 1);
   } else {

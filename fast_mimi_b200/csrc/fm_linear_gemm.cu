@@ -11,7 +11,7 @@
 // Unlike the QKV projection kernel, which keeps its x tile resident because K is only 512, both operands
 // stream here: a stage holds a 128 x 64 slice of a and a 128 x 64 slice of W per CTA (32 KB), five or six stages deep.
 // Two CTAs form a pair (cluster of 2, tcgen05 cta_group::2): one tcgen05.mma multiplies the pair's 256 rows by
-// 256 weight rows, each CTA contributing half of the weight tile.  Accumulators: two 256-column TMEM buffers
+// 256 (or 128) weight rows, each CTA contributing half of the weight tile.  Accumulators: two 256-column TMEM buffers
 // per CTA, so the epilogue of one unit overlaps the MMAs of the next.  Persistent: (row-tile pair, 256-wide
 // output tile) units, numbered row-tile-major, are dealt round-robin to the pairs, so the output tiles of a
 // row tile are computed at the same time by neighbouring pairs and share its a slices through L2.
@@ -22,8 +22,8 @@
 //           not the tensor core, bounds the kernel, and eight warps cannot hide its latencies.  Five warps per SM
 //           sub-partition leave 96 registers per thread at launch; the load / issue warpgroup shrinks to 32 and the
 //           epilogue warpgroups grow to 112 (setmaxnreg: 512 x 112 + 128 x 32 = 640 x 96).
-//   narrow  warps 0-7 epilogue (two 64-column groups each), warps 8 and 9 producer and issuer; six stages (the
-//           shared memory of eight staging slabs buys the sixth, which the K = 2048 layer uses).
+//   narrow  warps 0-7 epilogue (two 64-column groups each, one with 128-wide units), warps 8 and 9 producer and issuer;
+//           six (seven) stages (the shared memory of eight staging slabs buys the sixth, which the K = 2048 layer uses).
 #include <type_traits>
 
 #include "fm_common.cuh"
@@ -34,28 +34,26 @@ namespace fm {
 
 namespace lin {
 constexpr int kBlockM = 128;           // rows per CTA
-constexpr int kBlockN = 256;           // outputs per unit
-constexpr int kHalfN = kBlockN / 2;    // weight rows loaded by each CTA of the pair
 constexpr int kBlockK = 64;            // one 128-byte swizzle row of 16-bit values
 constexpr int kABytes = kBlockM * kBlockK * 2;   // 16 KB
-constexpr int kBBytes = kHalfN * kBlockK * 2;    // 16 KB
-constexpr int kStageBytes = kABytes + kBBytes;
 constexpr int kSlabBytes = 32 * 128;             // one warp's staging: 32 rows x 128 bytes
-template <bool kWide> struct Shape {
-  static constexpr int kStages = kWide ? 5 : 6;
+template <bool kWide, int kBlockN> struct Shape {
+  static constexpr int kHalfN = kBlockN / 2;              // weight rows loaded by each CTA of the pair
+  static constexpr int kStageBytes = kABytes + kHalfN * kBlockK * 2;
+  static constexpr int kStages = kWide ? 5 : (kBlockN == 256 ? 6 : 7);
   static constexpr int kEpiWarps = kWide ? 16 : 8;
-  static constexpr int kGroupsPerWarp = 16 / kEpiWarps;   // a unit has four 64-column groups per lane group
+  static constexpr int kGroupsPerWarp = kBlockN / 16 / kEpiWarps;   // a unit has kBlockN / 64 64-column groups per lane group
+  static constexpr int kTmemCols = 2 * kBlockN;
   // wide: five warpgroups, the last one holds the producer and the issuer; narrow: epilogue warps + 2
   static constexpr int kThreads = kWide ? (kEpiWarps + 4) * 32 : (kEpiWarps + 2) * 32;
   static constexpr int kSmemBytes = 1024 /*align*/ + kStages * kStageBytes + kEpiWarps * kSlabBytes + 256;
 };
 constexpr int kEpiRegs = 112, kIssueRegs = 32;
-static_assert(512 * kEpiRegs + 128 * kIssueRegs <= Shape<true>::kThreads * 96, "register pool of the launch");
-constexpr int kTmemCols = 512;
+static_assert(512 * kEpiRegs + 128 * kIssueRegs <= Shape<true, 256>::kThreads * 96, "register pool of the launch");
 
 struct Barriers {
-  uint64_t full[6];            // used in the leader: bytes of both CTAs' a and W slices
-  uint64_t empty[6];           // per CTA: stage consumed by the tensor core
+  uint64_t full[7];            // used in the leader: bytes of both CTAs' a and W slices
+  uint64_t empty[7];           // per CTA: stage consumed by the tensor core
   uint64_t acc_full[2];        // per CTA: accumulator buffer complete
   uint64_t acc_empty[2];       // used in the leader: the epilogue warps of both CTAs drained the buffer
   uint32_t tmem_base;
@@ -72,19 +70,21 @@ struct LinearArgs {
   int M, N, K;
   int gelu;               // 1: exact GELU on the accumulator before scale / residual
   uint4* records;         // kOut 3: [M, N / 64] candidate records
+  void* y;                // [M, N]: stored directly where there is a residual, through the tensor map otherwise
 };
 
 // kOut: 0 = BF16, 1 = FP16, 2 = FP32 (type of y and of the residual); 3 = no y at all: the products are the inner
 // products x . e_j of a nearest-entry search and the epilogue reduces every 64 of them to one 16-byte record
 // {min_j d_j, 64-bit mask of the entries with d_j <= min + margin[row]},  d_j = |e_j|^2 - 2 x . e_j  (see fm_rvq.cu).
-template <int kOut, bool kWide>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(lin::Shape<kWide>::kThreads, 1)
+template <int kOut, bool kWide, int kBlockN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(lin::Shape<kWide, kBlockN>::kThreads, 1)
 linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
                    const __grid_constant__ CUtensorMap tmap_y, LinearArgs args, int total_units, uint32_t idesc,
                    int* status) {
   using namespace lin;
-  constexpr int kStages = Shape<kWide>::kStages, kEpiWarps = Shape<kWide>::kEpiWarps;
-  constexpr int kGroupsPerWarp = Shape<kWide>::kGroupsPerWarp;
+  using S = Shape<kWide, kBlockN>;
+  constexpr int kStages = S::kStages, kEpiWarps = S::kEpiWarps, kGroupsPerWarp = S::kGroupsPerWarp;
+  constexpr int kStageBytes = S::kStageBytes, kHalfN = S::kHalfN, kTmemCols = S::kTmemCols;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_stage = smem;                                  // kStages x [a slice | W slice]
@@ -205,7 +205,84 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     const int gsel = warp >> 2;   // which of the unit's four 64-column groups (wide), or which two (narrow)
     const uint32_t acc_empty_leader = map_to_cta(smem_u32(&bars->acc_empty[0]), 0);
     uint8_t* slab = smem_out + warp * kSlabBytes;
-    for (int i = 0; i < u_count; ++i) {
+    bool done = false;
+    if constexpr (kOut < 3) {
+      if (args.resid != nullptr) {
+        // With a residual, accumulator rows cross the slab so that every lane finishes four columns of eight rows, and
+        // residual and result are read and written as whole 128-byte (16 bit: 64-byte) lines by neighbouring lanes.  When
+        // each lane fetched its own row's residual a load instruction touched 32 cache lines: 17 us of load-unit time per
+        // 256 x 256 unit, more than its products take at K = 2048 (o_proj with an FP32 stream: 14 us at any row count).
+        // A piece's residual (32 columns) is asked for one piece ahead.
+        done = true;
+        using T16 = typename std::conditional<kOut == 1, __half, __nv_bfloat16>::type;
+        using R = typename std::conditional<kOut == 2, float4, uint2>::type;             // four values
+        constexpr int kElem = kOut == 2 ? 4 : 2, kPieces = 2 * kGroupsPerWarp;
+        const int r0 = lg * 32 + (lane >> 3), c4 = 4 * (lane & 7);
+        const int n_pieces = u_count * kPieces;
+        auto first_row = [&](int i) { return (2 * ((pair + i * n_pairs) / n_tiles) + static_cast<int>(rank)) * kBlockM + r0; };
+        auto first_col = [&](int i, int p) { return ((pair + i * n_pairs) % n_tiles) * kBlockN + (gsel * kPieces + p) * 32 + c4; };
+        auto fetch = [&](int idx, R (&r)[8]) {
+          const int i = idx / kPieces, row = first_row(i);
+          const uint8_t* src = static_cast<const uint8_t*>(args.resid) + (static_cast<long long>(row) * args.N + first_col(i, idx % kPieces)) * kElem;
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (row + 4 * k < args.M) r[k] = *reinterpret_cast<const R*>(src + static_cast<long long>(4 * k) * args.N * kElem);
+        };
+        R res[8];
+        if (n_pieces > 0) fetch(0, res);
+#pragma unroll 1
+        for (int idx = 0; idx < n_pieces; ++idx) {
+          const int i = idx / kPieces, p = idx % kPieces, buf = i & 1;
+          if (p == 0) {
+            mbar_wait(&bars->acc_full[buf], static_cast<uint32_t>(i >> 1) & 1u, ctl, status, kErrWaitMma);
+            tc_fence_after_sync();
+          }
+          uint32_t acc[32];
+          tmem_ld32(tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + static_cast<uint32_t>(buf * kBlockN + (gsel * kPieces + p) * 32), acc);
+          R next[8];
+          if (idx + 1 < n_pieces) fetch(idx + 1, next);
+          const int col = first_col(i, p);
+          const float4 sc = args.scale != nullptr ? __ldg(reinterpret_cast<const float4*>(args.scale + col)) : make_float4(1.f, 1.f, 1.f, 1.f);
+          tmem_ld_wait();
+          if (p == kPieces - 1) {
+            // Last read of the accumulator by this warp: hand it back before the arithmetic and the stores.
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster_relaxed(acc_empty_leader + static_cast<uint32_t>(buf) * 8u);
+          }
+          float v[32];
+#pragma unroll
+          for (int c = 0; c < 32; ++c) v[c] = __uint_as_float(acc[c]);
+          if (args.gelu) {
+#pragma unroll
+            for (int c = 0; c < 32; c += 2) gelu_erf2(v[c], v[c + 1]);
+          }
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            *reinterpret_cast<float4*>(slab + sw128_offset(lane, c)) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+          __syncwarp();
+          const int row = first_row(i);
+          uint8_t* dst = static_cast<uint8_t*>(args.y) + (static_cast<long long>(row) * args.N + col) * kElem;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            float4 o = *reinterpret_cast<const float4*>(slab + sw128_offset(4 * k + (lane >> 3), lane & 7));
+            o.x *= sc.x; o.y *= sc.y; o.z *= sc.z; o.w *= sc.w;
+            if constexpr (kOut == 2) {
+              o.x += res[k].x; o.y += res[k].y; o.z += res[k].z; o.w += res[k].w;
+              if (row + 4 * k < args.M) *reinterpret_cast<float4*>(dst + static_cast<long long>(4 * k) * args.N * 4) = o;
+            } else {
+              const float2 ra = Pack16<T16>::unpack(res[k].x), rb = Pack16<T16>::unpack(res[k].y);
+              if (row + 4 * k < args.M)
+                *reinterpret_cast<uint2*>(dst + static_cast<long long>(4 * k) * args.N * 2) =
+                    make_uint2(Pack16<T16>::pack(o.x + ra.x, o.y + ra.y), Pack16<T16>::pack(o.z + rb.x, o.w + rb.y));
+            }
+            res[k] = next[k];
+          }
+          __syncwarp();
+        }
+      }
+    }
+    for (int i = 0; !done && i < u_count; ++i) {
       const int u = pair + i * n_pairs, row_tile = u / n_tiles, ntile = u % n_tiles;
       const int m0 = (2 * row_tile + static_cast<int>(rank)) * kBlockM;
       const long long row = static_cast<long long>(m0) + lg * 32 + lane;
@@ -258,7 +335,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         }
         if (args.gelu) {
 #pragma unroll
-          for (int c = 0; c < 64; ++c) v[c] = gelu_erf(v[c]);
+          for (int c = 0; c < 64; c += 2) gelu_erf2(v[c], v[c + 1]);
         }
         if (args.scale != nullptr) {
           const float4* s4 = reinterpret_cast<const float4*>(args.scale + col0);   // same address in every lane
@@ -266,30 +343,6 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           for (int j = 0; j < 16; ++j) {
             const float4 s = __ldg(s4 + j);
             v[4 * j] *= s.x; v[4 * j + 1] *= s.y; v[4 * j + 2] *= s.z; v[4 * j + 3] *= s.w;
-          }
-        }
-        if (args.resid != nullptr && row_ok) {
-          if constexpr (kOut == 2) {
-            const float4* r4 = reinterpret_cast<const float4*>(static_cast<const float*>(args.resid) + row * args.N + col0);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float4 r = r4[j];
-              v[4 * j] += r.x; v[4 * j + 1] += r.y; v[4 * j + 2] += r.z; v[4 * j + 3] += r.w;
-            }
-          } else {
-            using T16 = typename std::conditional<kOut == 1, __half, __nv_bfloat16>::type;
-            const uint4* r4 = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(args.resid) + row * args.N + col0);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const uint4 r = r4[j];
-              const uint32_t w4[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float2 f = Pack16<T16>::unpack(w4[e]);
-                v[8 * j + 2 * e] += f.x;
-                v[8 * j + 2 * e + 1] += f.y;
-              }
-            }
           }
         }
         if constexpr (kOut == 2) {
@@ -352,10 +405,40 @@ static int encode_2d(CUtensorMap* map, CUtensorMapDataType type, int elem_bytes,
   return encode_tiled(map, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
+template <int kOut, bool kWide, int kBlockN>
+static int launch_pairs(const void* a, const void* w, void* y, const LinearArgs& args, int pair_tiles, int max_pairs, int in_dtype,
+                        int out_dtype, int* status, cudaStream_t st, int dependent) {
+  using namespace lin;
+  using S = Shape<kWide, kBlockN>;
+  CUtensorMap tmap_a, tmap_w, tmap_y;
+  const CUtensorMapDataType t16 = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;   // any 16-bit element type moves alike
+  const uint64_t M = static_cast<uint64_t>(args.M), N = static_cast<uint64_t>(args.N), K = static_cast<uint64_t>(args.K);
+  int rc = encode_2d(&tmap_a, t16, 2, a, M, K, kBlockM, kBlockK);
+  if (rc != 0) return rc;
+  rc = encode_2d(&tmap_w, t16, 2, w, N, K, S::kHalfN, kBlockK);
+  if (rc != 0) return rc;
+  if (out_dtype == 3)      // no tiled store in this mode: a placeholder map over a
+    rc = encode_2d(&tmap_y, t16, 2, a, M, K, 32, 64);
+  else if (out_dtype == 2)
+    rc = encode_2d(&tmap_y, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, y, M, N, 32, 32);
+  else
+    rc = encode_2d(&tmap_y, t16, 2, y, M, N, 32, 64);
+  if (rc != 0) return rc;
+  const int total_units = pair_tiles * (args.N / kBlockN);
+  const int n_pairs = total_units < max_pairs ? total_units : max_pairs;
+  const int fmt = in_dtype == 1 ? 0 : 1;   // tcgen05 kind::f16 operand format: 0 = F16, 1 = BF16
+  const uint32_t idesc = umma_idesc_f16(2 * kBlockM, kBlockN, fmt, fmt, 0, 0);
+  auto kern = linear_gemm_kernel<kOut, kWide, kBlockN>;
+  rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), S::kSmemBytes);
+  if (rc != 0) return rc;
+  return launch_kernel(kern, dim3(2 * n_pairs), S::kThreads, S::kSmemBytes, st, 1, dependent, tmap_a, tmap_w, tmap_y, args, total_units,
+                       idesc, status);
+}
+
 int launch_linear_gemm(const void* a, const void* w, void* y, const float* scale, const void* resid, int M, int N,
                        int K, int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent) {
   using namespace lin;
-  if (M < 0 || N <= 0 || K <= 0 || N % kBlockN != 0 || K % kBlockK != 0) return -1;
+  if (M < 0 || N <= 0 || K <= 0 || N % 256 != 0 || K % kBlockK != 0) return -1;
   if (in_dtype < 0 || in_dtype > 1 || out_dtype < 0 || out_dtype > 3) return -1;
   if (M == 0) return 0;
   if (a == nullptr || w == nullptr || y == nullptr) return -1;
@@ -365,42 +448,25 @@ int launch_linear_gemm(const void* a, const void* w, void* y, const float* scale
     return -3;
   if (out_dtype != 3 && few_row_tiles(M, N))
     return launch_linear_small(a, w, y, scale, resid, M, N, K, in_dtype, out_dtype, gelu, status, st, dependent);
-  CUtensorMap tmap_a, tmap_w, tmap_y;
-  const CUtensorMapDataType t16 = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;   // any 16-bit element type moves alike
-  int rc = encode_2d(&tmap_a, t16, 2, a, static_cast<uint64_t>(M), static_cast<uint64_t>(K), kBlockM, kBlockK);
-  if (rc != 0) return rc;
-  rc = encode_2d(&tmap_w, t16, 2, w, static_cast<uint64_t>(N), static_cast<uint64_t>(K), kHalfN, kBlockK);
-  if (rc != 0) return rc;
-  if (out_dtype == 3)      // no tiled store in this mode: a placeholder map over a
-    rc = encode_2d(&tmap_y, t16, 2, a, static_cast<uint64_t>(M), static_cast<uint64_t>(K), 32, 64);
-  else if (out_dtype == 2)
-    rc = encode_2d(&tmap_y, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, y, static_cast<uint64_t>(M), static_cast<uint64_t>(N), 32, 32);
-  else
-    rc = encode_2d(&tmap_y, t16, 2, y, static_cast<uint64_t>(M), static_cast<uint64_t>(N), 32, 64);
-  if (rc != 0) return rc;
-  const int m_tiles = (M + kBlockM - 1) / kBlockM;
-  const int pair_tiles = (m_tiles + 1) / 2;
-  const int total_units = pair_tiles * (N / kBlockN);
+  // 256 x 256 units, or 256 x 128 where those fill the pairs better: a unit of half the width costs a little more than
+  // half the time (its a slices are fetched twice as often), so the narrow form has to save a quarter of a wave.
+  const int pair_tiles = ((M + kBlockM - 1) / kBlockM + 1) / 2;
   const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
-  const int n_pairs = total_units < max_pairs ? total_units : max_pairs;
-  const int fmt = in_dtype == 1 ? 0 : 1;   // tcgen05 kind::f16 operand format: 0 = F16, 1 = BF16
-  const uint32_t idesc = umma_idesc_f16(2 * kBlockM, kBlockN, fmt, fmt, 0, 0);
-  LinearArgs args = {scale, resid, M, N, K, gelu ? 1 : 0, out_dtype == 3 ? static_cast<uint4*>(y) : nullptr};
   // The wide shape where the epilogue carries arithmetic (GELU, candidate records), the narrow one otherwise.
   const bool wide = gelu || out_dtype == 3;
-  using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, LinearArgs, int, uint32_t, int*);
-  Kern kern;
+  const int waves256 = (pair_tiles * (N / 256) + max_pairs - 1) / max_pairs, waves128 = (pair_tiles * (N / 128) + max_pairs - 1) / max_pairs;
+  const bool halves = !wide && 9 * waves128 < 16 * waves256;
+  LinearArgs args = {scale, resid, M, N, K, gelu ? 1 : 0, out_dtype == 3 ? static_cast<uint4*>(y) : nullptr, y};
+  using Fn = int (*)(const void*, const void*, void*, const LinearArgs&, int, int, int, int, int*, cudaStream_t, int);
+  Fn fn;
   if (wide)
-    kern = out_dtype == 3 ? linear_gemm_kernel<3, true>
-                          : (out_dtype == 2 ? linear_gemm_kernel<2, true> : (out_dtype == 1 ? linear_gemm_kernel<1, true> : linear_gemm_kernel<0, true>));
+    fn = out_dtype == 3 ? launch_pairs<3, true, 256>
+                        : (out_dtype == 2 ? launch_pairs<2, true, 256> : (out_dtype == 1 ? launch_pairs<1, true, 256> : launch_pairs<0, true, 256>));
+  else if (halves)
+    fn = out_dtype == 2 ? launch_pairs<2, false, 128> : (out_dtype == 1 ? launch_pairs<1, false, 128> : launch_pairs<0, false, 128>);
   else
-    kern = out_dtype == 2 ? linear_gemm_kernel<2, false> : (out_dtype == 1 ? linear_gemm_kernel<1, false> : linear_gemm_kernel<0, false>);
-  const int smem_bytes = wide ? Shape<true>::kSmemBytes : Shape<false>::kSmemBytes;
-  const int threads = wide ? Shape<true>::kThreads : Shape<false>::kThreads;
-  rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes);
-  if (rc != 0) return rc;
-  return launch_kernel(kern, dim3(2 * n_pairs), threads, smem_bytes, st, 1, dependent, tmap_a, tmap_w, tmap_y, args, total_units,
-                       idesc, status);
+    fn = out_dtype == 2 ? launch_pairs<2, false, 256> : (out_dtype == 1 ? launch_pairs<1, false, 256> : launch_pairs<0, false, 256>);
+  return fn(a, w, y, args, pair_tiles, max_pairs, in_dtype, out_dtype, status, st, dependent);
 }
 
 }  // namespace fm

@@ -4,11 +4,12 @@
 // What bounds such a call is latency and the number of SMs that pull weights out of L2, not arithmetic: the pair
 // kernels (fm_linear_gemm.cu, fm_qkv_gemm.cu) cut the output into 256 x 256 tiles, so that 125 rows x 512 outputs at
 // K = 2048 occupied 4 of 148 SMs, each walking 32 K-chunks one after the other (33 us; here 5 us).  Here a block owns
-// 128 rows x 64 outputs (one attention head) and a SLICE of K: the blocks of a thread-block cluster share one output
+// 128 rows x 64 outputs (one attention head; or x 32) and a SLICE of K: the blocks of a thread-block cluster share one output
 // tile and split K between them, so the same layer runs on 64 SMs with four chunks each.  The partial sums meet in
-// distributed shared memory: row r of the tile belongs to cluster rank r % S, every block writes its FP32 partials of
-// that row straight into the owner's shared memory, one cluster barrier, and the owner adds them in rank order (the
-// result does not depend on timing), applies the epilogue and stores whole 64-byte segments.
+// distributed shared memory: row r of the tile belongs to cluster rank r % S, every block sends its FP32 partials of an
+// owner's rows with one bulk copy per warp and owner (single 16-byte remote stores took 1.5 us for a full tile), and the
+// owner adds them in rank order (the result does not depend on timing), applies the epilogue and stores whole 64-byte
+// segments.
 //
 // Weights do not depend on the kernel in front, so in a chain of dependent launches the W slices of the first stages
 // are requested before the wait for that kernel and arrive while it still runs.  About 105 KB of shared memory and 64
@@ -23,21 +24,21 @@ namespace fm {
 
 namespace small {
 constexpr int kBlockM = 128;
-constexpr int kBlockN = 64;
 constexpr int kBlockK = 64;
 constexpr int kStages = 3;
 constexpr int kABytes = kBlockM * kBlockK * 2;     // 16 KB
-constexpr int kBBytes = kBlockN * kBlockK * 2;     // 8 KB
-constexpr int kStageBytes = kABytes + kBBytes;
-constexpr int kRedBytes = kBlockM * kBlockN * 4;   // S sources x (128 / S) rows x 64 FP32
 constexpr int kThreads = 192;
-constexpr int kTmemCols = 64;
-constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kRedBytes + 128;
+template <int kBlockN> struct Tile {
+  static constexpr int kStageBytes = kABytes + kBlockN * kBlockK * 2;
+  static constexpr int kRedBytes = kBlockM * kBlockN * 4;      // S sources x (128 / S) rows x FP32 columns
+  static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kRedBytes + 128;
+};
 
 struct Barriers {
   uint64_t full[kStages];
   uint64_t empty[kStages];
   uint64_t acc_full;
+  uint64_t red_full;         // the partial sums of this block's rows have arrived from every block of the cluster
   uint32_t tmem_base;
   CtaCtl ctl;
 };
@@ -45,17 +46,23 @@ static_assert(sizeof(Barriers) <= 128, "barrier block too large");
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ void st_cluster_v4(uint32_t addr, float a, float b, float c, float d) {
-  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+// Copy from this block's shared memory into that of a block of the cluster (both addresses 16-byte aligned); the bytes are
+// counted on a barrier of the destination.
+__device__ __forceinline__ void bulk_copy_to_cta(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "r"(smem_u32(src)), "r"(bytes), "r"(bar) : "memory");
 }
 }  // namespace small
 
 // kOut: 0 = BF16, 1 = FP16, 2 = FP32 output and residual; 3 = q | k | v with RoPE (VT: type of v)
-template <int kOut, typename VT>
+template <int kOut, typename VT, int kBlockN>
 __global__ void __launch_bounds__(small::kThreads)
 linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
                     const __grid_constant__ SmallArgs args, uint32_t idesc, int* status) {
   using namespace small;
+  constexpr int kStageBytes = Tile<kBlockN>::kStageBytes, kRedBytes = Tile<kBlockN>::kRedBytes, kTmemCols = kBlockN;
+  constexpr int kHalves = kBlockN / 32;
+  constexpr uint32_t kRowBytes = kBlockN * 4;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* red = smem + kStages * kStageBytes;
@@ -67,6 +74,10 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const int n0 = ntile * kBlockN;
   const int m0 = static_cast<int>(blockIdx.y) * kBlockM;
   const int chunk0 = rank * args.chunks;
+  // Row r of the tile belongs to rank r % S.
+  const int log_s = 31 - __clz(split);
+  const int valid = args.M - m0 < kBlockM ? args.M - m0 : kBlockM;
+  const int n_own = (valid - rank + split - 1) >> log_s;
 
   // read early: a status set before this chain began stops every kernel of it (the stores are left out)
   const bool skip = status != nullptr && *reinterpret_cast<volatile int*>(status) != 0;
@@ -76,8 +87,10 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       mbar_init(&bars->empty[i], 1);
     }
     mbar_init(&bars->acc_full, 1);
+    mbar_init(&bars->red_full, 1);
     bars->ctl.abort = 0;
     fence_mbar_init();
+    if (split > 1 && n_own > 0) mbar_arrive_expect_tx(&bars->red_full, static_cast<uint32_t>(split * n_own) * kRowBytes);
   }
   if (warp == 5) {
     tmem_alloc(&bars->tmem_base, kTmemCols);
@@ -130,41 +143,53 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   }
   griddep_wait();                          // residual and outputs belong to the chain
   // The rows this block owns: rank, rank + S, ... of the tile; eight threads per row, columns 4j.. and 32 + 4j...
-  const int log_s = 31 - __clz(split);
-  const int valid = args.M - m0 < kBlockM ? args.M - m0 : kBlockM;
-  const int n_items = skip ? 0 : ((valid - rank + split - 1) >> log_s) * 8;
+  const int n_items = skip ? 0 : n_own * 8;
   auto item_row = [&](int item) { return m0 + ((item >> 3) << log_s) + rank; };
   PieceOperands ops;
   int item = static_cast<int>(threadIdx.x);
-  if (item < n_items) load_operands<kOut>(args, item_row(item), ntile, item & 7, ops);
+  if (item < n_items) load_operands<kOut, kHalves>(args, item_row(item), ntile, item & 7, ops);
   if (warp < 4) {
     mbar_wait(&bars->acc_full, 0, ctl, status, kErrWaitMma);
     tc_fence_after_sync();
   }
-  if (split > 1) cluster_wait();           // every block of the cluster runs
+  __syncwarp();
+  if (split > 1) cluster_wait();           // every block of the cluster runs and has armed its barrier
   if (warp < 4) {
+    // Rows grouped by owner in the stage memory (this block's products are complete, nothing else uses it), then one bulk
+    // copy per owner.
     const int row = warp * 32 + lane;
-    const int owner = row & (split - 1), slot = rank * (kBlockM >> log_s) + (row >> log_s);
-    uint32_t red_addr = smem_u32(red);
-    if (split > 1) red_addr = map_to_cta(red_addr, static_cast<uint32_t>(owner));
+    const uint32_t staged = static_cast<uint32_t>((row & (split - 1)) * (kBlockM >> log_s) + (row >> log_s));
+    uint8_t* stage = split > 1 ? smem : red;
     const uint32_t t_row = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < kHalves; ++h) {
       uint32_t v[32];
       tmem_ld32(t_row + h * 32, v);
       tmem_ld_wait();
-      if (m0 + row < args.M) {
+      if (row < valid) {
 #pragma unroll
         for (int c = 0; c < 8; ++c)
-          st_cluster_v4(red_addr + red_offset(slot, h * 8 + c), __uint_as_float(v[4 * c]), __uint_as_float(v[4 * c + 1]),
-                        __uint_as_float(v[4 * c + 2]), __uint_as_float(v[4 * c + 3]));
+          *reinterpret_cast<uint4*>(stage + red_offset<kBlockN>(staged, h * 8 + c, row)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
       }
     }
     tc_fence_before_sync();
+    if (split > 1) {
+      fence_proxy_async_smem();
+      __syncwarp();
+      // this warp's rows of owner `lane`: a contiguous piece of (32 / S) rows, fewer at the end of the matrix
+      const int first = warp * (32 >> log_s);
+      int rows = ((valid - lane + split - 1) >> log_s) - first;
+      if (rows > (32 >> log_s)) rows = 32 >> log_s;
+      if (lane < split && rows > 0)
+        bulk_copy_to_cta(map_to_cta(smem_u32(red + (rank * (kBlockM >> log_s) + first) * kRowBytes), static_cast<uint32_t>(lane)),
+                         smem + (lane * (kBlockM >> log_s) + first) * kRowBytes, static_cast<uint32_t>(rows) * kRowBytes,
+                         map_to_cta(smem_u32(&bars->red_full), static_cast<uint32_t>(lane)));
+    }
   }
   if (split > 1) {
-    cluster_arrive();
-    cluster_wait();
+    if (n_own > 0) mbar_wait_cluster(&bars->red_full, 0, ctl, status, kErrWaitConsumer);
+    __syncwarp();
+    cluster_arrive();                      // this block's rows are complete; see the end
   } else {
     __syncthreads();
   }
@@ -174,16 +199,20 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     float lo[4] = {0.f, 0.f, 0.f, 0.f}, hi[4] = {0.f, 0.f, 0.f, 0.f};
     for (int s = 0; s < split; ++s) {
       const uint32_t r = s * (kBlockM >> log_s) + local;
-      const float4 a = *reinterpret_cast<const float4*>(red + red_offset(r, j));
-      const float4 b = *reinterpret_cast<const float4*>(red + red_offset(r, j + 8));
+      const float4 a = *reinterpret_cast<const float4*>(red + red_offset<kBlockN>(r, j, (local << log_s) + rank));
       lo[0] += a.x; lo[1] += a.y; lo[2] += a.z; lo[3] += a.w;
-      hi[0] += b.x; hi[1] += b.y; hi[2] += b.z; hi[3] += b.w;
+      if constexpr (kHalves == 2) {
+        const float4 b = *reinterpret_cast<const float4*>(red + red_offset<kBlockN>(r, j + 8, (local << log_s) + rank));
+        hi[0] += b.x; hi[1] += b.y; hi[2] += b.z; hi[3] += b.w;
+      }
     }
     const PieceOperands now = ops;
-    if (item + kThreads < n_items) load_operands<kOut>(args, item_row(item + kThreads), ntile, (item + kThreads) & 7, ops);
-    finish_piece<kOut, VT>(args, lo, hi, now, item_row(item), ntile, j, status);
+    if (item + kThreads < n_items) load_operands<kOut, kHalves>(args, item_row(item + kThreads), ntile, (item + kThreads) & 7, ops);
+    finish_piece<kOut, VT, kHalves>(args, lo, hi, now, item_row(item), ntile, j, status);
   }
 
+  __syncwarp();
+  if (split > 1) cluster_wait();        // every block has its rows: nobody's copies still read this block's memory
   __syncthreads();
   if (ctl->abort) __nanosleep(20000);   // copies that may still be in flight get time to land
   if (warp == 5) {
@@ -197,7 +226,7 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 // pair kernels are faster: at K = 512, N = 2048 1024 rows (256 tiles) take 9.1 us here and 10.9 us there, 1500 rows (384
 // tiles) 13.9 against 10.9; at K = 2048, N = 512 3678 rows (232 tiles) 17.1 against 22.1, 5000 rows (320) 27.5 against 22.5.
 bool few_row_tiles(int M, int N) {
-  return static_cast<long long>((M + small::kBlockM - 1) / small::kBlockM) * (N / small::kBlockN) <= 2ll * sm_count();
+  return static_cast<long long>((M + small::kBlockM - 1) / small::kBlockM) * (N / 64) <= 2ll * sm_count();
 }
 
 // Blocks per cluster: as many as keep the grid within one block per SM and divide the K chunks.
@@ -207,8 +236,8 @@ static int choose_split(int tiles, int k_chunks) {
   return s;
 }
 
-template <int kOut, typename VT>
-static int launch_small(const void* a, const void* w, SmallArgs& args, int K, int in_dtype, int* status,
+template <int kOut, typename VT, int kBlockN>
+static int launch_tiles(const void* a, const void* w, SmallArgs& args, int K, int in_dtype, int* status,
                         cudaStream_t st, int dependent) {
   using namespace small;
   CUtensorMap tmap_a, tmap_w;
@@ -221,11 +250,24 @@ static int launch_small(const void* a, const void* w, SmallArgs& args, int K, in
   args.chunks = K / kBlockK / args.split;
   const int fmt = in_dtype == 1 ? 0 : 1;
   const uint32_t idesc = umma_idesc_f16(kBlockM, kBlockN, fmt, fmt, 0, 0);
-  auto kern = linear_small_kernel<kOut, VT>;
-  rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
+  auto kern = linear_small_kernel<kOut, VT, kBlockN>;
+  rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), Tile<kBlockN>::kSmemBytes);
   if (rc != 0) return rc;
-  return launch_kernel(kern, dim3(n_tiles * args.split, m_tiles), kThreads, kSmemBytes, st, args.split, dependent, tmap_a,
+  return launch_kernel(kern, dim3(n_tiles * args.split, m_tiles), kThreads, Tile<kBlockN>::kSmemBytes, st, args.split, dependent, tmap_a,
                        tmap_w, args, idesc, status);
+}
+
+// 64-column tiles, or 32 where 64 would leave the K split at its limit of eight with SMs to spare: the partial sums that
+// cross the cluster are what a split costs (28 KB out of and into every block at eight blocks of 64 columns, about 1.9 us;
+// 14 KB with 32), and halving the tile halves them.
+template <int kOut, typename VT>
+static int launch_small(const void* a, const void* w, SmallArgs& args, int K, int in_dtype, int* status, cudaStream_t st,
+                        int dependent) {
+  if constexpr (kOut != 3) {
+    if (static_cast<long long>((args.M + 127) / 128) * (args.N / 64) * 8 <= sm_count())
+      return launch_tiles<kOut, VT, 32>(a, w, args, K, in_dtype, status, st, dependent);
+  }
+  return launch_tiles<kOut, VT, 64>(a, w, args, K, in_dtype, status, st, dependent);
 }
 
 int launch_linear_small(const void* a, const void* w, void* y, const float* scale, const void* resid, int M, int N, int K,

@@ -6,7 +6,7 @@
 // its eight epilogue warps normalise the rows, one warp per row at a time, straight into the swizzled operand tile, and
 // the whole K = 512 of its weight slice (64 KB) sits in shared memory, requested before the wait for the kernel in front.
 // There is no K split, hence no cluster and no reduction.  Every block repeats the normalisation of its rows (32 or 64 KB
-// of x from L2), which is what limits the rows: beyond 256 the separate LayerNorm kernel is cheaper.
+// of x from L2), which is what limits the rows.
 //
 // The tensor core multiplies 128 rows whatever kRows is; the operand tile of a K chunk is only kRows rows high, so what
 // it reads past them is the next chunk (or the weights): finite or not, those products stay in accumulator rows that
@@ -209,7 +209,7 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       if (lane < kRows) {
 #pragma unroll
         for (int c = 0; c < 8; ++c)
-          *reinterpret_cast<uint4*>(smem_o + small::red_offset(lane, h * 8 + c)) =
+          *reinterpret_cast<uint4*>(smem_o + small::red_offset(lane, h * 8 + c, lane)) =
               make_uint4(a[4 * c], a[4 * c + 1], a[4 * c + 2], a[4 * c + 3]);
       }
     }
@@ -218,8 +218,8 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   __syncthreads();
   if (warp < kWarps && item < n_items) {    // kRows * 8 pieces, one per thread at most
     const int local = item >> 3, j = item & 7;
-    const float4 a = *reinterpret_cast<const float4*>(smem_o + small::red_offset(local, j));
-    const float4 c = *reinterpret_cast<const float4*>(smem_o + small::red_offset(local, j + 8));
+    const float4 a = *reinterpret_cast<const float4*>(smem_o + small::red_offset(local, j, local));
+    const float4 c = *reinterpret_cast<const float4*>(smem_o + small::red_offset(local, j + 8, local));
     float lo[4] = {a.x, a.y, a.z, a.w}, hi[4] = {c.x, c.y, c.z, c.w};
     finish_piece<kOut, VT>(args, lo, hi, ops, m0 + local, ntile, j, status);
   }
@@ -230,10 +230,14 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   }
 }
 
-// 16 rows per block while that leaves at most two blocks per SM, 32 up to 256 rows.
-static int rows_per_block(int M, int N) { return static_cast<long long>((M + 15) / 16) * (N / 64) <= 2ll * sm_count() ? 16 : 32; }
+static long long blocks_for(int M, int N, int rows) { return static_cast<long long>((M + rows - 1) / rows) * (N / lnlin::kBlockN); }
+// 16 rows per block while that is at most one block per SM, else 32; beyond one block per SM of those the separate
+// LayerNorm kernel is cheaper.  More blocks than SMs do not pay: two of them leave no room on an SM for the next kernel's
+// block, which then starts (and asks for its weights) only when they have ended (125 rows: fc2 began 5 us after fc1's
+// first blocks were done instead of 2).
+static int rows_per_block(int M, int N) { return blocks_for(M, N, 16) <= sm_count() ? 16 : 32; }
 
-bool few_rows_with_norm(int M) { return M <= 256; }
+bool few_rows_with_norm(int M, int N) { return blocks_for(M, N, 32) <= sm_count(); }
 
 template <int kIn, int kTc, int kOut, typename VT>
 static int launch_rows(const CUtensorMap& tmap_w, const LnArgs& ln, const SmallArgs& args, uint32_t idesc, int* status,

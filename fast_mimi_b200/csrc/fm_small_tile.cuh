@@ -10,9 +10,11 @@
 namespace fm {
 
 namespace small {
-// 16-byte piece `c` (0..15) of row `r` of the reduction buffer; the low three bits are permuted by the row so that
-// eight lanes with consecutive rows (writing) or consecutive pieces (reading) touch eight different bank groups.
-__device__ __forceinline__ uint32_t red_offset(uint32_t r, uint32_t c) { return r * 256u + ((c ^ (r & 7u)) << 4); }
+// 16-byte piece `c` of FP32 row `r` of 64 (or 32) columns; the low three bits are permuted by `key`, the row's number in
+// the tile, so that eight lanes with consecutive rows (writing) or consecutive pieces (reading) touch eight different
+// bank groups.
+template <int kCols = 64>
+__device__ __forceinline__ uint32_t red_offset(uint32_t r, uint32_t c, uint32_t key) { return r * (kCols * 4u) + ((c ^ (key & 7u)) << 4); }
 }  // namespace small
 
 struct SmallArgs {
@@ -27,14 +29,15 @@ struct SmallArgs {
 
 // What the epilogue of eight values of row `row` of output tile `ntile` (64 columns, one attention head) reads besides the
 // product: columns 4j .. 4j + 3 ([0]) and 32 + 4j .. ([1]), the two halves of RoPE pairs.  Asked for before the product
-// is complete, so that its latency does not follow the reduction's.
+// is complete, so that its latency does not follow the reduction's.  With tiles of 32 columns (kHalves 1) a piece is four
+// values.
 // kOut: 0 = BF16, 1 = FP16, 2 = FP32 output and residual; 3 = q | k | v with RoPE.
 struct PieceOperands {
   float4 a[2];            // residual, or cos and sin
   float4 s[2];            // per-channel scale
 };
 
-template <int kOut>
+template <int kOut, int kHalves = 2>
 __device__ __forceinline__ void load_operands(const SmallArgs& args, int row, int ntile, int j, PieceOperands& p) {
   if constexpr (kOut == 3) {
     if (ntile < 16) {     // q and k
@@ -45,10 +48,10 @@ __device__ __forceinline__ void load_operands(const SmallArgs& args, int row, in
       p.a[1] = *reinterpret_cast<const float4*>(ep.sin + at);
     }
   } else {
-    const int col = ntile * 64 + 4 * j;
+    const int col = ntile * 32 * kHalves + 4 * j;
     const long long at = static_cast<long long>(row) * args.N + col;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < kHalves; ++h) {
       p.s[h] = args.scale != nullptr ? __ldg(reinterpret_cast<const float4*>(args.scale + col + 32 * h)) : make_float4(1.f, 1.f, 1.f, 1.f);
       p.a[h] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (args.resid != nullptr) {
@@ -66,7 +69,7 @@ __device__ __forceinline__ void load_operands(const SmallArgs& args, int row, in
 }
 
 // The epilogue itself: lo and hi are the product's columns 4j .. and 32 + 4j ..
-template <int kOut, typename VT>
+template <int kOut, typename VT, int kHalves = 2>
 __device__ __forceinline__ void finish_piece(const SmallArgs& args, float (&lo)[4], float (&hi)[4], const PieceOperands& p,
                                              int row, int ntile, int j, int* status) {
   if constexpr (kOut == 3) {
@@ -106,14 +109,14 @@ __device__ __forceinline__ void finish_piece(const SmallArgs& args, float (&lo)[
       }
     }
   } else {
-    const long long at = static_cast<long long>(row) * args.N + ntile * 64 + 4 * j;
+    const long long at = static_cast<long long>(row) * args.N + ntile * 32 * kHalves + 4 * j;
     float* part[2] = {lo, hi};
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < kHalves; ++h) {
       float* v = part[h];
       if (args.gelu) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = gelu_erf(v[e]);
+        gelu_erf2(v[0], v[1]);
+        gelu_erf2(v[2], v[3]);
       }
       if (args.scale != nullptr) {
         v[0] *= p.s[h].x; v[1] *= p.s[h].y; v[2] *= p.s[h].z; v[3] *= p.s[h].w;

@@ -13,9 +13,12 @@
 // up to three items in flight) and two groups of four warps take them in turn.  What limited the earlier forms was not
 // the copy but the arithmetic around it: a dot product per lane, its conversions and shuffles cost 6400 warp instructions
 // per item, half of the SM's issue slots at full bandwidth.  Here each warp multiplies its 64 slots with mma.sync
-// (m16n8k16, queries as rows, FP32 accumulation): about 600 instructions per item, the same for one query as for eight,
-// so a call of up to eight frames costs the ring's bytes once.  Probabilities stay FP32-grade: they enter P V as the sum
-// of two 16-bit parts.  (tcgen05 would need 128 rows and tensor-memory round trips for at most 8 queries.)
+// (m16n8k16, FP32 accumulation): about 400 instructions per item, the same for one query as for eight, so a call of up to
+// eight frames costs the ring's bytes once.  Keys and dimensions are the 16 rows of a product and the eight queries its
+// columns: with the queries as rows half of every product was padding, and the chain of products (8 cycles each, 21 when
+// one waits for the one before) was what a warp spent its time on (1024 streams, eight layers: 1082 us against 964).
+// Probabilities stay FP32-grade: they enter P V as the sum of two 16-bit parts.  (tcgen05 would need 128 rows
+// and tensor-memory round trips for at most 8 queries.)
 //
 // Rows that are already in the ring do not depend on the projection, so in a chain of dependent launches the first items
 // are requested before the wait for it.  A block has an item's ring rows in shared memory before it stores that item's
@@ -25,6 +28,7 @@
 #include "fm_common.cuh"
 #include "fm_kernels.h"
 #include "fm_launch.h"
+#include "fm_warp_mma.cuh"
 
 namespace fm {
 
@@ -49,25 +53,6 @@ constexpr int smem_bytes(int stages) {
 }
 static_assert(smem_bytes(kMaxStages) <= 232448, "exceeds the 227 KB a block may use");
 
-__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-// c (rows 0-7 of the 16 x 8 tile; rows 8-15 carry no query) += a[16 x 16] b[16 x 8]
-template <typename T>
-__device__ __forceinline__ void mma_rows8(float (&c)[2], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
-  float z0 = 0.f, z1 = 0.f;
-  if constexpr (std::is_same<T, __half>::value)
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(z0), "+f"(z1) : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
-  else
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(z0), "+f"(z1) : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
-}
 // x, y as hi + lo, both parts of type T
 template <typename T>
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& lo) {
@@ -141,7 +126,7 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   } else {
     griddep_wait();
     const int cg = warp / kGroupWarps, gw = warp % kGroupWarps, gt = threadIdx.x - cg * kGroupWarps * 32;
-    const int g = lane >> 2, cpair = (lane & 3) * 2;     // mma fragments: query row g; columns cpair, cpair + 1
+    const int g = lane >> 2, cpair = (lane & 3) * 2;     // mma fragments
     uint8_t* new_k = smem_new + cg * kNewBytes;
     uint8_t* new_v = new_k + kNewBytes / 2;
     float* merge = smem_merge + cg * (kMergeBytes / 4);
@@ -172,9 +157,9 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         }
       }
     };
-    auto take = [&](uint32_t (&qa)[4][2], uint4 (&nk)[2], uint4 (&nv)[2]) {
+    auto take = [&](uint32_t (&qb)[4][2], uint4 (&nk)[2], uint4 (&nv)[2]) {
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks) { qa[ks][0] = q_next[ks][0]; qa[ks][1] = q_next[ks][1]; }
+      for (int ks = 0; ks < 4; ++ks) { qb[ks][0] = q_next[ks][0]; qb[ks][1] = q_next[ks][1]; }
 #pragma unroll
       for (int e = 0; e < 2; ++e) { nk[e] = k_next[e]; nv[e] = v_next[e]; }
     };
@@ -185,9 +170,9 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
       const int st = n % a.stages;
       const int s = static_cast<int>(item >> 3), h = static_cast<int>(item & 7);
       const size_t new0 = static_cast<size_t>(s) * a.T * 512 + h * 64;
-      uint32_t qa[4][2];
+      uint32_t qb[4][2];
       uint4 nk[2], nv[2];
-      take(qa, nk, nv);
+      take(qb, nk, nv);
       if (item + static_cast<long long>(kGroups) * gridDim.x < a.n_items)
         fetch(item + static_cast<long long>(kGroups) * gridDim.x);
       if (a.n_loaded > 0) mbar_wait(&c->full[st], static_cast<uint32_t>(n / a.stages) & 1u, ctl, status, kErrWaitTma);
@@ -231,93 +216,107 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         }
       }
 
-      // ---- scores of this warp's eight (nine: with the new rows) 8-key tiles
-      const int n_tiles = a.n_loaded > slot0 ? (a.n_loaded - slot0 + 7) >> 3 : 0;     // of eight
-      float sc[10][2];
-      float m = -INFINITY;
-      const int lo = a.delta + g - a.window + 1, hi = a.delta + g;                    // visible rows of query g
+      // ---- scores, keys as rows: four tiles of 16 keys, and the new rows as a fifth for the group's last warp
+      const int n_tiles = a.n_loaded > slot0 ? (a.n_loaded - slot0 + 15) >> 4 : 0;    // of four
+      const bool has_new = gw == kGroupWarps - 1;
+      auto in_use = [&](int mt) { return mt < 4 ? mt < n_tiles : has_new; };          // the same for the whole warp
+      float sc[5][4];                                   // keys g (two queries) and g + 8 of each tile
 #pragma unroll
-      for (int nt = 0; nt < 10; ++nt) {
-        sc[nt][0] = sc[nt][1] = -INFINITY;
-        const bool fresh = nt >= 8;
-        if (fresh ? (gw == kGroupWarps - 1 && nt == 8) : nt < n_tiles) {              // the same for the whole warp
-          // x4: keys lane % 8 of the tile, dimensions 8 (lane / 8) .. of the first, then of the second half
-          const int key = fresh ? (lane & 7) : slot0 + nt * 8 + (lane & 7);
-          const uint32_t base = smem_u32(fresh ? new_k : tile_k);
-          uint32_t b01[4], b23[4];
-          ldmatrix4(b01, base + sw128_offset(key, lane >> 3));
-          ldmatrix4(b23, base + sw128_offset(key, 4 + (lane >> 3)));
-          float acc[2] = {0.f, 0.f};
-          mma_rows8<__nv_bfloat16>(acc, qa[0][0], qa[0][1], b01[0], b01[1]);
-          mma_rows8<__nv_bfloat16>(acc, qa[1][0], qa[1][1], b01[2], b01[3]);
-          mma_rows8<__nv_bfloat16>(acc, qa[2][0], qa[2][1], b23[0], b23[1]);
-          mma_rows8<__nv_bfloat16>(acc, qa[3][0], qa[3][1], b23[2], b23[3]);
+      for (int mt = 0; mt < 5; ++mt) sc[mt][0] = sc[mt][1] = sc[mt][2] = sc[mt][3] = 0.f;
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            int r;
-            if (fresh) {
-              r = a.delta + cpair + e;
-            } else {
-              const int j = slot0 + nt * 8 + cpair + e;
-              r = j - first;
-              if (r < 0) r += a.slots;
-              if (j >= a.n_loaded || r >= a.delta) r = -1 << 20;
-            }
-            if (r >= lo && r <= hi && r >= 0) sc[nt][e] = acc[e] * a.scale_log2e;
-            m = fmaxf(m, sc[nt][e]);
+      for (int ks = 0; ks < 4; ++ks) {
+#pragma unroll
+        for (int mt = 0; mt < 5; ++mt) {
+          if (in_use(mt)) {
+            uint32_t ka[4];                             // keys lane % 16, dimensions 16 ks + 8 (lane / 16) ..
+            ldmatrix4(ka, smem_u32(mt < 4 ? tile_k : new_k) + sw128_offset((mt < 4 ? slot0 + mt * 16 : 0) + (lane & 15), 2 * ks + (lane >> 4)));
+            mma_16x8x16<__nv_bfloat16>(sc[mt], ka, qb[ks][0], qb[ks][1]);
           }
         }
       }
-      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-      const float m_use = m == -INFINITY ? 0.f : m;
-      float l = 0.f;
+      // visible rows of query t: delta + t - window < r <= delta + t
+      float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll
-      for (int nt = 0; nt < 10; ++nt) {
+      for (int mt = 0; mt < 5; ++mt) {
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          sc[nt][e] = ex2_approx(sc[nt][e] - m_use);
-          l += sc[nt][e];
+        for (int e = 0; e < 4; ++e) {
+          const int key = g + 8 * (e >> 1), t = cpair + (e & 1);
+          int r;
+          if (mt == 4) {
+            r = a.delta + key;
+          } else {
+            const int j = slot0 + mt * 16 + key;
+            r = j - first;
+            if (r < 0) r += a.slots;
+            if (j >= a.n_loaded || r >= a.delta) r = -(1 << 28);
+          }
+          const bool seen = in_use(mt) && r <= a.delta + t && r > a.delta + t - a.window;
+          sc[mt][e] = seen ? sc[mt][e] * a.scale_log2e : -INFINITY;
+          m[e & 1] = fmaxf(m[e & 1], sc[mt][e]);
         }
       }
-      l += __shfl_xor_sync(0xffffffffu, l, 1);
-      l += __shfl_xor_sync(0xffffffffu, l, 2);
+      float m_use[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+#pragma unroll
+        for (int x = 4; x < 32; x <<= 1) m[e] = fmaxf(m[e], __shfl_xor_sync(0xffffffffu, m[e], x));
+        m_use[e] = m[e] == -INFINITY ? 0.f : m[e];
+      }
+#pragma unroll
+      for (int mt = 0; mt < 5; ++mt) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          sc[mt][e] = ex2_approx(sc[mt][e] - m_use[e & 1]);
+          l[e & 1] += sc[mt][e];
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+#pragma unroll
+        for (int x = 4; x < 32; x <<= 1) l[e] += __shfl_xor_sync(0xffffffffu, l[e], x);
+      }
 
-      // ---- O = P V, 16 keys per step
-      float o[8][2];
+      // ---- O^T = V^T P^T, 16 keys per step, dimensions as rows.  A score fragment has keys along the lanes' groups and
+      // queries inside them; as an operand it must be the other way round (movmatrix).
+      float o[4][4];                                    // dimensions 16 d + g and + 8, two queries each
 #pragma unroll
-      for (int d = 0; d < 8; ++d) o[d][0] = o[d][1] = 0.f;
+      for (int d = 0; d < 4; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f;
 #pragma unroll
-      for (int ks = 0; ks < 5; ++ks) {
-        const bool fresh = ks == 4;
-        if (fresh ? gw == kGroupWarps - 1 : 2 * ks < n_tiles) {
+      for (int mt = 0; mt < 5; ++mt) {
+        if (in_use(mt)) {
           uint32_t h0, l0, h1, l1;
-          split_pair<VT>(sc[2 * ks][0], sc[2 * ks][1], h0, l0);
-          split_pair<VT>(sc[2 * ks + 1][0], sc[2 * ks + 1][1], h1, l1);
-          const int key = (fresh ? 0 : slot0 + ks * 16) + (lane & 15);
-          const uint32_t base = smem_u32(fresh ? new_v : tile_v);
+          split_pair<VT>(sc[mt][0], sc[mt][1], h0, l0);
+          split_pair<VT>(sc[mt][2], sc[mt][3], h1, l1);
+          h0 = movmatrix_trans(h0); h1 = movmatrix_trans(h1);
+          l0 = movmatrix_trans(l0); l1 = movmatrix_trans(l1);
+          const uint32_t base = smem_u32(mt < 4 ? tile_v : new_v);
+          const int key = (mt < 4 ? slot0 + mt * 16 : 0) + (lane & 7) + ((lane >> 4) << 3);
+          uint32_t va[4][4];
 #pragma unroll
-          for (int dp = 0; dp < 4; ++dp) {               // 16 dimensions: two 8-wide column tiles
-            uint32_t b[4];
-            ldmatrix4_trans(b, base + sw128_offset(key, dp * 2 + (lane >> 4)));
-            mma_rows8<VT>(o[2 * dp], h0, h1, b[0], b[1]);
-            mma_rows8<VT>(o[2 * dp], l0, l1, b[0], b[1]);
-            mma_rows8<VT>(o[2 * dp + 1], h0, h1, b[2], b[3]);
-            mma_rows8<VT>(o[2 * dp + 1], l0, l1, b[2], b[3]);
-          }
+          for (int d = 0; d < 4; ++d) ldmatrix4_trans(va[d], base + sw128_offset(key, 2 * d + ((lane >> 3) & 1)));
+#pragma unroll
+          for (int d = 0; d < 4; ++d) mma_16x8x16<VT>(o[d], va[d], h0, h1);
+#pragma unroll
+          for (int d = 0; d < 4; ++d) mma_16x8x16<VT>(o[d], va[d], l0, l1);
         }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&c->empty[st]);         // this warp's reads of the stage are done
 
       // ---- four-way merge
-      if (g < a.T) {
 #pragma unroll
-        for (int d = 0; d < 8; ++d)
-          *reinterpret_cast<float2*>(merge + (gw * kMaxT + g) * 64 + d * 8 + cpair) = make_float2(o[d][0], o[d][1]);
-        if ((lane & 3) == 0) {
-          c->m[cg][gw][g] = m;
-          c->l[cg][gw][g] = l;
+      for (int e = 0; e < 2; ++e) {
+        const int t = cpair + e;
+        if (t < a.T) {
+#pragma unroll
+          for (int d = 0; d < 4; ++d) {
+            merge[(gw * kMaxT + t) * 64 + d * 16 + g] = o[d][e];
+            merge[(gw * kMaxT + t) * 64 + d * 16 + 8 + g] = o[d][2 + e];
+          }
+          if (g == 0) {
+            c->m[cg][gw][t] = m[e];
+            c->l[cg][gw][t] = l[e];
+          }
         }
       }
       named_bar_sync(1 + cg, kGroupWarps * 32);
