@@ -32,7 +32,10 @@ constexpr int kThreads = (kGroups * kWarps + 1) * 32;
 constexpr int kRowBytes = 128;
 
 struct Ctl {
-  uint64_t full[kStages];
+  // One "loaded" barrier per stage and group (item n: n % (2 stages)), so that one group waits for all its phases: shared
+  // by the groups in turn, a group done with item n - 2 before item n - 3 has landed would take a phase of the same parity
+  // for its own.
+  uint64_t full[kStages * kGroups];
   uint64_t empty[kStages];
   CtaCtl ctl;
   alignas(16) uint16_t qrow[kStages][64];   // the item's 64 query values, copied in with its ring slices
@@ -130,10 +133,8 @@ ring_decode_attn_kernel(const uint16_t* __restrict__ q, const uint16_t* __restri
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kStages; ++i) {
-      mbar_init(&c->full[i], 1);
-      mbar_init(&c->empty[i], kWarps);
-    }
+    for (int i = 0; i < kStages * kGroups; ++i) mbar_init(&c->full[i], 1);
+    for (int i = 0; i < kStages; ++i) mbar_init(&c->empty[i], kWarps);
     c->ctl.abort = 0;
     fence_mbar_init();
   }
@@ -161,11 +162,12 @@ ring_decode_attn_kernel(const uint16_t* __restrict__ q, const uint16_t* __restri
         const uint32_t use = static_cast<uint32_t>(n / kStages);
         mbar_wait(&c->empty[st], (use & 1u) ^ 1u, ctl, status, kErrWaitConsumer);
         const uint32_t bytes = static_cast<uint32_t>(valid_slots(item)) * kRowBytes;
-        mbar_arrive_expect_tx(&c->full[st], 2 * bytes + 128);
-        bulk_load_1d(&c->qrow[st][0], q + static_cast<size_t>(item) * 64, 128, &c->full[st]);
+        uint64_t* full = &c->full[n % (kStages * kGroups)];
+        mbar_arrive_expect_tx(full, 2 * bytes + 128);
+        bulk_load_1d(&c->qrow[st][0], q + static_cast<size_t>(item) * 64, 128, full);
         const size_t src = static_cast<size_t>(item) * ring_slots * 64;
-        bulk_load_1d(stage_base + (2 * st) * tile_bytes, ring_k + src, bytes, &c->full[st]);
-        bulk_load_1d(stage_base + (2 * st + 1) * tile_bytes, ring_v + src, bytes, &c->full[st]);
+        bulk_load_1d(stage_base + (2 * st) * tile_bytes, ring_k + src, bytes, full);
+        bulk_load_1d(stage_base + (2 * st + 1) * tile_bytes, ring_v + src, bytes, full);
       }
     }
   } else {
@@ -178,10 +180,9 @@ ring_decode_attn_kernel(const uint16_t* __restrict__ q, const uint16_t* __restri
     for (long long item = blockIdx.x + static_cast<long long>(cg) * gridDim.x; item < n_items;
          item += static_cast<long long>(kGroups) * gridDim.x, n += kGroups) {
       const int st = n % kStages;
-      const uint32_t use = static_cast<uint32_t>(n / kStages);
       const int nv = valid_slots(static_cast<int>(item));
       const int s = static_cast<int>(item >> 3), h = static_cast<int>(item & 7);
-      mbar_wait(&c->full[st], use & 1u, ctl, status, kErrWaitTma);
+      mbar_wait(&c->full[n % (kStages * kGroups)], static_cast<uint32_t>(n / (kStages * kGroups)) & 1u, ctl, status, kErrWaitTma);
       const uint8_t* ks = stage_base + (2 * st) * tile_bytes;
       const uint8_t* vs = stage_base + (2 * st + 1) * tile_bytes;
       float qf[8];

@@ -42,7 +42,11 @@ constexpr int kStageBytes = 2 * kTileBytes;
 constexpr int kNewBytes = 2 * 16 * 128;               // new K and V rows of a group's item, padded to 16
 constexpr int kMergeBytes = kGroupWarps * kMaxT * 64 * 4;
 struct Ctl {
-  uint64_t full[kMaxStages];
+  // One "loaded" barrier per stage AND group: item n has barrier n % (2 stages), so that its phases are all waited for by
+  // one group.  With one per stage and three stages the groups took a barrier's phases in turn, and a group that was done
+  // with item n - 2 while item n - 3 was still on its way took the phase before that one for its own (the parity of a
+  // phase cannot tell the one two before from it): it read, and gave back, a stage that was being filled.
+  uint64_t full[kMaxStages * kGroups];
   uint64_t empty[kMaxStages];
   CtaCtl ctl;
   float m[kGroups][kGroupWarps][kMaxT];
@@ -88,9 +92,9 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < a.stages; ++i) {
-      mbar_init(&c->full[i], 1);
       mbar_init(&c->empty[i], kGroupWarps);
     }
+    for (int i = 0; i < kGroups * a.stages; ++i) mbar_init(&c->full[i], 1);
     c->ctl.abort = 0;
     fence_mbar_init();
   }
@@ -116,9 +120,10 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         for (int item = blockIdx.x; item < a.n_items; item += gridDim.x, ++n) {
           const int st = n % a.stages;
           mbar_wait(&c->empty[st], (static_cast<uint32_t>(n / a.stages) & 1u) ^ 1u, ctl, status, kErrWaitConsumer);
-          mbar_arrive_expect_tx(&c->full[st], 2u * static_cast<uint32_t>(a.n_loaded) * 128u);
-          tma_load_2d(smem + st * kStageBytes, &tmap_k, &c->full[st], 0, item * a.slots);
-          tma_load_2d(smem + st * kStageBytes + kTileBytes, &tmap_v, &c->full[st], 0, item * a.slots);
+          uint64_t* full = &c->full[n % (kGroups * a.stages)];
+          mbar_arrive_expect_tx(full, 2u * static_cast<uint32_t>(a.n_loaded) * 128u);
+          tma_load_2d(smem + st * kStageBytes, &tmap_k, full, 0, item * a.slots);
+          tma_load_2d(smem + st * kStageBytes + kTileBytes, &tmap_v, full, 0, item * a.slots);
         }
       }
       griddep_wait();
@@ -175,7 +180,8 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
       take(qb, nk, nv);
       if (item + static_cast<long long>(kGroups) * gridDim.x < a.n_items)
         fetch(item + static_cast<long long>(kGroups) * gridDim.x);
-      if (a.n_loaded > 0) mbar_wait(&c->full[st], static_cast<uint32_t>(n / a.stages) & 1u, ctl, status, kErrWaitTma);
+      if (a.n_loaded > 0)
+        mbar_wait(&c->full[n % (kGroups * a.stages)], static_cast<uint32_t>(n / (kGroups * a.stages)) & 1u, ctl, status, kErrWaitTma);
       uint8_t* tile_k = smem + st * kStageBytes;
       uint8_t* tile_v = tile_k + kTileBytes;
       if (gw == kGroupWarps - 1) {

@@ -91,3 +91,40 @@ def test_layer_follows_its_parameters():
     before = run()
     layer.self_attn.sliding_window = 4
     assert not torch.equal(run(), before)
+
+
+@pytest.mark.parametrize("streams", [38, 64, 333, 700])
+def test_many_streams_repeat_exactly(streams):
+    """More (stream, head) items than two per SM: three ring slices are in flight per block and its two groups of warps take
+    them in turn.  Which slice lands first must not matter: the same call repeats bit for bit, and its first and last streams
+    are those of a call by themselves (one item per block)."""
+    import fast_mimi_b200 as fm
+    g = torch.Generator(device="cuda").manual_seed(streams)
+    w = (torch.randn(1536, 512, device="cuda", generator=g) * 0.04).bfloat16()
+    x = torch.randn(streams, 512, device="cuda", generator=g).bfloat16()
+    ring_k = torch.randn(streams, 8, 250, 64, device="cuda", generator=g).bfloat16()
+    ring_v = torch.randn(streams, 8, 250, 64, device="cuda", generator=g).half()
+    layer = fm.MimiTransformerLayerB200().cuda()
+    cos, sin = fm.rope_tables(torch.arange(700, 701, device="cuda")[None])
+    some = [0, 1, streams - 1]
+
+    def step(rows):
+        k, v = ring_k[rows].clone(), ring_v[rows].clone()
+        return fm.ops.decode_step(x[rows].contiguous(), w, cos, sin, k, v, 700), k, v
+
+    def whole(rows):
+        ring = fm.MimiKVRing(1, len(rows), 250)
+        ring.ring_k.copy_(ring_k[rows][None])
+        ring.ring_v.copy_(ring_v[rows][None])
+        ring.advance(0, 700)
+        return layer(x[rows].float()[:, None], None, ring, (cos, sin))[0], ring.ring_k[0], ring.ring_v[0]
+
+    every = list(range(streams))
+    for call, bar in ((step, 1e-3), (whole, 1e-4)):
+        first = call(every)
+        for _ in range(20):
+            for a, b in zip(call(every), first):
+                assert torch.equal(a, b)
+        for a, b in zip(call(some), first):
+            assert O.rel_l2(a.double(), b[some].double()) < bar            # other splits of K: FP32 sums in another order
+    fm.check_status()
