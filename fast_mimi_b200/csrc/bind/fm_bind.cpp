@@ -78,6 +78,13 @@ int plan_clear(PyObject* self_obj) {
   return 0;
 }
 
+// What a tensor's contents are known by.  Throws for tensors without storage (wrappers of transforms) and without a version
+// counter (made in inference mode): such a one cannot be watched.
+void stamp(const at::Tensor& t, const void** data, uint32_t* version) {
+  *data = t.const_data_ptr();
+  *version = static_cast<uint32_t>(t._version());
+}
+
 // LayerPlan(watches, keep, params_address, status, like, value_like): watches is a list of (dict, key); keep the tensors
 // behind the parameter block at params_address (copied); status an int32 tensor; like / value_like tensors whose type and
 // device activations / ring values must have.
@@ -113,10 +120,12 @@ PyObject* plan_new(PyTypeObject* type, PyObject* args, PyObject*) {
       return nullptr;
     }
     Watch w = {dict, key, value, THPVariable_Check(value), nullptr, 0};
-    if (w.tensor) {
-      const at::Tensor& t = THPVariable_Unpack(value);
-      w.data = t.const_data_ptr();
-      w.version = static_cast<uint32_t>(t._version());
+    try {
+      if (w.tensor) stamp(THPVariable_Unpack(value), &w.data, &w.version);
+    } catch (const std::exception&) {
+      PyErr_SetObject(PyExc_KeyError, key);
+      Py_DECREF(self);
+      return nullptr;
     }
     Py_INCREF(dict);
     Py_INCREF(key);
@@ -133,8 +142,10 @@ bool unchanged(const LayerPlan* plan) {
       return false;
     }
     if (w.tensor) {
-      const at::Tensor& t = THPVariable_Unpack(w.value);
-      if (t.const_data_ptr() != w.data || static_cast<uint32_t>(t._version()) != w.version) return false;
+      const void* data;
+      uint32_t version;
+      stamp(THPVariable_Unpack(w.value), &data, &version);
+      if (data != w.data || version != w.version) return false;
     }
   }
   return true;
@@ -143,7 +154,7 @@ bool unchanged(const LayerPlan* plan) {
 PyTypeObject plan_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
 // layer_forward(plan, x, cos, sin, ring_k, ring_v, past) -> tensor, or None: not the ordinary case
-PyObject* layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+PyObject* layer_forward_checked(PyObject* const* a, Py_ssize_t n) {
   if (n != 7 || !PyObject_TypeCheck(a[0], &plan_type)) {
     PyErr_SetString(PyExc_TypeError, "layer_forward(plan, x, cos, sin, ring_k, ring_v, past)");
     return nullptr;
@@ -178,29 +189,36 @@ PyObject* layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     past = static_cast<int>(p);
   }
   if (!unchanged(plan)) Py_RETURN_NONE;
+  const fm_layer_params& q = plan->params;
+  const int64_t elem = static_cast<int64_t>(x.element_size());
+  int64_t bytes = B * T * (2048 + 512 * elem + (2 * q.ffn > 3072 ? 2 * q.ffn : 3072)) + 4096;
+  if (ring_k != nullptr) bytes += 2048 * B * ((past < q.window - 1 ? past : q.window - 1) + T);
+  const at::Tensor workspace = at::empty({bytes}, x.options().dtype(at::kByte));
+  at::Tensor y = at::empty(x.sizes(), x.options());
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+  const long long bstride = cos.size(0) == 1 ? 0 : T * 64;
+  // every address before the interpreter lock is given up: what has none throws
+  const void* x_data = x.const_data_ptr();
+  const float *cos_data = cos.const_data_ptr<float>(), *sin_data = sin.const_data_ptr<float>();
+  void *y_data = y.data_ptr(), *space = workspace.data_ptr();
   int rc = 0;
-  at::Tensor y;
-  try {
-    const fm_layer_params& q = plan->params;
-    const int64_t elem = static_cast<int64_t>(x.element_size());
-    int64_t bytes = B * T * (2048 + 512 * elem + (2 * q.ffn > 3072 ? 2 * q.ffn : 3072)) + 4096;
-    if (ring_k != nullptr) bytes += 2048 * B * ((past < q.window - 1 ? past : q.window - 1) + T);
-    const at::Tensor workspace = at::empty({bytes}, x.options().dtype(at::kByte));
-    y = at::empty(x.sizes(), x.options());
-    cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
-    const long long bstride = cos.size(0) == 1 ? 0 : T * 64;
-    Py_BEGIN_ALLOW_THREADS
-    rc = fm_layer_forward(&q, x.const_data_ptr(), y.data_ptr(), workspace.data_ptr(), bytes, cos.const_data_ptr<float>(),
-                          sin.const_data_ptr<float>(), bstride, static_cast<int>(B), static_cast<int>(T), ring_k, ring_v, past,
-                          slots, plan->status, stream);
-    Py_END_ALLOW_THREADS
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  Py_BEGIN_ALLOW_THREADS
+  rc = fm_layer_forward(&q, x_data, y_data, space, bytes, cos_data, sin_data, bstride, static_cast<int>(B), static_cast<int>(T),
+                        ring_k, ring_v, past, slots, plan->status, stream);
+  Py_END_ALLOW_THREADS
   if (rc != 0) return PyLong_FromLong(rc);
   plan->params.weights_settled = 1;
   return THPVariable_Wrap(std::move(y));
+}
+
+// No C++ exception leaves the module: whatever threw did so before the launch, and the Python side runs into it again and
+// raises it in its own type (out of memory, tensors without storage).
+PyObject* layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  try {
+    return layer_forward_checked(a, n);
+  } catch (const std::exception&) {
+    Py_RETURN_NONE;
+  }
 }
 
 PyMethodDef methods[] = {

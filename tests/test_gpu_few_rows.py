@@ -128,3 +128,18 @@ def test_many_streams_repeat_exactly(streams):
         for a, b in zip(call(some), first):
             assert O.rel_l2(a.double(), b[some].double()) < bar            # other splits of K: FP32 sums in another order
     fm.check_status()
+
+
+def test_layer_with_parameters_that_cannot_be_watched():
+    """LayerNorm parameters made in inference mode have no version counter: the call works without a plan."""
+    import fast_mimi_b200 as fm
+    layer = fm.MimiTransformerLayerB200().cuda()
+    p = _layer_params(4)
+    layer.load_state_dict(p)
+    with torch.inference_mode():
+        layer.input_layernorm.weight = torch.nn.Parameter(p["input_layernorm.weight"].cuda(), requires_grad=False)
+    x = torch.randn(1, 20, 512)
+    cs = fm.rope_tables(torch.arange(20, device="cuda")[None])
+    for _ in range(2):
+        got, _ = layer(x.cuda(), None, None, cs)
+        assert O.rel_l2(got.cpu() - x, O.transformer_layer(x, p) - x) < 2e-3
