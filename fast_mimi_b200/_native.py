@@ -22,7 +22,7 @@ class LayerParams(ctypes.Structure):
     """``fm_layer_params`` of the header."""
     _fields_ = [("ln1_weight", _P), ("ln1_bias", _P), ("w_qkv", _P), ("w_o", _P), ("attn_scale", _P), ("ln2_weight", _P),
                 ("ln2_bias", _P), ("w_fc1", _P), ("w_fc2", _P), ("mlp_scale", _P), ("ln1_eps", _F), ("ln2_eps", _F),
-                ("scale", _F), ("window", _I), ("stream_dtype", _I), ("value_dtype", _I), ("ffn", _I), ("weights_settled", _I)]
+                ("scale", _F), ("window", _I), ("stream_dtype", _I), ("value_dtype", _I), ("ffn", _I), ("weights_settled", _I), ("vec_dtype", _I)]
 
 
 #: name -> argtypes, in header order.  tests/test_host_logic.py checks this table against the header.

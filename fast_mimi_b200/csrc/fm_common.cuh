@@ -550,4 +550,22 @@ template <> struct Pack16<__nv_bfloat16> {
   }
 };
 
+// A vector of per-channel parameters (LayerNorm weight and bias, layer scale) in the type that the module keeps it in, read
+// where it lies: a converted copy would have to be kept in step with the module.  Type: 0 BF16, 1 FP16, 2 FP32.
+struct ParamVec {
+  const void* data;
+  int type;
+  ParamVec() = default;
+  __host__ __device__ ParamVec(const float* p) : data(p), type(2) {}
+  __host__ __device__ ParamVec(const void* p, int t) : data(p), type(t) {}
+  // values i .. i + 3, i a multiple of 4
+  __device__ __forceinline__ float4 load4(int i) const {
+    if (type == 2) return __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(data) + i));
+    const uint2 u = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(data) + i));
+    const float2 a = type == 1 ? Pack16<__half>::unpack(u.x) : Pack16<__nv_bfloat16>::unpack(u.x);
+    const float2 b = type == 1 ? Pack16<__half>::unpack(u.y) : Pack16<__nv_bfloat16>::unpack(u.y);
+    return make_float4(a.x, a.y, b.x, b.y);
+  }
+};
+
 }  // namespace fm

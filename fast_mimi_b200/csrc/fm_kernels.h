@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fm_common.cuh"
+
 namespace fm {
 
 // Where the projection epilogue puts its results.  Linear outputs are [M, 512] 16-bit tensors
@@ -60,23 +62,23 @@ int launch_out_proj_gemm(const void* a, const void* w, void* y, const float* out
                          int dtype_flags, int* status, cudaStream_t st);
 // y[M,N] = resid + scale * act(a[M,K] * w[N,K]^T); in_dtype 0 BF16 / 1 FP16; out_dtype 0 BF16 / 1 FP16 / 2 FP32
 // (type of y and resid); gelu 1 = exact GELU.  N a multiple of 256, K a multiple of 64.
-int launch_linear_gemm(const void* a, const void* w, void* y, const float* scale, const void* resid, int M, int N,
+int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N,
                        int K, int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent = 0);
 // The same two products for few rows (fm_linear_small.cu): 128 x 64 tiles, K split over a cluster.
 bool few_row_tiles(int M, int N);
 // LayerNorm folded into the product behind it (fm_ln_linear.cu) while one wave of blocks holds the rows: the chain-opening QKV projection and
 // gelu(LayerNorm(x) W^T).
 bool few_rows_with_norm(int M, int N);
-int launch_ln_qkv(const void* x, int x_dtype, const float* weight, const float* bias, float eps, const void* w_qkv,
+int launch_ln_qkv(const void* x, int x_dtype, ParamVec weight, ParamVec bias, float eps, const void* w_qkv,
                   const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status, cudaStream_t st, int dependent);
-int launch_ln_linear_gelu(const void* x, int x_dtype, const float* weight, const float* bias, float eps, const void* w, void* y,
+int launch_ln_linear_gelu(const void* x, int x_dtype, ParamVec weight, ParamVec bias, float eps, const void* w, void* y,
                           int M, int N, int tc_fp16, int* status, cudaStream_t st, int dependent);
-int launch_linear_small(const void* a, const void* w, void* y, const float* scale, const void* resid, int M, int N, int K,
+int launch_linear_small(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N, int K,
                         int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent);
 int launch_qkv_small(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status,
                      cudaStream_t st, int dependent);
 // LayerNorm over 512 channels; x_dtype 0 BF16 / 1 FP16 / 2 FP32, y_dtype 0 BF16 / 1 FP16.
-int launch_layernorm512(const void* x, int x_dtype, const float* weight, const float* bias, float eps, void* y,
+int launch_layernorm512(const void* x, int x_dtype, ParamVec weight, ParamVec bias, float eps, void* y,
                         int y_dtype, long long rows, cudaStream_t st, int dependent = 0);
 // Residual vector quantisation (fm_rvq.cu): candidate selection + exact FP32 decision for one layer, FP16 copy of
 // the residual, ordered FP32 decode.

@@ -66,13 +66,14 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
   Buffers b;
   if (lay_out(static_cast<uint8_t*>(workspace), rows, p.stream_dtype == 2 ? 4 : 2, p.ffn, lin_rows, &b) > workspace_bytes) return -7;
   if (workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return -3;
+  const auto vec = [&](const void* v) { return ParamVec(v, p.vec_dtype); };
   const int value_fp16 = p.value_dtype & 1;
   const int tc = (p.value_dtype & 2) ? 1 : 0;                    // 16-bit type of the products' operands: 0 BF16, 1 FP16
 
   const bool norm1_inside = few_rows_with_norm(rows, 1536), norm2_inside = few_rows_with_norm(rows, p.ffn);
   int rc = 0;
   if (!norm1_inside) {
-    rc = launch_layernorm512(x, p.stream_dtype, p.ln1_weight, p.ln1_bias, p.ln1_eps, b.h, tc, rows, st, 1);
+    rc = launch_layernorm512(x, p.stream_dtype, vec(p.ln1_weight), vec(p.ln1_bias), p.ln1_eps, b.h, tc, rows, st, 1);
     if (rc != 0) return rc;
   }
   const bool few_tiles = !few && few_attn_tiles(B, T) && (!cached || slots <= 256);
@@ -90,7 +91,7 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
     ep.ring_slots = 1;
     // The kernel that opens the chain may ask for W_qkv ahead of its wait only if W_qkv cannot be the work of the kernel
     // in front: not on the first call after the caller has (re)made it.
-    rc = norm1_inside ? launch_ln_qkv(x, p.stream_dtype, p.ln1_weight, p.ln1_bias, p.ln1_eps, p.w_qkv, ep, rows, p.value_dtype,
+    rc = norm1_inside ? launch_ln_qkv(x, p.stream_dtype, vec(p.ln1_weight), vec(p.ln1_bias), p.ln1_eps, p.w_qkv, ep, rows, p.value_dtype,
                                       status, st, p.weights_settled)
                       : launch_qkv_rope_gemm(b.h, p.w_qkv, ep, rows, p.value_dtype, status, st, 1);
     if (rc != 0) return rc;
@@ -115,18 +116,18 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
     }
   }
   if (rc != 0) return rc;
-  rc = launch_linear_gemm(b.core, p.w_o, b.x1, p.attn_scale, x, rows, 512, 512, value_fp16, p.stream_dtype, 0, status, st, 1);
+  rc = launch_linear_gemm(b.core, p.w_o, b.x1, vec(p.attn_scale), x, rows, 512, 512, value_fp16, p.stream_dtype, 0, status, st, 1);
   if (rc != 0) return rc;
   if (norm2_inside) {
-    rc = launch_ln_linear_gelu(b.x1, p.stream_dtype, p.ln2_weight, p.ln2_bias, p.ln2_eps, p.w_fc1, b.g, rows, p.ffn, tc, status,
+    rc = launch_ln_linear_gelu(b.x1, p.stream_dtype, vec(p.ln2_weight), vec(p.ln2_bias), p.ln2_eps, p.w_fc1, b.g, rows, p.ffn, tc, status,
                                st, 1);
   } else {
-    rc = launch_layernorm512(b.x1, p.stream_dtype, p.ln2_weight, p.ln2_bias, p.ln2_eps, b.h, tc, rows, st, 1);
+    rc = launch_layernorm512(b.x1, p.stream_dtype, vec(p.ln2_weight), vec(p.ln2_bias), p.ln2_eps, b.h, tc, rows, st, 1);
     if (rc != 0) return rc;
-    rc = launch_linear_gemm(b.h, p.w_fc1, b.g, nullptr, nullptr, rows, p.ffn, 512, tc, tc, 1, status, st, 1);
+    rc = launch_linear_gemm(b.h, p.w_fc1, b.g, ParamVec(nullptr), nullptr, rows, p.ffn, 512, tc, tc, 1, status, st, 1);
   }
   if (rc != 0) return rc;
-  return launch_linear_gemm(b.g, p.w_fc2, y, p.mlp_scale, b.x1, rows, 512, p.ffn, tc, p.stream_dtype, 0, status, st, 1);
+  return launch_linear_gemm(b.g, p.w_fc2, y, vec(p.mlp_scale), b.x1, rows, 512, p.ffn, tc, p.stream_dtype, 0, status, st, 1);
 }
 
 }  // namespace fm
@@ -135,7 +136,7 @@ extern "C" int fm_layer_forward(const fm_layer_params* params, const void* x, vo
                                 long long workspace_bytes, const float* cos, const float* sin, long long cos_bstride, int B,
                                 int T, void* ring_k, void* ring_v, int past, int ring_slots, int* status, void* stream) {
   if (params == nullptr || params->stream_dtype < 0 || params->stream_dtype > 2 || params->value_dtype < 0 ||
-      params->value_dtype > 3)
+      params->value_dtype > 3 || params->vec_dtype < 0 || params->vec_dtype > 2)
     return -1;
   return fm::layer_forward(*params, x, y, workspace, workspace_bytes, cos, sin, cos_bstride, B, T, ring_k, ring_v, past,
                            ring_slots, status, static_cast<cudaStream_t>(stream));

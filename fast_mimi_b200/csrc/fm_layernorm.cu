@@ -37,7 +37,7 @@ __device__ __forceinline__ void load4(const void* base, long long elem, float (&
 // kIn: 0 = BF16, 1 = FP16, 2 = FP32;  kOut: 0 = BF16, 1 = FP16
 template <int kIn, int kOut>
 __global__ void __launch_bounds__(ln::kWarpsPerBlock * 32)
-layernorm512_kernel(const void* __restrict__ x, const float* __restrict__ weight, const float* __restrict__ bias,
+layernorm512_kernel(const void* __restrict__ x, const ParamVec weight, const ParamVec bias,
                     float eps, void* __restrict__ y, long long rows) {
   using namespace ln;
   using TOut = typename std::conditional<kOut == 1, __half, __nv_bfloat16>::type;
@@ -52,8 +52,8 @@ layernorm512_kernel(const void* __restrict__ x, const float* __restrict__ weight
   float w[4][4], b[4][4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const float4 wf = __ldg(reinterpret_cast<const float4*>(weight + 128 * j + 4 * lane));
-    const float4 bf = __ldg(reinterpret_cast<const float4*>(bias + 128 * j + 4 * lane));
+    const float4 wf = weight.load4(128 * j + 4 * lane);
+    const float4 bf = bias.load4(128 * j + 4 * lane);
     w[j][0] = wf.x; w[j][1] = wf.y; w[j][2] = wf.z; w[j][3] = wf.w;
     b[j][0] = bf.x; b[j][1] = bf.y; b[j][2] = bf.z; b[j][3] = bf.w;
   }
@@ -90,19 +90,19 @@ layernorm512_kernel(const void* __restrict__ x, const float* __restrict__ weight
   }
 }
 
-int launch_layernorm512(const void* x, int x_dtype, const float* weight, const float* bias, float eps, void* y,
+int launch_layernorm512(const void* x, int x_dtype, ParamVec weight, ParamVec bias, float eps, void* y,
                         int y_dtype, long long rows, cudaStream_t st, int dependent) {
   using namespace ln;
   if (rows < 0 || x_dtype < 0 || x_dtype > 2 || y_dtype < 0 || y_dtype > 1) return -1;
   if (rows == 0) return 0;
-  if (x == nullptr || y == nullptr || weight == nullptr || bias == nullptr) return -1;
-  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(weight) |
-       reinterpret_cast<uintptr_t>(bias)) & 15u)
+  if (x == nullptr || y == nullptr || weight.data == nullptr || bias.data == nullptr) return -1;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(weight.data) |
+       reinterpret_cast<uintptr_t>(bias.data)) & 15u)
     return -3;
   const long long want = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
   const long long cap = static_cast<long long>(sm_count()) * 8;    // 8 resident blocks of 256 threads per SM
   const int grid = static_cast<int>(want < cap ? want : cap);
-  using Kern = void (*)(const void*, const float*, const float*, float, void*, long long);
+  using Kern = void (*)(const void*, ParamVec, ParamVec, float, void*, long long);
   static const Kern table[3][2] = {{layernorm512_kernel<0, 0>, layernorm512_kernel<0, 1>},
                                    {layernorm512_kernel<1, 0>, layernorm512_kernel<1, 1>},
                                    {layernorm512_kernel<2, 0>, layernorm512_kernel<2, 1>}};

@@ -65,7 +65,7 @@ static_assert(sizeof(Barriers) <= 256, "barrier block too large");
 }  // namespace lin
 
 struct LinearArgs {
-  const float* scale;     // [N] or null             (kOut 3: |e_j|^2 of the codebook entries)
+  ParamVec scale;         // [N] or null             (kOut 3: |e_j|^2 of the codebook entries, FP32)
   const void* resid;      // [M, N] in the output's type or null      (kOut 3: per-row candidate margin, [M] FP32)
   int M, N, K;
   int gelu;               // 1: exact GELU on the accumulator before scale / residual
@@ -242,7 +242,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           R next[8];
           if (idx + 1 < n_pieces) fetch(idx + 1, next);
           const int col = first_col(i, p);
-          const float4 sc = args.scale != nullptr ? __ldg(reinterpret_cast<const float4*>(args.scale + col)) : make_float4(1.f, 1.f, 1.f, 1.f);
+          const float4 sc = args.scale.data != nullptr ? args.scale.load4(col) : make_float4(1.f, 1.f, 1.f, 1.f);
           tmem_ld_wait();
           if (p == kPieces - 1) {
             // Last read of the accumulator by this warp: hand it back before the arithmetic and the stores.
@@ -313,7 +313,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         }
         if constexpr (kOut == 3) {
           // approximate distances of this row to entries col0 .. col0 + 63, their minimum and who is within the margin
-          const float4* q4 = reinterpret_cast<const float4*>(args.scale + col0);        // same address in every lane
+          const float4* q4 = reinterpret_cast<const float4*>(static_cast<const float*>(args.scale.data) + col0);        // same address in every lane
           float dmin = INFINITY;
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
@@ -337,11 +337,10 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
 #pragma unroll
           for (int c = 0; c < 64; c += 2) gelu_erf2(v[c], v[c + 1]);
         }
-        if (args.scale != nullptr) {
-          const float4* s4 = reinterpret_cast<const float4*>(args.scale + col0);   // same address in every lane
+        if (args.scale.data != nullptr) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const float4 s = __ldg(s4 + j);
+            const float4 s = args.scale.load4(col0 + 4 * j);         // same address in every lane
             v[4 * j] *= s.x; v[4 * j + 1] *= s.y; v[4 * j + 2] *= s.z; v[4 * j + 3] *= s.w;
           }
         }
@@ -435,16 +434,16 @@ static int launch_pairs(const void* a, const void* w, void* y, const LinearArgs&
                        idesc, status);
 }
 
-int launch_linear_gemm(const void* a, const void* w, void* y, const float* scale, const void* resid, int M, int N,
+int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N,
                        int K, int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent) {
   using namespace lin;
   if (M < 0 || N <= 0 || K <= 0 || N % 256 != 0 || K % kBlockK != 0) return -1;
   if (in_dtype < 0 || in_dtype > 1 || out_dtype < 0 || out_dtype > 3) return -1;
   if (M == 0) return 0;
   if (a == nullptr || w == nullptr || y == nullptr) return -1;
-  if (out_dtype == 3 && (scale == nullptr || resid == nullptr || gelu)) return -1;
+  if (out_dtype == 3 && (scale.data == nullptr || scale.type != 2 || resid == nullptr || gelu)) return -1;
   if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y) |
-       reinterpret_cast<uintptr_t>(scale) | reinterpret_cast<uintptr_t>(resid)) & 15u)
+       reinterpret_cast<uintptr_t>(scale.data) | reinterpret_cast<uintptr_t>(resid)) & 15u)
     return -3;
   if (out_dtype != 3 && few_row_tiles(M, N))
     return launch_linear_small(a, w, y, scale, resid, M, N, K, in_dtype, out_dtype, gelu, status, st, dependent);

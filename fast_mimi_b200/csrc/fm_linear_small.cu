@@ -270,7 +270,7 @@ static int launch_small(const void* a, const void* w, SmallArgs& args, int K, in
   return launch_tiles<kOut, VT, 64>(a, w, args, K, in_dtype, status, st, dependent);
 }
 
-int launch_linear_small(const void* a, const void* w, void* y, const float* scale, const void* resid, int M, int N, int K,
+int launch_linear_small(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N, int K,
                         int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent) {
   SmallArgs args = {};
   args.scale = scale;

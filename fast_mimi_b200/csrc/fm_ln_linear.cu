@@ -52,8 +52,8 @@ __device__ __forceinline__ void load4(const void* base, long long elem, float (&
 
 struct LnArgs {
   const void* x;          // [M, 512]
-  const float* weight;
-  const float* bias;
+  ParamVec weight;
+  ParamVec bias;
   float eps;
   int opens_chain;        // first kernel of a chain: lets the next one start only after its own wait
 };
@@ -125,8 +125,8 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float4 wf = __ldg(reinterpret_cast<const float4*>(ln.weight + 128 * j + 4 * lane));
-      const float4 bf = __ldg(reinterpret_cast<const float4*>(ln.bias + 128 * j + 4 * lane));
+      const float4 wf = ln.weight.load4(128 * j + 4 * lane);
+      const float4 bf = ln.bias.load4(128 * j + 4 * lane);
       w[j][0] = wf.x; w[j][1] = wf.y; w[j][2] = wf.z; w[j][3] = wf.w;
       b[j][0] = bf.x; b[j][1] = bf.y; b[j][2] = bf.z; b[j][3] = bf.w;
     }
@@ -259,11 +259,11 @@ static int launch_typed(const CUtensorMap& tmap_w, const LnArgs& ln, const Small
   return launch_rows<kIn, kTc, 3, __nv_bfloat16>(tmap_w, ln, args, idesc, status, st, dependent);
 }
 
-static int launch_ln(const void* x, int x_dtype, const float* weight, const float* bias, float eps, const void* w,
+static int launch_ln(const void* x, int x_dtype, ParamVec weight, ParamVec bias, float eps, const void* w,
                      const SmallArgs& args, int tc_fp16, int qkv, int value_fp16, int opens_chain, int* status, cudaStream_t st,
                      int dependent) {
   if (x_dtype < 0 || x_dtype > 2 || args.M <= 0 || args.N % lnlin::kBlockN != 0) return -1;
-  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(bias) |
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(weight.data) | reinterpret_cast<uintptr_t>(bias.data) |
        reinterpret_cast<uintptr_t>(w)) & 15u)
     return -3;
   CUtensorMap tmap_w;
@@ -278,7 +278,7 @@ static int launch_ln(const void* x, int x_dtype, const float* weight, const floa
   return table[x_dtype][tc_fp16 ? 1 : 0](tmap_w, ln, args, idesc, qkv, value_fp16, status, st, dependent);
 }
 
-int launch_ln_qkv(const void* x, int x_dtype, const float* weight, const float* bias, float eps, const void* w_qkv,
+int launch_ln_qkv(const void* x, int x_dtype, ParamVec weight, ParamVec bias, float eps, const void* w_qkv,
                   const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status, cudaStream_t st, int dependent) {
   SmallArgs args = {};
   args.M = M;
@@ -288,7 +288,7 @@ int launch_ln_qkv(const void* x, int x_dtype, const float* weight, const float* 
                    dependent);
 }
 
-int launch_ln_linear_gelu(const void* x, int x_dtype, const float* weight, const float* bias, float eps, const void* w, void* y,
+int launch_ln_linear_gelu(const void* x, int x_dtype, ParamVec weight, ParamVec bias, float eps, const void* w, void* y,
                           int M, int N, int tc_fp16, int* status, cudaStream_t st, int dependent) {
   SmallArgs args = {};
   args.y = y;

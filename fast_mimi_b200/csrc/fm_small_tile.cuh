@@ -18,7 +18,7 @@ __device__ __forceinline__ uint32_t red_offset(uint32_t r, uint32_t c, uint32_t 
 }  // namespace small
 
 struct SmallArgs {
-  const float* scale;     // [N] or null
+  ParamVec scale;         // [N] or null
   const void* resid;      // [M, N] in the output's type or null
   void* y;                // [M, N]
   int M, N, chunks;       // chunks: K / 64 / S, this block's share
@@ -52,7 +52,7 @@ __device__ __forceinline__ void load_operands(const SmallArgs& args, int row, in
     const long long at = static_cast<long long>(row) * args.N + col;
 #pragma unroll
     for (int h = 0; h < kHalves; ++h) {
-      p.s[h] = args.scale != nullptr ? __ldg(reinterpret_cast<const float4*>(args.scale + col + 32 * h)) : make_float4(1.f, 1.f, 1.f, 1.f);
+      p.s[h] = args.scale.data != nullptr ? args.scale.load4(col + 32 * h) : make_float4(1.f, 1.f, 1.f, 1.f);
       p.a[h] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (args.resid != nullptr) {
         if constexpr (kOut == 2) {
@@ -118,7 +118,7 @@ __device__ __forceinline__ void finish_piece(const SmallArgs& args, float (&lo)[
         gelu_erf2(v[0], v[1]);
         gelu_erf2(v[2], v[3]);
       }
-      if (args.scale != nullptr) {
+      if (args.scale.data != nullptr) {
         v[0] *= p.s[h].x; v[1] *= p.s[h].y; v[2] *= p.s[h].z; v[3] *= p.s[h].w;
       }
       if (args.resid != nullptr) {

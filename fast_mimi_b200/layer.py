@@ -100,7 +100,7 @@ class MimiTransformerLayerB200(nn.Module):
         return {**self.__dict__, "_plan": None}         # device addresses: rebuilt by the copy's first call
 
     def _native_plan(self, x: torch.Tensor):
-        """The parameter block of the native call for activations like ``x`` (16-bit weights, FP32 LayerNorm parameters and
+        """The parameter block of the native call for activations like ``x`` (16-bit weights, LayerNorm parameters and
         layer scales) and, where every parameter is an entry of its module, the plan that notices when one of them, a
         submodule or an option changes."""
         attn, mlp, ln1, ln2 = self.self_attn, self.mlp, self.input_layernorm, self.post_attention_layernorm
@@ -112,15 +112,22 @@ class MimiTransformerLayerB200(nn.Module):
         ops._need(tuple(fc1.shape) == (ffn, 512) and tuple(fc2.shape) == (512, ffn) and ffn % 256 == 0,
                   "the MLP must be 512 -> n -> 512 with n a multiple of 256")
         tc = attn._tc_input_dtype(x)
-        f32 = lambda p: p.detach().float().contiguous()       # no copy for FP32 parameters
-        keep = (f32(ln1.weight), f32(ln1.bias), attn.packed_qkv_weight(tc), attn.out_weight(attn.value_dtype),
-                f32(self.self_attn_layer_scale.scale), f32(ln2.weight), f32(ln2.bias), self._cast.get("fc1", fc1, tc),
-                self._cast.get("fc2", fc2, tc), f32(self.mlp_layer_scale.scale))
+        vectors = (ln1.weight, ln1.bias, self.self_attn_layer_scale.scale, ln2.weight, ln2.bias, self.mlp_layer_scale.scale)
+        # Read where they lie if they have one type; else as FP32 copies made for this call alone (no plan), since a write
+        # through ``.data`` would not show in a kept copy.
+        in_place = (len({p.dtype for p in vectors}) == 1 and vectors[0].dtype in ops._OUT_CODES
+                    and all(p.is_contiguous() and p.data_ptr() % 16 == 0 for p in vectors))
+        w1, b1, s1, w2, b2, s2 = (p.detach() if in_place else p.detach().float().contiguous() for p in vectors)
+        keep = (w1, b1, attn.packed_qkv_weight(tc), attn.out_weight(attn.value_dtype), s1, w2, b2, self._cast.get("fc1", fc1, tc),
+                self._cast.get("fc2", fc2, tc), s2)
         for t in keep:
             ops._need(t.is_cuda, "the layer's parameters must be on a CUDA device")
         params = _native.LayerParams(*(t.data_ptr() for t in keep), ln1.eps, ln2.eps, attn.scaling, attn.sliding_window,
                                      ops._OUT_CODES[x.dtype],
-                                     ops._VALUE_CODES[attn.value_dtype] | (2 if tc == torch.float16 else 0), ffn, 0)
+                                     ops._VALUE_CODES[attn.value_dtype] | (2 if tc == torch.float16 else 0), ffn, 0, ops._OUT_CODES[w1.dtype])
+        self._plan = None
+        if not in_place:
+            return params, keep
         watches = [(self._modules, n) for n in ("self_attn", "mlp", "input_layernorm", "post_attention_layernorm",
                                                 "self_attn_layer_scale", "mlp_layer_scale")]
         watches += [(attn._modules, n) for n in ("q_proj", "k_proj", "v_proj", "o_proj")]
@@ -134,7 +141,7 @@ class MimiTransformerLayerB200(nn.Module):
             like_value = torch.empty(0, dtype=attn.value_dtype)
             self._plan = _native.bind().LayerPlan(watches, keep, ctypes.addressof(params), ops.default_status(x.device), x, like_value)
         except KeyError:            # a computed parameter (parametrised weights and the like): nothing to watch
-            self._plan = None
+            pass
         return params, keep
 
     def _forward_checked(self, x, cos, sin, ring_k, ring_v, past) -> torch.Tensor:

@@ -33,7 +33,7 @@ int fm_abi_version(void);
  * MimiTransformerLayer.forward (src/fast_mimi/model.py:2026-2061).
  *   params      host struct of device pointers; matrices are row-major [out, in] and 16 bit: w_qkv, w_fc1, w_fc2 in
  *               BF16 / FP16 by bit 1 of value_dtype, w_o in the value type (bit 0); LayerNorm parameters and layer
- *               scales FP32 (the scales may be NULL)
+ *               scales in vec_dtype (0 BF16, 1 FP16, 2 FP32), 16-byte aligned (the scales may be NULL)
  *               weights_settled: 0 on the first call after any of them was written on this stream (the call then starts
  *               only when everything in front of it has ended), 1 afterwards
  *   x, y        [B, T, 512] in stream_dtype (0 BF16, 1 FP16, 2 FP32), y != x
@@ -44,16 +44,16 @@ int fm_abi_version(void);
  *   cos, sin    [1 or B, T, 64] FP32 of the new frames' positions
  * The launches form a chain of programmatically dependent kernels on `stream`. */
 typedef struct fm_layer_params {
-  const float* ln1_weight;
-  const float* ln1_bias;
+  const void* ln1_weight;
+  const void* ln1_bias;
   const void* w_qkv;
   const void* w_o;
-  const float* attn_scale;
-  const float* ln2_weight;
-  const float* ln2_bias;
+  const void* attn_scale;
+  const void* ln2_weight;
+  const void* ln2_bias;
   const void* w_fc1;
   const void* w_fc2;
-  const float* mlp_scale;
+  const void* mlp_scale;
   float ln1_eps;
   float ln2_eps;
   float scale;
@@ -62,6 +62,7 @@ typedef struct fm_layer_params {
   int value_dtype;
   int ffn;
   int weights_settled;
+  int vec_dtype;
 } fm_layer_params;
 
 int fm_layer_forward(const fm_layer_params* params, const void* x, void* y, void* workspace, long long workspace_bytes,

@@ -143,3 +143,40 @@ def test_layer_with_parameters_that_cannot_be_watched():
     for _ in range(2):
         got, _ = layer(x.cuda(), None, None, cs)
         assert O.rel_l2(got.cpu() - x, O.transformer_layer(x, p) - x) < 2e-3
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows", [20, 400, 5000])
+def test_layer_reads_its_vectors_where_they_lie(dtype, rows):
+    """LayerNorm parameters and layer scales written through ``.data`` (no version counter moves) show in the next call: with
+    the LayerNorm folded into the products, with both kinds of linear kernel behind a LayerNorm kernel, and for a module
+    whose vectors have several types."""
+    import fast_mimi_b200 as fm
+    layer = fm.MimiTransformerLayerB200().cuda()
+    layer.load_state_dict(_layer_params(5))
+    layer = layer.to(dtype)
+    T = min(rows, 500)
+    x = torch.randn(rows // T, T, 512).to(dtype)
+    cs = fm.rope_tables(torch.arange(T, device="cuda")[None])
+
+    def check():
+        p = {k: v.float().cpu() for k, v in layer.state_dict().items()}
+        want = O.transformer_layer(x.float(), p)
+        got, _ = layer(x.cuda(), None, None, cs)
+        # the result's own rounding, over what the layer adds
+        bar = {torch.float32: 2e-3, torch.float16: 4e-3, torch.bfloat16: 2e-2}[dtype] * float(want.norm() / (want - x.float()).norm())
+        assert O.rel_l2(got.float().cpu() - x.float(), want - x.float()) < bar
+
+    with torch.no_grad():
+        check()
+        for norm in (layer.input_layernorm, layer.post_attention_layernorm):
+            norm.weight.data.mul_(1.5)
+            norm.bias.data.add_(0.25)
+        layer.self_attn_layer_scale.scale.data.mul_(3.0)
+        layer.mlp_layer_scale.scale.data.mul_(-2.0)
+        check()
+        layer.input_layernorm.float()
+        check()
+        layer.input_layernorm.weight.data.mul_(0.5)
+        check()
+    fm.check_status()
