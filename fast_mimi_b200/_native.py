@@ -35,8 +35,13 @@ SIGNATURES: dict[str, list] = {
     "fm_layernorm_f16": [_P, _I, _P, _P, _F, _P, _I, _LL, _P],
     "fm_rvq_select_f32": [_P, _I, _P, _P, _P, _P, _P, _P, _LL, _I, _F, _F, _P, _P],
     "fm_conv_rows_split": [_P, _P, _P, _I, _I, _I, _I, _I, _P],
+    "fm_conv_frames_split": [_P, _P, _P, _I, _I, _I, _I, _I, _P],
+    "fm_linear_split_f32": [_P, _P, _LL, _I, _P, _P, _P, _LL, _I, _I, _I, _I, _I, _P, _P],
+    "fm_upsample2_channels_f32": [_P, _P, _P, _I, _I, _I, _P],
+    "fm_rvq_decode_split": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "fm_upsample2_f32": [_P, _P, _P, _I, _I, _I, _P],
     "fm_split_half": [_P, _P, _P, _LL, _P],
+    "fm_rvq_encode_f32": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _LL, _I, _I, _F, _P, _P],
     "fm_rvq_prepare_f32": [_P, _P, _P, _LL, _F, _F, _P],
     "fm_rvq_candidates_f16": [_P, _P, _P, _P, _P, _LL, _I, _P, _P],
     "fm_rvq_select_rec_f32": [_P, _P, _P, _P, _P, _P, _P, _LL, _I, _F, _F, _P, _P],

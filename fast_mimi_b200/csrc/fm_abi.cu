@@ -206,6 +206,21 @@ int fm_conv_rows_split(const float* x, void* hi, void* lo, int B, int T, int C, 
   return fm::launch_conv_rows_split(x, hi, lo, B, T, C, kernel, stride, static_cast<cudaStream_t>(stream));
 }
 
+int fm_conv_frames_split(const float* x, void* hi, void* lo, int B, int T, int C, int kernel, int stride, void* stream) {
+  return fm::launch_conv_frames_split(x, hi, lo, B, T, C, kernel, stride, static_cast<cudaStream_t>(stream));
+}
+
+int fm_linear_split_f32(const void* a_hi, const void* a_lo, long long a_rows, int a_cols, const void* w_hi, const void* w_lo,
+                        float* y, long long rows, int clip_rows, int clip_valid, int by_channel, int n_out, int k_in, int* status,
+                        void* stream) {
+  return fm::launch_linear_split(a_hi, a_lo, a_rows, a_cols, w_hi, w_lo, y, rows, clip_rows, clip_valid, by_channel, n_out, k_in, status,
+                                 static_cast<cudaStream_t>(stream));
+}
+
+int fm_upsample2_channels_f32(const float* x, const float* w, float* y, int B, int T, int C, void* stream) {
+  return fm::launch_upsample2_channels(x, w, y, B, T, C, static_cast<cudaStream_t>(stream));
+}
+
 int fm_upsample2_f32(const float* x, const float* w, float* y, int B, int T, int C, void* stream) {
   return fm::launch_upsample2_depthwise(x, w, y, B, T, C, static_cast<cudaStream_t>(stream));
 }
@@ -228,6 +243,13 @@ int fm_rvq_select_rec_f32(const void* records, const float* codebook, float* res
                                    e_max_next, tau_rel, status, static_cast<cudaStream_t>(stream));
 }
 
+int fm_rvq_encode_f32(float* residual, void* residual16, float* tau, void* records, const void* codebooks16, const float* codebooks,
+                      const float* e_sq, const float* e_max, long long* codes, int* n_candidates, long long rows, int n_codes, int layers,
+                      float tau_rel, int* status, void* stream) {
+  return fm::launch_rvq_encode(residual, residual16, tau, records, codebooks16, codebooks, e_sq, e_max, codes, n_candidates, rows,
+                               n_codes, layers, tau_rel, status, static_cast<cudaStream_t>(stream));
+}
+
 int fm_rvq_prepare_f32(const float* x, void* residual16, float* tau, long long rows, float e_max, float tau_rel,
                        void* stream) {
   return fm::launch_rvq_prepare(x, residual16, tau, rows, e_max, tau_rel, static_cast<cudaStream_t>(stream));
@@ -235,6 +257,12 @@ int fm_rvq_prepare_f32(const float* x, void* residual16, float* tau, long long r
 
 int fm_rvq_to_half(const float* x, void* y, long long rows, void* stream) {
   return fm::launch_rvq_to_half(x, y, rows, static_cast<cudaStream_t>(stream));
+}
+
+int fm_rvq_decode_split(const long long* codes, const float* books0, const float* books1, void* hi, void* lo, int B, int T,
+                        int n_layers, int n0, int n_codes0, int n_codes1, int* bad_code, void* stream) {
+  return fm::launch_rvq_decode_split(codes, books0, books1, hi, lo, B, T, n_layers, n0, n_codes0, n_codes1, bad_code,
+                                     static_cast<cudaStream_t>(stream));
 }
 
 int fm_rvq_decode_f32(const long long* codes, const float* codebooks, float* out, long long rows, int n_layers,

@@ -550,6 +550,20 @@ template <> struct Pack16<__nv_bfloat16> {
   }
 };
 
+// Eight values as FP16 hi + lo parts: hi = round(x), lo = round(x - hi).
+__device__ __forceinline__ void split_half8(const float4& a, const float4& b, uint4& hi, uint4& lo) {
+  const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  uint32_t h[4], l[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    h[e] = Pack16<__half>::pack(v[2 * e], v[2 * e + 1]);
+    const float2 back = Pack16<__half>::unpack(h[e]);
+    l[e] = Pack16<__half>::pack(v[2 * e] - back.x, v[2 * e + 1] - back.y);
+  }
+  hi = make_uint4(h[0], h[1], h[2], h[3]);
+  lo = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
 // A vector of per-channel parameters (LayerNorm weight and bias, layer scale) in the type that the module keeps it in, read
 // where it lies: a converted copy would have to be kept in step with the module.  Type: 0 BF16, 1 FP16, 2 FP32.
 struct ParamVec {

@@ -7,13 +7,51 @@
 // (-T) % 2 frames, both repeating the edge frame, then nn.Conv1d).  On frame-major activations [B, T, 512] output
 // frame t is a 2048-long inner product: the four consecutive frames 2t-2 .. 2t+1 (clamped to the clip) against
 // the kernel laid out as W2[c_out, j * 512 + c_in] = W[c_out, c_in, j].  So the convolution is a linear with
-// K = 2048 over rows that overlap in memory; this file only gathers those rows (with the edge clamping) and splits
-// them into FP16 hi + lo parts; the products run on the tensor-core linear kernel (hi W_hi + hi W_lo + lo W_hi with
-// FP32 accumulation: FP32-grade accuracy, which the code decisions that follow need).
+// K = 2048 over rows that overlap in memory.  This file lays the frames out with their padding and splits them into FP16
+// hi + lo parts; the products run on the tensor-core linear kernel (hi W_hi + hi W_lo + lo W_hi with FP32 accumulation:
+// FP32-grade accuracy, which the code decisions that follow need).
 #include "fm_common.cuh"
 #include "fm_kernels.h"
 
 namespace fm {
+
+// Padded frames, for a kernel that is a multiple of the stride: clip b has stride * (T_out + kernel / stride - 1) frames, the
+// first kernel - stride and the odd last one repeating the edge.  Seen as rows of `stride` frames, output frame t is
+// rows t .. t + kernel / stride - 1 of its clip, which the product reads as they lie: every frame is written once, and not
+// kernel / stride times as in the gathered rows below.  HBM-bound: four bytes read and four written per value
+// (128000 frames of 512: 85 us, 6.2 TB/s).
+// One thread per 8 values.
+__global__ void __launch_bounds__(256)
+conv_frames_split_kernel(const float* __restrict__ x, uint16_t* __restrict__ hi, uint16_t* __restrict__ lo, int B, int T, int T_pad,
+                         int left, int C) {
+  const int c8 = C / 8;
+  const long long total = static_cast<long long>(B) * T_pad * c8;
+  const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {
+    const long long r = i / c8;
+    const int piece = static_cast<int>(i - r * c8);
+    const int b = static_cast<int>(r / T_pad);
+    int f = static_cast<int>(r - static_cast<long long>(b) * T_pad) - left;
+    f = f < 0 ? 0 : (f > T - 1 ? T - 1 : f);
+    const float4* src = reinterpret_cast<const float4*>(x + (static_cast<long long>(b) * T + f) * C + piece * 8);
+    const float4 a = __ldg(src), c = __ldg(src + 1);
+    uint4 h, l;
+    split_half8(a, c, h, l);
+    reinterpret_cast<uint4*>(hi)[i] = h;
+    reinterpret_cast<uint4*>(lo)[i] = l;
+  }
+}
+
+int launch_conv_frames_split(const float* x, void* hi, void* lo, int B, int T, int C, int kernel, int stride, cudaStream_t st) {
+  if (B <= 0 || T <= 0) return (B == 0 || T == 0) ? 0 : -1;
+  if (C <= 0 || C % 8 != 0 || stride <= 0 || kernel < stride || kernel % stride != 0 || kernel > 16) return -1;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 15u) return -3;
+  const int T_pad = stride * ((T + stride - 1) / stride + kernel / stride - 1);
+  const long long want = (static_cast<long long>(B) * T_pad * (C / 8) + 255) / 256, cap = static_cast<long long>(sm_count()) * 8;
+  conv_frames_split_kernel<<<static_cast<int>(want < cap ? want : cap), 256, 0, st>>>(
+      x, static_cast<uint16_t*>(hi), static_cast<uint16_t*>(lo), B, T, T_pad, kernel - stride, C);
+  return static_cast<int>(cudaGetLastError());
+}
 
 // One thread per 8 values of a gathered row: rows [B * T_out, 4 * C], x [B, T, C] FP32 (C a multiple of 8).
 __global__ void __launch_bounds__(256)
@@ -33,16 +71,10 @@ conv_rows_split_kernel(const float* __restrict__ x, uint16_t* __restrict__ hi, u
     f = f < 0 ? 0 : (f > T - 1 ? T - 1 : f);
     const float4* src = reinterpret_cast<const float4*>(x + (b * T + f) * C + piece * 8);
     const float4 a = __ldg(src), c = __ldg(src + 1);
-    const float v[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
-    uint32_t h[4], l[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      h[e] = Pack16<__half>::pack(v[2 * e], v[2 * e + 1]);
-      const float2 back = Pack16<__half>::unpack(h[e]);
-      l[e] = Pack16<__half>::pack(v[2 * e] - back.x, v[2 * e + 1] - back.y);
-    }
-    reinterpret_cast<uint4*>(hi)[i] = make_uint4(h[0], h[1], h[2], h[3]);
-    reinterpret_cast<uint4*>(lo)[i] = make_uint4(l[0], l[1], l[2], l[3]);
+    uint4 h, l;
+    split_half8(a, c, h, l);
+    reinterpret_cast<uint4*>(hi)[i] = h;
+    reinterpret_cast<uint4*>(lo)[i] = l;
   }
 }
 
@@ -91,6 +123,43 @@ upsample2_depthwise_kernel(const float* __restrict__ x, const float* __restrict_
     o.w = wc[12 + j] * a.w + wc[12 + j + 2] * p.w;
     reinterpret_cast<float4*>(y + (b * 2 * T + n) * C)[cq] = o;
   }
+}
+
+// The same from channel-major x [B, C, T], in which the quantiser's decode leaves it: a tile of 32 frames (and the one in
+// front) x 32 channels turns round in shared memory, so that both sides move whole lines and no transposed copy is made.
+__global__ void __launch_bounds__(256)
+upsample2_channels_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int T, int C) {
+  __shared__ float tile[32][34];                      // [channel][frame t0 - 1 ..]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int t0 = static_cast<int>(blockIdx.x) * 32, c0 = static_cast<int>(blockIdx.y) * 32;
+  const long long b = blockIdx.z;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int c = warp + 8 * i;
+    const float* src = x + (b * C + c0 + c) * T;
+    if (t0 + lane < T) tile[c][lane + 1] = __ldg(src + t0 + lane);
+    if (lane == 0) tile[c][0] = t0 > 0 ? __ldg(src + t0 - 1) : 0.f;
+  }
+  __syncthreads();
+  const float4 k = __ldg(reinterpret_cast<const float4*>(w) + c0 + lane);      // this lane's channel
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = warp + 8 * i;
+    if (t0 + t >= T) break;
+    const float p = tile[lane][t], a = tile[lane][t + 1];
+    float* dst = y + (b * 2 * T + 2 * (t0 + t)) * C + c0 + lane;
+    dst[0] = k.x * a + k.z * p;
+    dst[C] = k.y * a + k.w * p;
+  }
+}
+
+int launch_upsample2_channels(const float* x, const float* w, float* y, int B, int T, int C, cudaStream_t st) {
+  if (B <= 0 || T <= 0) return (B == 0 || T == 0) ? 0 : -1;
+  if (C <= 0 || C % 32 != 0 || B > 65535 || C / 32 > 65535) return -1;
+  if ((reinterpret_cast<uintptr_t>(x) & 3u) | ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15u)) return -3;
+  const dim3 grid(static_cast<unsigned>((T + 31) / 32), static_cast<unsigned>(C / 32), static_cast<unsigned>(B));
+  upsample2_channels_kernel<<<grid, 256, 0, st>>>(x, w, y, T, C);
+  return static_cast<int>(cudaGetLastError());
 }
 
 int launch_upsample2_depthwise(const float* x, const float* w, float* y, int B, int T, int C, cudaStream_t st) {

@@ -64,6 +64,38 @@ int launch_out_proj_gemm(const void* a, const void* w, void* y, const float* out
 // (type of y and resid); gelu 1 = exact GELU.  N a multiple of 256, K a multiple of 64.
 int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N,
                        int K, int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent = 0);
+// Split-precision product y = (a_hi + a_lo)(w_hi + w_lo)^T in FP32 grade (all four FP16; lo lo left out).  `a` is [a_rows,
+// a_cols]; row r of the product has K = a_cols * n values and lies in rows r .. r + n - 1 of `a` (n = 1: a plain matrix; n = 2:
+// a convolution of twice its stride over padded frames).  Of every clip_rows rows the first clip_valid are results, stored
+// back to back: y [rows * clip_valid / clip_rows, N]; or, with by_channel, clip by clip with the channels outside: y
+// [rows / clip_rows, N, clip_valid].
+struct SplitRows {
+  int a_chunks;           // a_cols / 64
+  int clip_rows, clip_valid;
+  int by_channel;
+  __host__ __device__ __forceinline__ int out_row(int row, int M) const {
+    if (row >= M) return -1;
+    if (clip_rows == clip_valid) return row;
+    const int clip = row / clip_rows, t = row - clip * clip_rows;
+    return t < clip_valid ? clip * clip_valid + t : -1;
+  }
+  // channel 0 of a row in the by_channel layout; channels are clip_valid values apart
+  __host__ __device__ __forceinline__ long long out_at(int row, int M, int N) const {
+    const int clip = row / clip_rows, t = row - clip * clip_rows;
+    return row < M && t < clip_valid ? static_cast<long long>(clip) * N * clip_valid + t : -1;
+  }
+};
+struct SplitLow {
+  const void *a, *w;
+  long long a_rows;
+};
+int launch_linear_split(const void* a_hi, const void* a_lo, long long a_rows, int a_cols, const void* w_hi, const void* w_lo, float* y,
+                        long long rows, int clip_rows, int clip_valid, int by_channel, int N, int K, int* status, cudaStream_t st);
+int launch_linear_split_small(const void* a_hi, const void* w_hi, const SplitLow& low, const SplitRows& map, float* y, int M, int N,
+                              int K, int* status, cudaStream_t st);
+// Padded frames of a causal convolution (kernel a multiple of stride), split into FP16 hi + lo parts: clip b has
+// stride * (ceil(T / stride) + kernel / stride - 1) frames of C values (fm_downsample.cu).
+int launch_conv_frames_split(const float* x, void* hi, void* lo, int B, int T, int C, int kernel, int stride, cudaStream_t st);
 // The same two products for few rows (fm_linear_small.cu): 128 x 64 tiles, K split over a cluster.
 bool few_row_tiles(int M, int N);
 // LayerNorm folded into the product behind it (fm_ln_linear.cu) while one wave of blocks holds the rows: the chain-opening QKV projection and
@@ -97,10 +129,19 @@ int launch_split_half(const float* x, void* hi, void* lo, long long n, cudaStrea
 // margins in `tau` (written for the next layer by the decision kernel, for the first layer by launch_rvq_prepare).
 int launch_rvq_select_rec(const void* records, const float* codebook, float* resid, void* resid16, long long* codes,
                           int* n_candidates, float* tau, long long rows, int n_codes, float e_max_next, float tau_rel,
-                          int* status, cudaStream_t st);
+                          int* status, cudaStream_t st, int dependent = 0, int last = 0);
+int launch_rvq_encode(float* resid, void* resid16, float* tau, void* records, const void* books16, const float* books, const float* e_sq,
+                      const float* e_max, long long* codes, int* n_candidates, long long rows, int n_codes, int layers, float tau_rel,
+                      int* status, cudaStream_t st);
 int launch_rvq_prepare(const float* x, void* resid16, float* tau, long long rows, float e_max, float tau_rel,
                        cudaStream_t st);
 int launch_rvq_to_half(const float* x, void* y, long long rows, cudaStream_t st);
+// Ordered sums of one or two stacks (the first n0 of the n_layers rows of codes [B, n_layers, T]; the rest) as FP16 hi + lo
+// parts [B * T, 256 or 512].
+int launch_rvq_decode_split(const long long* codes, const float* books0, const float* books1, void* hi, void* lo, int B, int T,
+                            int n_layers, int n0, int n_codes0, int n_codes1, int* bad_code, cudaStream_t st);
+// The upsampling from [B, C, T] (fm_downsample.cu).
+int launch_upsample2_channels(const float* x, const float* w, float* y, int B, int T, int C, cudaStream_t st);
 int launch_rvq_decode(const long long* codes, const float* codebooks, float* out, long long rows, int n_layers,
                       int n_codes, int* bad_code, cudaStream_t st);
 int launch_band_attn_prefill(const void* q, const void* k, const void* v, void* out, int B, int T, int window,

@@ -71,17 +71,24 @@ struct LinearArgs {
   int gelu;               // 1: exact GELU on the accumulator before scale / residual
   uint4* records;         // kOut 3: [M, N / 64] candidate records
   void* y;                // [M, N]: stored directly where there is a residual, through the tensor map otherwise
+  SplitRows rows;         // kOut 4
 };
 
 // kOut: 0 = BF16, 1 = FP16, 2 = FP32 (type of y and of the residual); 3 = no y at all: the products are the inner
 // products x . e_j of a nearest-entry search and the epilogue reduces every 64 of them to one 16-byte record
 // {min_j d_j, 64-bit mask of the entries with d_j <= min + margin[row]},  d_j = |e_j|^2 - 2 x . e_j  (see fm_rvq.cu).
+// 4 = FP32 y of a split-precision product: both operands are pairs of FP16 matrices hi + lo, and K runs three times,
+// lo W_hi, hi W_lo, hi W_hi (the small terms first), into one accumulator.  As three products that handed FP32 sums on
+// through memory the same work moved 20 bytes per output value instead of four (64000 rows, K = 2048, N = 512: 317 us here,
+// 1.27 PFLOP/s over the three terms).
 template <int kOut, bool kWide, int kBlockN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(lin::Shape<kWide, kBlockN>::kThreads, 1)
 linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
-                   const __grid_constant__ CUtensorMap tmap_y, LinearArgs args, int total_units, uint32_t idesc,
-                   int* status) {
+                   const __grid_constant__ CUtensorMap tmap_y, const __grid_constant__ CUtensorMap tmap_a_lo,
+                   const __grid_constant__ CUtensorMap tmap_w_lo, const __grid_constant__ LinearArgs args, int total_units,
+                   uint32_t idesc, int* status) {
   using namespace lin;
+  constexpr bool kSplit = kOut == 4, kF32 = kOut == 2 || kOut == 4;
   using S = Shape<kWide, kBlockN>;
   constexpr int kStages = S::kStages, kEpiWarps = S::kEpiWarps, kGroupsPerWarp = S::kGroupsPerWarp;
   constexpr int kStageBytes = S::kStageBytes, kHalfN = S::kHalfN, kTmemCols = S::kTmemCols;
@@ -96,7 +103,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   const uint32_t rank = cluster_cta_rank();
   const bool leader = rank == 0;
   const int n_tiles = args.N / kBlockN;
-  const int k_chunks = args.K / kBlockK;
+  const int k_part = args.K / kBlockK, k_chunks = kSplit ? 3 * k_part : k_part;
   // Units are dealt round-robin: at any moment neighbouring pairs work on the output tiles of the SAME rows,
   // so the slices of a that one of them pulls from HBM are L2 hits for the others (with contiguous ranges
   // per pair the second output tile of a row tile came 30 us after the first and its a tile had been evicted:
@@ -140,14 +147,21 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     if (lane == 0) {
       tma_prefetch_desc(&tmap_a);
       tma_prefetch_desc(&tmap_w);
+      if constexpr (kSplit) {
+        tma_prefetch_desc(&tmap_a_lo);
+        tma_prefetch_desc(&tmap_w_lo);
+      }
+      auto load_w = [&](uint8_t* dst, int kc, uint64_t* bar, int n0) {
+        if constexpr (kSplit) tma_load_2d_pair(dst, kc / k_part == 1 ? &tmap_w_lo : &tmap_w, bar, kc % k_part * kBlockK, n0);
+        else tma_load_2d_pair(dst, &tmap_w, bar, kc * kBlockK, n0);
+      };
       int stage = 0;
       uint32_t phase = 0;
       // The W slices of the first stages do not depend on the kernel in front: they are requested before the wait.
       const int ahead = u_count > 0 ? (k_chunks < kStages ? k_chunks : kStages) : 0;
       for (int kc = 0; kc < ahead; ++kc) {
         if (leader) mbar_arrive_expect_tx(&bars->full[kc], 2 * kStageBytes);
-        tma_load_2d_pair(smem_stage + kc * kStageBytes + kABytes, &tmap_w, &bars->full[kc], kc * kBlockK,
-                         (pair % n_tiles) * kBlockN + static_cast<int>(rank) * kHalfN);
+        load_w(smem_stage + kc * kStageBytes + kABytes, kc, &bars->full[kc], (pair % n_tiles) * kBlockN + static_cast<int>(rank) * kHalfN);
       }
       griddep_wait();
       for (int i = 0; i < u_count; ++i) {
@@ -161,8 +175,13 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             if (leader) mbar_arrive_expect_tx(&bars->full[stage], 2 * kStageBytes);
           }
           uint8_t* dst = smem_stage + stage * kStageBytes;
-          tma_load_2d_pair(dst, &tmap_a, &bars->full[stage], kc * kBlockK, m0);
-          if (!early) tma_load_2d_pair(dst + kABytes, &tmap_w, &bars->full[stage], kc * kBlockK, n0);
+          if constexpr (kSplit) {
+            const int k = kc % k_part;            // a row of the product continues in the matrix's next row
+            tma_load_2d_pair(dst, kc < k_part ? &tmap_a_lo : &tmap_a, &bars->full[stage], k % args.rows.a_chunks * kBlockK, m0 + k / args.rows.a_chunks);
+          } else {
+            tma_load_2d_pair(dst, &tmap_a, &bars->full[stage], kc * kBlockK, m0);
+          }
+          if (!early) load_w(dst + kABytes, kc, &bars->full[stage], n0);
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
       }
@@ -206,8 +225,8 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     const uint32_t acc_empty_leader = map_to_cta(smem_u32(&bars->acc_empty[0]), 0);
     uint8_t* slab = smem_out + warp * kSlabBytes;
     bool done = false;
-    if constexpr (kOut < 3) {
-      if (args.resid != nullptr) {
+    if constexpr (kOut != 3) {
+      if (kSplit || args.resid != nullptr) {
         // With a residual, accumulator rows cross the slab so that every lane finishes four columns of eight rows, and
         // residual and result are read and written as whole 128-byte (16 bit: 64-byte) lines by neighbouring lanes.  When
         // each lane fetched its own row's residual a load instruction touched 32 cache lines: 17 us of load-unit time per
@@ -215,13 +234,14 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         // A piece's residual (32 columns) is asked for one piece ahead.
         done = true;
         using T16 = typename std::conditional<kOut == 1, __half, __nv_bfloat16>::type;
-        using R = typename std::conditional<kOut == 2, float4, uint2>::type;             // four values
-        constexpr int kElem = kOut == 2 ? 4 : 2, kPieces = 2 * kGroupsPerWarp;
+        using R = typename std::conditional<kF32, float4, uint2>::type;             // four values
+        constexpr int kElem = kF32 ? 4 : 2, kPieces = 2 * kGroupsPerWarp;
         const int r0 = lg * 32 + (lane >> 3), c4 = 4 * (lane & 7);
         const int n_pieces = u_count * kPieces;
         auto first_row = [&](int i) { return (2 * ((pair + i * n_pairs) / n_tiles) + static_cast<int>(rank)) * kBlockM + r0; };
         auto first_col = [&](int i, int p) { return ((pair + i * n_pairs) % n_tiles) * kBlockN + (gsel * kPieces + p) * 32 + c4; };
         auto fetch = [&](int idx, R (&r)[8]) {
+          if (kSplit) return;
           const int i = idx / kPieces, row = first_row(i);
           const uint8_t* src = static_cast<const uint8_t*>(args.resid) + (static_cast<long long>(row) * args.N + first_col(i, idx % kPieces)) * kElem;
 #pragma unroll
@@ -242,7 +262,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           R next[8];
           if (idx + 1 < n_pieces) fetch(idx + 1, next);
           const int col = first_col(i, p);
-          const float4 sc = args.scale.data != nullptr ? args.scale.load4(col) : make_float4(1.f, 1.f, 1.f, 1.f);
+          const float4 sc = !kSplit && args.scale.data != nullptr ? args.scale.load4(col) : make_float4(1.f, 1.f, 1.f, 1.f);
           tmem_ld_wait();
           if (p == kPieces - 1) {
             // Last read of the accumulator by this warp: hand it back before the arithmetic and the stores.
@@ -253,7 +273,20 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           float v[32];
 #pragma unroll
           for (int c = 0; c < 32; ++c) v[c] = __uint_as_float(acc[c]);
-          if (args.gelu) {
+          if constexpr (kSplit) {
+            if (args.rows.by_channel) {           // neighbouring lanes hold neighbouring frames of a channel
+              const int chan0 = ((pair + i * n_pairs) % n_tiles) * kBlockN + (gsel * kPieces + p) * 32;
+              const long long at = args.rows.out_at((2 * ((pair + i * n_pairs) / n_tiles) + static_cast<int>(rank)) * kBlockM + lg * 32 + lane,
+                                                    args.M, args.N);
+              float* dst = static_cast<float*>(args.y) + at + static_cast<long long>(chan0) * args.rows.clip_valid;
+              if (at >= 0) {
+#pragma unroll
+                for (int c = 0; c < 32; ++c) dst[static_cast<long long>(c) * args.rows.clip_valid] = v[c];
+              }
+              continue;
+            }
+          }
+          if (!kSplit && args.gelu) {
 #pragma unroll
             for (int c = 0; c < 32; c += 2) gelu_erf2(v[c], v[c + 1]);
           }
@@ -266,8 +299,13 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
             float4 o = *reinterpret_cast<const float4*>(slab + sw128_offset(4 * k + (lane >> 3), lane & 7));
+            if constexpr (kSplit) {
+              const int at = args.rows.out_row(row + 4 * k, args.M);
+              if (at >= 0) *reinterpret_cast<float4*>(static_cast<float*>(args.y) + static_cast<long long>(at) * args.N + col) = o;
+              continue;
+            }
             o.x *= sc.x; o.y *= sc.y; o.z *= sc.z; o.w *= sc.w;
-            if constexpr (kOut == 2) {
+            if constexpr (kF32) {
               o.x += res[k].x; o.y += res[k].y; o.z += res[k].z; o.w += res[k].w;
               if (row + 4 * k < args.M) *reinterpret_cast<float4*>(dst + static_cast<long long>(4 * k) * args.N * 4) = o;
             } else {
@@ -344,7 +382,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             v[4 * j] *= s.x; v[4 * j + 1] *= s.y; v[4 * j + 2] *= s.z; v[4 * j + 3] *= s.w;
           }
         }
-        if constexpr (kOut == 2) {
+        if constexpr (kF32) {
           // FP32 output: two 32-column halves (128-byte rows) through the same 4 KB slab.
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -405,19 +443,26 @@ static int encode_2d(CUtensorMap* map, CUtensorMapDataType type, int elem_bytes,
 }
 
 template <int kOut, bool kWide, int kBlockN>
-static int launch_pairs(const void* a, const void* w, void* y, const LinearArgs& args, int pair_tiles, int max_pairs, int in_dtype,
+static int launch_pairs(const void* a, const void* w, const SplitLow* low, void* y, const LinearArgs& args, int pair_tiles, int max_pairs, int in_dtype,
                         int out_dtype, int* status, cudaStream_t st, int dependent) {
   using namespace lin;
   using S = Shape<kWide, kBlockN>;
-  CUtensorMap tmap_a, tmap_w, tmap_y;
+  CUtensorMap tmap_a, tmap_w, tmap_y, tmap_a_lo = {}, tmap_w_lo = {};
   const CUtensorMapDataType t16 = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;   // any 16-bit element type moves alike
   const uint64_t M = static_cast<uint64_t>(args.M), N = static_cast<uint64_t>(args.N), K = static_cast<uint64_t>(args.K);
-  int rc = encode_2d(&tmap_a, t16, 2, a, M, K, kBlockM, kBlockK);
+  const uint64_t a_rows = kOut == 4 ? static_cast<uint64_t>(low->a_rows) : M;
+  const uint64_t a_cols = kOut == 4 ? static_cast<uint64_t>(args.rows.a_chunks) * kBlockK : K;
+  int rc = encode_2d(&tmap_a, t16, 2, a, a_rows, a_cols, kBlockM, kBlockK);
   if (rc != 0) return rc;
   rc = encode_2d(&tmap_w, t16, 2, w, N, K, S::kHalfN, kBlockK);
   if (rc != 0) return rc;
-  if (out_dtype == 3)      // no tiled store in this mode: a placeholder map over a
-    rc = encode_2d(&tmap_y, t16, 2, a, M, K, 32, 64);
+  if constexpr (kOut == 4) {
+    rc = encode_2d(&tmap_a_lo, t16, 2, low->a, a_rows, a_cols, kBlockM, kBlockK);
+    if (rc == 0) rc = encode_2d(&tmap_w_lo, t16, 2, low->w, N, K, S::kHalfN, kBlockK);
+    if (rc != 0) return rc;
+  }
+  if (out_dtype >= 3)      // no tiled store in these modes: a placeholder map over a
+    rc = encode_2d(&tmap_y, t16, 2, a, a_rows, a_cols, 32, 64);
   else if (out_dtype == 2)
     rc = encode_2d(&tmap_y, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, y, M, N, 32, 32);
   else
@@ -430,8 +475,8 @@ static int launch_pairs(const void* a, const void* w, void* y, const LinearArgs&
   auto kern = linear_gemm_kernel<kOut, kWide, kBlockN>;
   rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), S::kSmemBytes);
   if (rc != 0) return rc;
-  return launch_kernel(kern, dim3(2 * n_pairs), S::kThreads, S::kSmemBytes, st, 1, dependent, tmap_a, tmap_w, tmap_y, args, total_units,
-                       idesc, status);
+  return launch_kernel(kern, dim3(2 * n_pairs), S::kThreads, S::kSmemBytes, st, 1, dependent, tmap_a, tmap_w, tmap_y, tmap_a_lo,
+                       tmap_w_lo, args, total_units, idesc, status);
 }
 
 int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N,
@@ -455,8 +500,8 @@ int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, co
   const bool wide = gelu || out_dtype == 3;
   const int waves256 = (pair_tiles * (N / 256) + max_pairs - 1) / max_pairs, waves128 = (pair_tiles * (N / 128) + max_pairs - 1) / max_pairs;
   const bool halves = !wide && 9 * waves128 < 16 * waves256;
-  LinearArgs args = {scale, resid, M, N, K, gelu ? 1 : 0, out_dtype == 3 ? static_cast<uint4*>(y) : nullptr, y};
-  using Fn = int (*)(const void*, const void*, void*, const LinearArgs&, int, int, int, int, int*, cudaStream_t, int);
+  LinearArgs args = {scale, resid, M, N, K, gelu ? 1 : 0, out_dtype == 3 ? static_cast<uint4*>(y) : nullptr, y, {}};
+  using Fn = int (*)(const void*, const void*, const SplitLow*, void*, const LinearArgs&, int, int, int, int, int*, cudaStream_t, int);
   Fn fn;
   if (wide)
     fn = out_dtype == 3 ? launch_pairs<3, true, 256>
@@ -465,7 +510,30 @@ int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, co
     fn = out_dtype == 2 ? launch_pairs<2, false, 128> : (out_dtype == 1 ? launch_pairs<1, false, 128> : launch_pairs<0, false, 128>);
   else
     fn = out_dtype == 2 ? launch_pairs<2, false, 256> : (out_dtype == 1 ? launch_pairs<1, false, 256> : launch_pairs<0, false, 256>);
-  return fn(a, w, y, args, pair_tiles, max_pairs, in_dtype, out_dtype, status, st, dependent);
+  return fn(a, w, nullptr, y, args, pair_tiles, max_pairs, in_dtype, out_dtype, status, st, dependent);
+}
+
+int launch_linear_split(const void* a_hi, const void* a_lo, long long a_rows, int a_cols, const void* w_hi, const void* w_lo, float* y,
+                        long long rows, int clip_rows, int clip_valid, int by_channel, int N, int K, int* status, cudaStream_t st) {
+  using namespace lin;
+  if (rows < 0 || a_rows > 0x7fffffffLL || a_rows < rows || N <= 0 || K <= 0 || N % 256 != 0 || a_cols <= 0 || a_cols % kBlockK != 0 ||
+      K % a_cols != 0 || clip_rows <= 0 || clip_valid <= 0 || clip_valid > clip_rows)
+    return -1;
+  if (rows == 0) return 0;
+  if (a_hi == nullptr || a_lo == nullptr || w_hi == nullptr || w_lo == nullptr || y == nullptr) return -1;
+  if ((reinterpret_cast<uintptr_t>(a_hi) | reinterpret_cast<uintptr_t>(a_lo) | reinterpret_cast<uintptr_t>(w_hi) |
+       reinterpret_cast<uintptr_t>(w_lo) | reinterpret_cast<uintptr_t>(y)) & 15u)
+    return -3;
+  const int M = static_cast<int>(rows);
+  const SplitLow low = {a_lo, w_lo, a_rows};
+  const SplitRows map = {a_cols / kBlockK, clip_rows, clip_valid, by_channel};
+  if (few_row_tiles(M, N)) return launch_linear_split_small(a_hi, w_hi, low, map, y, M, N, K, status, st);
+  const int pair_tiles = ((M + kBlockM - 1) / kBlockM + 1) / 2;
+  const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
+  const int waves256 = (pair_tiles * (N / 256) + max_pairs - 1) / max_pairs, waves128 = (pair_tiles * (N / 128) + max_pairs - 1) / max_pairs;
+  const LinearArgs args = {ParamVec(nullptr), nullptr, M, N, K, 0, nullptr, y, map};
+  auto fn = 9 * waves128 < 16 * waves256 ? launch_pairs<4, false, 128> : launch_pairs<4, false, 256>;      // as above
+  return fn(a_hi, w_hi, &low, y, args, pair_tiles, max_pairs, 1, 4, status, st, 0);
 }
 
 }  // namespace fm

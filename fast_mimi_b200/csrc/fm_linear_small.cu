@@ -54,10 +54,12 @@ __device__ __forceinline__ void bulk_copy_to_cta(uint32_t dst, const void* src, 
 }
 }  // namespace small
 
-// kOut: 0 = BF16, 1 = FP16, 2 = FP32 output and residual; 3 = q | k | v with RoPE (VT: type of v)
+// kOut: 0 = BF16, 1 = FP16, 2 = FP32 output and residual; 3 = q | k | v with RoPE (VT: type of v); 4 = FP32 output of a
+// split-precision product: K runs three times (lo W_hi, hi W_lo, hi W_hi), shared out like any other K
 template <int kOut, typename VT, int kBlockN>
 __global__ void __launch_bounds__(small::kThreads)
 linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
+                    const __grid_constant__ CUtensorMap tmap_a_lo, const __grid_constant__ CUtensorMap tmap_w_lo,
                     const __grid_constant__ SmallArgs args, uint32_t idesc, int* status) {
   using namespace small;
   constexpr int kStageBytes = Tile<kBlockN>::kStageBytes, kRedBytes = Tile<kBlockN>::kRedBytes, kTmemCols = kBlockN;
@@ -107,20 +109,35 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   if (warp == 4) {
     if (lane == 0) {
       tma_prefetch_desc(&tmap_a);
+      auto load_a = [&](int st, int kc) {
+        if constexpr (kOut == 4) {
+          const int k = kc % args.k_part;         // a row of the product continues in the matrix's next row
+          tma_load_2d(smem + st * kStageBytes, kc < args.k_part ? &tmap_a_lo : &tmap_a, &bars->full[st],
+                      k % args.rows.a_chunks * kBlockK, m0 + k / args.rows.a_chunks);
+        } else {
+          tma_load_2d(smem + st * kStageBytes, &tmap_a, &bars->full[st], kc * kBlockK, m0);
+        }
+      };
+      auto load_w = [&](int st, int kc) {
+        if constexpr (kOut == 4)
+          tma_load_2d(smem + st * kStageBytes + kABytes, kc / args.k_part == 1 ? &tmap_w_lo : &tmap_w, &bars->full[st],
+                      kc % args.k_part * kBlockK, n0);
+        else
+          tma_load_2d(smem + st * kStageBytes + kABytes, &tmap_w, &bars->full[st], kc * kBlockK, n0);
+      };
       const int ahead = args.chunks < kStages ? args.chunks : kStages;
       for (int i = 0; i < ahead; ++i) {
         mbar_arrive_expect_tx(&bars->full[i], kStageBytes);
-        tma_load_2d(smem + i * kStageBytes + kABytes, &tmap_w, &bars->full[i], (chunk0 + i) * kBlockK, n0);
+        load_w(i, chunk0 + i);
       }
       griddep_wait();
-      for (int i = 0; i < ahead; ++i)
-        tma_load_2d(smem + i * kStageBytes, &tmap_a, &bars->full[i], (chunk0 + i) * kBlockK, m0);
+      for (int i = 0; i < ahead; ++i) load_a(i, chunk0 + i);
       for (int i = ahead; i < args.chunks; ++i) {
         const int st = i % kStages;
         mbar_wait(&bars->empty[st], (static_cast<uint32_t>(i / kStages) & 1u) ^ 1u, ctl, status, kErrWaitConsumer);
         mbar_arrive_expect_tx(&bars->full[st], kStageBytes);
-        tma_load_2d(smem + st * kStageBytes + kABytes, &tmap_w, &bars->full[st], (chunk0 + i) * kBlockK, n0);
-        tma_load_2d(smem + st * kStageBytes, &tmap_a, &bars->full[st], (chunk0 + i) * kBlockK, m0);
+        load_w(st, chunk0 + i);
+        load_a(st, chunk0 + i);
       }
     }
     __syncwarp();
@@ -238,23 +255,32 @@ static int choose_split(int tiles, int k_chunks) {
 
 template <int kOut, typename VT, int kBlockN>
 static int launch_tiles(const void* a, const void* w, SmallArgs& args, int K, int in_dtype, int* status,
-                        cudaStream_t st, int dependent) {
+                        cudaStream_t st, int dependent, const SplitLow* low) {
   using namespace small;
-  CUtensorMap tmap_a, tmap_w;
-  int rc = encode_rows_16bit(&tmap_a, a, static_cast<uint64_t>(args.M), static_cast<uint64_t>(K), kBlockM, kBlockK);
+  CUtensorMap tmap_a, tmap_w, tmap_a_lo = {}, tmap_w_lo = {};
+  const uint64_t a_rows = kOut == 4 ? static_cast<uint64_t>(low->a_rows) : static_cast<uint64_t>(args.M);
+  const uint64_t a_cols = kOut == 4 ? static_cast<uint64_t>(args.rows.a_chunks) * kBlockK : static_cast<uint64_t>(K);
+  int rc = encode_rows_16bit(&tmap_a, a, a_rows, a_cols, kBlockM, kBlockK);
   if (rc != 0) return rc;
   rc = encode_rows_16bit(&tmap_w, w, static_cast<uint64_t>(args.N), static_cast<uint64_t>(K), kBlockN, kBlockK);
   if (rc != 0) return rc;
   const int m_tiles = (args.M + kBlockM - 1) / kBlockM, n_tiles = args.N / kBlockN;
-  args.split = choose_split(m_tiles * n_tiles, K / kBlockK);
-  args.chunks = K / kBlockK / args.split;
+  if constexpr (kOut == 4) {
+    rc = encode_rows_16bit(&tmap_a_lo, low->a, a_rows, a_cols, kBlockM, kBlockK);
+    if (rc == 0) rc = encode_rows_16bit(&tmap_w_lo, low->w, static_cast<uint64_t>(args.N), static_cast<uint64_t>(K), kBlockN, kBlockK);
+    if (rc != 0) return rc;
+  }
+  args.k_part = K / kBlockK;
+  const int k_chunks = kOut == 4 ? 3 * args.k_part : args.k_part;
+  args.split = choose_split(m_tiles * n_tiles, k_chunks);
+  args.chunks = k_chunks / args.split;
   const int fmt = in_dtype == 1 ? 0 : 1;
   const uint32_t idesc = umma_idesc_f16(kBlockM, kBlockN, fmt, fmt, 0, 0);
   auto kern = linear_small_kernel<kOut, VT, kBlockN>;
   rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), Tile<kBlockN>::kSmemBytes);
   if (rc != 0) return rc;
   return launch_kernel(kern, dim3(n_tiles * args.split, m_tiles), kThreads, Tile<kBlockN>::kSmemBytes, st, args.split, dependent, tmap_a,
-                       tmap_w, args, idesc, status);
+                       tmap_w, tmap_a_lo, tmap_w_lo, args, idesc, status);
 }
 
 // 64-column tiles, or 32 where 64 would leave the K split at its limit of eight with SMs to spare: the partial sums that
@@ -262,12 +288,12 @@ static int launch_tiles(const void* a, const void* w, SmallArgs& args, int K, in
 // 14 KB with 32), and halving the tile halves them.
 template <int kOut, typename VT>
 static int launch_small(const void* a, const void* w, SmallArgs& args, int K, int in_dtype, int* status, cudaStream_t st,
-                        int dependent) {
+                        int dependent, const SplitLow* low = nullptr) {
   if constexpr (kOut != 3) {
     if (static_cast<long long>((args.M + 127) / 128) * (args.N / 64) * 8 <= sm_count())
-      return launch_tiles<kOut, VT, 32>(a, w, args, K, in_dtype, status, st, dependent);
+      return launch_tiles<kOut, VT, 32>(a, w, args, K, in_dtype, status, st, dependent, low);
   }
-  return launch_tiles<kOut, VT, 64>(a, w, args, K, in_dtype, status, st, dependent);
+  return launch_tiles<kOut, VT, 64>(a, w, args, K, in_dtype, status, st, dependent, low);
 }
 
 int launch_linear_small(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N, int K,
@@ -282,6 +308,16 @@ int launch_linear_small(const void* a, const void* w, void* y, ParamVec scale, c
   if (out_dtype == 2) return launch_small<2, __half>(a, w, args, K, in_dtype, status, st, dependent);
   if (out_dtype == 1) return launch_small<1, __half>(a, w, args, K, in_dtype, status, st, dependent);
   return launch_small<0, __half>(a, w, args, K, in_dtype, status, st, dependent);
+}
+
+int launch_linear_split_small(const void* a_hi, const void* w_hi, const SplitLow& low, const SplitRows& map, float* y, int M, int N,
+                              int K, int* status, cudaStream_t st) {
+  SmallArgs args = {};
+  args.y = y;
+  args.M = M;
+  args.N = N;
+  args.rows = map;
+  return launch_small<4, __half>(a_hi, w_hi, args, K, 1, status, st, 0, &low);
 }
 
 int launch_qkv_small(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status,

@@ -23,6 +23,7 @@
 // 5.86e-3.  Callers pass 4.5e-3 / 6.0e-3.
 #include "fm_common.cuh"
 #include "fm_kernels.h"
+#include "fm_launch.h"
 
 namespace fm {
 
@@ -168,35 +169,62 @@ __device__ __forceinline__ float rvq_margin(float xx, float e_max, float tau_rel
   return tau_rel * sqrtf(xx) * e_max + 3.1e-5f * e_max;
 }
 
+// Bound by the residual's way through memory and by latency: a frame is a chain of loads (record, entry, store).  So a
+// frame's record and residual are asked for one frame ahead; where one entry alone is a candidate (five frames of six) it has
+// won and its distance is not evaluated; and after the last layer (kLast) the residual is neither updated nor, for those
+// frames, read.
+template <bool kLast>
 __global__ void __launch_bounds__(rvq::kWarps * 32)
 rvq_select_rec_kernel(const uint4* __restrict__ records, const float* __restrict__ codebook, float* __restrict__ resid,
                       uint16_t* __restrict__ resid16, long long* __restrict__ codes, int* __restrict__ n_candidates,
                       float* __restrict__ tau, long long rows, int n_groups, float e_max_next, float tau_rel,
                       int* __restrict__ status) {
   using namespace rvq;
+  griddep_launch();
+  griddep_wait();
   const int lane = threadIdx.x & 31;
   const long long warp0 = static_cast<long long>(blockIdx.x) * kWarps + (threadIdx.x >> 5);
   const long long stride = static_cast<long long>(gridDim.x) * kWarps;
+  struct Frame {
+    uint4 rec;                 // this lane's group (entries 64 * lane .. 64 * lane + 63): its minimum and its mask
+    float4 a, b;               // this lane's eight residual values
+    float margin;
+  };
+  auto fetch_x = [&](long long row, Frame& f) {
+    const float4* xr = reinterpret_cast<const float4*>(resid + row * kDim + lane * 8);
+    f.a = xr[0];
+    f.b = xr[1];
+  };
+  auto fetch = [&](long long row, Frame& f) {
+    f.rec = make_uint4(__float_as_uint(INFINITY), 0u, 0u, 0u);
+    if (lane < n_groups) f.rec = records[row * n_groups + lane];
+    f.margin = tau[row];
+    if constexpr (!kLast) fetch_x(row, f);
+  };
+  Frame next;
+  if (warp0 < rows) fetch(warp0, next);
   for (long long row = warp0; row < rows; row += stride) {
-    float x[8];
-    {
-      const float4* xr = reinterpret_cast<const float4*>(resid + row * kDim + lane * 8);
-      const float4 a = xr[0], b = xr[1];
-      x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-    }
-    // this lane's group (entries 64 * lane .. 64 * lane + 63): its minimum and its mask
-    uint4 rec = make_uint4(__float_as_uint(INFINITY), 0u, 0u, 0u);
-    if (lane < n_groups) rec = records[row * n_groups + lane];
-    const float gmin = __uint_as_float(rec.x);
+    Frame f = next;
+    if (row + stride < rows) fetch(row + stride, next);
+    const float gmin = __uint_as_float(f.rec.x);
     float d_min = gmin;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) d_min = fminf(d_min, __shfl_xor_sync(0xffffffffu, d_min, o));
-    const float limit = d_min + tau[row];
-    unsigned long long mine = gmin <= limit ? (static_cast<unsigned long long>(rec.z) << 32) | rec.y : 0ull;
+    const float limit = d_min + f.margin;
+    const unsigned long long mine = gmin <= limit ? (static_cast<unsigned long long>(f.rec.z) << 32) | f.rec.y : 0ull;
 
     float best = INFINITY;
     int best_j = 0, n_cand = 0;
     unsigned lanes = __ballot_sync(0xffffffffu, mine != 0ull);
+    if (__reduce_add_sync(0xffffffffu, __popcll(mine)) == 1 && limit < INFINITY) {
+      const int src = __ffs(lanes) - 1;
+      best_j = src * 64 + __ffsll(static_cast<long long>(__shfl_sync(0xffffffffu, mine, src))) - 1;
+      n_cand = 1;
+      lanes = 0u;
+    } else if constexpr (kLast) {
+      fetch_x(row, f);
+    }
+    float x[8] = {f.a.x, f.a.y, f.a.z, f.a.w, f.b.x, f.b.y, f.b.z, f.b.w};
     while (lanes != 0u) {
       const int src = __ffs(lanes) - 1;
       lanes &= lanes - 1u;
@@ -223,7 +251,7 @@ rvq_select_rec_kernel(const uint4* __restrict__ records, const float* __restrict
         }
       }
     }
-    {
+    if constexpr (!kLast) {
       const float4* er = reinterpret_cast<const float4*>(codebook + static_cast<size_t>(best_j) * kDim + lane * 8);
       const float4 a = __ldg(er), b = __ldg(er + 1);
       const float ev[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
@@ -256,6 +284,7 @@ __global__ void __launch_bounds__(rvq::kWarps * 32)
 rvq_prepare_kernel(const float* __restrict__ x, uint16_t* __restrict__ resid16, float* __restrict__ tau, long long rows,
                    float e_max, float tau_rel) {
   using namespace rvq;
+  griddep_launch();
   const int lane = threadIdx.x & 31;
   const long long warp0 = static_cast<long long>(blockIdx.x) * kWarps + (threadIdx.x >> 5);
   const long long stride = static_cast<long long>(gridDim.x) * kWarps;
@@ -295,16 +324,10 @@ split_half_kernel(const float* __restrict__ x, uint16_t* __restrict__ hi, uint16
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = i0; i < n8; i += stride) {
     const float4 a = reinterpret_cast<const float4*>(x)[2 * i], b = reinterpret_cast<const float4*>(x)[2 * i + 1];
-    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    uint32_t h[4], l[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      h[e] = Pack16<__half>::pack(v[2 * e], v[2 * e + 1]);
-      const float2 back = Pack16<__half>::unpack(h[e]);
-      l[e] = Pack16<__half>::pack(v[2 * e] - back.x, v[2 * e + 1] - back.y);
-    }
-    reinterpret_cast<uint4*>(hi)[i] = make_uint4(h[0], h[1], h[2], h[3]);
-    reinterpret_cast<uint4*>(lo)[i] = make_uint4(l[0], l[1], l[2], l[3]);
+    uint4 h, l;
+    split_half8(a, b, h, l);
+    reinterpret_cast<uint4*>(hi)[i] = h;
+    reinterpret_cast<uint4*>(lo)[i] = l;
   }
 }
 
@@ -329,6 +352,51 @@ rvq_decode_kernel(const long long* __restrict__ codes, const float* __restrict__
       acc.x += e.x; acc.y += e.y; acc.z += e.z; acc.w += e.w;
     }
     reinterpret_cast<float4*>(out + row * kDim)[sub] = acc;
+  }
+}
+
+// The same sums for the output projections: as FP16 hi + lo parts, of both stacks of a split quantiser side by side, from
+// codes as the caller holds them.  64 threads per frame and stack, four dimensions each; a frame's entries are independent
+// loads (eight in flight), added in the layers' order.
+__global__ void __launch_bounds__(256)
+rvq_decode_split_kernel(const long long* __restrict__ codes, const float* __restrict__ books0, const float* __restrict__ books1,
+                        uint16_t* __restrict__ hi, uint16_t* __restrict__ lo, int rows, int T, int n_layers, int n0, int n_codes0,
+                        int n_codes1, int* __restrict__ bad_code) {
+  using namespace rvq;
+  const int stacks = n0 < n_layers ? 2 : 1, per_block = 4 / stacks;
+  const int sub = threadIdx.x & 63, stack = stacks == 2 ? (threadIdx.x >> 6) & 1 : 0;
+  const float* books = stack == 0 ? books0 : books1;
+  const int n_codes = stack == 0 ? n_codes0 : n_codes1, l0 = stack == 0 ? 0 : n0, l1 = stack == 0 ? n0 : n_layers;
+  for (long long row = static_cast<long long>(blockIdx.x) * per_block + (threadIdx.x >> 6) / stacks; row < rows;
+       row += static_cast<long long>(gridDim.x) * per_block) {
+    const long long b = row / T, t = row - b * T;
+    const long long* code = codes + b * n_layers * T + t;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int l = l0; l < l1; l += 8) {
+      float4 e[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (l + i < l1) {
+          long long c = code[static_cast<long long>(l + i) * T];
+          if (c < 0 || c >= n_codes) {                // recorded, not dereferenced
+            if (bad_code != nullptr) atomicExch(bad_code, 1);
+            c = 0;
+          }
+          e[i] = __ldg(reinterpret_cast<const float4*>(books + (static_cast<size_t>(l + i - l0) * n_codes + static_cast<size_t>(c)) * kDim + sub * 4));
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (l + i < l1) {
+          acc.x += e[i].x; acc.y += e[i].y; acc.z += e[i].z; acc.w += e[i].w;
+        }
+      }
+    }
+    const uint32_t h0 = Pack16<__half>::pack(acc.x, acc.y), h1 = Pack16<__half>::pack(acc.z, acc.w);
+    const float2 b0 = Pack16<__half>::unpack(h0), b1 = Pack16<__half>::unpack(h1);
+    const long long at = (row * stacks + stack) * kDim + sub * 4;
+    *reinterpret_cast<uint2*>(hi + at) = make_uint2(h0, h1);
+    *reinterpret_cast<uint2*>(lo + at) = make_uint2(Pack16<__half>::pack(acc.x - b0.x, acc.y - b0.y), Pack16<__half>::pack(acc.z - b1.x, acc.w - b1.y));
   }
 }
 
@@ -365,7 +433,7 @@ int launch_rvq_select(const void* scores, int scores_fp16, const float* e_sq, co
 
 int launch_rvq_select_rec(const void* records, const float* codebook, float* resid, void* resid16, long long* codes,
                           int* n_candidates, float* tau, long long rows, int n_codes, float e_max_next, float tau_rel,
-                          int* status, cudaStream_t st) {
+                          int* status, cudaStream_t st, int dependent, int last) {
   if (rows < 0 || n_codes <= 0 || n_codes % 64 != 0 || n_codes > 2048 || !(e_max_next >= 0.f) || !(tau_rel >= 0.f)) return -1;
   if (rows == 0) return 0;
   if (records == nullptr || codebook == nullptr || resid == nullptr || resid16 == nullptr || codes == nullptr || tau == nullptr)
@@ -374,10 +442,29 @@ int launch_rvq_select_rec(const void* records, const float* codebook, float* res
        reinterpret_cast<uintptr_t>(resid16)) & 15u)
     return -3;
   const int grid = grid_for((rows + rvq::kWarps - 1) / rvq::kWarps, 8);
-  rvq_select_rec_kernel<<<grid, rvq::kWarps * 32, 0, st>>>(static_cast<const uint4*>(records), codebook, resid,
-                                                          static_cast<uint16_t*>(resid16), codes, n_candidates, tau, rows,
-                                                          n_codes / 64, e_max_next, tau_rel, status);
-  return static_cast<int>(cudaGetLastError());
+  return launch_kernel(last ? rvq_select_rec_kernel<true> : rvq_select_rec_kernel<false>, dim3(grid), rvq::kWarps * 32, 0, st, 1, dependent,
+                       static_cast<const uint4*>(records), codebook, resid, static_cast<uint16_t*>(resid16), codes, n_candidates, tau,
+                       rows, n_codes / 64, e_max_next, tau_rel, status);
+}
+
+// The whole stack: the launches of all layers behind one another, each allowed to begin while the one in front still runs.
+int launch_rvq_encode(float* resid, void* resid16, float* tau, void* records, const void* books16, const float* books, const float* e_sq,
+                      const float* e_max, long long* codes, int* n_candidates, long long rows, int n_codes, int layers, float tau_rel,
+                      int* status, cudaStream_t st) {
+  if (rows < 0 || rows > 0x7fffffffLL || layers <= 0 || n_codes <= 0 || n_codes % 256 != 0 || n_codes > 2048 || e_max == nullptr) return -1;
+  if (rows == 0) return 0;
+  int rc = launch_rvq_prepare(resid, resid16, tau, rows, e_max[0], tau_rel, st);
+  for (int l = 0; l < layers && rc == 0; ++l) {
+    const size_t entry0 = static_cast<size_t>(l) * n_codes;
+    rc = launch_linear_gemm(resid16, static_cast<const uint16_t*>(books16) + entry0 * rvq::kDim, records, e_sq + entry0, tau,
+                            static_cast<int>(rows), n_codes, rvq::kDim, 1, 3, 0, status, st, 1);
+    if (rc != 0) return rc;
+    const int last = l + 1 == layers;
+    rc = launch_rvq_select_rec(records, books + entry0 * rvq::kDim, resid, resid16, codes + l * rows,
+                               n_candidates != nullptr ? n_candidates + l * rows : nullptr, tau, rows, n_codes,
+                               last ? 0.f : e_max[l + 1], tau_rel, status, st, 1, last);
+  }
+  return rc;
 }
 
 int launch_rvq_prepare(const float* x, void* resid16, float* tau, long long rows, float e_max, float tau_rel,
@@ -406,6 +493,22 @@ int launch_split_half(const float* x, void* hi, void* lo, long long n, cudaStrea
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 15u) return -3;
   const long long n8 = n / 8;
   split_half_kernel<<<grid_for((n8 + 255) / 256, 8), 256, 0, st>>>(x, static_cast<uint16_t*>(hi), static_cast<uint16_t*>(lo), n8);
+  return static_cast<int>(cudaGetLastError());
+}
+
+int launch_rvq_decode_split(const long long* codes, const float* books0, const float* books1, void* hi, void* lo, int B, int T,
+                            int n_layers, int n0, int n_codes0, int n_codes1, int* bad_code, cudaStream_t st) {
+  const long long rows = static_cast<long long>(B) * T;
+  if (B < 0 || T < 0 || rows > 0x7fffffffLL || n0 <= 0 || n0 > n_layers || n_codes0 <= 0 || (n0 < n_layers && n_codes1 <= 0)) return -1;
+  if (rows == 0) return 0;
+  if (codes == nullptr || books0 == nullptr || (n0 < n_layers && books1 == nullptr) || hi == nullptr || lo == nullptr) return -1;
+  if ((reinterpret_cast<uintptr_t>(books0) | reinterpret_cast<uintptr_t>(books1) | reinterpret_cast<uintptr_t>(hi) |
+       reinterpret_cast<uintptr_t>(lo)) & 15u)
+    return -3;
+  const int per_block = n0 < n_layers ? 2 : 4;
+  rvq_decode_split_kernel<<<grid_for((rows + per_block - 1) / per_block, 8), 256, 0, st>>>(
+      codes, books0, books1, static_cast<uint16_t*>(hi), static_cast<uint16_t*>(lo), static_cast<int>(rows), T, n_layers, n0, n_codes0,
+      n_codes1, bad_code);
   return static_cast<int>(cudaGetLastError());
 }
 

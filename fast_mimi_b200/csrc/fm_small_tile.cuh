@@ -25,13 +25,15 @@ struct SmallArgs {
   int split;              // S, blocks per cluster
   int gelu;
   QkvEpilogueArgs qkv;    // kOut 3
+  SplitRows rows;         // kOut 4
+  int k_part;             // kOut 4: K / 64 of one of the three products
 };
 
 // What the epilogue of eight values of row `row` of output tile `ntile` (64 columns, one attention head) reads besides the
 // product: columns 4j .. 4j + 3 ([0]) and 32 + 4j .. ([1]), the two halves of RoPE pairs.  Asked for before the product
 // is complete, so that its latency does not follow the reduction's.  With tiles of 32 columns (kHalves 1) a piece is four
 // values.
-// kOut: 0 = BF16, 1 = FP16, 2 = FP32 output and residual; 3 = q | k | v with RoPE.
+// kOut: 0 = BF16, 1 = FP16, 2 = FP32 output and residual; 3 = q | k | v with RoPE; 4 = FP32 output of a split-precision product.
 struct PieceOperands {
   float4 a[2];            // residual, or cos and sin
   float4 s[2];            // per-channel scale
@@ -47,7 +49,7 @@ __device__ __forceinline__ void load_operands(const SmallArgs& args, int row, in
       p.a[0] = *reinterpret_cast<const float4*>(ep.cos + at);
       p.a[1] = *reinterpret_cast<const float4*>(ep.sin + at);
     }
-  } else {
+  } else if constexpr (kOut != 4) {
     const int col = ntile * 32 * kHalves + 4 * j;
     const long long at = static_cast<long long>(row) * args.N + col;
 #pragma unroll
@@ -108,6 +110,23 @@ __device__ __forceinline__ void finish_piece(const SmallArgs& args, float (&lo)[
         *reinterpret_cast<uint2*>(dst + 32) = phi;
       }
     }
+  } else if constexpr (kOut == 4) {
+    if (args.rows.by_channel) {
+      const long long at = args.rows.out_at(row, args.M, args.N), step = args.rows.clip_valid;
+      if (at < 0) return;
+      float* y = static_cast<float*>(args.y) + at + (ntile * 32 * kHalves + 4 * j) * step;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        y[e * step] = lo[e];
+        if constexpr (kHalves == 2) y[(32 + e) * step] = hi[e];
+      }
+      return;
+    }
+    const int out = args.rows.out_row(row, args.M);
+    if (out < 0) return;
+    float* y = static_cast<float*>(args.y) + static_cast<long long>(out) * args.N + ntile * 32 * kHalves + 4 * j;
+    *reinterpret_cast<float4*>(y) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+    if constexpr (kHalves == 2) *reinterpret_cast<float4*>(y + 32) = make_float4(hi[0], hi[1], hi[2], hi[3]);
   } else {
     const long long at = static_cast<long long>(row) * args.N + ntile * 32 * kHalves + 4 * j;
     float* part[2] = {lo, hi};

@@ -71,12 +71,18 @@ class MimiUpsampleB200(nn.Module):
             raise ValueError("only the causal trimming of Mimi's configuration (two trailing frames) is built")
         self.conv = inner
 
+    def _taps(self) -> torch.Tensor:
+        return self.conv.weight.detach().float().reshape(self.conv.in_channels, 4).contiguous()
+
     def frames(self, x: torch.Tensor) -> torch.Tensor:
         """``x [B, T, C]`` (frame-major) -> ``[B, 2T, C]`` float32."""
-        w = self.conv.weight.detach().float().reshape(self.conv.in_channels, 4).contiguous()
-        return ops.upsample2(x.float().contiguous(), w)
+        return ops.upsample2(x.float().contiguous(), self._taps())
 
     def forward(self, hidden_states: torch.Tensor) -> torch.Tensor:
         if not hidden_states.is_cuda:
             raise RuntimeError("MimiUpsampleB200 runs on a CUDA device only; there is no CPU path")
-        return self.frames(hidden_states.transpose(1, 2)).transpose(1, 2).to(hidden_states.dtype)
+        x = hidden_states
+        if (x.dtype == torch.float32 and x.dim() == 3 and x.is_contiguous() and x.shape[1] == self.conv.in_channels
+                and x.shape[1] % 32 == 0 and x.shape[0] <= 65535):
+            return ops.upsample2_channels(x, self._taps()).transpose(1, 2)
+        return self.frames(x.transpose(1, 2)).transpose(1, 2).to(x.dtype)

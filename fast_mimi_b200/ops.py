@@ -6,6 +6,8 @@ used only for device memory and streams.
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _native
@@ -514,7 +516,6 @@ def band_attention_fp32(q, k, v, *, window, scale, q_offset=0, k_offset=0, frame
         out = torch.empty(q.shape, dtype=torch.float32, device=q.device)
     _need(out.shape == q.shape and out.dtype == torch.float32 and out.stride(-1) == 1, "out must be shaped like q")
     strides = _strides3(q, frame_major) + _strides3(k, frame_major) + _strides3(v, frame_major) + _strides3(out, frame_major)
-    import ctypes
     arr = (ctypes.c_longlong * 12)(*strides)
     rc = lib.fm_band_attn_fp32_verify(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, H, D, Tq, Tk,
                                       int(q_offset), int(k_offset), int(window), float(scale),
@@ -573,6 +574,20 @@ class RVQCodebooks:
         self.layers, self.entries = codebooks.shape[0], codebooks.shape[1]
 
 
+def _rvq_search(resid, books: RVQCodebooks, codes, cand, st, resid16=None):
+    """The stack's layers on ``resid [rows, 256]`` float32, which is overwritten, into ``codes [layers, rows]``."""
+    layers, rows = codes.shape
+    if resid16 is None:
+        resid16 = torch.empty(rows, RVQ_DIM, dtype=torch.float16, device=resid.device)
+    tau = torch.empty(rows, dtype=torch.float32, device=resid.device)
+    records = torch.empty(rows, books.entries // 64, 4, dtype=torch.int32, device=resid.device)
+    rc = _native.load().fm_rvq_encode_f32(
+        resid.data_ptr(), resid16.data_ptr(), tau.data_ptr(), records.data_ptr(), books.half.data_ptr(), books.vectors.data_ptr(),
+        books.sq.data_ptr(), (ctypes.c_float * len(books.e_max))(*books.e_max), codes.data_ptr(), _ptr(cand), rows, books.entries,
+        layers, RVQ_TAU_REL[torch.float32], st, _stream())          # FP32 accumulators feed the comparison directly
+    _native.check(rc, "fm_rvq_encode_f32")
+
+
 def rvq_encode(x, books: RVQCodebooks, num_quantizers=None, *, return_candidates=False, scores_dtype=None, status=None):
     """Codes ``[layers, rows]`` int64 of the residual quantiser stack for ``x [rows, 256]`` float32 (the output
     of the branch's ``input_proj``).  Per layer: inner products with all entries on the tensor core (FP16
@@ -591,21 +606,7 @@ def rvq_encode(x, books: RVQCodebooks, num_quantizers=None, *, return_candidates
     cand = torch.empty(layers, rows, dtype=torch.int32, device=x.device) if return_candidates else None
     st = _status_ptr(status, x)
     if scores_dtype is None:
-        tau_rel = RVQ_TAU_REL[torch.float32]          # FP32 accumulators feed the comparison directly
-        tau = torch.empty(rows, dtype=torch.float32, device=x.device)
-        records = torch.empty(rows, books.entries // 64, 4, dtype=torch.int32, device=x.device)
-        _native.check(lib.fm_rvq_prepare_f32(resid.data_ptr(), resid16.data_ptr(), tau.data_ptr(), rows, books.e_max[0],
-                                             tau_rel, _stream()), "fm_rvq_prepare_f32")
-        for l in range(layers):
-            rc = lib.fm_rvq_candidates_f16(resid16.data_ptr(), books.half[l].data_ptr(), books.sq[l].data_ptr(),
-                                           tau.data_ptr(), records.data_ptr(), rows, books.entries, st, _stream())
-            _native.check(rc, "fm_rvq_candidates_f16")
-            e_next = books.e_max[l + 1] if l + 1 < layers else 0.0
-            rc = lib.fm_rvq_select_rec_f32(records.data_ptr(), books.vectors[l].data_ptr(), resid.data_ptr(),
-                                           resid16.data_ptr(), codes[l].data_ptr(),
-                                           cand[l].data_ptr() if cand is not None else None, tau.data_ptr(), rows,
-                                           books.entries, e_next, tau_rel, st, _stream())
-            _native.check(rc, "fm_rvq_select_rec_f32")
+        _rvq_search(resid, books, codes, cand, st, resid16)
         return (codes, cand) if return_candidates else codes
     _need(scores_dtype in RVQ_TAU_REL, "scores_dtype must be None, float16 or float32")
     scores = torch.empty(rows, books.entries, dtype=scores_dtype, device=x.device)
@@ -632,14 +633,33 @@ def split_half(x):
 
 def linear_split(x, w_parts, *, status=None):
     """``x [rows, K] @ w^T`` with FP32-grade accuracy on the FP16 tensor core: ``x`` float32, ``w_parts`` the pair
-    ``split_half(w)`` of a float32 ``[N, K]`` weight.  Three products with FP32 accumulation chained through the
-    linear kernel's FP32 residual input: ``hi W_hi + hi W_lo + lo W_hi`` (the dropped ``lo W_lo`` term is below
-    2^-22 of the result).  K a multiple of 64, N of 256."""
+    ``split_half(w)`` of a float32 ``[N, K]`` weight.  One product over three times K with FP32 accumulation:
+    ``hi W_hi + hi W_lo + lo W_hi`` (the dropped ``lo W_lo`` term is below 2^-22 of the result).  K a multiple of 64, N of
+    256."""
+    return _linear_parts(split_half(x.contiguous()), w_parts, x.shape[:-1], status)
+
+
+def _check_weight_parts(w_parts, k):
     w_hi, w_lo = w_parts
-    x_hi, x_lo = split_half(x.contiguous())
-    y = linear(x_hi, w_lo, out_dtype=torch.float32, status=status)
-    y2 = linear(x_lo, w_hi, residual=y, out_dtype=torch.float32, status=status)
-    return linear(x_hi, w_hi, residual=y2, out_dtype=torch.float32, out=y, status=status)
+    for w in w_parts:
+        _need(w.is_cuda and w.dtype == torch.float16 and w.is_contiguous() and w.dim() == 2 and w.shape == w_hi.shape
+              and w.shape[1] == k, f"w must be contiguous torch.float16 [N, {k}]")
+    _need(k % 64 == 0 and w_hi.shape[0] % 256 == 0, "K must be a multiple of 64 and N a multiple of 256")
+    return w_hi, w_lo
+
+
+def _linear_parts(x_parts, w_parts, shape, status):
+    """``linear_split`` of an already split ``x`` (``[.., K]`` each part): float32 ``[*shape, N]``."""
+    x_hi, x_lo = x_parts
+    k = x_hi.shape[-1]
+    w_hi, w_lo = _check_weight_parts(w_parts, k)
+    rows, n = x_hi.numel() // k, w_hi.shape[0]
+    y = torch.empty((*shape, n), dtype=torch.float32, device=x_hi.device)
+    if rows:
+        rc = _native.load().fm_linear_split_f32(x_hi.data_ptr(), x_lo.data_ptr(), rows, k, w_hi.data_ptr(), w_lo.data_ptr(),
+                                                y.data_ptr(), rows, 1, 1, 0, n, k, _status_ptr(status, x_hi), _stream())
+        _native.check(rc, "fm_linear_split_f32")
+    return y
 
 
 def downsample_conv(x, w_parts, *, kernel=4, stride=2, status=None):
@@ -653,14 +673,37 @@ def downsample_conv(x, w_parts, *, kernel=4, stride=2, status=None):
     w_hi, w_lo = w_parts
     _need(w_hi.shape == w_lo.shape and w_hi.shape[1] == kernel * C, f"weight parts must be [C_out, {kernel * C}]")
     t_out = (T + stride - 1) // stride
+    if kernel % stride == 0 and (stride * C) % 64 == 0 and B * t_out > 0:
+        # frames laid out once with their padding; a row of the product is kernel / stride rows of `stride` frames
+        _check_weight_parts(w_parts, kernel * C)
+        extra = kernel // stride - 1
+        hi = torch.empty(B * (t_out + extra), stride * C, dtype=torch.float16, device=x.device)
+        lo = torch.empty_like(hi)
+        _native.check(lib.fm_conv_frames_split(x.data_ptr(), hi.data_ptr(), lo.data_ptr(), B, T, C, kernel, stride, _stream()),
+                      "fm_conv_frames_split")
+        y = torch.empty(B, t_out, w_hi.shape[0], dtype=torch.float32, device=x.device)
+        rc = lib.fm_linear_split_f32(hi.data_ptr(), lo.data_ptr(), hi.shape[0], stride * C, w_hi.data_ptr(), w_lo.data_ptr(),
+                                     y.data_ptr(), hi.shape[0] - extra, t_out + extra, t_out, 0, w_hi.shape[0], kernel * C,
+                                     _status_ptr(status, x), _stream())
+        _native.check(rc, "fm_linear_split_f32")
+        return y
     hi = torch.empty(B * t_out, kernel * C, dtype=torch.float16, device=x.device)
     lo = torch.empty_like(hi)
     _native.check(lib.fm_conv_rows_split(x.data_ptr(), hi.data_ptr(), lo.data_ptr(), B, T, C, kernel, stride, _stream()),
                   "fm_conv_rows_split")
-    y = linear(hi, w_lo, out_dtype=torch.float32, status=status)
-    y2 = linear(lo, w_hi, residual=y, out_dtype=torch.float32, status=status)
-    y = linear(hi, w_hi, residual=y2, out_dtype=torch.float32, out=y, status=status)
-    return y.view(B, t_out, w_hi.shape[0])
+    return _linear_parts((hi, lo), w_parts, (B, t_out), status)
+
+
+def upsample2_channels(x, weight):
+    """``upsample2`` of channel-major activations: ``x [B, C, T]`` float32 (C a multiple of 32) -> ``[B, 2T, C]``."""
+    _need(x.is_cuda and x.dtype == torch.float32 and x.dim() == 3 and x.is_contiguous(), "x must be contiguous CUDA float32 [B, C, T]")
+    B, C, T = x.shape
+    _need(weight.is_cuda and weight.dtype == torch.float32 and weight.is_contiguous() and tuple(weight.shape) == (C, 4)
+          and C % 32 == 0 and B <= 65535, f"weight must be contiguous CUDA float32 [{C}, 4]")
+    y = torch.empty(B, 2 * T, C, dtype=torch.float32, device=x.device)
+    _native.check(_native.load().fm_upsample2_channels_f32(x.data_ptr(), weight.data_ptr(), y.data_ptr(), B, T, C, _stream()),
+                  "fm_upsample2_channels_f32")
+    return y
 
 
 def upsample2(x, weight):
@@ -673,6 +716,36 @@ def upsample2(x, weight):
           and C % 4 == 0, f"weight must be contiguous CUDA float32 [{C}, 4]")
     y = torch.empty(B, 2 * T, C, dtype=torch.float32, device=x.device)
     _native.check(lib.fm_upsample2_f32(x.data_ptr(), weight.data_ptr(), y.data_ptr(), B, T, C, _stream()), "fm_upsample2_f32")
+    return y
+
+
+def rvq_decode_project(codes, first: RVQCodebooks, second: RVQCodebooks | None, w_parts, *, status=None):
+    """The ordered sums of one or two quantiser stacks and their output projections: ``codes [B, K, T]`` int64 (the first
+    stack's layers first) -> ``[B, N, T]`` float32.  ``w_parts``: ``split_half`` of ``[N, 256]``, or of the stacks'
+    projections side by side, ``[N, 512]``."""
+    lib = _native.load()
+    _need(codes.is_cuda and codes.dtype == torch.int64 and codes.dim() == 3, "codes must be CUDA int64 [batch, layers, frames]")
+    B, K, T = codes.shape
+    n0 = K if second is None else first.layers
+    _need(0 < n0 <= first.layers and (second is None or 0 < K - n0 <= second.layers), "more code layers than codebooks")
+    width = RVQ_DIM * (1 if second is None else 2)
+    w_hi, w_lo = _check_weight_parts(w_parts, width)
+    codes = codes.contiguous()
+    hi = torch.empty(B * T, width, dtype=torch.float16, device=codes.device)
+    lo = torch.empty_like(hi)
+    y = torch.empty(B, w_hi.shape[0], T, dtype=torch.float32, device=codes.device)
+    bad = torch.zeros(1, dtype=torch.int32, device=codes.device)
+    if B * T:
+        rc = lib.fm_rvq_decode_split(codes.data_ptr(), first.vectors.data_ptr(), None if second is None else second.vectors.data_ptr(),
+                                     hi.data_ptr(), lo.data_ptr(), B, T, K, n0, first.entries,
+                                     0 if second is None else second.entries, bad.data_ptr(), _stream())
+        _native.check(rc, "fm_rvq_decode_split")
+        rc = lib.fm_linear_split_f32(hi.data_ptr(), lo.data_ptr(), B * T, width, w_hi.data_ptr(), w_lo.data_ptr(), y.data_ptr(), B * T,
+                                     T, T, 1, w_hi.shape[0], width, _status_ptr(status, codes), _stream())
+        _native.check(rc, "fm_linear_split_f32")
+    if int(bad.item()) != 0:
+        raise RuntimeError("rvq_decode: a code index is outside the codebook")
+    check_status(codes.device, status)      # the stream is already synchronised by the read above
     return y
 
 

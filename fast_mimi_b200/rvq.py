@@ -17,6 +17,20 @@ import torch.nn as nn
 from . import ops
 
 
+class _Frames:
+    """Embeddings ``[B, C, T]`` as frame-major float32 rows, with their FP16 hi + lo parts made once for all branches."""
+
+    def __init__(self, embeddings: torch.Tensor) -> None:
+        B, _, T = embeddings.shape
+        self.rows = embeddings.float().permute(0, 2, 1).reshape(B * T, -1).contiguous()
+        self._parts = None
+
+    def parts(self):
+        if self._parts is None:
+            self._parts = ops.split_half(self.rows)
+        return self._parts
+
+
 class MimiRVQB200:
     def __init__(self, codebooks: torch.Tensor, input_proj: torch.Tensor | None, output_proj: torch.Tensor | None) -> None:
         self.books = ops.RVQCodebooks(codebooks)
@@ -27,12 +41,10 @@ class MimiRVQB200:
         self._out_parts = None if self.output_proj is None else ops.split_half(self.output_proj)
 
     @staticmethod
-    def _project(x: torch.Tensor, w: torch.Tensor, parts) -> torch.Tensor:
+    def _on_tensor_core(w: torch.Tensor) -> bool:
         # the tensor-core kernel takes K in multiples of 64 and N in multiples of 256 (Mimi: 512 -> 256 and back);
         # other geometries (the reference's tiny test configuration) take the FP32 CUDA-core kernel
-        if w.shape[1] % 64 == 0 and w.shape[0] % 256 == 0:
-            return ops.linear_split(x, parts)
-        return ops.linear_fp32(x, w)
+        return w.shape[1] % 64 == 0 and w.shape[0] % 256 == 0
 
     @classmethod
     def from_reference(cls, rvq: nn.Module) -> "MimiRVQB200":
@@ -45,21 +57,38 @@ class MimiRVQB200:
     def encode(self, embeddings: torch.Tensor, num_quantizers: int | None = None) -> torch.Tensor:
         ops._need(embeddings.is_cuda and embeddings.dim() == 3, "embeddings must be CUDA [batch, channels, frames]")
         B, _, T = embeddings.shape
-        x = embeddings.float().permute(0, 2, 1).reshape(B * T, -1)
-        if self.input_proj is not None:
-            x = self._project(x.contiguous(), self.input_proj, self._in_parts)
-        codes = ops.rvq_encode(x.contiguous(), self.books, num_quantizers)
+        layers = self._layers(num_quantizers)
+        codes = torch.empty(layers, B * T, dtype=torch.int64, device=embeddings.device)
+        self._encode_frames(_Frames(embeddings), codes)
         # codes are the end of the device pipeline: a recorded error (a timed-out wait in a kernel upstream, a
         # non-finite residual) must not leave as plausible-looking indices
         ops.check_status(embeddings.device)
-        return codes.view(codes.shape[0], B, T)
+        return codes.view(layers, B, T)
+
+    def _layers(self, num_quantizers: int | None) -> int:
+        layers = self.books.layers if num_quantizers is None else int(num_quantizers)
+        ops._need(0 < layers <= self.books.layers, "num_quantizers out of range")
+        return layers
+
+    def _encode_frames(self, frames: "_Frames", codes: torch.Tensor) -> None:
+        """Codes of the first ``len(codes)`` layers into ``codes [layers, frames]``; nothing is read back."""
+        if self.input_proj is None:
+            x = frames.rows.clone()
+        elif self._on_tensor_core(self.input_proj):
+            x = ops._linear_parts(frames.parts(), self._in_parts, (len(frames.rows),), None)
+        else:
+            x = ops.linear_fp32(frames.rows, self.input_proj)
+        ops._need(x.shape[1] == ops.RVQ_DIM, "x must be CUDA float32 [rows, 256]")
+        ops._rvq_search(x, self.books, codes, None, ops._status_ptr(None, x))
 
     def decode(self, codes: torch.Tensor) -> torch.Tensor:
         ops._need(codes.is_cuda and codes.dim() == 3, "codes must be CUDA [batch, quantizers, frames]")
         B, K, T = codes.shape
+        if self.output_proj is not None and self._on_tensor_core(self.output_proj):
+            return ops.rvq_decode_project(codes, self.books, None, self._out_parts)
         q = ops.rvq_decode(codes.transpose(0, 1).reshape(K, B * T).contiguous(), self.books)
         if self.output_proj is not None:
-            q = self._project(q, self.output_proj, self._out_parts)
+            q = ops.linear_fp32(q, self.output_proj)
         return q.view(B, T, -1).permute(0, 2, 1).contiguous()
 
 
@@ -68,6 +97,18 @@ class MimiSplitRVQB200:
         self.semantic, self.acoustic = semantic, acoustic
         self.num_semantic_quantizers = semantic.books.layers
         self.max_num_quantizers = semantic.books.layers + acoustic.books.layers
+        self._joint: tuple | None = None
+        self._joint_out_parts()
+
+    def _joint_out_parts(self):
+        """Both output projections as one weight over [semantic | acoustic], whose accumulator then adds the branches; made
+        once for a pair of branches, ``None`` where they do not fit together."""
+        sem, aco = self.semantic, self.acoustic
+        w0, w1 = sem.output_proj, aco.output_proj
+        if self._joint is None or self._joint[0] is not w0 or self._joint[1] is not w1:
+            fits = w0 is not None and w1 is not None and w0.shape == w1.shape and sem._on_tensor_core(w0) and w0.device == w1.device
+            self._joint = (w0, w1, ops.split_half(torch.cat((w0, w1), dim=1)) if fits else None)
+        return self._joint[2]
 
     @classmethod
     def from_reference(cls, split: nn.Module) -> "MimiSplitRVQB200":
@@ -78,15 +119,27 @@ class MimiSplitRVQB200:
         count = self.max_num_quantizers if num_quantizers is None else int(num_quantizers)
         if not self.num_semantic_quantizers <= count <= self.max_num_quantizers:
             raise ValueError(f"num_quantizers must be in [{self.num_semantic_quantizers}, {self.max_num_quantizers}]")
-        codes = self.semantic.encode(embeddings)
-        if count > self.num_semantic_quantizers:
-            codes = torch.cat((codes, self.acoustic.encode(embeddings, count - self.num_semantic_quantizers)), dim=0)
-        return codes
+        ops._need(embeddings.is_cuda and embeddings.dim() == 3, "embeddings must be CUDA [batch, channels, frames]")
+        B, _, T = embeddings.shape
+        n_sem = self.semantic._layers(None)
+        acoustic = count - self.num_semantic_quantizers
+        codes = torch.empty(n_sem + acoustic, B * T, dtype=torch.int64, device=embeddings.device)
+        frames = _Frames(embeddings)
+        self.semantic._encode_frames(frames, codes[:n_sem])
+        if acoustic > 0:
+            self.acoustic._layers(acoustic)
+            self.acoustic._encode_frames(frames, codes[n_sem:])
+        ops.check_status(embeddings.device)
+        return codes.view(len(codes), B, T)
 
     def decode(self, codes: torch.Tensor) -> torch.Tensor:
         """``codes [B, K, T]``: semantic layers first (src/fast_mimi/model.py:2408-2444 per branch); the two
         branches' outputs are added."""
         n_sem = self.num_semantic_quantizers
+        if codes.is_cuda and codes.dim() == 3 and n_sem == self.semantic.books.layers < codes.shape[1]:
+            parts = self._joint_out_parts()
+            if parts is not None:
+                return ops.rvq_decode_project(codes, self.semantic.books, self.acoustic.books, parts)
         out = self.semantic.decode(codes[:, :n_sem].contiguous())
         if codes.shape[1] > n_sem:
             out = out + self.acoustic.decode(codes[:, n_sem:].contiguous())

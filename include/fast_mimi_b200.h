@@ -180,9 +180,24 @@ int fm_rvq_select_f32(const void* scores, int scores_dtype, const float* e_sq, c
  * MimiConv1d(512, 512, kernel 4, stride 2, no bias, replicate padding, causal), src/fast_mimi/model.py:2734-2744):
  * for frame-major FP32 x [B, T, C], row (b, t) of the result is frames stride*t - (kernel - stride) .. + kernel - 1
  * of clip b, clamped to the clip (replicate padding on both sides), C values each, as FP16 hi + lo parts
- * [B * ceil(T / stride), kernel * C].  The convolution itself is then fm_linear_f16 with the kernel laid out as
- * [C_out, kernel * C_in] (three products: hi W_hi + hi W_lo + lo W_hi, FP32 residual chaining). */
+ * [B * ceil(T / stride), kernel * C].  The convolution itself is then fm_linear_split_f32 with the kernel laid out as
+ * [C_out, kernel * C_in]. */
 int fm_conv_rows_split(const float* x, void* hi, void* lo, int B, int T, int C, int kernel, int stride, void* stream);
+
+/* The same convolution's input for a kernel that is a multiple of the stride: the padded frames themselves, each written
+ * once, as FP16 hi + lo parts [B, stride * (ceil(T / stride) + kernel / stride - 1), C]. */
+int fm_conv_frames_split(const float* x, void* hi, void* lo, int B, int T, int C, int kernel, int stride, void* stream);
+
+/* y = (a_hi + a_lo)(w_hi + w_lo)^T in FP32 grade on the FP16 tensor core (hi W_hi + hi W_lo + lo W_hi in one accumulator):
+ * the 1 x 1 projections around the quantiser (src/fast_mimi/model.py:2392-2406) and the downsampling convolution.
+ *   a_hi/lo  [a_rows, a_cols] FP16, a_cols a multiple of 64; w_hi/lo [n_out, k_in] FP16, n_out a multiple of 256
+ *   rows     row r of the product lies in rows r .. r + k_in / a_cols - 1 of a (k_in = a_cols: a plain matrix; over
+ *            padded frames seen as rows of `stride` frames: the convolution); rows <= a_rows
+ *   y        FP32 [.., n_out]: of every clip_rows rows the first clip_valid, back to back (equal: all rows); with
+ *            by_channel [rows / clip_rows, n_out, clip_valid] */
+int fm_linear_split_f32(const void* a_hi, const void* a_lo, long long a_rows, int a_cols, const void* w_hi, const void* w_lo,
+                        float* y, long long rows, int clip_rows, int clip_valid, int by_channel, int n_out, int k_in, int* status,
+                        void* stream);
 
 /* The stride-2 upsampling that precedes the decoder transformer (MimiModel.upsample: MimiConvTranspose1d(512, 512,
  * kernel 4, stride 2, groups 512, no bias), src/fast_mimi/model.py:2745-2753; its forward trims the last two output
@@ -190,12 +205,23 @@ int fm_conv_rows_split(const float* x, void* hi, void* lo, int B, int T, int C, 
  * y[b, n, c] = w[c, n % 2] x[b, n / 2, c] + w[c, n % 2 + 2] x[b, n / 2 - 1, c]. */
 int fm_upsample2_f32(const float* x, const float* w, float* y, int B, int T, int C, void* stream);
 
+/* The same from channel-major x [B, C, T], in which the quantiser's decode leaves it (C a multiple of 32). */
+int fm_upsample2_channels_f32(const float* x, const float* w, float* y, int B, int T, int C, void* stream);
+
 /* x = hi + lo, both FP16 (hi = round(x), lo = round(x - hi)), n a multiple of 8 values: the operands of an
- * FP32-grade product on the FP16 tensor core (hi W_hi + hi W_lo + lo W_hi via fm_linear_f16 with FP32 residual
- * chaining).  Used for the quantiser's 1 x 1 input / output projections (nn.Conv1d(kernel 1, no bias),
+ * FP32-grade product on the FP16 tensor core (fm_linear_split_f32).  Used for the quantiser's 1 x 1 input / output projections (nn.Conv1d(kernel 1, no bias),
  * src/fast_mimi/model.py:2392-2406, applied at :2417 and :2443), whose results decide code indices and must
  * therefore keep FP32 accuracy. */
 int fm_split_half(const float* x, void* hi, void* lo, long long n, void* stream);
+
+/* The three calls below for a whole stack (src/fast_mimi/model.py:2408-2429), as one chain of dependent launches:
+ *   residual     [rows, 256] FP32, the stack's input; overwritten
+ *   residual16   [rows, 256] FP16, tau [rows], records [rows, n_codes / 64] x 16 B: workspaces
+ *   codebooks(16) [layers, n_codes, 256], e_sq [layers, n_codes], e_max [layers] in HOST memory
+ *   codes        [layers, rows]; n_candidates [layers, rows] or NULL */
+int fm_rvq_encode_f32(float* residual, void* residual16, float* tau, void* records, const void* codebooks16, const float* codebooks,
+                      const float* e_sq, const float* e_max, long long* codes, int* n_candidates, long long rows, int n_codes, int layers,
+                      float tau_rel, int* status, void* stream);
 
 /* The same layer without the scores' round trip through memory (replaces the same reference lines as
  * fm_rvq_select_f32: src/fast_mimi/model.py:2277-2291, :2420-2427), three calls:
@@ -226,6 +252,12 @@ int fm_rvq_to_half(const float* x, void* y, long long rows, void* stream);
  *   bad_code: optional device int set to 1 when an index is out of range (that index is then read as 0). */
 int fm_rvq_decode_f32(const long long* codes, const float* codebooks, float* out, long long rows, int n_layers,
                       int n_codes, int* bad_code, void* stream);
+
+/* The same sums of the two stacks of a split quantiser (src/fast_mimi/model.py:2447-2480) as FP16 hi + lo parts, the
+ * operands of their output projections: codes [B, n_layers, T], the first n0 layers of codebooks books0 [n0, n_codes0, 256],
+ * the others of books1 -> hi, lo [B * T, 512] (first stack in columns 0..255; n0 = n_layers: [B * T, 256]). */
+int fm_rvq_decode_split(const long long* codes, const float* books0, const float* books1, void* hi, void* lo, int B, int T,
+                        int n_layers, int n0, int n_codes0, int n_codes1, int* bad_code, void* stream);
 
 /* The part of MimiAttention.forward between the input and o_proj (src/fast_mimi/model.py:1896-1951) for a call
  * without cache: fm_attention_fused_bf16 for clips of 128 < T <= 256 frames, else fm_qkv_rope_bf16 followed by

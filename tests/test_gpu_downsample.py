@@ -99,3 +99,38 @@ def test_upsample_module_keeps_the_reference_call_shape():
         mod(x.cpu())
     with pytest.raises(ValueError):
         fm.MimiUpsampleB200(types.SimpleNamespace(conv=torch.nn.ConvTranspose1d(512, 512, 4, 2, bias=False)))
+
+
+@pytest.mark.parametrize("kernel,stride,C", [(6, 2, 64), (3, 2, 64), (4, 4, 128), (2, 1, 64), (4, 2, 16)])
+@pytest.mark.parametrize("B,T", [(1, 5), (9, 130), (70, 140)])
+def test_convolutions_of_other_shapes(kernel, stride, C, B, T):
+    """Kernels of one to three strides over padded frames, one that is no multiple of its stride and one whose rows are too
+    narrow (gathered rows), against FP64."""
+    import fast_mimi_b200 as fm
+    g = torch.Generator().manual_seed(kernel * 100 + T)
+    weight = torch.randn(256, C, kernel, generator=g) / (C * kernel) ** 0.5
+    x = torch.randn(B, T, C, generator=g)
+    pad = (-T) % stride
+    wide = torch.nn.functional.pad(x.double().transpose(1, 2), (kernel - stride, pad), mode="replicate")
+    want = torch.nn.functional.conv1d(wide, weight.double(), stride=stride).transpose(1, 2)
+    if (kernel * C) % 64 != 0:
+        pytest.skip("K must be a multiple of 64")
+    got = fm.ops.downsample_conv(x.cuda(), _weight_parts(weight), kernel=kernel, stride=stride).cpu()
+    assert got.shape == want.shape
+    assert float((got - want).abs().max() / want.abs().max()) < 2e-6
+
+
+@pytest.mark.parametrize("B,T", [(1, 1), (2, 32), (3, 33), (2, 64), (64, 125)])
+def test_upsample_from_channel_major(B, T):
+    """The tile that turns round in shared memory gives what the frame-major kernel gives, but for which of the two
+    products is rounded before the sum: each result is within 2^-24 (|w a| + |w p| + |y|) of the exact one."""
+    import types
+    import fast_mimi_b200 as fm
+    conv = torch.nn.ConvTranspose1d(512, 512, 4, 2, groups=512, bias=False).cuda()
+    mod = fm.MimiUpsampleB200(types.SimpleNamespace(conv=conv, padding_left=0, padding_right=2))
+    x = torch.randn(B, 512, T, device="cuda")
+    got, want = mod(x).detach(), mod.frames(x.transpose(1, 2)).transpose(1, 2)
+    with torch.no_grad():
+        conv.weight.abs_()
+    size = mod.frames(x.abs().transpose(1, 2)).transpose(1, 2)              # |w a| + |w p|
+    assert bool(((got - want).abs() <= 2.0 ** -22 * size).all())

@@ -154,3 +154,25 @@ def test_split_quantizer_wrapper_matches_oracle_encode_and_decode():
     assert O.rel_l2(dec, ref) < 1e-5
     with pytest.raises(ValueError):
         native.encode(emb.cuda(), 0)
+
+
+@pytest.mark.parametrize("B,T,stacks", [(1, 1, 2), (3, 43, 2), (2, 300, 1), (64, 125, 2), (7, 1000, 1)])
+def test_decode_with_projection_matches_fp64(B, T, stacks):
+    """Ordered sums, hi + lo split, joint projection and the channel-major store, with few rows (split K) and many (pairs)."""
+    import fast_mimi_b200 as fm
+    g = torch.Generator().manual_seed(B * 100 + T)
+    books = [torch.randn(n, 512, 256, generator=g) for n in ((1, 9)[:stacks] if stacks == 2 else (9,))]
+    w = [torch.randn(512, 256, 1, generator=g) / 16 for _ in books]
+    branch = [fm.MimiRVQB200(b.cuda(), None, p.cuda()) for b, p in zip(books, w)]
+    q = fm.MimiSplitRVQB200(*branch) if stacks == 2 else branch[0]
+    codes = torch.randint(0, 512, (B, 10 if stacks == 2 else 9, T), generator=g)
+    want, l = 0, 0
+    for b, p in zip(books, w):
+        sums = sum(b[i][codes[:, l + i]].double() for i in range(len(b)))       # [B, T, 256]
+        want, l = want + torch.einsum("btk,ck->bct", sums, p[:, :, 0].double()), l + len(b)
+    got = q.decode(codes.cuda())
+    assert got.shape == want.shape and got.is_contiguous()
+    assert float((got.cpu().double() - want).abs().max() / want.abs().max()) < 2e-6
+    codes[B - 1, 0, T - 1] = 512
+    with pytest.raises(RuntimeError, match="outside the codebook"):
+        q.decode(codes.cuda())
