@@ -36,7 +36,7 @@ SIGNATURES: dict[str, list] = {
     "fm_rvq_select_f32": [_P, _I, _P, _P, _P, _P, _P, _P, _LL, _I, _F, _F, _P, _P],
     "fm_conv_rows_split": [_P, _P, _P, _I, _I, _I, _I, _I, _P],
     "fm_conv_frames_split": [_P, _P, _P, _I, _I, _I, _I, _I, _P],
-    "fm_linear_split_f32": [_P, _P, _LL, _I, _P, _P, _P, _LL, _I, _I, _I, _I, _I, _P, _P],
+    "fm_linear_split_f32": [_P, _P, _LL, _I, _P, _P, _P, _LL, _I, _I, _I, _I, _I, _I, _P, _P],
     "fm_upsample2_channels_f32": [_P, _P, _P, _I, _I, _I, _P],
     "fm_rvq_decode_split": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "fm_upsample2_f32": [_P, _P, _P, _I, _I, _I, _P],
@@ -48,6 +48,7 @@ SIGNATURES: dict[str, list] = {
     "fm_rvq_to_half": [_P, _P, _LL, _P],
     "fm_rvq_decode_f32": [_P, _P, _P, _LL, _I, _I, _P, _P],
     "fm_band_attn_prefill_bf16": [_P, _P, _P, _P, _I, _I, _I, _F, _I, _P, _P],
+    "fm_window_attention": [_P, _P, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _F, _I, _P, _P],
     "fm_attention_prefill_bf16": [_P, _P, _P, _P, _LL, _P, _P, _P, _P, _I, _I, _I, _F, _I, _P, _P],
     "fm_band_attn_chunk_bf16": [_P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _P, _P],
     "fm_attention_fused_bf16": [_P, _P, _P, _P, _LL, _P, _I, _I, _I, _F, _I, _P, _P],

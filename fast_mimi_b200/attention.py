@@ -45,9 +45,11 @@ def native_window_attention(query: torch.Tensor, key: torch.Tensor, value: torch
     def frames(t, dtype):   # [B,H,T,D] -> contiguous [B,T,H*D] (a no-op view for the reference's layout)
         return t.transpose(1, 2).to(dtype).contiguous().view(B, T, H * D)
 
+    if ops.window_attention_takes(query, key, value, value_dtype):
+        return ops.window_attention(query, key, value, window=window, scale=scale, value_dtype=value_dtype)
     out = ops.band_attention_prefill(frames(query, torch.bfloat16), frames(key, torch.bfloat16),
                                      frames(value, value_dtype), window=window, scale=scale)
-    return out.view(B, T, H, D).transpose(1, 2).to(query.dtype)
+    return out.view(B, T, H, D).to(query.dtype).transpose(1, 2)
 
 
 def window_attention_fp32(query, key, value, *, scale, window, q_offset=0, k_offset=0):
@@ -68,6 +70,10 @@ def window_attention_nlc(query: torch.Tensor, key: torch.Tensor, value: torch.Te
               "query must be [B, 8, T, 64]")
     ops._need(key.shape == query.shape and value.shape == query.shape, "key/value must match query")
     B, H, T, D = query.shape
+
+    if ops.window_attention_takes(query, key, value, value_dtype):
+        out = ops.window_attention(query, key, value, window=window, scale=scale, value_dtype=value_dtype)
+        return out.transpose(1, 2).view(B, T, H * D)
 
     def frames(t, dtype):
         return t.transpose(1, 2).to(dtype).contiguous().view(B, T, H * D)

@@ -122,6 +122,16 @@ static int prefill_two_kernels(const void* x, const void* w_qkv, const float* co
                                       static_cast<cudaStream_t>(stream), 1);
 }
 
+int fm_window_attention(const void* q, const void* k, const void* v, int in_dtype, const long long* strides, void* q_ws, void* k_ws,
+                        void* v_ws, void* out16, float* out32, int B, int T, int window, float scale, int value_dtype, int* status,
+                        void* stream) {
+  if (strides == nullptr || value_dtype < 0 || value_dtype > 1) return -1;
+  const void* const qkv[3] = {q, k, v};
+  void* const ws[3] = {q_ws, k_ws, v_ws};
+  return fm::launch_window_attention(qkv, in_dtype, strides, ws, out16, out32, B, T, window, scale, value_dtype, status,
+                                     static_cast<cudaStream_t>(stream));
+}
+
 int fm_attention_prefill_bf16(const void* x, const void* w_qkv, const float* cos, const float* sin,
                               long long cos_bstride, void* q_ws, void* k_ws, void* v_ws, void* out, int B, int T,
                               int window, float scale, int value_dtype, int* status, void* stream) {
@@ -211,9 +221,9 @@ int fm_conv_frames_split(const float* x, void* hi, void* lo, int B, int T, int C
 }
 
 int fm_linear_split_f32(const void* a_hi, const void* a_lo, long long a_rows, int a_cols, const void* w_hi, const void* w_lo,
-                        float* y, long long rows, int clip_rows, int clip_valid, int by_channel, int n_out, int k_in, int* status,
+                        float* y, long long rows, int clip_rows, int clip_valid, int by_channel, int n_mats, int n_out, int k_in, int* status,
                         void* stream) {
-  return fm::launch_linear_split(a_hi, a_lo, a_rows, a_cols, w_hi, w_lo, y, rows, clip_rows, clip_valid, by_channel, n_out, k_in, status,
+  return fm::launch_linear_split(a_hi, a_lo, a_rows, a_cols, w_hi, w_lo, y, rows, clip_rows, clip_valid, by_channel, n_mats, n_out, k_in, status,
                                  static_cast<cudaStream_t>(stream));
 }
 

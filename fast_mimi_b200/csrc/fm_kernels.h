@@ -68,11 +68,19 @@ int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, co
 // a_cols]; row r of the product has K = a_cols * n values and lies in rows r .. r + n - 1 of `a` (n = 1: a plain matrix; n = 2:
 // a convolution of twice its stride over padded frames).  Of every clip_rows rows the first clip_valid are results, stored
 // back to back: y [rows * clip_valid / clip_rows, N]; or, with by_channel, clip by clip with the channels outside: y
-// [rows / clip_rows, N, clip_valid].
+// [rows / clip_rows, N, clip_valid].  n_mats > 1: y is so many matrices [.., N / n_mats], one behind the other (several weights'
+// products with the same rows).
 struct SplitRows {
   int a_chunks;           // a_cols / 64
   int clip_rows, clip_valid;
   int by_channel;
+  int cols;               // N / n_mats
+  long long mat_step;     // values of one of the matrices
+  // where column `col` (of a tile that lies in one matrix) of result row `row` goes
+  __host__ __device__ __forceinline__ long long at(int row, int col) const {
+    const int mat = col / cols;
+    return mat * mat_step + static_cast<long long>(row) * cols + (col - mat * cols);
+  }
   __host__ __device__ __forceinline__ int out_row(int row, int M) const {
     if (row >= M) return -1;
     if (clip_rows == clip_valid) return row;
@@ -90,7 +98,7 @@ struct SplitLow {
   long long a_rows;
 };
 int launch_linear_split(const void* a_hi, const void* a_lo, long long a_rows, int a_cols, const void* w_hi, const void* w_lo, float* y,
-                        long long rows, int clip_rows, int clip_valid, int by_channel, int N, int K, int* status, cudaStream_t st);
+                        long long rows, int clip_rows, int clip_valid, int by_channel, int n_mats, int N, int K, int* status, cudaStream_t st);
 int launch_linear_split_small(const void* a_hi, const void* w_hi, const SplitLow& low, const SplitRows& map, float* y, int M, int N,
                               int K, int* status, cudaStream_t st);
 // Padded frames of a causal convolution (kernel a multiple of stride), split into FP16 hi + lo parts: clip b has
@@ -174,8 +182,13 @@ int launch_attn_fused_clip(const void* x, const void* w_qkv, const float* cos, c
 bool use_fused_clip(int B, int T);
 int launch_band_attn_clip(const void* q, const void* k, const void* v, void* out, int B, int T, int window,
                           float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent = 0);
+// out_fp32: out is FP32 (else the value type)
 int launch_band_attn_long(const void* q, const void* k, const void* v, void* out, int B, int T, int window,
-                          float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent = 0);
+                          float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent = 0, int out_fp32 = 0);
+bool band_attn_long_takes(int T, int window);
+// Banded attention on [B, 8, T, 64] tensors of any float type and strides (fm_window.cu).
+int launch_window_attention(const void* const* qkv, int in_type, const long long* strides, void* const* ws, void* out16, float* out32,
+                            int B, int T, int window, float scale, int value_is_fp16, int* status, cudaStream_t st);
 int launch_ring_decode_attn(const void* q, const void* ring_k, const void* ring_v, float* out,
                             const int* stream_pos, int pos_base, int S, int ring_slots, float scale,
                             int value_is_fp16, int* status, cudaStream_t st);

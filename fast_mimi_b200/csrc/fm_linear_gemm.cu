@@ -301,7 +301,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             float4 o = *reinterpret_cast<const float4*>(slab + sw128_offset(4 * k + (lane >> 3), lane & 7));
             if constexpr (kSplit) {
               const int at = args.rows.out_row(row + 4 * k, args.M);
-              if (at >= 0) *reinterpret_cast<float4*>(static_cast<float*>(args.y) + static_cast<long long>(at) * args.N + col) = o;
+              if (at >= 0) *reinterpret_cast<float4*>(static_cast<float*>(args.y) + args.rows.at(at, col)) = o;
               continue;
             }
             o.x *= sc.x; o.y *= sc.y; o.z *= sc.z; o.w *= sc.w;
@@ -514,10 +514,10 @@ int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, co
 }
 
 int launch_linear_split(const void* a_hi, const void* a_lo, long long a_rows, int a_cols, const void* w_hi, const void* w_lo, float* y,
-                        long long rows, int clip_rows, int clip_valid, int by_channel, int N, int K, int* status, cudaStream_t st) {
+                        long long rows, int clip_rows, int clip_valid, int by_channel, int n_mats, int N, int K, int* status, cudaStream_t st) {
   using namespace lin;
   if (rows < 0 || a_rows > 0x7fffffffLL || a_rows < rows || N <= 0 || K <= 0 || N % 256 != 0 || a_cols <= 0 || a_cols % kBlockK != 0 ||
-      K % a_cols != 0 || clip_rows <= 0 || clip_valid <= 0 || clip_valid > clip_rows)
+      K % a_cols != 0 || n_mats <= 0 || N % (256 * n_mats) != 0 || (by_channel && n_mats != 1) || clip_rows <= 0 || clip_valid <= 0 || clip_valid > clip_rows)
     return -1;
   if (rows == 0) return 0;
   if (a_hi == nullptr || a_lo == nullptr || w_hi == nullptr || w_lo == nullptr || y == nullptr) return -1;
@@ -526,7 +526,8 @@ int launch_linear_split(const void* a_hi, const void* a_lo, long long a_rows, in
     return -3;
   const int M = static_cast<int>(rows);
   const SplitLow low = {a_lo, w_lo, a_rows};
-  const SplitRows map = {a_cols / kBlockK, clip_rows, clip_valid, by_channel};
+  const long long results = (rows + clip_rows - 1) / clip_rows * clip_valid - (rows % clip_rows != 0 && rows % clip_rows < clip_valid ? clip_valid - rows % clip_rows : 0);
+  const SplitRows map = {a_cols / kBlockK, clip_rows, clip_valid, by_channel, N / n_mats, results * (N / n_mats)};
   if (few_row_tiles(M, N)) return launch_linear_split_small(a_hi, w_hi, low, map, y, M, N, K, status, st);
   const int pair_tiles = ((M + kBlockM - 1) / kBlockM + 1) / 2;
   const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;

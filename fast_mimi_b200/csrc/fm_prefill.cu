@@ -341,7 +341,7 @@ int launch_band_attn_prefill(const void* q, const void* k, const void* v, void* 
   if (T > kTile && T <= 2 * kTile && B <= (1 << 27))
     return launch_band_attn_clip(q, k, v, out, B, T, window, scale, value_is_fp16, status, st, dependent);
   // Longer clips whose window spans exactly three key tiles per query tile take the run-walking kernel.
-  if (T > 2 * kTile && window > kTile + 1 && window <= 2 * kTile + 1 && B <= (1 << 27))
+  if (band_attn_long_takes(T, window) && B <= (1 << 27))
     return launch_band_attn_long(q, k, v, out, B, T, window, scale, value_is_fp16, status, st, dependent);
   return launch_general(q, k, v, out, B, T, T, 0, window, scale, value_is_fp16, status, st, dependent);
 }

@@ -91,11 +91,13 @@ struct Walk {
 };
 }  // namespace longclip
 
-template <typename VT>
+// OT: type of the result.  FP32 rows (256 bytes per lane) go straight from registers to memory as whole 32-byte sectors;
+// 16-bit rows through the slabs and a tiled store.
+template <typename VT, typename OT>
 __global__ void __launch_bounds__(longclip::kThreads, 1)
 band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_out,
-                      int n_runs, int n_seg, int seg_tiles, int n_tiles, int T, int window, float scale_log2e,
+                      float* __restrict__ out32, int n_runs, int n_seg, int seg_tiles, int n_tiles, int T, int window, float scale_log2e,
                       int* status) {
   using namespace longclip;
   using namespace attn_tile;
@@ -305,6 +307,24 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       tc_fence_after_sync();
       mbar_wait(&sh->xl_full[x], xph, ctl, status, kErrWaitConsumer);
       l_row += sh->xl[x][r][0] + sh->xl[x][r][1];
+      if constexpr (std::is_same<OT, float>::value) {
+        uint32_t o[64];
+        tmem_ld32(slot + kOCol, *reinterpret_cast<uint32_t(*)[32]>(&o[0]));
+        tmem_ld32(slot + kOCol + 32, *reinterpret_cast<uint32_t(*)[32]>(&o[32]));
+        tmem_ld_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh->slot_free[team]);
+        if (i < T) {
+          const float inv = 1.f / l_row;
+          float* dst = out32 + (static_cast<long long>(w.clip()) * T + i) * 512 + w.head() * kD;
+#pragma unroll
+          for (int d = 0; d < kD; ++d) o[d] = __float_as_uint(__uint_as_float(o[d]) * inv);
+#pragma unroll
+          for (int d = 0; d < kD; d += 8) st_global_v8(dst + d, o + d);
+        }
+        continue;
+      }
       // The previous step's stores out of the slabs must have read them.
       uint8_t* slab = smem_stage + lg * kSlabBytes;
       if (n >= 1) mbar_wait(&sh->out_done, static_cast<uint32_t>(n - 1) & 1u, ctl, status, kErrWaitConsumer);
@@ -344,18 +364,24 @@ static int encode_long_map(CUtensorMap* map, const void* base, int B, int T, uin
                       CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
+// three key tiles per query tile: the window must reach into tile t-2 and not beyond it
+bool band_attn_long_takes(int T, int window) {
+  return T > 2 * longclip::kTile && window > longclip::kTile + 1 && window <= 2 * longclip::kTile + 1;
+}
+
 int launch_band_attn_long(const void* q, const void* k, const void* v, void* out, int B, int T, int window, float scale,
-                          int value_is_fp16, int* status, cudaStream_t st, int dependent) {
+                          int value_is_fp16, int* status, cudaStream_t st, int dependent, int out_fp32) {
   using namespace longclip;
-  // three key tiles per query tile: the window must reach into tile t-2 and not beyond it
-  if (T <= 2 * kTile || B <= 0 || window <= kTile + 1 || window > 2 * kTile + 1) return -1;
+  if (B <= 0 || !band_attn_long_takes(T, window)) return -1;
+  if (out_fp32 && (reinterpret_cast<uintptr_t>(out) & 31u) != 0) return -3;
   CUtensorMap tq, tk, tv, tout;
   int rc = encode_long_map(&tq, q, B, T, kTile);
   if (rc == 0) rc = encode_long_map(&tk, k, B, T, kTile);
   if (rc == 0) rc = encode_long_map(&tv, v, B, T, kTile);     // element size is what matters: 16 bit
-  if (rc == 0) rc = encode_long_map(&tout, out, B, T, 32);
+  if (rc == 0) rc = out_fp32 ? encode_long_map(&tout, q, B, T, 32) : encode_long_map(&tout, out, B, T, 32);   // FP32: a placeholder
   if (rc != 0) return rc;
-  auto kern = value_is_fp16 ? band_attn_long_kernel<__half> : band_attn_long_kernel<__nv_bfloat16>;
+  auto kern = out_fp32 ? (value_is_fp16 ? band_attn_long_kernel<__half, float> : band_attn_long_kernel<__nv_bfloat16, float>)
+                       : (value_is_fp16 ? band_attn_long_kernel<__half, __half> : band_attn_long_kernel<__nv_bfloat16, __nv_bfloat16>);
   rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
   if (rc != 0) return rc;
   const int sms = sm_count();
@@ -372,7 +398,8 @@ int launch_band_attn_long(const void* q, const void* k, const void* v, void* out
   if (n_runs_ll > 0x7fffffffLL) return -1;
   const int n_runs = static_cast<int>(n_runs_ll);
   const int grid = n_runs < sms ? n_runs : sms;
-  return launch_kernel(kern, dim3(grid), kThreads, kSmemBytes, st, 1, dependent, tq, tk, tv, tout, n_runs, n_seg, seg_tiles,
+  return launch_kernel(kern, dim3(grid), kThreads, kSmemBytes, st, 1, dependent, tq, tk, tv, tout,
+                       out_fp32 ? static_cast<float*>(out) : nullptr, n_runs, n_seg, seg_tiles,
                        n_tiles, T, window, scale * 1.4426950408889634f, status);
 }
 

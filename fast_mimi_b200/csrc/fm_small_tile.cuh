@@ -124,7 +124,7 @@ __device__ __forceinline__ void finish_piece(const SmallArgs& args, float (&lo)[
     }
     const int out = args.rows.out_row(row, args.M);
     if (out < 0) return;
-    float* y = static_cast<float*>(args.y) + static_cast<long long>(out) * args.N + ntile * 32 * kHalves + 4 * j;
+    float* y = static_cast<float*>(args.y) + args.rows.at(out, ntile * 32 * kHalves + 4 * j);
     *reinterpret_cast<float4*>(y) = make_float4(lo[0], lo[1], lo[2], lo[3]);
     if constexpr (kHalves == 2) *reinterpret_cast<float4*>(y + 32) = make_float4(hi[0], hi[1], hi[2], hi[3]);
   } else {

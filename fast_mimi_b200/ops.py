@@ -267,6 +267,40 @@ def band_attention_prefill(q, k, v, *, window=250, scale=0.125, out=None, status
     return out
 
 
+def window_attention_takes(q, k, v, value_dtype) -> bool:
+    """Whether ``window_attention`` reads these ``[B, 8, T, 64]`` tensors as they are: one float type of at most 32 bit that is
+    FP32 or the value type (a result of another 16-bit type than the values' is a conversion more), 16-byte aligned."""
+    per = 4 if q.dtype == torch.float32 else 8
+    return (q.dtype in (torch.float32, value_dtype) and value_dtype in _VALUE_CODES and q.dtype == k.dtype == v.dtype
+            and q.shape[0] <= 65535 and q.numel() > 0
+            and all(t.is_cuda and t.device == q.device and t.stride(3) == 1 and t.data_ptr() % 16 == 0
+                    and all(s % per == 0 for s in t.stride()[:3]) for t in (q, k, v)))
+
+
+def window_attention(q, k, v, *, window=250, scale=0.125, value_dtype=torch.float16, status=None):
+    """Banded attention over rotated ``q, k`` and ``v [B, 8, T, 64]`` as a model holds them (``window_attention_takes``): one
+    launch brings what is not yet there into the kernels' layout, and an FP32 result is stored as such.  Returns
+    ``[B, 8, T, 64]`` in ``q``'s type, frame-major in memory."""
+    B, H, T, D = q.shape
+    code = _OUT_CODES[q.dtype]
+    strides, ws, keep = [], [], []
+    for t, want in ((q, torch.bfloat16), (k, torch.bfloat16), (v, value_dtype)):
+        s = list(t.stride()[:3])
+        strides += s
+        as_is = t.dtype == want and s[1] == D and s[2] == H * D and (B == 1 or s[0] == T * H * D)
+        keep.append(None if as_is else torch.empty(B, T, H * D, dtype=want, device=q.device))
+        ws.append(_ptr(keep[-1]))
+    fp32 = q.dtype == torch.float32
+    out = torch.empty(B, T, H, D, dtype=q.dtype, device=q.device)
+    stored = T > 256 and 129 < window <= 257          # the kernel for long clips stores FP32 itself
+    out16 = None if fp32 and stored else (torch.empty(B, T, H * D, dtype=value_dtype, device=q.device) if fp32 else out)
+    rc = _native.load().fm_window_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), code, (ctypes.c_longlong * 9)(*strides), *ws,
+                                            _ptr(out16), out.data_ptr() if fp32 else None, B, T, window, scale,
+                                            _VALUE_CODES[value_dtype], _status_ptr(status, q), _stream())
+    _native.check(rc, "fm_window_attention")
+    return out.transpose(1, 2)
+
+
 def attention_prefill(x, w_qkv, cos, sin, *, window=250, scale=0.125, value_dtype=torch.float16,
                       workspace=None, out=None, status=None):
     """Projection + RoPE + banded attention for a call without cache; returns ``[B,T,512]`` value_dtype.  Whole clips
@@ -648,16 +682,17 @@ def _check_weight_parts(w_parts, k):
     return w_hi, w_lo
 
 
-def _linear_parts(x_parts, w_parts, shape, status):
-    """``linear_split`` of an already split ``x`` (``[.., K]`` each part): float32 ``[*shape, N]``."""
+def _linear_parts(x_parts, w_parts, shape, status, mats=None):
+    """``linear_split`` of an already split ``x`` (``[.., K]`` each part): float32 ``[*shape, N]``, or with ``mats`` the products
+    of that many weights side by side in ``w_parts``, ``[mats, *shape, N / mats]``."""
     x_hi, x_lo = x_parts
     k = x_hi.shape[-1]
     w_hi, w_lo = _check_weight_parts(w_parts, k)
     rows, n = x_hi.numel() // k, w_hi.shape[0]
-    y = torch.empty((*shape, n), dtype=torch.float32, device=x_hi.device)
+    y = torch.empty((*shape, n) if mats is None else (mats, *shape, n // mats), dtype=torch.float32, device=x_hi.device)
     if rows:
         rc = _native.load().fm_linear_split_f32(x_hi.data_ptr(), x_lo.data_ptr(), rows, k, w_hi.data_ptr(), w_lo.data_ptr(),
-                                                y.data_ptr(), rows, 1, 1, 0, n, k, _status_ptr(status, x_hi), _stream())
+                                                y.data_ptr(), rows, 1, 1, 0, mats or 1, n, k, _status_ptr(status, x_hi), _stream())
         _native.check(rc, "fm_linear_split_f32")
     return y
 
@@ -683,7 +718,7 @@ def downsample_conv(x, w_parts, *, kernel=4, stride=2, status=None):
                       "fm_conv_frames_split")
         y = torch.empty(B, t_out, w_hi.shape[0], dtype=torch.float32, device=x.device)
         rc = lib.fm_linear_split_f32(hi.data_ptr(), lo.data_ptr(), hi.shape[0], stride * C, w_hi.data_ptr(), w_lo.data_ptr(),
-                                     y.data_ptr(), hi.shape[0] - extra, t_out + extra, t_out, 0, w_hi.shape[0], kernel * C,
+                                     y.data_ptr(), hi.shape[0] - extra, t_out + extra, t_out, 0, 1, w_hi.shape[0], kernel * C,
                                      _status_ptr(status, x), _stream())
         _native.check(rc, "fm_linear_split_f32")
         return y
@@ -741,7 +776,7 @@ def rvq_decode_project(codes, first: RVQCodebooks, second: RVQCodebooks | None, 
                                      0 if second is None else second.entries, bad.data_ptr(), _stream())
         _native.check(rc, "fm_rvq_decode_split")
         rc = lib.fm_linear_split_f32(hi.data_ptr(), lo.data_ptr(), B * T, width, w_hi.data_ptr(), w_lo.data_ptr(), y.data_ptr(), B * T,
-                                     T, T, 1, w_hi.shape[0], width, _status_ptr(status, codes), _stream())
+                                     T, T, 1, 1, w_hi.shape[0], width, _status_ptr(status, codes), _stream())
         _native.check(rc, "fm_linear_split_f32")
     if int(bad.item()) != 0:
         raise RuntimeError("rvq_decode: a code index is outside the codebook")

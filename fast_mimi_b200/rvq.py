@@ -70,9 +70,12 @@ class MimiRVQB200:
         ops._need(0 < layers <= self.books.layers, "num_quantizers out of range")
         return layers
 
-    def _encode_frames(self, frames: "_Frames", codes: torch.Tensor) -> None:
-        """Codes of the first ``len(codes)`` layers into ``codes [layers, frames]``; nothing is read back."""
-        if self.input_proj is None:
+    def _encode_frames(self, frames: "_Frames", codes: torch.Tensor, x: torch.Tensor | None = None) -> None:
+        """Codes of the first ``len(codes)`` layers into ``codes [layers, frames]``; nothing is read back.  ``x``: the frames
+        after the projection, if they are at hand (overwritten)."""
+        if x is not None:
+            pass
+        elif self.input_proj is None:
             x = frames.rows.clone()
         elif self._on_tensor_core(self.input_proj):
             x = ops._linear_parts(frames.parts(), self._in_parts, (len(frames.rows),), None)
@@ -97,8 +100,20 @@ class MimiSplitRVQB200:
         self.semantic, self.acoustic = semantic, acoustic
         self.num_semantic_quantizers = semantic.books.layers
         self.max_num_quantizers = semantic.books.layers + acoustic.books.layers
+        self._joint_in: tuple | None = None
         self._joint: tuple | None = None
+        self._joint_in_parts()
         self._joint_out_parts()
+
+    def _joint_in_parts(self):
+        """Both input projections as one weight ``[2 * 256, hidden]``, so that the embeddings are read once."""
+        sem, aco = self.semantic, self.acoustic
+        w0, w1 = sem.input_proj, aco.input_proj
+        if self._joint_in is None or self._joint_in[0] is not w0 or self._joint_in[1] is not w1:
+            fits = (w0 is not None and w1 is not None and w0.shape == w1.shape and w0.shape[0] == ops.RVQ_DIM
+                    and sem._on_tensor_core(w0) and w0.device == w1.device)
+            self._joint_in = (w0, w1, ops.split_half(torch.cat((w0, w1), dim=0)) if fits else None)
+        return self._joint_in[2]
 
     def _joint_out_parts(self):
         """Both output projections as one weight over [semantic | acoustic], whose accumulator then adds the branches; made
@@ -125,10 +140,15 @@ class MimiSplitRVQB200:
         acoustic = count - self.num_semantic_quantizers
         codes = torch.empty(n_sem + acoustic, B * T, dtype=torch.int64, device=embeddings.device)
         frames = _Frames(embeddings)
-        self.semantic._encode_frames(frames, codes[:n_sem])
+        x = [None, None]
         if acoustic > 0:
             self.acoustic._layers(acoustic)
-            self.acoustic._encode_frames(frames, codes[n_sem:])
+            parts = self._joint_in_parts()
+            if parts is not None:
+                x = ops._linear_parts(frames.parts(), parts, (B * T,), None, mats=2)
+        self.semantic._encode_frames(frames, codes[:n_sem], x[0])
+        if acoustic > 0:
+            self.acoustic._encode_frames(frames, codes[n_sem:], x[1])
         ops.check_status(embeddings.device)
         return codes.view(len(codes), B, T)
 

@@ -96,6 +96,17 @@ int fm_qkv_rope_bf16(const void* x, const void* w_qkv, const float* cos, const f
 int fm_band_attn_prefill_bf16(const void* q, const void* k, const void* v, void* out, int B, int T,
                               int window, float scale, int value_dtype, int* status, void* stream);
 
+/* The same on rotated q, k, v as a model holds them (_native_window_attention, src/fast_mimi/model.py:1589-1624): tensors
+ * [B, 8, T, 64] of in_dtype (0 BF16, 1 FP16, 2 FP32), last dimension contiguous, 16-byte aligned.
+ *   strides   HOST array of nine: batch, head, frame strides of q, k, v in values (multiples of 16 bytes)
+ *   q/k/v_ws  [B, T, 512] 16 bit: the converted tensors; NULL for one that already is frame-major and of the right type
+ *             (BF16 for q and k, value_dtype for v)
+ *   out16     [B, T, 512] value_dtype; out32 [B, T, 512] FP32 or NULL.  With out32 the result goes there, and out16 is a
+ *             workspace that may be NULL where T > 256 and 129 < window <= 257 */
+int fm_window_attention(const void* q, const void* k, const void* v, int in_dtype, const long long* strides, void* q_ws, void* k_ws,
+                        void* v_ws, void* out16, float* out32, int B, int T, int window, float scale, int value_dtype, int* status,
+                        void* stream);
+
 /* Banded attention of Tq query frames against Tk >= Tq key / value frames whose last Tq rows are the queries' own
  * frames and whose first Tk - Tq rows are older (cached) frames: the masked SDPA of a cached call with
  * query_offset - key_offset = Tk - Tq (src/fast_mimi/model.py:1672-1677, :2194-2205) on rotated q [B,Tq,512] BF16,
@@ -194,9 +205,10 @@ int fm_conv_frames_split(const float* x, void* hi, void* lo, int B, int T, int C
  *   rows     row r of the product lies in rows r .. r + k_in / a_cols - 1 of a (k_in = a_cols: a plain matrix; over
  *            padded frames seen as rows of `stride` frames: the convolution); rows <= a_rows
  *   y        FP32 [.., n_out]: of every clip_rows rows the first clip_valid, back to back (equal: all rows); with
- *            by_channel [rows / clip_rows, n_out, clip_valid] */
+ *            by_channel [rows / clip_rows, n_out, clip_valid]; with n_mats > 1 that many matrices of n_out / n_mats
+ *            (a multiple of 256) columns, one behind the other */
 int fm_linear_split_f32(const void* a_hi, const void* a_lo, long long a_rows, int a_cols, const void* w_hi, const void* w_lo,
-                        float* y, long long rows, int clip_rows, int clip_valid, int by_channel, int n_out, int k_in, int* status,
+                        float* y, long long rows, int clip_rows, int clip_valid, int by_channel, int n_mats, int n_out, int k_in, int* status,
                         void* stream);
 
 /* The stride-2 upsampling that precedes the decoder transformer (MimiModel.upsample: MimiConvTranspose1d(512, 512,

@@ -112,3 +112,37 @@ def test_prefill_and_decode_replay_inside_a_cuda_graph():
         # the order of the FP32 sums
         assert O.rel_l2(o.cpu(), eager.cpu()) < 1e-5, t
     assert ops.read_status(st) == 0
+
+
+@pytest.mark.parametrize("dtype,value_dtype", [(torch.float32, torch.float16), (torch.float32, torch.bfloat16),
+                                               (torch.float16, torch.float16), (torch.bfloat16, torch.bfloat16),
+                                               (torch.bfloat16, torch.float16)])
+@pytest.mark.parametrize("B,T,window", [(1, 1, 250), (2, 33, 250), (3, 200, 250), (2, 257, 250), (2, 600, 250), (1, 300, 64)])
+def test_window_attention_reads_every_layout(dtype, value_dtype, B, T, window):
+    """The one-launch conversion against tensors converted one by one: layouts ([B, T, 8, 64], [B, 8, T, 64], slices of a packed
+    projection, a batch expanded from one clip, one that is not 16-byte aligned), types, every attention kernel behind it."""
+    import fast_mimi_b200 as fm
+    from fast_mimi_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(T)
+    make = lambda *s: (torch.randn(*s, device="cuda", generator=g) * 0.5).to(dtype)
+    packed = make(B, T, 3, 8, 64)
+    layouts = {
+        "frame-major": [make(B, T, 8, 64).transpose(1, 2) for _ in range(3)],
+        "head-major": [make(B, 8, T, 64) for _ in range(3)],
+        "packed": [packed[:, :, i].transpose(1, 2) for i in range(3)],
+        "expanded": [make(1, T, 8, 64).transpose(1, 2).expand(B, -1, -1, -1) for _ in range(3)],
+    }
+    if dtype == torch.float32:          # (16-bit tensors that need no conversion have to be aligned)
+        layouts["odd"] = [make(B * T * 512 + 1)[1:].view(B, T, 8, 64).transpose(1, 2) for _ in range(3)]
+    for name, (q, k, v) in layouts.items():
+        got = fm.native_window_attention(q, k, v, scale=0.125, window=window, value_dtype=value_dtype)
+        frames = lambda t, d: t.transpose(1, 2).to(d).contiguous().view(B, T, 512)
+        want = ops.band_attention_prefill(frames(q, torch.bfloat16), frames(k, torch.bfloat16), frames(v, value_dtype),
+                                          window=window, scale=0.125).view(B, T, 8, 64).transpose(1, 2)
+        assert got.dtype == dtype and got.shape == q.shape and got.transpose(1, 2).is_contiguous(), name
+        if dtype == torch.float32 and T > 256 and window > 129:          # not rounded on the way: half a unit of 16 bits
+            unit = 2.0 ** (-11 if value_dtype == torch.float16 else -8)
+            assert bool(((got - want.float()).abs() <= unit * got.abs() + 2.0 ** -25).all()), name
+        else:
+            assert torch.equal(got, want.to(dtype)), name
+    fm.check_status()

@@ -176,3 +176,16 @@ def test_decode_with_projection_matches_fp64(B, T, stacks):
     codes[B - 1, 0, T - 1] = 512
     with pytest.raises(RuntimeError, match="outside the codebook"):
         q.decode(codes.cuda())
+
+
+@pytest.mark.parametrize("rows", [1, 63, 5000, 20001])
+def test_split_precision_products_of_two_weights(rows):
+    """Two weights behind one another give two matrices, with few rows and many, equal to the products one by one up to the
+    order of FP32 sums."""
+    import fast_mimi_b200 as fm
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, 512, device="cuda", generator=g)
+    w = torch.randn(512, 512, device="cuda", generator=g) / 512 ** 0.5
+    got = fm.ops._linear_parts(fm.ops.split_half(x), fm.ops.split_half(w), (rows,), None, mats=2)
+    want = (x.double() @ w.double().T).view(rows, 2, 256).transpose(0, 1)
+    assert got.shape == want.shape and float((got - want).abs().max() / want.abs().max()) < 2e-6
