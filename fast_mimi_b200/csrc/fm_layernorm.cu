@@ -50,17 +50,25 @@ layernorm512_kernel(const void* __restrict__ x, const ParamVec weight, const Par
   const long long stride = static_cast<long long>(gridDim.x) * kWarpsPerBlock;
   // this lane's channels: 4*lane + 128*j + (0..3); weight and bias stay in registers across frames
   float w[4][4], b[4][4];
+  uint4 w_raw[4], b_raw[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const float4 wf = weight.load4(128 * j + 4 * lane);
-    const float4 bf = bias.load4(128 * j + 4 * lane);
+    w_raw[j] = weight.raw4(128 * j + 4 * lane);
+    b_raw[j] = bias.raw4(128 * j + 4 * lane);
+  }
+  float v[4][4];
+  if (warp0 < rows) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) load4<kIn>(x, warp0 * kHidden + 128 * j + 4 * lane, v[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float4 wf = weight.value4(w_raw[j]);
+    const float4 bf = bias.value4(b_raw[j]);
     w[j][0] = wf.x; w[j][1] = wf.y; w[j][2] = wf.z; w[j][3] = wf.w;
     b[j][0] = bf.x; b[j][1] = bf.y; b[j][2] = bf.z; b[j][3] = bf.w;
   }
   for (long long row = warp0; row < rows; row += stride) {
-    float v[4][4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) load4<kIn>(x, row * kHidden + 128 * j + 4 * lane, v[j]);
     float sum = 0.f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) sum += (v[j][0] + v[j][1]) + (v[j][2] + v[j][3]);
@@ -86,6 +94,10 @@ layernorm512_kernel(const void* __restrict__ x, const ParamVec weight, const Par
       for (int e = 0; e < 4; ++e) o[e] = v[j][e] * rstd * w[j][e] + b[j][e];
       const uint2 packed = make_uint2(Pack16<TOut>::pack(o[0], o[1]), Pack16<TOut>::pack(o[2], o[3]));
       *reinterpret_cast<uint2*>(static_cast<uint16_t*>(y) + row * kHidden + 128 * j + 4 * lane) = packed;
+    }
+    if (row + stride < rows) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) load4<kIn>(x, (row + stride) * kHidden + 128 * j + 4 * lane, v[j]);
     }
   }
 }

@@ -262,7 +262,9 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           R next[8];
           if (idx + 1 < n_pieces) fetch(idx + 1, next);
           const int col = first_col(i, p);
-          const float4 sc = !kSplit && args.scale.data != nullptr ? args.scale.load4(col) : make_float4(1.f, 1.f, 1.f, 1.f);
+          const bool scaled = !kSplit && args.scale.data != nullptr;
+          uint4 sc_raw = make_uint4(0u, 0u, 0u, 0u);
+          if (scaled) sc_raw = args.scale.raw4(col);
           tmem_ld_wait();
           if (p == kPieces - 1) {
             // Last read of the accumulator by this warp: hand it back before the arithmetic and the stores.
@@ -294,6 +296,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           for (int c = 0; c < 8; ++c)
             *reinterpret_cast<float4*>(slab + sw128_offset(lane, c)) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
           __syncwarp();
+          const float4 sc = scaled ? args.scale.value4(sc_raw) : make_float4(1.f, 1.f, 1.f, 1.f);
           const int row = first_row(i);
           uint8_t* dst = static_cast<uint8_t*>(args.y) + (static_cast<long long>(row) * args.N + col) * kElem;
 #pragma unroll

@@ -108,7 +108,7 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   int item = static_cast<int>(threadIdx.x);
   if (warp < kWarps) {
     // this lane's channels: 4 * lane + 128 * j + (0..3)
-    float w[4][4], b[4][4];
+    uint4 w_raw[4], b_raw[4];
     griddep_wait();
     if (ln.opens_chain) griddep_launch();
     float v[kRows / kWarps][4][4];
@@ -125,10 +125,8 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float4 wf = ln.weight.load4(128 * j + 4 * lane);
-      const float4 bf = ln.bias.load4(128 * j + 4 * lane);
-      w[j][0] = wf.x; w[j][1] = wf.y; w[j][2] = wf.z; w[j][3] = wf.w;
-      b[j][0] = bf.x; b[j][1] = bf.y; b[j][2] = bf.z; b[j][3] = bf.w;
+      w_raw[j] = ln.weight.raw4(128 * j + 4 * lane);
+      b_raw[j] = ln.bias.raw4(128 * j + 4 * lane);
     }
     if (item < n_items) load_operands<kOut>(args, m0 + (item >> 3), ntile, item & 7, ops);
     // the same sums in the same order as layernorm512_kernel
@@ -161,6 +159,14 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
       for (int i = 0; i < kRows / kWarps; ++i) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], o);
+    }
+    float w[4][4], b[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 wf = ln.weight.value4(w_raw[j]);
+      const float4 bf = ln.bias.value4(b_raw[j]);
+      w[j][0] = wf.x; w[j][1] = wf.y; w[j][2] = wf.z; w[j][3] = wf.w;
+      b[j][0] = bf.x; b[j][1] = bf.y; b[j][2] = bf.z; b[j][3] = bf.w;
     }
 #pragma unroll
     for (int i = 0; i < kRows / kWarps; ++i) {

@@ -36,7 +36,7 @@ struct SmallArgs {
 // kOut: 0 = BF16, 1 = FP16, 2 = FP32 output and residual; 3 = q | k | v with RoPE; 4 = FP32 output of a split-precision product.
 struct PieceOperands {
   float4 a[2];            // residual, or cos and sin
-  float4 s[2];            // per-channel scale
+  uint4 s[2];             // per-channel scale, as it lies
 };
 
 template <int kOut, int kHalves = 2>
@@ -54,7 +54,7 @@ __device__ __forceinline__ void load_operands(const SmallArgs& args, int row, in
     const long long at = static_cast<long long>(row) * args.N + col;
 #pragma unroll
     for (int h = 0; h < kHalves; ++h) {
-      p.s[h] = args.scale.data != nullptr ? args.scale.load4(col + 32 * h) : make_float4(1.f, 1.f, 1.f, 1.f);
+      if (args.scale.data != nullptr) p.s[h] = args.scale.raw4(col + 32 * h);
       p.a[h] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (args.resid != nullptr) {
         if constexpr (kOut == 2) {
@@ -138,7 +138,8 @@ __device__ __forceinline__ void finish_piece(const SmallArgs& args, float (&lo)[
         gelu_erf2(v[2], v[3]);
       }
       if (args.scale.data != nullptr) {
-        v[0] *= p.s[h].x; v[1] *= p.s[h].y; v[2] *= p.s[h].z; v[3] *= p.s[h].w;
+        const float4 s = args.scale.value4(p.s[h]);
+        v[0] *= s.x; v[1] *= s.y; v[2] *= s.z; v[3] *= s.w;
       }
       if (args.resid != nullptr) {
         v[0] += p.a[h].x; v[1] += p.a[h].y; v[2] += p.a[h].z; v[3] += p.a[h].w;
