@@ -136,7 +136,8 @@ extern "C" int fm_layer_forward(const fm_layer_params* params, const void* x, vo
                                 long long workspace_bytes, const float* cos, const float* sin, long long cos_bstride, int B,
                                 int T, void* ring_k, void* ring_v, int past, int ring_slots, int* status, void* stream) {
   if (params == nullptr || params->stream_dtype < 0 || params->stream_dtype > 2 || params->value_dtype < 0 ||
-      params->value_dtype > 3 || params->vec_dtype < 0 || params->vec_dtype > 2)
+      params->value_dtype > 3 || params->vec_dtype < 0 || params->vec_dtype > 2 ||
+      (params->stream_dtype == 2 && params->vec_dtype != 2))
     return -1;
   return fm::layer_forward(*params, x, y, workspace, workspace_bytes, cos, sin, cos_bstride, B, T, ring_k, ring_v, past,
                            ring_slots, status, static_cast<cudaStream_t>(stream));

@@ -53,8 +53,8 @@ layernorm512_kernel(const void* __restrict__ x, const ParamVec weight, const Par
   uint4 w_raw[4], b_raw[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    w_raw[j] = weight.raw4(128 * j + 4 * lane);
-    b_raw[j] = bias.raw4(128 * j + 4 * lane);
+    w_raw[j] = weight.raw4<kIn == 2>(128 * j + 4 * lane);
+    b_raw[j] = bias.raw4<kIn == 2>(128 * j + 4 * lane);
   }
   float v[4][4];
   if (warp0 < rows) {
@@ -63,8 +63,8 @@ layernorm512_kernel(const void* __restrict__ x, const ParamVec weight, const Par
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const float4 wf = weight.value4(w_raw[j]);
-    const float4 bf = bias.value4(b_raw[j]);
+    const float4 wf = weight.value4<kIn == 2>(w_raw[j]);
+    const float4 bf = bias.value4<kIn == 2>(b_raw[j]);
     w[j][0] = wf.x; w[j][1] = wf.y; w[j][2] = wf.z; w[j][3] = wf.w;
     b[j][0] = bf.x; b[j][1] = bf.y; b[j][2] = bf.z; b[j][3] = bf.w;
   }
@@ -106,6 +106,7 @@ int launch_layernorm512(const void* x, int x_dtype, ParamVec weight, ParamVec bi
                         int y_dtype, long long rows, cudaStream_t st, int dependent) {
   using namespace ln;
   if (rows < 0 || x_dtype < 0 || x_dtype > 2 || y_dtype < 0 || y_dtype > 1) return -1;
+  if (x_dtype == 2 && (weight.type != 2 || bias.type != 2)) return -1;
   if (rows == 0) return 0;
   if (x == nullptr || y == nullptr || weight.data == nullptr || bias.data == nullptr) return -1;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(weight.data) |

@@ -84,8 +84,8 @@ struct LinearArgs {
 template <int kOut, bool kWide, int kBlockN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(lin::Shape<kWide, kBlockN>::kThreads, 1)
 linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
-                   const __grid_constant__ CUtensorMap tmap_y, const __grid_constant__ CUtensorMap tmap_a_lo,
-                   const __grid_constant__ CUtensorMap tmap_w_lo, const __grid_constant__ LinearArgs args, int total_units,
+                   const __grid_constant__ CUtensorMap tmap_y, const __grid_constant__ SplitMaps<kOut == 4> low,
+                   const __grid_constant__ LinearArgs args, int total_units,
                    uint32_t idesc, int* status) {
   using namespace lin;
   constexpr bool kSplit = kOut == 4, kF32 = kOut == 2 || kOut == 4;
@@ -148,11 +148,11 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
       tma_prefetch_desc(&tmap_a);
       tma_prefetch_desc(&tmap_w);
       if constexpr (kSplit) {
-        tma_prefetch_desc(&tmap_a_lo);
-        tma_prefetch_desc(&tmap_w_lo);
+        tma_prefetch_desc(&low.a);
+        tma_prefetch_desc(&low.w);
       }
       auto load_w = [&](uint8_t* dst, int kc, uint64_t* bar, int n0) {
-        if constexpr (kSplit) tma_load_2d_pair(dst, kc / k_part == 1 ? &tmap_w_lo : &tmap_w, bar, kc % k_part * kBlockK, n0);
+        if constexpr (kSplit) tma_load_2d_pair(dst, kc / k_part == 1 ? &low.w : &tmap_w, bar, kc % k_part * kBlockK, n0);
         else tma_load_2d_pair(dst, &tmap_w, bar, kc * kBlockK, n0);
       };
       int stage = 0;
@@ -177,7 +177,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           uint8_t* dst = smem_stage + stage * kStageBytes;
           if constexpr (kSplit) {
             const int k = kc % k_part;            // a row of the product continues in the matrix's next row
-            tma_load_2d_pair(dst, kc < k_part ? &tmap_a_lo : &tmap_a, &bars->full[stage], k % args.rows.a_chunks * kBlockK, m0 + k / args.rows.a_chunks);
+            tma_load_2d_pair(dst, kc < k_part ? &low.a : &tmap_a, &bars->full[stage], k % args.rows.a_chunks * kBlockK, m0 + k / args.rows.a_chunks);
           } else {
             tma_load_2d_pair(dst, &tmap_a, &bars->full[stage], kc * kBlockK, m0);
           }
@@ -264,7 +264,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           const int col = first_col(i, p);
           const bool scaled = !kSplit && args.scale.data != nullptr;
           uint4 sc_raw = make_uint4(0u, 0u, 0u, 0u);
-          if (scaled) sc_raw = args.scale.raw4(col);
+          if (scaled) sc_raw = args.scale.raw4<kF32>(col);
           tmem_ld_wait();
           if (p == kPieces - 1) {
             // Last read of the accumulator by this warp: hand it back before the arithmetic and the stores.
@@ -296,7 +296,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           for (int c = 0; c < 8; ++c)
             *reinterpret_cast<float4*>(slab + sw128_offset(lane, c)) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
           __syncwarp();
-          const float4 sc = scaled ? args.scale.value4(sc_raw) : make_float4(1.f, 1.f, 1.f, 1.f);
+          const float4 sc = scaled ? args.scale.value4<kF32>(sc_raw) : make_float4(1.f, 1.f, 1.f, 1.f);
           const int row = first_row(i);
           uint8_t* dst = static_cast<uint8_t*>(args.y) + (static_cast<long long>(row) * args.N + col) * kElem;
 #pragma unroll
@@ -450,7 +450,8 @@ static int launch_pairs(const void* a, const void* w, const SplitLow* low, void*
                         int out_dtype, int* status, cudaStream_t st, int dependent) {
   using namespace lin;
   using S = Shape<kWide, kBlockN>;
-  CUtensorMap tmap_a, tmap_w, tmap_y, tmap_a_lo = {}, tmap_w_lo = {};
+  CUtensorMap tmap_a, tmap_w, tmap_y;
+  SplitMaps<kOut == 4> low_maps = {};
   const CUtensorMapDataType t16 = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;   // any 16-bit element type moves alike
   const uint64_t M = static_cast<uint64_t>(args.M), N = static_cast<uint64_t>(args.N), K = static_cast<uint64_t>(args.K);
   const uint64_t a_rows = kOut == 4 ? static_cast<uint64_t>(low->a_rows) : M;
@@ -460,8 +461,8 @@ static int launch_pairs(const void* a, const void* w, const SplitLow* low, void*
   rc = encode_2d(&tmap_w, t16, 2, w, N, K, S::kHalfN, kBlockK);
   if (rc != 0) return rc;
   if constexpr (kOut == 4) {
-    rc = encode_2d(&tmap_a_lo, t16, 2, low->a, a_rows, a_cols, kBlockM, kBlockK);
-    if (rc == 0) rc = encode_2d(&tmap_w_lo, t16, 2, low->w, N, K, S::kHalfN, kBlockK);
+    rc = encode_2d(&low_maps.a, t16, 2, low->a, a_rows, a_cols, kBlockM, kBlockK);
+    if (rc == 0) rc = encode_2d(&low_maps.w, t16, 2, low->w, N, K, S::kHalfN, kBlockK);
     if (rc != 0) return rc;
   }
   if (out_dtype >= 3)      // no tiled store in these modes: a placeholder map over a
@@ -478,8 +479,8 @@ static int launch_pairs(const void* a, const void* w, const SplitLow* low, void*
   auto kern = linear_gemm_kernel<kOut, kWide, kBlockN>;
   rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), S::kSmemBytes);
   if (rc != 0) return rc;
-  return launch_kernel(kern, dim3(2 * n_pairs), S::kThreads, S::kSmemBytes, st, 1, dependent, tmap_a, tmap_w, tmap_y, tmap_a_lo,
-                       tmap_w_lo, args, total_units, idesc, status);
+  return launch_kernel(kern, dim3(2 * n_pairs), S::kThreads, S::kSmemBytes, st, 1, dependent, tmap_a, tmap_w, tmap_y, low_maps,
+                       args, total_units, idesc, status);
 }
 
 int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N,

@@ -59,7 +59,7 @@ __device__ __forceinline__ void bulk_copy_to_cta(uint32_t dst, const void* src, 
 template <int kOut, typename VT, int kBlockN>
 __global__ void __launch_bounds__(small::kThreads)
 linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
-                    const __grid_constant__ CUtensorMap tmap_a_lo, const __grid_constant__ CUtensorMap tmap_w_lo,
+                    const __grid_constant__ SplitMaps<kOut == 4> low,
                     const __grid_constant__ SmallArgs args, uint32_t idesc, int* status) {
   using namespace small;
   constexpr int kStageBytes = Tile<kBlockN>::kStageBytes, kRedBytes = Tile<kBlockN>::kRedBytes, kTmemCols = kBlockN;
@@ -112,7 +112,7 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       auto load_a = [&](int st, int kc) {
         if constexpr (kOut == 4) {
           const int k = kc % args.k_part;         // a row of the product continues in the matrix's next row
-          tma_load_2d(smem + st * kStageBytes, kc < args.k_part ? &tmap_a_lo : &tmap_a, &bars->full[st],
+          tma_load_2d(smem + st * kStageBytes, kc < args.k_part ? &low.a : &tmap_a, &bars->full[st],
                       k % args.rows.a_chunks * kBlockK, m0 + k / args.rows.a_chunks);
         } else {
           tma_load_2d(smem + st * kStageBytes, &tmap_a, &bars->full[st], kc * kBlockK, m0);
@@ -120,7 +120,7 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       };
       auto load_w = [&](int st, int kc) {
         if constexpr (kOut == 4)
-          tma_load_2d(smem + st * kStageBytes + kABytes, kc / args.k_part == 1 ? &tmap_w_lo : &tmap_w, &bars->full[st],
+          tma_load_2d(smem + st * kStageBytes + kABytes, kc / args.k_part == 1 ? &low.w : &tmap_w, &bars->full[st],
                       kc % args.k_part * kBlockK, n0);
         else
           tma_load_2d(smem + st * kStageBytes + kABytes, &tmap_w, &bars->full[st], kc * kBlockK, n0);
@@ -257,7 +257,8 @@ template <int kOut, typename VT, int kBlockN>
 static int launch_tiles(const void* a, const void* w, SmallArgs& args, int K, int in_dtype, int* status,
                         cudaStream_t st, int dependent, const SplitLow* low) {
   using namespace small;
-  CUtensorMap tmap_a, tmap_w, tmap_a_lo = {}, tmap_w_lo = {};
+  CUtensorMap tmap_a, tmap_w;
+  SplitMaps<kOut == 4> low_maps = {};
   const uint64_t a_rows = kOut == 4 ? static_cast<uint64_t>(low->a_rows) : static_cast<uint64_t>(args.M);
   const uint64_t a_cols = kOut == 4 ? static_cast<uint64_t>(args.rows.a_chunks) * kBlockK : static_cast<uint64_t>(K);
   int rc = encode_rows_16bit(&tmap_a, a, a_rows, a_cols, kBlockM, kBlockK);
@@ -266,8 +267,8 @@ static int launch_tiles(const void* a, const void* w, SmallArgs& args, int K, in
   if (rc != 0) return rc;
   const int m_tiles = (args.M + kBlockM - 1) / kBlockM, n_tiles = args.N / kBlockN;
   if constexpr (kOut == 4) {
-    rc = encode_rows_16bit(&tmap_a_lo, low->a, a_rows, a_cols, kBlockM, kBlockK);
-    if (rc == 0) rc = encode_rows_16bit(&tmap_w_lo, low->w, static_cast<uint64_t>(args.N), static_cast<uint64_t>(K), kBlockN, kBlockK);
+    rc = encode_rows_16bit(&low_maps.a, low->a, a_rows, a_cols, kBlockM, kBlockK);
+    if (rc == 0) rc = encode_rows_16bit(&low_maps.w, low->w, static_cast<uint64_t>(args.N), static_cast<uint64_t>(K), kBlockN, kBlockK);
     if (rc != 0) return rc;
   }
   args.k_part = K / kBlockK;
@@ -280,7 +281,7 @@ static int launch_tiles(const void* a, const void* w, SmallArgs& args, int K, in
   rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), Tile<kBlockN>::kSmemBytes);
   if (rc != 0) return rc;
   return launch_kernel(kern, dim3(n_tiles * args.split, m_tiles), kThreads, Tile<kBlockN>::kSmemBytes, st, args.split, dependent, tmap_a,
-                       tmap_w, tmap_a_lo, tmap_w_lo, args, idesc, status);
+                       tmap_w, low_maps, args, idesc, status);
 }
 
 // 64-column tiles, or 32 where 64 would leave the K split at its limit of eight with SMs to spare: the partial sums that

@@ -125,8 +125,8 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      w_raw[j] = ln.weight.raw4(128 * j + 4 * lane);
-      b_raw[j] = ln.bias.raw4(128 * j + 4 * lane);
+      w_raw[j] = ln.weight.raw4<kIn == 2>(128 * j + 4 * lane);
+      b_raw[j] = ln.bias.raw4<kIn == 2>(128 * j + 4 * lane);
     }
     if (item < n_items) load_operands<kOut>(args, m0 + (item >> 3), ntile, item & 7, ops);
     // the same sums in the same order as layernorm512_kernel
@@ -163,8 +163,8 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     float w[4][4], b[4][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float4 wf = ln.weight.value4(w_raw[j]);
-      const float4 bf = ln.bias.value4(b_raw[j]);
+      const float4 wf = ln.weight.value4<kIn == 2>(w_raw[j]);
+      const float4 bf = ln.bias.value4<kIn == 2>(b_raw[j]);
       w[j][0] = wf.x; w[j][1] = wf.y; w[j][2] = wf.z; w[j][3] = wf.w;
       b[j][0] = bf.x; b[j][1] = bf.y; b[j][2] = bf.z; b[j][3] = bf.w;
     }

@@ -54,7 +54,7 @@ __device__ __forceinline__ void load_operands(const SmallArgs& args, int row, in
     const long long at = static_cast<long long>(row) * args.N + col;
 #pragma unroll
     for (int h = 0; h < kHalves; ++h) {
-      if (args.scale.data != nullptr) p.s[h] = args.scale.raw4(col + 32 * h);
+      if (args.scale.data != nullptr) p.s[h] = args.scale.raw4<kOut == 2>(col + 32 * h);
       p.a[h] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (args.resid != nullptr) {
         if constexpr (kOut == 2) {
@@ -138,7 +138,7 @@ __device__ __forceinline__ void finish_piece(const SmallArgs& args, float (&lo)[
         gelu_erf2(v[2], v[3]);
       }
       if (args.scale.data != nullptr) {
-        const float4 s = args.scale.value4(p.s[h]);
+        const float4 s = args.scale.value4<kOut == 2>(p.s[h]);
         v[0] *= s.x; v[1] *= s.y; v[2] *= s.z; v[3] *= s.w;
       }
       if (args.resid != nullptr) {

@@ -113,9 +113,10 @@ class MimiTransformerLayerB200(nn.Module):
                   "the MLP must be 512 -> n -> 512 with n a multiple of 256")
         tc = attn._tc_input_dtype(x)
         vectors = (ln1.weight, ln1.bias, self.self_attn_layer_scale.scale, ln2.weight, ln2.bias, self.mlp_layer_scale.scale)
-        # Read where they lie if they have one type; else as FP32 copies made for this call alone (no plan), since a write
+        # Read where they lie if they have one type (FP32 in an FP32 residual stream); else as FP32 copies made for this call alone (no plan), since a write
         # through ``.data`` would not show in a kept copy.
         in_place = (len({p.dtype for p in vectors}) == 1 and vectors[0].dtype in ops._OUT_CODES
+                    and (x.dtype != torch.float32 or vectors[0].dtype == torch.float32)
                     and all(p.is_contiguous() and p.data_ptr() % 16 == 0 for p in vectors))
         w1, b1, s1, w2, b2, s2 = (p.detach() if in_place else p.detach().float().contiguous() for p in vectors)
         keep = (w1, b1, attn.packed_qkv_weight(tc), attn.out_weight(attn.value_dtype), s1, w2, b2, self._cast.get("fc1", fc1, tc),

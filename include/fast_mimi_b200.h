@@ -33,7 +33,7 @@ int fm_abi_version(void);
  * MimiTransformerLayer.forward (src/fast_mimi/model.py:2026-2061).
  *   params      host struct of device pointers; matrices are row-major [out, in] and 16 bit: w_qkv, w_fc1, w_fc2 in
  *               BF16 / FP16 by bit 1 of value_dtype, w_o in the value type (bit 0); LayerNorm parameters and layer
- *               scales in vec_dtype (0 BF16, 1 FP16, 2 FP32), 16-byte aligned (the scales may be NULL)
+ *               scales in vec_dtype (0 BF16, 1 FP16, 2 FP32; FP32 if stream_dtype is), 16-byte aligned (the scales may be NULL)
  *               weights_settled: 0 on the first call after any of them was written on this stream (the call then starts
  *               only when everything in front of it has ended), 1 afterwards
  *   x, y        [B, T, 512] in stream_dtype (0 BF16, 1 FP16, 2 FP32), y != x

@@ -164,7 +164,7 @@ def test_layer_reads_its_vectors_where_they_lie(dtype, rows):
         want = O.transformer_layer(x.float(), p)
         got, _ = layer(x.cuda(), None, None, cs)
         # the result's own rounding, over what the layer adds
-        bar = {torch.float32: 2e-3, torch.float16: 4e-3, torch.bfloat16: 2e-2}[dtype] * float(want.norm() / (want - x.float()).norm())
+        bar = {torch.float32: 2e-3, torch.float16: 4e-3, torch.bfloat16: 2e-2}[x.dtype] * float(want.norm() / (want - x.float()).norm())
         assert O.rel_l2(got.float().cpu() - x.float(), want - x.float()) < bar
 
     with torch.no_grad():
@@ -176,6 +176,12 @@ def test_layer_reads_its_vectors_where_they_lie(dtype, rows):
         layer.mlp_layer_scale.scale.data.mul_(-2.0)
         check()
         layer.input_layernorm.float()
+        check()
+        layer.input_layernorm.weight.data.mul_(0.5)
+        check()
+        layer = layer.to(torch.bfloat16)               # a 16-bit module in an FP32 stream
+        layer.input_layernorm.weight.data.mul_(2.0)
+        x = x.float()
         check()
         layer.input_layernorm.weight.data.mul_(0.5)
         check()
