@@ -153,10 +153,18 @@ bool unchanged(const LayerPlan* plan) {
 
 PyTypeObject plan_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
-// layer_forward(plan, x, cos, sin, ring_k, ring_v, past) -> tensor, or None: not the ordinary case
+// An int argument, or -1 for what is none (a value for the Python side to look at).
+long int_of(PyObject* o) {
+  const long v = PyLong_AsLong(o);
+  if (v == -1 && PyErr_Occurred()) PyErr_Clear();
+  return v;
+}
+
+// layer_forward(plan, x, cos, sin, ring_k, ring_v, layer, past) -> tensor, or None: not the ordinary case.  The rings are those
+// of all layers, [layers, streams, 8, slots, 64]: the caller's own tensors, of which nothing is kept.
 PyObject* layer_forward_checked(PyObject* const* a, Py_ssize_t n) {
-  if (n != 7 || !PyObject_TypeCheck(a[0], &plan_type)) {
-    PyErr_SetString(PyExc_TypeError, "layer_forward(plan, x, cos, sin, ring_k, ring_v, past)");
+  if (n != 8 || !PyObject_TypeCheck(a[0], &plan_type)) {
+    PyErr_SetString(PyExc_TypeError, "layer_forward(plan, x, cos, sin, ring_k, ring_v, layer, past)");
     return nullptr;
   }
   LayerPlan* plan = reinterpret_cast<LayerPlan*>(a[0]);
@@ -177,14 +185,13 @@ PyObject* layer_forward_checked(PyObject* const* a, Py_ssize_t n) {
   if (a[4] != Py_None) {
     if (!THPVariable_Check(a[4]) || !THPVariable_Check(a[5])) Py_RETURN_NONE;
     const at::Tensor &k = THPVariable_Unpack(a[4]), &v = THPVariable_Unpack(a[5]);
-    if (!k.is_cuda() || k.scalar_type() != at::kBFloat16 || k.dim() != 4 || k.size(0) != B || k.size(1) != 8 || k.size(3) != 64 ||
-        !k.is_contiguous() || !v.is_cuda() || v.scalar_type() != plan->value || v.sizes() != k.sizes() || !v.is_contiguous())
+    const long layer = int_of(a[6]), p = int_of(a[7]);
+    if (!k.is_cuda() || k.scalar_type() != at::kBFloat16 || k.dim() != 5 || k.size(1) != B || k.size(2) != 8 || k.size(4) != 64 ||
+        layer < 0 || layer >= k.size(0) || !k.is_contiguous() || !v.is_cuda() || v.scalar_type() != plan->value || v.sizes() != k.sizes() || !v.is_contiguous())
       Py_RETURN_NONE;
-    slots = static_cast<int>(k.size(2));
-    ring_k = k.data_ptr();
-    ring_v = v.data_ptr();
-    const long p = PyLong_AsLong(a[6]);
-    if (p == -1 && PyErr_Occurred()) return nullptr;
+    slots = static_cast<int>(k.size(3));
+    ring_k = static_cast<uint16_t*>(k.data_ptr()) + layer * k.stride(0);
+    ring_v = static_cast<uint16_t*>(v.data_ptr()) + layer * k.stride(0);
     if (p < 0 || p > 0x7fffffffL - T) Py_RETURN_NONE;
     past = static_cast<int>(p);
   }
@@ -223,7 +230,7 @@ PyObject* layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 PyMethodDef methods[] = {
     {"layer_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(layer_forward)), METH_FASTCALL,
-     "layer_forward(plan, x, cos, sin, ring_k, ring_v, past) -> tensor, an int (native status), or None (not the ordinary case)"},
+     "layer_forward(plan, x, cos, sin, ring_k, ring_v, layer, past) -> tensor, an int (native status), or None (not the ordinary case)"},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fm_bind", "host side of the native calls", -1, methods};

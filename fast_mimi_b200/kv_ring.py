@@ -31,14 +31,11 @@ class MimiKVRing:
         self.ring_k = torch.zeros(shape, dtype=torch.bfloat16, device=device)
         self.ring_v = torch.zeros(shape, dtype=value_dtype, device=device)
         self._cumulative_lengths = [0] * num_layers
-        self._rings: tuple | None = None
 
     def layer_rings(self, layer_idx: int) -> tuple[torch.Tensor, torch.Tensor]:
-        """One layer's ``(ring_k, ring_v)``, ``[streams, 8, window, 64]`` each (the views are made once)."""
-        r = self._rings
-        if r is None or r[0] is not self.ring_k or r[1] is not self.ring_v:
-            r = self._rings = (self.ring_k, self.ring_v, list(zip(self.ring_k.unbind(0), self.ring_v.unbind(0))))
-        return r[2][layer_idx]
+        """One layer's ``(ring_k, ring_v)``, ``[streams, 8, window, 64]`` each.  Views made on every call: kept ones came apart
+        from the ring when it was pickled or its storage replaced."""
+        return self.ring_k[layer_idx], self.ring_v[layer_idx]
 
     # ---- bookkeeping with MimiKVCache's semantics -------------------------------------------
     def configure_sliding_window(self, sliding_window: int) -> None:

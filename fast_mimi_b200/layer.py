@@ -145,18 +145,23 @@ class MimiTransformerLayerB200(nn.Module):
             pass
         return params, keep
 
-    def _forward_checked(self, x, cos, sin, ring_k, ring_v, past) -> torch.Tensor:
+    def _forward_checked(self, x, cos, sin, cache, past) -> torch.Tensor:
         """The call with everything looked at: arguments of other types or layouts, changed parameters, errors."""
         attn = self.self_attn
         x = x.contiguous()
         cos, sin = cos.to(torch.float32).contiguous(), sin.to(torch.float32).contiguous()
         params, keep = self._native_plan(x)
         if self._plan is not None:
-            y = _native.bind().layer_forward(self._plan, x, cos, sin, ring_k, ring_v, past)
+            y = _native.bind().layer_forward(self._plan, x, cos, sin, *self._rings(cache), past)
             if isinstance(y, torch.Tensor):
                 return y
         return ops.layer_forward(params, x, cos, sin, value_dtype=attn.value_dtype,
-                                 ring=None if ring_k is None else (ring_k, ring_v), past=past, window=attn.sliding_window)
+                                 ring=None if cache is None else cache.layer_rings(attn.layer_idx), past=past,
+                                 window=attn.sliding_window)
+
+    def _rings(self, cache) -> tuple:
+        """What the native call takes of a cache: the rings of all layers and the layer's number in them."""
+        return (None, None, 0) if cache is None else (cache.ring_k, cache.ring_v, self.self_attn.layer_idx)
 
     def forward(self, hidden_states: torch.Tensor, attention_mask: torch.Tensor | None, past_key_values,
                 position_embeddings: tuple[torch.Tensor, torch.Tensor], output_attentions: bool = False,
@@ -169,20 +174,18 @@ class MimiTransformerLayerB200(nn.Module):
             raise RuntimeError("key-padding masks are not supported; pass None or the 4-D causal band mask")
         cache = past_key_values
         if cache is None or isinstance(cache, MimiKVRing):
-            ring_k = ring_v = None
             past = 0
             if cache is not None:
                 attn = self.self_attn
                 ops._need(cache.num_streams == hidden_states.shape[0], "cache was created for a different number of streams")
                 ops._need(cache.sliding_window == attn.sliding_window, "cache window differs from the module's")
-                ring_k, ring_v = cache.layer_rings(attn.layer_idx)
                 past = cache.get_seq_length(attn.layer_idx)
             cos, sin = position_embeddings
             out = None
             if self._plan is not None:
-                out = _native.bind().layer_forward(self._plan, hidden_states, cos, sin, ring_k, ring_v, past)
+                out = _native.bind().layer_forward(self._plan, hidden_states, cos, sin, *self._rings(cache), past)
             if out is None:
-                out = self._forward_checked(hidden_states, cos, sin, ring_k, ring_v, past)
+                out = self._forward_checked(hidden_states, cos, sin, cache, past)
             elif type(out) is int:
                 _native.check(out, "fm_layer_forward")
             if cache is not None:

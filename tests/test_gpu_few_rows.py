@@ -75,6 +75,27 @@ def test_layer_on_live_streams_matches_the_oracle(streams, window):
     fm.check_status()
 
 
+def test_layer_follows_its_ring():
+    """A session whose ring goes through pickle, then gets new storage, half way: outputs and rings are those of a session
+    left alone."""
+    import pickle
+    import fast_mimi_b200 as fm
+    layer = fm.MimiTransformerLayerB200(layer_idx=1).cuda()
+    plain, other = fm.MimiKVRing(2, 2, 250), fm.MimiKVRing(2, 2, 250)
+    x = torch.randn(4, 2, 1, 512, device="cuda")
+    for i in range(4):
+        if i == 2:
+            other = pickle.loads(pickle.dumps(other))
+        elif i == 3:
+            other.ring_k.data, other.ring_v.data = other.ring_k.clone(), other.ring_v.clone()
+        cs = fm.rope_tables(torch.tensor([[i]], device="cuda"))
+        a, b = layer(x[i], None, plain, cs)[0], layer(x[i], None, other, cs)[0]
+        assert torch.equal(a, b)
+        for s, t in zip(plain.ordered(1), other.ordered(1)):
+            assert torch.equal(s, t)
+    fm.check_status()
+
+
 def test_layer_follows_its_parameters():
     """The layer's parameter block is rebuilt when a parameter is written to, replaced, or the options change."""
     import fast_mimi_b200 as fm

@@ -82,6 +82,25 @@ def test_ring_ordered_view_wraps():
     assert k[0, 0, :, 0].tolist() == [2, 3, 4, 5]
 
 
+@pytest.mark.parametrize("change", ["pickle", "data", "copy"])
+def test_a_layer_s_rings_are_the_ring(change):
+    """What a layer reads and writes is the ring's own memory, also after the ring went through pickle or got new storage."""
+    import copy
+    import pickle
+    from fast_mimi_b200 import MimiKVRing
+    ring = MimiKVRing(2, 1, 4, device="cpu")
+    ring.layer_rings(1)
+    if change == "pickle":
+        ring = pickle.loads(pickle.dumps(ring))
+    elif change == "copy":
+        ring = copy.deepcopy(ring)
+    else:
+        ring.ring_k.data, ring.ring_v.data = ring.ring_k.clone(), ring.ring_v.clone()
+    for whole, part in zip((ring.ring_k, ring.ring_v), ring.layer_rings(1)):
+        part[0, 3, 2] = 5.0
+        assert bool((whole[1, 0, 3, 2] == 5.0).all())
+
+
 def test_shard_bounds_cover_everything_once():
     from fast_mimi_b200 import shard_bounds
     for n in (0, 1, 7, 16, 512, 4096):
