@@ -184,25 +184,29 @@ class MimiTransformerLayerB200(nn.Module):
             out = None
             if self._plan is not None:
                 out = _native.bind().layer_forward(self._plan, hidden_states, cos, sin, *self._rings(cache), past)
-            if out is None:
-                out = self._forward_checked(hidden_states, cos, sin, cache, past)
-            elif type(out) is int:
+            if type(out) is int:
                 _native.check(out, "fm_layer_forward")
-            if cache is not None:
-                cache.advance(attn.layer_idx, hidden_states.shape[1])
-            return out, None
+            if out is None and (cache is None or cache.ring_v.dtype == self.self_attn.value_dtype):
+                out = self._forward_checked(hidden_states, cos, sin, cache, past)
+            if out is not None:
+                if cache is not None:
+                    cache.advance(attn.layer_idx, hidden_states.shape[1])
+                return out, None
         if self.mlp.fc1.bias is not None or self.self_attn.o_proj.bias is not None:
             raise RuntimeError("the fused layer expects bias-free projections, as in Mimi's checkpoints")
         attn = self.self_attn
         x = hidden_states.contiguous()
-        # a cache object of another kind: the kernels one by one around its own update
+        # a cache object of another kind, or a ring whose values have not the module's type: the kernels one by one around the
+        # attention's own way with it
         stream_dtype = x.dtype
         tc = attn._tc_input_dtype(x)
         cos, sin = (t.to(torch.float32).contiguous() for t in position_embeddings)
         ln1, ln2 = self.input_layernorm, self.post_attention_layernorm
         f32 = lambda p: p.detach().float().contiguous()       # no copy for FP32 parameters
         h = ops.layer_norm(x, f32(ln1.weight), f32(ln1.bias), eps=ln1.eps, out_dtype=tc)
-        core = attn._forward_tc(h, past_key_values, cos, sin)
+        core = attn._forward_tc(h, past_key_values, cos, sin)      # FP32 from the one-frame kernel, else the ring's type
+        if core.dtype not in ops._VALUE_CODES:
+            core = core.to(attn.value_dtype)
         x1 = ops.linear(core, attn.out_weight(core.dtype), scale=f32(self.self_attn_layer_scale.scale), residual=x,
                         out_dtype=stream_dtype)
         h2 = ops.layer_norm(x1, f32(ln2.weight), f32(ln2.bias), eps=ln2.eps, out_dtype=tc)

@@ -96,6 +96,28 @@ def test_layer_follows_its_ring():
     fm.check_status()
 
 
+@pytest.mark.parametrize("module,ring", [(torch.float16, torch.bfloat16), (torch.bfloat16, torch.float16)])
+def test_layer_on_a_ring_of_the_other_value_type(module, ring):
+    """The ring decides the type its values have, whatever the module was built with.  Bar: one BF16 rounding each of values,
+    probabilities, result and W_o at most (2^-9 / sqrt 3 of their size), in quadrature 2.3e-3."""
+    import fast_mimi_b200 as fm
+    p = _layer_params(31)
+    layer = fm.MimiTransformerLayerB200(value_dtype=module).cuda()
+    layer.load_state_dict(p)
+    cache, ref = fm.MimiKVRing(1, 2, 250, value_dtype=ring), O.KVCacheOracle()
+    g = torch.Generator().manual_seed(31)
+    past = 0
+    for T in (1, 5, 240, 1, 30):
+        x = torch.randn(2, T, 512, generator=g)
+        cos, sin = fm.rope_tables(torch.arange(past, past + T)[None])
+        got, _ = layer(x.cuda(), None, cache, (cos.cuda(), sin.cuda()))
+        want = O.transformer_layer(x, p, cache=ref)
+        assert O.rel_l2(got.cpu() - x, want - x) < ROUND[torch.bfloat16], (T, past)
+        past += T
+        assert cache.get_seq_length(0) == past
+    fm.check_status()
+
+
 def test_layer_follows_its_parameters():
     """The layer's parameter block is rebuilt when a parameter is written to, replaced, or the options change."""
     import fast_mimi_b200 as fm
