@@ -486,12 +486,21 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return r;
 }
 
+// 1 for x >= 0, else 0.
+__device__ __forceinline__ float step_ge0(float x) {
+  float r;
+  asm("set.ge.f32.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // Exact-form GELU  0.5 x (1 + erf(x / sqrt 2))  of two values, with erf from the rational approximation
 //   erf(z) = 1 - (1 + a1 z + ... + a6 z^6)^-16,  z >= 0,  |error| <= 3e-7   (Abramowitz & Stegun 7.1.28)
-// which makes it  max(x, 0) - 0.5 |x| r  with r = (...)^-16 and the powers of 1 / sqrt 2 folded into the coefficients:
-// nine issue slots per value in packed arithmetic (17 before with scalar FMAs, about 40 with erff()), one of them the
-// reciprocal.  The epilogue of fc1 is bound by these slots, not by the tensor core; the approximation error is far below
-// the rounding of the result to 16 bit.  Large |x| overflows the power to +inf, whose reciprocal is 0, i.e. erf = 1.
+// which makes it  x g  with  g = 1 - r / 2 for x >= 0 and r / 2 below, r = (...)^-16 and the powers of 1 / sqrt 2 folded into
+// the coefficients: ten issue slots per value in packed arithmetic (17 with scalar FMAs, about 40 with erff()), one of them
+// the reciprocal.  The epilogue of fc1 is bound by these slots, not by the tensor core; the approximation error is far below
+// the rounding of the result to 16 bit.  Large |x| overflows the power to +inf, whose reciprocal is 0, i.e. erf = 1; as a
+// product the result is then x for +inf and NaN (0 times infinity, as in torch) for -inf, where max(x, 0) - |x| r / 2, one slot
+// less, was NaN for both.
 __device__ __forceinline__ void gelu_erf2(float& x0, float& x1) {
   constexpr float kS = 0.70710678118654752f;
   constexpr float a1 = 0.0705230784f * kS, a2 = 0.0422820123f * kS * kS, a3 = 0.0092705272f * kS * kS * kS;
@@ -506,8 +515,9 @@ __device__ __forceinline__ void gelu_erf2(float& x0, float& x1) {
   t = f2_fma(z, t, f2_pack(1.f, 1.f));
   t = f2_mul(t, t); t = f2_mul(t, t); t = f2_mul(t, t); t = f2_mul(t, t);
   const float2 p = f2_unpack(t);
-  const unsigned long long r = f2_pack(rcp_approx(p.x), rcp_approx(p.y));
-  const float2 y = f2_unpack(f2_fma(f2_mul(z, f2_pack(-0.5f, -0.5f)), r, f2_pack(fmaxf(x0, 0.f), fmaxf(x1, 0.f))));
+  const unsigned long long r = f2_pack(copysignf(rcp_approx(p.x), x0), copysignf(rcp_approx(p.y), x1));
+  const unsigned long long g = f2_fma(r, f2_pack(-0.5f, -0.5f), f2_pack(step_ge0(x0), step_ge0(x1)));
+  const float2 y = f2_unpack(f2_mul(f2_pack(x0, x1), g));
   x0 = y.x;
   x1 = y.y;
 }

@@ -57,6 +57,22 @@ def test_linear_epilogues_match_oracle(rows, shape):
     assert fm.ops.read_status(st) == 0
 
 
+@pytest.mark.parametrize("rows", [5, 5000])
+def test_gelu_of_infinities(rows):
+    """Infinite and huge accumulators through the GELU of both linear kernels: +inf stays, -inf and NaN are NaN as in torch, a
+    finite one gives itself or zero."""
+    import fast_mimi_b200 as fm
+    a = torch.ones(rows, 64, dtype=torch.float16, device="cuda")
+    a[0, 3], a[1, 3], a[2, 3], a[3, 3], a[4, 3] = float("inf"), -float("inf"), float("nan"), 65504.0, -65504.0
+    w = torch.full((256, 64), 0.5, dtype=torch.float16, device="cuda")
+    want = torch.nn.functional.gelu(a.double() @ w.double().T)
+    assert bool(torch.isinf(want[0]).all()) and bool(torch.isnan(want[1:3]).all())
+    for out_dtype in (torch.float32, torch.float16, torch.bfloat16):
+        got = fm.ops.linear(a, w, activation="gelu", out_dtype=out_dtype)
+        torch.testing.assert_close(got.double(), want, rtol=ROUND[torch.bfloat16], atol=0.0, equal_nan=True)
+    fm.check_status()
+
+
 def test_linear_rejects_bad_geometry():
     import fast_mimi_b200 as fm
     a = torch.zeros(4, 100, dtype=torch.float16, device="cuda")
