@@ -154,16 +154,25 @@ few_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const int warp_lo = a.delta + q0 + qw * 16 - a.window + 1, warp_hi = a.delta + q0 + qw * 16 + 15;
     int n = 0;
     // One 64-key tile; row_of(column) gives a key's row, or a number below every band for a slot nobody sees.
-    auto tile = [&](auto row_of, bool all_visible, bool any_visible, int zero_row) {
+    auto tile = [&](auto row_of, bool all_visible, bool any_visible, bool from_ring) {
       const int st = n % kStages;
       mbar_wait(&c->full[st], static_cast<uint32_t>(n / kStages) & 1u, ctl, status, kErrWaitTma);
       ++n;
       if (any_visible) {
         const uint32_t kb = smem_u32(smem_kv + 2 * st * kTileBytes), vb = kb + kTileBytes;
-        if (zero_row >= 0) {               // what a slot that left the window holds must not reach the sums as 0 * x
-          if (lane < 8) *reinterpret_cast<uint4*>(smem_kv + (2 * st + 1) * kTileBytes + zero_row * 128 + lane * 16) = make_uint4(0u, 0u, 0u, 0u);
-          fence_proxy_async_smem();
-          __syncwarp();
+        if (from_ring) {
+          // What a slot outside the window holds must not reach the sums as 0 * x: one in a full ring of `window` slots,
+          // any number, and frames long past in a ring not yet full, where it has more.  Every warp clears those of its keys.
+          const bool gone = row_of(key0 + lane) < 0;
+          if (gone) {
+#pragma unroll
+            for (int p = 0; p < 8; ++p)
+              *reinterpret_cast<uint4*>(smem_kv + (2 * st + 1) * kTileBytes + (key0 + lane) * 128 + p * 16) = make_uint4(0u, 0u, 0u, 0u);
+          }
+          if (__any_sync(0xffffffffu, gone)) {
+            fence_proxy_async_smem();                    // before the stage's next TMA load
+            __syncwarp();
+          }
         }
         float sc[4][4];
 #pragma unroll
@@ -235,31 +244,16 @@ few_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     };
     for (int i = 0; i < n_ring; ++i) {
       if (!ring_tile_visible(i)) continue;
-      int zero_row = -1;
-      // slots of rows >= delta: the frames a full ring still holds that are no longer visible (slots - delta of them, one
-      // for a ring of `window` slots); further ones only in rings with spare slots
-      for (int r = a.delta; r < a.n_loaded; ++r) {
-        int slot = first + r;
-        if (slot >= a.slots) slot -= a.slots;
-        if (slot / kTile == i) {
-          if (zero_row >= 0 && lane < 8) {
-            const int st = n % kStages;
-            mbar_wait(&c->full[st], static_cast<uint32_t>(n / kStages) & 1u, ctl, status, kErrWaitTma);
-            *reinterpret_cast<uint4*>(smem_kv + (2 * st + 1) * kTileBytes + zero_row * 128 + lane * 16) = make_uint4(0u, 0u, 0u, 0u);
-          }
-          zero_row = slot % kTile;
-        }
-      }
       tile([&](int col) {
         const int slot = i * kTile + col;
         const int r = ring_row(slot);
         return slot >= a.n_loaded || r >= a.delta ? -(1 << 28) : r;
-      }, false, true, zero_row);
+      }, false, true, true);
     }
     for (int j = new_lo; j <= new_hi; ++j) {
       const int r0 = a.delta + j * kTile;
       tile([&](int col) { return r0 + col; }, r0 + kTile - 1 <= a.delta + q0 + qw * 16 && r0 > warp_hi - a.window,
-           r0 + key0 <= warp_hi && r0 + key0 + 31 >= warp_lo, -1);
+           r0 + key0 <= warp_hi && r0 + key0 + 31 >= warp_lo, false);
     }
     // ---- normalise, round, and out through this warp's 16 rows of the query tile
 #pragma unroll

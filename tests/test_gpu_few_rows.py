@@ -75,6 +75,39 @@ def test_layer_on_live_streams_matches_the_oracle(streams, window):
     fm.check_status()
 
 
+# rings with spare slots, partly filled and wrapped, and one of `window` slots; T: the streaming kernel, the few-tile kernel with
+# and without the ring's update inside, the linearised path (slots > 256)
+@pytest.mark.parametrize("slots,past", [(256, 150), (256, 300), (250, 90), (120, 500), (100, 400), (300, 350)])
+@pytest.mark.parametrize("T", [1, 8, 20, 100])
+def test_slots_outside_the_window_do_not_show(slots, past, T):
+    """A layer call over a ring of more slots than the window, non-finite wherever a slot is empty or has left the window:
+    output and new rows are those over a ring that holds the window alone.  Bar: the sums run in another order, and a flipped
+    rounding of a 16-bit operand is 2^-11 of one value in many."""
+    import fast_mimi_b200 as fm
+    S, window = 2, 100
+    layer = fm.MimiTransformerLayerB200(sliding_window=window).cuda()
+    layer.load_state_dict(_layer_params(17))
+    g = torch.Generator(device="cuda").manual_seed(past)
+    ring = fm.MimiKVRing(1, S, window)
+    ring.advance(0, past)
+    k = torch.full((S, 8, slots, 64), float("nan"), dtype=torch.bfloat16, device="cuda")
+    v = k.half()
+    at = torch.arange(past - min(past, window - 1), past, device="cuda")
+    for spare, tight in ((k, ring.ring_k[0]), (v, ring.ring_v[0])):
+        rows = torch.randn(S, 8, len(at), 64, device="cuda", generator=g).to(spare.dtype)
+        spare[:, :, at % slots], tight[:, :, at % window] = rows, rows
+    x = torch.randn(S, T, 512, device="cuda", generator=g)
+    cs = fm.rope_tables(torch.arange(past, past + T, device="cuda")[None])
+    want, _ = layer(x, None, ring, cs)
+    params, keep = layer._native_plan(x)
+    got = fm.ops.layer_forward(params, x, *cs, value_dtype=torch.float16, ring=(k, v), past=past, window=window)
+    assert O.rel_l2(got - x, want - x) < 5e-4
+    new = torch.arange(max(past, past + T - window), past + T, device="cuda")
+    for spare, tight in ((k, ring.ring_k[0]), (v, ring.ring_v[0])):
+        assert torch.equal(spare[:, :, new % slots], tight[:, :, new % window])
+    fm.check_status()
+
+
 def test_layer_follows_its_ring():
     """A session whose ring goes through pickle, then gets new storage, half way: outputs and rings are those of a session
     left alone."""
