@@ -223,7 +223,16 @@ int fm_conv_frames_split(const float* x, void* hi, void* lo, int B, int T, int C
 int fm_linear_split_f32(const void* a_hi, const void* a_lo, long long a_rows, int a_cols, const void* w_hi, const void* w_lo,
                         float* y, long long rows, int clip_rows, int clip_valid, int by_channel, int n_mats, int n_out, int k_in, int* status,
                         void* stream) {
-  return fm::launch_linear_split(a_hi, a_lo, a_rows, a_cols, w_hi, w_lo, y, rows, clip_rows, clip_valid, by_channel, n_mats, n_out, k_in, status,
+  return fm::launch_linear_split(a_hi, a_lo, a_rows, a_cols, w_hi, w_lo, y, rows, clip_rows, clip_valid, by_channel, n_mats, 1, n_out, k_in,
+                                 status, static_cast<cudaStream_t>(stream));
+}
+
+int fm_linear_split_sum_f32(const void* a_hi, const void* a_lo, const void* w_hi, const void* w_lo, float* y, int B, int T, int n_out,
+                            int k_in, int* status, void* stream) {
+  if (B < 0 || T < 0) return -1;
+  const long long rows = static_cast<long long>(B) * T;
+  if (rows == 0) return 0;
+  return fm::launch_linear_split(a_hi, a_lo, rows, k_in, w_hi, w_lo, y, rows, T, T, 1, 1, 2, n_out, k_in, status,
                                  static_cast<cudaStream_t>(stream));
 }
 

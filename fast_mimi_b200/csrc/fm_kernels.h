@@ -69,11 +69,14 @@ int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, co
 // a convolution of twice its stride over padded frames).  Of every clip_rows rows the first clip_valid are results, stored
 // back to back: y [rows * clip_valid / clip_rows, N]; or, with by_channel, clip by clip with the channels outside: y
 // [rows / clip_rows, N, clip_valid].  n_mats > 1: y is so many matrices [.., N / n_mats], one behind the other (several weights'
-// products with the same rows).
+// products with the same rows).  parts = 2: the two halves of K are products of their own (two matrices side by side), whose
+// sums are added once in FP32.  Together in one accumulator they lose bits that two products do not: the tensor core cuts
+// every addend to the accumulator's exponent (K = 512 as one sum 7.0e-7 of the result against 64 bits, as two of 256 4.5e-7).
 struct SplitRows {
   int a_chunks;           // a_cols / 64
   int clip_rows, clip_valid;
   int by_channel;
+  int parts;              // K ranges that have an accumulator each, added in FP32: 1 or 2
   int cols;               // N / n_mats
   long long mat_step;     // values of one of the matrices
   // where column `col` (of a tile that lies in one matrix) of result row `row` goes
@@ -93,6 +96,27 @@ struct SplitRows {
     return row < M && t < clip_valid ? static_cast<long long>(clip) * N * clip_valid + t : -1;
   }
 };
+// The K chunks of a split-precision product in the order of its sums: part by part, in a part lo W_hi, hi W_lo, hi W_hi (the
+// small terms first).
+struct SplitWalk {
+  int part_chunks;        // K chunks of a part in one term
+  int part, term, k;      // k: chunk of the operands
+  __device__ __forceinline__ SplitWalk(int chunks, int index) : part_chunks(chunks), part(index / (3 * chunks)) {
+    const int left = index - 3 * chunks * part;
+    term = left / chunks;
+    k = part * chunks + left - term * chunks;
+  }
+  __device__ __forceinline__ bool a_low() const { return term == 0; }
+  __device__ __forceinline__ bool w_low() const { return term == 1; }
+  __device__ __forceinline__ void next() {
+    if (++k < (part + 1) * part_chunks) return;
+    if (++term == 3) {
+      term = 0;
+      ++part;
+    }
+    k = part * part_chunks;
+  }
+};
 // Tensor maps of the lo parts: a kernel argument of split-precision products alone (256 bytes more cost every launch of the
 // others a quarter of a microsecond).
 template <bool kSplit> struct SplitMaps {};
@@ -102,7 +126,8 @@ struct SplitLow {
   long long a_rows;
 };
 int launch_linear_split(const void* a_hi, const void* a_lo, long long a_rows, int a_cols, const void* w_hi, const void* w_lo, float* y,
-                        long long rows, int clip_rows, int clip_valid, int by_channel, int n_mats, int N, int K, int* status, cudaStream_t st);
+                        long long rows, int clip_rows, int clip_valid, int by_channel, int n_mats, int parts, int N, int K, int* status,
+                        cudaStream_t st);
 int launch_linear_split_small(const void* a_hi, const void* w_hi, const SplitLow& low, const SplitRows& map, float* y, int M, int N,
                               int K, int* status, cudaStream_t st);
 // Padded frames of a causal convolution (kernel a multiple of stride), split into FP16 hi + lo parts: clip b has

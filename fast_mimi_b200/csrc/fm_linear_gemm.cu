@@ -78,7 +78,8 @@ struct LinearArgs {
 // products x . e_j of a nearest-entry search and the epilogue reduces every 64 of them to one 16-byte record
 // {min_j d_j, 64-bit mask of the entries with d_j <= min + margin[row]},  d_j = |e_j|^2 - 2 x . e_j  (see fm_rvq.cu).
 // 4 = FP32 y of a split-precision product: both operands are pairs of FP16 matrices hi + lo, and K runs three times,
-// lo W_hi, hi W_lo, hi W_hi (the small terms first), into one accumulator.  As three products that handed FP32 sums on
+// lo W_hi, hi W_lo, hi W_hi (the small terms first), into one accumulator (or, for two products that are to be added, into one
+// each).  As three products that handed FP32 sums on
 // through memory the same work moved 20 bytes per output value instead of four (64000 rows, K = 2048, N = 512: 317 us here,
 // 1.27 PFLOP/s over the three terms).
 template <int kOut, bool kWide, int kBlockN>
@@ -103,7 +104,9 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   const uint32_t rank = cluster_cta_rank();
   const bool leader = rank == 0;
   const int n_tiles = args.N / kBlockN;
-  const int k_part = args.K / kBlockK, k_chunks = kSplit ? 3 * k_part : k_part;
+  const int k_chunks = (kSplit ? 3 : 1) * (args.K / kBlockK);
+  // accumulators per unit (a split-precision product of two parts fills both buffers), K chunks of one
+  const int n_acc = kSplit ? args.rows.parts : 1, part_chunks = args.K / kBlockK / n_acc, acc_chunks = k_chunks / n_acc;
   // Units are dealt round-robin: at any moment neighbouring pairs work on the output tiles of the SAME rows,
   // so the slices of a that one of them pulls from HBM are L2 hits for the others (with contiguous ranges
   // per pair the second output tile of a row tile came 30 us after the first and its a tile had been evicted:
@@ -151,24 +154,26 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         tma_prefetch_desc(&low.a);
         tma_prefetch_desc(&low.w);
       }
-      auto load_w = [&](uint8_t* dst, int kc, uint64_t* bar, int n0) {
-        if constexpr (kSplit) tma_load_2d_pair(dst, kc / k_part == 1 ? &low.w : &tmap_w, bar, kc % k_part * kBlockK, n0);
+      auto load_w = [&](uint8_t* dst, int kc, const SplitWalk& w, uint64_t* bar, int n0) {
+        if constexpr (kSplit) tma_load_2d_pair(dst, w.w_low() ? &low.w : &tmap_w, bar, w.k * kBlockK, n0);
         else tma_load_2d_pair(dst, &tmap_w, bar, kc * kBlockK, n0);
       };
       int stage = 0;
       uint32_t phase = 0;
       // The W slices of the first stages do not depend on the kernel in front: they are requested before the wait.
       const int ahead = u_count > 0 ? (k_chunks < kStages ? k_chunks : kStages) : 0;
-      for (int kc = 0; kc < ahead; ++kc) {
+      SplitWalk first(part_chunks, 0);
+      for (int kc = 0; kc < ahead; ++kc, first.next()) {
         if (leader) mbar_arrive_expect_tx(&bars->full[kc], 2 * kStageBytes);
-        load_w(smem_stage + kc * kStageBytes + kABytes, kc, &bars->full[kc], (pair % n_tiles) * kBlockN + static_cast<int>(rank) * kHalfN);
+        load_w(smem_stage + kc * kStageBytes + kABytes, kc, first, &bars->full[kc], (pair % n_tiles) * kBlockN + static_cast<int>(rank) * kHalfN);
       }
       griddep_wait();
       for (int i = 0; i < u_count; ++i) {
         const int u = pair + i * n_pairs, row_tile = u / n_tiles, ntile = u % n_tiles;
         const int m0 = (2 * row_tile + static_cast<int>(rank)) * kBlockM;
         const int n0 = ntile * kBlockN + static_cast<int>(rank) * kHalfN;
-        for (int kc = 0; kc < k_chunks; ++kc) {
+        SplitWalk w(part_chunks, 0);
+        for (int kc = 0; kc < k_chunks; ++kc, w.next()) {
           const bool early = i == 0 && kc < ahead;
           if (!early) {
             mbar_wait(&bars->empty[stage], phase ^ 1u, ctl, status, kErrWaitConsumer);
@@ -176,12 +181,12 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           }
           uint8_t* dst = smem_stage + stage * kStageBytes;
           if constexpr (kSplit) {
-            const int k = kc % k_part;            // a row of the product continues in the matrix's next row
-            tma_load_2d_pair(dst, kc < k_part ? &low.a : &tmap_a, &bars->full[stage], k % args.rows.a_chunks * kBlockK, m0 + k / args.rows.a_chunks);
+            // a row of the product continues in the matrix's next row
+            tma_load_2d_pair(dst, w.a_low() ? &low.a : &tmap_a, &bars->full[stage], w.k % args.rows.a_chunks * kBlockK, m0 + w.k / args.rows.a_chunks);
           } else {
             tma_load_2d_pair(dst, &tmap_a, &bars->full[stage], kc * kBlockK, m0);
           }
-          if (!early) load_w(dst + kABytes, kc, &bars->full[stage], n0);
+          if (!early) load_w(dst + kABytes, kc, w, &bars->full[stage], n0);
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
       }
@@ -194,13 +199,13 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
       const bool elected = elect_one();
       int stage = 0;
       uint32_t phase = 0;
-      for (int i = 0; i < u_count; ++i) {
+      for (int i = 0; i < u_count * n_acc; ++i) {            // accumulators, taken by the buffers in turn
         const int buf = i & 1;
         const uint32_t use = static_cast<uint32_t>(i >> 1);
         mbar_wait(&bars->acc_empty[buf], (use & 1u) ^ 1u, ctl, status, kErrWaitConsumer);
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * kBlockN);
-        for (int kc = 0; kc < k_chunks; ++kc) {
+        for (int kc = 0; kc < acc_chunks; ++kc) {
           mbar_wait(&bars->full[stage], phase, ctl, status, kErrWaitTma);
           tc_fence_after_sync();
           const uint32_t base = smem_u32(smem_stage + stage * kStageBytes);
@@ -252,13 +257,16 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         if (n_pieces > 0) fetch(0, res);
 #pragma unroll 1
         for (int idx = 0; idx < n_pieces; ++idx) {
-          const int i = idx / kPieces, p = idx % kPieces, buf = i & 1;
+          const int i = idx / kPieces, p = idx % kPieces, buf = n_acc == 2 ? 0 : i & 1;
           if (p == 0) {
-            mbar_wait(&bars->acc_full[buf], static_cast<uint32_t>(i >> 1) & 1u, ctl, status, kErrWaitMma);
+            const uint32_t parity = static_cast<uint32_t>(n_acc == 2 ? i : i >> 1) & 1u;
+            mbar_wait(&bars->acc_full[buf], parity, ctl, status, kErrWaitMma);
+            if (n_acc == 2) mbar_wait(&bars->acc_full[1], parity, ctl, status, kErrWaitMma);
             tc_fence_after_sync();
           }
           uint32_t acc[32];
-          tmem_ld32(tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + static_cast<uint32_t>(buf * kBlockN + (gsel * kPieces + p) * 32), acc);
+          const uint32_t t_piece = tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + static_cast<uint32_t>(buf * kBlockN + (gsel * kPieces + p) * 32);
+          tmem_ld32(t_piece, acc);
           R next[8];
           if (idx + 1 < n_pieces) fetch(idx + 1, next);
           const int col = first_col(i, p);
@@ -266,11 +274,23 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           uint4 sc_raw = make_uint4(0u, 0u, 0u, 0u);
           if (scaled) sc_raw = args.scale.raw4<kF32>(col);
           tmem_ld_wait();
+          if constexpr (kSplit) {
+            if (n_acc == 2) {
+              uint32_t other[32];
+              tmem_ld32(t_piece + kBlockN, other);
+              tmem_ld_wait();
+#pragma unroll
+              for (int c = 0; c < 32; ++c) acc[c] = __float_as_uint(__uint_as_float(acc[c]) + __uint_as_float(other[c]));
+            }
+          }
           if (p == kPieces - 1) {
             // Last read of the accumulator by this warp: hand it back before the arithmetic and the stores.
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster_relaxed(acc_empty_leader + static_cast<uint32_t>(buf) * 8u);
+            if (lane == 0) {
+              mbar_arrive_cluster_relaxed(acc_empty_leader + static_cast<uint32_t>(buf) * 8u);
+              if (n_acc == 2) mbar_arrive_cluster_relaxed(acc_empty_leader + 8u);
+            }
           }
           float v[32];
 #pragma unroll
@@ -518,10 +538,12 @@ int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, co
 }
 
 int launch_linear_split(const void* a_hi, const void* a_lo, long long a_rows, int a_cols, const void* w_hi, const void* w_lo, float* y,
-                        long long rows, int clip_rows, int clip_valid, int by_channel, int n_mats, int N, int K, int* status, cudaStream_t st) {
+                        long long rows, int clip_rows, int clip_valid, int by_channel, int n_mats, int parts, int N, int K, int* status,
+                        cudaStream_t st) {
   using namespace lin;
   if (rows < 0 || a_rows > 0x7fffffffLL || a_rows < rows || N <= 0 || K <= 0 || N % 256 != 0 || a_cols <= 0 || a_cols % kBlockK != 0 ||
-      K % a_cols != 0 || n_mats <= 0 || N % (256 * n_mats) != 0 || (by_channel && n_mats != 1) || clip_rows <= 0 || clip_valid <= 0 || clip_valid > clip_rows)
+      K % a_cols != 0 || n_mats <= 0 || N % (256 * n_mats) != 0 || (by_channel && n_mats != 1) || parts < 1 || parts > 2 ||
+      K % (parts * kBlockK) != 0 || clip_rows <= 0 || clip_valid <= 0 || clip_valid > clip_rows)
     return -1;
   if (rows == 0) return 0;
   if (a_hi == nullptr || a_lo == nullptr || w_hi == nullptr || w_lo == nullptr || y == nullptr) return -1;
@@ -531,7 +553,7 @@ int launch_linear_split(const void* a_hi, const void* a_lo, long long a_rows, in
   const int M = static_cast<int>(rows);
   const SplitLow low = {a_lo, w_lo, a_rows};
   const long long results = (rows + clip_rows - 1) / clip_rows * clip_valid - (rows % clip_rows != 0 && rows % clip_rows < clip_valid ? clip_valid - rows % clip_rows : 0);
-  const SplitRows map = {a_cols / kBlockK, clip_rows, clip_valid, by_channel, N / n_mats, results * (N / n_mats)};
+  const SplitRows map = {a_cols / kBlockK, clip_rows, clip_valid, by_channel, parts, N / n_mats, results * (N / n_mats)};
   if (few_row_tiles(M, N)) return launch_linear_split_small(a_hi, w_hi, low, map, y, M, N, K, status, st);
   const int pair_tiles = ((M + kBlockM - 1) / kBlockM + 1) / 2;
   const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;

@@ -55,14 +55,14 @@ __device__ __forceinline__ void bulk_copy_to_cta(uint32_t dst, const void* src, 
 }  // namespace small
 
 // kOut: 0 = BF16, 1 = FP16, 2 = FP32 output and residual; 3 = q | k | v with RoPE (VT: type of v); 4 = FP32 output of a
-// split-precision product: K runs three times (lo W_hi, hi W_lo, hi W_hi), shared out like any other K
+// split-precision product: K runs three times (lo W_hi, hi W_lo, hi W_hi; part by part), shared out like any other K
 template <int kOut, typename VT, int kBlockN>
 __global__ void __launch_bounds__(small::kThreads)
 linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
                     const __grid_constant__ SplitMaps<kOut == 4> low,
                     const __grid_constant__ SmallArgs args, uint32_t idesc, int* status) {
   using namespace small;
-  constexpr int kStageBytes = Tile<kBlockN>::kStageBytes, kRedBytes = Tile<kBlockN>::kRedBytes, kTmemCols = kBlockN;
+  constexpr int kStageBytes = Tile<kBlockN>::kStageBytes, kRedBytes = Tile<kBlockN>::kRedBytes, kTmemCols = (kOut == 4 ? 2 : 1) * kBlockN;
   constexpr int kHalves = kBlockN / 32;
   constexpr uint32_t kRowBytes = kBlockN * 4;
   extern __shared__ uint8_t smem_raw[];
@@ -76,6 +76,9 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const int n0 = ntile * kBlockN;
   const int m0 = static_cast<int>(blockIdx.y) * kBlockM;
   const int chunk0 = rank * args.chunks;
+  // Two parts of a split-precision product in one block have an accumulator each; shared out over an even number of blocks,
+  // every block has chunks of one part.
+  const bool two_acc = kOut == 4 && args.rows.parts == 2 && split == 1;
   // Row r of the tile belongs to rank r % S.
   const int log_s = 31 - __clz(split);
   const int valid = args.M - m0 < kBlockM ? args.M - m0 : kBlockM;
@@ -111,19 +114,20 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       tma_prefetch_desc(&tmap_a);
       auto load_a = [&](int st, int kc) {
         if constexpr (kOut == 4) {
-          const int k = kc % args.k_part;         // a row of the product continues in the matrix's next row
-          tma_load_2d(smem + st * kStageBytes, kc < args.k_part ? &low.a : &tmap_a, &bars->full[st],
-                      k % args.rows.a_chunks * kBlockK, m0 + k / args.rows.a_chunks);
+          const SplitWalk w(args.part_chunks, kc);  // a row of the product continues in the matrix's next row
+          tma_load_2d(smem + st * kStageBytes, w.a_low() ? &low.a : &tmap_a, &bars->full[st],
+                      w.k % args.rows.a_chunks * kBlockK, m0 + w.k / args.rows.a_chunks);
         } else {
           tma_load_2d(smem + st * kStageBytes, &tmap_a, &bars->full[st], kc * kBlockK, m0);
         }
       };
       auto load_w = [&](int st, int kc) {
-        if constexpr (kOut == 4)
-          tma_load_2d(smem + st * kStageBytes + kABytes, kc / args.k_part == 1 ? &low.w : &tmap_w, &bars->full[st],
-                      kc % args.k_part * kBlockK, n0);
-        else
+        if constexpr (kOut == 4) {
+          const SplitWalk w(args.part_chunks, kc);
+          tma_load_2d(smem + st * kStageBytes + kABytes, w.w_low() ? &low.w : &tmap_w, &bars->full[st], w.k * kBlockK, n0);
+        } else {
           tma_load_2d(smem + st * kStageBytes + kABytes, &tmap_w, &bars->full[st], kc * kBlockK, n0);
+        }
       };
       const int ahead = args.chunks < kStages ? args.chunks : kStages;
       for (int i = 0; i < ahead; ++i) {
@@ -143,8 +147,10 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     __syncwarp();
   } else if (warp == 5) {
     const bool one = elect_one();
+    const int half = two_acc ? args.chunks / 2 : args.chunks;
     for (int i = 0; i < args.chunks; ++i) {
       const int st = i % kStages;
+      const uint32_t d_tmem = tmem_base + (i < half ? 0u : static_cast<uint32_t>(kBlockN));
       mbar_wait(&bars->full[st], static_cast<uint32_t>(i / kStages) & 1u, ctl, status, kErrWaitTma);
       tc_fence_after_sync();
       const uint32_t base = smem_u32(smem + st * kStageBytes);
@@ -152,7 +158,7 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       const uint64_t b_desc = umma_desc_sw128(base + kABytes);
 #pragma unroll
       for (int ks = 0; ks < kBlockK / 16; ++ks)
-        if (one) tc_mma_ss(tmem_base, a_desc + 2u * ks, b_desc + 2u * ks, idesc, (i | ks) != 0 ? 1u : 0u);
+        if (one) tc_mma_ss(d_tmem, a_desc + 2u * ks, b_desc + 2u * ks, idesc, ((i < half ? i : i - half) | ks) != 0 ? 1u : 0u);
       if (one) tc_commit(&bars->empty[st]);
     }
     if (one) tc_commit(&bars->acc_full);
@@ -183,6 +189,13 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       uint32_t v[32];
       tmem_ld32(t_row + h * 32, v);
       tmem_ld_wait();
+      if (two_acc) {
+        uint32_t other[32];
+        tmem_ld32(t_row + kBlockN + h * 32, other);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) + __uint_as_float(other[c]));
+      }
       if (row < valid) {
 #pragma unroll
         for (int c = 0; c < 8; ++c)
@@ -271,8 +284,8 @@ static int launch_tiles(const void* a, const void* w, SmallArgs& args, int K, in
     if (rc == 0) rc = encode_rows_16bit(&low_maps.w, low->w, static_cast<uint64_t>(args.N), static_cast<uint64_t>(K), kBlockN, kBlockK);
     if (rc != 0) return rc;
   }
-  args.k_part = K / kBlockK;
-  const int k_chunks = kOut == 4 ? 3 * args.k_part : args.k_part;
+  if constexpr (kOut == 4) args.part_chunks = K / kBlockK / args.rows.parts;
+  const int k_chunks = (kOut == 4 ? 3 : 1) * (K / kBlockK);
   args.split = choose_split(m_tiles * n_tiles, k_chunks);
   args.chunks = k_chunks / args.split;
   const int fmt = in_dtype == 1 ? 0 : 1;

@@ -26,7 +26,7 @@ struct SmallArgs {
   int gelu;
   QkvEpilogueArgs qkv;    // kOut 3
   SplitRows rows;         // kOut 4
-  int k_part;             // kOut 4: K / 64 of one of the three products
+  int part_chunks;        // kOut 4: K chunks of a part in one of the three products
 };
 
 // What the epilogue of eight values of row `row` of output tile `ntile` (64 columns, one attention head) reads besides the

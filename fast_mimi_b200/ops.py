@@ -775,9 +775,14 @@ def rvq_decode_project(codes, first: RVQCodebooks, second: RVQCodebooks | None, 
                                      hi.data_ptr(), lo.data_ptr(), B, T, K, n0, first.entries,
                                      0 if second is None else second.entries, bad.data_ptr(), _stream())
         _native.check(rc, "fm_rvq_decode_split")
-        rc = lib.fm_linear_split_f32(hi.data_ptr(), lo.data_ptr(), B * T, width, w_hi.data_ptr(), w_lo.data_ptr(), y.data_ptr(), B * T,
-                                     T, T, 1, 1, w_hi.shape[0], width, _status_ptr(status, codes), _stream())
-        _native.check(rc, "fm_linear_split_f32")
+        st, n_out = _status_ptr(status, codes), w_hi.shape[0]
+        if second is None:
+            rc = lib.fm_linear_split_f32(hi.data_ptr(), lo.data_ptr(), B * T, width, w_hi.data_ptr(), w_lo.data_ptr(), y.data_ptr(), B * T,
+                                         T, T, 1, 1, n_out, width, st, _stream())
+        else:      # each stack in an accumulator of its own, as precise as two products and their sum
+            rc = lib.fm_linear_split_sum_f32(hi.data_ptr(), lo.data_ptr(), w_hi.data_ptr(), w_lo.data_ptr(), y.data_ptr(), B, T, n_out,
+                                             width, st, _stream())
+        _native.check(rc, "fm_linear_split")
     if int(bad.item()) != 0:
         raise RuntimeError("rvq_decode: a code index is outside the codebook")
     check_status(codes.device, status)      # the stream is already synchronised by the read above

@@ -116,8 +116,8 @@ class MimiSplitRVQB200:
         return self._joint_in[2]
 
     def _joint_out_parts(self):
-        """Both output projections as one weight over [semantic | acoustic], whose accumulator then adds the branches; made
-        once for a pair of branches, ``None`` where they do not fit together."""
+        """Both output projections as one weight over [semantic | acoustic], whose product adds the branches; made once for a
+        pair of branches, ``None`` where they do not fit together."""
         sem, aco = self.semantic, self.acoustic
         w0, w1 = sem.output_proj, aco.output_proj
         if self._joint is None or self._joint[0] is not w0 or self._joint[1] is not w1:

@@ -211,6 +211,12 @@ int fm_linear_split_f32(const void* a_hi, const void* a_lo, long long a_rows, in
                         float* y, long long rows, int clip_rows, int clip_valid, int by_channel, int n_mats, int n_out, int k_in, int* status,
                         void* stream);
 
+/* The sum of two such products, each with an accumulator of its own and the two added in FP32: the output projections of a
+ * split quantiser's branches (src/fast_mimi/model.py:2447-2480).  The halves of k_in (a multiple of 128) are the branches, side
+ * by side in a [B * T, k_in] and w [n_out, k_in]; y [B, n_out, T]. */
+int fm_linear_split_sum_f32(const void* a_hi, const void* a_lo, const void* w_hi, const void* w_lo, float* y, int B, int T, int n_out,
+                            int k_in, int* status, void* stream);
+
 /* The stride-2 upsampling that precedes the decoder transformer (MimiModel.upsample: MimiConvTranspose1d(512, 512,
  * kernel 4, stride 2, groups 512, no bias), src/fast_mimi/model.py:2745-2753; its forward trims the last two output
  * frames): x [B, T, C] FP32 frame-major, w [C, 4] FP32 (the ConvTranspose1d weight [C, 1, 4]) -> y [B, 2T, C] FP32,

@@ -178,6 +178,23 @@ def test_decode_with_projection_matches_fp64(B, T, stacks):
         q.decode(codes.cuda())
 
 
+# one block per tile of K slices, two, both parts in one block (few rows), pairs of blocks with 128- and 256-wide units
+@pytest.mark.parametrize("rows", [13, 200, 750, 1300, 4000, 6000, 20000])
+def test_joint_decode_is_as_precise_as_the_branches(rows):
+    """Both output projections in one product: its distance from 64 bits is that of two products, each in one accumulator (as
+    calls of many rows have it), and their FP32 sum.  Bar: 5 % for the FP32 sums of K slices."""
+    import fast_mimi_b200 as fm
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    n = lambda *s, std=1.0: torch.empty(s, device="cuda").normal_(0, std, generator=g)
+    branch = lambda: fm.MimiRVQB200(n(1, 2048, 256), None, n(512, 256, 1, std=256 ** -0.5))
+    q = fm.MimiSplitRVQB200(branch(), branch())
+    codes = torch.randint(0, 2048, (1, 2, rows), device="cuda", generator=g)
+    exact = sum(b.books.vectors[0].double()[codes[0, i]] @ b.output_proj.double().T for i, b in enumerate((q.semantic, q.acoustic))).T
+    many = codes.repeat(1, 1, -(-6000 // rows))
+    apart = q.semantic.decode(many[:, :1]) + q.acoustic.decode(many[:, 1:])
+    assert O.rel_l2(q.decode(codes)[0], exact) < 1.05 * O.rel_l2(apart[0, :, :rows], exact)
+
+
 @pytest.mark.parametrize("rows", [1, 63, 5000, 20001])
 def test_split_precision_products_of_two_weights(rows):
     """Two weights behind one another give two matrices, with few rows and many, equal to the products one by one up to the
