@@ -441,7 +441,9 @@ __device__ __forceinline__ void st_global_v8(void* p, const uint32_t* w) {
 
 // Programmatic dependent launch.  A kernel of a chain waits here for the kernel in front of it (completed, its writes
 // visible); without the launch attribute both are no-ops.  What comes BEFORE the wait may only read what no kernel of
-// the chain writes (weights).
+// the chain writes (weights).  What a kernel of the chain writes is read with __ldcg or by TMA, i.e. from L2, and never with
+// __ldg or through a const __restrict__ pointer: the read-only path asks for data that stays as it is while the kernel
+// runs, which began before that one was done, and L1 may hold a line that a kernel of the chain on the same SM read earlier.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The status word of the chain was already non-zero when this kernel began: it does nothing, but still waits for the
 // kernel in front, so that its own end means that everything before it has ended too.

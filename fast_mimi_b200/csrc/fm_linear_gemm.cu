@@ -251,7 +251,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           const uint8_t* src = static_cast<const uint8_t*>(args.resid) + (static_cast<long long>(row) * args.N + first_col(i, idx % kPieces)) * kElem;
 #pragma unroll
           for (int k = 0; k < 8; ++k)
-            if (row + 4 * k < args.M) r[k] = *reinterpret_cast<const R*>(src + static_cast<long long>(4 * k) * args.N * kElem);
+            if (row + 4 * k < args.M) r[k] = __ldcg(reinterpret_cast<const R*>(src + static_cast<long long>(4 * k) * args.N * kElem));
         };
         R res[8];
         if (n_pieces > 0) fetch(0, res);
@@ -383,7 +383,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             v[4 * j + 2] = fmaf(-2.f, v[4 * j + 2], q.z); v[4 * j + 3] = fmaf(-2.f, v[4 * j + 3], q.w);
             dmin = fminf(dmin, fminf(fminf(v[4 * j], v[4 * j + 1]), fminf(v[4 * j + 2], v[4 * j + 3])));
           }
-          const float limit = dmin + (row_ok ? __ldg(static_cast<const float*>(args.resid) + row) : 0.f);
+          const float limit = dmin + (row_ok ? __ldcg(static_cast<const float*>(args.resid) + row) : 0.f);
           uint32_t m_lo = 0u, m_hi = 0u;
 #pragma unroll
           for (int c = 0; c < 32; ++c) {

@@ -175,7 +175,7 @@ __device__ __forceinline__ float rvq_margin(float xx, float e_max, float tau_rel
 // frames, read.
 template <bool kLast>
 __global__ void __launch_bounds__(rvq::kWarps * 32)
-rvq_select_rec_kernel(const uint4* __restrict__ records, const float* __restrict__ codebook, float* __restrict__ resid,
+rvq_select_rec_kernel(const uint4* records, const float* __restrict__ codebook, float* __restrict__ resid,
                       uint16_t* __restrict__ resid16, long long* __restrict__ codes, int* __restrict__ n_candidates,
                       float* __restrict__ tau, long long rows, int n_groups, float e_max_next, float tau_rel,
                       int* __restrict__ status) {
@@ -190,15 +190,16 @@ rvq_select_rec_kernel(const uint4* __restrict__ records, const float* __restrict
     float4 a, b;               // this lane's eight residual values
     float margin;
   };
+  // records, residual and margins are written by kernels that may have run beside this one's prologue: from L2 (see griddep_wait)
   auto fetch_x = [&](long long row, Frame& f) {
     const float4* xr = reinterpret_cast<const float4*>(resid + row * kDim + lane * 8);
-    f.a = xr[0];
-    f.b = xr[1];
+    f.a = __ldcg(xr);
+    f.b = __ldcg(xr + 1);
   };
   auto fetch = [&](long long row, Frame& f) {
     f.rec = make_uint4(__float_as_uint(INFINITY), 0u, 0u, 0u);
-    if (lane < n_groups) f.rec = records[row * n_groups + lane];
-    f.margin = tau[row];
+    if (lane < n_groups) f.rec = __ldcg(records + row * n_groups + lane);
+    f.margin = __ldcg(tau + row);
     if constexpr (!kLast) fetch_x(row, f);
   };
   Frame next;

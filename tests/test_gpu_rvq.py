@@ -178,6 +178,21 @@ def test_decode_with_projection_matches_fp64(B, T, stacks):
         q.decode(codes.cuda())
 
 
+@pytest.mark.parametrize("rows", [1, 63, 500])
+def test_search_repeats_exactly(rows):
+    """The chain of dependent launches over 31 layers, whose kernels share SMs and rewrite the same few buffers layer by layer:
+    every call gives the codes of the form that goes through memory one launch at a time."""
+    import fast_mimi_b200 as fm
+    gen, embed_sum, usage, _ = rvq_recipe(rows, 31)
+    scale = 0.7 ** torch.arange(31.0)
+    books = fm.ops.RVQCodebooks((_books(embed_sum, usage) * scale[:, None, None]).cuda())
+    x = torch.randn(rows, 256, generator=gen).cuda()
+    want = fm.ops.rvq_encode(x, books, scores_dtype=torch.float32)
+    for _ in range(50):
+        assert torch.equal(fm.ops.rvq_encode(x, books), want)
+    fm.check_status()
+
+
 # one block per tile of K slices, two, both parts in one block (few rows), pairs of blocks with 128- and 256-wide units
 @pytest.mark.parametrize("rows", [13, 200, 750, 1300, 4000, 6000, 20000])
 def test_joint_decode_is_as_precise_as_the_branches(rows):
