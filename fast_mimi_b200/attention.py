@@ -29,6 +29,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
+from ._origin import Origin
 from .kv_ring import LinearKVCache, MimiKVRing
 
 
@@ -98,6 +99,8 @@ def rope_tables(position_ids: torch.Tensor, *, head_dim: int = 64, theta: float 
 
 
 class MimiAttentionB200(nn.Module):
+    _packed_from = _wo16_from = Origin()        # what the 16-bit copies were made from
+
     def __init__(self, hidden_size: int = 512, num_heads: int = 8, head_dim: int = 64, sliding_window: int = 250,
                  layer_idx: int = 0, precision: str = "tc", value_dtype: torch.dtype = torch.float16,
                  input_dtype: torch.dtype | None = None) -> None:
@@ -123,9 +126,7 @@ class MimiAttentionB200(nn.Module):
         self.v_proj = nn.Linear(hidden_size, num_heads * head_dim, bias=False)
         self.o_proj = nn.Linear(num_heads * head_dim, hidden_size, bias=False)
         self._packed: torch.Tensor | None = None
-        self._packed_key: tuple | None = None
         self._wo16: torch.Tensor | None = None
-        self._wo16_key: tuple | None = None
 
     @classmethod
     def from_reference(cls, attn: nn.Module, precision: str = "tc",
@@ -151,19 +152,17 @@ class MimiAttentionB200(nn.Module):
         """``cat(Wq, Wk, Wv)`` as a 16-bit ``[1536, 512]`` tensor, rebuilt when a projection weight changes
         (the reference packs once the same way: src/fast_mimi/_packed_qkv.py:139-150)."""
         ws = (self.q_proj.weight, self.k_proj.weight, self.v_proj.weight)
-        key = tuple((w.data_ptr(), w._version, w.device) for w in ws) + (dtype,)
-        if self._packed is None or self._packed_key != key:
+        if self._packed is None or self._packed.dtype != dtype or not self._packed_from.still(*ws):
             self._packed = torch.cat([w.detach() for w in ws], dim=0).to(dtype).contiguous()
-            self._packed_key = key
+            self._packed_from = Origin(*ws)
         return self._packed
 
     def out_weight(self, dtype: torch.dtype) -> torch.Tensor:
         """``o_proj.weight`` as a 16-bit tensor, rebuilt when the weight changes."""
         w = self.o_proj.weight
-        key = (w.data_ptr(), w._version, w.device, dtype)
-        if self._wo16 is None or self._wo16_key != key:
+        if self._wo16 is None or self._wo16.dtype != dtype or not self._wo16_from.still(w):
             self._wo16 = w.detach().to(dtype).contiguous()
-            self._wo16_key = key
+            self._wo16_from = Origin(w)
         return self._wo16
 
     def _tc_input_dtype(self, hidden_states: torch.Tensor) -> torch.dtype:

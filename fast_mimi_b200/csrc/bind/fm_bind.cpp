@@ -6,7 +6,7 @@
 //
 // `LayerPlan` holds what a layer's native call needs (the parameter block, the tensors behind it) and what it was made
 // from: dictionary entries of the modules (parameters, submodules, options) with the objects found there, and for tensors
-// their storage address and version counter.  `layer_forward` returns None when anything has changed or anything about
+// their storage, version counter, type and layout.  `layer_forward` returns None when anything has changed or anything about
 // the arguments is out of the ordinary; the Python side then validates, rebuilds or raises.
 #include <Python.h>
 
@@ -14,20 +14,40 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
-#include <string>
+#include <memory>
+#include <optional>
+#include <utility>
 #include <vector>
 
 #include "../../../include/fast_mimi_b200.h"
 
 namespace {
 
+// What a tensor's contents are known by.  The storage counts by its identity: assigning a parameter's .data moves no version
+// counter, and an address is given out again once its storage is gone.  The weak reference keeps the identity, not the memory.
+// Throws for tensors without storage (wrappers of transforms) and without a version counter (made in inference mode): such a
+// one cannot be watched.
+struct Stamp {
+  explicit Stamp(const at::Tensor& t)
+      : storage(t.storage().getWeakStorageImpl()), data(t.const_data_ptr()), version(static_cast<uint32_t>(t._version())),
+        dtype(t.scalar_type()), sizes(t.sizes()), strides(t.strides()) {}
+  bool still(const at::Tensor& t) const {
+    return t.storage().unsafeGetStorageImpl() == storage._unsafe_get_target() && t.const_data_ptr() == data &&
+           static_cast<uint32_t>(t._version()) == version && t.scalar_type() == dtype && t.sizes() == at::IntArrayRef(sizes) &&
+           t.strides() == at::IntArrayRef(strides);
+  }
+  c10::weak_intrusive_ptr<c10::StorageImpl> storage;
+  const void* data;
+  uint32_t version;
+  c10::ScalarType dtype;
+  c10::DimVector sizes, strides;
+};
+
 struct Watch {
   PyObject* dict;
   PyObject* key;
   PyObject* value;
-  bool tensor;
-  const void* data;
-  uint32_t version;
+  std::optional<Stamp> stamp;      // of a tensor
 };
 
 struct LayerPlan {
@@ -78,13 +98,6 @@ int plan_clear(PyObject* self_obj) {
   return 0;
 }
 
-// What a tensor's contents are known by.  Throws for tensors without storage (wrappers of transforms) and without a version
-// counter (made in inference mode): such a one cannot be watched.
-void stamp(const at::Tensor& t, const void** data, uint32_t* version) {
-  *data = t.const_data_ptr();
-  *version = static_cast<uint32_t>(t._version());
-}
-
 // LayerPlan(watches, keep, params_address, status, like, value_like): watches is a list of (dict, key); keep the tensors
 // behind the parameter block at params_address (copied); status an int32 tensor; like / value_like tensors whose type and
 // device activations / ring values must have.
@@ -119,9 +132,9 @@ PyObject* plan_new(PyTypeObject* type, PyObject* args, PyObject*) {
       Py_DECREF(self);
       return nullptr;
     }
-    Watch w = {dict, key, value, THPVariable_Check(value), nullptr, 0};
+    Watch w = {dict, key, value, std::nullopt};
     try {
-      if (w.tensor) stamp(THPVariable_Unpack(value), &w.data, &w.version);
+      if (THPVariable_Check(value)) w.stamp.emplace(THPVariable_Unpack(value));
     } catch (const std::exception&) {
       PyErr_SetObject(PyExc_KeyError, key);
       Py_DECREF(self);
@@ -130,7 +143,7 @@ PyObject* plan_new(PyTypeObject* type, PyObject* args, PyObject*) {
     Py_INCREF(dict);
     Py_INCREF(key);
     Py_INCREF(value);
-    self->watches->push_back(w);
+    self->watches->push_back(std::move(w));
   }
   return reinterpret_cast<PyObject*>(self);
 }
@@ -141,12 +154,7 @@ bool unchanged(const LayerPlan* plan) {
       PyErr_Clear();
       return false;
     }
-    if (w.tensor) {
-      const void* data;
-      uint32_t version;
-      stamp(THPVariable_Unpack(w.value), &data, &version);
-      if (data != w.data || version != w.version) return false;
-    }
+    if (w.stamp && !w.stamp->still(THPVariable_Unpack(w.value))) return false;
   }
   return true;
 }
@@ -228,8 +236,66 @@ PyObject* layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
 }
 
+constexpr const char* kStampsName = "_fm_bind.stamps";
+
+void stamps_free(PyObject* capsule) {
+  delete static_cast<std::vector<Stamp>*>(PyCapsule_GetPointer(capsule, kStampsName));
+}
+
+// stamps(*tensors) -> an object for still().
+PyObject* stamps(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  try {
+    auto made = std::make_unique<std::vector<Stamp>>();
+    for (Py_ssize_t i = 0; i < n; ++i) {
+      if (!THPVariable_Check(a[i])) {
+        PyErr_SetString(PyExc_TypeError, "stamps(*tensors)");
+        return nullptr;
+      }
+      made->emplace_back(THPVariable_Unpack(a[i]));
+    }
+    PyObject* capsule = PyCapsule_New(made.get(), kStampsName, stamps_free);
+    if (capsule != nullptr) made.release();
+    return capsule;
+  } catch (const c10::Error& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+    return nullptr;
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+}
+
+// still(stamps, *tensors) -> whether these are the stamped tensors, unchanged.
+PyObject* still(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n < 1) {
+    PyErr_SetString(PyExc_TypeError, "still(stamps, *tensors)");
+    return nullptr;
+  }
+  const auto* seen = static_cast<const std::vector<Stamp>*>(PyCapsule_GetPointer(a[0], kStampsName));
+  if (seen == nullptr) return nullptr;
+  if (static_cast<Py_ssize_t>(seen->size()) != n - 1) Py_RETURN_FALSE;
+  try {
+    for (Py_ssize_t i = 1; i < n; ++i)
+      if (!THPVariable_Check(a[i]) || !(*seen)[i - 1].still(THPVariable_Unpack(a[i]))) Py_RETURN_FALSE;
+  } catch (const c10::Error& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+    return nullptr;
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+  Py_RETURN_TRUE;
+}
+
+template <PyObject* (*kFn)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyCFunction fast_call() {
+  return reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(kFn));
+}
+
 PyMethodDef methods[] = {
-    {"layer_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(layer_forward)), METH_FASTCALL,
+    {"stamps", fast_call<stamps>(), METH_FASTCALL, "stamps(*tensors) -> what their contents are known by"},
+    {"still", fast_call<still>(), METH_FASTCALL, "still(stamps, *tensors) -> whether these are the stamped tensors, unchanged"},
+    {"layer_forward", fast_call<layer_forward>(), METH_FASTCALL,
      "layer_forward(plan, x, cos, sin, ring_k, ring_v, layer, past) -> tensor, an int (native status), or None (not the ordinary case)"},
     {nullptr, nullptr, 0, nullptr}};
 

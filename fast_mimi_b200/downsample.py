@@ -18,9 +18,12 @@ import torch
 import torch.nn as nn
 
 from . import ops
+from ._origin import Origin
 
 
 class MimiDownsampleB200(nn.Module):
+    _parts_from = Origin()                      # what the weight's hi + lo parts were made from
+
     def __init__(self, conv: nn.Module) -> None:
         """``conv``: a module with the reference's ``MimiConv1d`` attributes (``conv`` = ``nn.Conv1d``, ``causal``,
         ``pad_mode``); its weight is shared, not copied."""
@@ -33,15 +36,13 @@ class MimiDownsampleB200(nn.Module):
         self.conv = inner
         self.kernel, self.stride = inner.kernel_size[0], inner.stride[0]
         self._parts = None
-        self._key = None
 
     def _weight_parts(self):
         w = self.conv.weight
-        key = (w.data_ptr(), w._version, w.device)
-        if self._parts is None or self._key != key:
+        if self._parts is None or not self._parts_from.still(w):
             # W2[c_out, j * C + c_in] = W[c_out, c_in, j]: the row layout of ops.downsample_conv
             w2 = w.detach().float().permute(0, 2, 1).reshape(w.shape[0], -1).contiguous()
-            self._parts, self._key = ops.split_half(w2), key
+            self._parts, self._parts_from = ops.split_half(w2), Origin(w)
         return self._parts
 
     def frames(self, x: torch.Tensor) -> torch.Tensor:

@@ -25,6 +25,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import _native, ops
+from ._origin import Origin
 from .attention import MimiAttentionB200
 from .kv_ring import MimiKVRing
 
@@ -58,11 +59,13 @@ class _Cast16:
     def __init__(self) -> None:
         self._store: dict = {}
 
+    def __setstate__(self, state) -> None:
+        self._store = {}                        # a copied or unpickled module makes its own
+
     def get(self, name: str, p: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
-        key = (p.data_ptr(), p._version, p.device, dtype)
         hit = self._store.get(name)
-        if hit is None or hit[0] != key:
-            hit = (key, p.detach().to(dtype).contiguous())
+        if hit is None or hit[1].dtype != dtype or not hit[0].still(p):
+            hit = (Origin(p), p.detach().to(dtype).contiguous())
             self._store[name] = hit
         return hit[1]
 

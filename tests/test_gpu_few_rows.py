@@ -169,6 +169,30 @@ def test_layer_follows_its_parameters():
     assert not torch.equal(run(), before)
 
 
+def test_layer_follows_an_assigned_data():
+    """Two assignments of ``.data`` in a row give a parameter the memory of its first storage again.  The new values have the
+    size of the old ones (larger q and LayerNorm weights sharpen the softmax and magnify the rounding of its scores), so the bar
+    is that of the layer's other tests."""
+    import fast_mimi_b200 as fm
+    p = _layer_params(8)
+    layer = fm.MimiTransformerLayerB200().cuda()
+    layer.load_state_dict(p)
+    x = torch.randn(1, 20, 512)
+    cs = fm.rope_tables(torch.arange(20, device="cuda")[None])
+    layer(x.cuda(), None, None, cs)
+    came_back = 0
+    for name in ("mlp.fc1.weight", "mlp.fc2.weight", "self_attn.q_proj.weight", "self_attn.o_proj.weight", "input_layernorm.weight"):
+        w = layer.get_parameter(name)
+        at, a, b = w.data_ptr(), p[name] * 0.5, -p[name]
+        w.data = a.cuda()
+        w.data = b.cuda()
+        came_back += w.data_ptr() == at
+        p[name] = b
+        got, _ = layer(x.cuda(), None, None, cs)
+        assert O.rel_l2(got.cpu() - x, O.transformer_layer(x, p) - x) < 2e-3, name
+    assert came_back > 0           # else the allocator has changed and this shows nothing
+
+
 @pytest.mark.parametrize("streams", [38, 64, 333, 700])
 def test_many_streams_repeat_exactly(streams):
     """More (stream, head) items than two per SM: three ring slices are in flight per block and its two groups of warps take

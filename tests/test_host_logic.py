@@ -171,3 +171,33 @@ def test_rope_tables_match_the_oracle():
         oc, os_ = O.rope_tables(pos[b])
         assert torch.equal(cos[b], oc) and torch.equal(sin[b], os_)
     assert torch.equal(cos[..., :32], cos[..., 32:])
+
+
+def test_kept_copies_follow_an_assigned_data():
+    """A 16-bit copy of a weight is made anew when ``.data`` is assigned, also where the parameter comes back to an address it had
+    (adapters merged one after the other do that) or lies in the same memory another way round, and when a module is copied."""
+    import copy
+    import pickle
+    import numpy as np
+    import fast_mimi_b200 as fm
+    layer = fm.MimiTransformerLayerB200()
+    reads = {"o_proj": lambda l: (l.self_attn.o_proj.weight, l.self_attn.out_weight(torch.float16)),
+             "q_proj": lambda l: (l.self_attn.q_proj.weight, l.self_attn.packed_qkv_weight(torch.float16)[:512]),
+             "fc1": lambda l: (l.mlp.fc1.weight, l._cast.get("fc1", l.mlp.fc1.weight, torch.float16))}
+    for read in reads.values():
+        w, made = read(layer)
+        assert torch.equal(made, w.half()) and read(layer)[1].data_ptr() == made.data_ptr()
+        memory = np.zeros(tuple(w.shape), dtype=np.float32)
+        for value in (1.0, 2.0, 3.0):
+            memory[:, 0] = value
+            w.data = torch.from_numpy(memory)                # a storage of its own at the same address
+            assert torch.equal(read(layer)[1], w.half()), value
+            if w.shape[0] == w.shape[1]:
+                w.data = w.data.t()
+                assert torch.equal(read(layer)[1], w.half()), value
+    for other in (copy.deepcopy(layer), pickle.loads(pickle.dumps(layer))):
+        with torch.no_grad():
+            for w in (other.self_attn.o_proj.weight, other.self_attn.q_proj.weight, other.mlp.fc1.weight):
+                w.data = w.data + 1.0
+        for read in reads.values():
+            assert torch.equal(read(other)[1], read(other)[0].half())
