@@ -17,8 +17,8 @@
 // eight frames costs the ring's bytes once.  Keys and dimensions are the 16 rows of a product and the eight queries its
 // columns: with the queries as rows half of every product was padding, and the chain of products (8 cycles each, 21 when
 // one waits for the one before) was what a warp spent its time on (1024 streams, eight layers: 1082 us against 964).
-// Probabilities stay FP32-grade: they enter P V as the sum of two 16-bit parts.  (tcgen05 would need 128 rows
-// and tensor-memory round trips for at most 8 queries.)
+// Probabilities keep the bits of FP32: they enter P V as sums of 16-bit parts.  (tcgen05 would need 128 rows and
+// tensor-memory round trips for at most 8 queries.)
 //
 // Rows that are already in the ring do not depend on the projection, so in a chain of dependent launches the first items
 // are requested before the wait for it.  A block has an item's ring rows in shared memory before it stores that item's
@@ -57,12 +57,22 @@ constexpr int smem_bytes(int stages) {
 }
 static_assert(smem_bytes(kMaxStages) <= 232448, "exceeds the 227 KB a block may use");
 
-// x, y as hi + lo, both parts of type T
+// Probabilities as operands of type T without losing bits of FP32: as a sum of kParts values.  BF16 has eight significant bits
+// and the range of FP32: three parts are all 24.  FP16 has eleven, and a sign on the second part makes two of them 24 to within
+// the last bit, but nothing below 2^-24: probabilities carry a factor of 2^kShift, the sum they are divided by likewise.  (As two
+// parts each and unscaled, an FP16 result carried by probabilities of 2^-20 was off by up to 4e-3, one of BF16 by 2^-17 of its terms.)
+template <typename T> struct Parts { static constexpr int kParts = 3; static constexpr float kShift = 0.f; };
+template <> struct Parts<__half> { static constexpr int kParts = 2; static constexpr float kShift = 15.f; };
+
 template <typename T>
-__device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& lo) {
-  hi = Pack16<T>::pack(x, y);
-  const float2 b = Pack16<T>::unpack(hi);
-  lo = Pack16<T>::pack(x - b.x, y - b.y);
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t (&part)[Parts<T>::kParts]) {
+#pragma unroll
+  for (int i = 0; i < Parts<T>::kParts; ++i) {
+    part[i] = Pack16<T>::pack(x, y);
+    const float2 b = Pack16<T>::unpack(part[i]);
+    x -= b.x;
+    y -= b.y;
+  }
 }
 }  // namespace stream
 
@@ -266,7 +276,7 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
       for (int e = 0; e < 2; ++e) {
 #pragma unroll
         for (int x = 4; x < 32; x <<= 1) m[e] = fmaxf(m[e], __shfl_xor_sync(0xffffffffu, m[e], x));
-        m_use[e] = m[e] == -INFINITY ? 0.f : m[e];
+        m_use[e] = m[e] == -INFINITY ? 0.f : m[e] - Parts<VT>::kShift;
       }
 #pragma unroll
       for (int mt = 0; mt < 5; ++mt) {
@@ -290,20 +300,24 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
 #pragma unroll
       for (int mt = 0; mt < 5; ++mt) {
         if (in_use(mt)) {
-          uint32_t h0, l0, h1, l1;
-          split_pair<VT>(sc[mt][0], sc[mt][1], h0, l0);
-          split_pair<VT>(sc[mt][2], sc[mt][3], h1, l1);
-          h0 = movmatrix_trans(h0); h1 = movmatrix_trans(h1);
-          l0 = movmatrix_trans(l0); l1 = movmatrix_trans(l1);
+          uint32_t p0[Parts<VT>::kParts], p1[Parts<VT>::kParts];
+          split_pair<VT>(sc[mt][0], sc[mt][1], p0);
+          split_pair<VT>(sc[mt][2], sc[mt][3], p1);
+#pragma unroll
+          for (int i = 0; i < Parts<VT>::kParts; ++i) {
+            p0[i] = movmatrix_trans(p0[i]);
+            p1[i] = movmatrix_trans(p1[i]);
+          }
           const uint32_t base = smem_u32(mt < 4 ? tile_v : new_v);
           const int key = (mt < 4 ? slot0 + mt * 16 : 0) + (lane & 7) + ((lane >> 4) << 3);
           uint32_t va[4][4];
 #pragma unroll
           for (int d = 0; d < 4; ++d) ldmatrix4_trans(va[d], base + sw128_offset(key, 2 * d + ((lane >> 3) & 1)));
 #pragma unroll
-          for (int d = 0; d < 4; ++d) mma_16x8x16<VT>(o[d], va[d], h0, h1);
+          for (int i = 0; i < Parts<VT>::kParts; ++i) {
 #pragma unroll
-          for (int d = 0; d < 4; ++d) mma_16x8x16<VT>(o[d], va[d], l0, l1);
+            for (int d = 0; d < 4; ++d) mma_16x8x16<VT>(o[d], va[d], p0[i], p1[i]);
+          }
         }
       }
       __syncwarp();

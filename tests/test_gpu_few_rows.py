@@ -108,6 +108,50 @@ def test_slots_outside_the_window_do_not_show(slots, past, T):
     fm.check_status()
 
 
+@pytest.mark.parametrize("value_dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T", [1, 8])
+def test_streaming_probabilities_keep_the_bits_of_fp32(value_dtype, T):
+    """A layer whose output is the attention core of a chosen query over a chosen ring.  FP16 values: all that counts comes
+    from probabilities of about 2^-20 beside one of 1 whose value is 0.  BF16 values: +1 and -1 in turn, under probabilities that
+    differ by 2^-12 of themselves.  Bar: the result's own rounding; FP32 exponentials (2^-22) add 1e-3 of the BF16 result."""
+    import fast_mimi_b200 as fm
+    layer = fm.MimiTransformerLayerB200(value_dtype=value_dtype).cuda()
+    q, k, v = torch.zeros(8, 64), torch.zeros(8, 250, 64), torch.zeros(8, 250, 64)
+    q[:, 0], q[:, 1] = 8.0, 2.0 ** -3                         # logits k_0 + 2^-6 k_1
+    with torch.no_grad():
+        for p in layer.parameters():
+            p.zero_()
+        layer.input_layernorm.bias[0] = 1.0
+        layer.self_attn.q_proj.weight[:, 0] = q.reshape(-1)
+        layer.self_attn.o_proj.weight.copy_(torch.eye(512))
+        layer.self_attn_layer_scale.scale.fill_(1.0)
+    past = 300
+    at = torch.arange(past - 249, past) % 250                 # oldest first; a call of T frames leaves the oldest out one by one
+    if value_dtype == torch.float16:
+        k[:, at, 0] = (torch.arange(8) / 16)[:, None]
+        k[:, at[-1], 0] = 14.0
+        v[:, at[:-1]] = 1.0
+    else:
+        k[:, at, 0] = -torch.tensor([1.0, 1.125, 1.25, 1.5] * 2)[:, None]
+        k[:, at[-1], 0] = 0.0
+        k[:, at[1:-1:2], 1] = -(2.0 ** -6)
+        v[:, at[:-1:2]], v[:, at[1:-1:2]] = 1.0, -1.0
+    ring = fm.MimiKVRing(1, 1, 250, value_dtype=value_dtype)
+    ring.ring_k[0, 0], ring.ring_v[0, 0] = k.cuda(), v.cuda()
+    assert torch.equal(ring.ring_k[0, 0].float().cpu(), k)
+    ring.advance(0, past)
+    one = torch.ones(1, T, 64, device="cuda")
+    got = layer(torch.zeros(1, T, 512, device="cuda"), None, ring, (one, one * 0))[0].cpu().view(T, 8, 64)
+    new = torch.zeros(8, T, 64)
+    kk, vv = torch.cat((k[:, at], new), dim=1).double(), torch.cat((v[:, at], new), dim=1).double()
+    for t in range(T):
+        s = torch.einsum("hd,hnd->hn", q.double(), kk[:, t:t + 250]) * 0.125
+        want = torch.einsum("hn,hnd->hd", torch.softmax(s, dim=-1), vv[:, t:t + 250])
+        if value_dtype == torch.float16 or t % 2 == 0:        # else one sign is in the majority, nothing cancels
+            assert O.rel_l2(got[t], want) < ROUND[value_dtype], t
+    fm.check_status()
+
+
 def test_layer_follows_its_ring():
     """A session whose ring goes through pickle, then gets new storage, half way: outputs and rings are those of a session
     left alone."""
