@@ -43,6 +43,10 @@ int encode_tiled(CUtensorMap* map, CUtensorMapDataType dtype, uint32_t rank, voi
                  CUtensorMapSwizzle swizzle);
 // [rows, cols] row-major 16-bit matrix, boxes of box_rows x box_cols, 128-byte swizzle.
 int encode_rows_16bit(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols);
+// The projection kernels read the rotary tables four values at a time.
+inline bool rope_tables_aligned(const float* cos, const float* sin, long long bstride) {
+  return ((reinterpret_cast<uintptr_t>(cos) | reinterpret_cast<uintptr_t>(sin) | static_cast<uintptr_t>(bstride) * sizeof(float)) & 15u) == 0;
+}
 // Multiprocessors of the current device.
 int sm_count();
 // Opt a kernel into `bytes` of dynamic shared memory once per (kernel, device).

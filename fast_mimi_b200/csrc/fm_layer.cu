@@ -56,6 +56,7 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
   const long long rows_ll = static_cast<long long>(B) * T;
   if (B < 0 || T < 0 || rows_ll > 0x7fffffffLL || p.window <= 0 || p.ffn <= 0 || p.ffn % 256 != 0) return -1;
   if (rows_ll == 0) return 0;
+  if (!rope_tables_aligned(cos, sin, cos_bstride)) return -3;
   const bool cached = ring_k != nullptr;
   if (cached && (ring_v == nullptr || past < 0 || slots < p.window)) return -1;
   const int rows = static_cast<int>(rows_ll);

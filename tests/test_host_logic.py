@@ -201,3 +201,22 @@ def test_kept_copies_follow_an_assigned_data():
                 w.data = w.data + 1.0
         for read in reads.values():
             assert torch.equal(read(other)[1], read(other)[0].half())
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="made-up addresses: only where nothing can be launched")
+@pytest.mark.parametrize("offset", [4, 8])
+@pytest.mark.parametrize("rows", [1, 40, 5000])
+def test_misaligned_rotary_tables_are_refused(rows, offset):
+    """The projections read the tables 16 bytes at a time: a table that starts between such addresses is an error of the call
+    (-3) on every path, before anything is launched.  The addresses are made up; nothing looks behind them."""
+    import ctypes
+    from fast_mimi_b200 import _native
+    lib = _native.load()
+    a, n = 1 << 20, None
+    params = _native.LayerParams(*[a] * 10, 1e-5, 1e-5, 0.125, 250, 2, 1, 2048, 0, 2)
+    for cos, sin in ((a + offset, a), (a, a + offset)):
+        assert lib.fm_qkv_rope_bf16(a, a, cos, sin, 0, a, a, a, 1, rows, 1, n, n) == -3
+        assert lib.fm_layer_forward(ctypes.byref(params), a, a, a, 1 << 40, cos, sin, 0, 1, rows, n, n, 0, 0, n, n) == -3
+        assert lib.fm_attention_prefill_bf16(a, a, cos, sin, 0, a, a, a, a, 1, rows, 250, 0.125, 1, n, n) == -3
+        assert lib.fm_attention_chunk_bf16(a, a, cos, sin, 0, a, a, a, a, a, a, a, a, 1, rows, 300, 250, 250, 0.125, 1, n, n) == -3
+        assert lib.fm_decode_step_bf16(a, a, cos, sin, 0, n, 300, a, a, a, a, 1, 250, 0.125, 1, n, n) == -3
