@@ -71,6 +71,8 @@ class _Cast16:
 
 
 class MimiTransformerLayerB200(nn.Module):
+    _plan = None            # of the class, so that layers pickled before there were plans have none
+
     def __init__(self, hidden_size: int = 512, intermediate_size: int = 2048, num_heads: int = 8, head_dim: int = 64,
                  sliding_window: int = 250, layer_idx: int = 0, norm_eps: float = 1e-5,
                  layer_scale_initial_scale: float = 0.01, value_dtype: torch.dtype = torch.float16) -> None:
@@ -82,7 +84,6 @@ class MimiTransformerLayerB200(nn.Module):
         self.self_attn_layer_scale = _LayerScale(hidden_size, layer_scale_initial_scale)
         self.mlp_layer_scale = _LayerScale(hidden_size, layer_scale_initial_scale)
         self._cast = _Cast16()
-        self._plan = None
 
     @classmethod
     def from_reference(cls, layer: nn.Module, value_dtype: torch.dtype = torch.float16) -> "MimiTransformerLayerB200":

@@ -96,12 +96,13 @@ class MimiRVQB200:
 
 
 class MimiSplitRVQB200:
+    _joint_in: tuple | None = None          # of the class, so that quantisers pickled before there were joint projections
+    _joint: tuple | None = None             # make theirs on the first call
+
     def __init__(self, semantic: MimiRVQB200, acoustic: MimiRVQB200) -> None:
         self.semantic, self.acoustic = semantic, acoustic
         self.num_semantic_quantizers = semantic.books.layers
         self.max_num_quantizers = semantic.books.layers + acoustic.books.layers
-        self._joint_in: tuple | None = None
-        self._joint: tuple | None = None
         self._joint_in_parts()
         self._joint_out_parts()
 

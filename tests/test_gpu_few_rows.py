@@ -330,3 +330,27 @@ def test_layer_reads_its_vectors_where_they_lie(dtype, rows):
         layer.input_layernorm.weight.data.mul_(0.5)
         check()
     fm.check_status()
+
+
+def test_objects_without_what_is_kept_between_calls():
+    """Layers, rings and quantisers that were pickled before they kept anything between calls lack those attributes."""
+    import fast_mimi_b200 as fm
+
+    def stripped(made, names):
+        old = type(made).__new__(type(made))
+        old.__dict__.update({k: v for k, v in made.__dict__.items() if k not in names})
+        return old
+
+    layer, ring = fm.MimiTransformerLayerB200().cuda(), fm.MimiKVRing(1, 1, 250)
+    old, old_ring = stripped(layer, {"_plan"}), stripped(fm.MimiKVRing(1, 1, 250), {"_rings"})
+    old.self_attn = stripped(layer.self_attn, {"_packed_from", "_wo16_from", "_packed", "_wo16"})
+    old.self_attn._packed = old.self_attn._wo16 = None
+    x, cs = torch.randn(1, 20, 512, device="cuda"), fm.rope_tables(torch.arange(20, device="cuda")[None])
+    assert torch.equal(old(x, None, old_ring, cs)[0], layer(x, None, ring, cs)[0])
+    branch = lambda: fm.MimiRVQB200(torch.randn(1, 2048, 256, device="cuda"), torch.randn(256, 512, 1, device="cuda"),
+                                    torch.randn(512, 256, 1, device="cuda"))
+    split = fm.MimiSplitRVQB200(branch(), branch())
+    old = stripped(split, {"_joint", "_joint_in"})
+    e = torch.randn(1, 512, 5, device="cuda")
+    codes = split.encode(e)
+    assert torch.equal(old.encode(e), codes) and torch.equal(old.decode(codes), split.decode(codes))
