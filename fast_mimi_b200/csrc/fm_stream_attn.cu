@@ -370,7 +370,8 @@ int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k
                        cudaStream_t st, int dependent) {
   using namespace stream;
   if (S <= 0 || T <= 0) return (S == 0 || T == 0) ? 0 : -1;
-  if (past < 0 || window <= 0 || slots < window || slots > 256 || T > kMaxT || S > (1 << 19)) return -1;
+  if (past < 0 || window <= 0 || slots < window || slots > 256 || T > kMaxT) return -1;
+  if (static_cast<long long>(S) * 8 * slots > 0x7fffffffLL) return -1;      // a ring row is a coordinate of the tensor maps
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
        reinterpret_cast<uintptr_t>(ring_k) | reinterpret_cast<uintptr_t>(ring_v) | reinterpret_cast<uintptr_t>(out)) & 15u)
     return -3;

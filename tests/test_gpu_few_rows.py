@@ -274,6 +274,20 @@ def test_many_streams_repeat_exactly(streams):
     fm.check_status()
 
 
+def test_layer_on_half_a_million_streams():
+    """A ring's size, not the number of streams, is what the streaming kernel is limited by.  Bar as above: K in other splits."""
+    import fast_mimi_b200 as fm
+    streams, some = (1 << 19) + 1, [0, 1, 1 << 19]
+    layer = fm.MimiTransformerLayerB200(sliding_window=2).cuda()
+    ring, few = fm.MimiKVRing(1, streams, 2), fm.MimiKVRing(1, len(some), 2)
+    for past in range(3):
+        x = torch.randn(streams, 1, 512, device="cuda")
+        cs = fm.rope_tables(torch.tensor([[past]], device="cuda"))
+        a, b = layer(x, None, ring, cs)[0][some], layer(x[some], None, few, cs)[0]
+        assert O.rel_l2(a - x[some], b - x[some]) < 1e-3
+    fm.check_status()
+
+
 def test_layer_with_parameters_that_cannot_be_watched():
     """LayerNorm parameters made in inference mode have no version counter: the call works without a plan."""
     import fast_mimi_b200 as fm
