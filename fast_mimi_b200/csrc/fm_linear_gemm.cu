@@ -503,6 +503,20 @@ static int launch_pairs(const void* a, const void* w, const SplitLow* low, void*
                        args, total_units, idesc, status);
 }
 
+// 256 x 128 units instead of 256 x 256 where they save part of a wave in a call whose rows cross the slab (a residual, a
+// split-precision product): there a half unit costs about half plus 1 / 128 per K chunk of a whole one (its a slices are fetched
+// twice as often).  Without the slab it costs two thirds to three quarters, and no wave that it saves is worth that.  (What one
+// wave of half units would hold, the few-row tiles take.)  Measured, whole -> half units, in us:
+//   residual         K =  512, N =  512, 12000 rows (2 -> 3 waves) 18.8 -> 16.7, 22000 rows (3 -> 5) 31.8 -> 29.1
+//                    K = 1024, N = 1024, FP16, 5000 rows (2 -> 3) 27.2 -> 24.2, 16000 rows (4 -> 7) 38.7 -> 42.9
+//                    K = 2048, N =  512, 14000 rows (2 -> 3) 35.2 -> 36.7, 22000 rows (3 -> 5) 49.9 -> 56.2
+//   split precision  K =  256, N =  512, 12000 rows (2 -> 3) 29.3 -> 25.0;  K = 512, 33.2 -> 37.1;  K = 2048, 84.4 -> 113.1
+//   neither          K =  512, N =  512, 12000 rows (2 -> 3) 12.6 -> 14.6;  K = 1024, N = 1024, 16000 rows (4 -> 7) 29.0 -> 37.2
+static bool half_units(int pair_tiles, int N, int max_pairs, int k_chunks) {
+  const int waves256 = (pair_tiles * (N / 256) + max_pairs - 1) / max_pairs, waves128 = (pair_tiles * (N / 128) + max_pairs - 1) / max_pairs;
+  return static_cast<long long>(64 + k_chunks) * waves128 < 128ll * waves256;
+}
+
 int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N,
                        int K, int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent) {
   using namespace lin;
@@ -516,14 +530,11 @@ int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, co
     return -3;
   if (out_dtype != 3 && few_row_tiles(M, N))
     return launch_linear_small(a, w, y, scale, resid, M, N, K, in_dtype, out_dtype, gelu, status, st, dependent);
-  // 256 x 256 units, or 256 x 128 where those fill the pairs better: a unit of half the width costs a little more than
-  // half the time (its a slices are fetched twice as often), so the narrow form has to save a quarter of a wave.
   const int pair_tiles = ((M + kBlockM - 1) / kBlockM + 1) / 2;
   const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
   // The wide shape where the epilogue carries arithmetic (GELU, candidate records), the narrow one otherwise.
   const bool wide = gelu || out_dtype == 3;
-  const int waves256 = (pair_tiles * (N / 256) + max_pairs - 1) / max_pairs, waves128 = (pair_tiles * (N / 128) + max_pairs - 1) / max_pairs;
-  const bool halves = !wide && 9 * waves128 < 16 * waves256;
+  const bool halves = !wide && resid != nullptr && half_units(pair_tiles, N, max_pairs, K / kBlockK);
   LinearArgs args = {scale, resid, M, N, K, gelu ? 1 : 0, out_dtype == 3 ? static_cast<uint4*>(y) : nullptr, y, {}};
   using Fn = int (*)(const void*, const void*, const SplitLow*, void*, const LinearArgs&, int, int, int, int, int*, cudaStream_t, int);
   Fn fn;
@@ -557,9 +568,8 @@ int launch_linear_split(const void* a_hi, const void* a_lo, long long a_rows, in
   if (few_row_tiles(M, N)) return launch_linear_split_small(a_hi, w_hi, low, map, y, M, N, K, status, st);
   const int pair_tiles = ((M + kBlockM - 1) / kBlockM + 1) / 2;
   const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
-  const int waves256 = (pair_tiles * (N / 256) + max_pairs - 1) / max_pairs, waves128 = (pair_tiles * (N / 128) + max_pairs - 1) / max_pairs;
   const LinearArgs args = {ParamVec(nullptr), nullptr, M, N, K, 0, nullptr, y, map};
-  auto fn = 9 * waves128 < 16 * waves256 ? launch_pairs<4, false, 128> : launch_pairs<4, false, 256>;      // as above
+  auto fn = half_units(pair_tiles, N, max_pairs, 3 * (K / kBlockK)) ? launch_pairs<4, false, 128> : launch_pairs<4, false, 256>;
   return fn(a_hi, w_hi, &low, y, args, pair_tiles, max_pairs, 1, 4, status, st, 0);
 }
 

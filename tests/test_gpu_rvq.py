@@ -193,8 +193,8 @@ def test_search_repeats_exactly(rows):
     fm.check_status()
 
 
-# one block per tile of K slices, two, both parts in one block (few rows), pairs of blocks with 128- and 256-wide units
-@pytest.mark.parametrize("rows", [13, 200, 750, 1300, 4000, 6000, 20000])
+# one block per tile of K slices, two, both parts in one block (few rows), pairs of blocks; 12000: 128-wide units for a branch
+@pytest.mark.parametrize("rows", [13, 200, 750, 1300, 4000, 6000, 12000, 20000])
 def test_joint_decode_is_as_precise_as_the_branches(rows):
     """Both output projections in one product: its distance from 64 bits is that of two products, each in one accumulator (as
     calls of many rows have it), and their FP32 sum.  Bar: 5 % for the FP32 sums of K slices."""
