@@ -193,6 +193,35 @@ def test_search_repeats_exactly(rows):
     fm.check_status()
 
 
+@pytest.mark.parametrize("rows", [1, 70, 5000])
+def test_search_one_layer_at_a_time(rows):
+    """The calls a host that drives the layers itself makes (margins, candidate records, decision) give the codes of the whole
+    search, and leave the residual and the margins of the layer behind the last one."""
+    import fast_mimi_b200 as fm
+    from fast_mimi_b200 import _native
+    layers, entries = 4, 512
+    books = fm.ops.RVQCodebooks(torch.randn(layers, entries, 256, generator=torch.Generator().manual_seed(2)).cuda())
+    x = torch.randn(rows, 256, generator=torch.Generator().manual_seed(rows)).cuda() * 2
+    want, n_want = fm.ops.rvq_encode(x, books, return_candidates=True)
+    lib, st, stream = _native.load(), fm.ops.new_status("cuda"), torch.cuda.current_stream().cuda_stream
+    resid, resid16, tau = x.clone(), torch.empty(rows, 256, dtype=torch.float16, device="cuda"), torch.empty(rows, device="cuda")
+    records = torch.empty(rows, entries // 64, 4, dtype=torch.int32, device="cuda")
+    codes, n_cand = torch.empty_like(want), torch.empty_like(n_want)
+    tau_rel = fm.ops.RVQ_TAU_REL[torch.float32]
+    run = lambda name, *args: _native.check(getattr(lib, name)(*(a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args), stream), name)
+    run("fm_rvq_prepare_f32", resid, resid16, tau, rows, books.e_max[0], tau_rel)
+    for l in range(layers):
+        run("fm_rvq_candidates_f16", resid16, books.half[l], books.sq[l], tau, records, rows, entries, st)
+        run("fm_rvq_select_rec_f32", records, books.vectors[l], resid, resid16, codes[l], n_cand[l], tau, rows, entries,
+            books.e_max[min(l + 1, layers - 1)], tau_rel, st)
+    assert torch.equal(codes, want) and torch.equal(n_cand, n_want)
+    left = x
+    for l in range(layers):
+        left = left - books.vectors[l][want[l]]
+    assert torch.equal(resid, left) and torch.equal(resid16, left.half())
+    assert fm.ops.read_status(st) == 0
+
+
 # one block per tile of K slices, two, both parts in one block (few rows), pairs of blocks; 12000: 128-wide units for a branch
 @pytest.mark.parametrize("rows", [13, 200, 750, 1300, 4000, 6000, 12000, 20000])
 def test_joint_decode_is_as_precise_as_the_branches(rows):
