@@ -633,7 +633,8 @@ def profile_case(which: str) -> None:
     a handful of launches): prefill = 256 clips x 250 frames, one layer; decode = 512 streams on a
     full ring, one layer; layer = one whole transformer layer on 256 clips x 250 frames (LayerNorm and the
     three epilogue variants of the linear kernel); longclip = 16 clips x 2500 frames, three input sets in
-    rotation; rvq = 64 000 vectors through two quantiser layers.  Prints nothing that is a benchmark value."""
+    rotation; rvq = 64 000 vectors through two quantiser layers; few = one layer on a clip of 125 frames, on five streams by 50
+    frames and on 1024 streams by one, and banded attention on FP32 q, k, v of 16 clips x 2500 frames.  Prints nothing that is a benchmark value."""
     import fast_mimi_b200 as fm
     from fast_mimi_b200 import ops
     dev = torch.device("cuda", 0)
@@ -669,6 +670,22 @@ def profile_case(which: str) -> None:
         with torch.no_grad():
             for _ in range(3):
                 layer(x, None, None, (cos, sin), False)
+    elif which == "few":
+        layer = fm.MimiTransformerLayerB200().to(dev)
+        with torch.no_grad():
+            for streams, frames, past in ((1, 125, None), (5, 50, 400), (1024, 1, 400)):
+                ring = None if past is None else fm.MimiKVRing(1, streams, WINDOW, device=dev)
+                if ring is not None:
+                    ring.ring_k.normal_(generator=g)
+                    ring.ring_v.normal_(generator=g)
+                    ring.advance(0, past)
+                x = torch.randn(streams, frames, HIDDEN, device=dev, generator=g)
+                cos = torch.ones(1, frames, 64, device=dev); sin = torch.zeros(1, frames, 64, device=dev)
+                for _ in range(3):
+                    layer(x, None, ring, (cos, sin), False)
+            qkv = [torch.randn(16, 2500, 8, 64, device=dev, generator=g).transpose(1, 2) / 8 for _ in range(3)]
+            for _ in range(3):
+                fm.native_window_attention(*qkv, scale=0.125, window=WINDOW)
     elif which == "rvq":
         books = ops.RVQCodebooks(torch.randn(2, 2048, 256, device=dev, generator=g))
         xq = torch.randn(64000, 256, device=dev, generator=g) * 1.5
@@ -969,7 +986,7 @@ def main() -> None:
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--no-decode", action="store_true", help="skip the streaming-decode measurement")
     ap.add_argument("--no-cpu", action="store_true", help="skip the CPU oracle baseline")
-    ap.add_argument("--profile-case", choices=["prefill", "fused", "chunk", "decode", "layer", "longclip", "rvq"],
+    ap.add_argument("--profile-case", choices=["prefill", "fused", "chunk", "decode", "layer", "longclip", "rvq", "few"],
                     help="run a small case for ncu and exit")
     ap.add_argument("--workload", default="prefill", choices=["prefill", "longclip", "stream", "streamlayer", "stack", "rvq"],
                     help="prefill = headline (config 3); longclip / stream = configs 4 / 5, stack = whole transformer layers, rvq = the quantiser after the encoder transformer; one extra JSON line each")

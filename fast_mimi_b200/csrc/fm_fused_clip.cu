@@ -518,8 +518,11 @@ attn_fused_clip_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
 }
 
 // One pair of CTAs owns a clip at a time, so the one-kernel form takes 36 us (+ 5) per wave of clips however full the wave
-// is; projection kernel + attention kernel take 0.53 us per clip of 250 frames (+ 8.4).  Measured at T = 250: 1 clip 40 us
-// against 16, 64 clips 43 / 43, 90 clips 77 / 56, 148 clips 78 / 87, 180 clips 112 / 104, 512 clips 249 / 268.
+// is and, as both 128-frame tiles are always computed, whatever T; projection kernel + attention kernel take 0.53 us per clip
+// of 250 frames (+ 8.4), about in proportion to T.  Measured, one kernel / two, in us: T = 250: 1 clip 40 / 17, 64 clips 46 / 45,
+// 90 clips 79 / 59, 148 clips 79 / 85, 180 clips 113 / 104, 222 clips 115 / 124, 512 clips 256-265 / 278; T = 200: 64 clips
+// 46 / 44, 148 clips 78 / 77, 222 clips 111 / 108, 512 clips 247 / 239; T = 140: 64 clips 42 / 36, 512 clips 243 / 192.  (At
+// T = 140 the two kernels take up to a third longer than in proportion, which moves no decision.)
 bool use_fused_clip(int B, int T) {
   const int pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1, waves = (B + pairs - 1) / pairs;
   return 36.0 * waves + 5.0 <= 0.00212 * static_cast<double>(B) * T + 8.4;

@@ -197,10 +197,9 @@ int launch_ring_linearize(const void* ring_k, const void* ring_v, const void* k_
 int launch_ring_append(const void* k_new, const void* v_new, void* ring_k, void* ring_v, int S, int T, int past,
                        int slots, cudaStream_t st, int dependent = 0);
 // T <= 8 new frames per stream over its ring (at most 256 slots), ring update included (fm_stream_attn.cu).
-// out_dtype: 2 = FP32, anything else = the value type.
 int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k, void* ring_v, void* out, int S, int T,
-                       int past, int slots, int window, float scale, int value_is_fp16, int out_dtype, int* status,
-                       cudaStream_t st, int dependent = 0);
+                       int past, int slots, int window, float scale, int value_is_fp16, int* status, cudaStream_t st,
+                       int dependent = 0);
 // Attention for few query tiles (fm_few_attn.cu): at most two 64-query blocks per SM.  ring_k null: clips; else T new frames
 // per stream on top of the ring, which the kernel also updates where one block has a whole (stream, head).
 bool few_attn_tiles(int S, int T);

@@ -30,7 +30,7 @@ struct Buffers {
   void *h, *q, *k, *v, *core, *x1, *g, *k_lin, *v_lin;
 };
 
-// The workspace of one call.  `delta`: cached rows laid out in front of the new ones (chunks only).
+// The workspace of one call.  `lin_rows`: cached and new rows laid out frame by frame (the linearised path only).
 long long lay_out(uint8_t* base, long long rows, int elem, int ffn, long long lin_rows, Buffers* b) {
   Arena a = {base, 0};
   b->h = a.take(rows * 1024);
@@ -102,8 +102,7 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
     } else if (!cached) {
       rc = launch_band_attn_prefill(b.q, b.k, b.v, b.core, B, T, p.window, p.scale, value_fp16, status, st, 1);
     } else if (few) {
-      rc = launch_stream_attn(b.q, b.k, b.v, ring_k, ring_v, b.core, B, T, past, slots, p.window, p.scale, value_fp16, 0,
-                              status, st, 1);
+      rc = launch_stream_attn(b.q, b.k, b.v, ring_k, ring_v, b.core, B, T, past, slots, p.window, p.scale, value_fp16, status, st, 1);
     } else {
       if (delta > 0) {
         rc = launch_ring_linearize(ring_k, ring_v, b.k, b.v, b.k_lin, b.v_lin, B, T, delta, past, slots, st, 1);

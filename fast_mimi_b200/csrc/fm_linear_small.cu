@@ -3,7 +3,7 @@
 //
 // What bounds such a call is latency and the number of SMs that pull weights out of L2, not arithmetic: the pair
 // kernels (fm_linear_gemm.cu, fm_qkv_gemm.cu) cut the output into 256 x 256 tiles, so that 125 rows x 512 outputs at
-// K = 2048 occupied 4 of 148 SMs, each walking 32 K-chunks one after the other (33 us; here 5 us).  Here a block owns
+// K = 2048 occupied 4 of 148 SMs, each walking 32 K-chunks one after the other (with an FP32 residual 20.8 us; here 6.8 us).  Here a block owns
 // 128 rows x 64 outputs (one attention head; or x 32) and a SLICE of K: the blocks of a thread-block cluster share one output
 // tile and split K between them, so the same layer runs on 64 SMs with four chunks each.  The partial sums meet in
 // distributed shared memory: row r of the tile belongs to cluster rank r % S, every block sends its FP32 partials of an

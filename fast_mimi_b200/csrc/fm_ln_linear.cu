@@ -35,19 +35,6 @@ struct Barriers {
 // The operand tile comes first: the tensor core reads up to 128 - kRows rows past its last chunk, i.e. into the weights.
 constexpr int smem_bytes(int rows) { return 1024 + kChunks * (rows * 128 + kWBytes) + rows * 256 + 64; }
 static_assert(sizeof(Barriers) <= 64, "barrier block too large");
-
-template <int kIn>
-__device__ __forceinline__ void load4(const void* base, long long elem, float (&v)[4]) {
-  if constexpr (kIn == 2) {
-    const float4 f = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(base) + elem));
-    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-  } else {
-    using T16 = typename std::conditional<kIn == 1, __half, __nv_bfloat16>::type;
-    const uint2 u = __ldcg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(base) + elem));
-    const float2 a = Pack16<T16>::unpack(u.x), b = Pack16<T16>::unpack(u.y);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-  }
-}
 }  // namespace lnlin
 
 struct LnArgs {

@@ -79,15 +79,15 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t (&part)[Pa
 struct StreamArgs {
   const uint16_t *q, *k, *v;     // [S, T, 512]
   uint16_t *ring_k, *ring_v;     // [S, 8, slots, 64]
-  void* out;                     // [S, T, 512]
+  uint16_t* out;                 // [S, T, 512]
   int n_items, T, past, delta, slots, window;
   int n_loaded;                  // ring rows per item that the tensor maps' boxes cover: min(past, slots)
   int stages;
   float scale_log2e;
 };
 
-// VT: value type of the ring and v; OT: type of the result
-template <typename VT, typename OT>
+// VT: type of the ring's values, v and the result
+template <typename VT>
 __global__ void __launch_bounds__(stream::kThreads, 1)
 stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                    const __grid_constant__ StreamArgs a, int* status) {
@@ -354,9 +354,7 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         }
         const size_t at = new0 + static_cast<size_t>(t) * 512 + d;
         const float y = num / den;
-        if constexpr (std::is_same<OT, float>::value) static_cast<float*>(a.out)[at] = y;
-        else if constexpr (std::is_same<OT, __half>::value) static_cast<__half*>(a.out)[at] = __float2half_rn(y);
-        else static_cast<__nv_bfloat16*>(a.out)[at] = __float2bfloat16_rn(y);
+        a.out[at] = static_cast<uint16_t>(Pack16<VT>::pack(y, 0.f));
       }
       named_bar_sync(1 + cg, kGroupWarps * 32);          // the merge buffer and the new rows' tiles are free again
     }
@@ -366,7 +364,7 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
 }
 
 int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k, void* ring_v, void* out, int S, int T,
-                       int past, int slots, int window, float scale, int value_is_fp16, int out_dtype, int* status,
+                       int past, int slots, int window, float scale, int value_is_fp16, int* status,
                        cudaStream_t st, int dependent) {
   using namespace stream;
   if (S <= 0 || T <= 0) return (S == 0 || T == 0) ? 0 : -1;
@@ -387,12 +385,9 @@ int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k
   int stages = (n_items + sms - 1) / sms;               // one item per block: one stage, and room for other blocks
   if (stages > kMaxStages) stages = kMaxStages;
   StreamArgs a = {static_cast<const uint16_t*>(q), static_cast<const uint16_t*>(k), static_cast<const uint16_t*>(v),
-                  static_cast<uint16_t*>(ring_k), static_cast<uint16_t*>(ring_v), out, n_items, T, past, delta, slots, window,
+                  static_cast<uint16_t*>(ring_k), static_cast<uint16_t*>(ring_v), static_cast<uint16_t*>(out), n_items, T, past, delta, slots, window,
                   n_loaded, stages, scale * 1.4426950408889634f};
-  using Kern = void (*)(CUtensorMap, CUtensorMap, StreamArgs, int*);
-  Kern kern;
-  if (value_is_fp16) kern = out_dtype == 2 ? stream_attn_kernel<__half, float> : stream_attn_kernel<__half, __half>;
-  else kern = out_dtype == 2 ? stream_attn_kernel<__nv_bfloat16, float> : stream_attn_kernel<__nv_bfloat16, __nv_bfloat16>;
+  auto kern = value_is_fp16 ? stream_attn_kernel<__half> : stream_attn_kernel<__nv_bfloat16>;
   const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes(stages));
   if (rc != 0) return rc;
   return launch_kernel(kern, dim3(n_items < sms ? n_items : sms), kThreads, smem_bytes(stages), st, 1, dependent, tk, tv, a, status);

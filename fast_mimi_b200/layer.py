@@ -13,8 +13,10 @@ chain of dependent launches:
 
 The residual stream keeps the caller's dtype (FP32 stays FP32: both residual adds happen in the FP32 epilogue
 of a GEMM); only the operands of the tensor-core products are rounded to 16 bit.  Calls with a cache (a
-``MimiKVRing``) differ only in the attention core: ring decode for one new frame per stream, the chunk path for
-several; LayerNorms, projections and the MLP are the same kernels.
+``MimiKVRing``) differ only in the attention core: up to eight new frames per stream read and update the ring in one
+kernel, longer chunks of few streams take the kernel for few query tiles (which reads the ring where it lies), all others
+lay ring and new rows out frame by frame for the tiled kernel.  A ring whose values have not the module's type, or a cache
+of another kind, takes the attention module's kernels one by one.
 """
 from __future__ import annotations
 

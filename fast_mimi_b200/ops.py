@@ -292,7 +292,7 @@ def window_attention(q, k, v, *, window=250, scale=0.125, value_dtype=torch.floa
         ws.append(_ptr(keep[-1]))
     fp32 = q.dtype == torch.float32
     out = torch.empty(B, T, H, D, dtype=q.dtype, device=q.device)
-    stored = T > 256 and 129 < window <= 257          # the kernel for long clips stores FP32 itself
+    stored = T > 256 and 129 < window <= 257          # the kernel for long clips stores FP32 itself (the header's rule for out16)
     out16 = None if fp32 and stored else (torch.empty(B, T, H * D, dtype=value_dtype, device=q.device) if fp32 else out)
     rc = _native.load().fm_window_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), code, (ctypes.c_longlong * 9)(*strides), *ws,
                                             _ptr(out16), out.data_ptr() if fp32 else None, B, T, window, scale,
