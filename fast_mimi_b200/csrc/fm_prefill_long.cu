@@ -18,6 +18,13 @@
 // far job 4-w visible 32-key groups and warp w of the diagonal job w+1, so the four SM sub-partitions carry
 // the same load.  Tiles before the clip's first frame are not loaded; their jobs run empty.
 // Warps 0-15: softmax teams.  Warp 16: Q/K loads + score products.  Warp 17: P V products.  Warp 18: V loads.
+//
+// FP32 q, k, v (a model's own, any strides) are converted on the way: quarter tiles of 32 rows arrive by TMA in a staging
+// buffer, three for each of two warps (18 and 19), which round them (q, k to BF16, v to its type) into the tiles' places.  The
+// kernel is bound by its chain of steps, not by memory, so the 12 bytes a value triple costs instead of 6 pass behind it; a
+// converting pass in front (18 bytes a triple at the copy rate) took 51 of 141 us for 16 clips of 2500 frames, 25 clips of 1500
+// frames 132; now 107 and 102.  Two warps are what the register file has room for beside the others; what counts is the little
+// they do besides (a proxy fence, an index division and a walk of its own for every quarter tile: 141 us).
 #include "fm_attn_tile.cuh"
 #include "fm_common.cuh"
 #include "fm_kernels.h"
@@ -38,7 +45,13 @@ constexpr int kThreads = (kSoftmaxWarps + kIssueWarps) * 32;
 constexpr int kTmemCols = 128 * kSlots;
 constexpr uint32_t kPCol = 0, kOCol = 64;           // inside a slot: P over the consumed S, then O
 
+// FP32 inputs: staged quarter tiles of the converting warps
+constexpr int kQuarterRows = 32, kQuarterBytes = kQuarterRows * kD * 4;
+constexpr int kConvertWarps = 2, kStaged = 3;
+constexpr int threads(bool f32_in) { return kThreads + (f32_in ? 32 : 0); }
+
 struct Shared {
+  uint64_t staged[kConvertWarps][kStaged];   // a quarter tile has landed
   uint64_t qk_full[2];     // Q and the new K tile(s) of the step in this Q buffer have landed
   uint64_t v_full[2];      // the new V tile(s) of the step have landed
   uint64_t qk_done[2];     // the step's score products have completed: its Q buffer and its far K tile are dead
@@ -55,9 +68,11 @@ struct Shared {
   float xm[4][kTile][3];   // by step % 4
   float xl[4][kTile][2];
 };
-constexpr int kSmemBytes = 1024 + 2 * kRing * kTileBytes + 2 * kTileBytes + 4 * kSlabBytes +
-                           static_cast<int>((sizeof(Shared) + 127) & ~size_t(127));
-static_assert(kSmemBytes <= 232448, "exceeds the 227 KB a CTA may use");
+__host__ __device__ constexpr int stage_bytes(bool f32_in) { return f32_in ? kConvertWarps * kStaged * kQuarterBytes : 4 * kSlabBytes; }
+constexpr int smem_bytes(bool f32_in) {
+  return 1024 + 2 * kRing * kTileBytes + 2 * kTileBytes + stage_bytes(f32_in) + static_cast<int>((sizeof(Shared) + 127) & ~size_t(127));
+}
+static_assert(smem_bytes(true) <= 232448, "exceeds the 227 KB a CTA may use");
 
 // The steps a CTA takes: an equal share [begin, end) of all (clip, head, query tile) triples in that order, i.e. at most a rest
 // of one sequence, whole ones, and the beginning of another; each of those is a run.  (Whole sequences dealt out in turn: 128
@@ -91,8 +106,9 @@ struct Walk {
 
 // OT: type of the result.  FP32 rows (256 bytes per lane) go straight from registers to memory as whole 32-byte sectors;
 // 16-bit rows through the slabs and a tiled store.
-template <typename VT, typename OT>
-__global__ void __launch_bounds__(longclip::kThreads, 1)
+// kF32In: q, k, v are FP32 (the result too).
+template <typename VT, typename OT, bool kF32In>
+__global__ void __launch_bounds__(longclip::threads(kF32In), 1)
 band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_out,
                       float* __restrict__ out32, int n_steps, int n_tiles, int T, int window, float scale_log2e,
@@ -106,16 +122,16 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   uint8_t* smem_k = smem;                              // kRing tiles
   uint8_t* smem_v = smem_k + kRing * kTileBytes;       // kRing tiles
   uint8_t* smem_q = smem_v + kRing * kTileBytes;       // two tiles
-  uint8_t* smem_stage = smem_q + 2 * kTileBytes;       // four slabs
-  Shared* sh = reinterpret_cast<Shared*>(smem_stage + 4 * kSlabBytes);
+  uint8_t* smem_stage = smem_q + 2 * kTileBytes;       // four slabs, or staged FP32 quarter tiles
+  Shared* sh = reinterpret_cast<Shared*>(smem_stage + stage_bytes(kF32In));
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&sh->qk_full[i], 1);
-      mbar_init(&sh->v_full[i], 1);
+      mbar_init(&sh->qk_full[i], kF32In ? kConvertWarps : 1);
+      mbar_init(&sh->v_full[i], kF32In ? kConvertWarps : 1);
       mbar_init(&sh->qk_done[i], 1);
       mbar_init(&sh->pv_done[i], 1);
     }
@@ -128,6 +144,7 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       mbar_init(&sh->xm_full[i], 12);
       mbar_init(&sh->xl_full[i], 8);
     }
+    for (int i = 0; kF32In && i < kConvertWarps * kStaged; ++i) mbar_init(&sh->staged[i / kStaged][i % kStaged], 1);
     sh->ctl.abort = 0;
     fence_mbar_init();
   }
@@ -157,12 +174,12 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     auto slot_addr = [&](int g) { return tmem_base + static_cast<uint32_t>((g & 3) * kTile); };
     if (role == 0) {
       // ---------------------------------------------------------- Q / K loads + score products
-      if (one) {
+      if (!kF32In && one) {
         tma_prefetch_desc(&tmap_q);
         tma_prefetch_desc(&tmap_k);
       }
       auto load_qk = [&](const Walk& w) {
-        if (!one) return;
+        if (kF32In || !one) return;
         const int b = w.n & 1;
         const int u_lo = w.first() ? w.first_tile_loaded() : w.t;     // K tiles u_lo .. t arrive with this step
         mbar_arrive_expect_tx(&sh->qk_full[b], static_cast<uint32_t>((w.t - u_lo + 2) * kTileBytes));
@@ -240,6 +257,103 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           tc_commit(&sh->o_full[(3 * n) & 3]);
           tc_commit(&sh->pv_done[n & 1]);
         }
+      }
+    } else if (kF32In) {
+      // ---------------------------------------------------------- FP32 tiles into their places (two warps)
+      // A step's tiles in the order of their use: its new K tiles and Q, then its new V tiles; this warp has quarters 2c and
+      // 2c + 1 of each.  Copies run kStaged quarters ahead of the conversion.
+      const int c = role - 2;
+      uint8_t* staging = smem_stage + c * kStaged * kQuarterBytes;
+      // Copies: their own walk, with what a run's tiles have in common worked out once.
+      Walk to_ask(n_steps, n_tiles);
+      int ask_nk = 0, ask_tile = 0, ask_half = 0, ask_head = 0, ask_clip = 0, asked = 0;
+      auto open_step = [&]() {
+        if (to_ask.first()) {
+          ask_head = to_ask.head();
+          ask_clip = to_ask.clip();
+        }
+        ask_nk = to_ask.first() ? to_ask.t - to_ask.first_tile_loaded() + 1 : 1;
+      };
+      open_step();
+      auto ask = [&]() {
+        if (!to_ask.valid()) return;
+        const CUtensorMap* map = ask_tile < ask_nk ? &tmap_k : (ask_tile == ask_nk ? &tmap_q : &tmap_v);
+        const int u = to_ask.t - (ask_tile < ask_nk ? ask_nk - 1 - ask_tile : (ask_tile == ask_nk ? 0 : 2 * ask_nk - ask_tile));
+        if (one) {
+          uint64_t* bar = &sh->staged[c][asked];
+          mbar_arrive_expect_tx(bar, kQuarterBytes);
+          tma_load_4d(staging + asked * kQuarterBytes, map, bar, 0, u * kTile + (2 * c + ask_half) * kQuarterRows, ask_head, ask_clip);
+        }
+        if (++asked == kStaged) asked = 0;
+        if (ask_half == 0) {
+          ask_half = 1;
+          return;
+        }
+        ask_half = 0;
+        if (++ask_tile <= 2 * ask_nk) return;
+        ask_tile = 0;
+        to_ask.next();
+        open_step();
+      };
+      if (one) {
+        tma_prefetch_desc(&tmap_q);
+        tma_prefetch_desc(&tmap_k);
+        tma_prefetch_desc(&tmap_v);
+      }
+      for (int i = 0; i < kStaged; ++i) ask();
+      int slot = 0;
+      uint32_t slot_phase = 0;
+      const uint32_t src_lane = static_cast<uint32_t>((lane >> 3) * (kD * 4) + (lane & 7) * 32);
+      // This warp's half of a tile: eight values a lane and turn, row lane / 8 of four, 16 bytes of the tile's row.
+      auto convert = [&](uint8_t* dst, auto type) {
+        using T16 = decltype(type);
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+          mbar_wait(&sh->staged[c][slot], slot_phase, ctl, status, kErrWaitTma);
+          const uint8_t* src = staging + slot * kQuarterBytes + src_lane;
+          uint8_t* out = dst + (2 * c + half) * (kQuarterRows * 128);
+          float4 v[8][2];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            v[e][0] = *reinterpret_cast<const float4*>(src + e * (4 * kD * 4));
+            v[e][1] = *reinterpret_cast<const float4*>(src + e * (4 * kD * 4) + 16);
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            *reinterpret_cast<uint4*>(out + sw128_offset(e * 4 + (lane >> 3), lane & 7)) =
+                make_uint4(Pack16<T16>::pack(v[e][0].x, v[e][0].y), Pack16<T16>::pack(v[e][0].z, v[e][0].w),
+                           Pack16<T16>::pack(v[e][1].x, v[e][1].y), Pack16<T16>::pack(v[e][1].z, v[e][1].w));
+          __syncwarp();
+          ask();                              // into the quarter just read
+          if (++slot == kStaged) {
+            slot = 0;
+            slot_phase ^= 1u;
+          }
+        }
+      };
+      auto publish = [&](uint64_t* bar) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar);
+      };
+      for (Walk w(n_steps, n_tiles); w.valid(); w.next()) {
+        const int n = w.n, u_lo = w.first() ? w.first_tile_loaded() : w.t;
+        // the Q buffer and the slots of the new K tiles, then those of the V tiles, are free: as where TMA fills them
+        if (w.first()) {
+          if (n >= 1) mbar_wait(&sh->qk_done[(n - 1) & 1], step_phase(n - 1), ctl, status, kErrWaitMma);
+        } else if (n >= 2) {
+          mbar_wait(&sh->qk_done[n & 1], step_phase(n - 2), ctl, status, kErrWaitMma);
+        }
+        for (int u = u_lo; u <= w.t; ++u) convert(smem_k + (u & 3) * kTileBytes, __nv_bfloat16());
+        convert(smem_q + (n & 1) * kTileBytes, __nv_bfloat16());
+        publish(&sh->qk_full[n & 1]);
+        if (w.first()) {
+          if (n >= 1) mbar_wait(&sh->pv_done[(n - 1) & 1], step_phase(n - 1), ctl, status, kErrWaitMma);
+        } else if (w.t - 2 >= w.t0) {
+          mbar_wait(&sh->pv_done[n & 1], step_phase(n - 2), ctl, status, kErrWaitMma);
+        }
+        for (int u = u_lo; u <= w.t; ++u) convert(smem_v + (u & 3) * kTileBytes, VT());
+        publish(&sh->v_full[n & 1]);
       }
     } else if (role == 2) {
       // ---------------------------------------------------------- V loads
@@ -352,6 +466,15 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   }
 }
 
+// q, k, v as FP32 tensors [B, 8, T, 64] of any strides (in values): (64, T, 8, B), boxes of a quarter tile
+static int encode_f32_map(CUtensorMap* map, const void* base, const long long* strides, int B, int T) {
+  const cuuint64_t dims[4] = {64, static_cast<cuuint64_t>(T), 8, static_cast<cuuint64_t>(B)};
+  const cuuint64_t bytes[3] = {static_cast<cuuint64_t>(strides[2]) * 4, static_cast<cuuint64_t>(strides[1]) * 4,
+                               static_cast<cuuint64_t>(B > 1 ? strides[0] : 512) * 4};
+  const cuuint32_t box[4] = {64, longclip::kQuarterRows, 1, 1}, estr[4] = {1, 1, 1, 1};
+  return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(base), dims, bytes, box, estr, CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+
 static int encode_long_map(CUtensorMap* map, const void* base, int B, int T, uint32_t box_rows) {
   // [B, T, 512] 16-bit viewed as (512 fastest, T, B); box = 64 columns x box_rows frames of one clip.
   const cuuint64_t dims[3] = {512, static_cast<cuuint64_t>(T), static_cast<cuuint64_t>(B)};
@@ -367,6 +490,15 @@ bool band_attn_long_takes(int T, int window) {
   return T > 2 * longclip::kTile && window > longclip::kTile + 1 && window <= 2 * longclip::kTile + 1;
 }
 
+// The steps of B clips of T frames and the blocks that share them.
+static int long_steps(int B, int T, int* n_steps, int* n_tiles) {
+  *n_tiles = (T + longclip::kTile - 1) / longclip::kTile;
+  const long long steps = static_cast<long long>(B) * 8 * *n_tiles;
+  *n_steps = steps > 0x7fffffffLL ? 0 : static_cast<int>(steps);
+  const int sms = sm_count();
+  return *n_steps < sms ? *n_steps : sms;
+}
+
 int launch_band_attn_long(const void* q, const void* k, const void* v, void* out, int B, int T, int window, float scale,
                           int value_is_fp16, int* status, cudaStream_t st, int dependent, int out_fp32) {
   using namespace longclip;
@@ -378,17 +510,47 @@ int launch_band_attn_long(const void* q, const void* k, const void* v, void* out
   if (rc == 0) rc = encode_long_map(&tv, v, B, T, kTile);     // element size is what matters: 16 bit
   if (rc == 0) rc = out_fp32 ? encode_long_map(&tout, q, B, T, 32) : encode_long_map(&tout, out, B, T, 32);   // FP32: a placeholder
   if (rc != 0) return rc;
-  auto kern = out_fp32 ? (value_is_fp16 ? band_attn_long_kernel<__half, float> : band_attn_long_kernel<__nv_bfloat16, float>)
-                       : (value_is_fp16 ? band_attn_long_kernel<__half, __half> : band_attn_long_kernel<__nv_bfloat16, __nv_bfloat16>);
-  rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
+  auto kern = out_fp32 ? (value_is_fp16 ? band_attn_long_kernel<__half, float, false> : band_attn_long_kernel<__nv_bfloat16, float, false>)
+                       : (value_is_fp16 ? band_attn_long_kernel<__half, __half, false> : band_attn_long_kernel<__nv_bfloat16, __nv_bfloat16, false>);
+  rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes(false));
   if (rc != 0) return rc;
-  const int sms = sm_count();
-  const int n_tiles = (T + kTile - 1) / kTile;
-  const long long steps = static_cast<long long>(B) * 8 * n_tiles;
-  if (steps > 0x7fffffffLL) return -1;
-  const int n_steps = static_cast<int>(steps), grid = n_steps < sms ? n_steps : sms;
-  return launch_kernel(kern, dim3(grid), kThreads, kSmemBytes, st, 1, dependent, tq, tk, tv, tout,
+  int n_steps, n_tiles;
+  const int grid = long_steps(B, T, &n_steps, &n_tiles);
+  if (n_steps == 0) return -1;
+  return launch_kernel(kern, dim3(grid), threads(false), smem_bytes(false), st, 1, dependent, tq, tk, tv, tout,
                        out_fp32 ? static_cast<float*>(out) : nullptr, n_steps, n_tiles, T, window, scale * 1.4426950408889634f, status);
+}
+
+// The strides that a tensor map can have.
+bool band_attn_long_takes_f32(const long long* strides, int B) {
+  for (int i = 0; i < 9; ++i) {
+    if (i % 3 == 0 && B == 1) continue;
+    if (strides[i] < 4 || strides[i] % 4 != 0 || strides[i] >= (1ll << 38)) return false;
+  }
+  return true;
+}
+
+int launch_band_attn_long_f32(const void* const* qkv, const long long* strides, float* out, int B, int T, int window, float scale,
+                              int value_is_fp16, int* status, cudaStream_t st) {
+  using namespace longclip;
+  if (B <= 0 || !band_attn_long_takes(T, window) || !band_attn_long_takes_f32(strides, B)) return -1;
+  if ((reinterpret_cast<uintptr_t>(out) & 31u) != 0) return -3;
+  CUtensorMap maps[4];
+  int rc = 0;
+  for (int i = 0; i < 3 && rc == 0; ++i) {
+    if ((reinterpret_cast<uintptr_t>(qkv[i]) & 15u) != 0) return -3;
+    rc = encode_f32_map(&maps[i], qkv[i], strides + 3 * i, B, T);
+  }
+  if (rc != 0) return rc;
+  maps[3] = maps[0];                                   // a placeholder: FP32 rows are stored from registers
+  auto kern = value_is_fp16 ? band_attn_long_kernel<__half, float, true> : band_attn_long_kernel<__nv_bfloat16, float, true>;
+  rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes(true));
+  if (rc != 0) return rc;
+  int n_steps, n_tiles;
+  const int grid = long_steps(B, T, &n_steps, &n_tiles);
+  if (n_steps == 0) return -1;
+  return launch_kernel(kern, dim3(grid), threads(true), smem_bytes(true), st, 1, 0, maps[0], maps[1], maps[2], maps[3], out, n_steps, n_tiles, T,
+                       window, scale * 1.4426950408889634f, status);
 }
 
 }  // namespace fm

@@ -431,3 +431,29 @@ def test_objects_without_what_is_kept_between_calls():
     e = torch.randn(1, 512, 5, device="cuda")
     codes = split.encode(e)
     assert torch.equal(old.encode(e), codes) and torch.equal(old.decode(codes), split.decode(codes))
+
+
+@pytest.mark.parametrize("B,T,window", [(1, 257, 250), (2, 384, 130), (1, 385, 257), (3, 640, 250), (5, 1001, 249), (20, 300, 250)])
+@pytest.mark.parametrize("value_dtype", [torch.float16, torch.bfloat16])
+def test_fp32_tensors_of_any_layout_in_long_clips(B, T, window, value_dtype):
+    """FP32 q, k, v are rounded inside the attention kernel.  The rounding is that of the converting pass, which tensors with a
+    stride that a tensor map cannot have (a clip repeated by expand) still take: equal bit for bit.  Shares of a block begin and
+    end anywhere in a sequence.  Bound: q and k in BF16 (2^-9 each, over sqrt(64) terms), v and probabilities in 16 bit."""
+    from fast_mimi_b200 import ops
+    torch.manual_seed(T + window)
+    layouts = [lambda: torch.randn(B, T, 8, 64, device="cuda").transpose(1, 2), lambda: torch.randn(B, 8, T, 64, device="cuda"),
+               lambda: torch.randn(T, B, 8, 72, device="cuda")[..., :64].permute(1, 2, 0, 3),
+               lambda: torch.randn(B, T, 3, 8, 64, device="cuda")[:, :, 1].transpose(1, 2)]
+    q, k, v = layouts[0](), layouts[1](), layouts[2]()
+    y = ops.window_attention(q, k, v, window=window, value_dtype=value_dtype)
+    again = ops.window_attention(*(t.clone(memory_format=torch.contiguous_format) for t in (q, k, v)), window=window, value_dtype=value_dtype)
+    assert torch.equal(y, again)
+    for b in {0, B - 1}:
+        twice = ops.window_attention(*(t[b:b + 1].expand(2, -1, -1, -1) for t in (q, k, v)), window=window, value_dtype=value_dtype)
+        assert torch.equal(twice[0], y[b]) and torch.equal(twice[1], y[b])
+    q, k, v = (layouts[3]() for _ in range(3))
+    y = ops.window_attention(q, k, v, window=window, value_dtype=value_dtype)
+    i = torch.arange(T, device="cuda")
+    seen = (i[None] <= i[:, None]) & (i[None] > i[:, None] - window)
+    ref = torch.softmax((q.double() @ k.double().transpose(-1, -2) * 0.125).masked_fill(~seen, float("-inf")), -1) @ v.double()
+    assert O.rel_l2(y.double().cpu(), ref.cpu()) < (8e-3 if value_dtype == torch.float16 else 1e-2)
