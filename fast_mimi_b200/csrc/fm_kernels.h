@@ -174,6 +174,10 @@ int launch_rvq_select_rec(const void* records, const float* codebook, float* res
 int launch_rvq_encode(float* resid, void* resid16, float* tau, void* records, const void* books16, const float* books, const float* e_sq,
                       const float* e_max, long long* codes, int* n_candidates, long long rows, int n_codes, int layers, float tau_rel,
                       int* status, cudaStream_t st);
+// The whole search in one kernel for few vectors (fm_rvq_stack.cu); nothing but codes is written.
+bool rvq_stack_takes(long long rows, int n_codes, int layers);
+int launch_rvq_stack(const float* x, const void* books16, const float* books, const float* e_sq, const float* e_max, long long* codes,
+                     long long rows, int layers, float tau_rel, int* status, cudaStream_t st);
 int launch_rvq_prepare(const float* x, void* resid16, float* tau, long long rows, float e_max, float tau_rel,
                        cudaStream_t st);
 int launch_rvq_to_half(const float* x, void* y, long long rows, cudaStream_t st);

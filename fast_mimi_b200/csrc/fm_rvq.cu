@@ -454,6 +454,8 @@ int launch_rvq_encode(float* resid, void* resid16, float* tau, void* records, co
                       int* status, cudaStream_t st) {
   if (rows < 0 || rows > 0x7fffffffLL || layers <= 0 || n_codes <= 0 || n_codes % 256 != 0 || n_codes > 2048 || e_max == nullptr) return -1;
   if (rows == 0) return 0;
+  if (n_candidates == nullptr && rvq_stack_takes(rows, n_codes, layers))
+    return launch_rvq_stack(resid, books16, books, e_sq, e_max, codes, rows, layers, tau_rel, status, st);
   int rc = launch_rvq_prepare(resid, resid16, tau, rows, e_max[0], tau_rel, st);
   for (int l = 0; l < layers && rc == 0; ++l) {
     const size_t entry0 = static_cast<size_t>(l) * n_codes;

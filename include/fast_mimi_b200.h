@@ -233,7 +233,8 @@ int fm_upsample2_channels_f32(const float* x, const float* w, float* y, int B, i
 int fm_split_half(const float* x, void* hi, void* lo, long long n, void* stream);
 
 /* The three calls below for a whole stack (src/fast_mimi/model.py:2408-2429), as one chain of dependent launches:
- *   residual     [rows, 256] FP32, the stack's input; overwritten
+ * or, for few vectors without n_candidates, as one kernel:
+ *   residual     [rows, 256] FP32, the stack's input; contents undefined afterwards
  *   residual16   [rows, 256] FP16, tau [rows], records [rows, n_codes / 64] x 16 B: workspaces
  *   codebooks(16) [layers, n_codes, 256], e_sq [layers, n_codes], e_max [layers] in HOST memory
  *   codes        [layers, rows]; n_candidates [layers, rows] or NULL */

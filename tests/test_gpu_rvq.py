@@ -250,3 +250,36 @@ def test_split_precision_products_of_two_weights(rows):
     got = fm.ops._linear_parts(fm.ops.split_half(x), fm.ops.split_half(w), (rows,), None, mats=2)
     want = (x.double() @ w.double().T).view(rows, 2, 256).transpose(0, 1)
     assert got.shape == want.shape and float((got - want).abs().max() / want.abs().max()) < 2e-6
+
+
+@pytest.mark.parametrize("rows", [1, 31, 32, 33, 63, 224, 225])
+@pytest.mark.parametrize("layers", [1, 2, 3, 32])
+def test_search_of_few_vectors_in_one_kernel(rows, layers):
+    """Without candidate counts few vectors take one kernel for the whole stack, with them the chain of products and decisions:
+    the same codes, also where every entry has a twin (the lower index wins) and for a vector of zeros."""
+    from fast_mimi_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(rows * 40 + layers)
+    books = torch.randn(layers, 2048, 256, device="cuda", generator=g) * 0.6 ** torch.arange(layers, device="cuda").clamp(max=7)[:, None, None]
+    books[-1, 1024:] = books[-1, :1024].flip(0)
+    books = ops.RVQCodebooks(books)
+    x = torch.randn(rows, 256, device="cuda", generator=g)
+    x[rows // 2] = 0.0
+    codes = ops.rvq_encode(x, books)
+    chain, _ = ops.rvq_encode(x, books, return_candidates=True)
+    assert torch.equal(codes, chain)
+    assert int(codes[-1].max()) < 1024
+    ops.check_status()
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_one_kernel_search_reports_a_vector_that_is_not_finite(value):
+    from fast_mimi_b200 import ops
+    books = ops.RVQCodebooks(torch.randn(3, 2048, 256, device="cuda"))
+    x = torch.randn(40, 256, device="cuda")
+    good = ops.rvq_encode(x, books)
+    x[35, 7] = value
+    status = ops.new_status("cuda")
+    codes = ops.rvq_encode(x, books, status=status)
+    assert ops.read_status(status) == 105
+    keep = [i for i in range(40) if i != 35]
+    assert torch.equal(codes[:, keep], good[:, keep])
