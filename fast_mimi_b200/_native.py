@@ -62,6 +62,7 @@ SIGNATURES: dict[str, list] = {
     "fm_rope_fp32_verify": [_P, _P, _P, _I, _I, _I, _I, _LL, _P],
     "fm_selftest_wait_timeout": [_P, _I, _P, _P],
     "fm_read_status": [_P, _P],
+    "fm_read_words": [_P, _P, _P, _P],
 }
 
 _lock = threading.Lock()

@@ -106,7 +106,20 @@ def check_status(device=None, status: torch.Tensor | None = None) -> None:
     must be discarded; clear it with ``.zero_()`` after handling the error.  The kernels never synchronise,
     so callers of the attention / layer modules call this at their own synchronisation points."""
     st = default_status(device if device is not None else torch.cuda.current_device()) if status is None else status
-    code = read_status(st)
+    _raise_status(read_status(st))
+
+
+def _check_codes(bad: torch.Tensor, device, status: torch.Tensor | None) -> None:
+    """``check_status`` for a call that looked codes up, with the call's own error word read in the same wait."""
+    words = (ctypes.c_int * 2)()
+    _native.check(_native.load().fm_read_words((default_status(device) if status is None else status).data_ptr(), bad.data_ptr(), words,
+                                               _stream()), "fm_read_words")
+    if words[1] != 0:
+        raise RuntimeError("rvq_decode: a code index is outside the codebook")
+    _raise_status(words[0])
+
+
+def _raise_status(code: int) -> None:
     if code != 0:
         raise RuntimeError(f"fast_mimi_b200: device status {code} ({STATUS_NAMES.get(code, 'unknown code')}); "
                            "outputs written since the last check are not valid; clear the word with .zero_()")
@@ -783,9 +796,7 @@ def rvq_decode_project(codes, first: RVQCodebooks, second: RVQCodebooks | None, 
             rc = lib.fm_linear_split_sum_f32(hi.data_ptr(), lo.data_ptr(), w_hi.data_ptr(), w_lo.data_ptr(), y.data_ptr(), B, T, n_out,
                                              width, st, _stream())
         _native.check(rc, "fm_linear_split")
-    if int(bad.item()) != 0:
-        raise RuntimeError("rvq_decode: a code index is outside the codebook")
-    check_status(codes.device, status)      # the stream is already synchronised by the read above
+    _check_codes(bad, codes.device, status)
     return y
 
 
@@ -802,7 +813,5 @@ def rvq_decode(codes, books: RVQCodebooks):
     rc = lib.fm_rvq_decode_f32(codes.data_ptr(), books.vectors.data_ptr(), out.data_ptr(), rows, layers, books.entries,
                                bad.data_ptr(), _stream())
     _native.check(rc, "fm_rvq_decode_f32")
-    if int(bad.item()) != 0:
-        raise RuntimeError("rvq_decode: a code index is outside the codebook")
-    check_status(codes.device)      # the stream is already synchronised by the read above
+    _check_codes(bad, codes.device, None)
     return out

@@ -343,6 +343,9 @@ int fm_rope_fp32_verify(float* t, const float* cos, const float* sin, int B, int
 
 /* Synchronise `stream` and return the device status word (0 = all bounded waits completed). */
 int fm_read_status(const int* status, void* stream);
+/* The same for two words at once, with one wait: a status word and the error word of a call, either NULL (read as 0), into
+ * words[2] in HOST memory; 0 or a cudaError_t. */
+int fm_read_words(const int* a, const int* b, int* words, void* stream);
 
 #ifdef __cplusplus
 }
