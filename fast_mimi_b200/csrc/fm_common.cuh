@@ -610,6 +610,11 @@ struct ParamVec {
     return make_float4(a.x, a.y, b.x, b.y);
   }
   __device__ __forceinline__ float4 load4(int i) const { return value4(raw4(i)); }
+  __device__ __forceinline__ float at(int i) const {
+    if (type == 2) return __ldg(static_cast<const float*>(data) + i);
+    const uint16_t u = __ldg(static_cast<const uint16_t*>(data) + i);
+    return type == 1 ? __half2float(__ushort_as_half(u)) : __bfloat162float(__ushort_as_bfloat16(u));
+  }
 };
 
 // Four neighbouring values of an activation, from L2, as FP32 (kIn: 0 BF16, 1 FP16, 2 FP32).

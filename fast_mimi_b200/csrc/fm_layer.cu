@@ -77,6 +77,8 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
     rc = launch_layernorm512(x, p.stream_dtype, vec(p.ln1_weight), vec(p.ln1_bias), p.ln1_eps, b.h, tc, rows, st, 1);
     if (rc != 0) return rc;
   }
+  const bool projected = few && stream_attn_projects(B, T);     // the attention kernel goes on to x1
+  const StreamOut proj = {p.w_o, x, b.x1, vec(p.attn_scale), p.stream_dtype};
   const bool few_tiles = !few && few_attn_tiles(B, T) && (!cached || slots <= 256);
   if (whole_clip && !few_tiles && use_fused_clip(B, T)) {
     rc = launch_attn_fused_clip(b.h, p.w_qkv, cos, sin, cos_bstride, b.core, B, T, p.window, p.scale, p.value_dtype, status, st, 1);
@@ -102,7 +104,8 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
     } else if (!cached) {
       rc = launch_band_attn_prefill(b.q, b.k, b.v, b.core, B, T, p.window, p.scale, value_fp16, status, st, 1);
     } else if (few) {
-      rc = launch_stream_attn(b.q, b.k, b.v, ring_k, ring_v, b.core, B, T, past, slots, p.window, p.scale, value_fp16, status, st, 1);
+      rc = launch_stream_attn(b.q, b.k, b.v, ring_k, ring_v, b.core, B, T, past, slots, p.window, p.scale, value_fp16, status, st, 1,
+                              projected ? &proj : nullptr);
     } else {
       if (delta > 0) {
         rc = launch_ring_linearize(ring_k, ring_v, b.k, b.v, b.k_lin, b.v_lin, B, T, delta, past, slots, st, 1);
@@ -116,7 +119,7 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
     }
   }
   if (rc != 0) return rc;
-  rc = launch_linear_gemm(b.core, p.w_o, b.x1, vec(p.attn_scale), x, rows, 512, 512, value_fp16, p.stream_dtype, 0, status, st, 1);
+  if (!projected) rc = launch_linear_gemm(b.core, p.w_o, b.x1, vec(p.attn_scale), x, rows, 512, 512, value_fp16, p.stream_dtype, 0, status, st, 1);
   if (rc != 0) return rc;
   if (norm2_inside) {
     rc = launch_ln_linear_gelu(b.x1, p.stream_dtype, vec(p.ln2_weight), vec(p.ln2_bias), p.ln2_eps, p.w_fc1, b.g, rows, p.ffn, tc, status,

@@ -23,6 +23,12 @@
 // Rows that are already in the ring do not depend on the projection, so in a chain of dependent launches the first items
 // are requested before the wait for it.  A block has an item's ring rows in shared memory before it stores that item's
 // new rows, and no other block touches its (stream, head): the ring is updated in place.
+//
+// While the heads of every stream have blocks of their own at the same time (up to 15 streams) the kernel goes on to the output
+// projection, x1 = residual + scale * core W_o^T: the eight blocks of a stream are a cluster, hand each other their heads'
+// rows through distributed shared memory, and each multiplies them with its 64 rows of W_o, which it asked for before the wait.  As
+// a kernel of its own the projection of a few rows was 4.6 us, a launch and a first load around 0.3 us of products
+// (one stream through eight layers 167 -> 151 us, 15 streams 188 -> 167; rings still empty 162 -> 141).
 #include <type_traits>
 
 #include "fm_common.cuh"
@@ -48,12 +54,15 @@ struct Ctl {
   // phase cannot tell the one two before from it): it read, and gave back, a stage that was being filled.
   uint64_t full[kMaxStages * kGroups];
   uint64_t empty[kMaxStages];
+  uint64_t w_full;
   CtaCtl ctl;
   float m[kGroups][kGroupWarps][kMaxT];
   float l[kGroups][kGroupWarps][kMaxT];
 };
-constexpr int smem_bytes(int stages) {
-  return 1024 + stages * kStageBytes + kGroups * (kNewBytes + kMergeBytes) + static_cast<int>(sizeof(Ctl));
+// Output projection: this block's rows of W_o (eight chunks of 64 x 64), and the eight heads' rows of the stream (8 x 64 each)
+constexpr int kOutBytes = 64 * 1024, kHeadsBytes = 8 * 1024;
+constexpr int smem_bytes(int stages, bool out_proj = false) {
+  return (out_proj ? kOutBytes + kHeadsBytes : 0) + 1024 + stages * kStageBytes + kGroups * (kNewBytes + kMergeBytes) + static_cast<int>(sizeof(Ctl));
 }
 static_assert(smem_bytes(kMaxStages) <= 232448, "exceeds the 227 KB a block may use");
 
@@ -84,18 +93,29 @@ struct StreamArgs {
   int n_loaded;                  // ring rows per item that the tensor maps' boxes cover: min(past, slots)
   int stages;
   float scale_log2e;
+  // output projection
+  const void* resid;             // [S, T, 512] of stream_type
+  void* x1;
+  ParamVec out_scale;
+  int stream_type;               // 0 BF16, 1 FP16, 2 FP32
 };
 
+// kOut: a block has one item, the eight heads of a stream are a cluster, and the result goes through the output projection.
 // VT: type of the ring's values, v and the result
-template <typename VT>
+template <typename VT, bool kOut>
 __global__ void __launch_bounds__(stream::kThreads, 1)
 stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
-                   const __grid_constant__ StreamArgs a, int* status) {
+                   const __grid_constant__ CUtensorMap tmap_o, const __grid_constant__ StreamArgs a, int* status) {
   using namespace stream;
-  if (chain_stopped(status)) return;
+  // A status set before this chain began: nothing is stored.  The blocks of a cluster write into one another's memory and
+  // stay to the end.
+  const bool skip = kOut && status != nullptr && *reinterpret_cast<volatile int*>(status) != 0;
+  if (!kOut && chain_stopped(status)) return;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* smem_new = smem + a.stages * kStageBytes;
+  uint8_t* smem_out = smem + a.stages * kStageBytes;           // kOut: W_o, then the heads
+  uint8_t* smem_heads = smem_out + kOutBytes;
+  uint8_t* smem_new = kOut ? smem_heads + kHeadsBytes : smem_out;
   float* smem_merge = reinterpret_cast<float*>(smem_new + kGroups * kNewBytes);
   Ctl* c = reinterpret_cast<Ctl*>(smem_new + kGroups * (kNewBytes + kMergeBytes));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -105,6 +125,7 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
       mbar_init(&c->empty[i], kGroupWarps);
     }
     for (int i = 0; i < kGroups * a.stages; ++i) mbar_init(&c->full[i], 1);
+    if (kOut) mbar_init(&c->w_full, 1);
     c->ctl.abort = 0;
     fence_mbar_init();
   }
@@ -116,13 +137,21 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
     *reinterpret_cast<uint4*>(smem + tile * kTileBytes + a.n_loaded * 128 + piece * 16) = zero;
   }
   for (int i = threadIdx.x; i < kGroups * kNewBytes / 16; i += kThreads) *reinterpret_cast<uint4*>(smem_new + i * 16) = zero;
+  if (kOut)
+    for (int i = threadIdx.x; i < kHeadsBytes / 16; i += kThreads) *reinterpret_cast<uint4*>(smem_heads + i * 16) = zero;
   fence_proxy_async_smem();
   __syncthreads();
+  if (kOut) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // this block's memory may be written
   griddep_launch();
   CtaCtl* ctl = &c->ctl;
 
   if (warp == kGroups * kGroupWarps) {
     if (lane == 0) {
+      if constexpr (kOut) {
+        mbar_arrive_expect_tx(&c->w_full, kOutBytes);
+#pragma unroll
+        for (int kc = 0; kc < 8; ++kc) tma_load_2d(smem_out + kc * 8192, &tmap_o, &c->w_full, kc * 64, static_cast<int>(blockIdx.x & 7) * 64);
+      }
       if (a.n_loaded > 0) {
         tma_prefetch_desc(&tmap_k);
         tma_prefetch_desc(&tmap_v);
@@ -201,7 +230,7 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
           if (piece < n_pieces) {
             *reinterpret_cast<uint4*>(new_k + sw128_offset(t, piece & 7)) = nk[e];
             *reinterpret_cast<uint4*>(new_v + sw128_offset(t, piece & 7)) = nv[e];
-            if (t >= a.T - a.slots) {                    // of two rows for one slot the newer stays
+            if (t >= a.T - a.slots && !skip) {           // of two rows for one slot the newer stays
               const size_t at = (static_cast<size_t>(item) * a.slots + (a.past + t) % a.slots) * 64 + (piece & 7) * 8;
               *reinterpret_cast<uint4*>(a.ring_k + at) = nk[e];
               *reinterpret_cast<uint4*>(a.ring_v + at) = nv[e];
@@ -340,6 +369,32 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         }
       }
       named_bar_sync(1 + cg, kGroupWarps * 32);
+      if constexpr (kOut) {
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");            // the other heads' blocks run
+        // two values a thread, to the eight blocks of the stream
+        for (int i = gt; i < a.T * 32; i += kGroupWarps * 32) {
+          const int t = i >> 5, d = 2 * (i & 31);
+          float mx = -INFINITY;
+#pragma unroll
+          for (int w = 0; w < kGroupWarps; ++w) mx = fmaxf(mx, c->m[cg][w][t]);
+          float num[2] = {0.f, 0.f}, den = 0.f;
+#pragma unroll
+          for (int w = 0; w < kGroupWarps; ++w) {
+            const float f = ex2_approx(c->m[cg][w][t] - mx);
+            const float2 v = *reinterpret_cast<const float2*>(&merge[(w * kMaxT + t) * 64 + d]);
+            num[0] = fmaf(f, v.x, num[0]);
+            num[1] = fmaf(f, v.y, num[1]);
+            den = fmaf(f, c->l[cg][w][t], den);
+          }
+          const uint32_t pair = Pack16<VT>::pack(num[0] / den, num[1] / den);
+          const uint32_t at = smem_u32(smem_heads + h * 1024) + sw128_offset(t, d >> 3) + (d & 7) * 2;
+#pragma unroll
+          for (uint32_t peer = 0; peer < 8; ++peer)
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_cta(at, peer)), "r"(pair) : "memory");
+        }
+        __syncwarp();
+        continue;                                        // the block's only item
+      }
       for (int i = gt; i < a.T * 64; i += kGroupWarps * 32) {
         const int t = i >> 6, d = i & 63;
         float mx = -INFINITY;
@@ -359,13 +414,71 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
       named_bar_sync(1 + cg, kGroupWarps * 32);          // the merge buffer and the new rows' tiles are free again
     }
   }
+  if constexpr (kOut) {
+    __syncwarp();
+    if (warp >= kGroupWarps) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");     // the first group is past it
+    cluster_sync_all();                                  // every head's rows have arrived
+    float* red = reinterpret_cast<float*>(smem);         // the ring's stage is done with: eight partial results of 8 x 64
+    if (warp < 8) {
+      // y^T = W_o core^T: 64 rows of W_o, the stream's frames as eight columns; warp w has K of head w
+      mbar_wait(&c->w_full, 0, ctl, status, kErrWaitTma);
+      __syncwarp();
+      float y[4][4];
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt) y[mt][0] = y[mt][1] = y[mt][2] = y[mt][3] = 0.f;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t b[4];
+        ldmatrix4(b, smem_u32(smem_heads + warp * 1024) + sw128_offset(lane & 7, 4 * half + (lane >> 3)));
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+#pragma unroll
+          for (int mt = 0; mt < 4; ++mt) {
+            uint32_t w[4];
+            ldmatrix4(w, smem_u32(smem_out + warp * 8192) + sw128_offset(mt * 16 + (lane & 15), 4 * half + 2 * ks + (lane >> 4)));
+            mma_16x8x16<VT>(y[mt], w, b[2 * ks], b[2 * ks + 1]);
+          }
+        }
+      }
+      const int g = lane >> 2, cpair = (lane & 3) * 2;
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) red[(warp * 8 + cpair + (e & 1)) * 64 + mt * 16 + g + 8 * (e >> 1)] = y[mt][e];
+      }
+    }
+    __syncthreads();
+    const int channel = static_cast<int>(blockIdx.x & 7) * 64 + (threadIdx.x & 63);
+    const long long row0 = static_cast<long long>(blockIdx.x >> 3) * a.T;
+    for (int t = static_cast<int>(threadIdx.x) >> 6; t < a.T && threadIdx.x < 256; t += 4) {
+      float v = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) v += red[(w * 8 + t) * 64 + (threadIdx.x & 63)];
+      const long long at = (row0 + t) * 512 + channel;
+      v = v * a.out_scale.at(channel);
+      if (a.stream_type == 2) {
+        v += __ldcg(static_cast<const float*>(a.resid) + at);
+        if (!skip) static_cast<float*>(a.x1)[at] = v;
+      } else if (a.stream_type == 1) {
+        v += __half2float(__ushort_as_half(__ldcg(static_cast<const uint16_t*>(a.resid) + at)));
+        if (!skip) static_cast<uint16_t*>(a.x1)[at] = __half_as_ushort(__float2half_rn(v));
+      } else {
+        v += __bfloat162float(__ushort_as_bfloat16(__ldcg(static_cast<const uint16_t*>(a.resid) + at)));
+        if (!skip) static_cast<uint16_t*>(a.x1)[at] = __bfloat16_as_ushort(__float2bfloat16_rn(v));
+      }
+    }
+  }
   __syncthreads();
   if (ctl->abort) __nanosleep(20000);
 }
 
+// With 64 KB of W_o a block fills an SM, and the device holds 15 clusters of eight such blocks: a sixteenth stream would wait for a
+// second wave (4 us a layer, what the projection saves: 16 streams 191 us with its own launch).
+bool stream_attn_projects(int S, int T) { return S <= 15 && S * 8 <= sm_count() && T <= stream::kMaxT; }
+
 int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k, void* ring_v, void* out, int S, int T,
                        int past, int slots, int window, float scale, int value_is_fp16, int* status,
-                       cudaStream_t st, int dependent) {
+                       cudaStream_t st, int dependent, const StreamOut* proj) {
   using namespace stream;
   if (S <= 0 || T <= 0) return (S == 0 || T == 0) ? 0 : -1;
   if (past < 0 || window <= 0 || slots < window || slots > 256 || T > kMaxT) return -1;
@@ -387,10 +500,23 @@ int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k
   StreamArgs a = {static_cast<const uint16_t*>(q), static_cast<const uint16_t*>(k), static_cast<const uint16_t*>(v),
                   static_cast<uint16_t*>(ring_k), static_cast<uint16_t*>(ring_v), static_cast<uint16_t*>(out), n_items, T, past, delta, slots, window,
                   n_loaded, stages, scale * 1.4426950408889634f};
-  auto kern = value_is_fp16 ? stream_attn_kernel<__half> : stream_attn_kernel<__nv_bfloat16>;
-  const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes(stages));
+  CUtensorMap to = {};
+  if (proj != nullptr) {
+    if (!stream_attn_projects(S, T)) return -1;
+    if ((reinterpret_cast<uintptr_t>(proj->w_o) | reinterpret_cast<uintptr_t>(proj->resid) | reinterpret_cast<uintptr_t>(proj->x1)) & 15u) return -3;
+    const int rc = encode_rows_16bit(&to, proj->w_o, 512, 512, 64, 64);
+    if (rc != 0) return rc;
+    a.resid = proj->resid;
+    a.x1 = proj->x1;
+    a.out_scale = proj->scale;
+    a.stream_type = proj->stream_type;
+  }
+  auto kern = proj != nullptr ? (value_is_fp16 ? stream_attn_kernel<__half, true> : stream_attn_kernel<__nv_bfloat16, true>)
+                              : (value_is_fp16 ? stream_attn_kernel<__half, false> : stream_attn_kernel<__nv_bfloat16, false>);
+  const int bytes = smem_bytes(stages, proj != nullptr);
+  const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), bytes);
   if (rc != 0) return rc;
-  return launch_kernel(kern, dim3(n_items < sms ? n_items : sms), kThreads, smem_bytes(stages), st, 1, dependent, tk, tv, a, status);
+  return launch_kernel(kern, dim3(n_items < sms ? n_items : sms), kThreads, bytes, st, proj != nullptr ? 8 : 1, dependent, tk, tv, to, a, status);
 }
 
 }  // namespace fm

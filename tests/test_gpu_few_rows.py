@@ -152,6 +152,41 @@ def test_streaming_probabilities_keep_the_bits_of_fp32(value_dtype, T):
     fm.check_status()
 
 
+@pytest.mark.parametrize("T", [1, 2, 8])
+@pytest.mark.parametrize("past", [0, 3, 249, 700])
+@pytest.mark.parametrize("dtype,value_dtype", [(torch.float32, torch.float16), (torch.bfloat16, torch.bfloat16), (torch.float16, torch.float16)])
+def test_output_projection_behind_the_heads_of_a_stream(T, past, dtype, value_dtype):
+    """Up to 15 streams the attention kernel goes on to the output projection, 16 take a kernel for it: what a stream's rows come
+    to must not depend on it but for the order of FP32 sums (2^-21 of the branch) and, where that flips the rounding of an
+    operand behind it, 16-bit units (2^-9 BF16, 2^-11 FP16, over 512 terms with random signs).  Rings are equal bit for bit."""
+    import fast_mimi_b200 as fm
+    layer = fm.MimiTransformerLayerB200(value_dtype=value_dtype).cuda()
+    layer.load_state_dict(_layer_params(T + past), strict=True)
+    layer = layer.to(dtype)
+    g = torch.Generator(device="cuda").manual_seed(past)
+    x = torch.randn(16, T, 512, device="cuda", generator=g).to(dtype)
+    cs = fm.rope_tables(torch.arange(past, past + T, device="cuda")[None])
+    rings = [fm.MimiKVRing(1, n, 250, value_dtype=value_dtype) for n in (16, 15, 1)]
+    for t in (rings[0].ring_k, rings[0].ring_v):
+        t.normal_(generator=g)
+    outs = []
+    for ring in rings:
+        n = ring.num_streams
+        ring.ring_k.copy_(rings[0].ring_k[:, :n]) if ring is not rings[0] else None
+        ring.ring_v.copy_(rings[0].ring_v[:, :n]) if ring is not rings[0] else None
+    for ring in rings:
+        ring.advance(0, past)
+        outs.append(layer(x[:ring.num_streams], None, ring, cs)[0])
+    for ring, y in zip(rings[1:], outs[1:]):
+        n = ring.num_streams
+        assert torch.equal(ring.ring_k[0], rings[0].ring_k[0, :n]) and torch.equal(ring.ring_v[0], rings[0].ring_v[0, :n])
+        want = outs[0][:n].float() - x[:n].float()
+        bound = {torch.float32: 1e-3, torch.float16: 4e-3, torch.bfloat16: 2e-2}[dtype]
+        assert O.rel_l2((y.float() - x[:n].float()).cpu(), want.cpu()) < bound
+    assert torch.equal(outs[1][:1], outs[2])
+    fm.check_status()
+
+
 def test_layer_follows_its_ring():
     """A session whose ring goes through pickle, then gets new storage, half way: outputs and rings are those of a session
     left alone."""
