@@ -55,6 +55,7 @@ struct Ctl {
   uint64_t full[kMaxStages * kGroups];
   uint64_t empty[kMaxStages];
   uint64_t w_full;
+  uint64_t heads_full;     // the stream's eight heads have sent their rows
   CtaCtl ctl;
   float m[kGroups][kGroupWarps][kMaxT];
   float l[kGroups][kGroupWarps][kMaxT];
@@ -129,9 +130,13 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
       mbar_init(&c->empty[i], kGroupWarps);
     }
     for (int i = 0; i < kGroups * a.stages; ++i) mbar_init(&c->full[i], 1);
-    if (kOut) mbar_init(&c->w_full, 1);
+    if (kOut) {
+      mbar_init(&c->w_full, 1);
+      mbar_init(&c->heads_full, 1);
+    }
     c->ctl.abort = 0;
     fence_mbar_init();
+    if (kOut) mbar_arrive_expect_tx(&c->heads_full, 1024u * static_cast<uint32_t>(a.T));
   }
   // Slots past the loaded ones and rows past the new ones are never written: zeros, so that a probability of zero times
   // what lies there is zero.
@@ -393,8 +398,9 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
           const uint32_t pair = Pack16<VT>::pack(num[0] / den, num[1] / den);
           const uint32_t at = smem_u32(smem_heads + h * 1024) + sw128_offset(t, d >> 3) + (d & 7) * 2;
 #pragma unroll
-          for (uint32_t peer = 0; peer < 8; ++peer)
-            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_cta(at, peer)), "r"(pair) : "memory");
+          for (uint32_t peer = 0; peer < 8; ++peer)    // counted where they arrive: a barrier of the cluster would be a fence besides
+            asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
+                         ::"r"(map_to_cta(at, peer)), "r"(pair), "r"(map_to_cta(smem_u32(&c->heads_full), peer)) : "memory");
         }
         __syncwarp();
         continue;                                        // the block's only item
@@ -421,11 +427,12 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   if constexpr (kOut) {
     __syncwarp();
     if (warp >= kGroupWarps) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");     // the first group is past it
-    cluster_sync_all();                                  // every head's rows have arrived
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // this block has sent what it had to send
     float* red = reinterpret_cast<float*>(smem);         // the ring's stage is done with: eight partial results of 8 x 64
     if (warp < 8) {
       // y^T = W_o core^T: 64 rows of W_o, the stream's frames as eight columns; warp w has K of head w
       mbar_wait(&c->w_full, 0, ctl, status, kErrWaitTma);
+      mbar_wait_cluster(&c->heads_full, 0, ctl, status, kErrWaitConsumer);
       __syncwarp();
       float y[4][4];
 #pragma unroll
@@ -471,6 +478,10 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         if (!skip) static_cast<uint16_t*>(out.x1)[at] = __bfloat16_as_ushort(__float2bfloat16_rn(v));
       }
     }
+  }
+  if constexpr (kOut) {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");        // nobody still writes into a block that has left
   }
   __syncthreads();
   if (ctl->abort) __nanosleep(20000);
