@@ -204,8 +204,8 @@ int launch_ring_append(const void* k_new, const void* v_new, void* ring_k, void*
 int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k, void* ring_v, void* out, int S, int T,
                        int past, int slots, int window, float scale, int value_is_fp16, int* status, cudaStream_t st,
                        int dependent = 0, const struct StreamOut* proj = nullptr);
-// With `proj` the result goes through the output projection, x1 = resid + scale * out W_o^T (rows of stream_type), and `out` is
-// not written: for as many streams as stream_attn_projects says.
+// With `proj` the result goes through the output projection, x1 = resid + scale * out W_o^T (rows of stream_type; no scale: one), and
+// `out` is not written: for as many streams as stream_attn_projects says.
 struct StreamOut {
   const void *w_o, *resid;
   void* x1;

@@ -101,7 +101,7 @@ template <> struct StreamOutArgs<true> {
   CUtensorMap w_o;
   const void* resid;             // [S, T, 512] of stream_type
   void* x1;
-  ParamVec scale;
+  ParamVec scale;                // without data: one
   int stream_type;               // 0 BF16, 1 FP16, 2 FP32
 };
 
@@ -466,7 +466,7 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
 #pragma unroll
       for (int w = 0; w < 8; ++w) v += red[(w * 8 + t) * 64 + (threadIdx.x & 63)];
       const long long at = (row0 + t) * 512 + channel;
-      v = v * out.scale.at(channel);
+      if (out.scale.data != nullptr) v *= out.scale.at(channel);
       if (out.stream_type == 2) {
         v += __ldcg(static_cast<const float*>(out.resid) + at);
         if (!skip) static_cast<float*>(out.x1)[at] = v;
@@ -525,7 +525,9 @@ int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k
     return value_is_fp16 ? launch(stream_attn_kernel<__half, false>, none, 1) : launch(stream_attn_kernel<__nv_bfloat16, false>, none, 1);
   }
   if (!stream_attn_projects(S, T)) return -1;
-  if ((reinterpret_cast<uintptr_t>(proj->w_o) | reinterpret_cast<uintptr_t>(proj->resid) | reinterpret_cast<uintptr_t>(proj->x1)) & 15u) return -3;
+  if ((reinterpret_cast<uintptr_t>(proj->w_o) | reinterpret_cast<uintptr_t>(proj->resid) | reinterpret_cast<uintptr_t>(proj->x1) |
+       reinterpret_cast<uintptr_t>(proj->scale.data)) & 15u)
+    return -3;
   StreamOutArgs<true> o = {};
   const int rc = encode_rows_16bit(&o.w_o, proj->w_o, 512, 512, 64, 64);
   if (rc != 0) return rc;

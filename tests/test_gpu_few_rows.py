@@ -187,6 +187,40 @@ def test_output_projection_behind_the_heads_of_a_stream(T, past, dtype, value_dt
     fm.check_status()
 
 
+@pytest.mark.parametrize("T", [1, 8])
+@pytest.mark.parametrize("streams", [1, 15, 16])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_live_streams_without_layer_scales(streams, T, dtype):
+    """The native call takes a layer without scales (NULL) as one whose scales are one, bit for bit, whichever kernel does the
+    output projection, and refuses scales off a 16-byte boundary."""
+    import fast_mimi_b200 as fm
+    layer = fm.MimiTransformerLayerB200().cuda()
+    layer.load_state_dict(_layer_params(31), strict=True)
+    layer = layer.to(dtype).requires_grad_(False)
+    layer.self_attn_layer_scale.scale.fill_(1.0)
+    layer.mlp_layer_scale.scale.fill_(1.0)
+    g = torch.Generator(device="cuda").manual_seed(streams + T)
+    x = torch.randn(streams, T, 512, device="cuda", generator=g).to(dtype)
+    past = 40
+    cos, sin = fm.rope_tables(torch.arange(past, past + T, device="cuda")[None])
+    ring = fm.MimiKVRing(1, streams, 250)
+    for t in (ring.ring_k, ring.ring_v):
+        t.normal_(generator=g)
+    params, keep = layer._native_plan(x)
+    one_k, one_v = ring.ring_k[0].clone(), ring.ring_v[0].clone()
+    call = lambda k, v: fm.ops.layer_forward(params, x, cos, sin, value_dtype=torch.float16, ring=(k, v), past=past, window=250)
+    ones = call(one_k, one_v)
+    scale = params.attn_scale
+    params.attn_scale = scale + x.element_size()
+    with pytest.raises(RuntimeError, match="misaligned"):
+        call(ring.ring_k[0].clone(), ring.ring_v[0].clone())
+    params.attn_scale = params.mlp_scale = None
+    null_k, null_v = ring.ring_k[0].clone(), ring.ring_v[0].clone()
+    assert torch.equal(call(null_k, null_v), ones)
+    assert torch.equal(null_k, one_k) and torch.equal(null_v, one_v)
+    fm.check_status()
+
+
 def test_layer_follows_its_ring():
     """A session whose ring goes through pickle, then gets new storage, half way: outputs and rings are those of a session
     left alone."""
