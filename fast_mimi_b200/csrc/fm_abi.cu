@@ -1,10 +1,11 @@
 // extern "C" entry points of libfast_mimi_b200.so (declared in include/fast_mimi_b200.h) and the
 // small host helpers they share.  No torch types, no allocation, no synchronisation except
-// fm_read_status.
+// fm_read_status and fm_read_words.
 #include "../../include/fast_mimi_b200.h"
 
 #include <mutex>
 
+#include "fm_host_words.h"
 #include "fm_kernels.h"
 
 namespace fm {
@@ -56,21 +57,6 @@ int sm_count() {
   if (dev < kMaxDev) known[dev] = sms;
   return sms;
 }
-
-// Pinned words of a host thread, given back when it ends: copies to them do not block, so that one wait serves several.
-struct HostWords {
-  int* data = nullptr;
-  bool ready() {
-    if (data == nullptr && cudaHostAlloc(reinterpret_cast<void**>(&data), 2 * sizeof(int), cudaHostAllocPortable) != cudaSuccess) {
-      (void)cudaGetLastError();
-      data = nullptr;
-    }
-    return data != nullptr;
-  }
-  ~HostWords() {
-    if (data != nullptr) (void)cudaFreeHost(data);
-  }
-};
 
 int ensure_dynamic_smem(const void* kernel, int bytes) {
   // cudaFuncSetAttribute is per device; remember the largest size granted to each (kernel, device) pair
@@ -401,25 +387,13 @@ int fm_selftest_wait_timeout(int* status, int limit_us, int* observed, void* str
 }
 
 int fm_read_status(const int* status, void* stream) {
-  int words[2] = {0, 0};
+  int words[2];
   const int rc = fm_read_words(status, nullptr, words, stream);
   return rc != 0 ? rc : words[0];
 }
 
 int fm_read_words(const int* a, const int* b, int* words, void* stream) {
-  const cudaStream_t st = static_cast<cudaStream_t>(stream);
-  words[0] = words[1] = 0;
-  if (a == nullptr && b == nullptr) return static_cast<int>(cudaStreamSynchronize(st));
-  thread_local fm::HostWords host;
-  if (!host.ready()) return static_cast<int>(cudaErrorMemoryAllocation);
-  cudaError_t e = cudaSuccess;
-  if (a != nullptr) e = cudaMemcpyAsync(host.data, a, sizeof(int), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess && b != nullptr) e = cudaMemcpyAsync(host.data + 1, b, sizeof(int), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return static_cast<int>(e);
-  if (a != nullptr) words[0] = host.data[0];
-  if (b != nullptr) words[1] = host.data[1];
-  return 0;
+  return static_cast<int>(fm::read_words(a, b, words, static_cast<cudaStream_t>(stream)));
 }
 
 }  // extern "C"

@@ -341,10 +341,12 @@ int fm_linear_fp32_verify(const float* x, const float* w, float* y, int M, int N
 int fm_rope_fp32_verify(float* t, const float* cos, const float* sin, int B, int T, int H, int D,
                         long long cos_bstride, void* stream);
 
-/* Synchronise `stream` and return the device status word (0 = all bounded waits completed). */
+/* Synchronise `stream` and return the device status word (0 = all bounded waits completed; else its code, >= 101, or a
+ * cudaError_t). */
 int fm_read_status(const int* status, void* stream);
 /* The same for two words at once, with one wait: a status word and the error word of a call, either NULL (read as 0), into
- * words[2] in HOST memory; 0 or a cudaError_t. */
+ * words[2] in HOST memory; 0 or a cudaError_t.  The first read page-locks one page of the library, for as long as the process
+ * runs; where it cannot, reads work all the same and take a wait per word. */
 int fm_read_words(const int* a, const int* b, int* words, void* stream);
 
 #ifdef __cplusplus
