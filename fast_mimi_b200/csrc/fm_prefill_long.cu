@@ -29,6 +29,7 @@
 #include "fm_common.cuh"
 #include "fm_kernels.h"
 #include "fm_launch.h"
+#include "fm_shares.h"
 
 namespace fm {
 
@@ -74,22 +75,22 @@ constexpr int smem_bytes(bool f32_in) {
 }
 static_assert(smem_bytes(true) <= 232448, "exceeds the 227 KB a CTA may use");
 
-// The steps a CTA takes: an equal share [begin, end) of all (clip, head, query tile) triples in that order, i.e. at most a rest
-// of one sequence, whole ones, and the beginning of another; each of those is a run.  (Whole sequences dealt out in turn: 128
-// sequences of 20 tiles took 20 steps on 128 of 148 SMs, now 18 at most on all of them, 16 clips of 2500 FP32 frames with their
-// conversion 146.9 -> 140.5 us; 200 sequences of 12 tiles took 24 steps, now 17, 25 clips of 1500 frames 158 -> 132 us; 40 clips of 700
-// frames 116 -> 98 us.)  A run re-reads the two K / V tiles in front of it.  Every role of the kernel walks the same
-// steps with the same counter n, which the barrier phases are derived from.
+// The steps a CTA takes: an equal share [begin, end) of all (clip, head, query tile) triples in that order (fm_shares.h), i.e. at
+// most a rest of one sequence, whole ones, and the beginning of another; each of those is a run.  (Whole sequences dealt out in turn:
+// 128 sequences of 20 tiles took 20 steps on 128 of 148 SMs, now 18 at most, 16 clips of 2500 FP32 frames with their conversion
+// in front 146.9 -> 140.5 us; 200 sequences of 12 tiles took 24 steps, now 17, 25 clips of 1500 frames 158 -> 132 us; 40 clips of 700
+// frames 116 -> 98 us.)  A run re-reads the two K / V tiles in front of it, and its first step waits for all of them: shares that
+// differ by one step so as to occupy every SM begin anywhere, shares of the same number often at a sequence's beginning (FP32: 16
+// clips of 513 frames 37.9 -> 33.3 us, 18 of 700 44.1 -> 40.1, 36 of 257 41.9 -> 37.8, 36 of 900 95.4 -> 93.2).  Every role of the
+// kernel walks the same steps with the same counter n, which the barrier phases are derived from.
 struct Walk {
   int n_tiles, at, end;
   int t, t0, n;
   __device__ __forceinline__ Walk(int n_steps, int n_tiles_) : n_tiles(n_tiles_), n(0) {
-    at = share(n_steps, static_cast<int>(blockIdx.x));
-    end = share(n_steps, static_cast<int>(blockIdx.x) + 1);
+    const Shares shares(n_steps, static_cast<int>(gridDim.x));
+    at = shares.first(static_cast<int>(blockIdx.x));
+    end = shares.first(static_cast<int>(blockIdx.x) + 1);
     t = t0 = at % n_tiles;
-  }
-  __device__ __forceinline__ static int share(int n_steps, int block) {
-    return static_cast<int>(static_cast<long long>(n_steps) * block / static_cast<int>(gridDim.x));
   }
   __device__ __forceinline__ bool valid() const { return at < end; }
   __device__ __forceinline__ bool first() const { return t == t0; }
@@ -495,8 +496,7 @@ static int long_steps(int B, int T, int* n_steps, int* n_tiles) {
   *n_tiles = (T + longclip::kTile - 1) / longclip::kTile;
   const long long steps = static_cast<long long>(B) * 8 * *n_tiles;
   *n_steps = steps > 0x7fffffffLL ? 0 : static_cast<int>(steps);
-  const int sms = sm_count();
-  return *n_steps < sms ? *n_steps : sms;
+  return *n_steps > 0 ? Shares(*n_steps, sm_count()).used() : 0;
 }
 
 int launch_band_attn_long(const void* q, const void* k, const void* v, void* out, int B, int T, int window, float scale,
