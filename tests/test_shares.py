@@ -11,6 +11,7 @@ from conftest import ROOT
 
 PROGRAM = r"""
 #include "fm_shares.h"
+#include <initializer_list>
 #include <cstdio>
 #define CHECK(x) do { if (!(x)) { std::printf("line %d: %s (sequences %d of %d tiles, %d blocks)\n", __LINE__, #x, seqs, tiles, blocks); return 1; } } while (0)
 int main() {
