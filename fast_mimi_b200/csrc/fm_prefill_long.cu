@@ -75,32 +75,30 @@ constexpr int smem_bytes(bool f32_in) {
 }
 static_assert(smem_bytes(true) <= 232448, "exceeds the 227 KB a CTA may use");
 
-// The steps a CTA takes: an equal share [begin, end) of all (clip, head, query tile) triples in that order (fm_shares.h), i.e. at
-// most a rest of one sequence, whole ones, and the beginning of another; each of those is a run.  (Whole sequences dealt out in turn:
-// 128 sequences of 20 tiles took 20 steps on 128 of 148 SMs, now 18 at most, 16 clips of 2500 FP32 frames with their conversion
-// in front 146.9 -> 140.5 us; 200 sequences of 12 tiles took 24 steps, now 17, 25 clips of 1500 frames 158 -> 132 us; 40 clips of 700
-// frames 116 -> 98 us.)  A run re-reads the two K / V tiles in front of it, and its first step waits for all of them: shares that
-// differ by one step so as to occupy every SM begin anywhere, shares of the same number often at a sequence's beginning (FP32: 16
-// clips of 513 frames 37.9 -> 33.3 us, 18 of 700 44.1 -> 40.1, 36 of 257 41.9 -> 37.8, 36 of 900 95.4 -> 93.2).  Every role of the
-// kernel walks the same steps with the same counter n, which the barrier phases are derived from.
+// The steps a CTA takes: an equal share of all (clip, head, query tile) triples in that order (fm_shares.h), i.e. at most a rest of
+// one sequence, whole ones, and the beginning of another; each of those is a run.  (Whole sequences dealt out in turn: 128 sequences
+// of 20 tiles took 20 steps on 128 of 148 SMs, now 18 at most, 16 FP16 clips of 2500 frames 116.6 -> 107.2 us; 200 sequences of 12
+// tiles took 24 steps, now 17.)  A run re-reads the two K / V tiles in front of it and its first step waits for all of them, so shares
+// keep to sequences where that takes no block more steps: rounded to occupy every SM, they began anywhere (FP16, 9 clips of 513 frames
+// 19.4 with segments of each sequence, 20.4 without, now 18.6; FP32, 18 of 700 42.4 -> 38.2, 36 of 257 39.4 -> 35.3, 36 of 900
+// 93.8 -> 89.1).  Every role of the kernel walks the same steps with the same counter n, which the barrier phases are derived from.
 struct Walk {
-  int n_tiles, at, end;
-  int t, t0, n;
-  __device__ __forceinline__ Walk(int n_steps, int n_tiles_) : n_tiles(n_tiles_), n(0) {
-    const Shares shares(n_steps, static_cast<int>(gridDim.x));
-    at = shares.first(static_cast<int>(blockIdx.x));
-    end = shares.first(static_cast<int>(blockIdx.x) + 1);
-    t = t0 = at % n_tiles;
+  int n_tiles, seq, t, t0, n, steps;
+  __device__ __forceinline__ explicit Walk(const Shares& shares) : n_tiles(shares.tiles), n(0) {
+    shares.share(static_cast<int>(blockIdx.x), &seq, &t, &steps);
+    t0 = t;
   }
-  __device__ __forceinline__ bool valid() const { return at < end; }
+  __device__ __forceinline__ bool valid() const { return n < steps; }
   __device__ __forceinline__ bool first() const { return t == t0; }
-  __device__ __forceinline__ int clip() const { return (at / n_tiles) >> 3; }
-  __device__ __forceinline__ int head() const { return (at / n_tiles) & 7; }
+  __device__ __forceinline__ int clip() const { return seq >> 3; }
+  __device__ __forceinline__ int head() const { return seq & 7; }
   __device__ __forceinline__ int first_tile_loaded() const { return t0 - 2 > 0 ? t0 - 2 : 0; }   // run's oldest halo tile
   __device__ __forceinline__ void next() {
     ++n;
-    ++at;
-    if (++t == n_tiles) t = t0 = 0;
+    if (++t == n_tiles) {
+      t = t0 = 0;
+      ++seq;
+    }
   }
 };
 }  // namespace longclip
@@ -112,7 +110,7 @@ template <typename VT, typename OT, bool kF32In>
 __global__ void __launch_bounds__(longclip::threads(kF32In), 1)
 band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_out,
-                      float* __restrict__ out32, int n_steps, int n_tiles, int T, int window, float scale_log2e,
+                      float* __restrict__ out32, const __grid_constant__ Shares shares, int T, int window, float scale_log2e,
                       int* status) {
   using namespace longclip;
   using namespace attn_tile;
@@ -188,7 +186,7 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         for (int u = u_lo; u <= w.t; ++u)
           tma_load_3d(smem_k + (u & 3) * kTileBytes, &tmap_k, &sh->qk_full[b], w.head() * kD, u * kTile, w.clip());
       };
-      Walk cur(n_steps, n_tiles), nxt(n_steps, n_tiles);
+      Walk cur(shares), nxt = cur;
       if (cur.valid()) {
         load_qk(cur);
         nxt.next();
@@ -233,7 +231,7 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       }
     } else if (role == 1) {
       // ---------------------------------------------------------- P V products
-      for (Walk w(n_steps, n_tiles); w.valid(); w.next()) {
+      for (Walk w(shares); w.valid(); w.next()) {
         const int n = w.n;
         mbar_wait(&sh->v_full[n & 1], step_phase(n), ctl, status, kErrWaitTma);
         for (int kind = 0; kind < 3; ++kind)
@@ -266,7 +264,7 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       const int c = role - 2;
       uint8_t* staging = smem_stage + c * kStaged * kQuarterBytes;
       // Copies: their own walk, with what a run's tiles have in common worked out once.
-      Walk to_ask(n_steps, n_tiles);
+      Walk to_ask(shares);
       int ask_nk = 0, ask_tile = 0, ask_half = 0, ask_head = 0, ask_clip = 0, asked = 0;
       auto open_step = [&]() {
         if (to_ask.first()) {
@@ -337,7 +335,7 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         __syncwarp();
         if (lane == 0) mbar_arrive(bar);
       };
-      for (Walk w(n_steps, n_tiles); w.valid(); w.next()) {
+      for (Walk w(shares); w.valid(); w.next()) {
         const int n = w.n, u_lo = w.first() ? w.first_tile_loaded() : w.t;
         // the Q buffer and the slots of the new K tiles, then those of the V tiles, are free: as where TMA fills them
         if (w.first()) {
@@ -359,7 +357,7 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     } else if (role == 2) {
       // ---------------------------------------------------------- V loads
       if (one) tma_prefetch_desc(&tmap_v);
-      for (Walk w(n_steps, n_tiles); w.valid(); w.next()) {
+      for (Walk w(shares); w.valid(); w.next()) {
         const int n = w.n, b = n & 1;
         int u_lo = w.t;
         if (w.first()) {
@@ -383,7 +381,7 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     const int lg = warp & 3;                  // TMEM lane group
     const int r = lg * 32 + lane;             // row of the tile == TMEM lane
     const uint32_t slot = tmem_base + static_cast<uint32_t>(team * kTile) + (static_cast<uint32_t>(lg * 32) << 16);
-    for (Walk w(n_steps, n_tiles); w.valid(); w.next()) {
+    for (Walk w(shares); w.valid(); w.next()) {
       const int n = w.n, x = n & 3;
       const uint32_t xph = static_cast<uint32_t>(n >> 2) & 1u;     // this exchange buffer's use number
       const int kind = ((team - 3 * n) % 4 + 4) % 4;               // the job of this step that runs in this team's slot
@@ -491,12 +489,12 @@ bool band_attn_long_takes(int T, int window) {
   return T > 2 * longclip::kTile && window > longclip::kTile + 1 && window <= 2 * longclip::kTile + 1;
 }
 
-// The steps of B clips of T frames and the blocks that share them.
-static int long_steps(int B, int T, int* n_steps, int* n_tiles) {
-  *n_tiles = (T + longclip::kTile - 1) / longclip::kTile;
-  const long long steps = static_cast<long long>(B) * 8 * *n_tiles;
-  *n_steps = steps > 0x7fffffffLL ? 0 : static_cast<int>(steps);
-  return *n_steps > 0 ? Shares(*n_steps, sm_count()).used() : 0;
+// The steps of B clips of T frames (at least one) dealt out; false: too many.
+static bool long_shares(int B, int T, Shares* shares) {
+  const int tiles = (T + longclip::kTile - 1) / longclip::kTile;
+  if (static_cast<long long>(B) * 8 * tiles > 0x7fffffffLL) return false;
+  *shares = Shares(B * 8, tiles, sm_count());
+  return true;
 }
 
 int launch_band_attn_long(const void* q, const void* k, const void* v, void* out, int B, int T, int window, float scale,
@@ -514,11 +512,10 @@ int launch_band_attn_long(const void* q, const void* k, const void* v, void* out
                        : (value_is_fp16 ? band_attn_long_kernel<__half, __half, false> : band_attn_long_kernel<__nv_bfloat16, __nv_bfloat16, false>);
   rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes(false));
   if (rc != 0) return rc;
-  int n_steps, n_tiles;
-  const int grid = long_steps(B, T, &n_steps, &n_tiles);
-  if (n_steps == 0) return -1;
-  return launch_kernel(kern, dim3(grid), threads(false), smem_bytes(false), st, 1, dependent, tq, tk, tv, tout,
-                       out_fp32 ? static_cast<float*>(out) : nullptr, n_steps, n_tiles, T, window, scale * 1.4426950408889634f, status);
+  Shares shares;
+  if (!long_shares(B, T, &shares)) return -1;
+  return launch_kernel(kern, dim3(shares.used()), threads(false), smem_bytes(false), st, 1, dependent, tq, tk, tv, tout,
+                       out_fp32 ? static_cast<float*>(out) : nullptr, shares, T, window, scale * 1.4426950408889634f, status);
 }
 
 // The strides that a tensor map can have.
@@ -546,10 +543,9 @@ int launch_band_attn_long_f32(const void* const* qkv, const long long* strides, 
   auto kern = value_is_fp16 ? band_attn_long_kernel<__half, float, true> : band_attn_long_kernel<__nv_bfloat16, float, true>;
   rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes(true));
   if (rc != 0) return rc;
-  int n_steps, n_tiles;
-  const int grid = long_steps(B, T, &n_steps, &n_tiles);
-  if (n_steps == 0) return -1;
-  return launch_kernel(kern, dim3(grid), threads(true), smem_bytes(true), st, 1, 0, maps[0], maps[1], maps[2], maps[3], out, n_steps, n_tiles, T,
+  Shares shares;
+  if (!long_shares(B, T, &shares)) return -1;
+  return launch_kernel(kern, dim3(shares.used()), threads(true), smem_bytes(true), st, 1, 0, maps[0], maps[1], maps[2], maps[3], out, shares, T,
                        window, scale * 1.4426950408889634f, status);
 }
 

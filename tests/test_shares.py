@@ -18,19 +18,28 @@ int main() {
   for (int blocks : {1, 2, 7, 132, 148})
     for (int seqs = 8; seqs <= 400; seqs += 8)
       for (int tiles : {3, 4, 5, 8, 12, 20, 79}) {
-        const int n = seqs * tiles;
-        const fm::Shares s(n, blocks);
-        const int used = s.used();
-        CHECK(used >= 1 && used <= blocks && used <= n && s.first(0) == 0 && s.first(used) == n);
-        CHECK(fm::Shares(n, used).per_block == s.per_block);                   // the kernel, which has the number of its blocks, deals alike
-        CHECK(s.per_block == (n + blocks - 1) / blocks);                       // no block could have fewer
-        for (int b = 0; b < used; ++b) CHECK(s.first(b + 1) > s.first(b) && s.first(b + 1) - s.first(b) <= s.per_block);
-        // where a share is a whole number of sequences or a whole part of one, none begins inside of a sequence but at such a part
-        if (s.per_block % tiles == 0) for (int b = 0; b < used; ++b) CHECK(s.first(b) % tiles == 0);
-        if (tiles % s.per_block == 0) for (int b = 0; b < used; ++b) CHECK(s.first(b) / tiles == (s.first(b + 1) - 1) / tiles);
+        const fm::Shares s(seqs, tiles, blocks);
+        const int n = seqs * tiles, used = s.used(), most = (n + blocks - 1) / blocks;
+        CHECK(used >= 1 && used <= blocks && used <= n);
+        int at = 0, crossing = 0, inside = 0;
+        for (int b = 0; b < used; ++b) {
+          int seq, tile, steps;
+          s.share(b, &seq, &tile, &steps);
+          CHECK(tile >= 0 && tile < tiles && seq * tiles + tile == at && steps >= 1 && steps <= most);
+          at += steps;
+          crossing += tile + steps > tiles;
+          inside += tile != 0;
+        }
+        CHECK(at == n);
+        // whole sequences, or parts of one, wherever that takes no block more steps than the fewest
+        if (most % tiles == 0) CHECK(inside == 0);
+        if (seqs * ((tiles + most - 1) / most) <= blocks) CHECK(crossing == 0);
       }
-  const int seqs = 0, tiles = 0, blocks = 148;
-  CHECK(fm::Shares(0x7fffffff, 148).first(148) == 0x7fffffff && fm::Shares(0x7fffffff, 148).first(147) < 0x7fffffff);
+  const int seqs = 0x7ffffff8 / 3 / 8 * 8, tiles = 3, blocks = 148;      // as many steps as an int can count
+  int seq, tile, steps;
+  const fm::Shares most(seqs, tiles, blocks);
+  most.share(most.used() - 1, &seq, &tile, &steps);
+  CHECK(seq * 3 + tile + steps == seqs * 3 && steps > 0 && most.used() <= blocks);
   std::puts("ok");
   return 0;
 }
