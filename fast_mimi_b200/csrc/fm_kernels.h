@@ -232,7 +232,7 @@ int launch_band_attn_long(const void* q, const void* k, const void* v, void* out
                           float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent = 0, int out_fp32 = 0);
 bool band_attn_long_takes(int T, int window);
 // The same on FP32 q, k, v [B, 8, T, 64] of the given strides (three of each, in values: clip, head, frame), FP32 result.
-bool band_attn_long_takes_f32(const long long* strides, int B);
+bool band_attn_long_takes_f32(const long long* strides, int B, int T);
 int launch_band_attn_long_f32(const void* const* qkv, const long long* strides, float* out, int B, int T, int window, float scale,
                               int value_is_fp16, int* status, cudaStream_t st);
 // Banded attention on [B, 8, T, 64] tensors of any float type and strides (fm_window.cu).

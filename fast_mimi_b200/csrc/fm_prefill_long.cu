@@ -19,7 +19,7 @@
 // the same load.  Tiles before the clip's first frame are not loaded; their jobs run empty.
 // Warps 0-15: softmax teams.  Warp 16: Q/K loads + score products.  Warp 17: P V products.  Warp 18: V loads.
 //
-// FP32 q, k, v (a model's own, any strides) are converted on the way: quarter tiles of 32 rows arrive by TMA in a staging
+// FP32 q, k, v (a model's own, any strides) of calls with some steps a block are converted on the way: quarter tiles of 32 rows arrive by TMA in a staging
 // buffer, three for each of two warps (18 and 19), which round them (q, k to BF16, v to its type) into the tiles' places.  The
 // kernel is bound by its chain of steps, not by memory, so the 12 bytes a value triple costs instead of 6 pass behind it; a
 // converting pass in front (18 bytes a triple at the copy rate) took 51 of 141 us for 16 clips of 2500 frames, 25 clips of 1500
@@ -518,19 +518,29 @@ int launch_band_attn_long(const void* q, const void* k, const void* v, void* out
                        out_fp32 ? static_cast<float*>(out) : nullptr, shares, T, window, scale * 1.4426950408889634f, status);
 }
 
-// The strides that a tensor map can have.
-bool band_attn_long_takes_f32(const long long* strides, int B) {
+// Strides that a tensor map can have, and enough steps a block.  The two converting warps keep up with the chain of steps, but where a
+// run begins the first step waits until they have made seven tiles instead of three, and a short call is little else; a converting
+// pass in front costs 1 us and 0.7 ns a frame.  Inside from five steps on, from seven where short sequences begin and end inside of shares.
+// GPU time, FP32, in front -> inside:
+//   1 or 2 steps   1 clip of 257 frames 8.6 -> 11.8 us, 1 of 2500 15.6 -> 20.1, 8 of 300 14.3 -> 16.3
+//   3 or 4         8 of 900 28.8 -> 31.5, 12 of 700 31.0 -> 31.9, 16 of 385 25.6 -> 26.0
+//   5 or 6         25 of 257 28.8 -> 33.6 and 25 of 385 (shares run on) 37.8 -> 41.2; 9 of 1200 38.8 -> 37.1, 18 of 513 33.8 -> 31.4
+//   7 and more     14 of 900 49.4 -> 46.5, 36 of 900 112 -> 89, 16 of 2500 135 -> 105; 45 of 257 46.5 -> 48.5
+bool band_attn_long_takes_f32(const long long* strides, int B, int T) {
   for (int i = 0; i < 9; ++i) {
     if (i % 3 == 0 && B == 1) continue;
     if (strides[i] < 4 || strides[i] % 4 != 0 || strides[i] >= (1ll << 38)) return false;
   }
-  return true;
+  Shares s;
+  if (!long_shares(B, T, &s)) return false;
+  const bool run_on = s.cuts == 0 && s.per_block % s.tiles != 0;
+  return s.per_block >= (run_on && s.tiles <= 5 ? 7 : 5);
 }
 
 int launch_band_attn_long_f32(const void* const* qkv, const long long* strides, float* out, int B, int T, int window, float scale,
                               int value_is_fp16, int* status, cudaStream_t st) {
   using namespace longclip;
-  if (B <= 0 || !band_attn_long_takes(T, window) || !band_attn_long_takes_f32(strides, B)) return -1;
+  if (B <= 0 || !band_attn_long_takes(T, window) || !band_attn_long_takes_f32(strides, B, T)) return -1;
   if ((reinterpret_cast<uintptr_t>(out) & 31u) != 0) return -3;
   CUtensorMap maps[4];
   int rc = 0;

@@ -1,11 +1,11 @@
 // Banded attention on q, k, v as a model holds them (sm_100a): any of FP32, BF16 and FP16, [B, 8, T, 64] with any strides and a
 // contiguous last dimension (reference: _native_window_attention, src/fast_mimi/model.py:1589-1624).
 //
-// The attention kernels read frame-major 16-bit tensors.  The kernel for long clips rounds FP32 tensors itself on the way in,
-// whatever their strides, as far as a tensor map can have them (fm_prefill_long.cu: 16 clips of 2500 frames 107 us; a converting pass in front
-// took 51 of 141 us).  For the others bringing FP32 inputs there is HBM-bound: 12 bytes read and six written per value
-// triple, one launch for the three.  The way back is free where the kernel for long clips stores FP32 (a converting pass
-// over the result took 51 us).
+// The attention kernels read frame-major 16-bit tensors.  The kernel for long clips rounds FP32 tensors itself on the way in where its
+// blocks have some steps each, whatever the strides, as far as a tensor map can have them (fm_prefill_long.cu: 16 clips of 2500 frames 105 us,
+// 135 with a converting pass in front).  For the others bringing FP32 inputs there is HBM-bound: 12 bytes read and six
+// written per value triple, one launch for the three.  The way back is free where the kernel for long clips stores FP32 (a
+// converting pass over the result took 51 us).
 #include "fm_common.cuh"
 #include "fm_kernels.h"
 #include "fm_launch.h"
@@ -112,7 +112,7 @@ int launch_window_attention(const void* const* qkv, int in_type, const long long
     in16[i] = ws[i];
   }
   const bool direct = out32 != nullptr && band_attn_long_takes(T, window_size);
-  const bool converts = direct && in_type == 2 && band_attn_long_takes_f32(strides, B);     // the attention kernel itself
+  const bool converts = direct && in_type == 2 && band_attn_long_takes_f32(strides, B, T);     // the attention kernel itself
   if ((reinterpret_cast<uintptr_t>(out16) | reinterpret_cast<uintptr_t>(out32)) & 15u) return -3;
   if (!direct && out16 == nullptr) return -1;
   if (converts) return launch_band_attn_long_f32(qkv, strides, out32, B, T, window_size, scale, value_is_fp16, status, st);

@@ -502,10 +502,13 @@ def test_objects_without_what_is_kept_between_calls():
     assert torch.equal(old.encode(e), codes) and torch.equal(old.decode(codes), split.decode(codes))
 
 
-@pytest.mark.parametrize("B,T,window", [(1, 257, 250), (2, 384, 130), (1, 385, 257), (3, 640, 250), (5, 1001, 249), (20, 300, 250)])
+# one to four steps a block (a converting pass in front), then inside: five (a sequence each), six (two sequences), seven and eight
+# (shares that run on from one sequence into the next)
+@pytest.mark.parametrize("B,T,window", [(1, 257, 250), (2, 384, 130), (1, 385, 257), (3, 640, 250), (5, 1001, 249), (20, 300, 250),
+                                        (18, 513, 130), (37, 300, 249), (19, 700, 257), (45, 260, 250)])
 @pytest.mark.parametrize("value_dtype", [torch.float16, torch.bfloat16])
 def test_fp32_tensors_of_any_layout_in_long_clips(B, T, window, value_dtype):
-    """FP32 q, k, v are rounded inside the attention kernel.  The rounding is that of the converting pass, which tensors with a
+    """FP32 q, k, v of calls with some steps a block are rounded inside the attention kernel.  The rounding is that of the converting pass, which tensors with a
     stride that a tensor map cannot have (a clip repeated by expand) still take: equal bit for bit.  Shares of a block begin and
     end anywhere in a sequence.  Bound: q and k in BF16 (2^-9 each, over sqrt(64) terms), v and probabilities in 16 bit."""
     from fast_mimi_b200 import ops
