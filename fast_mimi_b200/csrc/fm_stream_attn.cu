@@ -429,6 +429,9 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
     if (warp >= kGroupWarps) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");     // the first group is past it
     asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // this block has sent what it had to send
     float* red = reinterpret_cast<float*>(smem);         // the ring's stage is done with: eight partial results of 8 x 64
+    const int channel = static_cast<int>(blockIdx.x & 7) * 64 + (threadIdx.x & 63);
+    float scale = 1.f;                                   // asked for ahead of the wait (in the loop over frames: 1 % for five frames)
+    if (warp < 8 && out.scale.data != nullptr) scale = out.scale.at(channel);
     if (warp < 8) {
       // y^T = W_o core^T: 64 rows of W_o, the stream's frames as eight columns; warp w has K of head w
       mbar_wait(&c->w_full, 0, ctl, status, kErrWaitTma);
@@ -459,14 +462,13 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
       }
     }
     __syncthreads();
-    const int channel = static_cast<int>(blockIdx.x & 7) * 64 + (threadIdx.x & 63);
     const long long row0 = static_cast<long long>(blockIdx.x >> 3) * a.T;
     for (int t = static_cast<int>(threadIdx.x) >> 6; t < a.T && threadIdx.x < 256; t += 4) {
       float v = 0.f;
 #pragma unroll
       for (int w = 0; w < 8; ++w) v += red[(w * 8 + t) * 64 + (threadIdx.x & 63)];
       const long long at = (row0 + t) * 512 + channel;
-      if (out.scale.data != nullptr) v *= out.scale.at(channel);
+      v *= scale;
       if (out.stream_type == 2) {
         v += __ldcg(static_cast<const float*>(out.resid) + at);
         if (!skip) static_cast<float*>(out.x1)[at] = v;
