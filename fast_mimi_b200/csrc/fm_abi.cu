@@ -5,6 +5,7 @@
 
 #include <mutex>
 
+#include "fm_device_fact.h"
 #include "fm_host_words.h"
 #include "fm_kernels.h"
 
@@ -47,15 +48,14 @@ int encode_rows_16bit(CUtensorMap* map, const void* base, uint64_t rows, uint64_
 }
 
 int sm_count() {
-  constexpr int kMaxDev = 64;
-  static int known[kMaxDev];           // written with the same value by whoever asks first
-  int dev = 0, sms = 0;
+  static DeviceFact sms;
+  int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 1;
-  if (dev < kMaxDev && known[dev] > 0) return known[dev];
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (sms <= 0) sms = 1;
-  if (dev < kMaxDev) known[dev] = sms;
-  return sms;
+  const int n = sms.get(dev, [dev] {
+    int count = 0;
+    return cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? count : -1;
+  });
+  return n > 0 ? n : 1;
 }
 
 int ensure_dynamic_smem(const void* kernel, int bytes) {

@@ -1,4 +1,4 @@
-// Launch helper: optional thread-block cluster, optional programmatic dependency on the kernel in front.
+// Launch helpers: optional thread-block cluster, optional programmatic dependency on the kernel in front; how many clusters run at once.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -32,6 +32,25 @@ inline int launch_kernel(void (*kern)(KArgs...), dim3 grid, int threads, int sme
   cfg.attrs = attr;
   cfg.numAttrs = n;
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
+}
+
+// Clusters of `cluster` blocks of a kernel, whose attributes are set, that the current device holds at once; -1: not to be found out.
+template <typename... KArgs>
+inline int resident_clusters(void (*kern)(KArgs...), int threads, int smem_bytes, int cluster) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(cluster));
+  cfg.blockDim = dim3(static_cast<unsigned>(threads));
+  cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess) return n;
+  (void)cudaGetLastError();
+  return -1;
 }
 
 }  // namespace fm

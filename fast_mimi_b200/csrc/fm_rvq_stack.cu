@@ -14,6 +14,7 @@
 // us, and 17 launches less for 8 layers (a 5 s utterance end to end, bound by the host, 200 -> 183 us).  Of the 12300 cycles of a layer the
 // two crossings take 4500, the products 2100 (ldmatrix at the rate of shared memory), the exact distances 1400, the new residual 2700.
 #include "fm_common.cuh"
+#include "fm_device_fact.h"
 #include "fm_kernels.h"
 #include "fm_launch.h"
 #include "fm_warp_mma.cuh"
@@ -254,32 +255,20 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books, const __grid_co
 }
 
 namespace {
-// Clusters of 16 blocks that the device runs at once (0: none).
+// Clusters of 16 blocks that the device runs at once (0: none, or not to be found out just now).
 int stack_slots() {
-  constexpr int kMaxDev = 64;
-  static int known[kMaxDev];             // slots + 1, written with the same value by whoever asks first
+  static DeviceFact slots;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  if (dev < kMaxDev && known[dev] > 0) return known[dev] - 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(rvqs::kCtas);
-  cfg.blockDim = dim3(rvqs::kThreads);
-  cfg.dynamicSmemBytes = rvqs::kSmemBytes;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = rvqs::kCtas;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (ensure_dynamic_smem(reinterpret_cast<const void*>(rvq_stack_kernel), rvqs::kSmemBytes) != 0 ||
-      cudaFuncSetAttribute(rvq_stack_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, rvq_stack_kernel, &cfg) != cudaSuccess) {
-    (void)cudaGetLastError();
-    n = 0;
-  }
-  if (dev < kMaxDev) known[dev] = n + 1;
-  return n;
+  const int n = slots.get(dev, [] {
+    if (ensure_dynamic_smem(reinterpret_cast<const void*>(rvq_stack_kernel), rvqs::kSmemBytes) != 0 ||
+        cudaFuncSetAttribute(rvq_stack_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return -1;
+    }
+    return resident_clusters(rvq_stack_kernel, rvqs::kThreads, rvqs::kSmemBytes, rvqs::kCtas);
+  });
+  return n > 0 ? n : 0;
 }
 }  // namespace
 
