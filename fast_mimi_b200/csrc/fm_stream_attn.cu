@@ -24,7 +24,7 @@
 // are requested before the wait for it.  A block has an item's ring rows in shared memory before it stores that item's
 // new rows, and no other block touches its (stream, head): the ring is updated in place.
 //
-// While the heads of every stream have blocks of their own at the same time (up to 15 streams) the kernel goes on to the output
+// While the heads of every stream have blocks of their own at the same time (up to 15 streams on a B200) the kernel goes on to the output
 // projection, x1 = residual + scale * core W_o^T: the eight blocks of a stream are a cluster, hand each other their heads'
 // rows through distributed shared memory, and each multiplies them with its 64 rows of W_o, which it asked for before the wait.  As
 // a kernel of its own the projection of a few rows was 4.6 us, a launch and a first load around 0.3 us of products
@@ -32,6 +32,7 @@
 #include <type_traits>
 
 #include "fm_common.cuh"
+#include "fm_device_fact.h"
 #include "fm_kernels.h"
 #include "fm_launch.h"
 #include "fm_warp_mma.cuh"
@@ -489,9 +490,19 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   if (ctl->abort) __nanosleep(20000);
 }
 
-// With 64 KB of W_o a block fills an SM, and the device holds 15 clusters of eight such blocks: a sixteenth stream would wait for a
-// second wave (4 us a layer, what the projection saves: 16 streams 191 us with its own launch).
-bool stream_attn_projects(int S, int T) { return S <= 15 && S * 8 <= sm_count() && T <= stream::kMaxT; }
+// With 64 KB of W_o a block fills an SM; as many streams as the device holds clusters of eight such blocks at once (15 on a B200), since
+// one more waits for a second wave (4 us a layer, what the projection saves).  GPU time of eight FP32 layers on full rings, a kernel of
+// its own -> here: 1 stream of one frame 149.9 -> 125, 15 streams of 1, 2 and 8 frames 167.5 -> 155, 183.0 -> 160 and 197.9 -> 182.
+bool stream_attn_projects(int S, int T) {
+  static DeviceFact clusters;
+  int dev = 0;
+  if (T > stream::kMaxT || cudaGetDevice(&dev) != cudaSuccess) return false;
+  return S <= clusters.get(dev, [] {
+    const auto kern = stream_attn_kernel<__half, true>;        // the one for BF16 values takes as much
+    const int bytes = stream::smem_bytes(1, true);
+    return ensure_dynamic_smem(reinterpret_cast<const void*>(kern), bytes) == 0 ? resident_clusters(kern, stream::kThreads, bytes, 8) : -1;
+  });
+}
 
 int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k, void* ring_v, void* out, int S, int T,
                        int past, int slots, int window, float scale, int value_is_fp16, int* status,
