@@ -188,6 +188,55 @@ def test_output_projection_behind_the_heads_of_a_stream(T, past, dtype, value_dt
 
 
 @pytest.mark.parametrize("T", [1, 8])
+@pytest.mark.parametrize("past", [0, 90, 700])
+@pytest.mark.parametrize("dtype,value_dtype", [(torch.float32, torch.float16), (torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float16),
+                                               (torch.float16, torch.float16)])
+def test_live_streams_against_64_bits(T, past, dtype, value_dtype):
+    """A layer's call for 15 streams (output projection behind the attention) and for 16 (a kernel of its own), from the parameters, the
+    rings and the input as they are held, against the same in 64 bits.  FP32 streams: 2e-3 of what the layer adds, the bar of the
+    layer without a cache.  16-bit streams are rounded twice on the way (2^-9 BF16, 2^-11 FP16 each at most), which covers
+    what the branches add to that.  Both routes round alike but for the order of FP32 sums: neither is 5 % further off."""
+    import fast_mimi_b200 as fm
+    window = slots = 250
+    layer = fm.MimiTransformerLayerB200(value_dtype=value_dtype).cuda()
+    layer.load_state_dict(_layer_params(90 + T + past), strict=True)
+    layer = layer.to(dtype).requires_grad_(False)
+    g = torch.Generator(device="cuda").manual_seed(past + T)
+    x = torch.randn(16, T, 512, device="cuda", generator=g).to(dtype)
+    cos, sin = fm.rope_tables(torch.arange(past, past + T, device="cuda")[None])
+    first = fm.MimiKVRing(1, 16, window, value_dtype=value_dtype)
+    for t in (first.ring_k, first.ring_v):
+        t.normal_(generator=g)
+    held = [t[0].double() for t in (first.ring_k, first.ring_v)]                     # [16, 8, slots, 64]
+    got = {}
+    for n in (15, 16):
+        ring = fm.MimiKVRing(1, n, window, value_dtype=value_dtype)
+        ring.ring_k.copy_(first.ring_k[:, :n])
+        ring.ring_v.copy_(first.ring_v[:, :n])
+        ring.advance(0, past)
+        got[n] = layer(x[:n], None, ring, (cos, sin))[0][:15].double()
+    p = {k: v.double() for k, v in layer.state_dict().items()}
+    xd = x.double()
+    norm = lambda t, name: torch.nn.functional.layer_norm(t, (512,), p[name + ".weight"], p[name + ".bias"], 1e-5)
+    h = norm(xd, "input_layernorm")
+    q, k, v = ((h @ p[f"self_attn.{n}_proj.weight"].T).view(16, T, 8, 64).transpose(1, 2) for n in "qkv")
+    turn = lambda t: t * cos.double()[:, None] + O.rotate_half(t) * sin.double()[:, None]
+    at = torch.arange(max(0, past - window + 1), past, device="cuda")
+    keys, values = torch.cat((held[0][:, :, at % slots], turn(k)), 2), torch.cat((held[1][:, :, at % slots], v), 2)
+    pos = torch.cat((at, torch.arange(past, past + T, device="cuda")))
+    new = pos[-T:, None]
+    seen = (pos[None] <= new) & (pos[None] > new - window)
+    core = torch.softmax((turn(q) @ keys.transpose(-1, -2) * 0.125).masked_fill(~seen, float("-inf")), -1) @ values
+    x1 = xd + core.transpose(1, 2).reshape(16, T, 512) @ p["self_attn.o_proj.weight"].T * p["self_attn_layer_scale.scale"]
+    y = x1 + torch.nn.functional.gelu(norm(x1, "post_attention_layernorm") @ p["mlp.fc1.weight"].T) @ p["mlp.fc2.weight"].T * p["mlp_layer_scale.scale"]
+    base = xd[:15] if dtype == torch.float32 else torch.zeros_like(xd[:15])
+    off = {n: O.rel_l2(got[n] - base, y[:15] - base) for n in got}
+    assert max(off.values()) < {torch.float32: 2e-3, torch.bfloat16: 2 ** -8, torch.float16: 2 ** -10}[dtype], off
+    assert max(off.values()) < 1.05 * min(off.values()), off
+    fm.check_status()
+
+
+@pytest.mark.parametrize("T", [1, 8])
 @pytest.mark.parametrize("streams", [1, 15, 16])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 def test_live_streams_without_layer_scales(streams, T, dtype):
