@@ -100,7 +100,8 @@ int fm_band_attn_prefill_bf16(const void* q, const void* k, const void* v, void*
  * [B, 8, T, 64] of in_dtype (0 BF16, 1 FP16, 2 FP32), last dimension contiguous, 16-byte aligned.
  *   strides   HOST array of nine: batch, head, frame strides of q, k, v in values (multiples of 16 bytes)
  *   q/k/v_ws  [B, T, 512] 16 bit: the converted tensors; NULL for one that already is frame-major and of the right type
- *             (BF16 for q and k, value_dtype for v); not written where the attention kernel rounds FP32 tensors itself
+ *             (BF16 for q and k, value_dtype for v); not written where the attention kernel rounds FP32 tensors itself (FP32
+ *             result, T > 256, 129 < window <= 257, five to seven query tiles of 128 per SM and more)
  *   out16     [B, T, 512] value_dtype; out32 [B, T, 512] FP32 or NULL.  With out32 the result goes there, and out16 is a
  *             workspace that may be NULL where T > 256 and 129 < window <= 257 */
 int fm_window_attention(const void* q, const void* k, const void* v, int in_dtype, const long long* strides, void* q_ws, void* k_ws,
@@ -232,8 +233,8 @@ int fm_upsample2_channels_f32(const float* x, const float* w, float* y, int B, i
  * therefore keep FP32 accuracy. */
 int fm_split_half(const float* x, void* hi, void* lo, long long n, void* stream);
 
-/* The three calls below for a whole stack (src/fast_mimi/model.py:2408-2429), as one chain of dependent launches:
- * or, for few vectors without n_candidates, as one kernel:
+/* The three calls below for a whole stack (src/fast_mimi/model.py:2408-2429): as one chain of dependent launches, or, for few
+ * vectors without n_candidates, as one kernel that leaves the workspaces alone.
  *   residual     [rows, 256] FP32, the stack's input; contents undefined afterwards
  *   residual16   [rows, 256] FP16, tau [rows], records [rows, n_codes / 64] x 16 B: workspaces
  *   codebooks(16) [layers, n_codes, 256], e_sq [layers, n_codes], e_max [layers] in HOST memory
