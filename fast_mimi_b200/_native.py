@@ -25,6 +25,11 @@ class LayerParams(ctypes.Structure):
                 ("scale", _F), ("window", _I), ("stream_dtype", _I), ("value_dtype", _I), ("ffn", _I), ("weights_settled", _I), ("vec_dtype", _I)]
 
 
+class RvqStack(ctypes.Structure):
+    """``fm_rvq_stack`` of the header."""
+    _fields_ = [("residual", _P), ("codebooks16", _P), ("codebooks", _P), ("e_sq", _P), ("e_max", ctypes.POINTER(_F)), ("codes", _P), ("layers", _I)]
+
+
 #: name -> argtypes, in header order.  tests/test_host_logic.py checks this table against the header.
 SIGNATURES: dict[str, list] = {
     "fm_abi_version": [],
@@ -43,6 +48,7 @@ SIGNATURES: dict[str, list] = {
     "fm_upsample2_f32": [_P, _P, _P, _I, _I, _I, _P],
     "fm_split_half": [_P, _P, _P, _LL, _P],
     "fm_rvq_encode_f32": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _LL, _I, _I, _F, _P, _P],
+    "fm_rvq_encode_stacks_f32": [ctypes.POINTER(RvqStack), _I, _P, _P, _P, _LL, _I, _F, _P, _P],
     "fm_rvq_prepare_f32": [_P, _P, _P, _LL, _F, _F, _P],
     "fm_rvq_candidates_f16": [_P, _P, _P, _P, _P, _LL, _I, _P, _P],
     "fm_rvq_select_rec_f32": [_P, _P, _P, _P, _P, _P, _P, _LL, _I, _F, _F, _P, _P],

@@ -283,6 +283,17 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
+// Same shape, 32 columns.
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]),
+      "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
 // Same shape, 8 columns.
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
   asm volatile(
@@ -540,6 +551,10 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
 // kernel whose launch bound leaves every thread R registers may hand registers of warps that need few to warps that
 // need many: the donors shrink first, the receivers' request blocks until the registers are free, so the sum after
 // all requests must not exceed threads x R.
+// How far from the least approximate distance to a codebook's entries the nearest one's may lie (fm_rvq.cu): the relative part is
+// FP16 rounding of both operands, the absolute part residual values below FP16's normal range.
+__device__ __forceinline__ float rvq_margin(float xx, float e_max, float tau_rel) { return tau_rel * sqrtf(xx) * e_max + 3.1e-5f * e_max; }
+
 template <int N> __device__ __forceinline__ void warpgroup_reg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }

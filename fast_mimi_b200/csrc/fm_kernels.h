@@ -174,10 +174,22 @@ int launch_rvq_select_rec(const void* records, const float* codebook, float* res
 int launch_rvq_encode(float* resid, void* resid16, float* tau, void* records, const void* books16, const float* books, const float* e_sq,
                       const float* e_max, long long* codes, int* n_candidates, long long rows, int n_codes, int layers, float tau_rel,
                       int* status, cudaStream_t st);
+// One or two stacks over vectors of their own, the same number of them and of entries per codebook.
+struct RvqStack {
+  float* residual;        // [rows, 256], overwritten
+  const void* books16;    // [layers, n_codes, 256] FP16, FP32
+  const float *books, *e_sq, *e_max;      // e_max [layers] in host memory
+  long long* codes;       // [layers, rows]
+  int layers;
+};
+int launch_rvq_encode_stacks(const RvqStack* stacks, int n_stacks, void* resid16, float* tau, void* records, long long rows, int n_codes,
+                             float tau_rel, int* status, cudaStream_t st);
+// The whole search in one kernel for many vectors (fm_rvq_tiles.cu); the workspaces are left alone.
+bool rvq_tiles_take(const RvqStack* stacks, int n_stacks, long long rows, int n_codes);
+int launch_rvq_tiles(const RvqStack* stacks, int n_stacks, long long rows, int n_codes, float tau_rel, int* status, cudaStream_t st);
 // The whole search in one kernel for few vectors (fm_rvq_stack.cu); nothing but codes is written.
-bool rvq_stack_takes(long long rows, int n_codes, int layers);
-int launch_rvq_stack(const float* x, const void* books16, const float* books, const float* e_sq, const float* e_max, long long* codes,
-                     long long rows, int layers, float tau_rel, int* status, cudaStream_t st);
+bool rvq_stack_takes(const RvqStack* stacks, int n_stacks, long long rows, int n_codes);
+int launch_rvq_stack(const RvqStack* stacks, int n_stacks, long long rows, float tau_rel, int* status, cudaStream_t st);
 int launch_rvq_prepare(const float* x, void* resid16, float* tau, long long rows, float e_max, float tau_rel,
                        cudaStream_t st);
 int launch_rvq_to_half(const float* x, void* y, long long rows, cudaStream_t st);

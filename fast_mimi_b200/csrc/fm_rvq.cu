@@ -164,11 +164,6 @@ rvq_select_kernel(const void* __restrict__ scores, const float* __restrict__ e_s
 // minimum, so the union of the masks of the groups whose minimum is within the margin of the global one contains every
 // true candidate; the extra ones only cost an exact evaluation each.  The margin of a frame depends on its residual
 // norm, which the previous layer's decision kernel (or rvq_prepare_kernel before the first layer) leaves in `tau`.
-__device__ __forceinline__ float rvq_margin(float xx, float e_max, float tau_rel) {
-  // relative part: FP16 rounding of both operands; absolute part: residual values below FP16's normal range
-  return tau_rel * sqrtf(xx) * e_max + 3.1e-5f * e_max;
-}
-
 // Bound by the residual's way through memory and by latency: a frame is a chain of loads (record, entry, store).  So a
 // frame's record and residual are asked for one frame ahead; where one entry alone is a candidate (five frames of six) it has
 // won and its distance is not evaluated; and after the last layer (kLast) the residual is neither updated nor, for those
@@ -454,8 +449,9 @@ int launch_rvq_encode(float* resid, void* resid16, float* tau, void* records, co
                       int* status, cudaStream_t st) {
   if (rows < 0 || rows > 0x7fffffffLL || layers <= 0 || n_codes <= 0 || n_codes % 256 != 0 || n_codes > 2048 || e_max == nullptr) return -1;
   if (rows == 0) return 0;
-  if (n_candidates == nullptr && rvq_stack_takes(rows, n_codes, layers))
-    return launch_rvq_stack(resid, books16, books, e_sq, e_max, codes, rows, layers, tau_rel, status, st);
+  const RvqStack stack = {resid, books16, books, e_sq, e_max, codes, layers};
+  if (n_candidates == nullptr && rvq_tiles_take(&stack, 1, rows, n_codes)) return launch_rvq_tiles(&stack, 1, rows, n_codes, tau_rel, status, st);
+  if (n_candidates == nullptr && rvq_stack_takes(&stack, 1, rows, n_codes)) return launch_rvq_stack(&stack, 1, rows, tau_rel, status, st);
   int rc = launch_rvq_prepare(resid, resid16, tau, rows, e_max[0], tau_rel, st);
   for (int l = 0; l < layers && rc == 0; ++l) {
     const size_t entry0 = static_cast<size_t>(l) * n_codes;
@@ -468,6 +464,23 @@ int launch_rvq_encode(float* resid, void* resid16, float* tau, void* records, co
                                last ? 0.f : e_max[l + 1], tau_rel, status, st, 1, last);
   }
   return rc;
+}
+
+int launch_rvq_encode_stacks(const RvqStack* stacks, int n_stacks, void* resid16, float* tau, void* records, long long rows, int n_codes,
+                             float tau_rel, int* status, cudaStream_t st) {
+  if (stacks == nullptr || n_stacks < 1 || n_stacks > 2 || rows < 0) return -1;
+  if (rows == 0) return 0;
+  for (int i = 0; i < n_stacks; ++i)
+    if (stacks[i].layers <= 0 || stacks[i].e_max == nullptr) return -1;
+  if (rvq_stack_takes(stacks, n_stacks, rows, n_codes)) return launch_rvq_stack(stacks, n_stacks, rows, tau_rel, status, st);
+  if (rvq_tiles_take(stacks, n_stacks, rows, n_codes)) return launch_rvq_tiles(stacks, n_stacks, rows, n_codes, tau_rel, status, st);
+  for (int i = 0; i < n_stacks; ++i) {
+    const RvqStack& s = stacks[i];
+    const int rc = launch_rvq_encode(s.residual, resid16, tau, records, s.books16, s.books, s.e_sq, s.e_max, s.codes, nullptr, rows, n_codes,
+                                     s.layers, tau_rel, status, st);
+    if (rc != 0) return rc;
+  }
+  return 0;
 }
 
 int launch_rvq_prepare(const float* x, void* resid16, float* tau, long long rows, float e_max, float tau_rel,

@@ -11,7 +11,8 @@
 //              (distance, index) over the cluster wins
 //   residual   every block subtracts the winner for itself: a warp holds its two vectors in registers all along
 // so a layer crosses the cluster twice, and nothing but codes is written.  63 vectors: 7 layers 66 -> 55 us, 31 layers 273 -> 219
-// us, and 16 launches less for stacks of 1 and 7 layers, 18 otherwise (a 5 s utterance end to end, bound by the host, 200 -> 183 us).  Of the 12300 cycles of a layer the
+// us, and 16 launches less for stacks of 1 and 7 layers, 18 otherwise (a 5 s utterance end to end, bound by the host, 200 -> 183 us;
+// both stacks as two rows of one grid, which the device runs side by side up to three clusters each, 182 -> 169).  Of the 12300 cycles of a layer the
 // two crossings take 4500, the products 2100 (ldmatrix at the rate of shared memory), the exact distances 1400, the new residual 2700.
 #include "fm_common.cuh"
 #include "fm_device_fact.h"
@@ -51,18 +52,25 @@ __device__ __forceinline__ void st_cluster_u64(uint32_t addr, unsigned long long
 }  // namespace rvqs
 
 struct RvqStackArgs {
-  const float* x;              // [rows, 256]
-  const float* books;          // [layers, 2048, 256]
-  const float* e_sq;           // [layers, 2048]
-  long long* codes;            // [layers, rows]
-  int rows, layers;
+  struct Stack {
+    const float* x;            // [rows, 256]
+    const float* books;        // [layers, 2048, 256]
+    const float* e_sq;         // [layers, 2048]
+    long long* codes;          // [layers, rows]
+    int layers;
+    float e_max[rvqs::kMaxLayers];
+  };
+  Stack stack[2];              // a row of the grid has one
+  int rows;
   float tau_rel;
-  float e_max[rvqs::kMaxLayers];
 };
 
 __global__ void __launch_bounds__(rvqs::kThreads, 1)
-rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books, const __grid_constant__ RvqStackArgs a, int* status) {
+rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_constant__ CUtensorMap tmap_books1,
+                 const __grid_constant__ RvqStackArgs args, int* status) {
   using namespace rvqs;
+  const RvqStackArgs::Stack& a = args.stack[blockIdx.y];
+  const CUtensorMap* tmap_books = blockIdx.y == 0 ? &tmap_books0 : &tmap_books1;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem_book = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_x = smem_book + 2 * kBookBytes;                // FP16 residuals: four chunks of 64 dimensions, 32 rows each
@@ -72,14 +80,14 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books, const __grid_co
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = static_cast<int>(threadIdx.x);
   const int rank = static_cast<int>(cluster_cta_rank());
   const int r0 = static_cast<int>(blockIdx.x) / kCtas * kRows;
-  const int n = a.rows - r0 < kRows ? a.rows - r0 : kRows;
+  const int n = args.rows - r0 < kRows ? args.rows - r0 : kRows;
   // read early: a status set before this call leaves the stores out
   const bool skip = status != nullptr && *reinterpret_cast<volatile int*>(status) != 0;
   auto load_book = [&](int l) {
     uint8_t* dst = smem_book + (l & 1) * kBookBytes;
     mbar_arrive_expect_tx(&sh->full[l & 1], kBookBytes);
 #pragma unroll
-    for (int kc = 0; kc < kDim / 64; ++kc) tma_load_2d(dst + kc * kChunkBytes, &tmap_books, &sh->full[l & 1], kc * 64, l * kCodes + rank * kEntries);
+    for (int kc = 0; kc < kDim / 64; ++kc) tma_load_2d(dst + kc * kChunkBytes, tmap_books, &sh->full[l & 1], kc * 64, l * kCodes + rank * kEntries);
   };
   if (tid == 0) {
     mbar_init(&sh->full[0], 1);
@@ -120,7 +128,7 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books, const __grid_co
       exact[0] = make_float4(x[i][0], x[i][1], x[i][2], x[i][3]);
       exact[1] = make_float4(x[i][4], x[i][5], x[i][6], x[i][7]);
       if (lane == 0) {
-        sh->margin[f] = a.tau_rel * sqrtf(xx) * a.e_max[l] + 3.1e-5f * a.e_max[l];
+        sh->margin[f] = rvq_margin(xx, a.e_max[l], args.tau_rel);
         sh->best_in[f] = ~0ull;
       }
     }
@@ -235,7 +243,7 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books, const __grid_co
       const bool none = best == ~0ull;                         // a residual that is not finite: no candidate
       const int j = none ? 0 : static_cast<int>(best & 0xffffffffu);
       if (rank == 0 && lane == 0 && f < n && !skip) {
-        a.codes[static_cast<size_t>(l) * a.rows + r0 + f] = j;
+        a.codes[static_cast<size_t>(l) * args.rows + r0 + f] = j;
         if (none && status != nullptr) atomicMax(status, static_cast<int>(kErrNonFinite));
       }
       if (l + 1 < a.layers) {
@@ -274,32 +282,41 @@ int stack_slots() {
 
 // As many vectors as the device's clusters hold at once (7 x 32 on a B200): a second wave costs as much as the first, the chain
 // next to nothing more (7 layers of 224 vectors 55 us here, 72 there; 225 vectors 99 and 70).
-bool rvq_stack_takes(long long rows, int n_codes, int layers) {
-  return n_codes == rvqs::kCodes && layers <= rvqs::kMaxLayers && rows <= static_cast<long long>(rvqs::kRows) * stack_slots();
+// Two stacks are two rows of one grid, whether or not the device holds both at once.
+bool rvq_stack_takes(const RvqStack* stacks, int n_stacks, long long rows, int n_codes) {
+  for (int i = 0; i < n_stacks; ++i)
+    if (stacks[i].layers > rvqs::kMaxLayers) return false;
+  return n_codes == rvqs::kCodes && rows <= static_cast<long long>(rvqs::kRows) * stack_slots();
 }
 
-int launch_rvq_stack(const float* x, const void* books16, const float* books, const float* e_sq, const float* e_max, long long* codes,
-                     long long rows, int layers, float tau_rel, int* status, cudaStream_t st) {
+int launch_rvq_stack(const RvqStack* stacks, int n_stacks, long long rows, float tau_rel, int* status, cudaStream_t st) {
   using namespace rvqs;
-  if (x == nullptr || books16 == nullptr || books == nullptr || e_sq == nullptr || codes == nullptr || !(tau_rel >= 0.f)) return -1;
-  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(books) | reinterpret_cast<uintptr_t>(books16)) & 15u) return -3;
+  if (n_stacks < 1 || n_stacks > 2 || !(tau_rel >= 0.f)) return -1;
   RvqStackArgs a = {};
-  a.x = x;
-  a.books = books;
-  a.e_sq = e_sq;
-  a.codes = codes;
-  a.rows = static_cast<int>(rows);
-  a.layers = layers;
-  a.tau_rel = tau_rel;
-  for (int l = 0; l < layers; ++l) {
-    if (!(e_max[l] >= 0.f)) return -1;
-    a.e_max[l] = e_max[l];
+  CUtensorMap maps[2];
+  for (int i = 0; i < n_stacks; ++i) {
+    const RvqStack& s = stacks[i];
+    if (s.residual == nullptr || s.books16 == nullptr || s.books == nullptr || s.e_sq == nullptr || s.codes == nullptr) return -1;
+    if ((reinterpret_cast<uintptr_t>(s.residual) | reinterpret_cast<uintptr_t>(s.books) | reinterpret_cast<uintptr_t>(s.books16)) & 15u) return -3;
+    RvqStackArgs::Stack& d = a.stack[i];
+    d.x = s.residual;
+    d.books = s.books;
+    d.e_sq = s.e_sq;
+    d.codes = s.codes;
+    d.layers = s.layers;
+    for (int l = 0; l < s.layers; ++l) {
+      if (!(s.e_max[l] >= 0.f)) return -1;
+      d.e_max[l] = s.e_max[l];
+    }
+    const int rc = encode_rows_16bit(&maps[i], s.books16, static_cast<uint64_t>(s.layers) * kCodes, kDim, kEntries, 64);
+    if (rc != 0) return rc;
   }
-  CUtensorMap map;
-  const int rc = encode_rows_16bit(&map, books16, static_cast<uint64_t>(layers) * kCodes, kDim, kEntries, 64);
-  if (rc != 0) return rc;
-  const int clusters = static_cast<int>((rows + kRows - 1) / kRows);
-  return launch_kernel(rvq_stack_kernel, dim3(clusters * kCtas), kThreads, kSmemBytes, st, kCtas, 0, map, a, status);
+  if (n_stacks == 1) maps[1] = maps[0];
+  a.rows = static_cast<int>(rows);
+  a.tau_rel = tau_rel;
+  const unsigned clusters = static_cast<unsigned>((rows + kRows - 1) / kRows);
+  return launch_kernel(rvq_stack_kernel, dim3(clusters * kCtas, static_cast<unsigned>(n_stacks)), kThreads, kSmemBytes, st, kCtas, 0, maps[0], maps[1],
+                       a, status);
 }
 
 }  // namespace fm

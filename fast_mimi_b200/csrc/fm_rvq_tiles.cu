@@ -1,0 +1,651 @@
+// Residual vector quantisation of many vectors: all layers of one or two stacks in one kernel (sm_100a).  Same decisions as the
+// chain of products and decision kernels in fm_rvq.cu (src/fast_mimi/model.py:2277-2291, :2408-2429).
+//
+// That chain is bound by what lies between its products: records (512 B a frame and layer) and residuals (FP32 and FP16, 2.5 KB)
+// go through memory, and neither kernel's units are busy while the other runs.  Here a pair of blocks owns 256 vectors through
+// their layers: FP32 residuals in tensor memory beside the accumulators, their FP16 copies, the products' A operand, in shared
+// memory.  The codebooks stream past them, one entry per vector and layer is fetched in FP32, and nothing but codes is written.
+// (Residuals in memory cost 384 KB of L2 traffic a layer and block, 15000 cycles; two tiles of 256 vectors a pair, in turn or side by
+// side, leave no room for them on the chip.)
+//
+// A score has to cost little: 128 x 2048 of them a layer and block cross four schedulers while the tensor core makes them in 17400
+// cycles.  So |e|^2 is part of the product (sixteen more columns of K: -|e|^2 / 2 in three FP16 parts against a power of two), and
+// x.e - |e|^2 / 2 is only compared: the largest of 32 against the largest that the four threads of a vector have seen so far, and
+// one by one only where eight of them come within the margin of that.  What does is listed and decided at the end of the layer by
+// exact FP32 distances.
+//
+// Of the 46000 cycles that a layer takes 28000 are scores (the tensor core issues for 18000 of them; a thread looks at 64 scores in
+// 2100, for 2176 of products), 3000 the candidates, 6500 the exact distances of the one vector in seven that has several, 4000 the new
+// residuals (a thread reads a quarter of its vector's entry, sector by sector), 4000 until the next scores arrive.
+//
+// Warps 0-15: scores, decisions, residuals.  Warp 16: codebooks.  Warp 17: MMA (leader block only).  Warps 18, 19: -|e|^2 / 2.
+#include <math.h>
+
+#include "fm_common.cuh"
+#include "fm_kernels.h"
+#include "fm_launch.h"
+
+namespace fm {
+
+namespace rvqt {
+constexpr int kDim = 256, kBlockM = 128, kTileRows = 2 * kBlockM;
+constexpr int kEpiWarps = 16, kThreads = (kEpiWarps + 4) * 32;
+constexpr int kEpiRegs = 112, kIssueRegs = 32;
+static_assert(512 * kEpiRegs + 128 * kIssueRegs <= kThreads * 96, "register pool of the launch");
+constexpr int kEntries = 128, kShare = 64, kGroup = 32;        // of a step of products; of a thread's share of every other step; looked at at once
+constexpr int kSlices = kDim / 64;                             // of 64 dimensions: of K, and of a vector, one for each of its four threads
+constexpr int kChunkBytes = kBlockM * 128, kXBytes = kSlices * kChunkBytes;
+constexpr int kSliceBytes = kEntries / 2 * 128;                // this block's half of a step's entries, one slice
+constexpr int kStages = 3, kStageBytes = kSlices * kSliceBytes;
+constexpr int kOnesBytes = kBlockM * 32, kTailBytes = kEntries / 2 * 32;       // sixteen more columns of K, rows of 32 bytes
+constexpr int kTails = 4;
+constexpr int kList = 8;                                       // candidates that a thread remembers
+constexpr int kMany = 255;                                     // ... or more than that: every entry is one
+constexpr int kBatch = 8, kBatchPitch = kDim + 4;               // of 32 vectors, how many are decided exactly at once; floats from one to the next
+constexpr int kMaxLayers = 32, kMaxPairs = 80;
+constexpr int kTmemCols = 512, kResidual = 2 * kEntries;       // columns: two accumulators, then the residuals
+
+struct Stack {
+  float* x;                    // [rows, 256]: the vectors, overwritten with residuals where there is another layer
+  const float* books;          // [layers, n_codes, 256]
+  const float* e_sq;           // [layers, n_codes]
+  long long* codes;            // [layers, rows]
+  int layers;
+  float e_max[kMaxLayers];
+  float unit[kMaxLayers];      // power of two that -|e|^2 / 2 is a multiple of
+};
+struct Args {
+  Stack stack[2];
+  int rows, n_codes;
+  float tau_rel;
+  int first[2][kMaxPairs + 1];         // pair i has the tiles first[s][i] .. first[s][i + 1] of stack s
+};
+
+// What a pair works on: its tiles of the first stack, then those of the second, layer by layer.
+struct Walk {
+  int next, end, next1, end1;
+  int stack, tile, layer, layers;
+  bool alive;
+  __device__ __forceinline__ Walk(const Args& a, int pair) {
+    next = a.first[0][pair];
+    end = a.first[0][pair + 1];
+    next1 = a.first[1][pair];
+    end1 = a.first[1][pair + 1];
+    open(a);
+  }
+  __device__ __forceinline__ void open(const Args& a) {
+    stack = next < end ? 0 : 1;
+    alive = stack == 0 || next1 < end1;
+    tile = stack == 0 ? next++ : next1++;
+    layer = 0;
+    layers = stack == 0 ? a.stack[0].layers : a.stack[1].layers;
+  }
+  __device__ __forceinline__ void step(const Args& a) {
+    if (++layer == layers) open(a);
+  }
+};
+
+struct Shared {
+  uint64_t full[kStages], empty[kStages];      // full: in the leader, bytes of both blocks
+  uint64_t acc_full[2], acc_empty[2];          // acc_empty: in the leader, the epilogue warps of both blocks
+  uint64_t x_ready;                            // in the leader: both blocks' residuals are in place
+  uint64_t tail_full[kTails], tail_empty[kTails];        // tail_full: in the leader, both blocks' -|e|^2 / 2 of a step
+  uint32_t tmem_base, skip;
+  CtaCtl ctl;
+  Stack stack[2];
+  alignas(16) float lead[kBlockM][4];          // largest scores of a vector's four threads so far
+  alignas(16) float square[kBlockM][4];        // of a vector's four slices
+  uint32_t list[kBlockM][4][kList];            // their candidates: a score, rounded up to 21 bits, and the entry
+  alignas(4) uint8_t listed[kBlockM][4];
+  uint16_t winner[kBlockM];                    // where distances decided
+  alignas(16) float exact[4][kBatch][kBatchPitch];
+};
+constexpr int kSmemBytes = 1024 + kXBytes + kStages * kStageBytes + kOnesBytes + kTails * kTailBytes + static_cast<int>(sizeof(Shared));
+static_assert(kSmemBytes <= 232448, "shared memory");
+
+// Bar of the four warps that share a lane group of tensor memory, i.e. 32 vectors.
+__device__ __forceinline__ void team_sync(int lg) {
+  __syncwarp();
+  asm volatile("bar.sync %0, 128;" ::"r"(lg + 1) : "memory");
+}
+__device__ __forceinline__ void warp_vote() {
+  asm volatile("{\n\t.reg .b32 r;\n\t.reg .pred p;\n\tsetp.eq.u32 p, 0, 0;\n\tvote.sync.ballot.b32 r, p, 0xffffffff;\n\t}" ::: "memory");
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ void load_global8(const float* p, float (&v)[8]) {      // one sector; p 32-byte aligned
+  asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+               : "l"(p));
+}
+// The sixteen columns' descriptor: rows of 32 bytes, 32-byte swizzle, eight rows are 256 bytes.
+__device__ __forceinline__ uint64_t tail_desc(uint32_t smem_addr) {
+  return static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(1) << 16) | (static_cast<uint64_t>(256 >> 4) << 32) |
+         (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(6) << 61);
+}
+// A score that is no smaller, in the upper 21 bits.
+__device__ __forceinline__ uint32_t round_up(float v) {
+  const uint32_t b = __float_as_uint(v);
+  return ((b >> 31) != 0u ? b : b + 2047u) & ~2047u;
+}
+}  // namespace rvqt
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(rvqt::kThreads, 1)
+rvq_tiles_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_constant__ CUtensorMap tmap_books1,
+                 const __grid_constant__ rvqt::Args a, uint32_t idesc, int* status) {
+  using namespace rvqt;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem_x = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem_stage = smem_x + kXBytes;
+  uint8_t* smem_ones = smem_stage + kStages * kStageBytes;     // the sixteen columns of A
+  uint8_t* smem_tail = smem_ones + kOnesBytes;                 // and of B, of the steps in flight
+  Shared* sh = reinterpret_cast<Shared*>(smem_tail + kTails * kTailBytes);
+  CtaCtl* ctl = &sh->ctl;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_cta_rank();
+  const bool leader = rank == 0;
+  const int pair = static_cast<int>(blockIdx.x >> 1);
+  const int n_steps = a.n_codes / kEntries;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(&sh->full[i], 1);
+      mbar_init(&sh->empty[i], 1);
+    }
+    mbar_init(&sh->x_ready, 2 * kEpiWarps);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&sh->acc_full[i], 1);
+      mbar_init(&sh->acc_empty[i], kEpiWarps);       // half of the warps of either block
+    }
+    for (int i = 0; i < kTails; ++i) {
+      mbar_init(&sh->tail_full[i], 4);
+      mbar_init(&sh->tail_empty[i], 1);
+    }
+    ctl->abort = 0;
+    sh->skip = (status != nullptr && *reinterpret_cast<volatile int*>(status) != 0) ? 1u : 0u;
+    fence_mbar_init();
+  }
+  for (int i = static_cast<int>(threadIdx.x); i < kTails * kTailBytes / 16; i += kThreads) reinterpret_cast<uint4*>(smem_tail)[i] = make_uint4(0u, 0u, 0u, 0u);
+  fence_proxy_async_smem();
+  if (threadIdx.x == 0) sh->stack[0] = a.stack[0];
+  if (threadIdx.x == 32) sh->stack[1] = a.stack[1];
+  if (warp == kEpiWarps) {
+    tmem_alloc_pair(&sh->tmem_base, kTmemCols);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = sh->tmem_base;
+  const bool skip = ld_shared_cluster_u32(map_to_cta(smem_u32(&sh->skip), 0)) != 0;
+
+  if (skip) {
+    // a kernel in front already reported an error through this status word: do nothing
+  } else if (warp >= kEpiWarps) {
+    warpgroup_reg_dec<kIssueRegs>();
+    if (warp == kEpiWarps && lane == 0) {
+      // ---------------------------------------------------------- codebooks
+      tma_prefetch_desc(&tmap_books0);
+      tma_prefetch_desc(&tmap_books1);
+      int stage = 0;
+      uint32_t phase = 0;
+      for (Walk w(a, pair); w.alive; w.step(a)) {
+        const CUtensorMap* map = w.stack == 0 ? &tmap_books0 : &tmap_books1;
+        const int row0 = w.layer * a.n_codes + static_cast<int>(rank) * (kEntries / 2);
+#pragma unroll 1
+        for (int nt = 0; nt < n_steps; ++nt) {
+          mbar_wait(&sh->empty[stage], phase ^ 1u, ctl, status, kErrWaitConsumer);
+          if (leader) mbar_arrive_expect_tx(&sh->full[stage], 2 * kStageBytes);
+#pragma unroll
+          for (int kc = 0; kc < kSlices; ++kc)
+            tma_load_2d_pair(smem_stage + stage * kStageBytes + kc * kSliceBytes, map, &sh->full[stage], kc * 64, row0 + nt * kEntries);
+          if (++stage == kStages) { stage = 0; phase ^= 1u; }
+        }
+      }
+    } else if (warp == kEpiWarps + 1 && leader) {
+      // ---------------------------------------------------------- products
+      const bool elected = elect_one();
+      const uint64_t x_desc = umma_desc_sw128(smem_u32(smem_x)), ones_desc = tail_desc(smem_u32(smem_ones));
+      uint32_t step = 0, turn = 0, phase = 0;
+      int stage = 0;
+      for (Walk w(a, pair); w.alive; w.step(a), ++turn) {
+        mbar_wait_cluster(&sh->x_ready, turn & 1u, ctl, status, kErrWaitConsumer);
+#pragma unroll 1
+        for (int nt = 0; nt < n_steps; ++nt, ++step) {
+          const uint32_t buf = step & 1u, parity = (step >> 1) & 1u;
+          mbar_wait(&sh->acc_empty[buf], parity ^ 1u, ctl, status, kErrWaitConsumer);
+          tc_fence_after_sync();
+          const uint32_t d_tmem = tmem_base + buf * kEntries;
+          mbar_wait(&sh->full[stage], phase, ctl, status, kErrWaitTma);
+          const uint32_t tail = step % kTails;
+          mbar_wait_cluster(&sh->tail_full[tail], (step / kTails) & 1u, ctl, status, kErrWaitConsumer);
+          warp_vote();                             // behind a wait alone the products would be issued half as fast
+          tc_fence_after_sync();
+          const uint64_t b_desc = umma_desc_sw128(smem_u32(smem_stage + stage * kStageBytes));
+#pragma unroll
+          for (int k = 0; k < 4 * kSlices; ++k)
+            if (elected)
+              tc_mma_ss_pair(d_tmem, x_desc + static_cast<uint64_t>((k / 4) * kChunkBytes >> 4) + 2u * (k % 4),
+                             b_desc + static_cast<uint64_t>((k / 4) * kSliceBytes >> 4) + 2u * (k % 4), idesc, k != 0 ? 1u : 0u);
+          // |e|^2 last: the tensor core cuts every addend to the accumulator's exponent
+          if (elected) {
+            tc_mma_ss_pair(d_tmem, ones_desc, tail_desc(smem_u32(smem_tail + tail * kTailBytes)), idesc, 1u);
+            tc_commit_pair(&sh->acc_full[buf], 3);
+            tc_commit_pair(&sh->empty[stage], 3);
+            tc_commit_pair(&sh->tail_empty[tail], 3);
+          }
+          if (++stage == kStages) { stage = 0; phase ^= 1u; }
+        }
+      }
+    } else if (warp >= kEpiWarps + 2) {
+      // ---------------------------------------------------------- -|e|^2 / 2 of this block's half of a step's entries, one a thread
+      const uint32_t tail_full_leader = map_to_cta(smem_u32(&sh->tail_full[0]), 0);
+      const int r = (warp - kEpiWarps - 2) * 32 + lane;
+      uint32_t step = 0;
+      for (Walk w(a, pair); w.alive; w.step(a)) {
+        const Stack& s = sh->stack[w.stack];
+        const float* e_sq = s.e_sq + static_cast<size_t>(w.layer) * a.n_codes + rank * (kEntries / 2) + r;
+        const float factor = -0.5f / s.unit[w.layer];
+        float q = __ldg(e_sq);
+#pragma unroll 1
+        for (int nt = 0; nt < n_steps; ++nt, ++step) {
+          const uint32_t tail = step % kTails;
+          const float v = q * factor;
+          if (nt + 1 < n_steps) q = __ldg(e_sq + (nt + 1) * kEntries);
+          const __half hi = __float2half_rn(v);
+          const float rest = v - __half2float(hi);
+          const __half mid = __float2half_rn(rest), low = __float2half_rn(rest - __half2float(mid));
+          mbar_wait(&sh->tail_empty[tail], ((step / kTails) & 1u) ^ 1u, ctl, status, kErrWaitConsumer);
+          // the first eight of the row's sixteen columns (A is the same in both halves)
+          *reinterpret_cast<uint2*>(smem_tail + tail * kTailBytes + r * 32 + (((r >> 2) & 1) << 4)) =
+              make_uint2(__half_as_ushort(hi) | (static_cast<uint32_t>(__half_as_ushort(mid)) << 16), __half_as_ushort(low));
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(tail_full_leader + tail * 8u);
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ scores, decisions, residuals
+    warpgroup_reg_inc<kEpiRegs>();
+    // This thread's vector, its slice of the vector's dimensions, and its share of the entries: one half of every other step.
+    const int lg = warp & 3, q = warp >> 2, row = lg * 32 + lane;
+    const uint32_t acc_empty_leader = map_to_cta(smem_u32(&sh->acc_empty[0]), 0);
+    const uint32_t x_ready_leader = map_to_cta(smem_u32(&sh->x_ready), 0);
+    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(lg * 32) << 16), t_residual = t_row + kResidual + q * 64;
+    auto vector = [&](int tile) { return static_cast<long long>(tile) * kTileRows + static_cast<int>(rank) * kBlockM + row; };
+    // 32 dimensions of the thread's slice enter a layer: in FP32, in FP16, and their squares.
+    auto enter = [&](int part, const float (&x)[32], float& square) {
+#pragma unroll
+      for (int k = 0; k < 32; ++k) square = fmaf(x[k], x[k], square);
+      uint32_t bits[32];
+#pragma unroll
+      for (int k = 0; k < 32; ++k) bits[k] = __float_as_uint(x[k]);
+      tmem_st32(t_residual + part * 32, bits);
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        *reinterpret_cast<uint4*>(smem_x + q * kChunkBytes + sw128_offset(static_cast<uint32_t>(row), static_cast<uint32_t>(part * 4 + c))) =
+            make_uint4(Pack16<__half>::pack(x[8 * c], x[8 * c + 1]), Pack16<__half>::pack(x[8 * c + 2], x[8 * c + 3]),
+                       Pack16<__half>::pack(x[8 * c + 4], x[8 * c + 5]), Pack16<__half>::pack(x[8 * c + 6], x[8 * c + 7]));
+    };
+    auto publish = [&](float square, float unit) {
+      sh->square[row][q] = square;
+      sh->lead[row][q] = -INFINITY;
+      if (q < 2)                                   // this thread's eight of A's sixteen more columns
+        *reinterpret_cast<uint4*>(smem_ones + row * 32 + q * 16) = make_uint4(Pack16<__half>::pack(unit, unit), Pack16<__half>::pack(unit, 0.f), 0u, 0u);
+      tmem_st_wait();
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(x_ready_leader);
+      team_sync(lg);
+    };
+    auto begin_task = [&](const Walk& w) {
+      const Stack& s = sh->stack[w.stack];
+      const long long v = vector(w.tile);
+      float square = 0.f;
+#pragma unroll 1
+      for (int part = 0; part < 2; ++part) {
+        float x[32];
+#pragma unroll
+        for (int k = 0; k < 32; ++k) x[k] = 0.f;
+        if (v < a.rows) {
+          const float4* src = reinterpret_cast<const float4*>(s.x + v * kDim + q * 64 + part * 32);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const float4 f = __ldcg(src + k);
+            x[4 * k] = f.x; x[4 * k + 1] = f.y; x[4 * k + 2] = f.z; x[4 * k + 3] = f.w;
+          }
+        }
+        enter(part, x, square);
+      }
+      publish(square, s.unit[0]);
+    };
+
+    uint32_t use = 0;                              // of this thread's accumulator
+    const uint32_t buf = static_cast<uint32_t>(q >> 1);
+    Walk w(a, pair);
+    if (w.alive) begin_task(w);
+#pragma unroll 1
+    while (w.alive) {
+      const Stack& s = sh->stack[w.stack];
+      const int layer = w.layer;
+      // The margin of the vector (fm_rvq.cu).  Scores are half the distances, and what the tensor core cuts off beside |e|^2 / 2 is
+      // added.  Where the vector is not finite, or none, nothing is a candidate.
+      float margin;
+      {
+        const float4 sq = *reinterpret_cast<const float4*>(sh->square[row]);
+        const float e_max = s.e_max[layer];
+        margin = 0.5f * (rvq_margin((sq.x + sq.y) + (sq.z + sq.w), e_max, a.tau_rel) + 9.5367431640625e-7f * e_max * e_max);
+        if (!(margin < INFINITY) || vector(w.tile) >= a.rows) margin = NAN;
+      }
+      // ---- the scores of this thread's entries
+      {
+        uint32_t* list = sh->list[row][q];
+        volatile float* known = sh->lead[row];
+        float best = -INFINITY;
+        int n = 0;
+#pragma unroll 1
+        for (int nt = static_cast<int>(buf); nt < n_steps; nt += 2, ++use) {
+          // what the other three know is as good a bound, however old
+          float lead = fmaxf(max3(known[0], known[1], known[2]), fmaxf(known[3], best));
+          mbar_wait(&sh->acc_full[buf], use & 1u, ctl, status, kErrWaitMma);
+          tc_fence_after_sync();
+          // both groups of 32 at once, so that the accumulator is free again before they are looked at
+          uint32_t scores[kShare / kGroup][kGroup];
+#pragma unroll
+          for (int part = 0; part < kShare / kGroup; ++part)
+            tmem_ld32(t_row + buf * kEntries + static_cast<uint32_t>((q & 1) * kShare + part * kGroup), scores[part]);
+          tmem_ld_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster_relaxed(acc_empty_leader + buf * 8u);
+#pragma unroll
+          for (int part = 0; part < kShare / kGroup; ++part) {
+            const uint32_t(&raw)[kGroup] = scores[part];
+            float m[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint32_t* r = raw + 8 * j;
+              m[j] = max3(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]));
+              m[j] = max3(m[j], __uint_as_float(r[3]), __uint_as_float(r[4]));
+              m[j] = max3(m[j], __uint_as_float(r[5]), __uint_as_float(r[6]));
+              m[j] = fmaxf(m[j], __uint_as_float(r[7]));
+            }
+            const float top = fmaxf(max3(m[0], m[1], m[2]), m[3]);
+            const bool near = top >= lead - margin;
+            lead = fmaxf(lead, top);
+            best = fmaxf(best, top);
+            if (__any_sync(0xffffffffu, near)) {
+              const float limit = near ? top - margin : NAN;         // of this group's entries
+              uint32_t mask = 0u;
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                if (__any_sync(0xffffffffu, m[j] >= limit)) {
+#pragma unroll
+                  for (int c = 8 * j; c < 8 * j + 8; ++c)
+                    if (__uint_as_float(raw[c]) >= limit) mask |= 1u << c;
+                }
+              }
+              if (n != kMany) {
+                const uint32_t key = round_up(top) | static_cast<uint32_t>(nt * kEntries + (q & 1) * kShare + part * kGroup);
+                for (; mask != 0u; mask &= mask - 1u) {
+                  if (n == kList) {                // those that are out of reach by now go
+                    n = 0;
+#pragma unroll 1
+                    for (int i = 0; i < kList; ++i) {
+                      const uint32_t old = list[i];
+                      if (__uint_as_float(old & ~2047u) >= lead - margin) list[n++] = old;
+                    }
+                    if (n == kList) {
+                      n = kMany;
+                      break;
+                    }
+                  }
+                  list[n++] = key + static_cast<uint32_t>(__ffs(mask) - 1);
+                }
+              }
+              __syncwarp();
+            }
+          }
+          known[q] = best;
+        }
+        sh->listed[row][q] = static_cast<uint8_t>(n);
+      }
+      team_sync(lg);
+      // ---- the decision; every entry that is within the margin of the largest score of all four threads
+      const bool last = layer + 1 == w.layers;
+      const long long v = vector(w.tile);
+      const float* book = s.books + static_cast<size_t>(layer) * a.n_codes * kDim;
+      int code = 0;
+      {
+        const float4 l = *reinterpret_cast<const float4*>(sh->lead[row]);
+        const float limit = fmaxf(max3(l.x, l.y, l.z), l.w) - margin;
+        const int listed = sh->listed[row][q];
+        if (listed != kMany) {
+          int kept = 0;
+          for (int i = 0; i < listed; ++i) {
+            const uint32_t key = sh->list[row][q][i];
+            if (__uint_as_float(key & ~2047u) >= limit) sh->list[row][q][kept++] = key;
+          }
+          sh->listed[row][q] = static_cast<uint8_t>(kept);
+        }
+        team_sync(lg);
+        const uchar4 kept = *reinterpret_cast<const uchar4*>(sh->listed[row]);
+        const int n = kept.x + kept.y + kept.z + kept.w;
+        if (n == 0 && q == 0 && v < a.rows && status != nullptr) atomicMax(status, static_cast<int>(kErrNonFinite));     // not finite
+        if (n == 1) code = static_cast<int>(sh->list[row][kept.x != 0 ? 0 : (kept.y != 0 ? 1 : (kept.z != 0 ? 2 : 3))][0] & 2047u);       // the only candidate has won
+        // The others' residuals cross shared memory, a few vectors at a time, and a warp takes a vector: its candidates' distances,
+        // added up as in fm_rvq.cu.  (The four warps come to the same rounds.)
+#pragma unroll 1
+        for (unsigned open = __ballot_sync(0xffffffffu, n > 1); open != 0u;) {
+          unsigned rest = open;
+#pragma unroll
+          for (int i = 0; i < kBatch; ++i) rest &= rest - 1u;
+          const unsigned batch = open ^ rest;
+          const int place = __popc(batch & ((1u << lane) - 1u));
+          const bool mine = (batch >> lane & 1u) != 0u;
+#pragma unroll
+          for (int part = 0; part < 2; ++part) {
+            uint32_t x[32];
+            tmem_ld32(t_residual + part * 32, x);
+            tmem_ld_wait();
+            if (mine) {
+#pragma unroll
+              for (int c = 0; c < 8; ++c)
+                *reinterpret_cast<uint4*>(&sh->exact[lg][place][q * 64 + part * 32 + 4 * c]) = make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
+            }
+          }
+          team_sync(lg);
+#pragma unroll 1
+          for (int i = q; i < __popc(batch); i += 4) {
+            unsigned behind = batch;
+            for (int k = 0; k < i; ++k) behind &= behind - 1u;
+            const int r = lg * 32 + __ffs(behind) - 1;
+            const uchar4 count = *reinterpret_cast<const uchar4*>(sh->listed[r]);
+            const bool every = count.x == kMany || count.y == kMany || count.z == kMany || count.w == kMany;
+            const int entries = every ? a.n_codes : count.x + count.y + count.z + count.w;
+            // lane k * kList + i: place i of thread k's list
+            const uint32_t key = sh->list[r][lane / kList][lane % kList];
+            unsigned keys = __ballot_sync(0xffffffffu, lane % kList < sh->listed[r][lane / kList]);
+            const float4* src = reinterpret_cast<const float4*>(sh->exact[lg][i]) + 2 * lane;
+            const float4 xa = src[0], xb = src[1];
+            const float x[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+            float least = INFINITY;
+            int win = 0;
+#pragma unroll 1
+            for (int c = 0; c < entries; c += 4) {
+              float e[4][8], sum[4];
+              int j[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const int from = __shfl_sync(0xffffffffu, static_cast<int>(key & 2047u), (__ffs(keys) - 1) & 31);
+                keys &= keys - 1u;
+                j[k] = c + k < entries ? (every ? c + k : from) : -1;
+                if (j[k] >= 0) load_global8(book + static_cast<size_t>(j[k]) * kDim + 8 * lane, e[k]);
+              }
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                sum[k] = 0.f;
+#pragma unroll
+                for (int d = 0; d < 8; ++d) {
+                  const float diff = x[d] - e[k][d];
+                  sum[k] = fmaf(diff, diff, sum[k]);
+                }
+              }
+#pragma unroll
+              for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+              }
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                if (j[k] >= 0 && (sum[k] < least || (sum[k] == least && j[k] < win))) {      // ties go to the lower index (argmin's rule)
+                  least = sum[k];
+                  win = j[k];
+                }
+              }
+            }
+            if (lane == 0) sh->winner[r] = static_cast<uint16_t>(win);
+          }
+          team_sync(lg);
+          if (mine) code = sh->winner[row];
+          open = rest;
+        }
+        if (q == 0 && v < a.rows) s.codes[static_cast<long long>(layer) * a.rows + v] = code;
+      }
+      // ---- the new residuals
+      if (!last) {
+        float square = 0.f;
+#pragma unroll 1
+        for (int part = 0; part < 2; ++part) {
+          uint32_t bits[32];
+          tmem_ld32(t_residual + part * 32, bits);
+          float e[4][8];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) load_global8(book + static_cast<size_t>(code) * kDim + q * 64 + part * 32 + 8 * c, e[c]);
+          tmem_ld_wait();
+          float x[32];
+#pragma unroll
+          for (int i = 0; i < 32; ++i) x[i] = v < a.rows ? __uint_as_float(bits[i]) - e[i >> 3][i & 7] : 0.f;
+          enter(part, x, square);
+        }
+        publish(square, s.unit[layer + 1]);
+      }
+      w.step(a);
+      if (w.alive && last) begin_task(w);
+    }
+  }
+
+  // Neither block may leave (or release tensor memory) while its partner can still signal it.
+  tc_fence_before_sync();
+  __syncthreads();
+  if (ctl->abort) __nanosleep(20000);   // copies that may still be in flight get time to land
+  cluster_sync_all();
+  if (warp == kEpiWarps) {
+    tc_fence_after_sync();
+    tmem_dealloc_pair(tmem_base, kTmemCols);
+  }
+}
+
+namespace {
+// Deals the tiles of both stacks to `pairs` pairs: those of the longer stack evenly, those of the other to whoever has fewest
+// layers so far.
+void deal(rvqt::Args* a, int tiles, int stacks, int pairs) {
+  int load[rvqt::kMaxPairs], count[2][rvqt::kMaxPairs] = {};
+  for (int p = 0; p < pairs; ++p) {
+    count[0][p] = tiles / pairs + (p < tiles % pairs ? 1 : 0);
+    load[p] = count[0][p] * a->stack[0].layers;
+  }
+  for (int left = stacks == 2 ? tiles : 0; left > 0;) {
+    int least = load[0];
+    for (int p = 1; p < pairs; ++p) least = load[p] < least ? load[p] : least;
+    for (int p = 0; p < pairs && left > 0; ++p) {
+      if (load[p] != least) continue;
+      ++count[1][p];
+      load[p] += a->stack[1].layers;
+      --left;
+    }
+  }
+  for (int s = 0; s < 2; ++s) {
+    a->first[s][0] = 0;
+    for (int p = 0; p < pairs; ++p) a->first[s][p + 1] = a->first[s][p] + count[s][p];
+  }
+}
+}  // namespace
+
+// -|e|^2 / 2 has to fit FP16 times the largest power of two that FP16 holds, entries are read by whole sectors, and the time has to
+// pay.  A pair takes 26 us a layer however few vectors it has, whereas the chain spreads a layer over the whole device, so what counts
+// is how evenly tiles come out (1 + 7 layers, in us, chain -> here: 6000 vectors 146 -> 169, 9000 172 -> 171,
+// 16000 248 -> 182, 18944, the most that a tile per pair holds, 276 -> 210, 24000 332 -> 339, 32000 417 -> 385, 48000 645 -> 548, 64000
+// 831 -> 716; 32 layers of 16000 973 -> 711).  The chain's layer is 13.5 us + 1.1 for every 1000 vectors, 1.65 for those past 32000, whose
+// records and residuals no longer stay in L2.
+bool rvq_tiles_take(const RvqStack* stacks, int n_stacks, long long rows, int n_codes) {
+  using namespace rvqt;
+  if (n_stacks < 1 || n_stacks > 2 || rows > 0x7fffffffLL || n_codes % (2 * kEntries) != 0 || n_codes > 2048) return false;
+  int layers = 0, longer = 0;
+  for (int i = 0; i < n_stacks; ++i) {
+    const RvqStack& s = stacks[i];
+    if (s.layers < 1 || s.layers > kMaxLayers || s.e_max == nullptr || (reinterpret_cast<uintptr_t>(s.books) & 31u) != 0) return false;
+    for (int l = 0; l < s.layers; ++l)
+      if (!(s.e_max[l] <= 16384.f)) return false;
+    layers += s.layers;
+    longer = s.layers > longer ? s.layers : longer;
+  }
+  const long long tiles = (rows + kTileRows - 1) / kTileRows, pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
+  const long long even = (tiles * layers + pairs - 1) / pairs, uneven = (tiles + pairs - 1) / pairs * longer;    // layers of the busiest pair
+  const double chain = 13.5 + 1.1e-3 * static_cast<double>(rows) + (rows > 32000 ? 0.55e-3 * static_cast<double>(rows - 32000) : 0.0);
+  return 26.0 * static_cast<double>(even > uneven ? even : uneven) < chain * layers;
+}
+
+int launch_rvq_tiles(const RvqStack* stacks, int n_stacks, long long rows, int n_codes, float tau_rel, int* status, cudaStream_t st) {
+  using namespace rvqt;
+  if (n_stacks < 1 || n_stacks > 2 || rows <= 0 || rows > 0x7fffffffLL || n_codes <= 0 || n_codes > 2048 || n_codes % (2 * kEntries) != 0 || !(tau_rel >= 0.f)) return -1;
+  Args a = {};
+  CUtensorMap maps[2];
+  const int longer = n_stacks == 2 && stacks[1].layers > stacks[0].layers ? 1 : 0;
+  for (int i = 0; i < n_stacks; ++i) {
+    const RvqStack& s = stacks[i ^ longer];
+    if (s.residual == nullptr || s.books16 == nullptr || s.books == nullptr || s.e_sq == nullptr || s.e_max == nullptr || s.codes == nullptr ||
+        s.layers <= 0 || s.layers > kMaxLayers)
+      return -1;
+    if ((reinterpret_cast<uintptr_t>(s.residual) | reinterpret_cast<uintptr_t>(s.books16) | reinterpret_cast<uintptr_t>(s.books) |
+         reinterpret_cast<uintptr_t>(s.e_sq)) & 15u)
+      return -3;
+    Stack& d = a.stack[i];
+    d.x = s.residual;
+    d.books = s.books;
+    d.e_sq = s.e_sq;
+    d.codes = s.codes;
+    d.layers = s.layers;
+    for (int l = 0; l < s.layers; ++l) {
+      if (!(s.e_max[l] >= 0.f)) return -1;
+      d.e_max[l] = s.e_max[l];
+      int exponent = 0;                        // -|e|^2 / 2 in units of the least power of two that keeps it below 2^14
+      frexpf(0.5f * s.e_max[l] * s.e_max[l], &exponent);
+      exponent -= 14;
+      d.unit[l] = ldexpf(1.f, exponent < -14 ? -14 : (exponent > 15 ? 15 : exponent));
+    }
+    const int rc = encode_rows_16bit(&maps[i], s.books16, static_cast<uint64_t>(s.layers) * n_codes, kDim, kEntries / 2, 64);
+    if (rc != 0) return rc;
+  }
+  if (n_stacks == 1) maps[1] = maps[0];
+  a.rows = static_cast<int>(rows);
+  a.n_codes = n_codes;
+  a.tau_rel = tau_rel;
+  const long long tiles = (rows + kTileRows - 1) / kTileRows;
+  int pairs = sm_count() / 2;
+  if (pairs > kMaxPairs) pairs = kMaxPairs;
+  if (pairs < 1) pairs = 1;
+  if (tiles * n_stacks < pairs) pairs = static_cast<int>(tiles) * n_stacks;
+  deal(&a, static_cast<int>(tiles), n_stacks, pairs);
+  const uint32_t idesc = umma_idesc_f16(kTileRows, kEntries, 0, 0, 0, 0);
+  const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(rvq_tiles_kernel), kSmemBytes);
+  if (rc != 0) return rc;
+  return launch_kernel(rvq_tiles_kernel, dim3(static_cast<unsigned>(2 * pairs)), kThreads, kSmemBytes, st, 1, 0, maps[0], maps[1], a, idesc, status);
+}
+
+}  // namespace fm

@@ -621,17 +621,34 @@ class RVQCodebooks:
         self.layers, self.entries = codebooks.shape[0], codebooks.shape[1]
 
 
-def _rvq_search(resid, books: RVQCodebooks, codes, cand, st, resid16=None):
+def _rvq_workspace(rows, entries, device):
+    """FP16 copy of the residuals, margins and candidate records of a search: the memory and where they lie in it."""
+    half, recs = rows * RVQ_DIM * 2, rows * (entries // 64) * 16
+    ws = torch.empty(half + recs + rows * 4, dtype=torch.uint8, device=device)
+    at = ws.data_ptr()
+    return ws, at, at + half + recs, at + half
+
+
+def _rvq_search_stacks(resid, books, codes, st):
+    """Two stacks with codebooks of one size: layers of ``books[i]`` on ``resid[i] [rows, 256]`` float32, which is overwritten, into
+    ``codes[i] [layers, rows]``."""
+    rows, entries = codes[0].shape[1], books[0].entries
+    ws, resid16, tau, records = _rvq_workspace(rows, entries, codes[0].device)
+    stacks = (_native.RvqStack * len(books))(*[
+        (x.data_ptr(), b.half.data_ptr(), b.vectors.data_ptr(), b.sq.data_ptr(), (ctypes.c_float * len(b.e_max))(*b.e_max), c.data_ptr(), len(c))
+        for x, b, c in zip(resid, books, codes)])
+    rc = _native.load().fm_rvq_encode_stacks_f32(stacks, len(books), resid16, tau, records, rows, entries, RVQ_TAU_REL[torch.float32], st, _stream())
+    _native.check(rc, "fm_rvq_encode_stacks_f32")
+
+
+def _rvq_search(resid, books: RVQCodebooks, codes, cand, st):
     """The stack's layers on ``resid [rows, 256]`` float32, which is overwritten, into ``codes [layers, rows]``."""
     layers, rows = codes.shape
-    if resid16 is None:
-        resid16 = torch.empty(rows, RVQ_DIM, dtype=torch.float16, device=resid.device)
-    tau = torch.empty(rows, dtype=torch.float32, device=resid.device)
-    records = torch.empty(rows, books.entries // 64, 4, dtype=torch.int32, device=resid.device)
+    ws, resid16, tau, records = _rvq_workspace(rows, books.entries, resid.device)
     rc = _native.load().fm_rvq_encode_f32(
-        resid.data_ptr(), resid16.data_ptr(), tau.data_ptr(), records.data_ptr(), books.half.data_ptr(), books.vectors.data_ptr(),
-        books.sq.data_ptr(), (ctypes.c_float * len(books.e_max))(*books.e_max), codes.data_ptr(), _ptr(cand), rows, books.entries,
-        layers, RVQ_TAU_REL[torch.float32], st, _stream())          # FP32 accumulators feed the comparison directly
+        resid.data_ptr(), resid16, tau, records, books.half.data_ptr(), books.vectors.data_ptr(), books.sq.data_ptr(),
+        (ctypes.c_float * len(books.e_max))(*books.e_max), codes.data_ptr(), _ptr(cand), rows, books.entries, layers,
+        RVQ_TAU_REL[torch.float32], st, _stream())          # FP32 accumulators feed the comparison directly
     _native.check(rc, "fm_rvq_encode_f32")
 
 
@@ -648,14 +665,14 @@ def rvq_encode(x, books: RVQCodebooks, num_quantizers=None, *, return_candidates
     _need(0 < layers <= books.layers, "num_quantizers out of range")
     rows = x.shape[0]
     resid = x.contiguous().clone()
-    resid16 = torch.empty(rows, RVQ_DIM, dtype=torch.float16, device=x.device)
     codes = torch.empty(layers, rows, dtype=torch.int64, device=x.device)
     cand = torch.empty(layers, rows, dtype=torch.int32, device=x.device) if return_candidates else None
     st = _status_ptr(status, x)
     if scores_dtype is None:
-        _rvq_search(resid, books, codes, cand, st, resid16)
+        _rvq_search(resid, books, codes, cand, st)
         return (codes, cand) if return_candidates else codes
     _need(scores_dtype in RVQ_TAU_REL, "scores_dtype must be None, float16 or float32")
+    resid16 = torch.empty(rows, RVQ_DIM, dtype=torch.float16, device=x.device)
     scores = torch.empty(rows, books.entries, dtype=scores_dtype, device=x.device)
     _native.check(lib.fm_rvq_to_half(resid.data_ptr(), resid16.data_ptr(), rows, _stream()), "fm_rvq_to_half")
     for l in range(layers):

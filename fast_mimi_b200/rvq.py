@@ -147,6 +147,10 @@ class MimiSplitRVQB200:
             parts = self._joint_in_parts()
             if parts is not None:
                 x = ops._linear_parts(frames.parts(), parts, (B * T,), None, mats=2)
+                if self.semantic.books.entries == self.acoustic.books.entries:
+                    ops._rvq_search_stacks(x, (self.semantic.books, self.acoustic.books), (codes[:n_sem], codes[n_sem:]), ops._status_ptr(None, x))
+                    ops.check_status(embeddings.device)
+                    return codes.view(len(codes), B, T)
         self.semantic._encode_frames(frames, codes[:n_sem], x[0])
         if acoustic > 0:
             self.acoustic._encode_frames(frames, codes[n_sem:], x[1])

@@ -233,8 +233,8 @@ int fm_upsample2_channels_f32(const float* x, const float* w, float* y, int B, i
  * therefore keep FP32 accuracy. */
 int fm_split_half(const float* x, void* hi, void* lo, long long n, void* stream);
 
-/* The three calls below for a whole stack (src/fast_mimi/model.py:2408-2429): as one chain of dependent launches, or, for few
- * vectors without n_candidates, as one kernel that leaves the workspaces alone.
+/* The three calls below for a whole stack (src/fast_mimi/model.py:2408-2429): as one chain of dependent launches, or, without
+ * n_candidates, as one kernel that leaves the workspaces alone, for few vectors and for as many as fill the device.
  *   residual     [rows, 256] FP32, the stack's input; contents undefined afterwards
  *   residual16   [rows, 256] FP16, tau [rows], records [rows, n_codes / 64] x 16 B: workspaces
  *   codebooks(16) [layers, n_codes, 256], e_sq [layers, n_codes], e_max [layers] in HOST memory
@@ -242,6 +242,20 @@ int fm_split_half(const float* x, void* hi, void* lo, long long n, void* stream)
 int fm_rvq_encode_f32(float* residual, void* residual16, float* tau, void* records, const void* codebooks16, const float* codebooks,
                       const float* e_sq, const float* e_max, long long* codes, int* n_candidates, long long rows, int n_codes, int layers,
                       float tau_rel, int* status, void* stream);
+
+/* Two stacks (or one) at once, each over vectors of its own, as a split quantiser has them (src/fast_mimi/model.py:2447-2480);
+ * arguments as in fm_rvq_encode_f32, `rows` and `n_codes` the same for both, workspaces shared. */
+typedef struct {
+  float* residual;
+  const void* codebooks16;
+  const float* codebooks;
+  const float* e_sq;
+  const float* e_max;
+  long long* codes;
+  int layers;
+} fm_rvq_stack;
+int fm_rvq_encode_stacks_f32(const fm_rvq_stack* stacks, int n_stacks, void* residual16, float* tau, void* records, long long rows,
+                             int n_codes, float tau_rel, int* status, void* stream);
 
 /* The same layer without the scores' round trip through memory (replaces the same reference lines as
  * fm_rvq_select_f32: src/fast_mimi/model.py:2277-2291, :2420-2427), three calls:

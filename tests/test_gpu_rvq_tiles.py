@@ -1,0 +1,74 @@
+"""The quantiser search of many vectors in one kernel against the chain of products and decision kernels, whose codes it has to give:
+``return_candidates`` asks for the chain."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _books(layers, entries, gen, same=0):
+    e = torch.randn(layers, entries, 256, device="cuda", generator=gen) * (0.6 ** torch.arange(layers, device="cuda").clamp(max=7))[:, None, None]
+    if same:                                     # entries that nothing tells apart: the lowest index wins
+        e[:, 100:100 + same] = e[:, 100:101]
+    return e
+
+
+# A tile is 256 vectors and 74 pairs of blocks take one each: 18944 is the most of a wave; 9217 and 18700 end inside a block's rows.
+@pytest.mark.parametrize("rows,layers,entries,scale", [(9217, 8, 2048, 1.0), (18944, 3, 2048, 1.0), (18700, 5, 1024, 300.0), (33000, 2, 256, 1e-3)])
+def test_codes_equal_the_chains(rows, layers, entries, scale):
+    import fast_mimi_b200 as fm
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    books = fm.ops.RVQCodebooks(_books(layers, entries, gen) * scale)
+    x = torch.randn(rows, 256, device="cuda", generator=gen) * (1.5 * scale)
+    x[5] = 0.0                                   # all margin, no direction
+    want, cand = fm.ops.rvq_encode(x, books, return_candidates=True)
+    assert torch.equal(fm.ops.rvq_encode(x, books), want)
+    assert int(cand.max()) > 1                   # exact distances did decide somewhere
+
+
+@pytest.mark.parametrize("same", [9, 40, 700])   # beyond what a thread, a vector remembers; of every block's entries
+def test_entries_that_are_the_same(same):
+    import fast_mimi_b200 as fm
+    gen = torch.Generator(device="cuda").manual_seed(same)
+    e = _books(2, 2048, gen, same)
+    books = fm.ops.RVQCodebooks(e)
+    x = torch.randn(9000, 256, device="cuda", generator=gen)
+    x[::50] = e[0, 100] * 0.9                    # these want the repeated entry, and again for what is left
+    want = fm.ops.rvq_encode(x, books, return_candidates=True)[0]
+    got = fm.ops.rvq_encode(x, books)
+    assert torch.equal(got, want) and bool((got[0, ::50] == 100).all())
+
+
+@pytest.mark.parametrize("frames", [3100, 23, 70])        # dealt to pairs of blocks; one wave of clusters, two
+def test_both_stacks_of_a_split_quantiser(frames):
+    """1 + 7 layers in one launch against either branch by itself."""
+    import fast_mimi_b200 as fm
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    branch = lambda n: fm.MimiRVQB200(_books(n, 2048, gen), torch.randn(256, 512, 1, device="cuda", generator=gen) * 512 ** -0.5, None)
+    q = fm.MimiSplitRVQB200(branch(1), branch(7))
+    e = torch.randn(3, 512, frames, device="cuda", generator=gen)
+    got = q.encode(e)
+    rows = e.permute(0, 2, 1).reshape(-1, 512)
+    for branch, part in ((q.semantic, got[:1]), (q.acoustic, got[1:])):
+        x = fm.ops.linear_split(rows, fm.ops.split_half(branch.input_proj))
+        want = fm.ops.rvq_encode(x, branch.books, return_candidates=True)[0]
+        assert torch.equal(part.reshape(len(part), -1), want)
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), 1e30])
+def test_a_vector_that_is_not_finite(value):
+    import fast_mimi_b200 as fm
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    books = fm.ops.RVQCodebooks(_books(2, 2048, gen))
+    x = torch.randn(12000, 256, device="cuda", generator=gen)
+    x[4321, 7] = value
+    st = fm.ops.new_status("cuda")
+    got = fm.ops.rvq_encode(x, books, status=st)
+    assert fm.ops.read_status(st) == 105
+    st = fm.ops.new_status("cuda")
+    want = fm.ops.rvq_encode(x, books, return_candidates=True, status=st)[0]
+    assert fm.ops.read_status(st) == 105
+    keep = torch.arange(len(x), device="cuda") != 4321
+    assert torch.equal(got[0, keep], want[0, keep])        # (the chain's later kernels stop at the first error)
