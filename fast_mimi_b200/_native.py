@@ -43,6 +43,9 @@ SIGNATURES: dict[str, list] = {
     "fm_conv_frames_split": [_P, _P, _P, _I, _I, _I, _I, _I, _P],
     "fm_linear_split_f32": [_P, _P, _LL, _I, _P, _P, _P, _LL, _I, _I, _I, _I, _I, _I, _P, _P],
     "fm_linear_split_sum_f32": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P],
+    "fm_split_direct": [_LL, _I, _I],
+    "fm_linear_rows_f32": [_P, _P, _P, _P, _LL, _I, _I, _I, _P, _P],
+    "fm_conv_frames_f32": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "fm_upsample2_channels_f32": [_P, _P, _P, _I, _I, _I, _P],
     "fm_rvq_decode_split": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "fm_upsample2_f32": [_P, _P, _P, _I, _I, _I, _P],

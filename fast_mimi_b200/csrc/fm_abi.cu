@@ -237,6 +237,18 @@ int fm_linear_split_sum_f32(const void* a_hi, const void* a_lo, const void* w_hi
                                  static_cast<cudaStream_t>(stream));
 }
 
+int fm_split_direct(long long rows, int n_out, int k_in) { return fm::split_gemm_takes(rows, n_out, k_in) ? 1 : 0; }
+
+int fm_linear_rows_f32(const float* x, const void* w_hi, const void* w_lo, float* y, long long rows, int n_mats, int n_out, int k_in, int* status,
+                       void* stream) {
+  return fm::launch_split_rows(x, w_hi, w_lo, y, rows, n_mats, n_out, k_in, status, static_cast<cudaStream_t>(stream));
+}
+
+int fm_conv_frames_f32(const float* x, const void* w_hi, const void* w_lo, float* y, int B, int T, int C, int kernel, int stride, int n_out, int* status,
+                       void* stream) {
+  return fm::launch_split_conv(x, w_hi, w_lo, y, B, T, C, kernel, stride, n_out, status, static_cast<cudaStream_t>(stream));
+}
+
 int fm_upsample2_channels_f32(const float* x, const float* w, float* y, int B, int T, int C, void* stream) {
   return fm::launch_upsample2_channels(x, w, y, B, T, C, static_cast<cudaStream_t>(stream));
 }

@@ -134,6 +134,14 @@ int launch_linear_split(const void* a_hi, const void* a_lo, long long a_rows, in
                         cudaStream_t st);
 int launch_linear_split_small(const void* a_hi, const void* w_hi, const SplitLow& low, const SplitRows& map, float* y, int M, int N,
                               int K, int* status, cudaStream_t st);
+// The same from an operand as it lies, split on the way (fm_split_gemm.cu), for many rows: FP32 rows [rows, K], or frames [B, T, C] of
+// a causal convolution.  K a multiple of 128, at least 256.
+// Whether there are rows enough for them to be the faster form.
+bool split_gemm_takes(long long rows, int N, int K);
+int launch_split_rows(const float* x, const void* w_hi, const void* w_lo, float* y, long long rows, int n_mats, int N, int K, int* status,
+                      cudaStream_t st);
+int launch_split_conv(const float* x, const void* w_hi, const void* w_lo, float* y, int B, int T, int C, int kernel, int stride, int N, int* status,
+                      cudaStream_t st);
 // Padded frames of a causal convolution (kernel a multiple of stride), split into FP16 hi + lo parts: clip b has
 // stride * (ceil(T / stride) + kernel / stride - 1) frames of C values (fm_downsample.cu).
 int launch_conv_frames_split(const float* x, void* hi, void* lo, int B, int T, int C, int kernel, int stride, cudaStream_t st);

@@ -700,7 +700,8 @@ def linear_split(x, w_parts, *, status=None):
     ``split_half(w)`` of a float32 ``[N, K]`` weight.  One product over three times K with FP32 accumulation:
     ``hi W_hi + hi W_lo + lo W_hi`` (the dropped ``lo W_lo`` term is below 2^-22 of the result).  K a multiple of 64, N of
     256."""
-    return _linear_parts(split_half(x.contiguous()), w_parts, x.shape[:-1], status)
+    x = x.contiguous()
+    return _linear_rows(x, lambda: split_half(x), w_parts, x.shape[:-1], status)
 
 
 def _check_weight_parts(w_parts, k):
@@ -727,6 +728,21 @@ def _linear_parts(x_parts, w_parts, shape, status, mats=None):
     return y
 
 
+def _linear_rows(x, parts, w_parts, shape, status, mats=None):
+    """``_linear_parts`` from ``x [.., K]`` as it is where there are rows enough, else from its parts, ``parts()``."""
+    w_hi, w_lo = w_parts
+    lib, k, n = _native.load(), x.shape[-1], w_hi.shape[0]
+    rows = x.numel() // k if k else 0
+    if not (rows and x.is_cuda and x.dtype == torch.float32 and lib.fm_split_direct(rows, n, k)):
+        return _linear_parts(parts(), w_parts, shape, status, mats)
+    _check_weight_parts(w_parts, k)
+    y = torch.empty((*shape, n) if mats is None else (mats, *shape, n // mats), dtype=torch.float32, device=x.device)
+    rc = lib.fm_linear_rows_f32(x.data_ptr(), w_hi.data_ptr(), w_lo.data_ptr(), y.data_ptr(), rows, mats or 1, n, k, _status_ptr(status, x),
+                                _stream())
+    _native.check(rc, "fm_linear_rows_f32")
+    return y
+
+
 def downsample_conv(x, w_parts, *, kernel=4, stride=2, status=None):
     """The stride-2 causal, replicate-padded, bias-free convolution after the encoder transformer on frame-major
     activations: ``x [B, T, C]`` float32 -> ``[B, ceil(T / stride), C_out]`` float32.  ``w_parts`` =
@@ -738,6 +754,13 @@ def downsample_conv(x, w_parts, *, kernel=4, stride=2, status=None):
     w_hi, w_lo = w_parts
     _need(w_hi.shape == w_lo.shape and w_hi.shape[1] == kernel * C, f"weight parts must be [C_out, {kernel * C}]")
     t_out = (T + stride - 1) // stride
+    if C % 64 == 0 and stride <= kernel <= 16 and lib.fm_split_direct(B * t_out, w_hi.shape[0], kernel * C):
+        _check_weight_parts(w_parts, kernel * C)
+        y = torch.empty(B, t_out, w_hi.shape[0], dtype=torch.float32, device=x.device)
+        rc = lib.fm_conv_frames_f32(x.data_ptr(), w_hi.data_ptr(), w_lo.data_ptr(), y.data_ptr(), B, T, C, kernel, stride, w_hi.shape[0],
+                                    _status_ptr(status, x), _stream())
+        _native.check(rc, "fm_conv_frames_f32")
+        return y
     if kernel % stride == 0 and (stride * C) % 64 == 0 and B * t_out > 0:
         # frames laid out once with their padding; a row of the product is kernel / stride rows of `stride` frames
         _check_weight_parts(w_parts, kernel * C)

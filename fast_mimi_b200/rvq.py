@@ -18,7 +18,7 @@ from . import ops
 
 
 class _Frames:
-    """Embeddings ``[B, C, T]`` as frame-major float32 rows, with their FP16 hi + lo parts made once for all branches."""
+    """Embeddings ``[B, C, T]`` as frame-major float32 rows; their FP16 hi + lo parts, if asked for, are made once for all branches."""
 
     def __init__(self, embeddings: torch.Tensor) -> None:
         B, _, T = embeddings.shape
@@ -78,7 +78,7 @@ class MimiRVQB200:
         elif self.input_proj is None:
             x = frames.rows.clone()
         elif self._on_tensor_core(self.input_proj):
-            x = ops._linear_parts(frames.parts(), self._in_parts, (len(frames.rows),), None)
+            x = ops._linear_rows(frames.rows, frames.parts, self._in_parts, (len(frames.rows),), None)
         else:
             x = ops.linear_fp32(frames.rows, self.input_proj)
         ops._need(x.shape[1] == ops.RVQ_DIM, "x must be CUDA float32 [rows, 256]")
@@ -146,7 +146,7 @@ class MimiSplitRVQB200:
             self.acoustic._layers(acoustic)
             parts = self._joint_in_parts()
             if parts is not None:
-                x = ops._linear_parts(frames.parts(), parts, (B * T,), None, mats=2)
+                x = ops._linear_rows(frames.rows, frames.parts, parts, (B * T,), None, mats=2)
                 if self.semantic.books.entries == self.acoustic.books.entries:
                     ops._rvq_search_stacks(x, (self.semantic.books, self.acoustic.books), (codes[:n_sem], codes[n_sem:]), ops._status_ptr(None, x))
                     ops.check_status(embeddings.device)

@@ -218,6 +218,17 @@ int fm_linear_split_f32(const void* a_hi, const void* a_lo, long long a_rows, in
 int fm_linear_split_sum_f32(const void* a_hi, const void* a_lo, const void* w_hi, const void* w_lo, float* y, int B, int T, int n_out,
                             int k_in, int* status, void* stream);
 
+/* The same products from FP32 operands as they lie, which are split on the way to the tensor core, for many rows:
+ *   fm_linear_rows_f32   x [rows, k_in] -> y, n_mats matrices [rows, n_out / n_mats] (n_out / n_mats a multiple of 256)
+ *   fm_conv_frames_f32   x [B, T, C] (C a multiple of 64) and a causal convolution of `kernel` frames with replicate padding, its weight
+ *                        as [n_out, kernel * C] -> y [B, ceil(T / stride), n_out] (src/fast_mimi/model.py:2734-2744)
+ * k_in (kernel * C) a multiple of 128, at least 256; y on a 32-byte boundary.  fm_split_direct: 1 where that is the faster form. */
+int fm_split_direct(long long rows, int n_out, int k_in);
+int fm_linear_rows_f32(const float* x, const void* w_hi, const void* w_lo, float* y, long long rows, int n_mats, int n_out, int k_in, int* status,
+                       void* stream);
+int fm_conv_frames_f32(const float* x, const void* w_hi, const void* w_lo, float* y, int B, int T, int C, int kernel, int stride, int n_out, int* status,
+                       void* stream);
+
 /* The stride-2 upsampling that precedes the decoder transformer (MimiModel.upsample: MimiConvTranspose1d(512, 512,
  * kernel 4, stride 2, groups 512, no bias), src/fast_mimi/model.py:2745-2753; its forward trims the last two output
  * frames): x [B, T, C] FP32 frame-major, w [C, 4] FP32 (the ConvTranspose1d weight [C, 1, 4]) -> y [B, 2T, C] FP32,
