@@ -283,3 +283,34 @@ def test_one_kernel_search_reports_a_vector_that_is_not_finite(value):
     assert ops.read_status(status) == 105
     keep = [i for i in range(40) if i != 35]
     assert torch.equal(codes[:, keep], good[:, keep])
+
+
+@pytest.mark.parametrize("layers,n0", [(1, 1), (8, 1), (9, 3), (17, 16), (32, 1)])       # eight codes are on their way at once
+def test_decoded_parts_of_both_stacks(layers, n0):
+    """Sums in the layers' order, bit for bit, as FP16 hi + lo; codes outside a codebook are reported, wherever they stand."""
+    import fast_mimi_b200 as fm
+    g = torch.Generator(device="cuda").manual_seed(layers)
+    B, T, width = 3, 41, 256 if n0 == layers else 512
+    books = [torch.randn(n, e, 256, device="cuda", generator=g) for n, e in ((n0, 256), (max(layers - n0, 1), 512))]
+    codes = torch.randint(0, 256, (B, layers, T), device="cuda", generator=g)
+    want = torch.zeros(B, T, width, device="cuda")
+    for l in range(layers):
+        stack = int(l >= n0)
+        want[..., 256 * stack:256 * stack + 256] += books[stack][l - n0 if stack else l][codes[:, l]]
+
+    def run():
+        hi, lo = (torch.empty(B * T, width, dtype=torch.float16, device="cuda") for _ in range(2))
+        bad = torch.zeros(1, dtype=torch.int32, device="cuda")
+        rc = fm._native.load().fm_rvq_decode_split(codes.data_ptr(), books[0].data_ptr(), books[1].data_ptr() if n0 < layers else None, hi.data_ptr(),
+                                                   lo.data_ptr(), B, T, layers, n0, 256, 512 if n0 < layers else 0, bad.data_ptr(),
+                                                   torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        return hi.view(B, T, width), lo.view(B, T, width), int(bad)
+
+    hi, lo, bad = run()
+    assert bad == 0 and torch.equal(hi, want.half()) and torch.equal(lo, (want - want.half().float()).half())
+    for l, code in ((0, -1), (layers - 1, 512), (layers // 2, 1 << 40)):
+        before = codes[1, l, 7].clone()
+        codes[1, l, 7] = code
+        assert run()[2] == 1
+        codes[1, l, 7] = before
