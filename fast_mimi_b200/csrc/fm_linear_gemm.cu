@@ -505,8 +505,8 @@ static int launch_pairs(const void* a, const void* w, const SplitLow* low, void*
 
 // 256 x 128 units instead of 256 x 256 where they save part of a wave in a call whose rows cross the slab (a residual, a
 // split-precision product): there a half unit costs about half plus 1 / 128 per K chunk of a whole one (its a slices are fetched
-// twice as often).  Without the slab it costs two thirds to three quarters, and no wave that it saves is worth that.  (What one
-// wave of half units would hold, the few-row tiles take.)  Measured, whole -> half units, in us:
+// twice as often).  Without the slab it costs two thirds to three quarters, and no wave that it saves is worth that.  (One wave
+// of them: see one_wave_of_halves.)  Measured, whole -> half units, in us:
 //   residual         K =  512, N =  512, 12000 rows (2 -> 3 waves) 18.8 -> 16.7, 22000 rows (3 -> 5) 31.8 -> 29.1
 //                    K = 1024, N = 1024, FP16, 5000 rows (2 -> 3) 27.2 -> 24.2, 16000 rows (4 -> 7) 38.7 -> 42.9
 //                    K = 2048, N =  512, 14000 rows (2 -> 3) 35.2 -> 36.7, 22000 rows (3 -> 5) 49.9 -> 56.2
@@ -515,6 +515,16 @@ static int launch_pairs(const void* a, const void* w, const SplitLow* low, void*
 static bool half_units(int pair_tiles, int N, int max_pairs, int k_chunks) {
   const int waves256 = (pair_tiles * (N / 256) + max_pairs - 1) / max_pairs, waves128 = (pair_tiles * (N / 128) + max_pairs - 1) / max_pairs;
   return static_cast<long long>(64 + k_chunks) * waves128 < 128ll * waves256;
+}
+
+// Half units that are one wave, for rows that two of the few-row kernel's 128 x 64 blocks on an SM would hold: those fetch half as much
+// again from L2, and the second starts when the first has gone.  With one of them to an SM they are the faster form.  Measured, few-row
+// kernel -> half units, in us: K = 2048, N = 512, FP32 2000 rows (128 blocks) 12.4 -> 13.9, 2500 (160) 13.9 -> 13.9, 3678 (232) 15.7 ->
+// 14.0, 4500 (288) 16.7 -> 14.2, BF16 3678 rows 16.7 -> 14.4; K = 512, N = 512, FP32 3678 rows 8.8 -> 8.3, BF16 9.8 -> 8.5; K = 512,
+// N = 2048, GELU 500 rows (128) 8.0 -> 8.3, 1024 (256) 9.8 -> 8.3.
+static bool one_wave_of_halves(int M, int pair_tiles, int N, int max_pairs) {
+  return pair_tiles * static_cast<long long>(N / 128) <= max_pairs &&
+         static_cast<long long>((M + lin::kBlockM - 1) / lin::kBlockM) * (N / 64) > sm_count();
 }
 
 int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N,
@@ -528,13 +538,14 @@ int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, co
   if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y) |
        reinterpret_cast<uintptr_t>(scale.data) | reinterpret_cast<uintptr_t>(resid)) & 15u)
     return -3;
-  if (out_dtype != 3 && few_row_tiles(M, N))
-    return launch_linear_small(a, w, y, scale, resid, M, N, K, in_dtype, out_dtype, gelu, status, st, dependent);
   const int pair_tiles = ((M + kBlockM - 1) / kBlockM + 1) / 2;
   const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
-  // The wide shape where the epilogue carries arithmetic (GELU, candidate records), the narrow one otherwise.
-  const bool wide = gelu || out_dtype == 3;
-  const bool halves = !wide && resid != nullptr && half_units(pair_tiles, N, max_pairs, K / kBlockK);
+  const bool one_wave = out_dtype != 3 && one_wave_of_halves(M, pair_tiles, N, max_pairs);
+  if (out_dtype != 3 && !one_wave && few_row_tiles(M, N))
+    return launch_linear_small(a, w, y, scale, resid, M, N, K, in_dtype, out_dtype, gelu, status, st, dependent);
+  // The wide shape where the epilogue carries arithmetic (GELU, candidate records) for unit after unit, the narrow one otherwise.
+  const bool wide = !one_wave && (gelu || out_dtype == 3);
+  const bool halves = one_wave || (!wide && resid != nullptr && half_units(pair_tiles, N, max_pairs, K / kBlockK));
   LinearArgs args = {scale, resid, M, N, K, gelu ? 1 : 0, out_dtype == 3 ? static_cast<uint4*>(y) : nullptr, y, {}};
   using Fn = int (*)(const void*, const void*, const SplitLow*, void*, const LinearArgs&, int, int, int, int, int*, cudaStream_t, int);
   Fn fn;

@@ -166,3 +166,24 @@ def test_install_layers_replaces_every_layer_and_keeps_the_numbers():
     for p in params:
         ref = O.transformer_layer(ref, p)
     assert O.rel_l2(before - x, ref - x) < 2e-3
+
+
+# One wave of 256 x 128 units between the few-row kernel (one 128 x 64 block per SM) and 256 x 256 units: first and last row count
+# that takes it, for both widths, and rows that leave a tile ragged.
+@pytest.mark.parametrize("rows,n,k,gelu,out", [(2305, 512, 2048, False, torch.float32), (4608, 512, 512, False, torch.bfloat16),
+                                               (4501, 512, 2048, False, torch.float16), (4609, 512, 512, False, torch.float32),
+                                               (513, 2048, 512, True, torch.float16), (1024, 2048, 512, True, torch.bfloat16),
+                                               (1025, 2048, 512, True, torch.float16)])
+def test_linear_around_one_wave_of_half_units(rows, n, k, gelu, out):
+    import fast_mimi_b200 as fm
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    t16 = torch.bfloat16 if out == torch.bfloat16 else torch.float16
+    a = torch.randn(rows, k, device="cuda", generator=g).to(t16)
+    w = (torch.randn(n, k, device="cuda", generator=g) * k ** -0.5).to(t16)
+    extra = {} if gelu else {"scale": torch.rand(n, device="cuda", generator=g), "residual": torch.randn(rows, n, device="cuda", generator=g).to(out)}
+    got = fm.ops.linear(a, w, activation="gelu" if gelu else None, out_dtype=out, **extra)
+    want = a.double() @ w.double().T
+    want = torch.nn.functional.gelu(want) if gelu else extra["residual"].double() + extra["scale"].double() * want
+    far = float((got.double() - want).norm() / want.norm())
+    # one rounding of the result (half a unit in the last place, uniform: 2^-12 and 2^-9 over sqrt 3 times some), or FP32 sums
+    assert far < {torch.float32: 2e-6, torch.float16: 2.5e-4, torch.bfloat16: 2e-3}[out], far
