@@ -9,22 +9,23 @@
 // V tiles (tile u in slot u % 4); per step it loads only Q_t, K_t and V_t (48 KB for 128 frames), each byte
 // once.  A run's first step also loads its two halo tiles.
 //
-// The step's three 128 x 128 score tiles are three JOBS, as in the whole-clip kernel (fm_prefill_clip.cu):
-// tensor memory is four 128-column slots, job g = 3 * step + kind runs in slot g % 4 with softmax team g % 4;
-// S = Q K^T is turned in place into 16-bit P, which the tensor core reads from tensor memory for O = P V.
-// All three jobs belong to the same 128 query rows: the teams exchange row maxima (and later row sums)
-// through shared memory, use one common maximum, and the tensor core accumulates the three P V products
-// into the diagonal job's slot, whose team normalises and stores the rows.  The window gives warp w of the
+// The step's three 128 x 128 score tiles are three JOBS: far, mid and diagonal, each with 128 columns of tensor memory and a softmax
+// team of four warps of its own; S = Q K^T is turned in place into 16-bit P, which the tensor core reads from tensor memory for
+// O = P V.  All three jobs belong to the same 128 query rows: the teams exchange row maxima through shared memory, use one common
+// maximum, and the tensor core adds the three P V products into one of two accumulators beside the jobs' columns.  So a job's next
+// scores follow as soon as its own P has been read, and a fourth team normalises and stores the rows behind the others' backs.  (With
+// O in the diagonal job's columns and four columns' sets for three jobs in turn, a step held its columns until its last row was out:
+// 16 FP16 clips of 2500 frames, 18 steps a block, 107 us, now 101.)  The window gives warp w of the
 // far job 4-w visible 32-key groups and warp w of the diagonal job w+1, so the four SM sub-partitions carry
 // the same load.  Tiles before the clip's first frame are not loaded; their jobs run empty.
-// Warps 0-15: softmax teams.  Warp 16: Q/K loads + score products.  Warp 17: P V products.  Warp 18: V loads.
+// Warps 0-11: softmax teams.  Warps 12-15: results.  Warp 16: Q/K loads + score products.  Warp 17: P V products.  Warp 18: V loads.
 //
-// FP32 q, k, v (a model's own, any strides) of calls with some steps a block are converted on the way: quarter tiles of 32 rows arrive by TMA in a staging
-// buffer, three for each of two warps (18 and 19), which round them (q, k to BF16, v to its type) into the tiles' places.  The
+// FP32 q, k, v (a model's own, any strides) of calls with some steps a block are converted on the way: pieces of 16 rows arrive by TMA in a staging
+// buffer, three for each of four warps (18 to 21), which round them (q, k to BF16, v to its type) into the tiles' places.  The
 // kernel is bound by its chain of steps, not by memory, so the 12 bytes a value triple costs instead of 6 pass behind it; a
 // converting pass in front (18 bytes a triple at the copy rate) took 51 of 141 us for 16 clips of 2500 frames, 25 clips of 1500
-// frames 132; now 107 and 102.  Two warps are what the register file has room for beside the others; what counts is the little
-// they do besides (a proxy fence, an index division and a walk of its own for every quarter tile: 141 us).
+// frames 132; now 93 and 88 (two warps, which kept the others waiting once those had become faster: 104 and 98).  What counts is the
+// little they do besides (a proxy fence, an index division and a walk of its own for every piece: 141 us instead of 107 with two).
 #include "fm_attn_tile.cuh"
 #include "fm_common.cuh"
 #include "fm_kernels.h"
@@ -38,38 +39,37 @@ using attn_tile::kD;
 using attn_tile::kTile;
 constexpr int kTileBytes = kTile * kD * 2;          // 16 KB
 constexpr int kSlabBytes = 32 * 128;                // 32 rows x 64 x 16 bit
-constexpr int kSlots = 4;
+constexpr int kJobs = 3;
 constexpr int kRing = 4;                            // K tiles and V tiles kept: t-2, t-1, t and the next step's
-constexpr int kSoftmaxWarps = 4 * kSlots;
+constexpr int kSoftmaxWarps = 4 * (kJobs + 1);      // and those that store
 constexpr int kIssueWarps = 3;
 constexpr int kThreads = (kSoftmaxWarps + kIssueWarps) * 32;
-constexpr int kTmemCols = 128 * kSlots;
-constexpr uint32_t kPCol = 0, kOCol = 64;           // inside a slot: P over the consumed S, then O
+constexpr int kTmemCols = 512;
+constexpr uint32_t kOCol = 128 * kJobs;             // three jobs' scores, P over them; then two steps' O
 
-// FP32 inputs: staged quarter tiles of the converting warps
-constexpr int kQuarterRows = 32, kQuarterBytes = kQuarterRows * kD * 4;
-constexpr int kConvertWarps = 2, kStaged = 3;
-constexpr int threads(bool f32_in) { return kThreads + (f32_in ? 32 : 0); }
+// FP32 inputs: staged pieces of tiles, two of a tile for each converting warp
+constexpr int kConvertWarps = 4, kStaged = 3;
+constexpr int kPieceRows = kTile / (2 * kConvertWarps), kPieceBytes = kPieceRows * kD * 4;
+constexpr int threads(bool f32_in) { return kThreads + (f32_in ? (kConvertWarps - 1) * 32 : 0); }
 
 struct Shared {
-  uint64_t staged[kConvertWarps][kStaged];   // a quarter tile has landed
+  uint64_t staged[kConvertWarps][kStaged];   // a piece has landed
   uint64_t qk_full[2];     // Q and the new K tile(s) of the step in this Q buffer have landed
   uint64_t v_full[2];      // the new V tile(s) of the step have landed
   uint64_t qk_done[2];     // the step's score products have completed: its Q buffer and its far K tile are dead
-  uint64_t pv_done[2];     // the step's P V products have completed: its far V tile and its P slots are dead
-  uint64_t out_done;       // the four staged slabs have been read by their TMA stores
-  uint64_t s_full[kSlots];
-  uint64_t p_full[kSlots];
-  uint64_t o_full[kSlots];
-  uint64_t slot_free[kSlots];   // the team is done with the slot's tensor memory (tested for diagonal jobs)
+  uint64_t pv_done[2];     // the step's P V products have completed: its far V tile is dead, its O is there
+  uint64_t o_free[2];      // O has been read
+  uint64_t s_full[kJobs];  // by job, a phase a step
+  uint64_t p_full[kJobs];
+  uint64_t p_done[kJobs];  // the P V product that reads P has completed
   uint64_t xm_full[4];     // the three partial row maxima of a step are published (12 warps)
-  uint64_t xl_full[4];     // the row sums of the far and mid jobs are published (8 warps)
+  uint64_t xl_full[4];     // the row sums of the three jobs are published (12 warps)
   uint32_t tmem_base;
   CtaCtl ctl;
   float xm[4][kTile][3];   // by step % 4
-  float xl[4][kTile][2];
+  float xl[4][kTile][3];
 };
-__host__ __device__ constexpr int stage_bytes(bool f32_in) { return f32_in ? kConvertWarps * kStaged * kQuarterBytes : 4 * kSlabBytes; }
+__host__ __device__ constexpr int stage_bytes(bool f32_in) { return f32_in ? kConvertWarps * kStaged * kPieceBytes : 4 * kSlabBytes; }
 constexpr int smem_bytes(bool f32_in) {
   return 1024 + 2 * kRing * kTileBytes + 2 * kTileBytes + stage_bytes(f32_in) + static_cast<int>((sizeof(Shared) + 127) & ~size_t(127));
 }
@@ -121,7 +121,7 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   uint8_t* smem_k = smem;                              // kRing tiles
   uint8_t* smem_v = smem_k + kRing * kTileBytes;       // kRing tiles
   uint8_t* smem_q = smem_v + kRing * kTileBytes;       // two tiles
-  uint8_t* smem_stage = smem_q + 2 * kTileBytes;       // four slabs, or staged FP32 quarter tiles
+  uint8_t* smem_stage = smem_q + 2 * kTileBytes;       // four slabs, or staged FP32 pieces
   Shared* sh = reinterpret_cast<Shared*>(smem_stage + stage_bytes(kF32In));
 
   const int warp = threadIdx.x >> 5;
@@ -133,15 +133,16 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       mbar_init(&sh->v_full[i], kF32In ? kConvertWarps : 1);
       mbar_init(&sh->qk_done[i], 1);
       mbar_init(&sh->pv_done[i], 1);
+      mbar_init(&sh->o_free[i], 4);
     }
-    mbar_init(&sh->out_done, 4);
-    for (int i = 0; i < kSlots; ++i) {
+    for (int i = 0; i < kJobs; ++i) {
       mbar_init(&sh->s_full[i], 1);
       mbar_init(&sh->p_full[i], 4);
-      mbar_init(&sh->o_full[i], 1);
-      mbar_init(&sh->slot_free[i], 4);
+      mbar_init(&sh->p_done[i], 1);
+    }
+    for (int i = 0; i < 4; ++i) {
       mbar_init(&sh->xm_full[i], 12);
-      mbar_init(&sh->xl_full[i], 8);
+      mbar_init(&sh->xl_full[i], 12);
     }
     for (int i = 0; kF32In && i < kConvertWarps * kStaged; ++i) mbar_init(&sh->staged[i / kStaged][i % kStaged], 1);
     sh->ctl.abort = 0;
@@ -159,7 +160,6 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   const uint32_t tmem_base = sh->tmem_base;
   CtaCtl* ctl = &sh->ctl;
 
-  auto job_phase = [](int g) { return static_cast<uint32_t>(g >> 2) & 1u; };
   auto step_phase = [](int n) { return static_cast<uint32_t>(n >> 1) & 1u; };
 
   if (warp >= kSoftmaxWarps) {
@@ -170,7 +170,8 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     const bool one = elect_one();
     constexpr uint32_t idesc_qk = umma_idesc_f16(kTile, kTile, 1, 1, 0, 0);
     constexpr uint32_t idesc_pv = umma_idesc_f16(kTile, kD, Pack16<VT>::kFmt, Pack16<VT>::kFmt, 0, 1);
-    auto slot_addr = [&](int g) { return tmem_base + static_cast<uint32_t>((g & 3) * kTile); };
+    auto job_addr = [&](int kind) { return tmem_base + static_cast<uint32_t>(kind * kTile); };
+    auto out_addr = [&](int n) { return tmem_base + kOCol + static_cast<uint32_t>((n & 1) * kD); };
     if (role == 0) {
       // ---------------------------------------------------------- Q / K loads + score products
       if (!kF32In && one) {
@@ -202,24 +203,18 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         mbar_wait(&sh->qk_full[n & 1], step_phase(n), ctl, status, kErrWaitTma);
         const uint64_t qd = umma_desc_sw128(smem_u32(smem_q + (n & 1) * kTileBytes));
         for (int kind = 0; kind < 3; ++kind) {
-          const int g = 3 * n + kind;
-          if (g >= 4) {
-            // The slot's previous job must be out of it: a far / mid job when the P V products that read its P
-            // have completed, a diagonal job when its team has read O.
-            const int gp = g - 4;
-            if (gp % 3 != 2) mbar_wait(&sh->pv_done[(gp / 3) & 1], step_phase(gp / 3), ctl, status, kErrWaitMma);
-            else mbar_wait(&sh->slot_free[gp & 3], job_phase(gp), ctl, status, kErrWaitConsumer);
-          }
+          // the job's columns: its P of the step before has been read
+          if (n >= 1) mbar_wait(&sh->p_done[kind], static_cast<uint32_t>(n - 1) & 1u, ctl, status, kErrWaitMma);
           tc_fence_after_sync();
           const int u = cur.t - 2 + kind;              // key tile of this job
           if (u >= 0) {
             const uint64_t kd = umma_desc_sw128(smem_u32(smem_k + (u & 3) * kTileBytes));
 #pragma unroll
             for (int ks = 0; ks < kD / 16; ++ks)
-              if (one) tc_mma_ss(slot_addr(g), qd + 2u * ks, kd + 2u * ks, idesc_qk, ks != 0);
+              if (one) tc_mma_ss(job_addr(kind), qd + 2u * ks, kd + 2u * ks, idesc_qk, ks != 0);
           }
           if (one) {
-            tc_commit(&sh->s_full[g & 3]);
+            tc_commit(&sh->s_full[kind]);
             if (kind == 2) tc_commit(&sh->qk_done[n & 1]);
           }
         }
@@ -234,35 +229,31 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       for (Walk w(shares); w.valid(); w.next()) {
         const int n = w.n;
         mbar_wait(&sh->v_full[n & 1], step_phase(n), ctl, status, kErrWaitTma);
-        for (int kind = 0; kind < 3; ++kind)
-          mbar_wait(&sh->p_full[(3 * n + kind) & 3], job_phase(3 * n + kind), ctl, status, kErrWaitConsumer);
-        tc_fence_after_sync();
+        mbar_wait(&sh->o_free[n & 1], step_phase(n) ^ 1u, ctl, status, kErrWaitConsumer);
         bool accumulate = false;
         for (int kind = 0; kind < 3; ++kind) {
+          mbar_wait(&sh->p_full[kind], static_cast<uint32_t>(n) & 1u, ctl, status, kErrWaitConsumer);
+          tc_fence_after_sync();
           const int u = w.t - 2 + kind;
-          if (u < 0) continue;
-          // O (+)= P V: A = P from tensor memory (8 columns per 16 keys), B = V (MN-major, 2 KB per 16 keys)
-          const uint64_t v = umma_desc_sw128(smem_u32(smem_v + (u & 3) * kTileBytes));
+          if (u >= 0) {
+            // O (+)= P V: A = P from tensor memory (8 columns per 16 keys), B = V (MN-major, 2 KB per 16 keys)
+            const uint64_t v = umma_desc_sw128(smem_u32(smem_v + (u & 3) * kTileBytes));
 #pragma unroll
-          for (int ks = 0; ks < kTile / 16; ++ks)
-            if (one)
-              tc_mma_ts(slot_addr(3 * n + 2) + kOCol, slot_addr(3 * n + kind) + kPCol + 8u * ks,
-                        v + static_cast<uint64_t>(ks) * 128u, idesc_pv, (accumulate || ks != 0) ? 1u : 0u);
-          accumulate = true;
+            for (int ks = 0; ks < kTile / 16; ++ks)
+              if (one)
+                tc_mma_ts(out_addr(n), job_addr(kind) + 8u * ks, v + static_cast<uint64_t>(ks) * 128u, idesc_pv, (accumulate || ks != 0) ? 1u : 0u);
+            accumulate = true;
+          }
+          if (one) tc_commit(&sh->p_done[kind]);
         }
-        if (one) {
-          tc_commit(&sh->o_full[(3 * n + 2) & 3]);
-          tc_commit(&sh->o_full[(3 * n + 1) & 3]);   // nobody waits on these two; one completion per slot use
-          tc_commit(&sh->o_full[(3 * n) & 3]);
-          tc_commit(&sh->pv_done[n & 1]);
-        }
+        if (one) tc_commit(&sh->pv_done[n & 1]);
       }
     } else if (kF32In) {
       // ---------------------------------------------------------- FP32 tiles into their places (two warps)
-      // A step's tiles in the order of their use: its new K tiles and Q, then its new V tiles; this warp has quarters 2c and
-      // 2c + 1 of each.  Copies run kStaged quarters ahead of the conversion.
+      // A step's tiles in the order of their use: its new K tiles and Q, then its new V tiles; this warp has pieces 2c and
+      // 2c + 1 of each.  Copies run kStaged pieces ahead of the conversion.
       const int c = role - 2;
-      uint8_t* staging = smem_stage + c * kStaged * kQuarterBytes;
+      uint8_t* staging = smem_stage + c * kStaged * kPieceBytes;
       // Copies: their own walk, with what a run's tiles have in common worked out once.
       Walk to_ask(shares);
       int ask_nk = 0, ask_tile = 0, ask_half = 0, ask_head = 0, ask_clip = 0, asked = 0;
@@ -280,8 +271,8 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         const int u = to_ask.t - (ask_tile < ask_nk ? ask_nk - 1 - ask_tile : (ask_tile == ask_nk ? 0 : 2 * ask_nk - ask_tile));
         if (one) {
           uint64_t* bar = &sh->staged[c][asked];
-          mbar_arrive_expect_tx(bar, kQuarterBytes);
-          tma_load_4d(staging + asked * kQuarterBytes, map, bar, 0, u * kTile + (2 * c + ask_half) * kQuarterRows, ask_head, ask_clip);
+          mbar_arrive_expect_tx(bar, kPieceBytes);
+          tma_load_4d(staging + asked * kPieceBytes, map, bar, 0, u * kTile + (2 * c + ask_half) * kPieceRows, ask_head, ask_clip);
         }
         if (++asked == kStaged) asked = 0;
         if (ask_half == 0) {
@@ -309,21 +300,21 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
           mbar_wait(&sh->staged[c][slot], slot_phase, ctl, status, kErrWaitTma);
-          const uint8_t* src = staging + slot * kQuarterBytes + src_lane;
-          uint8_t* out = dst + (2 * c + half) * (kQuarterRows * 128);
-          float4 v[8][2];
+          const uint8_t* src = staging + slot * kPieceBytes + src_lane;
+          uint8_t* out = dst + (2 * c + half) * (kPieceRows * 128);
+          float4 v[kPieceRows / 4][2];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
+          for (int e = 0; e < kPieceRows / 4; ++e) {
             v[e][0] = *reinterpret_cast<const float4*>(src + e * (4 * kD * 4));
             v[e][1] = *reinterpret_cast<const float4*>(src + e * (4 * kD * 4) + 16);
           }
 #pragma unroll
-          for (int e = 0; e < 8; ++e)
+          for (int e = 0; e < kPieceRows / 4; ++e)
             *reinterpret_cast<uint4*>(out + sw128_offset(e * 4 + (lane >> 3), lane & 7)) =
                 make_uint4(Pack16<T16>::pack(v[e][0].x, v[e][0].y), Pack16<T16>::pack(v[e][0].z, v[e][0].w),
                            Pack16<T16>::pack(v[e][1].x, v[e][1].y), Pack16<T16>::pack(v[e][1].z, v[e][1].w));
           __syncwarp();
-          ask();                              // into the quarter just read
+          ask();                              // into the piece just read
           if (++slot == kStaged) {
             slot = 0;
             slot_phase ^= 1u;
@@ -376,82 +367,80 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       }
     }
   } else {
-    // ------------------------------------------------------------ softmax teams
-    const int team = warp >> 2;               // == slot
+    const int kind = warp >> 2;               // the job; 3: results
     const int lg = warp & 3;                  // TMEM lane group
     const int r = lg * 32 + lane;             // row of the tile == TMEM lane
-    const uint32_t slot = tmem_base + static_cast<uint32_t>(team * kTile) + (static_cast<uint32_t>(lg * 32) << 16);
-    for (Walk w(shares); w.valid(); w.next()) {
-      const int n = w.n, x = n & 3;
-      const uint32_t xph = static_cast<uint32_t>(n >> 2) & 1u;     // this exchange buffer's use number
-      const int kind = ((team - 3 * n) % 4 + 4) % 4;               // the job of this step that runs in this team's slot
-      if (kind == 3) continue;                                     // none: the slot belongs to a neighbouring step
-      const int g = 3 * n + kind;
-      const uint32_t ph = job_phase(g);
-      const int w_row0 = w.t * kTile + lg * 32;                    // first frame held by this warp
-      const int i = w_row0 + lane;
-      const GroupVis vis(i, w_row0, (w.t - 2 + kind) * kTile, window);
+    const uint32_t lanes = static_cast<uint32_t>(lg * 32) << 16;
+    if (kind < kJobs) {
+      // ---------------------------------------------------------- softmax teams
+      const uint32_t job = tmem_base + static_cast<uint32_t>(kind * kTile) + lanes;
+      for (Walk w(shares); w.valid(); w.next()) {
+        const int n = w.n, x = n & 3;
+        const uint32_t xph = static_cast<uint32_t>(n >> 2) & 1u;     // this exchange buffer's use number
+        const int w_row0 = w.t * kTile + lg * 32;                    // first frame held by this warp
+        const GroupVis vis(w_row0 + lane, w_row0, (w.t - 2 + kind) * kTile, window);
 
-      mbar_wait(&sh->s_full[team], ph, ctl, status, kErrWaitMma);
-      tc_fence_after_sync();
-      float m_raw = tile_row_max(slot, vis);                       // -inf for a job with nothing visible
-      sh->xm[x][r][kind] = m_raw;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sh->xm_full[x]);
-      mbar_wait(&sh->xm_full[x], xph, ctl, status, kErrWaitConsumer);
-      m_raw = fmaxf(fmaxf(sh->xm[x][r][0], sh->xm[x][r][1]), sh->xm[x][r][2]);
-      const float m_use = (m_raw == -INFINITY) ? 0.f : m_raw * scale_log2e;
-      float l_row = tile_row_probs<VT>(slot, slot + kPCol, vis, scale_log2e, m_use);
-      if (kind != 2) sh->xl[x][r][kind] = l_row;
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&sh->p_full[team]);
-        if (kind != 2) {
-          mbar_arrive(&sh->xl_full[x]);
-          mbar_arrive(&sh->slot_free[team]);   // keeps the barrier's phase in step with the slot's use count
-        }
-      }
-      if (kind != 2) continue;                 // the diagonal job's team finishes the rows
-
-      mbar_wait(&sh->o_full[team], ph, ctl, status, kErrWaitMma);
-      tc_fence_after_sync();
-      mbar_wait(&sh->xl_full[x], xph, ctl, status, kErrWaitConsumer);
-      l_row += sh->xl[x][r][0] + sh->xl[x][r][1];
-      if constexpr (std::is_same<OT, float>::value) {
-        uint32_t o[64];
-        tmem_ld32(slot + kOCol, *reinterpret_cast<uint32_t(*)[32]>(&o[0]));
-        tmem_ld32(slot + kOCol + 32, *reinterpret_cast<uint32_t(*)[32]>(&o[32]));
-        tmem_ld_wait();
+        mbar_wait(&sh->s_full[kind], static_cast<uint32_t>(n) & 1u, ctl, status, kErrWaitMma);
+        tc_fence_after_sync();
+        float m_raw = tile_row_max(job, vis);                        // -inf for a job with nothing visible
+        sh->xm[x][r][kind] = m_raw;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh->xm_full[x]);
+        mbar_wait(&sh->xm_full[x], xph, ctl, status, kErrWaitConsumer);
+        m_raw = fmaxf(fmaxf(sh->xm[x][r][0], sh->xm[x][r][1]), sh->xm[x][r][2]);
+        const float m_use = (m_raw == -INFINITY) ? 0.f : m_raw * scale_log2e;
+        sh->xl[x][r][kind] = tile_row_probs<VT>(job, job, vis, scale_log2e, m_use);
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sh->slot_free[team]);
-        if (i < T) {
-          const float inv = 1.f / l_row;
-          float* dst = out32 + (static_cast<long long>(w.clip()) * T + i) * 512 + w.head() * kD;
-#pragma unroll
-          for (int d = 0; d < kD; ++d) o[d] = __float_as_uint(__uint_as_float(o[d]) * inv);
-#pragma unroll
-          for (int d = 0; d < kD; d += 8) st_global_v8(dst + d, o + d);
+        if (lane == 0) {
+          mbar_arrive(&sh->p_full[kind]);
+          mbar_arrive(&sh->xl_full[x]);
         }
-        continue;
       }
-      // The previous step's stores out of the slabs must have read them.
-      uint8_t* slab = smem_stage + lg * kSlabBytes;
-      if (n >= 1) mbar_wait(&sh->out_done, static_cast<uint32_t>(n - 1) & 1u, ctl, status, kErrWaitConsumer);
-      stage_output_row<VT>(slot + kOCol, slab, lane, 1.f / l_row);
-      tc_fence_before_sync();
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&sh->slot_free[team]);
-        if (w_row0 < T) {                      // frames past T are clipped by the map
-          tma_store_3d(&tmap_out, slab, w.head() * kD, w_row0, w.clip());
-          bulk_commit_group();
-          bulk_wait_group_read<0>();
+    } else {
+      // ---------------------------------------------------------- results
+      for (Walk w(shares); w.valid(); w.next()) {
+        const int n = w.n, x = n & 3;
+        const int w_row0 = w.t * kTile + lg * 32, i = w_row0 + lane;
+        const uint32_t o_addr = tmem_base + kOCol + static_cast<uint32_t>((n & 1) * kD) + lanes;
+        mbar_wait(&sh->xl_full[x], static_cast<uint32_t>(n >> 2) & 1u, ctl, status, kErrWaitConsumer);
+        const float l_row = sh->xl[x][r][2] + (sh->xl[x][r][0] + sh->xl[x][r][1]);
+        mbar_wait(&sh->pv_done[n & 1], step_phase(n), ctl, status, kErrWaitMma);
+        tc_fence_after_sync();
+        if constexpr (std::is_same<OT, float>::value) {
+          uint32_t o[64];
+          tmem_ld32(o_addr, *reinterpret_cast<uint32_t(*)[32]>(&o[0]));
+          tmem_ld32(o_addr + 32, *reinterpret_cast<uint32_t(*)[32]>(&o[32]));
+          tmem_ld_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh->o_free[n & 1]);
+          if (i < T) {
+            const float inv = 1.f / l_row;
+            float* dst = out32 + (static_cast<long long>(w.clip()) * T + i) * 512 + w.head() * kD;
+#pragma unroll
+            for (int d = 0; d < kD; ++d) o[d] = __float_as_uint(__uint_as_float(o[d]) * inv);
+#pragma unroll
+            for (int d = 0; d < kD; d += 8) st_global_v8(dst + d, o + d);
+          }
+        } else {
+          uint8_t* slab = smem_stage + lg * kSlabBytes;
+          if (lane == 0) bulk_wait_group_read<0>();          // the store of the step before has read it
+          __syncwarp();
+          stage_output_row<VT>(o_addr, slab, lane, 1.f / l_row);
+          tc_fence_before_sync();
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(&sh->o_free[n & 1]);
+            if (w_row0 < T) {                                // frames past T are clipped by the map
+              tma_store_3d(&tmap_out, slab, w.head() * kD, w_row0, w.clip());
+              bulk_commit_group();
+            }
+          }
         }
-        mbar_arrive(&sh->out_done);
       }
+      if (lane == 0) bulk_wait_group_read<0>();
     }
   }
 
@@ -465,12 +454,12 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   }
 }
 
-// q, k, v as FP32 tensors [B, 8, T, 64] of any strides (in values): (64, T, 8, B), boxes of a quarter tile
+// q, k, v as FP32 tensors [B, 8, T, 64] of any strides (in values): (64, T, 8, B), boxes of a piece of a tile
 static int encode_f32_map(CUtensorMap* map, const void* base, const long long* strides, int B, int T) {
   const cuuint64_t dims[4] = {64, static_cast<cuuint64_t>(T), 8, static_cast<cuuint64_t>(B)};
   const cuuint64_t bytes[3] = {static_cast<cuuint64_t>(strides[2]) * 4, static_cast<cuuint64_t>(strides[1]) * 4,
                                static_cast<cuuint64_t>(B > 1 ? strides[0] : 512) * 4};
-  const cuuint32_t box[4] = {64, longclip::kQuarterRows, 1, 1}, estr[4] = {1, 1, 1, 1};
+  const cuuint32_t box[4] = {64, longclip::kPieceRows, 1, 1}, estr[4] = {1, 1, 1, 1};
   return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(base), dims, bytes, box, estr, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
@@ -518,7 +507,7 @@ int launch_band_attn_long(const void* q, const void* k, const void* v, void* out
                        out_fp32 ? static_cast<float*>(out) : nullptr, shares, T, window, scale * 1.4426950408889634f, status);
 }
 
-// Strides that a tensor map can have, and enough steps a block.  The two converting warps keep up with the chain of steps, but where a
+// Strides that a tensor map can have, and enough steps a block.  The converting warps keep up with the chain of steps, but where a
 // run begins the first step waits until they have made seven tiles instead of three, and a short call is little else; a converting
 // pass in front costs 1 us and 0.7 ns a frame.  Inside from five steps on, from seven where short sequences begin and end inside of shares.
 // GPU time, FP32, in front -> inside:
