@@ -3,6 +3,8 @@
 // (key j visible to query i iff max(i - window + 1, 0) <= j <= i; src/fast_mimi/model.py:1672-1676).
 #pragma once
 
+#include <type_traits>
+
 #include "fm_common.cuh"
 
 namespace fm {
@@ -26,6 +28,22 @@ struct GroupVis {
   __device__ __forceinline__ bool full(int c0) const { return c0 >= all_lo && c0 + 31 <= all_hi; }
 };
 
+// Which ends of the window cut into a group of 32 columns: none, its older end, its newer end, both.  A column is tested against
+// those alone: the far and the diagonal tile of a long clip have two such groups in every warp, and with both tests a group of the
+// former took 900 cycles instead of 600, which every step of that kernel waited for.
+template <typename F>
+__device__ __forceinline__ void with_tests(const GroupVis& g, int c0, F&& f) {
+  const bool older = c0 < g.all_lo, newer = c0 + 31 > g.all_hi;
+  if (!older && !newer) f(std::integral_constant<int, 0>());
+  else if (!newer) f(std::integral_constant<int, 1>());
+  else if (!older) f(std::integral_constant<int, 2>());
+  else f(std::integral_constant<int, 3>());
+}
+template <int kTests>
+__device__ __forceinline__ bool visible(int cc, int lo, int hi) {
+  return (!(kTests & 1) || cc >= lo) && (!(kTests & 2) || cc <= hi);
+}
+
 // Row maximum of the visible raw scores of a tile (this thread's row).
 __device__ __forceinline__ float tile_row_max(uint32_t s_addr, const GroupVis& g) {
   float m[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -35,14 +53,12 @@ __device__ __forceinline__ float tile_row_max(uint32_t s_addr, const GroupVis& g
     uint32_t s[32];
     tmem_ld32(s_addr + c0, s);
     tmem_ld_wait();
-    if (g.full(c0)) {
-#pragma unroll
-      for (int cc = 0; cc < 32; ++cc) m[cc & 3] = fmaxf(m[cc & 3], __uint_as_float(s[cc]));
-    } else {
+    const int lo = g.vis_lo - c0, hi = g.vis_hi - c0;
+    with_tests(g, c0, [&](auto tests) {
 #pragma unroll
       for (int cc = 0; cc < 32; ++cc)
-        if (c0 + cc >= g.vis_lo && c0 + cc <= g.vis_hi) m[cc & 3] = fmaxf(m[cc & 3], __uint_as_float(s[cc]));
-    }
+        if (visible<decltype(tests)::value>(cc, lo, hi)) m[cc & 3] = fmaxf(m[cc & 3], __uint_as_float(s[cc]));
+    });
   }
   return fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
 }
@@ -64,27 +80,20 @@ __device__ __forceinline__ float tile_row_probs(uint32_t s_addr, uint32_t p_addr
       uint32_t s[32];
       tmem_ld32(s_addr + c0, s);
       tmem_ld_wait();
-      if (g.full(c0)) {
-#pragma unroll
-        for (int cc = 0; cc < 32; cc += 2) {
-          const float p0 = ex2_approx(fmaf(__uint_as_float(s[cc]), scale_log2e, -m_use));
-          const float p1 = ex2_approx(fmaf(__uint_as_float(s[cc + 1]), scale_log2e, -m_use));
-          pk[cc / 2] = Pack16<VT>::pack(p0, p1);
-          l[(cc >> 1) & 3] += p0 + p1;
-        }
-      } else {
+      const int lo = g.vis_lo - c0, hi = g.vis_hi - c0;
+      with_tests(g, c0, [&](auto tests) {
 #pragma unroll
         for (int cc = 0; cc < 32; cc += 2) {
           float p[2];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const bool vis = c0 + cc + e >= g.vis_lo && c0 + cc + e <= g.vis_hi;
-            p[e] = vis ? ex2_approx(fmaf(__uint_as_float(s[cc + e]), scale_log2e, -m_use)) : 0.f;
+            p[e] = ex2_approx(fmaf(__uint_as_float(s[cc + e]), scale_log2e, -m_use));
+            if (!visible<decltype(tests)::value>(cc + e, lo, hi)) p[e] = 0.f;
           }
           pk[cc / 2] = Pack16<VT>::pack(p[0], p[1]);
           l[(cc >> 1) & 3] += p[0] + p[1];
         }
-      }
+      });
     }
     tmem_st16(p_addr + (c0 >> 1), pk);
   }
