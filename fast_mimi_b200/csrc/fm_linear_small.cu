@@ -255,6 +255,7 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 // Beyond that the blocks re-read activations and weights too often for what they save, and the 256 x 256 tiles of the
 // pair kernels are faster: at K = 512, N = 2048 1024 rows (256 tiles) take 9.1 us here and 10.9 us there, 1500 rows (384
 // tiles) 13.9 against 10.9; at K = 2048, N = 512 3678 rows (232 tiles) 17.1 against 22.1, 5000 rows (320) 27.5 against 22.5.
+// (Linear layers of more than one tile per SM take half units of the pair kernel where those are one wave: fm_linear_gemm.cu.)
 bool few_row_tiles(int M, int N) {
   return static_cast<long long>((M + small::kBlockM - 1) / small::kBlockM) * (N / 64) <= 2ll * sm_count();
 }

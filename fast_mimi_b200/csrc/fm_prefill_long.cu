@@ -15,7 +15,7 @@
 // maximum, and the tensor core adds the three P V products into one of two accumulators beside the jobs' columns.  So a job's next
 // scores follow as soon as its own P has been read, and a fourth team normalises and stores the rows behind the others' backs.  (With
 // O in the diagonal job's columns and four columns' sets for three jobs in turn, a step held its columns until its last row was out:
-// 16 FP16 clips of 2500 frames, 18 steps a block, 107 us, now 101.)  The window gives warp w of the
+// 16 FP16 clips of 2500 frames, 18 steps a block, 107 us, now 98, of which 3 by the tests in fm_attn_tile.cuh.)  The window gives warp w of the
 // far job 4-w visible 32-key groups and warp w of the diagonal job w+1, so the four SM sub-partitions carry
 // the same load.  Tiles before the clip's first frame are not loaded; their jobs run empty.
 // Warps 0-11: softmax teams.  Warps 12-15: results.  Warp 16: Q/K loads + score products.  Warp 17: P V products.  Warp 18: V loads.
@@ -24,7 +24,7 @@
 // buffer, three for each of four warps (18 to 21), which round them (q, k to BF16, v to its type) into the tiles' places.  The
 // kernel is bound by its chain of steps, not by memory, so the 12 bytes a value triple costs instead of 6 pass behind it; a
 // converting pass in front (18 bytes a triple at the copy rate) took 51 of 141 us for 16 clips of 2500 frames, 25 clips of 1500
-// frames 132; now 93 and 88 (two warps, which kept the others waiting once those had become faster: 104 and 98).  What counts is the
+// frames 132; now 91 and 87 (two warps, which kept the others waiting once those had become faster: 104 and 98).  What counts is the
 // little they do besides (a proxy fence, an index division and a walk of its own for every piece: 141 us instead of 107 with two).
 #include "fm_attn_tile.cuh"
 #include "fm_common.cuh"
