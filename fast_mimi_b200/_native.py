@@ -52,6 +52,7 @@ SIGNATURES: dict[str, list] = {
     "fm_split_half": [_P, _P, _P, _LL, _P],
     "fm_rvq_encode_f32": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _LL, _I, _I, _F, _P, _P],
     "fm_rvq_encode_stacks_f32": [ctypes.POINTER(RvqStack), _I, _P, _P, _P, _LL, _I, _F, _P, _P],
+    "fm_rvq_encode_tiles_f32": [ctypes.POINTER(RvqStack), _I, _LL, _I, _F, _P, _P],
     "fm_rvq_prepare_f32": [_P, _P, _P, _LL, _F, _F, _P],
     "fm_rvq_candidates_f16": [_P, _P, _P, _P, _P, _LL, _I, _P, _P],
     "fm_rvq_select_rec_f32": [_P, _P, _P, _P, _P, _P, _P, _LL, _I, _F, _F, _P, _P],

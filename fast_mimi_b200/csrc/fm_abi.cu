@@ -282,15 +282,26 @@ int fm_rvq_encode_f32(float* residual, void* residual16, float* tau, void* recor
                                n_codes, layers, tau_rel, status, static_cast<cudaStream_t>(stream));
 }
 
-int fm_rvq_encode_stacks_f32(const fm_rvq_stack* stacks, int n_stacks, void* residual16, float* tau, void* records, long long rows,
-                             int n_codes, float tau_rel, int* status, void* stream) {
+static int rvq_stacks(const fm_rvq_stack* stacks, int n_stacks, fm::RvqStack (&s)[2]) {
   if (stacks == nullptr || n_stacks < 1 || n_stacks > 2) return -1;
-  fm::RvqStack s[2] = {};
   for (int i = 0; i < n_stacks; ++i) {
     const fm_rvq_stack& a = stacks[i];
     s[i] = {a.residual, a.codebooks16, a.codebooks, a.e_sq, a.e_max, a.codes, a.layers};
   }
+  return 0;
+}
+
+int fm_rvq_encode_stacks_f32(const fm_rvq_stack* stacks, int n_stacks, void* residual16, float* tau, void* records, long long rows,
+                             int n_codes, float tau_rel, int* status, void* stream) {
+  fm::RvqStack s[2] = {};
+  if (rvq_stacks(stacks, n_stacks, s) != 0) return -1;
   return fm::launch_rvq_encode_stacks(s, n_stacks, residual16, tau, records, rows, n_codes, tau_rel, status, static_cast<cudaStream_t>(stream));
+}
+
+int fm_rvq_encode_tiles_f32(const fm_rvq_stack* stacks, int n_stacks, long long rows, int n_codes, float tau_rel, int* status, void* stream) {
+  fm::RvqStack s[2] = {};
+  if (rvq_stacks(stacks, n_stacks, s) != 0) return -1;
+  return fm::launch_rvq_tiles(s, n_stacks, rows, n_codes, tau_rel, status, static_cast<cudaStream_t>(stream));
 }
 
 int fm_rvq_prepare_f32(const float* x, void* residual16, float* tau, long long rows, float e_max, float tau_rel,

@@ -577,23 +577,40 @@ void deal(rvqt::Args* a, int tiles, int stacks, int pairs) {
 }
 }  // namespace
 
-// -|e|^2 / 2 has to fit FP16 times the largest power of two that FP16 holds, entries are read by whole sectors, and the time has to
-// pay.  A pair takes 26 us a layer however few vectors it has, whereas the chain spreads a layer over the whole device, so what counts
+namespace {
+// What the kernel needs of its stacks: -|e|^2 / 2 has to fit FP16 times the largest power of two that FP16 holds, and entries are read
+// by whole sectors.  0, -1, or -3 for an address.
+int cannot(const RvqStack* stacks, int n_stacks, long long rows, int n_codes) {
+  using namespace rvqt;
+  if (n_stacks < 1 || n_stacks > 2 || rows < 0 || rows > 0x7fffffffLL || n_codes <= 0 || n_codes % (2 * kEntries) != 0 || n_codes > 2048) return -1;
+  int rc = 0;
+  for (int i = 0; i < n_stacks; ++i) {
+    const RvqStack& s = stacks[i];
+    if (s.residual == nullptr || s.books16 == nullptr || s.books == nullptr || s.e_sq == nullptr || s.e_max == nullptr || s.codes == nullptr ||
+        s.layers < 1 || s.layers > kMaxLayers)
+      return -1;
+    for (int l = 0; l < s.layers; ++l)
+      if (!(s.e_max[l] >= 0.f && s.e_max[l] <= 16384.f)) return -1;
+    if (((reinterpret_cast<uintptr_t>(s.residual) | reinterpret_cast<uintptr_t>(s.books16) | reinterpret_cast<uintptr_t>(s.e_sq)) & 15u) != 0 ||
+        (reinterpret_cast<uintptr_t>(s.books) & 31u) != 0)
+      rc = -3;
+  }
+  return rc;
+}
+}  // namespace
+
+// The time has to pay.  A pair takes 26 us a layer however few vectors it has, whereas the chain spreads a layer over the whole device, so what counts
 // is how evenly tiles come out (1 + 7 layers, in us, chain -> here: 6000 vectors 146 -> 169, 9000 172 -> 171,
 // 16000 248 -> 182, 18944, the most that a tile per pair holds, 276 -> 210, 24000 332 -> 339, 32000 417 -> 385, 48000 645 -> 548, 64000
 // 831 -> 716; 32 layers of 16000 973 -> 711).  The chain's layer is 13.5 us + 1.1 for every 1000 vectors, 1.65 for those past 32000, whose
 // records and residuals no longer stay in L2.
 bool rvq_tiles_take(const RvqStack* stacks, int n_stacks, long long rows, int n_codes) {
   using namespace rvqt;
-  if (n_stacks < 1 || n_stacks > 2 || rows > 0x7fffffffLL || n_codes % (2 * kEntries) != 0 || n_codes > 2048) return false;
+  if (cannot(stacks, n_stacks, rows, n_codes) != 0) return false;
   int layers = 0, longer = 0;
   for (int i = 0; i < n_stacks; ++i) {
-    const RvqStack& s = stacks[i];
-    if (s.layers < 1 || s.layers > kMaxLayers || s.e_max == nullptr || (reinterpret_cast<uintptr_t>(s.books) & 31u) != 0) return false;
-    for (int l = 0; l < s.layers; ++l)
-      if (!(s.e_max[l] <= 16384.f)) return false;
-    layers += s.layers;
-    longer = s.layers > longer ? s.layers : longer;
+    layers += stacks[i].layers;
+    longer = stacks[i].layers > longer ? stacks[i].layers : longer;
   }
   const long long tiles = (rows + kTileRows - 1) / kTileRows, pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
   const long long even = (tiles * layers + pairs - 1) / pairs, uneven = (tiles + pairs - 1) / pairs * longer;    // layers of the busiest pair
@@ -603,18 +620,14 @@ bool rvq_tiles_take(const RvqStack* stacks, int n_stacks, long long rows, int n_
 
 int launch_rvq_tiles(const RvqStack* stacks, int n_stacks, long long rows, int n_codes, float tau_rel, int* status, cudaStream_t st) {
   using namespace rvqt;
-  if (n_stacks < 1 || n_stacks > 2 || rows <= 0 || rows > 0x7fffffffLL || n_codes <= 0 || n_codes > 2048 || n_codes % (2 * kEntries) != 0 || !(tau_rel >= 0.f)) return -1;
+  if (!(tau_rel >= 0.f)) return -1;
+  int rc = cannot(stacks, n_stacks, rows, n_codes);
+  if (rc != 0 || rows == 0) return rc;
   Args a = {};
   CUtensorMap maps[2];
   const int longer = n_stacks == 2 && stacks[1].layers > stacks[0].layers ? 1 : 0;
   for (int i = 0; i < n_stacks; ++i) {
     const RvqStack& s = stacks[i ^ longer];
-    if (s.residual == nullptr || s.books16 == nullptr || s.books == nullptr || s.e_sq == nullptr || s.e_max == nullptr || s.codes == nullptr ||
-        s.layers <= 0 || s.layers > kMaxLayers)
-      return -1;
-    if ((reinterpret_cast<uintptr_t>(s.residual) | reinterpret_cast<uintptr_t>(s.books16) | reinterpret_cast<uintptr_t>(s.books) |
-         reinterpret_cast<uintptr_t>(s.e_sq)) & 15u)
-      return -3;
     Stack& d = a.stack[i];
     d.x = s.residual;
     d.books = s.books;
@@ -622,14 +635,13 @@ int launch_rvq_tiles(const RvqStack* stacks, int n_stacks, long long rows, int n
     d.codes = s.codes;
     d.layers = s.layers;
     for (int l = 0; l < s.layers; ++l) {
-      if (!(s.e_max[l] >= 0.f)) return -1;
       d.e_max[l] = s.e_max[l];
       int exponent = 0;                        // -|e|^2 / 2 in units of the least power of two that keeps it below 2^14
       frexpf(0.5f * s.e_max[l] * s.e_max[l], &exponent);
       exponent -= 14;
       d.unit[l] = ldexpf(1.f, exponent < -14 ? -14 : (exponent > 15 ? 15 : exponent));
     }
-    const int rc = encode_rows_16bit(&maps[i], s.books16, static_cast<uint64_t>(s.layers) * n_codes, kDim, kEntries / 2, 64);
+    rc = encode_rows_16bit(&maps[i], s.books16, static_cast<uint64_t>(s.layers) * n_codes, kDim, kEntries / 2, 64);
     if (rc != 0) return rc;
   }
   if (n_stacks == 1) maps[1] = maps[0];
@@ -643,7 +655,7 @@ int launch_rvq_tiles(const RvqStack* stacks, int n_stacks, long long rows, int n
   if (tiles * n_stacks < pairs) pairs = static_cast<int>(tiles) * n_stacks;
   deal(&a, static_cast<int>(tiles), n_stacks, pairs);
   const uint32_t idesc = umma_idesc_f16(kTileRows, kEntries, 0, 0, 0, 0);
-  const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(rvq_tiles_kernel), kSmemBytes);
+  rc = ensure_dynamic_smem(reinterpret_cast<const void*>(rvq_tiles_kernel), kSmemBytes);
   if (rc != 0) return rc;
   return launch_kernel(rvq_tiles_kernel, dim3(static_cast<unsigned>(2 * pairs)), kThreads, kSmemBytes, st, 1, 0, maps[0], maps[1], a, idesc, status);
 }

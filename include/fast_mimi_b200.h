@@ -268,6 +268,10 @@ typedef struct {
 int fm_rvq_encode_stacks_f32(const fm_rvq_stack* stacks, int n_stacks, void* residual16, float* tau, void* records, long long rows,
                              int n_codes, float tau_rel, int* status, void* stream);
 
+/* The form of that which many vectors take, whether or not it is the faster one for so many: one kernel, no workspaces.  At most 32
+ * layers, e_max <= 16384, codebooks on a 32-byte boundary, all else on 16: -1 or -3 otherwise. */
+int fm_rvq_encode_tiles_f32(const fm_rvq_stack* stacks, int n_stacks, long long rows, int n_codes, float tau_rel, int* status, void* stream);
+
 /* The same layer without the scores' round trip through memory (replaces the same reference lines as
  * fm_rvq_select_f32: src/fast_mimi/model.py:2277-2291, :2420-2427), three calls:
  *   fm_rvq_prepare_f32     before the first layer: FP16 copy of x [rows, 256] and every frame's candidate margin

@@ -2,10 +2,27 @@
 ``return_candidates`` asks for the chain."""
 from __future__ import annotations
 
+import ctypes
+
 import pytest
 import torch
 
-pytestmark = pytest.mark.gpu
+
+def _stack(residual, half, vectors, sq, e_max, codes, layers):
+    from fast_mimi_b200 import _native
+    return _native.RvqStack(residual, half, vectors, sq, (ctypes.c_float * len(e_max))(*e_max), codes, layers)
+
+
+# (Of addresses that nothing reads: a call that went on would meet its error elsewhere.)
+@pytest.mark.parametrize("books,e_max,layers,want", [(0x10010, 1.0, 2, -3), (0x10004, 1.0, 2, -3), (0x10000, 16385.0, 2, -1), (0x10000, float("nan"), 2, -1),
+                                                     (0x10000, 1.0, 33, -1), (0x10000, 1.0, 0, -1), (0, 1.0, 2, -1)])
+def test_what_the_kernel_cannot_take_is_refused(books, e_max, layers, want):
+    """Its eight-wide loads and the FP16 parts of -|e|^2 / 2 set limits, whoever calls it."""
+    from fast_mimi_b200 import _native
+    stacks = (_native.RvqStack * 2)(_stack(0x20000, 0x30000, 0x40000, 0x50000, [1.0], 0x60000, 1),
+                                    _stack(0x20000, 0x30000, books, 0x50000, [1.0, e_max] + [1.0] * 31, 0x60000, layers))
+    assert _native.load().fm_rvq_encode_tiles_f32(stacks, 2, 18000, 2048, 4.5e-3, None, None) == want
+    assert _native.load().fm_rvq_encode_tiles_f32(stacks, 1, 18000, 2048 + 128, 4.5e-3, None, None) == -1
 
 
 def _books(layers, entries, gen, same=0):
@@ -16,6 +33,7 @@ def _books(layers, entries, gen, same=0):
 
 
 # A tile is 256 vectors and 74 pairs of blocks take one each: 18944 is the most of a wave; 9217 and 18700 end inside a block's rows.
+@pytest.mark.gpu
 @pytest.mark.parametrize("rows,layers,entries,scale", [(9217, 8, 2048, 1.0), (18944, 3, 2048, 1.0), (18700, 5, 1024, 300.0), (33000, 2, 256, 1e-3)])
 def test_codes_equal_the_chains(rows, layers, entries, scale):
     import fast_mimi_b200 as fm
@@ -28,6 +46,7 @@ def test_codes_equal_the_chains(rows, layers, entries, scale):
     assert int(cand.max()) > 1                   # exact distances did decide somewhere
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("same", [9, 40, 700])   # beyond what a thread, a vector remembers; of every block's entries
 def test_entries_that_are_the_same(same):
     import fast_mimi_b200 as fm
@@ -41,6 +60,7 @@ def test_entries_that_are_the_same(same):
     assert torch.equal(got, want) and bool((got[0, ::50] == 100).all())
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("frames", [3100, 23, 70])        # dealt to pairs of blocks; one wave of clusters, two
 def test_both_stacks_of_a_split_quantiser(frames):
     """1 + 7 layers in one launch against either branch by itself."""
@@ -57,6 +77,7 @@ def test_both_stacks_of_a_split_quantiser(frames):
         assert torch.equal(part.reshape(len(part), -1), want)
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("value", [float("nan"), float("inf"), 1e30])
 def test_a_vector_that_is_not_finite(value):
     import fast_mimi_b200 as fm
