@@ -40,8 +40,9 @@ constexpr int kStages = 3, kStageBytes = kSlices * kSliceBytes;
 constexpr int kOnesBytes = kBlockM * 32, kTailBytes = kEntries / 2 * 32;       // sixteen more columns of K, rows of 32 bytes
 constexpr int kTails = 4;
 constexpr int kList = 8;                                       // candidates that a thread remembers
-constexpr int kMany = 255;                                     // ... or more than that: every entry is one
-constexpr int kBatch = 8, kBatchPitch = kDim + 4;               // of 32 vectors, how many are decided exactly at once; floats from one to the next
+constexpr int kMany = 255;                                     // ... or more than that: the others are marked in `more`
+constexpr int kWords = 2048 / kGroup;                          // of marks
+constexpr int kBatch = 8, kBatchPitch = 1040;                  // of 32 vectors, how many are decided exactly at once; bytes from one to the next
 constexpr int kMaxLayers = 32, kMaxPairs = 80;
 constexpr int kTmemCols = 512, kResidual = 2 * kEntries;       // columns: two accumulators, then the residuals
 
@@ -98,7 +99,7 @@ struct Shared {
   uint32_t list[kBlockM][4][kList];            // their candidates: a score, rounded up to 21 bits, and the entry
   alignas(4) uint8_t listed[kBlockM][4];
   uint16_t winner[kBlockM];                    // where distances decided
-  alignas(16) float exact[4][kBatch][kBatchPitch];
+  uint32_t more[kWords][kBlockM];              // a bit an entry: a vector's candidates behind lists that are full (a word belongs to one of its threads)
 };
 constexpr int kSmemBytes = 1024 + kXBytes + kStages * kStageBytes + kOnesBytes + kTails * kTailBytes + static_cast<int>(sizeof(Shared));
 static_assert(kSmemBytes <= 232448, "shared memory");
@@ -130,6 +131,147 @@ __device__ __forceinline__ uint64_t tail_desc(uint32_t smem_addr) {
 __device__ __forceinline__ uint32_t round_up(float v) {
   const uint32_t b = __float_as_uint(v);
   return ((b >> 31) != 0u ? b : b + 2047u) & ~2047u;
+}
+__device__ __forceinline__ uint8_t* staged(uint8_t* area, int i) { return area + (i >> 1) * kChunkBytes + (i & 1) * kBatchPitch; }
+
+// Residuals of a team's vectors into their places in `area` (this thread's slice; -1: not this one).
+__device__ __forceinline__ void stage(uint8_t* area, int place, int q, uint32_t t_residual) {
+#pragma unroll
+  for (int part = 0; part < 2; ++part) {
+    uint32_t x[32];
+    tmem_ld32(t_residual + part * 32, x);
+    tmem_ld_wait();
+    if (place >= 0) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        *reinterpret_cast<uint4*>(staged(area, place) + q * 256 + part * 128 + 16 * c) = make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
+    }
+  }
+}
+
+// Vectors whose lists were full have many candidates, and much the same ones (entries that are equal, or nearly).  So each entry that is one
+// for any vector of the batch that is staged in `area` is read once, by one of the team's four warps, four of them at a time, and its distance
+// from all of the batch found, added up as ever.  (18000 vectors x 8 layers, 9 entries of zero in every codebook 295 us, 40 411, 600 2360, in the
+// chain 284, 388 and 2340; with one warp a vector and all 2048 entries as its candidates 7900, 10400 and 23600.)  Lane 8 * k + i keeps the nearest to vector i of the entries that came k-th.  Few registers: the loops over
+// scores need them all.  Returns the code of the thread's vector, if it is one of `many`.
+__device__ __forceinline__ int decide_crowd(Shared* sh, uint8_t* area, const float* book, unsigned many, uint32_t t_residual, int n_steps) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lg = warp & 3, q = warp >> 2, row = lg * 32 + lane;
+  uint32_t* marks = reinterpret_cast<uint32_t*>(area + 2 * kBatchPitch);                  // [kWords]
+  uint2* nearest = reinterpret_cast<uint2*>(area + 2 * kBatchPitch + 4 * kWords);        // [warp of the team][kBatch]: distance, entry
+  int code = 0;
+#pragma unroll 1
+  while (many != 0u) {
+    unsigned rest = many;
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) rest &= rest - 1u;
+    const unsigned batch = many ^ rest;
+    const int place = (batch >> lane & 1u) != 0u ? __popc(batch & ((1u << lane) - 1u)) : -1;
+    many = rest;
+    stage(area, place, q, t_residual);
+    if (q * 32 + lane < kWords) marks[q * 32 + lane] = 0u;
+    team_sync(lg);
+    if (place >= 0) {
+      const int listed = sh->listed[row][q];
+#pragma unroll 1
+      for (int i = 0; i < (listed == kMany ? kList : listed); ++i) {
+        const uint32_t j = sh->list[row][q][i] & 2047u;
+        atomicOr(marks + j / kGroup, 1u << j % kGroup);
+      }
+#pragma unroll 1
+      for (int i = q >> 1; listed == kMany && i < n_steps; i += 2) {
+#pragma unroll 1
+        for (int word = i * 4 + (q & 1) * 2; word < i * 4 + (q & 1) * 2 + 2; ++word)
+          if (sh->more[word][row] != 0u) atomicOr(marks + word, sh->more[word][row]);
+      }
+    }
+    team_sync(lg);
+    // every fourth entry is this warp's
+    const uint32_t own = 0x11111111u << q;
+    unsigned words0 = __ballot_sync(0xffffffffu, (marks[lane] & own) != 0u), words1 = __ballot_sync(0xffffffffu, (marks[32 + lane] & own) != 0u);
+    uint32_t word = 0u;
+    int first = 0;
+    auto next = [&]() {
+      if (word == 0u) {
+        if ((words0 | words1) == 0u) return -1;
+        const int at = words0 != 0u ? __ffs(words0) - 1 : 31 + __ffs(words1);
+        if (words0 != 0u) words0 &= words0 - 1u;
+        else words1 &= words1 - 1u;
+        word = marks[at] & own;
+        first = at * kGroup;
+      }
+      const int j = first + __ffs(word) - 1;
+      word &= word - 1u;
+      return j;
+    };
+    float least = INFINITY;
+    int win = 0;
+#pragma unroll 1
+    while ((word | words0 | words1) != 0u) {
+      float e[4][8];
+      int mine = -1;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int j = next();
+        load_global8(book + static_cast<size_t>(j >= 0 ? j : 0) * kDim + 8 * lane, e[k]);        // (under a test e would be alive all along)
+        if ((lane >> 3) == k) mine = j;
+      }
+#pragma unroll 1
+      for (int i = 0; i < __popc(batch); ++i) {
+        const float4* src = reinterpret_cast<const float4*>(staged(area, i)) + 2 * lane;
+        const float4 xa = src[0], xb = src[1];
+        const float x[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+        float sum[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          sum[k] = 0.f;
+#pragma unroll
+          for (int d = 0; d < 8; ++d) {
+            const float diff = x[d] - e[k][d];
+            sum[k] = fmaf(diff, diff, sum[k]);
+          }
+        }
+        // each lane goes on with half of the entries until one is left
+#pragma unroll
+        for (int o = 16; o >= 8; o >>= 1) {
+          const bool upper = (lane & o) != 0;
+#pragma unroll
+          for (int k = 0; k < o / 8; ++k) {
+            const float keep = upper ? sum[k + o / 8] : sum[k], give = upper ? sum[k] : sum[k + o / 8];
+            sum[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+          }
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], o);
+        if ((lane & 7) == i && mine >= 0 && sum[0] < least) {        // entries come in ascending order
+          least = sum[0];
+          win = mine;
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 8; o <= 16; o <<= 1) {
+      const float d = __shfl_xor_sync(0xffffffffu, least, o);
+      const int j = __shfl_xor_sync(0xffffffffu, win, o);
+      if (d < least || (d == least && j < win)) {          // ties go to the lower index (argmin's rule)
+        least = d;
+        win = j;
+      }
+    }
+    if (lane < kBatch) nearest[q * kBatch + lane] = make_uint2(__float_as_uint(least), static_cast<uint32_t>(win));
+    team_sync(lg);
+    if (place >= 0) {
+      uint2 best = nearest[place];
+#pragma unroll
+      for (int i = 1; i < 4; ++i) {
+        const uint2 n = nearest[i * kBatch + place];
+        const float d = __uint_as_float(n.x), d0 = __uint_as_float(best.x);
+        if (d < d0 || (d == d0 && n.y < best.y)) best = n;
+      }
+      code = static_cast<int>(best.y);
+    }
+    team_sync(lg);                                 // before the area is written again
+  }
+  return code;
 }
 }  // namespace rvqt
 
@@ -400,14 +542,18 @@ rvq_tiles_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
                       const uint32_t old = list[i];
                       if (__uint_as_float(old & ~2047u) >= lead - margin) list[n++] = old;
                     }
-                    if (n == kList) {
+                    if (n == kList) {              // they stay in the list, what comes is marked
                       n = kMany;
+#pragma unroll 1
+                      for (int i = static_cast<int>(buf); i < n_steps; i += 2)
+                        sh->more[i * 4 + (q & 1) * 2][row] = sh->more[i * 4 + (q & 1) * 2 + 1][row] = 0u;
                       break;
                     }
                   }
                   list[n++] = key + static_cast<uint32_t>(__ffs(mask) - 1);
                 }
               }
+              if (mask != 0u) sh->more[nt * 4 + (q & 1) * 2 + part][row] = mask;
               __syncwarp();
             }
           }
@@ -438,27 +584,20 @@ rvq_tiles_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
         const int n = kept.x + kept.y + kept.z + kept.w;
         if (n == 0 && q == 0 && v < a.rows && status != nullptr) atomicMax(status, static_cast<int>(kErrNonFinite));     // not finite
         if (n == 1) code = static_cast<int>(sh->list[row][kept.x != 0 ? 0 : (kept.y != 0 ? 1 : (kept.z != 0 ? 2 : 3))][0] & 2047u);       // the only candidate has won
-        // The others' residuals cross shared memory, a few vectors at a time, and a warp takes a vector: its candidates' distances,
-        // added up as in fm_rvq.cu.  (The four warps come to the same rounds.)
+        // The others' residuals cross shared memory, a few vectors at a time, where the team's FP16 copies lay (their products are
+        // complete), and a warp takes a vector: its candidates' distances, added up as in fm_rvq.cu.  (The four warps come to the same
+        // rounds.)
+        const unsigned many = __ballot_sync(0xffffffffu, kept.x == kMany || kept.y == kMany || kept.z == kMany || kept.w == kMany);
+        uint8_t* area = smem_x + lg * (32 * 128);
 #pragma unroll 1
-        for (unsigned open = __ballot_sync(0xffffffffu, n > 1); open != 0u;) {
+        for (unsigned open = __ballot_sync(0xffffffffu, n > 1) & ~many; open != 0u;) {
           unsigned rest = open;
 #pragma unroll
           for (int i = 0; i < kBatch; ++i) rest &= rest - 1u;
           const unsigned batch = open ^ rest;
           const int place = __popc(batch & ((1u << lane) - 1u));
           const bool mine = (batch >> lane & 1u) != 0u;
-#pragma unroll
-          for (int part = 0; part < 2; ++part) {
-            uint32_t x[32];
-            tmem_ld32(t_residual + part * 32, x);
-            tmem_ld_wait();
-            if (mine) {
-#pragma unroll
-              for (int c = 0; c < 8; ++c)
-                *reinterpret_cast<uint4*>(&sh->exact[lg][place][q * 64 + part * 32 + 4 * c]) = make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
-            }
-          }
+          stage(area, mine ? place : -1, q, t_residual);
           team_sync(lg);
 #pragma unroll 1
           for (int i = q; i < __popc(batch); i += 4) {
@@ -466,12 +605,11 @@ rvq_tiles_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
             for (int k = 0; k < i; ++k) behind &= behind - 1u;
             const int r = lg * 32 + __ffs(behind) - 1;
             const uchar4 count = *reinterpret_cast<const uchar4*>(sh->listed[r]);
-            const bool every = count.x == kMany || count.y == kMany || count.z == kMany || count.w == kMany;
-            const int entries = every ? a.n_codes : count.x + count.y + count.z + count.w;
+            const int entries = count.x + count.y + count.z + count.w;
             // lane k * kList + i: place i of thread k's list
             const uint32_t key = sh->list[r][lane / kList][lane % kList];
             unsigned keys = __ballot_sync(0xffffffffu, lane % kList < sh->listed[r][lane / kList]);
-            const float4* src = reinterpret_cast<const float4*>(sh->exact[lg][i]) + 2 * lane;
+            const float4* src = reinterpret_cast<const float4*>(staged(area, i)) + 2 * lane;
             const float4 xa = src[0], xb = src[1];
             const float x[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
             float least = INFINITY;
@@ -484,7 +622,7 @@ rvq_tiles_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
               for (int k = 0; k < 4; ++k) {
                 const int from = __shfl_sync(0xffffffffu, static_cast<int>(key & 2047u), (__ffs(keys) - 1) & 31);
                 keys &= keys - 1u;
-                j[k] = c + k < entries ? (every ? c + k : from) : -1;
+                j[k] = c + k < entries ? from : -1;
                 if (j[k] >= 0) load_global8(book + static_cast<size_t>(j[k]) * kDim + 8 * lane, e[k]);
               }
 #pragma unroll
@@ -514,6 +652,10 @@ rvq_tiles_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
           team_sync(lg);
           if (mine) code = sh->winner[row];
           open = rest;
+        }
+        if (many != 0u) {
+          const int found = decide_crowd(sh, area, book, many, t_residual, n_steps);
+          if ((many >> lane & 1u) != 0u) code = found;
         }
         if (q == 0 && v < a.rows) s.codes[static_cast<long long>(layer) * a.rows + v] = code;
       }

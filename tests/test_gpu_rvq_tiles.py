@@ -46,18 +46,59 @@ def test_codes_equal_the_chains(rows, layers, entries, scale):
     assert int(cand.max()) > 1                   # exact distances did decide somewhere
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("same", [9, 40, 700])   # beyond what a thread, a vector remembers; of every block's entries
-def test_entries_that_are_the_same(same):
+def _tiles(x, *books):
+    """Codes of one or two stacks over ``x`` from the kernel itself, whether or not it is the faster form."""
+    import fast_mimi_b200 as fm
+    from fast_mimi_b200 import _native
+    codes = [torch.empty(b.layers, len(x), dtype=torch.int64, device="cuda") for b in books]
+    stacks = (_native.RvqStack * len(books))(*[_stack(x.data_ptr(), b.half.data_ptr(), b.vectors.data_ptr(), b.sq.data_ptr(), b.e_max, c.data_ptr(), b.layers)
+                                               for b, c in zip(books, codes)])
+    st = fm.ops.new_status("cuda")
+    rc = _native.load().fm_rvq_encode_tiles_f32(stacks, len(books), len(x), books[0].entries, fm.ops.RVQ_TAU_REL[torch.float32], st.data_ptr(),
+                                                torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and fm.ops.read_status(st) == 0
+    return codes
+
+
+def _repeated(same, every, rows, layers=2, entries=2048):
+    """``same`` equal entries in every codebook, and vectors of which one in ``every`` wants them, again for what is left."""
     import fast_mimi_b200 as fm
     gen = torch.Generator(device="cuda").manual_seed(same)
-    e = _books(2, 2048, gen, same)
-    books = fm.ops.RVQCodebooks(e)
-    x = torch.randn(9000, 256, device="cuda", generator=gen)
-    x[::50] = e[0, 100] * 0.9                    # these want the repeated entry, and again for what is left
+    e = _books(layers, entries, gen, same)
+    x = torch.randn(rows, 256, device="cuda", generator=gen)
+    x[::every] = e[0, 100] * 0.9
+    return x, fm.ops.RVQCodebooks(e)
+
+
+# more than a thread remembers; than a vector's four threads do; of every thread's share; every vector, a batch of one
+@pytest.mark.gpu
+@pytest.mark.parametrize("same,every,entries", [(9, 50, 2048), (40, 50, 2048), (40, 3, 512), (700, 50, 2048), (1900, 1, 2048), (9, 255, 256)])
+def test_entries_that_are_the_same(same, every, entries):
+    import fast_mimi_b200 as fm
+    x, books = _repeated(same, every, 900, entries=entries)
     want = fm.ops.rvq_encode(x, books, return_candidates=True)[0]
-    got = fm.ops.rvq_encode(x, books)
-    assert torch.equal(got, want) and bool((got[0, ::50] == 100).all())
+    got, = _tiles(x, books)
+    assert torch.equal(got, want) and bool((got[0, ::every] == 100).all())
+
+
+# An empty codebook's entries, one in fifty, one in ten, each of the vectors; the chain looks at the marked entries alone.  The kernel is 0.7
+# to 1.2 of it; where full lists made all entries candidates it was 9 to 34.
+@pytest.mark.gpu
+@pytest.mark.parametrize("same,every", [(9, 1), (40, 50), (40, 10), (600, 50)])
+def test_entries_that_are_the_same_cost_no_more_than_in_the_chain(same, every):
+    import fast_mimi_b200 as fm
+    x, books = _repeated(same, every, 18000, layers=8)
+
+    def time(**kw):
+        fm.ops.rvq_encode(x, books, **kw)
+        events = [torch.cuda.Event(enable_timing=True) for _ in range(6)]
+        for ev in events:
+            ev.record()
+            fm.ops.rvq_encode(x, books, **kw)
+        torch.cuda.synchronize()
+        return min(a.elapsed_time(b) for a, b in zip(events, events[1:]))
+
+    assert time() < 2 * time(return_candidates=True)
 
 
 @pytest.mark.gpu
