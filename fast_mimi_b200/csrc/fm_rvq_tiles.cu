@@ -43,6 +43,7 @@ constexpr int kList = 8;                                       // candidates tha
 constexpr int kMany = 255;                                     // ... or more than that: the others are marked in `more`
 constexpr int kWords = 2048 / kGroup;                          // of marks
 constexpr int kBatch = 8, kBatchPitch = 1040;                  // of 32 vectors, how many are decided exactly at once; bytes from one to the next
+constexpr int kMarks = 2 * kBatchPitch + 3 * 32;                // behind them
 constexpr int kMaxLayers = 32, kMaxPairs = 80;
 constexpr int kTmemCols = 512, kResidual = 2 * kEntries;       // columns: two accumulators, then the residuals
 
@@ -132,7 +133,13 @@ __device__ __forceinline__ uint32_t round_up(float v) {
   const uint32_t b = __float_as_uint(v);
   return ((b >> 31) != 0u ? b : b + 2047u) & ~2047u;
 }
-__device__ __forceinline__ uint8_t* staged(uint8_t* area, int i) { return area + (i >> 1) * kChunkBytes + (i & 1) * kBatchPitch; }
+// A score as a number beyond kList, no smaller.
+__device__ __forceinline__ uint32_t full(float v) {
+  const uint32_t b = __float_as_uint(v);
+  return b > kList ? b : kList + 1;
+}
+// Place i of a batch in a team's 4 KB of each chunk; eight places begin on different banks.
+__device__ __forceinline__ uint8_t* staged(uint8_t* area, int i) { return area + (i >> 1) * (kChunkBytes + 32) + (i & 1) * kBatchPitch; }
 
 // Residuals of a team's vectors into their places in `area` (this thread's slice; -1: not this one).
 __device__ __forceinline__ void stage(uint8_t* area, int place, int q, uint32_t t_residual) {
@@ -149,15 +156,16 @@ __device__ __forceinline__ void stage(uint8_t* area, int place, int q, uint32_t 
   }
 }
 
-// Vectors whose lists were full have many candidates, and much the same ones (entries that are equal, or nearly).  So each entry that is one
-// for any vector of the batch that is staged in `area` is read once, by one of the team's four warps, four of them at a time, and its distance
-// from all of the batch found, added up as ever.  (18000 vectors x 8 layers, 9 entries of zero in every codebook 295 us, 40 411, 600 2360, in the
-// chain 284, 388 and 2340; with one warp a vector and all 2048 entries as its candidates 7900, 10400 and 23600.)  Lane 8 * k + i keeps the nearest to vector i of the entries that came k-th.  Few registers: the loops over
-// scores need them all.  Returns the code of the thread's vector, if it is one of `many`.
-__device__ __forceinline__ int decide_crowd(Shared* sh, uint8_t* area, const float* book, unsigned many, uint32_t t_residual, int n_steps) {
+// Vectors whose lists are full have many candidates, and much the same ones (entries that are equal, or nearly).  So each entry that is one for
+// any vector of the batch that is staged in `area` is read once, by one of the team's four warps, four of them at a time, and its distance from
+// all of the batch found, added up as ever.  (18000 vectors x 8 layers, 9 entries of zero in every codebook 224 us, 40 263, 600 961; in the chain
+// 284, 388 and 2340.  With one warp a vector and all 2048 entries as its candidates 7900, 10400 and 23600.)  Lane 8 * k + i keeps the nearest to
+// vector i of the entries that came k-th.  Returns the code of the thread's vector, if it is one of `many`.  A function of its own: the loops
+// over scores need all registers.
+__device__ __noinline__ int decide_crowd(Shared* sh, uint8_t* area, const float* book, unsigned many, uint32_t t_residual, int n_steps) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lg = warp & 3, q = warp >> 2, row = lg * 32 + lane;
-  uint32_t* marks = reinterpret_cast<uint32_t*>(area + 2 * kBatchPitch);                  // [kWords]
-  uint2* nearest = reinterpret_cast<uint2*>(area + 2 * kBatchPitch + 4 * kWords);        // [warp of the team][kBatch]: distance, entry
+  uint32_t* marks = reinterpret_cast<uint32_t*>(area + kMarks);                            // [kWords]
+  uint2* nearest = reinterpret_cast<uint2*>(area + kMarks + 4 * kWords);               // [warp of the team][kBatch]: distance, entry
   int code = 0;
 #pragma unroll 1
   while (many != 0u) {
@@ -212,7 +220,7 @@ __device__ __forceinline__ int decide_crowd(Shared* sh, uint8_t* area, const flo
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int j = next();
-        load_global8(book + static_cast<size_t>(j >= 0 ? j : 0) * kDim + 8 * lane, e[k]);        // (under a test e would be alive all along)
+        load_global8(book + static_cast<size_t>(j >= 0 ? j : 0) * kDim + 8 * lane, e[k]);
         if ((lane >> 3) == k) mine = j;
       }
 #pragma unroll 1
@@ -485,11 +493,11 @@ rvq_tiles_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
         if (!(margin < INFINITY) || vector(w.tile) >= a.rows) margin = NAN;
       }
       // ---- the scores of this thread's entries
+      uint32_t n = 0u;                             // of them in its list; beyond kList: it is full, and the largest of what it remembers
       {
         uint32_t* list = sh->list[row][q];
         volatile float* known = sh->lead[row];
         float best = -INFINITY;
-        int n = 0;
 #pragma unroll 1
         for (int nt = static_cast<int>(buf); nt < n_steps; nt += 2, ++use) {
           // what the other three know is as good a bound, however old
@@ -532,34 +540,41 @@ rvq_tiles_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
                     if (__uint_as_float(raw[c]) >= limit) mask |= 1u << c;
                 }
               }
-              if (n != kMany) {
-                const uint32_t key = round_up(top) | static_cast<uint32_t>(nt * kEntries + (q & 1) * kShare + part * kGroup);
-                for (; mask != 0u; mask &= mask - 1u) {
-                  if (n == kList) {                // those that are out of reach by now go
-                    n = 0;
+              const uint32_t key = round_up(top) | static_cast<uint32_t>(nt * kEntries + (q & 1) * kShare + part * kGroup);
+              for (; mask != 0u; mask &= mask - 1u) {
+                if (n >= kList) {
+                  if (n > kList) {                 // entries are marked; if all that it remembers is out of reach by now, it begins anew
+                    if (lead - margin > __uint_as_float(n)) n = 0u;
+                  } else {                         // those that are out of reach by now go, or they stay in the list and what comes is marked
+                    n = 0u;
+                    float most = -INFINITY;
 #pragma unroll 1
                     for (int i = 0; i < kList; ++i) {
                       const uint32_t old = list[i];
-                      if (__uint_as_float(old & ~2047u) >= lead - margin) list[n++] = old;
+                      const float score = __uint_as_float(old & ~2047u);
+                      most = fmaxf(most, score);
+                      if (score >= lead - margin) list[n++] = old;
                     }
-                    if (n == kList) {              // they stay in the list, what comes is marked
-                      n = kMany;
+                    if (n == kList) {
+                      n = full(most);
 #pragma unroll 1
                       for (int i = static_cast<int>(buf); i < n_steps; i += 2)
                         sh->more[i * 4 + (q & 1) * 2][row] = sh->more[i * 4 + (q & 1) * 2 + 1][row] = 0u;
-                      break;
                     }
                   }
-                  list[n++] = key + static_cast<uint32_t>(__ffs(mask) - 1);
+                  if (n > kList) {
+                    sh->more[nt * 4 + (q & 1) * 2 + part][row] = mask;
+                    n = full(fmaxf(top, __uint_as_float(n)));
+                    break;
+                  }
                 }
+                list[n++] = key + static_cast<uint32_t>(__ffs(mask) - 1);
               }
-              if (mask != 0u) sh->more[nt * 4 + (q & 1) * 2 + part][row] = mask;
               __syncwarp();
             }
           }
           known[q] = best;
         }
-        sh->listed[row][q] = static_cast<uint8_t>(n);
       }
       team_sync(lg);
       // ---- the decision; every entry that is within the margin of the largest score of all four threads
@@ -570,27 +585,28 @@ rvq_tiles_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
       {
         const float4 l = *reinterpret_cast<const float4*>(sh->lead[row]);
         const float limit = fmaxf(max3(l.x, l.y, l.z), l.w) - margin;
-        const int listed = sh->listed[row][q];
-        if (listed != kMany) {
-          int kept = 0;
-          for (int i = 0; i < listed; ++i) {
+        int kept_here = 0;
+        if (n <= kList) {
+          for (int i = 0; i < static_cast<int>(n); ++i) {
             const uint32_t key = sh->list[row][q][i];
-            if (__uint_as_float(key & ~2047u) >= limit) sh->list[row][q][kept++] = key;
+            if (__uint_as_float(key & ~2047u) >= limit) sh->list[row][q][kept_here++] = key;
           }
-          sh->listed[row][q] = static_cast<uint8_t>(kept);
+        } else if (__uint_as_float(n) >= limit) {
+          kept_here = kMany;
         }
+        sh->listed[row][q] = static_cast<uint8_t>(kept_here);
         team_sync(lg);
         const uchar4 kept = *reinterpret_cast<const uchar4*>(sh->listed[row]);
-        const int n = kept.x + kept.y + kept.z + kept.w;
-        if (n == 0 && q == 0 && v < a.rows && status != nullptr) atomicMax(status, static_cast<int>(kErrNonFinite));     // not finite
-        if (n == 1) code = static_cast<int>(sh->list[row][kept.x != 0 ? 0 : (kept.y != 0 ? 1 : (kept.z != 0 ? 2 : 3))][0] & 2047u);       // the only candidate has won
+        const int all = kept.x + kept.y + kept.z + kept.w;
+        if (all == 0 && q == 0 && v < a.rows && status != nullptr) atomicMax(status, static_cast<int>(kErrNonFinite));     // not finite
+        if (all == 1) code = static_cast<int>(sh->list[row][kept.x != 0 ? 0 : (kept.y != 0 ? 1 : (kept.z != 0 ? 2 : 3))][0] & 2047u);       // the only candidate has won
         // The others' residuals cross shared memory, a few vectors at a time, where the team's FP16 copies lay (their products are
         // complete), and a warp takes a vector: its candidates' distances, added up as in fm_rvq.cu.  (The four warps come to the same
         // rounds.)
         const unsigned many = __ballot_sync(0xffffffffu, kept.x == kMany || kept.y == kMany || kept.z == kMany || kept.w == kMany);
         uint8_t* area = smem_x + lg * (32 * 128);
 #pragma unroll 1
-        for (unsigned open = __ballot_sync(0xffffffffu, n > 1) & ~many; open != 0u;) {
+        for (unsigned open = __ballot_sync(0xffffffffu, all > 1) & ~many; open != 0u;) {
           unsigned rest = open;
 #pragma unroll
           for (int i = 0; i < kBatch; ++i) rest &= rest - 1u;
@@ -623,7 +639,8 @@ rvq_tiles_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
                 const int from = __shfl_sync(0xffffffffu, static_cast<int>(key & 2047u), (__ffs(keys) - 1) & 31);
                 keys &= keys - 1u;
                 j[k] = c + k < entries ? from : -1;
-                if (j[k] >= 0) load_global8(book + static_cast<size_t>(j[k]) * kDim + 8 * lane, e[k]);
+                // not under a test: e would be alive all through the kernel (18000 vectors x 8 layers 189 us instead of 180)
+                load_global8(book + static_cast<size_t>(j[k] >= 0 ? j[k] : 0) * kDim + 8 * lane, e[k]);
               }
 #pragma unroll
               for (int k = 0; k < 4; ++k) {

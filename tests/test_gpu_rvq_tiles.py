@@ -81,8 +81,9 @@ def test_entries_that_are_the_same(same, every, entries):
     assert torch.equal(got, want) and bool((got[0, ::every] == 100).all())
 
 
-# An empty codebook's entries, one in fifty, one in ten, each of the vectors; the chain looks at the marked entries alone.  The kernel is 0.7
-# to 1.2 of it; where full lists made all entries candidates it was 9 to 34.
+# Repeated entries that every vector wants, one in fifty, one in ten; the chain looks at the marked entries alone.  The kernel takes 0.16 to
+# 0.8 of its time; where full lists made all entries candidates it was 9 to 34 times the chain's, and with marks that a better score did not
+# wipe out 1.3 times.
 @pytest.mark.gpu
 @pytest.mark.parametrize("same,every", [(9, 1), (40, 50), (40, 10), (600, 50)])
 def test_entries_that_are_the_same_cost_no_more_than_in_the_chain(same, every):
@@ -98,7 +99,7 @@ def test_entries_that_are_the_same_cost_no_more_than_in_the_chain(same, every):
         torch.cuda.synchronize()
         return min(a.elapsed_time(b) for a, b in zip(events, events[1:]))
 
-    assert time() < 2 * time(return_candidates=True)
+    assert time() < 1.25 * time(return_candidates=True)
 
 
 @pytest.mark.gpu
