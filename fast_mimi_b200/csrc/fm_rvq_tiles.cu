@@ -24,11 +24,13 @@
 #include "fm_common.cuh"
 #include "fm_kernels.h"
 #include "fm_launch.h"
+#include "fm_rvq_deal.h"
 
 namespace fm {
 
 namespace rvqt {
 constexpr int kDim = 256, kBlockM = 128, kTileRows = 2 * kBlockM;
+static_assert(kTileRows == RvqDeal::kTileRows, "what is dealt");
 constexpr int kEpiWarps = 16, kThreads = (kEpiWarps + 4) * 32;
 constexpr int kEpiRegs = 112, kIssueRegs = 32;
 static_assert(512 * kEpiRegs + 128 * kIssueRegs <= kThreads * 96, "register pool of the launch");
@@ -44,7 +46,7 @@ constexpr int kMany = 255;                                     // ... or more th
 constexpr int kWords = 2048 / kGroup;                          // of marks
 constexpr int kBatch = 8, kBatchPitch = 1040;                  // of 32 vectors, how many are decided exactly at once; bytes from one to the next
 constexpr int kMarks = 2 * kBatchPitch + 3 * 32;                // behind them
-constexpr int kMaxLayers = 32, kMaxPairs = 80;
+constexpr int kMaxLayers = 32;
 constexpr int kTmemCols = 512, kResidual = 2 * kEntries;       // columns: two accumulators, then the residuals
 
 struct Stack {
@@ -60,7 +62,7 @@ struct Args {
   Stack stack[2];
   int rows, n_codes;
   float tau_rel;
-  int first[2][kMaxPairs + 1];         // pair i has the tiles first[s][i] .. first[s][i + 1] of stack s
+  RvqDeal deal;
 };
 
 // What a pair works on: its tiles of the first stack, then those of the second, layer by layer.
@@ -69,10 +71,10 @@ struct Walk {
   int stack, tile, layer, layers;
   bool alive;
   __device__ __forceinline__ Walk(const Args& a, int pair) {
-    next = a.first[0][pair];
-    end = a.first[0][pair + 1];
-    next1 = a.first[1][pair];
-    end1 = a.first[1][pair + 1];
+    next = a.deal.first[0][pair];
+    end = a.deal.first[0][pair + 1];
+    next1 = a.deal.first[1][pair];
+    end1 = a.deal.first[1][pair + 1];
     open(a);
   }
   __device__ __forceinline__ void open(const Args& a) {
@@ -711,32 +713,6 @@ rvq_tiles_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
 }
 
 namespace {
-// Deals the tiles of both stacks to `pairs` pairs: those of the longer stack evenly, those of the other to whoever has fewest
-// layers so far.
-void deal(rvqt::Args* a, int tiles, int stacks, int pairs) {
-  int load[rvqt::kMaxPairs], count[2][rvqt::kMaxPairs] = {};
-  for (int p = 0; p < pairs; ++p) {
-    count[0][p] = tiles / pairs + (p < tiles % pairs ? 1 : 0);
-    load[p] = count[0][p] * a->stack[0].layers;
-  }
-  for (int left = stacks == 2 ? tiles : 0; left > 0;) {
-    int least = load[0];
-    for (int p = 1; p < pairs; ++p) least = load[p] < least ? load[p] : least;
-    for (int p = 0; p < pairs && left > 0; ++p) {
-      if (load[p] != least) continue;
-      ++count[1][p];
-      load[p] += a->stack[1].layers;
-      --left;
-    }
-  }
-  for (int s = 0; s < 2; ++s) {
-    a->first[s][0] = 0;
-    for (int p = 0; p < pairs; ++p) a->first[s][p + 1] = a->first[s][p] + count[s][p];
-  }
-}
-}  // namespace
-
-namespace {
 // What the kernel needs of its stacks: -|e|^2 / 2 has to fit FP16 times the largest power of two that FP16 holds, and entries are read
 // by whole sectors.  0, -1, or -3 for an address.
 int cannot(const RvqStack* stacks, int n_stacks, long long rows, int n_codes) {
@@ -758,23 +734,15 @@ int cannot(const RvqStack* stacks, int n_stacks, long long rows, int n_codes) {
 }
 }  // namespace
 
-// The time has to pay.  A pair takes 26 us a layer however few vectors it has, whereas the chain spreads a layer over the whole device, so what counts
-// is how evenly tiles come out (1 + 7 layers, in us, chain -> here: 6000 vectors 146 -> 169, 9000 172 -> 171,
-// 16000 248 -> 182, 18944, the most that a tile per pair holds, 276 -> 210, 24000 332 -> 339, 32000 417 -> 385, 48000 645 -> 548, 64000
-// 831 -> 716; 32 layers of 16000 973 -> 711).  The chain's layer is 13.5 us + 1.1 for every 1000 vectors, 1.65 for those past 32000, whose
-// records and residuals no longer stay in L2.
+static RvqDeal deal_stacks(const RvqStack* stacks, int n_stacks, long long rows) {
+  const int l0 = stacks[0].layers, l1 = n_stacks == 2 ? stacks[1].layers : 0;
+  RvqDeal deal;
+  deal.make(rows, l0 > l1 ? l0 : l1, l0 > l1 ? l1 : l0 * (n_stacks - 1), sm_count());
+  return deal;
+}
+
 bool rvq_tiles_take(const RvqStack* stacks, int n_stacks, long long rows, int n_codes) {
-  using namespace rvqt;
-  if (cannot(stacks, n_stacks, rows, n_codes) != 0) return false;
-  int layers = 0, longer = 0;
-  for (int i = 0; i < n_stacks; ++i) {
-    layers += stacks[i].layers;
-    longer = stacks[i].layers > longer ? stacks[i].layers : longer;
-  }
-  const long long tiles = (rows + kTileRows - 1) / kTileRows, pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
-  const long long even = (tiles * layers + pairs - 1) / pairs, uneven = (tiles + pairs - 1) / pairs * longer;    // layers of the busiest pair
-  const double chain = 13.5 + 1.1e-3 * static_cast<double>(rows) + (rows > 32000 ? 0.55e-3 * static_cast<double>(rows - 32000) : 0.0);
-  return 26.0 * static_cast<double>(even > uneven ? even : uneven) < chain * layers;
+  return cannot(stacks, n_stacks, rows, n_codes) == 0 && rows > 0 && rvq_tiles_pay(deal_stacks(stacks, n_stacks, rows), rows, n_codes);
 }
 
 int launch_rvq_tiles(const RvqStack* stacks, int n_stacks, long long rows, int n_codes, float tau_rel, int* status, cudaStream_t st) {
@@ -807,16 +775,11 @@ int launch_rvq_tiles(const RvqStack* stacks, int n_stacks, long long rows, int n
   a.rows = static_cast<int>(rows);
   a.n_codes = n_codes;
   a.tau_rel = tau_rel;
-  const long long tiles = (rows + kTileRows - 1) / kTileRows;
-  int pairs = sm_count() / 2;
-  if (pairs > kMaxPairs) pairs = kMaxPairs;
-  if (pairs < 1) pairs = 1;
-  if (tiles * n_stacks < pairs) pairs = static_cast<int>(tiles) * n_stacks;
-  deal(&a, static_cast<int>(tiles), n_stacks, pairs);
+  a.deal = deal_stacks(stacks, n_stacks, rows);
   const uint32_t idesc = umma_idesc_f16(kTileRows, kEntries, 0, 0, 0, 0);
   rc = ensure_dynamic_smem(reinterpret_cast<const void*>(rvq_tiles_kernel), kSmemBytes);
   if (rc != 0) return rc;
-  return launch_kernel(rvq_tiles_kernel, dim3(static_cast<unsigned>(2 * pairs)), kThreads, kSmemBytes, st, 1, 0, maps[0], maps[1], a, idesc, status);
+  return launch_kernel(rvq_tiles_kernel, dim3(static_cast<unsigned>(2 * a.deal.pairs)), kThreads, kSmemBytes, st, 1, 0, maps[0], maps[1], a, idesc, status);
 }
 
 }  // namespace fm
