@@ -21,6 +21,8 @@
 // FP32 scores and 6 * 2^-11 |x||e| = 2.93e-3 |x||e| with FP16 scores.  The true winner's d may be too high and the
 // approximate minimum too low by that much each, so the candidate margin must be twice the bound: 3.9e-3 and
 // 5.86e-3.  Callers pass 4.5e-3 / 6.0e-3.
+#include <type_traits>
+
 #include "fm_common.cuh"
 #include "fm_kernels.h"
 #include "fm_launch.h"
@@ -355,6 +357,10 @@ rvq_decode_kernel(const long long* __restrict__ codes, const float* __restrict__
 // codes as the caller holds them.  64 threads per frame, four dimensions each.  Bound by the latency of two dependent loads, a code and
 // its entry, so eight codes are on their way at once, then eight entries, added in the layers' order.  (Where every code was looked at
 // before the next was asked for, a frame cost eight times that latency: 8000 frames of 8 codes 34 -> 19 us, 64000 204 -> 99, of 32 codes 794 -> 332.)
+// kLast: what holds the codes behind the last whole eight, 1, 2, 4 or 8.  What is past the end repeats the last code and is not added: a test
+// in front of its load would make the loads wait for one another.  (Eight always: 8000 frames of one code 9.7 us instead of 5.0, of nine 19.3
+// instead of 14.2.  Six or seven, which one by one took 10.3 and 11.2, are 11.6 and 12.0.)
+template <int kLast>
 __global__ void __launch_bounds__(256)
 rvq_decode_split_kernel(const long long* __restrict__ codes, const float* __restrict__ books0, const float* __restrict__ books1,
                         uint16_t* __restrict__ hi, uint16_t* __restrict__ lo, int rows, int T, int n_layers, int n0, int n_codes0,
@@ -365,14 +371,15 @@ rvq_decode_split_kernel(const long long* __restrict__ codes, const float* __rest
     const long long b = row / T, t = row - b * T;
     const long long* code = codes + b * n_layers * T + t;
     float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-    for (int l = 0; l < n_layers; l += 8) {
-      long long c[8];
+    auto add = [&](auto count, int l) {
+      constexpr int kCount = decltype(count)::value;
+      long long c[kCount];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) c[i] = code[static_cast<long long>(l + i < n_layers ? l + i : n_layers - 1) * T];
+      for (int i = 0; i < kCount; ++i) c[i] = code[static_cast<long long>(l + i < n_layers ? l + i : n_layers - 1) * T];
       bool bad = false;
-      float4 e[8];
+      float4 e[kCount];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < kCount; ++i) {
         const int at = l + i < n_layers ? l + i : n_layers - 1;
         const bool first = at < n0;
         const int n_codes = first ? n_codes0 : n_codes1;
@@ -382,13 +389,20 @@ rvq_decode_split_kernel(const long long* __restrict__ codes, const float* __rest
         e[i] = __ldg(reinterpret_cast<const float4*>(book) + sub);
       }
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < kCount; ++i) {
         if (l + i < n_layers) {
           float4& a = l + i < n0 ? acc[0] : acc[1];
           a.x += e[i].x; a.y += e[i].y; a.z += e[i].z; a.w += e[i].w;
         }
       }
       if (bad && bad_code != nullptr) atomicExch(bad_code, 1);
+    };
+    if constexpr (kLast == 8) {
+      for (int l = 0; l < n_layers; l += 8) add(std::integral_constant<int, 8>(), l);
+    } else {
+      int l = 0;
+      for (; l + kLast < n_layers; l += 8) add(std::integral_constant<int, 8>(), l);
+      add(std::integral_constant<int, kLast>(), l);
     }
 #pragma unroll
     for (int stack = 0; stack < 2; ++stack) {
@@ -528,9 +542,12 @@ int launch_rvq_decode_split(const long long* codes, const float* books0, const f
   if ((reinterpret_cast<uintptr_t>(books0) | reinterpret_cast<uintptr_t>(books1) | reinterpret_cast<uintptr_t>(hi) |
        reinterpret_cast<uintptr_t>(lo)) & 15u)
     return -3;
-  rvq_decode_split_kernel<<<grid_for((rows + 3) / 4, 8), 256, 0, st>>>(
-      codes, books0, books1, static_cast<uint16_t*>(hi), static_cast<uint16_t*>(lo), static_cast<int>(rows), T, n_layers, n0, n_codes0,
-      n_codes1, bad_code);
+  using Kernel = void (*)(const long long*, const float*, const float*, uint16_t*, uint16_t*, int, int, int, int, int, int, int*);
+  const int last = (n_layers - 1) % 8 + 1;
+  const Kernel kernel = last == 1 ? rvq_decode_split_kernel<1>
+                                  : (last == 2 ? rvq_decode_split_kernel<2> : (last <= 4 ? rvq_decode_split_kernel<4> : rvq_decode_split_kernel<8>));
+  kernel<<<grid_for((rows + 3) / 4, 8), 256, 0, st>>>(codes, books0, books1, static_cast<uint16_t*>(hi), static_cast<uint16_t*>(lo),
+                                                                        static_cast<int>(rows), T, n_layers, n0, n_codes0, n_codes1, bad_code);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -285,7 +285,7 @@ def test_one_kernel_search_reports_a_vector_that_is_not_finite(value):
     assert torch.equal(codes[:, keep], good[:, keep])
 
 
-@pytest.mark.parametrize("layers,n0", [(1, 1), (8, 1), (9, 3), (17, 16), (32, 1)])       # eight codes are on their way at once
+@pytest.mark.parametrize("layers,n0", [(1, 1), (2, 1), (3, 3), (4, 1), (5, 2), (8, 1), (9, 3), (12, 12), (17, 16), (32, 1)])      # eight codes at once, then 1, 2, 4 or 8
 def test_decoded_parts_of_both_stacks(layers, n0):
     """Sums in the layers' order, bit for bit, as FP16 hi + lo; codes outside a codebook are reported, wherever they stand."""
     import fast_mimi_b200 as fm
@@ -314,3 +314,27 @@ def test_decoded_parts_of_both_stacks(layers, n0):
         codes[1, l, 7] = code
         assert run()[2] == 1
         codes[1, l, 7] = before
+
+
+def test_decoding_one_code_takes_less_than_eight():
+    """A frame's time is that of its codes: 64000 frames of one take a third of eight's (three quarters where the one was asked for
+    eight times)."""
+    import fast_mimi_b200 as fm
+    g = torch.Generator(device="cuda").manual_seed(5)
+    books = torch.randn(8, 2048, 256, device="cuda", generator=g)
+    hi, lo = (torch.empty(64000, 256, dtype=torch.float16, device="cuda") for _ in range(2))
+    bad = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def time(layers):
+        codes = torch.randint(0, 2048, (512, layers, 125), device="cuda", generator=g)
+        events = [torch.cuda.Event(enable_timing=True) for _ in range(9)]
+        for ev in events:
+            ev.record()
+            for _ in range(4):
+                rc = fm._native.load().fm_rvq_decode_split(codes.data_ptr(), books.data_ptr(), None, hi.data_ptr(), lo.data_ptr(), 512, 125, layers, layers,
+                                                           2048, 0, bad.data_ptr(), torch.cuda.current_stream().cuda_stream)
+                assert rc == 0
+        torch.cuda.synchronize()
+        return min(a.elapsed_time(b) for a, b in zip(events, events[1:]))
+
+    assert time(1) < 0.55 * time(8)
