@@ -297,9 +297,16 @@ static int launch_source(const SplitGemmArgs& args, const void* w_hi, const void
 
 // Whole tiles of 256 x 256, each a chain of K / 64 slices, against the tiles and splits of K that the other kernels have for few rows
 // (K = 2048, N = 512: 1000 rows 37 us there, 49 here, 2500 rows 59 and 49; K = 512, N = 512: 2000 rows 25 and 25, 4800 rows 33 and 27;
-// K = 512, N = 256: 4096 rows 27 and 27, 16000 rows 41 and 29).
+// K = 512, N = 256: 4096 rows 27 and 27, 16000 rows 41 and 29).  With four slices the chain is little beside what a tile costs anyway,
+// and the few-row tiles are faster as long as they are one wave (K = 256, in us on the GPU alone, there and here: N = 512, 2048 rows 13.6 and
+// 15.7, 4736 rows 15.4 and 15.7, 5000 rows 20.1 and 15.8; N = 256, 4096 rows 13.6 and 15.7, 9472 rows 16.1 and 15.7, 12500 rows 22.0 and 16.2;
+// K = 384, N = 256, 4096 rows 16.9 and 17.4, N = 1024, 2048 rows 17.9 and 17.9).  And for every 256 outputs A is split anew, which many outputs and few
+// slices don't pay (K = 512, N = 4096: 2048 rows 35.3 and 33.6, 4096 rows 58.9 and 59.3, 8000 rows 92.8 and 98.0; N = 2048, 8000 rows 61.4 and
+// 59.8, 24000 rows 146 and 148; K = 1024, N = 4096, 6000 rows 134 and 132).
 bool split_gemm_takes(long long rows, int N, int K) {
-  return rows * N >= 1ll << 20 && N % sg::kBlockN == 0 && K >= 4 * sg::kBlockK && K % (2 * sg::kBlockK) == 0;
+  if (rows * N < 1ll << 20 || N % sg::kBlockN != 0 || K < 4 * sg::kBlockK || K % (2 * sg::kBlockK) != 0) return false;
+  if (K == 4 * sg::kBlockK && rows <= 0x7fffffffLL && few_row_tiles(static_cast<int>(rows), N)) return false;
+  return N < 2048 || K >= 1024 || rows * N <= 1ll << 24;
 }
 
 static bool bad_shape(long long rows, int N, int K) {

@@ -11,9 +11,10 @@ def _far(y, ref):
     return float((y.double() - ref).norm() / ref.norm())
 
 
-# Tiles of 256 rows x 256 outputs on 74 pairs: a ragged last tile, one block of a pair empty, more units than pairs.  FP32 sums of K
+# Tiles of 256 rows x 256 outputs on 74 pairs: a ragged last tile, one block of a pair empty, more units than pairs (four slices of K: as
+# many rows as more than a wave of few-row tiles).  FP32 sums of K
 # products: the bound is what the form with parts shows, within the spread of its own inputs (a tenth).
-@pytest.mark.parametrize("rows,n,k,mats", [(4097, 256, 512, 1), (2300, 512, 256, 2), (20000, 512, 512, 2), (1100, 1024, 640, 1)])
+@pytest.mark.parametrize("rows,n,k,mats", [(4097, 256, 512, 1), (4800, 512, 256, 2), (20000, 512, 512, 2), (1100, 1024, 640, 1)])
 def test_rows(rows, n, k, mats):
     import fast_mimi_b200 as fm
     ops = fm.ops
@@ -44,3 +45,38 @@ def test_convolution(B, T, C, kernel, stride):
     ref = (rows.double() @ (w[0].double() + w[1].double()).T).view(B, t_out, 512)
     assert direct == int(B * t_out >= 2048 and kernel * C % 128 == 0)
     assert got.shape == ref.shape and _far(got, ref) < 3e-6
+
+
+# Few slices and one wave of few-row tiles; many outputs, for each 256 of which the operand is split anew; the smallest of more slices, and many rows.
+@pytest.mark.parametrize("rows,n,k", [(2048, 512, 256), (4096, 256, 256), (1024, 1024, 256), (5000, 512, 256), (8000, 4096, 512), (1500, 4096, 512),
+                                      (2048, 512, 512), (3000, 512, 384), (20000, 256, 256)])
+def test_the_faster_form_is_taken(rows, n, k):
+    """Either form in a graph, so that the host's part doesn't count: the one that is taken is within a tenth of the other (1.15 to 1.17 of it for
+    few slices where rows x outputs alone decided)."""
+    import fast_mimi_b200 as fm
+    ops, lib = fm.ops, fm._native.load()
+    x = torch.randn(rows, k, device="cuda")
+    w = ops.split_half(torch.randn(n, k, device="cuda") * k ** -0.5)
+    y = torch.empty(rows, n, device="cuda")
+    stream = torch.cuda.Stream()
+
+    def direct():
+        assert lib.fm_linear_rows_f32(x.data_ptr(), w[0].data_ptr(), w[1].data_ptr(), y.data_ptr(), rows, 1, n, k, None, stream.cuda_stream) == 0
+
+    def time(call):
+        with torch.cuda.stream(stream):
+            call()
+            stream.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                for _ in range(8):
+                    call()
+            events = [torch.cuda.Event(enable_timing=True) for _ in range(9)]
+            for ev in events:
+                ev.record()
+                graph.replay()
+            stream.synchronize()
+        return min(a.elapsed_time(b) for a, b in zip(events, events[1:]))
+
+    times = time(lambda: ops._linear_parts(ops.split_half(x), w, (rows,), None)), time(direct)
+    assert times[lib.fm_split_direct(rows, n, k)] < 1.1 * min(times), times
