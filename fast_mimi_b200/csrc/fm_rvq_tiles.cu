@@ -485,8 +485,12 @@ rvq_tiles_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
     while (w.alive) {
       const Stack& s = sh->stack[w.stack];
       const int layer = w.layer;
-      // The margin of the vector (fm_rvq.cu).  Scores are half the distances, and what the tensor core cuts off beside |e|^2 / 2 is
-      // added.  Where the vector is not finite, or none, nothing is a candidate.
+      // The margin of the vector (fm_rvq.cu), halved as scores are half the distances, and what the tensor core cuts off beside
+      // |e|^2 / 2.  (It keeps addends down to 2^-25 of the largest one's power of two and cuts the result to 24 bits, as 1 - 1 + 2^-k shows.  In the
+      // last instruction the sum x.e and the least of the three parts lose less than 2^-25 of M, the larger of |x.e| and |e|^2 / 2, each, the
+      // result, which is less than 2 M, 2^-22 M, and |e|^2 was rounded by 2^-24: together 1.5 * 2^-22 M, of two scores at M = |e|^2 / 2
+      // 1.5 * 2^-22 |e|^2.  Taken: 2^-21.  For a larger M, and for the sixteen instructions before, 3e-5 |x||e| is in what tau_rel has to spare.)
+      // Where the vector is not finite, or none, nothing is a candidate.
       float margin;
       {
         const float4 sq = *reinterpret_cast<const float4*>(sh->square[row]);

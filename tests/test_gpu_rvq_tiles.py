@@ -103,6 +103,29 @@ def test_entries_that_are_the_same_cost_no_more_than_in_the_chain(same, every):
 
 
 @pytest.mark.gpu
+def test_scores_that_the_tensor_core_cuts_apart():
+    """Two entries as far from a short vector as FP32 can tell (in steps of 1/2), whose scores x.e - |e|^2 / 2 end on different steps of 1/4:
+    the lower index wins, as among equal ones.  Everything is an integer but x.e, 123 / 512 and 165 / 512 (cut to 16ths beside |e|^2 / 2), and what
+    the margin takes of the vector's length and of FP16's subnormals is less than 1/4."""
+    import fast_mimi_b200 as fm
+    gen = torch.Generator().manual_seed(1)
+    e = torch.randint(-250, 251, (1, 2048, 256), generator=gen).float()
+    e[0, :, 255] = 1000.0
+    e[0, 3, 255] = 0.0                           # shorter than the others by far more than any margin
+    e[0, 3, :2] = torch.tensor([123.0, 165.0])
+    e[0, 9] = e[0, 3]
+    e[0, 9, :2] = torch.tensor([165.0, 123.0])
+    square = float((e[0, 3].double() ** 2).sum())
+    assert 2 ** 22 < square < 2 ** 23 and (e.double() ** 2).sum(-1).max() < 2 ** 24
+    books = fm.ops.RVQCodebooks(e.cuda())
+    x = torch.zeros(300, 256, device="cuda")
+    x[::3, 0] = 2.0 ** -9
+    assert 2e-3 * 4.5e-3 * books.e_max[0] + 3.1e-5 * books.e_max[0] < 2 * 0.25
+    got, = _tiles(x, books)
+    assert torch.equal(got, fm.ops.rvq_encode(x, books, return_candidates=True)[0]) and bool((got == 3).all())
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("frames", [3100, 23, 70])        # dealt to pairs of blocks; one wave of clusters, two
 def test_both_stacks_of_a_split_quantiser(frames):
     """1 + 7 layers in one launch against either branch by itself."""
