@@ -32,21 +32,7 @@ def _books(layers, entries, gen, same=0):
     return e
 
 
-# A tile is 256 vectors and 74 pairs of blocks take one each: 18944 is the most of a wave; 9217 and 18700 end inside a block's rows.
-@pytest.mark.gpu
-@pytest.mark.parametrize("rows,layers,entries,scale", [(9217, 8, 2048, 1.0), (18944, 3, 2048, 1.0), (18700, 5, 1024, 300.0), (33000, 2, 256, 1e-3)])
-def test_codes_equal_the_chains(rows, layers, entries, scale):
-    import fast_mimi_b200 as fm
-    gen = torch.Generator(device="cuda").manual_seed(rows)
-    books = fm.ops.RVQCodebooks(_books(layers, entries, gen) * scale)
-    x = torch.randn(rows, 256, device="cuda", generator=gen) * (1.5 * scale)
-    x[5] = 0.0                                   # all margin, no direction
-    want, cand = fm.ops.rvq_encode(x, books, return_candidates=True)
-    assert torch.equal(fm.ops.rvq_encode(x, books), want)
-    assert int(cand.max()) > 1                   # exact distances did decide somewhere
-
-
-def _tiles(x, *books):
+def _tiles(x, *books, error=0):
     """Codes of one or two stacks over ``x`` from the kernel itself, whether or not it is the faster form."""
     import fast_mimi_b200 as fm
     from fast_mimi_b200 import _native
@@ -56,8 +42,39 @@ def _tiles(x, *books):
     st = fm.ops.new_status("cuda")
     rc = _native.load().fm_rvq_encode_tiles_f32(stacks, len(books), len(x), books[0].entries, fm.ops.RVQ_TAU_REL[torch.float32], st.data_ptr(),
                                                 torch.cuda.current_stream().cuda_stream)
-    assert rc == 0 and fm.ops.read_status(st) == 0
+    assert rc == 0 and fm.ops.read_status(st) == error
     return codes
+
+
+# A tile is 256 vectors, 74 pairs of blocks take one each at a time: one pair and a tile hardly begun, a wave of tiles, one more, tiles that
+# end inside a block's rows, two and three a pair, which then begin anew with other vectors behind the last layer.
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,layers,entries,scale", [(1, 2, 256, 1.0), (257, 3, 512, 1.0), (9217, 8, 2048, 1.0), (18944, 3, 2048, 1.0), (18945, 2, 2048, 1.0),
+                                                       (18700, 5, 1024, 300.0), (33000, 2, 256, 1e-3), (38000, 2, 1536, 1.0), (50001, 1, 768, 1.0),
+                                                       (3000, 32, 256, 1.0)])
+def test_codes_equal_the_chains(rows, layers, entries, scale):
+    import fast_mimi_b200 as fm
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    books = fm.ops.RVQCodebooks(_books(layers, entries, gen) * scale)
+    x = torch.randn(rows, 256, device="cuda", generator=gen) * (1.5 * scale)
+    x[5 % rows] = 0.0                            # all margin, no direction
+    want, cand = fm.ops.rvq_encode(x, books, return_candidates=True)
+    got, = _tiles(x, books)
+    assert torch.equal(got, want) and torch.equal(fm.ops.rvq_encode(x, books), want)
+    assert rows < 9000 or int(cand.max()) > 1    # exact distances did decide somewhere
+
+
+# Both stacks dealt to pairs: a tile of either, the longer one first or second; several of both, so that a pair goes on from the first to the
+# second and a few pairs have more of one and less of the other.
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,layers,entries", [(100, (1, 7), 2048), (9400, (7, 1), 2048), (9500, (3, 3), 512), (20000, (1, 3), 256), (64001, (1, 7), 2048)])
+def test_codes_of_two_stacks_equal_the_chains(rows, layers, entries):
+    import fast_mimi_b200 as fm
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    books = [fm.ops.RVQCodebooks(_books(n, entries, gen)) for n in layers]
+    x = torch.randn(rows, 256, device="cuda", generator=gen) * 1.5
+    for got, b in zip(_tiles(x, *books), books):
+        assert torch.equal(got, fm.ops.rvq_encode(x, b, return_candidates=True)[0])
 
 
 def _repeated(same, every, rows, layers=2, entries=2048):
@@ -126,7 +143,7 @@ def test_scores_that_the_tensor_core_cuts_apart():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("frames", [3100, 23, 70])        # dealt to pairs of blocks; one wave of clusters, two
+@pytest.mark.parametrize("frames", [4100, 23, 70])        # many vectors in tiles; one wave of clusters, two
 def test_both_stacks_of_a_split_quantiser(frames):
     """1 + 7 layers in one launch against either branch by itself."""
     import fast_mimi_b200 as fm
@@ -150,9 +167,7 @@ def test_a_vector_that_is_not_finite(value):
     books = fm.ops.RVQCodebooks(_books(2, 2048, gen))
     x = torch.randn(12000, 256, device="cuda", generator=gen)
     x[4321, 7] = value
-    st = fm.ops.new_status("cuda")
-    got = fm.ops.rvq_encode(x, books, status=st)
-    assert fm.ops.read_status(st) == 105
+    got, = _tiles(x, books, error=105)
     st = fm.ops.new_status("cuda")
     want = fm.ops.rvq_encode(x, books, return_candidates=True, status=st)[0]
     assert fm.ops.read_status(st) == 105
