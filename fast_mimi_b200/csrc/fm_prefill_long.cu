@@ -77,11 +77,11 @@ static_assert(smem_bytes(true) <= 232448, "exceeds the 227 KB a CTA may use");
 
 // The steps a CTA takes: an equal share of all (clip, head, query tile) triples in that order (fm_shares.h), i.e. at most a rest of
 // one sequence, whole ones, and the beginning of another; each of those is a run.  (Whole sequences dealt out in turn: 128 sequences
-// of 20 tiles took 20 steps on 128 of 148 SMs, now 18 at most, 16 FP16 clips of 2500 frames 116.6 -> 107.2 us; 200 sequences of 12
-// tiles took 24 steps, now 17.)  A run re-reads the two K / V tiles in front of it and its first step waits for all of them, so shares
-// keep to sequences where that takes no block more steps: rounded to occupy every SM, they began anywhere (FP16, 9 clips of 513 frames
-// 19.4 with segments of each sequence, 20.4 without, now 18.6; FP32, 18 of 700 42.4 -> 38.2, 36 of 257 39.4 -> 35.3, 36 of 900
-// 93.8 -> 89.1).  Every role of the kernel walks the same steps with the same counter n, which the barrier phases are derived from.
+// of 20 tiles took 20 steps on 128 of 148 SMs, now 18 at most, 200 sequences of 12 tiles 24 steps, now 17; 16 FP16 clips of 2500 frames 116.6 ->
+// 107.2 us with the chain of steps of then, which takes 98 now.)  A run re-reads the two K / V tiles in front of it and its first step waits for
+// all of them, so shares keep to sequences where that takes no block more steps: rounded to occupy every SM, they began anywhere (9 FP16
+// clips of 513 frames 20.4 us, with segments of each sequence 18.6, both of then).  Every role of the kernel walks the same steps with the
+// same counter n, which the barrier phases are derived from.
 struct Walk {
   int n_tiles, seq, t, t0, n, steps;
   __device__ __forceinline__ explicit Walk(const Shares& shares) : n_tiles(shares.tiles), n(0) {
@@ -249,7 +249,7 @@ band_attn_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         if (one) tc_commit(&sh->pv_done[n & 1]);
       }
     } else if (kF32In) {
-      // ---------------------------------------------------------- FP32 tiles into their places (two warps)
+      // ---------------------------------------------------------- FP32 tiles into their places (four warps)
       // A step's tiles in the order of their use: its new K tiles and Q, then its new V tiles; this warp has pieces 2c and
       // 2c + 1 of each.  Copies run kStaged pieces ahead of the conversion.
       const int c = role - 2;
@@ -509,12 +509,15 @@ int launch_band_attn_long(const void* q, const void* k, const void* v, void* out
 
 // Strides that a tensor map can have, and enough steps a block.  The converting warps keep up with the chain of steps, but where a
 // run begins the first step waits until they have made seven tiles instead of three, and a short call is little else; a converting
-// pass in front costs 1 us and 0.7 ns a frame.  Inside from five steps on, from seven where short sequences begin and end inside of shares.
-// GPU time, FP32, in front -> inside:
-//   1 or 2 steps   1 clip of 257 frames 8.6 -> 11.8 us, 1 of 2500 15.6 -> 20.1, 8 of 300 14.3 -> 16.3
-//   3 or 4         8 of 900 28.8 -> 31.5, 12 of 700 31.0 -> 31.9, 16 of 385 25.6 -> 26.0
-//   5 or 6         25 of 257 28.8 -> 33.6 and 25 of 385 (shares run on) 37.8 -> 41.2; 9 of 1200 38.8 -> 37.1, 18 of 513 33.8 -> 31.4
-//   7 and more     14 of 900 49.4 -> 46.5, 36 of 900 112 -> 89, 16 of 2500 135 -> 105; 45 of 257 46.5 -> 48.5
+// pass in front costs 1 us and 0.7 ns a frame.  Inside from four steps on, from six where short sequences begin and end inside of shares.
+// GPU time, FP32, in front -> inside (350 calls of 1 to 12 steps: what goes inside is 4 % slower there at most, what does not 9 % slower in front):
+//   1 or 2 steps   1 clip of 257 frames 8.7 -> 11.0 us, 1 of 2500 14.9 -> 17.1, 8 of 300 14.0 -> 14.2
+//   3              18 of 257 18.2 -> 18.2, 9 of 513 19.2 -> 19.7, 6 of 900 21.9 -> 23.0
+//   4              16 of 385 23.3 -> 22.5, 7 of 900 24.4 -> 25.4, 9 of 1000 30.9 -> 28.4, 6 of 1500 31.4 -> 27.5, 3 of 2500 28.3 -> 27.0; shares
+//                  run on: 12 of 700 29.5 -> 27.3, but 24 of 257 23.9 -> 27.1, 12 of 513 24.3 -> 26.1
+//   5              18 of 513 32.5 -> 27.3, 15 of 700 37.2 -> 32.4; run on: 25 of 257 26.3 -> 29.4, 28 of 300 30.4 -> 30.4, 23 of 385 32.3 -> 31.9
+//   6              37 of 257 35.1 -> 30.9; run on: 24 of 385 35.6 -> 34.8, 22 of 513 41.2 -> 37.4
+//   7 and more     41 of 257 41.0 -> 39.9, 19 of 700 49.0 -> 41.9, 18 of 900 57.9 -> 44.0, 11 of 2500 91.7 -> 65.7
 bool band_attn_long_takes_f32(const long long* strides, int B, int T) {
   for (int i = 0; i < 9; ++i) {
     if (i % 3 == 0 && B == 1) continue;
@@ -523,7 +526,7 @@ bool band_attn_long_takes_f32(const long long* strides, int B, int T) {
   Shares s;
   if (!long_shares(B, T, &s)) return false;
   const bool run_on = s.cuts == 0 && s.per_block % s.tiles != 0;
-  return s.per_block >= (run_on && s.tiles <= 5 ? 7 : 5);
+  return s.per_block >= (run_on && s.tiles <= 5 ? 6 : 4);
 }
 
 int launch_band_attn_long_f32(const void* const* qkv, const long long* strides, float* out, int B, int T, int window, float scale,

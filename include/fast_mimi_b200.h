@@ -101,7 +101,7 @@ int fm_band_attn_prefill_bf16(const void* q, const void* k, const void* v, void*
  *   strides   HOST array of nine: batch, head, frame strides of q, k, v in values (multiples of 16 bytes)
  *   q/k/v_ws  [B, T, 512] 16 bit: the converted tensors; NULL for one that already is frame-major and of the right type
  *             (BF16 for q and k, value_dtype for v); not written where the attention kernel rounds FP32 tensors itself (FP32
- *             result, T > 256, 129 < window <= 257, five to seven query tiles of 128 per SM and more)
+ *             result, T > 256, 129 < window <= 257, four to six query tiles of 128 per SM and more)
  *   out16     [B, T, 512] value_dtype; out32 [B, T, 512] FP32 or NULL.  With out32 the result goes there, and out16 is a
  *             workspace that may be NULL where T > 256 and 129 < window <= 257 */
 int fm_window_attention(const void* q, const void* k, const void* v, int in_dtype, const long long* strides, void* q_ws, void* k_ws,
