@@ -523,13 +523,13 @@ static bool half_units(int pair_tiles, int N, int max_pairs, int k_chunks) {
 // 14.0, 4500 (288) 16.7 -> 14.2, BF16 3678 rows 16.7 -> 14.4; K = 512, N = 512, FP32 3678 rows 8.8 -> 8.3, BF16 9.8 -> 8.5; K = 512,
 // N = 2048, GELU 500 rows (128) 8.0 -> 8.3, 1024 (256) 9.8 -> 8.3.
 // FP32 results of rows that hardly give any SM a second block are out sooner from the few-row kernel, whose last blocks are short where
-// their rows are few: K = 2048, N = 512 2305 rows 12.9 -> 14.0, 2400 13.1 -> 13.9, K = 512, N = 512 2400 rows 7.5 -> 8.1, N = 1024 1153 rows
-// 7.3 -> 7.8, 1280 8.0 -> 7.8, N = 2048 513 rows 7.3 -> 7.8.  16-bit ones are not: K = 2048, N = 512 2400 rows 14.0 -> 14.0, K = 512 8.6 -> 8.4,
-// N = 2048, GELU 513 rows 8.3 -> 8.1.
-static bool one_wave_of_halves(int M, int pair_tiles, int N, int max_pairs, bool fp32) {
+// their rows are few, in a call by itself: K = 2048, N = 512 2305 rows 12.9 -> 14.0, 2400 13.1 -> 13.9, K = 512, N = 512 2400 rows 7.5 -> 8.1, N = 1024
+// 1153 rows 7.3 -> 7.8, 1280 8.0 -> 7.8, N = 2048 513 rows 7.3 -> 7.8.  16-bit ones are not (K = 2048, N = 512 2400 rows 14.0 -> 14.0, K = 512 8.6 ->
+// 8.4, N = 2048, GELU 513 rows 8.3 -> 8.1), nor in a chain, whose next kernel finds an SM free the sooner (8 layers of 2313 rows 452 -> 430).
+static bool one_wave_of_halves(int M, int pair_tiles, int N, int max_pairs, bool fp32_alone) {
   const long long sms = sm_count();
   if (pair_tiles * static_cast<long long>(N / 128) > max_pairs) return false;
-  if (fp32) return static_cast<long long>(M) * N > (lin::kBlockM * 64 + 256) * sms;
+  if (fp32_alone) return static_cast<long long>(M) * N > (lin::kBlockM * 64 + 256) * sms;
   return static_cast<long long>((M + lin::kBlockM - 1) / lin::kBlockM) * (N / 64) > sms;
 }
 
@@ -546,7 +546,7 @@ int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, co
     return -3;
   const int pair_tiles = ((M + kBlockM - 1) / kBlockM + 1) / 2;
   const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
-  const bool one_wave = out_dtype != 3 && one_wave_of_halves(M, pair_tiles, N, max_pairs, out_dtype == 2);
+  const bool one_wave = out_dtype != 3 && one_wave_of_halves(M, pair_tiles, N, max_pairs, out_dtype == 2 && !dependent);
   if (out_dtype != 3 && !one_wave && few_row_tiles(M, N))
     return launch_linear_small(a, w, y, scale, resid, M, N, K, in_dtype, out_dtype, gelu, status, st, dependent);
   // The wide shape where the epilogue carries arithmetic (GELU, candidate records) for unit after unit, the narrow one otherwise.
