@@ -547,14 +547,14 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// Per-warpgroup register budget (four consecutive warps, aligned; one instruction executed by all of them).  A
-// kernel whose launch bound leaves every thread R registers may hand registers of warps that need few to warps that
-// need many: the donors shrink first, the receivers' request blocks until the registers are free, so the sum after
-// all requests must not exceed threads x R.
 // How far from the least approximate distance to a codebook's entries the nearest one's may lie (fm_rvq.cu): the relative part is
 // FP16 rounding of both operands, the absolute part residual values below FP16's normal range.
 __device__ __forceinline__ float rvq_margin(float xx, float e_max, float tau_rel) { return tau_rel * sqrtf(xx) * e_max + 3.1e-5f * e_max; }
 
+// Per-warpgroup register budget (four consecutive warps, aligned; one instruction executed by all of them).  A
+// kernel whose launch bound leaves every thread R registers may hand registers of warps that need few to warps that
+// need many: the donors shrink first, the receivers' request blocks until the registers are free, so the sum after
+// all requests must not exceed threads x R.
 template <int N> __device__ __forceinline__ void warpgroup_reg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }

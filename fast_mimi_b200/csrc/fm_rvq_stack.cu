@@ -12,7 +12,7 @@
 //   residual   every block subtracts the winner for itself: a warp holds its two vectors in registers all along
 // so a layer crosses the cluster twice, and nothing but codes is written.  63 vectors: 7 layers 66 -> 55 us, 31 layers 273 -> 219
 // us, and 16 launches less for stacks of 1 and 7 layers, 18 otherwise (a 5 s utterance end to end, bound by the host, 200 -> 183 us;
-// both stacks as two rows of one grid, which the device runs side by side up to three clusters each, 182 -> 169).  Of the 12300 cycles of a layer the
+// both stacks as two rows of one grid, which the device runs side by side up to three clusters each, 176 -> 172, no more than runs differ by).  Of the 12300 cycles of a layer the
 // two crossings take 4500, the products 2100 (ldmatrix at the rate of shared memory), the exact distances 1400, the new residual 2700.
 #include "fm_common.cuh"
 #include "fm_device_fact.h"

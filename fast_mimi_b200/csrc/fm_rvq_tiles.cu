@@ -11,12 +11,12 @@
 // A score has to cost little: 128 x 2048 of them a layer and block cross four schedulers while the tensor core makes them in 17400
 // cycles.  So |e|^2 is part of the product (sixteen more columns of K: -|e|^2 / 2 in three FP16 parts against a power of two), and
 // x.e - |e|^2 / 2 is only compared: the largest of 32 against the largest that the four threads of a vector have seen so far, and
-// one by one only where eight of them come within the margin of that.  What does is listed and decided at the end of the layer by
-// exact FP32 distances.
+// one by one only where eight of them come within the margin of that.  What does is listed, marked where the list is full, and decided at
+// the end of the layer by exact FP32 distances.
 //
-// Of the 46000 cycles that a layer takes 28000 are scores (the tensor core issues for 18000 of them; a thread looks at 64 scores in
-// 2100, for 2176 of products), 3000 the candidates, 6500 the exact distances of the one vector in seven that has several, 4000 the new
-// residuals (a thread reads a quarter of its vector's entry, sector by sector), 4000 until the next scores arrive.
+// Of the 42000 cycles that a layer takes 24000 are scores, 4500 of them until the first are there (the tensor core issues for 18000; a
+// thread looks at 64 scores in 2100, for 2176 of products), 3000 the candidates, 5500 the exact distances of the one vector in seven that
+// has several, 9000 the new residuals (a thread reads a quarter of its vector's entry, sector by sector).
 //
 // Warps 0-15: scores, decisions, residuals.  Warp 16: codebooks.  Warp 17: MMA (leader block only).  Warps 18, 19: -|e|^2 / 2.
 #include <math.h>
