@@ -159,6 +159,18 @@ int launch_linear_small(const void* a, const void* w, void* y, ParamVec scale, c
                         int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent);
 int launch_qkv_small(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status,
                      cudaStream_t st, int dependent);
+// Output projection, LayerNorm and MLP of a layer in one kernel (fm_layer_tail.cu), for as many rows as layer_tail_takes says:
+// y = x1 + mlp_scale * (gelu(LayerNorm(x1) w_fc1^T) w_fc2^T),  x1 = x + attn_scale * (core w_o^T).  A scale without data: one.
+struct LayerTail {
+  const void *core, *w_o, *w_fc1, *w_fc2;    // [M, 512] and [512, 512] of the value type; [2048, 512] and [512, 2048] of the MLP's
+  const void* x;                             // [M, 512] of stream_type (0 BF16, 1 FP16, 2 FP32), like y
+  void* y;
+  ParamVec attn_scale, mlp_scale, ln_weight, ln_bias;
+  float eps;
+  int stream_type, value_fp16, tc_fp16;
+};
+bool layer_tail_takes(int M, int ffn);
+int launch_layer_tail(const LayerTail& t, int M, int* status, cudaStream_t st, int dependent);
 // LayerNorm over 512 channels; x_dtype 0 BF16 / 1 FP16 / 2 FP32, y_dtype 0 BF16 / 1 FP16.
 int launch_layernorm512(const void* x, int x_dtype, ParamVec weight, ParamVec bias, float eps, void* y,
                         int y_dtype, long long rows, cudaStream_t st, int dependent = 0);

@@ -8,7 +8,8 @@
 // For few rows a layer is bound by what surrounds the arithmetic: driven kernel by kernel from Python a layer of one
 // clip cost 165 us of host time (checks, allocations, tensor maps, launches) for 84 us of GPU time.  Here the host makes
 // one call; the intermediate tensors live in one workspace of the caller; and every launch but those of other libraries
-// is allowed to begin (barriers, tensor memory, weight loads) while the kernel in front still runs.
+// is allowed to begin (barriers, tensor memory, weight loads) while the kernel in front still runs.  Up to 168 rows everything
+// behind the attention is one kernel (fm_layer_tail.cu).
 #include "../../include/fast_mimi_b200.h"
 
 #include "fm_kernels.h"
@@ -77,7 +78,8 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
     rc = launch_layernorm512(x, p.stream_dtype, vec(p.ln1_weight), vec(p.ln1_bias), p.ln1_eps, b.h, tc, rows, st, 1);
     if (rc != 0) return rc;
   }
-  const bool projected = few && stream_attn_projects(B, T);     // the attention kernel goes on to x1
+  const bool one_tail = layer_tail_takes(rows, p.ffn);          // everything behind the attention is one kernel
+  const bool projected = !one_tail && few && stream_attn_projects(B, T);     // the attention kernel goes on to x1
   const StreamOut proj = {p.w_o, x, b.x1, vec(p.attn_scale), p.stream_dtype};
   const bool few_tiles = !few && few_attn_tiles(B, T) && (!cached || slots <= 256);
   if (whole_clip && !few_tiles && use_fused_clip(B, T)) {
@@ -119,6 +121,11 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
     }
   }
   if (rc != 0) return rc;
+  if (one_tail) {
+    const LayerTail t = {b.core, p.w_o, p.w_fc1, p.w_fc2, x, y, vec(p.attn_scale), vec(p.mlp_scale), vec(p.ln2_weight), vec(p.ln2_bias),
+                         p.ln2_eps, p.stream_dtype, value_fp16, tc};
+    return launch_layer_tail(t, rows, status, st, 1);
+  }
   if (!projected) rc = launch_linear_gemm(b.core, p.w_o, b.x1, vec(p.attn_scale), x, rows, 512, 512, value_fp16, p.stream_dtype, 0, status, st, 1);
   if (rc != 0) return rc;
   if (norm2_inside) {

@@ -24,8 +24,8 @@
 // are requested before the wait for it.  A block has an item's ring rows in shared memory before it stores that item's
 // new rows, and no other block touches its (stream, head): the ring is updated in place.
 //
-// While the heads of every stream have blocks of their own at the same time (up to 15 streams on a B200) the kernel goes on to the output
-// projection, x1 = residual + scale * core W_o^T: the eight blocks of a stream are a cluster, hand each other their heads'
+// Where fm_layer_tail.cu does not take what follows (an MLP of another size than 2048) and while the heads of every stream have blocks
+// of their own at the same time (up to 15 streams on a B200), the kernel goes on to the output projection, x1 = residual + scale * core W_o^T: the eight blocks of a stream are a cluster, hand each other their heads'
 // rows through distributed shared memory, and each multiplies them with its 64 rows of W_o, which it asked for before the wait.  As
 // a kernel of its own the projection of a few rows was 4.6 us, a launch and a first load around 0.3 us of products.  The rows are sent
 // with st.async and counted where they arrive: a barrier of the cluster is a fence besides, for every warp (0.3 to 0.5 us a layer).

@@ -236,6 +236,44 @@ def test_live_streams_against_64_bits(T, past, dtype, value_dtype):
     fm.check_status()
 
 
+# rows: one, either side of a cluster's rows (8) and of what seven clusters of 8, 16 and 24 rows hold; two clips; an MLP of another size, for
+# which there is no such kernel
+@pytest.mark.parametrize("B,T,ffn", [(1, 1, 2048), (1, 8, 2048), (1, 9, 2048), (1, 56, 2048), (1, 57, 2048), (1, 112, 2048), (1, 113, 2048), (2, 61, 2048),
+                                     (1, 168, 2048), (1, 169, 2048), (1, 9, 1024)])
+@pytest.mark.parametrize("dtype,value_dtype", [(torch.float32, torch.float16), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16),
+                                               (torch.bfloat16, torch.float16), (torch.float16, torch.float16)])
+def test_layer_on_few_rows_against_64_bits(B, T, ffn, dtype, value_dtype):
+    """A layer on clips of few rows in all, where everything behind the attention is one kernel, against the same in 64 bits; bars as for
+    live streams below (BF16 values: their rounding, 2^-9, in front of the output projection).  In place it is the same bit for bit."""
+    import fast_mimi_b200 as fm
+    layer = fm.MimiTransformerLayerB200(intermediate_size=ffn, value_dtype=value_dtype).cuda()
+    p = _layer_params(T)
+    p["mlp.fc1.weight"], p["mlp.fc2.weight"] = p["mlp.fc1.weight"][:ffn].contiguous(), p["mlp.fc2.weight"][:, :ffn].contiguous()
+    layer.load_state_dict(p, strict=True)
+    layer = layer.to(dtype).requires_grad_(False)
+    g = torch.Generator(device="cuda").manual_seed(B * T)
+    x = torch.randn(B, T, 512, device="cuda", generator=g).to(dtype)
+    cos, sin = fm.rope_tables(torch.arange(T, device="cuda")[None])
+    y = layer(x, None, None, (cos, sin))[0]
+    p = {k: v.double() for k, v in layer.state_dict().items()}
+    xd = x.double()
+    norm = lambda t, name: torch.nn.functional.layer_norm(t, (512,), p[name + ".weight"], p[name + ".bias"], 1e-5)
+    q, k, v = ((norm(xd, "input_layernorm") @ p[f"self_attn.{n}_proj.weight"].T).view(B, T, 8, 64).transpose(1, 2) for n in "qkv")
+    turn = lambda t: t * cos.double()[:, None] + O.rotate_half(t) * sin.double()[:, None]
+    hidden = torch.ones(T, T, dtype=torch.bool, device="cuda").triu(1)
+    core = torch.softmax((turn(q) @ turn(k).transpose(-1, -2) * 0.125).masked_fill(hidden, float("-inf")), -1) @ v
+    x1 = xd + core.transpose(1, 2).reshape(B, T, 512) @ p["self_attn.o_proj.weight"].T * p["self_attn_layer_scale.scale"]
+    want = x1 + torch.nn.functional.gelu(norm(x1, "post_attention_layernorm") @ p["mlp.fc1.weight"].T) @ p["mlp.fc2.weight"].T * p["mlp_layer_scale.scale"]
+    base = xd if dtype == torch.float32 else torch.zeros_like(xd)
+    bar = {torch.float32: 2e-3 if value_dtype == torch.float16 else 4e-3, torch.bfloat16: 2 ** -8, torch.float16: 2 ** -10}[dtype]
+    assert O.rel_l2(y.double() - base, want - base) < bar
+    params, keep = layer._native_plan(x)
+    again = x.clone()
+    fm.ops.layer_forward(params, again, cos, sin, value_dtype=value_dtype, out=again)
+    assert torch.equal(again, y)
+    fm.check_status()
+
+
 @pytest.mark.parametrize("T", [1, 8])
 @pytest.mark.parametrize("streams", [1, 15, 16])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
