@@ -71,6 +71,7 @@ SIGNATURES: dict[str, list] = {
     "fm_linear_fp32_verify": [_P, _P, _P, _I, _I, _I, _P],
     "fm_rope_fp32_verify": [_P, _P, _P, _I, _I, _I, _I, _LL, _P],
     "fm_selftest_wait_timeout": [_P, _I, _P, _P],
+    "fm_rvq_decode_project_f32": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P],
     "fm_read_status": [_P, _P],
     "fm_read_words": [_P, _P, _P, _P],
 }
@@ -130,5 +131,6 @@ def check(rc: int, what: str) -> None:
                 -4: "cuTensorMapEncodeTiled unavailable",
                 -5: "more frames than the built-in workspace holds",
                 -7: "workspace too small",
+                -8: "no page-locked word",
                 -6: "clip length outside the fused kernel's range (128 < T <= 256)"}.get(rc, "CUDA error" if rc > 0 else "error")
         raise RuntimeError(f"{what} failed with status {rc} ({kind})")

@@ -236,6 +236,224 @@ PyObject* layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
 }
 
+// ---- The calls around the quantiser.  Nothing is kept between them: the tensors come with every call.  They return None for
+// anything out of the ordinary, (name, status) for a native call that refused, and leave raising to the Python side.
+
+const at::Tensor* tensor(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+// A plain CUDA tensor of a type and rank on the current device.
+bool plain(const at::Tensor* t, c10::ScalarType type, int64_t dim) {
+  return t != nullptr && t->is_cuda() && t->scalar_type() == type && t->dim() == dim && t->device().index() == c10::cuda::current_device();
+}
+
+// FP16 hi + lo parts of a weight [n, k] as the split-precision products take them.
+bool weight_parts(const at::Tensor* hi, const at::Tensor* lo, int64_t k) {
+  return plain(hi, at::kHalf, 2) && plain(lo, at::kHalf, 2) && hi->is_contiguous() && lo->is_contiguous() && hi->sizes() == lo->sizes() &&
+         hi->size(1) == k && k % 64 == 0 && hi->size(0) % 256 == 0 && hi->size(0) > 0;
+}
+
+PyObject* refused(const char* name, int rc) { return Py_BuildValue("(si)", name, rc); }
+
+// One allocation for two FP16 matrices of a size.
+at::Tensor two_parts(int64_t values, const at::Tensor& like) { return at::empty({2, values}, like.options().dtype(at::kHalf)); }
+
+// conv_frames(x [B, C, T], w_hi, w_lo, kernel, stride, status) -> [B, C_out, ceil(T / stride)]
+PyObject* conv_frames_checked(PyObject* const* a, Py_ssize_t n) {
+  if (n != 6) {
+    PyErr_SetString(PyExc_TypeError, "conv_frames(x, w_hi, w_lo, kernel, stride, status)");
+    return nullptr;
+  }
+  const at::Tensor *x = tensor(a[0]), *hi = tensor(a[1]), *lo = tensor(a[2]), *status = tensor(a[5]);
+  const long kernel = int_of(a[3]), stride = int_of(a[4]);
+  if (!plain(x, at::kFloat, 3) || stride < 1 || kernel < stride || kernel > 16 || !plain(status, at::kInt, 1)) Py_RETURN_NONE;
+  const int64_t B = x->size(0), C = x->size(1), T = x->size(2), t_out = (T + stride - 1) / stride;
+  if (!weight_parts(hi, lo, kernel * C) || B * T == 0 || B * (t_out + kernel) > 0x7fffffff || T > 0x7fffffff) Py_RETURN_NONE;
+  const int64_t n_out = hi->size(0);
+  const bool direct = C % 64 == 0 && fm_split_direct(B * t_out, static_cast<int>(n_out), static_cast<int>(kernel * C));
+  if (!direct && (kernel % stride != 0 || stride * C % 64 != 0)) Py_RETURN_NONE;
+  const at::Tensor frames = x->transpose(1, 2).contiguous();
+  const int64_t extra = kernel / stride - 1, rows = B * (t_out + extra), cols = stride * C;
+  at::Tensor parts;
+  if (!direct) parts = two_parts(rows * cols, frames);
+  const at::Tensor y = at::empty({B, t_out, n_out}, frames.options());
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+  const float* src = frames.const_data_ptr<float>();
+  const void *w_hi = hi->const_data_ptr(), *w_lo = lo->const_data_ptr();
+  float* out = y.data_ptr<float>();
+  int* st = status->data_ptr<int>();
+  uint16_t* part = direct ? nullptr : static_cast<uint16_t*>(parts.data_ptr());
+  const int b = static_cast<int>(B), t = static_cast<int>(T), c = static_cast<int>(C), ker = static_cast<int>(kernel), str = static_cast<int>(stride),
+            outs = static_cast<int>(n_out);
+  int rc = 0;
+  const char* what = "fm_conv_frames_f32";
+  Py_BEGIN_ALLOW_THREADS
+  if (direct) {
+    rc = fm_conv_frames_f32(src, w_hi, w_lo, out, b, t, c, ker, str, outs, st, stream);
+  } else {
+    what = "fm_conv_frames_split";
+    rc = fm_conv_frames_split(src, part, part + rows * cols, b, t, c, ker, str, stream);
+    if (rc == 0) {
+      what = "fm_linear_split_f32";
+      rc = fm_linear_split_f32(part, part + rows * cols, rows, static_cast<int>(cols), w_hi, w_lo, out, rows - extra, static_cast<int>(t_out + extra),
+                               static_cast<int>(t_out), 0, 1, outs, ker * c, st, stream);
+    }
+  }
+  Py_END_ALLOW_THREADS
+  if (rc != 0) return refused(what, rc);
+  return THPVariable_Wrap(y.transpose(1, 2));
+}
+
+// rvq_encode(embeddings [B, C, T], w_hi, w_lo, ((vectors, half, sq, e_max, layers), (..)), tau_rel, status): both branches' input projections
+// and their searches, then what the status word says -> codes [layers, B, T], or that word
+PyObject* rvq_encode_checked(PyObject* const* a, Py_ssize_t n) {
+  if (n != 6) {
+    PyErr_SetString(PyExc_TypeError, "rvq_encode(embeddings, w_hi, w_lo, stacks, tau_rel, status)");
+    return nullptr;
+  }
+  const at::Tensor *x = tensor(a[0]), *hi = tensor(a[1]), *lo = tensor(a[2]), *status = tensor(a[5]);
+  if (!plain(x, at::kFloat, 3) || !plain(status, at::kInt, 1) || !PyTuple_Check(a[3]) || PyTuple_GET_SIZE(a[3]) != 2 || !PyFloat_Check(a[4])) Py_RETURN_NONE;
+  const int64_t B = x->size(0), C = x->size(1), T = x->size(2), rows = B * T;
+  if (!weight_parts(hi, lo, C) || hi->size(0) != 512 || rows == 0 || rows > 0x7fffffff / 512) Py_RETURN_NONE;
+  constexpr int kMaxLayers = 64;
+  fm_rvq_stack stacks[2];
+  float e_max[2][kMaxLayers];
+  int64_t layers = 0, entries = 0;
+  for (int i = 0; i < 2; ++i) {
+    PyObject* s = PyTuple_GET_ITEM(a[3], i);
+    if (!PyTuple_Check(s) || PyTuple_GET_SIZE(s) != 5) Py_RETURN_NONE;
+    const at::Tensor *vectors = tensor(PyTuple_GET_ITEM(s, 0)), *half = tensor(PyTuple_GET_ITEM(s, 1)), *sq = tensor(PyTuple_GET_ITEM(s, 2));
+    PyObject* norms = PyTuple_GET_ITEM(s, 3);
+    const long count = int_of(PyTuple_GET_ITEM(s, 4));
+    if (!plain(vectors, at::kFloat, 3) || !plain(half, at::kHalf, 3) || !plain(sq, at::kFloat, 2) || !vectors->is_contiguous() || !half->is_contiguous() ||
+        !sq->is_contiguous() || half->sizes() != vectors->sizes() || vectors->size(2) != 256 || sq->size(0) != vectors->size(0) ||
+        sq->size(1) != vectors->size(1) || !PyList_Check(norms) || count < 1 || count > vectors->size(0) || count > kMaxLayers || PyList_GET_SIZE(norms) < count)
+      Py_RETURN_NONE;
+    if (i == 1 && vectors->size(1) != entries) Py_RETURN_NONE;
+    entries = vectors->size(1);
+    for (long l = 0; l < count; ++l) {
+      if (!PyFloat_Check(PyList_GET_ITEM(norms, l))) Py_RETURN_NONE;
+      e_max[i][l] = static_cast<float>(PyFloat_AS_DOUBLE(PyList_GET_ITEM(norms, l)));
+    }
+    stacks[i] = {nullptr, half->const_data_ptr(), vectors->const_data_ptr<float>(), sq->const_data_ptr<float>(), e_max[i], nullptr, static_cast<int>(count)};
+    layers += count;
+  }
+  const at::Tensor frames = x->transpose(1, 2).contiguous();
+  const bool direct = fm_split_direct(rows, 512, static_cast<int>(C));
+  at::Tensor parts;
+  if (!direct) parts = two_parts(rows * C, frames);
+  const at::Tensor projected = at::empty({2, rows, 256}, frames.options());
+  const at::Tensor codes = at::empty({layers, B, T}, frames.options().dtype(at::kLong));
+  const int64_t half_bytes = rows * 512, record_bytes = rows * (entries / 64) * 16;
+  const at::Tensor space = at::empty({half_bytes + record_bytes + rows * 4}, frames.options().dtype(at::kByte));
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+  const float* src = frames.const_data_ptr<float>();
+  const void *w_hi = hi->const_data_ptr(), *w_lo = lo->const_data_ptr();
+  float* both = projected.data_ptr<float>();
+  uint16_t* part = direct ? nullptr : static_cast<uint16_t*>(parts.data_ptr());
+  uint8_t* ws = static_cast<uint8_t*>(space.data_ptr());
+  int* st = status->data_ptr<int>();
+  stacks[0].residual = both;
+  stacks[1].residual = both + rows * 256;
+  stacks[0].codes = reinterpret_cast<long long*>(codes.data_ptr<int64_t>());
+  stacks[1].codes = stacks[0].codes + stacks[0].layers * rows;
+  const float tau_rel = static_cast<float>(PyFloat_AS_DOUBLE(a[4]));
+  const int width = static_cast<int>(C);
+  int rc = 0, words[2] = {0, 0};
+  const char* what = "fm_linear_rows_f32";
+  Py_BEGIN_ALLOW_THREADS
+  if (direct) {
+    rc = fm_linear_rows_f32(src, w_hi, w_lo, both, rows, 2, 512, width, st, stream);
+  } else {
+    what = "fm_split_half";
+    rc = fm_split_half(src, part, part + rows * C, rows * C, stream);
+    if (rc == 0) {
+      what = "fm_linear_split_f32";
+      rc = fm_linear_split_f32(part, part + rows * C, rows, width, w_hi, w_lo, both, rows, 1, 1, 0, 2, 512, width, st, stream);
+    }
+  }
+  if (rc == 0) {
+    what = "fm_rvq_encode_stacks_f32";
+    rc = fm_rvq_encode_stacks_f32(stacks, 2, ws, reinterpret_cast<float*>(ws + half_bytes + record_bytes), ws + half_bytes, rows, static_cast<int>(entries),
+                                  tau_rel, st, stream);
+  }
+  if (rc == 0) {
+    what = "fm_read_words";
+    rc = fm_read_words(st, nullptr, words, stream);
+  }
+  Py_END_ALLOW_THREADS
+  if (rc != 0) return refused(what, rc);
+  if (words[0] != 0) return PyLong_FromLong(words[0]);
+  return THPVariable_Wrap(codes);
+}
+
+// rvq_decode_project(codes [B, K, T], books0, books1 or None, w_hi, w_lo, status) -> (y [B, n, T], status word, whether a code was out of range)
+PyObject* rvq_decode_project_checked(PyObject* const* a, Py_ssize_t n) {
+  if (n != 6) {
+    PyErr_SetString(PyExc_TypeError, "rvq_decode_project(codes, books0, books1, w_hi, w_lo, status)");
+    return nullptr;
+  }
+  const at::Tensor *codes = tensor(a[0]), *books0 = tensor(a[1]), *books1 = a[2] == Py_None ? nullptr : tensor(a[2]);
+  const at::Tensor *hi = tensor(a[3]), *lo = tensor(a[4]), *status = tensor(a[5]);
+  const bool two = a[2] != Py_None;
+  if (!plain(codes, at::kLong, 3) || !plain(books0, at::kFloat, 3) || (two && !plain(books1, at::kFloat, 3)) || !plain(status, at::kInt, 1)) Py_RETURN_NONE;
+  const int64_t B = codes->size(0), K = codes->size(1), T = codes->size(2), n0 = two ? books0->size(0) : K, rows = B * T, width = two ? 512 : 256;
+  if (n0 < 1 || n0 > books0->size(0) || (two && (K <= n0 || K - n0 > books1->size(0))) || rows == 0 || rows > 0x7fffffff / 512 ||
+      !weight_parts(hi, lo, width) || books0->size(2) != 256 || !books0->is_contiguous() || (two && (books1->size(2) != 256 || !books1->is_contiguous())))
+    Py_RETURN_NONE;
+  const at::Tensor index = codes->contiguous();
+  const at::Tensor parts = two_parts(rows * width, *books0);
+  const int64_t n_out = hi->size(0);
+  at::Tensor y = at::empty({B, n_out, T}, books0->options());
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+  const long long* c = reinterpret_cast<const long long*>(index.const_data_ptr<int64_t>());
+  const float *first = books0->const_data_ptr<float>(), *second = two ? books1->const_data_ptr<float>() : nullptr;
+  uint16_t* part = static_cast<uint16_t*>(parts.data_ptr());
+  const void *w_hi = hi->const_data_ptr(), *w_lo = lo->const_data_ptr();
+  float* out = y.data_ptr<float>();
+  int* st = status->data_ptr<int>();
+  const int n_codes0 = static_cast<int>(books0->size(1)), n_codes1 = two ? static_cast<int>(books1->size(1)) : 0;
+  int rc = 0, words[2] = {0, 0};
+  Py_BEGIN_ALLOW_THREADS
+  rc = fm_rvq_decode_project_f32(c, first, second, part, part + rows * width, w_hi, w_lo, out, static_cast<int>(B), static_cast<int>(T), static_cast<int>(K),
+                                 static_cast<int>(n0), n_codes0, n_codes1, static_cast<int>(n_out), st, words, stream);
+  Py_END_ALLOW_THREADS
+  if (rc == -8) Py_RETURN_NONE;
+  if (rc != 0) return refused("fm_rvq_decode_project_f32", rc);
+  return Py_BuildValue("(Nii)", THPVariable_Wrap(std::move(y)), words[0], words[1]);
+}
+
+// upsample(x [B, C, T], weight [C, 1, 4]) -> [B, C, 2 T]
+PyObject* upsample_checked(PyObject* const* a, Py_ssize_t n) {
+  if (n != 2) {
+    PyErr_SetString(PyExc_TypeError, "upsample(x, weight)");
+    return nullptr;
+  }
+  const at::Tensor *x = tensor(a[0]), *w = tensor(a[1]);
+  if (!plain(x, at::kFloat, 3) || !plain(w, at::kFloat, 3) || !x->is_contiguous() || !w->is_contiguous()) Py_RETURN_NONE;
+  const int64_t B = x->size(0), C = x->size(1), T = x->size(2);
+  if (w->numel() != 4 * C || C % 32 != 0 || B > 65535 || B * C * T == 0 || T > 0x3fffffff) Py_RETURN_NONE;
+  const at::Tensor y = at::empty({B, 2 * T, C}, x->options());
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+  const float *src = x->const_data_ptr<float>(), *taps = w->const_data_ptr<float>();
+  float* out = y.data_ptr<float>();
+  int rc = 0;
+  Py_BEGIN_ALLOW_THREADS
+  rc = fm_upsample2_channels_f32(src, taps, out, static_cast<int>(B), static_cast<int>(T), static_cast<int>(C), stream);
+  Py_END_ALLOW_THREADS
+  if (rc != 0) return refused("fm_upsample2_channels_f32", rc);
+  return THPVariable_Wrap(y.transpose(1, 2));
+}
+
+// No C++ exception leaves the module (as in layer_forward); what threw did so before the first launch.
+template <PyObject* (*kFn)(PyObject* const*, Py_ssize_t)>
+PyObject* guarded(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  try {
+    return kFn(a, n);
+  } catch (const std::exception&) {
+    Py_RETURN_NONE;
+  }
+}
+
 constexpr const char* kStampsName = "_fm_bind.stamps";
 
 void stamps_free(PyObject* capsule) {
@@ -297,6 +515,14 @@ PyMethodDef methods[] = {
     {"still", fast_call<still>(), METH_FASTCALL, "still(stamps, *tensors) -> whether these are the stamped tensors, unchanged"},
     {"layer_forward", fast_call<layer_forward>(), METH_FASTCALL,
      "layer_forward(plan, x, cos, sin, ring_k, ring_v, layer, past) -> tensor, an int (native status), or None (not the ordinary case)"},
+    {"conv_frames", fast_call<guarded<conv_frames_checked>>(), METH_FASTCALL,
+     "conv_frames(x, w_hi, w_lo, kernel, stride, status) -> tensor, (name, native status), or None (not the ordinary case)"},
+    {"rvq_encode", fast_call<guarded<rvq_encode_checked>>(), METH_FASTCALL,
+     "rvq_encode(embeddings, w_hi, w_lo, stacks, tau_rel, status) -> codes, a status word, (name, native status), or None (not the ordinary case)"},
+    {"rvq_decode_project", fast_call<guarded<rvq_decode_project_checked>>(), METH_FASTCALL,
+     "rvq_decode_project(codes, books0, books1, w_hi, w_lo, status) -> (tensor, status word, bad code), (name, native status), or None (not the ordinary case)"},
+    {"upsample", fast_call<guarded<upsample_checked>>(), METH_FASTCALL,
+     "upsample(x, weight) -> tensor, (name, native status), or None (not the ordinary case)"},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fm_bind", "host side of the native calls", -1, methods};

@@ -1,6 +1,6 @@
 // extern "C" entry points of libfast_mimi_b200.so (declared in include/fast_mimi_b200.h) and the
 // small host helpers they share.  No torch types, no allocation, no synchronisation except
-// fm_read_status and fm_read_words.
+// fm_read_status, fm_read_words and fm_rvq_decode_project_f32.
 #include "../../include/fast_mimi_b200.h"
 
 #include <mutex>
@@ -424,6 +424,32 @@ int fm_read_status(const int* status, void* stream) {
   int words[2];
   const int rc = fm_read_words(status, nullptr, words, stream);
   return rc != 0 ? rc : words[0];
+}
+
+int fm_rvq_decode_project_f32(const long long* codes, const float* books0, const float* books1, void* hi, void* lo, const void* w_hi,
+                              const void* w_lo, float* y, int B, int T, int n_layers, int n0, int n_codes0, int n_codes1, int n_out,
+                              int* status, int* words, void* stream) {
+  if (B <= 0 || T <= 0 || n0 <= 0 || n0 > n_layers || words == nullptr) return -1;
+  words[0] = words[1] = 0;
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // A code out of range is written where the host reads it: no word to clear in front and none to copy behind.
+  fm::HostWords bad;
+  void* bad_code = nullptr;
+  if (!bad.locked()) return -8;
+  bad.data()[1] = 0;
+  if (cudaHostGetDevicePointer(&bad_code, bad.data() + 1, 0) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return -8;
+  }
+  const long long rows = static_cast<long long>(B) * T;
+  const int parts = n0 < n_layers ? 2 : 1, k_in = 256 * parts;
+  int rc = fm::launch_rvq_decode_split(codes, books0, parts == 2 ? books1 : nullptr, hi, lo, B, T, n_layers, n0, n_codes0, n_codes1,
+                                       static_cast<int*>(bad_code), st);
+  if (rc != 0) return rc;
+  rc = fm::launch_linear_split(hi, lo, rows, k_in, w_hi, w_lo, y, rows, T, T, 1, 1, parts, n_out, k_in, status, st);
+  const int read = static_cast<int>(fm::read_words(status, nullptr, words, st));         // waits, whatever was launched
+  words[1] = *static_cast<volatile int*>(bad.data() + 1);
+  return rc != 0 ? rc : read;
 }
 
 int fm_read_words(const int* a, const int* b, int* words, void* stream) {

@@ -21,6 +21,7 @@ class HostWords {
   HostWords(const HostWords&) = delete;
   HostWords& operator=(const HostWords&) = delete;
   int* data() { return pair_ < kPairs ? pool().words[pair_] : own_; }
+  bool locked() const { return pair_ < kPairs && pool().locked.load(std::memory_order_acquire); }      // kernels may write them
 
  private:
   static constexpr int kPairs = 64;

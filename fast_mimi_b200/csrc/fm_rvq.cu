@@ -395,7 +395,7 @@ rvq_decode_split_kernel(const long long* __restrict__ codes, const float* __rest
           a.x += e[i].x; a.y += e[i].y; a.z += e[i].z; a.w += e[i].w;
         }
       }
-      if (bad && bad_code != nullptr) atomicExch(bad_code, 1);
+      if (bad && bad_code != nullptr) *static_cast<volatile int*>(bad_code) = 1;      // perhaps in host memory: no atomic
     };
     if constexpr (kLast == 8) {
       for (int l = 0; l < n_layers; l += 8) add(std::integral_constant<int, 8>(), l);

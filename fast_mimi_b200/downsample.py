@@ -17,7 +17,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from . import ops
+from . import _native, ops
 from ._origin import Origin
 
 
@@ -54,6 +54,9 @@ class MimiDownsampleB200(nn.Module):
             raise RuntimeError("streaming (padding-cache) calls of the downsampling convolution are not built")
         if not hidden_states.is_cuda:
             raise RuntimeError("MimiDownsampleB200 runs on a CUDA device only; there is no CPU path")
+        y = _native.bind().conv_frames(hidden_states, *self._weight_parts(), self.kernel, self.stride, ops.default_status(hidden_states.device))
+        if y is not None:
+            return ops._made(y)
         y = self.frames(hidden_states.transpose(1, 2))
         return y.transpose(1, 2).to(hidden_states.dtype)
 
@@ -82,6 +85,9 @@ class MimiUpsampleB200(nn.Module):
     def forward(self, hidden_states: torch.Tensor) -> torch.Tensor:
         if not hidden_states.is_cuda:
             raise RuntimeError("MimiUpsampleB200 runs on a CUDA device only; there is no CPU path")
+        y = _native.bind().upsample(hidden_states, self.conv.weight)
+        if y is not None:
+            return ops._made(y)
         x = hidden_states
         if (x.dtype == torch.float32 and x.dim() == 3 and x.is_contiguous() and x.shape[1] == self.conv.in_channels
                 and x.shape[1] % 32 == 0 and x.shape[0] <= 65535):

@@ -114,9 +114,20 @@ def _check_codes(bad: torch.Tensor, device, status: torch.Tensor | None) -> None
     words = (ctypes.c_int * 2)()
     _native.check(_native.load().fm_read_words((default_status(device) if status is None else status).data_ptr(), bad.data_ptr(), words,
                                                _stream()), "fm_read_words")
-    if words[1] != 0:
+    _raise_words(*words)
+
+
+def _raise_words(status: int, bad: int) -> None:
+    if bad != 0:
         raise RuntimeError("rvq_decode: a code index is outside the codebook")
-    _raise_status(words[0])
+    _raise_status(status)
+
+
+def _made(result):
+    """What a call of the binding made, or the error of the native call that refused."""
+    if type(result) is tuple:
+        _native.check(result[1], result[0])
+    return result
 
 
 def _raise_status(code: int) -> None:
@@ -620,6 +631,10 @@ class RVQCodebooks:
         self.e_max = [float(v) for v in self.sq.max(dim=1).values.sqrt().cpu()]
         self.layers, self.entries = codebooks.shape[0], codebooks.shape[1]
 
+    def _native(self, layers: int) -> tuple:
+        """What the binding takes of a stack whose first ``layers`` codebooks are searched."""
+        return self.vectors, self.half, self.sq, self.e_max, layers
+
 
 def _rvq_workspace(rows, entries, device):
     """FP16 copy of the residuals, margins and candidate records of a search: the memory and where they lie in it."""
@@ -811,6 +826,14 @@ def rvq_decode_project(codes, first: RVQCodebooks, second: RVQCodebooks | None, 
     """The ordered sums of one or two quantiser stacks and their output projections: ``codes [B, K, T]`` int64 (the first
     stack's layers first) -> ``[B, N, T]`` float32.  ``w_parts``: ``split_half`` of ``[N, 256]``, or of the stacks'
     projections side by side, ``[N, 512]``."""
+    if codes.is_cuda:
+        made = _native.bind().rvq_decode_project(codes, first.vectors, None if second is None else second.vectors, *w_parts,
+                                                 default_status(codes.device) if status is None else status)
+        if made is not None:
+            if len(made) == 2:
+                _made(made)
+            _raise_words(*made[1:])
+            return made[0]
     lib = _native.load()
     _need(codes.is_cuda and codes.dtype == torch.int64 and codes.dim() == 3, "codes must be CUDA int64 [batch, layers, frames]")
     B, K, T = codes.shape

@@ -14,7 +14,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from . import ops
+from . import _native, ops
 
 
 class _Frames:
@@ -139,18 +139,27 @@ class MimiSplitRVQB200:
         B, _, T = embeddings.shape
         n_sem = self.semantic._layers(None)
         acoustic = count - self.num_semantic_quantizers
-        codes = torch.empty(n_sem + acoustic, B * T, dtype=torch.int64, device=embeddings.device)
-        frames = _Frames(embeddings)
         x = [None, None]
+        parts = None
         if acoustic > 0:
             self.acoustic._layers(acoustic)
             parts = self._joint_in_parts()
             if parts is not None:
-                x = ops._linear_rows(frames.rows, frames.parts, parts, (B * T,), None, mats=2)
-                if self.semantic.books.entries == self.acoustic.books.entries:
-                    ops._rvq_search_stacks(x, (self.semantic.books, self.acoustic.books), (codes[:n_sem], codes[n_sem:]), ops._status_ptr(None, x))
-                    ops.check_status(embeddings.device)
-                    return codes.view(len(codes), B, T)
+                sem, aco = self.semantic.books, self.acoustic.books
+                made = _native.bind().rvq_encode(embeddings, *parts, (sem._native(n_sem), aco._native(acoustic)), ops.RVQ_TAU_REL[torch.float32],
+                                                 ops.default_status(embeddings.device))
+                if type(made) is int:
+                    ops._raise_status(made)
+                if made is not None:
+                    return ops._made(made)
+        codes = torch.empty(n_sem + acoustic, B * T, dtype=torch.int64, device=embeddings.device)
+        frames = _Frames(embeddings)
+        if parts is not None:
+            x = ops._linear_rows(frames.rows, frames.parts, parts, (B * T,), None, mats=2)
+            if self.semantic.books.entries == self.acoustic.books.entries:
+                ops._rvq_search_stacks(x, (self.semantic.books, self.acoustic.books), (codes[:n_sem], codes[n_sem:]), ops._status_ptr(None, x))
+                ops.check_status(embeddings.device)
+                return codes.view(len(codes), B, T)
         self.semantic._encode_frames(frames, codes[:n_sem], x[0])
         if acoustic > 0:
             self.acoustic._encode_frames(frames, codes[n_sem:], x[1])

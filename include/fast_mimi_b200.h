@@ -371,6 +371,14 @@ int fm_linear_fp32_verify(const float* x, const float* w, float* y, int M, int N
 int fm_rope_fp32_verify(float* t, const float* cos, const float* sin, int B, int T, int H, int D,
                         long long cos_bstride, void* stream);
 
+/* fm_rvq_decode_split and the output projection behind it (fm_linear_split_f32 by channel, or fm_linear_split_sum_f32 with two stacks:
+ * n0 < n_layers), y [B, n_out, T]; then waits for `stream` and reads what the call has to report, like fm_read_words: words[0] the
+ * status word, words[1] 1 if an index was out of range (it was read as 0).  hi, lo: workspaces [B * T, 256 or 512] FP16.  -8: no
+ * page-locked word to be had, nothing launched. */
+int fm_rvq_decode_project_f32(const long long* codes, const float* books0, const float* books1, void* hi, void* lo, const void* w_hi,
+                              const void* w_lo, float* y, int B, int T, int n_layers, int n0, int n_codes0, int n_codes1, int n_out,
+                              int* status, int* words, void* stream);
+
 /* Synchronise `stream` and return the device status word (0 = all bounded waits completed; else its code, >= 101, or a
  * cudaError_t). */
 int fm_read_status(const int* status, void* stream);

@@ -338,3 +338,50 @@ def test_decoding_one_code_takes_less_than_eight():
         return min(a.elapsed_time(b) for a, b in zip(events, events[1:]))
 
     assert time(1) < 0.55 * time(8)
+
+
+@pytest.mark.parametrize("B,T", [(1, 1), (3, 21), (2, 1100)])
+@pytest.mark.parametrize("quantizers", [2, 8])
+def test_calls_of_the_binding_are_the_checked_ones(B, T, quantizers):
+    """Convolution, search, decode and upsampling through the binding give the bits of the checked calls behind them (which a type or
+    device out of the ordinary still takes), for embeddings and codes of any layout; what must raise does, and leaves the next
+    call alone."""
+    import types
+    import fast_mimi_b200 as fm
+    from fast_mimi_b200 import _native, ops
+    g = torch.Generator(device="cuda").manual_seed(T)
+    normal = lambda *shape: torch.randn(*shape, device="cuda", generator=g)
+    branch = lambda n: fm.MimiRVQB200(normal(n, 2048, 256) * 0.7, normal(256, 512, 1) / 512 ** 0.5, normal(512, 256, 1) / 16)
+    split = fm.MimiSplitRVQB200(branch(1), branch(7))
+    conv = torch.nn.Conv1d(512, 512, 4, 2, bias=False, device="cuda")
+    down = fm.MimiDownsampleB200(types.SimpleNamespace(conv=conv, causal=True, pad_mode="replicate"))
+    up = fm.MimiUpsampleB200(types.SimpleNamespace(conv=torch.nn.ConvTranspose1d(512, 512, 4, 2, groups=512, bias=False, device="cuda"), padding_left=0, padding_right=2))
+    frames = normal(B, T, 512)
+    want = down.frames(frames).transpose(1, 2)
+    for x in (frames.transpose(1, 2), frames.transpose(1, 2).contiguous()):
+        assert torch.equal(down(x), want)
+        assert torch.equal(split.encode(x, quantizers), split.encode(x.contiguous(), quantizers))
+    half = frames.half().transpose(1, 2)
+    codes = split.encode(half, quantizers)                                     # not float32: the checked calls
+    assert _native.bind().rvq_encode(half, *split._joint_in_parts(), (), 1.0, ops.default_status(half.device)) is None
+    assert torch.equal(split.encode(half.float(), quantizers), codes)
+    codes = codes.permute(1, 0, 2)                                             # [B, K, T], not contiguous
+    y = split.decode(codes)
+    assert torch.equal(y, split.decode(codes.contiguous()))
+    sums = [ops.rvq_decode(codes[:, k].transpose(0, 1).reshape(-1, B * T).contiguous(), b.books).view(B, T, 256) for k, b in
+            ((slice(0, 1), split.semantic), (slice(1, None), split.acoustic))]
+    exact = sum(s.double() @ b.output_proj.double().T for s, b in zip(sums, (split.semantic, split.acoustic))).transpose(1, 2)
+    assert O.rel_l2(y.double(), exact) < 1e-6
+    assert torch.equal(up(y), ops.upsample2_channels(y, up._taps()).transpose(1, 2))
+    assert torch.equal(up(y.double()), up.frames(y.double().transpose(1, 2)).transpose(1, 2).double())
+    for wrong in (-1, 2048):
+        bad = codes.clone()
+        bad[-1, -1, -1] = wrong
+        with pytest.raises(RuntimeError, match="outside the codebook"):
+            split.decode(bad)
+    bad = frames.clone()
+    bad[0, 0, 0] = float("nan")
+    with pytest.raises(RuntimeError, match="105"):
+        split.encode(bad.transpose(1, 2), quantizers)
+    ops.default_status(frames.device).zero_()
+    assert torch.equal(split.decode(codes), y)
