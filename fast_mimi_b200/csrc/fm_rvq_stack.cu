@@ -23,31 +23,31 @@
 namespace fm {
 
 namespace rvqs {
-constexpr int kCtas = 16, kRows = 32, kEntries = 128;          // of a cluster; of a block's share of a codebook
+constexpr int kCtas = 16, kEntries = 128;                      // of a cluster; of a block's share of a codebook
 constexpr int kCodes = kCtas * kEntries;
 constexpr int kDim = 256, kWarps = 16, kThreads = kWarps * 32;
 constexpr int kBookBytes = kEntries * kDim * 2, kChunkBytes = kEntries * 128;
 constexpr int kMaxLayers = 32;
+constexpr unsigned long long kNoCandidate = 0xfffffffdull << 32;      // below every distance that is not finite, above those that are
+constexpr int kMaxRows = 32;                                   // vectors of a cluster: 32 or 16
 struct Shared {
   uint64_t full[2];
+  uint64_t arrived[2];                             // all blocks' best candidates, of even and of odd layers
   CtaCtl ctl;
   uint32_t pad[3];
-  unsigned long long best[kRows][kCtas];     // (distance, index) of every block's best candidate
-  float min_of[kRows][kCtas];                // every block's smallest approximate distance
-  float min_in[8][kRows];                    // of 16 entries of this block
-  float limit[kRows];
-  float margin[kRows];
-  unsigned long long best_in[kRows];         // of this block's candidates
+  unsigned long long best[2][kMaxRows][kCtas];     // (distance, index) of every block's best candidate
+  float min_in[8][kMaxRows];                       // of 16 entries of this block
+  float margin[kMaxRows];
+  unsigned long long best_in[2][kMaxRows];         // of this block's candidates
   int n_listed;
-  uint16_t listed[kRows * kEntries];         // candidates: vector * 128 + entry
+  uint16_t listed[kMaxRows * kEntries];            // candidates: vector * 128 + entry
 };
-constexpr int kSmemBytes = 1024 + 2 * kBookBytes + kRows * kDim * (2 + 4) + static_cast<int>(sizeof(Shared));
+constexpr int smem_bytes(int rows) { return 1024 + 2 * kBookBytes + rows * kDim * (2 + 4) + static_cast<int>(sizeof(Shared)); }
 
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
-__device__ __forceinline__ void st_cluster_u64(uint32_t addr, unsigned long long v) {
-  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
+__device__ __forceinline__ void st_async_u64(uint32_t addr, unsigned long long v, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr), "l"(v), "r"(bar) : "memory");
 }
 }  // namespace rvqs
 
@@ -65,15 +65,18 @@ struct RvqStackArgs {
   float tau_rel;
 };
 
+template <int kRows>
 __global__ void __launch_bounds__(rvqs::kThreads, 1)
 rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_constant__ CUtensorMap tmap_books1,
                  const __grid_constant__ RvqStackArgs args, int* status) {
   using namespace rvqs;
+  constexpr int kMine = kRows / kWarps;                        // vectors of a warp
+  constexpr int kCols = kRows / 16;                            // columns of eight vectors of a warp's products
   const RvqStackArgs::Stack& a = args.stack[blockIdx.y];
   const CUtensorMap* tmap_books = blockIdx.y == 0 ? &tmap_books0 : &tmap_books1;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem_book = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* smem_x = smem_book + 2 * kBookBytes;                // FP16 residuals: four chunks of 64 dimensions, 32 rows each
+  uint8_t* smem_x = smem_book + 2 * kBookBytes;                // FP16 residuals: four chunks of 64 dimensions
   float* exact_x = reinterpret_cast<float*>(smem_x + kRows * kDim * 2);      // the residuals in FP32, for whichever warp needs them
   Shared* sh = reinterpret_cast<Shared*>(exact_x + kRows * kDim);
   CtaCtl* ctl = &sh->ctl;
@@ -92,16 +95,20 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
   if (tid == 0) {
     mbar_init(&sh->full[0], 1);
     mbar_init(&sh->full[1], 1);
+    mbar_init(&sh->arrived[0], 1);
+    mbar_init(&sh->arrived[1], 1);
     ctl->abort = 0;
     fence_mbar_init();
+    mbar_arrive_expect_tx(&sh->arrived[0], kRows * kCtas * 8);
+    mbar_arrive_expect_tx(&sh->arrived[1], kRows * kCtas * 8);
     load_book(0);
     if (a.layers > 1) load_book(1);
   }
 
-  // This warp's two vectors, eight values a lane, in every block of the cluster.
-  float x[2][8];
+  // This warp's vectors, eight values a lane, in every block of the cluster.
+  float x[kMine][8];
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
+  for (int i = 0; i < kMine; ++i) {
     const int f = warp + kWarps * i;
 #pragma unroll
     for (int k = 0; k < 8; ++k) x[i][k] = 0.f;
@@ -114,7 +121,7 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
   // FP16 copy, margin (the same sums in the same order as in fm_rvq.cu) and an empty set of candidates for the layer to come
   auto open_layer = [&](int l) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < kMine; ++i) {
       const int f = warp + kWarps * i;
       float xx = 0.f;
 #pragma unroll
@@ -129,41 +136,48 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
       exact[1] = make_float4(x[i][4], x[i][5], x[i][6], x[i][7]);
       if (lane == 0) {
         sh->margin[f] = rvq_margin(xx, a.e_max[l], args.tau_rel);
-        sh->best_in[f] = ~0ull;
+        sh->best_in[l & 1][f] = ~0ull;
       }
     }
     if (tid == 0) sh->n_listed = 0;
   };
   open_layer(0);
   __syncthreads();
-  cluster_arrive();                                            // this block runs: its shared memory may be written
+  cluster_arrive_relaxed();                                    // this block runs: its shared memory may be written
 
   const int g = lane >> 2, cpair = (lane & 3) * 2;
-  const int mt = warp >> 1, nh = warp & 1;                     // 16 entries x 16 vectors of the products
+  const int mt = warp >> 1, nh = warp & 1;                     // 16 entries x half of the vectors of the products
+  const int f0 = nh * (kRows / 2) + cpair;
   for (int l = 0; l < a.layers; ++l) {
     const float* sq = a.e_sq + static_cast<size_t>(l) * kCodes + rank * kEntries + mt * 16 + g;
     const float e_sq[2] = {__ldg(sq), __ldg(sq + 8)};
     mbar_wait(&sh->full[l & 1], static_cast<uint32_t>(l >> 1) & 1u, ctl, status, kErrWaitTma);
-    float d[2][4];
+    float d[kCols][4];
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) d[nt][0] = d[nt][1] = d[nt][2] = d[nt][3] = 0.f;
+    for (int nt = 0; nt < kCols; ++nt) d[nt][0] = d[nt][1] = d[nt][2] = d[nt][3] = 0.f;
     {
       const uint32_t book = smem_u32(smem_book + (l & 1) * kBookBytes), vec = smem_u32(smem_x);
 #pragma unroll
       for (int kc = 0; kc < kDim / 64; ++kc) {
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-          uint32_t ea[4], xb[4];
-          ldmatrix4(ea, book + kc * kChunkBytes + sw128_offset(mt * 16 + (lane & 15), 2 * ks + (lane >> 4)));
-          ldmatrix4(xb, vec + kc * (kRows * 128) + sw128_offset(nh * 16 + (lane & 7) + ((lane >> 4) << 3), 2 * ks + ((lane >> 3) & 1)));
-          mma_16x8x16<__half>(d[0], ea, xb[0], xb[1]);
-          mma_16x8x16<__half>(d[1], ea, xb[2], xb[3]);
+        for (int ks = 0; ks < 4; ks += 2) {
+          uint32_t ea[2][4], xb[kCols][4];
+#pragma unroll
+          for (int s = 0; s < 2; ++s) ldmatrix4(ea[s], book + kc * kChunkBytes + sw128_offset(mt * 16 + (lane & 15), 2 * (ks + s) + (lane >> 4)));
+#pragma unroll
+          for (int nt = 0; nt < kCols; ++nt)
+            ldmatrix4(xb[nt], vec + kc * (kRows * 128) + sw128_offset(nh * (kRows / 2) + nt * 8 + (lane & 7), 2 * ks + (lane >> 3)));
+#pragma unroll
+          for (int s = 0; s < 2; ++s) {
+#pragma unroll
+            for (int nt = 0; nt < kCols; ++nt) mma_16x8x16<__half>(d[nt], ea[s], xb[nt][2 * s], xb[nt][2 * s + 1]);
+          }
         }
       }
     }
     // approximate distances: entries g and g + 8 of the tile, vectors cpair and cpair + 1 of each eight
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
+    for (int nt = 0; nt < kCols; ++nt) {
       float m[2];
 #pragma unroll
       for (int e = 0; e < 4; ++e) d[nt][e] = fmaf(-2.f, d[nt][e], e_sq[e >> 1]);
@@ -174,73 +188,84 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
         m[0] = fminf(m[0], __shfl_xor_sync(0xffffffffu, m[0], o));
         m[1] = fminf(m[1], __shfl_xor_sync(0xffffffffu, m[1], o));
       }
-      if (g == 0) *reinterpret_cast<float2*>(&sh->min_in[mt][nh * 16 + nt * 8 + cpair]) = make_float2(m[0], m[1]);
+      if (g == 0) *reinterpret_cast<float2*>(&sh->min_in[mt][f0 + nt * 8]) = make_float2(m[0], m[1]);
     }
     __syncthreads();
     if (tid == 0 && l + 2 < a.layers) load_book(l + 2);        // the products are done with this layer's codebook
-    if (l == 0) cluster_wait();
-    {
-      const int f = tid & 31, peer = tid >> 5;                 // one of the block's 32 minima to one of 16 blocks
-      float m = sh->min_in[0][f];
+    // Candidates: within the margin of the least of this block's own entries, which all that are within it of the least of all are.
 #pragma unroll
-      for (int i = 1; i < 8; ++i) m = fminf(m, sh->min_in[i][f]);
-      st_cluster_f32(map_to_cta(smem_u32(&sh->min_of[f][rank]), static_cast<uint32_t>(peer)), m);
-    }
-    cluster_sync_all();
-    {
-      const int f = tid >> 4;
-      float m = sh->min_of[f][tid & 15];
+    for (int nt = 0; nt < kCols; ++nt) {
+      float2 m = *reinterpret_cast<const float2*>(&sh->min_in[0][f0 + nt * 8]);
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
-      if ((tid & 15) == 0) sh->limit[f] = m + sh->margin[f];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
+      for (int i = 1; i < 8; ++i) {
+        const float2 o = *reinterpret_cast<const float2*>(&sh->min_in[i][f0 + nt * 8]);
+        m.x = fminf(m.x, o.x);
+        m.y = fminf(m.y, o.y);
+      }
+      const float2 margin = *reinterpret_cast<const float2*>(&sh->margin[f0 + nt * 8]);
+      const float limit[2] = {m.x + margin.x, m.y + margin.y};
+      if (warp == nh && g == 0) {                              // one that is not finite: no candidate in any block, whatever the others find
+        if (!(limit[0] == limit[0])) atomicMin(&sh->best_in[l & 1][f0 + nt * 8], kNoCandidate);
+        if (!(limit[1] == limit[1])) atomicMin(&sh->best_in[l & 1][f0 + nt * 8 + 1], kNoCandidate);
+      }
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int f = nh * 16 + nt * 8 + cpair + (e & 1), j = mt * 16 + g + 8 * (e >> 1);
-        if (f < n && d[nt][e] <= sh->limit[f]) sh->listed[atomicAdd(&sh->n_listed, 1)] = static_cast<uint16_t>(f * kEntries + j);
+        const int f = f0 + nt * 8 + (e & 1), j = mt * 16 + g + 8 * (e >> 1);
+        if (f < n && d[nt][e] <= limit[e & 1]) sh->listed[atomicAdd(&sh->n_listed, 1)] = static_cast<uint16_t>(f * kEntries + j);
       }
     }
     __syncthreads();
-    // ---- this block's candidates, exactly, one warp each; the smaller distance wins, on ties the lower index (argmin's rule)
-    for (int c = warp; c < sh->n_listed; c += kWarps) {
-      const int f = sh->listed[c] / kEntries, j = rank * kEntries + sh->listed[c] % kEntries;
-      const float4* er = reinterpret_cast<const float4*>(a.books + (static_cast<size_t>(l) * kCodes + j) * kDim + lane * 8);
-      const float4 u = __ldg(er), v = __ldg(er + 1);
-      const float4* xr = reinterpret_cast<const float4*>(exact_x + f * kDim + lane * 8);
-      const float4 xa = xr[0], xb = xr[1];
-      const float ev[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w}, xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-      float acc = 0.f;
+    // ---- exactly, a warp up to four at a time; the smaller distance wins, on ties the lower index (argmin's rule)
+    const int n_listed = sh->n_listed;
+    for (int c0 = warp; c0 < n_listed; c0 += 4 * kWarps) {
+      float4 u[4], v[4];
+      int at[4];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const float t = xv[k] - ev[k];
-        acc = fmaf(t, t, acc);
+      for (int i = 0; i < 4; ++i) {
+        at[i] = sh->listed[c0 + i * kWarps < n_listed ? c0 + i * kWarps : c0];
+        const float4* er = reinterpret_cast<const float4*>(a.books + (static_cast<size_t>(l) * kCodes + rank * kEntries + at[i] % kEntries) * kDim + lane * 8);
+        u[i] = __ldg(er);
+        v[i] = __ldg(er + 1);
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      // a distance that is not finite loses to every other and leaves index 0, as where nothing is smaller than the best so far
-      const unsigned long long key = acc < INFINITY ? (static_cast<unsigned long long>(__float_as_uint(acc)) << 32) | static_cast<unsigned>(j)
-                                                    : 0xfffffffeull << 32;
-      if (lane == 0) atomicMin(&sh->best_in[f], key);
+      for (int i = 0; i < 4; ++i) {
+        const int f = at[i] / kEntries, j = rank * kEntries + at[i] % kEntries;
+        const float4* xr = reinterpret_cast<const float4*>(exact_x + f * kDim + lane * 8);
+        const float4 xa = xr[0], xb = xr[1];
+        const float ev[8] = {u[i].x, u[i].y, u[i].z, u[i].w, v[i].x, v[i].y, v[i].z, v[i].w}, xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+        float acc = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float t = xv[k] - ev[k];
+          acc = fmaf(t, t, acc);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        // a distance that is not finite loses to every other and leaves index 0, as where nothing is smaller than the best so far
+        const unsigned long long key = acc < INFINITY ? (static_cast<unsigned long long>(__float_as_uint(acc)) << 32) | static_cast<unsigned>(j)
+                                                      : 0xfffffffeull << 32;
+        if (lane == 0 && c0 + i * kWarps < n_listed) atomicMin(&sh->best_in[l & 1][f], key);
+      }
     }
     __syncthreads();
-    {
-      const int f = tid & 31, peer = tid >> 5;
-      st_cluster_u64(map_to_cta(smem_u32(&sh->best[f][rank]), static_cast<uint32_t>(peer)), sh->best_in[f]);
+    if (l == 0) cluster_wait();
+    if (tid < kRows * kCtas) {                                 // one of the block's best to one of 16 blocks, counted where it arrives
+      const int f = tid % kRows;
+      const uint32_t peer = static_cast<uint32_t>(tid / kRows);
+      st_async_u64(map_to_cta(smem_u32(&sh->best[l & 1][f][rank]), peer), sh->best_in[l & 1][f], map_to_cta(smem_u32(&sh->arrived[l & 1]), peer));
     }
-    cluster_sync_all();
+    mbar_wait_cluster(&sh->arrived[l & 1], static_cast<uint32_t>(l >> 1) & 1u, ctl, status, kErrWaitConsumer);
+    __syncwarp();
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < kMine; ++i) {
       const int f = warp + kWarps * i;
-      unsigned long long best = sh->best[f][lane & 15];
+      unsigned long long best = sh->best[l & 1][f][lane & 15];
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) {
         const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
         best = other < best ? other : best;
       }
-      const bool none = best == ~0ull;                         // a residual that is not finite: no candidate
+      const bool none = best == ~0ull || best == kNoCandidate; // a residual that is not finite
       const int j = none ? 0 : static_cast<int>(best & 0xffffffffu);
       if (rank == 0 && lane == 0 && f < n && !skip) {
         a.codes[static_cast<size_t>(l) * args.rows + r0 + f] = j;
@@ -254,6 +279,7 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
       }
     }
     if (l + 1 < a.layers) {
+      if (tid == 0) mbar_arrive_expect_tx(&sh->arrived[l & 1], kRows * kCtas * 8);       // for the layer after that
       open_layer(l + 1);
       __syncthreads();
     }
@@ -269,12 +295,15 @@ int stack_slots() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   const int n = slots.get(dev, [] {
-    if (ensure_dynamic_smem(reinterpret_cast<const void*>(rvq_stack_kernel), rvqs::kSmemBytes) != 0 ||
-        cudaFuncSetAttribute(rvq_stack_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    const auto allow = [](auto kern, int bytes) {
+      return ensure_dynamic_smem(reinterpret_cast<const void*>(kern), bytes) == 0 &&
+             cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    };
+    if (!allow(rvq_stack_kernel<16>, rvqs::smem_bytes(16)) || !allow(rvq_stack_kernel<32>, rvqs::smem_bytes(32))) {
       (void)cudaGetLastError();
       return -1;
     }
-    return resident_clusters(rvq_stack_kernel, rvqs::kThreads, rvqs::kSmemBytes, rvqs::kCtas);
+    return resident_clusters(rvq_stack_kernel<32>, rvqs::kThreads, rvqs::smem_bytes(32), rvqs::kCtas);
   });
   return n > 0 ? n : 0;
 }
@@ -286,7 +315,7 @@ int stack_slots() {
 bool rvq_stack_takes(const RvqStack* stacks, int n_stacks, long long rows, int n_codes) {
   for (int i = 0; i < n_stacks; ++i)
     if (stacks[i].layers > rvqs::kMaxLayers) return false;
-  return n_codes == rvqs::kCodes && rows <= static_cast<long long>(rvqs::kRows) * stack_slots();
+  return n_codes == rvqs::kCodes && rows <= static_cast<long long>(rvqs::kMaxRows) * stack_slots();
 }
 
 int launch_rvq_stack(const RvqStack* stacks, int n_stacks, long long rows, float tau_rel, int* status, cudaStream_t st) {
@@ -294,8 +323,9 @@ int launch_rvq_stack(const RvqStack* stacks, int n_stacks, long long rows, float
   if (n_stacks < 1 || n_stacks > 2 || !(tau_rel >= 0.f)) return -1;
   RvqStackArgs a = {};
   CUtensorMap maps[2];
+  const int longer = n_stacks == 2 && stacks[1].layers > stacks[0].layers ? 1 : 0;     // comes first
   for (int i = 0; i < n_stacks; ++i) {
-    const RvqStack& s = stacks[i];
+    const RvqStack& s = stacks[i == 0 ? longer : 1 - longer];
     if (s.residual == nullptr || s.books16 == nullptr || s.books == nullptr || s.e_sq == nullptr || s.codes == nullptr) return -1;
     if ((reinterpret_cast<uintptr_t>(s.residual) | reinterpret_cast<uintptr_t>(s.books) | reinterpret_cast<uintptr_t>(s.books16)) & 15u) return -3;
     RvqStackArgs::Stack& d = a.stack[i];
@@ -314,9 +344,14 @@ int launch_rvq_stack(const RvqStack* stacks, int n_stacks, long long rows, float
   if (n_stacks == 1) maps[1] = maps[0];
   a.rows = static_cast<int>(rows);
   a.tau_rel = tau_rel;
-  const unsigned clusters = static_cast<unsigned>((rows + kRows - 1) / kRows);
-  return launch_kernel(rvq_stack_kernel, dim3(clusters * kCtas, static_cast<unsigned>(n_stacks)), kThreads, kSmemBytes, st, kCtas, 0, maps[0], maps[1],
-                       a, status);
+  // 16 vectors a cluster while the device holds all clusters of the longer stack at once and the other one's, if some of those have to
+  // wait, end no later.
+  const int few = static_cast<int>((rows + 15) / 16), slots = stack_slots();
+  const bool sixteen = few <= slots && (n_stacks == 1 || 2 * few <= slots || 2 * a.stack[1].layers <= a.stack[0].layers);
+  const int per = sixteen ? 16 : 32;
+  auto kern = sixteen ? rvq_stack_kernel<16> : rvq_stack_kernel<32>;
+  return launch_kernel(kern, dim3(static_cast<unsigned>((rows + per - 1) / per) * kCtas, static_cast<unsigned>(n_stacks)), kThreads, smem_bytes(per), st, kCtas,
+                       0, maps[0], maps[1], a, status);
 }
 
 }  // namespace fm
