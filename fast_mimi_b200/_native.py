@@ -46,12 +46,14 @@ SIGNATURES: dict[str, list] = {
     "fm_split_direct": [_LL, _I, _I],
     "fm_linear_rows_f32": [_P, _P, _P, _P, _LL, _I, _I, _I, _P, _P],
     "fm_conv_frames_f32": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
+    "fm_conv_parts_f32": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "fm_upsample2_channels_f32": [_P, _P, _P, _I, _I, _I, _P],
     "fm_rvq_decode_split": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "fm_upsample2_f32": [_P, _P, _P, _I, _I, _I, _P],
     "fm_split_half": [_P, _P, _P, _LL, _P],
     "fm_rvq_encode_f32": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _LL, _I, _I, _F, _P, _P],
     "fm_rvq_encode_stacks_f32": [ctypes.POINTER(RvqStack), _I, _P, _P, _P, _LL, _I, _F, _P, _P],
+    "fm_rvq_encode_frames_f32": [_P, _I, _P, _P, ctypes.POINTER(RvqStack), _I, _LL, _I, _F, _P, _P],
     "fm_rvq_encode_tiles_f32": [ctypes.POINTER(RvqStack), _I, _LL, _I, _F, _P, _P],
     "fm_rvq_prepare_f32": [_P, _P, _P, _LL, _F, _F, _P],
     "fm_rvq_candidates_f16": [_P, _P, _P, _P, _P, _LL, _I, _P, _P],
@@ -132,5 +134,6 @@ def check(rc: int, what: str) -> None:
                 -5: "more frames than the built-in workspace holds",
                 -7: "workspace too small",
                 -8: "no page-locked word",
+                -9: "not a call for this form",
                 -6: "clip length outside the fused kernel's range (128 < T <= 256)"}.get(rc, "CUDA error" if rc > 0 else "error")
         raise RuntimeError(f"{what} failed with status {rc} ({kind})")

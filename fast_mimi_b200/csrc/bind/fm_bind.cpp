@@ -290,13 +290,8 @@ PyObject* conv_frames_checked(PyObject* const* a, Py_ssize_t n) {
   if (direct) {
     rc = fm_conv_frames_f32(src, w_hi, w_lo, out, b, t, c, ker, str, outs, st, stream);
   } else {
-    what = "fm_conv_frames_split";
-    rc = fm_conv_frames_split(src, part, part + rows * cols, b, t, c, ker, str, stream);
-    if (rc == 0) {
-      what = "fm_linear_split_f32";
-      rc = fm_linear_split_f32(part, part + rows * cols, rows, static_cast<int>(cols), w_hi, w_lo, out, rows - extra, static_cast<int>(t_out + extra),
-                               static_cast<int>(t_out), 0, 1, outs, ker * c, st, stream);
-    }
+    what = "fm_conv_parts_f32";
+    rc = fm_conv_parts_f32(src, part, part + rows * cols, w_hi, w_lo, out, b, t, c, ker, str, outs, st, stream);
   }
   Py_END_ALLOW_THREADS
   if (rc != 0) return refused(what, rc);
@@ -338,43 +333,54 @@ PyObject* rvq_encode_checked(PyObject* const* a, Py_ssize_t n) {
     layers += count;
   }
   const at::Tensor frames = x->transpose(1, 2).contiguous();
-  const bool direct = fm_split_direct(rows, 512, static_cast<int>(C));
-  at::Tensor parts;
-  if (!direct) parts = two_parts(rows * C, frames);
-  const at::Tensor projected = at::empty({2, rows, 256}, frames.options());
-  const at::Tensor codes = at::empty({layers, B, T}, frames.options().dtype(at::kLong));
-  const int64_t half_bytes = rows * 512, record_bytes = rows * (entries / 64) * 16;
-  const at::Tensor space = at::empty({half_bytes + record_bytes + rows * 4}, frames.options().dtype(at::kByte));
+  at::Tensor codes = at::empty({layers, B, T}, frames.options().dtype(at::kLong));
   cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
   const float* src = frames.const_data_ptr<float>();
   const void *w_hi = hi->const_data_ptr(), *w_lo = lo->const_data_ptr();
-  float* both = projected.data_ptr<float>();
-  uint16_t* part = direct ? nullptr : static_cast<uint16_t*>(parts.data_ptr());
-  uint8_t* ws = static_cast<uint8_t*>(space.data_ptr());
   int* st = status->data_ptr<int>();
-  stacks[0].residual = both;
-  stacks[1].residual = both + rows * 256;
   stacks[0].codes = reinterpret_cast<long long*>(codes.data_ptr<int64_t>());
   stacks[1].codes = stacks[0].codes + stacks[0].layers * rows;
   const float tau_rel = static_cast<float>(PyFloat_AS_DOUBLE(a[4]));
-  const int width = static_cast<int>(C);
-  int rc = 0, words[2] = {0, 0};
-  const char* what = "fm_linear_rows_f32";
-  Py_BEGIN_ALLOW_THREADS
-  if (direct) {
-    rc = fm_linear_rows_f32(src, w_hi, w_lo, both, rows, 2, 512, width, st, stream);
-  } else {
-    what = "fm_split_half";
-    rc = fm_split_half(src, part, part + rows * C, rows * C, stream);
-    if (rc == 0) {
-      what = "fm_linear_split_f32";
-      rc = fm_linear_split_f32(part, part + rows * C, rows, width, w_hi, w_lo, both, rows, 1, 1, 0, 2, 512, width, st, stream);
+  const int width = static_cast<int>(C), n_codes = static_cast<int>(entries);
+  int words[2] = {0, 0};
+  const char* what = "fm_rvq_encode_frames_f32";
+  int rc = fm_rvq_encode_frames_f32(src, width, w_hi, w_lo, stacks, 2, rows, n_codes, tau_rel, st, stream);
+  at::Tensor projected, parts, space;
+  float* both = nullptr;
+  uint16_t* part = nullptr;
+  uint8_t* ws = nullptr;
+  const bool chain = rc == -9;             // the projections, then the search
+  const int64_t half_bytes = rows * 512, record_bytes = rows * (entries / 64) * 16;
+  if (chain) {
+    projected = at::empty({2, rows, 256}, frames.options());
+    space = at::empty({half_bytes + record_bytes + rows * 4}, frames.options().dtype(at::kByte));
+    if (!fm_split_direct(rows, 512, width)) {
+      parts = two_parts(rows * C, frames);
+      part = static_cast<uint16_t*>(parts.data_ptr());
     }
+    both = projected.data_ptr<float>();
+    ws = static_cast<uint8_t*>(space.data_ptr());
+    stacks[0].residual = both;
+    stacks[1].residual = both + rows * 256;
   }
-  if (rc == 0) {
-    what = "fm_rvq_encode_stacks_f32";
-    rc = fm_rvq_encode_stacks_f32(stacks, 2, ws, reinterpret_cast<float*>(ws + half_bytes + record_bytes), ws + half_bytes, rows, static_cast<int>(entries),
-                                  tau_rel, st, stream);
+  Py_BEGIN_ALLOW_THREADS
+  if (chain) {
+    if (part == nullptr) {
+      what = "fm_linear_rows_f32";
+      rc = fm_linear_rows_f32(src, w_hi, w_lo, both, rows, 2, 512, width, st, stream);
+    } else {
+      what = "fm_split_half";
+      rc = fm_split_half(src, part, part + rows * C, rows * C, stream);
+      if (rc == 0) {
+        what = "fm_linear_split_f32";
+        rc = fm_linear_split_f32(part, part + rows * C, rows, width, w_hi, w_lo, both, rows, 1, 1, 0, 2, 512, width, st, stream);
+      }
+    }
+    if (rc == 0) {
+      what = "fm_rvq_encode_stacks_f32";
+      rc = fm_rvq_encode_stacks_f32(stacks, 2, ws, reinterpret_cast<float*>(ws + half_bytes + record_bytes), ws + half_bytes, rows, n_codes, tau_rel, st,
+                                    stream);
+    }
   }
   if (rc == 0) {
     what = "fm_read_words";
@@ -383,7 +389,7 @@ PyObject* rvq_encode_checked(PyObject* const* a, Py_ssize_t n) {
   Py_END_ALLOW_THREADS
   if (rc != 0) return refused(what, rc);
   if (words[0] != 0) return PyLong_FromLong(words[0]);
-  return THPVariable_Wrap(codes);
+  return THPVariable_Wrap(std::move(codes));
 }
 
 // rvq_decode_project(codes [B, K, T], books0, books1 or None, w_hi, w_lo, status) -> (y [B, n, T], status word, whether a code was out of range)

@@ -298,6 +298,18 @@ int fm_rvq_encode_stacks_f32(const fm_rvq_stack* stacks, int n_stacks, void* res
   return fm::launch_rvq_encode_stacks(s, n_stacks, residual16, tau, records, rows, n_codes, tau_rel, status, static_cast<cudaStream_t>(stream));
 }
 
+int fm_rvq_encode_frames_f32(const float* x, int k_in, const void* w_hi, const void* w_lo, const fm_rvq_stack* stacks, int n_stacks, long long rows,
+                             int n_codes, float tau_rel, int* status, void* stream) {
+  fm::RvqStack s[2] = {};
+  if (rvq_stacks(stacks, n_stacks, s) != 0 || rows < 0 || x == nullptr || w_hi == nullptr || w_lo == nullptr) return -1;
+  if (rows == 0) return 0;
+  for (int i = 0; i < n_stacks; ++i)
+    if (s[i].layers <= 0 || s[i].e_max == nullptr) return -1;
+  if (k_in != 512 || !fm::rvq_stack_takes(s, n_stacks, rows, n_codes)) return -9;
+  const fm::RvqFrames from = {x, w_hi, w_lo};
+  return fm::launch_rvq_stack(s, n_stacks, rows, tau_rel, status, static_cast<cudaStream_t>(stream), &from);
+}
+
 int fm_rvq_encode_tiles_f32(const fm_rvq_stack* stacks, int n_stacks, long long rows, int n_codes, float tau_rel, int* status, void* stream) {
   fm::RvqStack s[2] = {};
   if (rvq_stacks(stacks, n_stacks, s) != 0) return -1;
@@ -426,6 +438,18 @@ int fm_read_status(const int* status, void* stream) {
   return rc != 0 ? rc : words[0];
 }
 
+int fm_conv_parts_f32(const float* x, void* hi, void* lo, const void* w_hi, const void* w_lo, float* y, int B, int T, int C, int kernel, int stride,
+                      int n_out, int* status, void* stream) {
+  if (B <= 0 || T <= 0) return (B == 0 || T == 0) ? 0 : -1;
+  if (C <= 0 || stride <= 0 || kernel < stride || kernel % stride != 0) return -1;
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  int rc = fm::launch_conv_frames_split(x, hi, lo, B, T, C, kernel, stride, st);
+  if (rc != 0) return rc;
+  const int t_out = (T + stride - 1) / stride, extra = kernel / stride - 1;
+  const long long rows = static_cast<long long>(B) * (t_out + extra);
+  return fm::launch_linear_split(hi, lo, rows, stride * C, w_hi, w_lo, y, rows - extra, t_out + extra, t_out, 0, 1, 1, n_out, kernel * C, status, st, 1);
+}
+
 int fm_rvq_decode_project_f32(const long long* codes, const float* books0, const float* books1, void* hi, void* lo, const void* w_hi,
                               const void* w_lo, float* y, int B, int T, int n_layers, int n0, int n_codes0, int n_codes1, int n_out,
                               int* status, int* words, void* stream) {
@@ -446,7 +470,7 @@ int fm_rvq_decode_project_f32(const long long* codes, const float* books0, const
   int rc = fm::launch_rvq_decode_split(codes, books0, parts == 2 ? books1 : nullptr, hi, lo, B, T, n_layers, n0, n_codes0, n_codes1,
                                        static_cast<int*>(bad_code), st);
   if (rc != 0) return rc;
-  rc = fm::launch_linear_split(hi, lo, rows, k_in, w_hi, w_lo, y, rows, T, T, 1, 1, parts, n_out, k_in, status, st);
+  rc = fm::launch_linear_split(hi, lo, rows, k_in, w_hi, w_lo, y, rows, T, T, 1, 1, parts, n_out, k_in, status, st, 1);
   const int read = static_cast<int>(fm::read_words(status, nullptr, words, st));         // waits, whatever was launched
   words[1] = *static_cast<volatile int*>(bad.data() + 1);
   return rc != 0 ? rc : read;

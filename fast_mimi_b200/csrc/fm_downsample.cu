@@ -24,6 +24,7 @@ namespace fm {
 __global__ void __launch_bounds__(256)
 conv_frames_split_kernel(const float* __restrict__ x, uint16_t* __restrict__ hi, uint16_t* __restrict__ lo, int B, int T, int T_pad,
                          int left, int C) {
+  griddep_launch();                        // opens a chain; the product behind it waits for its end
   const int c8 = C / 8;
   const long long total = static_cast<long long>(B) * T_pad * c8;
   const long long step = static_cast<long long>(gridDim.x) * blockDim.x;

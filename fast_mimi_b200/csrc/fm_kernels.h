@@ -132,9 +132,9 @@ struct SplitLow {
 };
 int launch_linear_split(const void* a_hi, const void* a_lo, long long a_rows, int a_cols, const void* w_hi, const void* w_lo, float* y,
                         long long rows, int clip_rows, int clip_valid, int by_channel, int n_mats, int parts, int N, int K, int* status,
-                        cudaStream_t st);
+                        cudaStream_t st, int dependent = 0);
 int launch_linear_split_small(const void* a_hi, const void* w_hi, const SplitLow& low, const SplitRows& map, float* y, int M, int N,
-                              int K, int* status, cudaStream_t st);
+                              int K, int* status, cudaStream_t st, int dependent);
 // The same from an operand as it lies, split on the way (fm_split_gemm.cu), for many rows: FP32 rows [rows, K], or frames [B, T, C] of
 // a causal convolution.  K a multiple of 128, at least 256.
 // Whether there are rows enough for them to be the faster form.
@@ -210,7 +210,13 @@ bool rvq_tiles_take(const RvqStack* stacks, int n_stacks, long long rows, int n_
 int launch_rvq_tiles(const RvqStack* stacks, int n_stacks, long long rows, int n_codes, float tau_rel, int* status, cudaStream_t st);
 // The whole search in one kernel for few vectors (fm_rvq_stack.cu); nothing but codes is written.
 bool rvq_stack_takes(const RvqStack* stacks, int n_stacks, long long rows, int n_codes);
-int launch_rvq_stack(const RvqStack* stacks, int n_stacks, long long rows, float tau_rel, int* status, cudaStream_t st);
+// With `from` the vectors are projected on the way: x [rows, 512], w_hi and w_lo [256 n_stacks, 512]; `residual` is not looked at.
+struct RvqFrames {
+  const float* x;
+  const void *w_hi, *w_lo;
+};
+int launch_rvq_stack(const RvqStack* stacks, int n_stacks, long long rows, float tau_rel, int* status, cudaStream_t st,
+                     const RvqFrames* from = nullptr);
 int launch_rvq_prepare(const float* x, void* resid16, float* tau, long long rows, float e_max, float tau_rel,
                        cudaStream_t st);
 int launch_rvq_to_half(const float* x, void* y, long long rows, cudaStream_t st);

@@ -571,7 +571,7 @@ int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, co
 
 int launch_linear_split(const void* a_hi, const void* a_lo, long long a_rows, int a_cols, const void* w_hi, const void* w_lo, float* y,
                         long long rows, int clip_rows, int clip_valid, int by_channel, int n_mats, int parts, int N, int K, int* status,
-                        cudaStream_t st) {
+                        cudaStream_t st, int dependent) {
   using namespace lin;
   if (rows < 0 || a_rows > 0x7fffffffLL || a_rows < rows || N <= 0 || K <= 0 || N % 256 != 0 || a_cols <= 0 || a_cols % kBlockK != 0 ||
       K % a_cols != 0 || n_mats <= 0 || N % (256 * n_mats) != 0 || (by_channel && n_mats != 1) || parts < 1 || parts > 2 ||
@@ -586,12 +586,12 @@ int launch_linear_split(const void* a_hi, const void* a_lo, long long a_rows, in
   const SplitLow low = {a_lo, w_lo, a_rows};
   const long long results = (rows + clip_rows - 1) / clip_rows * clip_valid - (rows % clip_rows != 0 && rows % clip_rows < clip_valid ? clip_valid - rows % clip_rows : 0);
   const SplitRows map = {a_cols / kBlockK, clip_rows, clip_valid, by_channel, parts, N / n_mats, results * (N / n_mats)};
-  if (few_row_tiles(M, N)) return launch_linear_split_small(a_hi, w_hi, low, map, y, M, N, K, status, st);
+  if (few_row_tiles(M, N)) return launch_linear_split_small(a_hi, w_hi, low, map, y, M, N, K, status, st, dependent);
   const int pair_tiles = ((M + kBlockM - 1) / kBlockM + 1) / 2;
   const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
   const LinearArgs args = {ParamVec(nullptr), nullptr, M, N, K, 0, nullptr, y, map};
   auto fn = half_units(pair_tiles, N, max_pairs, 3 * (K / kBlockK)) ? launch_pairs<4, false, 128> : launch_pairs<4, false, 256>;
-  return fn(a_hi, w_hi, &low, y, args, pair_tiles, max_pairs, 1, 4, status, st, 0);
+  return fn(a_hi, w_hi, &low, y, args, pair_tiles, max_pairs, 1, 4, status, st, dependent);
 }
 
 }  // namespace fm

@@ -326,13 +326,13 @@ int launch_linear_small(const void* a, const void* w, void* y, ParamVec scale, c
 }
 
 int launch_linear_split_small(const void* a_hi, const void* w_hi, const SplitLow& low, const SplitRows& map, float* y, int M, int N,
-                              int K, int* status, cudaStream_t st) {
+                              int K, int* status, cudaStream_t st, int dependent) {
   SmallArgs args = {};
   args.y = y;
   args.M = M;
   args.N = N;
   args.rows = map;
-  return launch_small<4, __half>(a_hi, w_hi, args, K, 1, status, st, 0, &low);
+  return launch_small<4, __half>(a_hi, w_hi, args, K, 1, status, st, dependent, &low);
 }
 
 int launch_qkv_small(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status,

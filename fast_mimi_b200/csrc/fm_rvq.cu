@@ -366,6 +366,7 @@ rvq_decode_split_kernel(const long long* __restrict__ codes, const float* __rest
                         uint16_t* __restrict__ hi, uint16_t* __restrict__ lo, int rows, int T, int n_layers, int n0, int n_codes0,
                         int n_codes1, int* __restrict__ bad_code) {
   using namespace rvq;
+  griddep_launch();                        // opens a chain; the product behind it waits for its end
   const int stacks = n0 < n_layers ? 2 : 1, sub = threadIdx.x & 63;
   for (long long row = static_cast<long long>(blockIdx.x) * 4 + (threadIdx.x >> 6); row < rows; row += static_cast<long long>(gridDim.x) * 4) {
     const long long b = row / T, t = row - b * T;

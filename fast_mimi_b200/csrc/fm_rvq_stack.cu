@@ -2,18 +2,23 @@
 // products and decision kernels in fm_rvq.cu (src/fast_mimi/model.py:2277-2291, :2408-2429).
 //
 // For few vectors that chain is bound by its launches: two a layer of 4 to 7 us each on the GPU and 4 us each on the host, for
-// half a microsecond of products.  Here a thread-block cluster of 16 owns 32 vectors through the stack; block r has entries
+// half a microsecond of products.  Here a thread-block cluster of 16 owns 16 or 32 vectors through the stack; block r has entries
 // 128 r .. of every codebook.  Per layer
-//   products   128 entries (FP16, 64 KB by TMA, two codebooks in flight) x 32 residuals, K = 256, on mma.sync: a tcgen05 tile would
+//   products   128 entries (FP16, 64 KB by TMA, two codebooks in flight) x the residuals, K = 256, on mma.sync: a tcgen05 tile would
 //              be no faster for 32 columns and costs a hand-over through tensor memory
-//   minimum    of the approximate distances: in the block, then over the cluster through distributed shared memory
-//   decision   entries within the vector's margin of it are evaluated exactly in FP32, one warp each, and the smallest
-//              (distance, index) over the cluster wins
-//   residual   every block subtracts the winner for itself: a warp holds its two vectors in registers all along
-// so a layer crosses the cluster twice, and nothing but codes is written.  63 vectors: 7 layers 66 -> 55 us, 31 layers 273 -> 219
-// us, and 16 launches less for stacks of 1 and 7 layers, 18 otherwise (a 5 s utterance end to end, bound by the host, 200 -> 183 us;
-// both stacks as two rows of one grid, which the device runs side by side up to three clusters each, 176 -> 172, no more than runs differ by).  Of the 12300 cycles of a layer the
-// two crossings take 4500, the products 2100 (ldmatrix at the rate of shared memory), the exact distances 1400, the new residual 2700.
+//   candidates entries within the vector's margin of the least approximate distance of the block's own: no fewer than those within
+//              it of the least of all, and that one need not go round the cluster
+//   decision   evaluated exactly in FP32, one warp each and four in flight, and the smallest (distance, index) over the cluster
+//              wins: sent with st.async and counted where they arrive (a barrier of the cluster is a fence besides)
+//   residual   every block subtracts the winner for itself: a warp holds its vectors in registers all along
+// so a layer crosses the cluster once, and nothing but codes is written.  Stacks of 1 and 7 layers, in two rows of one grid, us: with two
+// crossings behind barriers and 32 vectors a cluster -> here: 1 vector 44.7 -> 28.6, 16 47.8 -> 36.0, 63 49.3 -> 36.6, 112 56.1 -> 43.4, 150
+// 57.9 -> 48.1, 224 58.2 -> 56.5; 1 and 31 layers of 63 vectors 212 -> 151.  (16 vectors a cluster: half the candidates and new
+// residuals a block; 113 to 224 vectors need the clusters of 32.)
+//
+// The form with the stacks' input projections inside (512 -> 256 as split-precision products) saves two launches and the vectors' way
+// through memory: 63 vectors, splitting + projection + search 47 us of kernels -> 38.7, 112 -> 82 us end to end with the convolution in front
+// and the host's part.
 #include "fm_common.cuh"
 #include "fm_device_fact.h"
 #include "fm_kernels.h"
@@ -26,6 +31,7 @@ namespace rvqs {
 constexpr int kCtas = 16, kEntries = 128;                      // of a cluster; of a block's share of a codebook
 constexpr int kCodes = kCtas * kEntries;
 constexpr int kDim = 256, kWarps = 16, kThreads = kWarps * 32;
+constexpr int kHidden = 512, kProjected = kDim / kCtas;         // channels in front of the projection; dimensions of a block
 constexpr int kBookBytes = kEntries * kDim * 2, kChunkBytes = kEntries * 128;
 constexpr int kMaxLayers = 32;
 constexpr unsigned long long kNoCandidate = 0xfffffffdull << 32;      // below every distance that is not finite, above those that are
@@ -33,8 +39,9 @@ constexpr int kMaxRows = 32;                                   // vectors of a c
 struct Shared {
   uint64_t full[2];
   uint64_t arrived[2];                             // all blocks' best candidates, of even and of odd layers
+  uint64_t x_full;                                 // the projected vectors
   CtaCtl ctl;
-  uint32_t pad[3];
+  uint32_t pad;
   unsigned long long best[2][kMaxRows][kCtas];     // (distance, index) of every block's best candidate
   float min_in[8][kMaxRows];                       // of 16 entries of this block
   float margin[kMaxRows];
@@ -46,6 +53,9 @@ constexpr int smem_bytes(int rows) { return 1024 + 2 * kBookBytes + rows * kDim 
 
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void st_async_f32(uint32_t addr, float v, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(__float_as_uint(v)), "r"(bar) : "memory");
+}
 __device__ __forceinline__ void st_async_u64(uint32_t addr, unsigned long long v, uint32_t bar) {
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr), "l"(v), "r"(bar) : "memory");
 }
@@ -58,14 +68,26 @@ struct RvqStackArgs {
     const float* e_sq;         // [layers, 2048]
     long long* codes;          // [layers, rows]
     int layers;
+    int w_row;                 // first row of the stack's projection in w_hi and w_lo
     float e_max[rvqs::kMaxLayers];
   };
   Stack stack[2];              // a row of the grid has one
+  const float* frames;         // of the form with the projection inside: [rows, 512], which x is made from
+  const uint16_t *w_hi, *w_lo; // [256 n_stacks, 512]
   int rows;
   float tau_rel;
 };
 
-template <int kRows>
+namespace rvqs {
+// c += W b for 32 values of K: lo and hi are a lane's eight of rows g and g + 8 of W, b its eight of row g of the other operand
+__device__ __forceinline__ void mma_32(float (&c)[4], const uint4& lo, const uint4& hi, const uint4& b) {
+  const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
+  mma_16x8x16<__half>(c, a0, b.x, b.y);
+  mma_16x8x16<__half>(c, a1, b.z, b.w);
+}
+}  // namespace rvqs
+
+template <int kRows, bool kProject>
 __global__ void __launch_bounds__(rvqs::kThreads, 1)
 rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_constant__ CUtensorMap tmap_books1,
                  const __grid_constant__ RvqStackArgs args, int* status) {
@@ -101,20 +123,82 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
     fence_mbar_init();
     mbar_arrive_expect_tx(&sh->arrived[0], kRows * kCtas * 8);
     mbar_arrive_expect_tx(&sh->arrived[1], kRows * kCtas * 8);
+    if (kProject) {
+      mbar_init(&sh->x_full, 1);
+      fence_mbar_init();
+      mbar_arrive_expect_tx(&sh->x_full, kRows * kDim * 4);
+    }
     load_book(0);
-    if (a.layers > 1) load_book(1);
+    if (!kProject && a.layers > 1) load_book(1);
   }
 
   // This warp's vectors, eight values a lane, in every block of the cluster.
   float x[kMine][8];
+  if constexpr (kProject) {
+    // Projection: 16 of the 256 dimensions a block, 32 of the 512 channels a warp.  Operands are FP16 hi + lo parts (of the frames: made
+    // here), the small terms in a sum of their own; K is permuted alike in both, so that a lane's share of 32 channels of a row lies
+    // together.
+    __syncthreads();
+    cluster_arrive_relaxed();                                  // this block runs: its shared memory may be written
+    const int g = lane >> 2, q = lane & 3;
+    float* red = reinterpret_cast<float*>(smem_book + kBookBytes);
+    uint4 w[2][2];                                             // rows g and g + 8; hi and lo
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const size_t at = static_cast<size_t>(a.w_row + rank * kProjected + e * 8 + g) * kHidden + warp * 32 + q * 8;
+      w[e][0] = __ldg(reinterpret_cast<const uint4*>(args.w_hi + at));
+      w[e][1] = __ldg(reinterpret_cast<const uint4*>(args.w_lo + at));
+    }
+    float4 v[kRows / 8][2];
+#pragma unroll
+    for (int t = 0; t < kRows / 8; ++t) {
+      const int f = t * 8 + g;
+      const float4* p = reinterpret_cast<const float4*>(args.frames + static_cast<size_t>(r0 + (f < n ? f : 0)) * kHidden + warp * 32 + q * 8);
+      v[t][0] = __ldg(p);
+      v[t][1] = __ldg(p + 1);
+    }
+#pragma unroll
+    for (int t = 0; t < kRows / 8; ++t) {
+      uint4 hi, lo;
+      split_half8(v[t][0], v[t][1], hi, lo);
+      float small[4] = {0.f, 0.f, 0.f, 0.f}, main[4] = {0.f, 0.f, 0.f, 0.f};
+      mma_32(small, w[0][0], w[1][0], lo);
+      mma_32(small, w[0][1], w[1][1], hi);
+      mma_32(main, w[0][0], w[1][0], hi);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int f = t * 8 + 2 * q + (e & 1), o = g + 8 * (e >> 1);
+        red[(warp * kRows + f) * kProjected + (o ^ ((q & 1) << 3))] = small[e] + main[e];
+      }
+    }
+    __syncthreads();
+    cluster_wait();
+    for (int i = tid; i < kRows * kProjected; i += kThreads) {
+      const int f = i / kProjected, o = i % kProjected;
+      float sum = 0.f;
+#pragma unroll
+      for (int k = 0; k < kWarps; ++k) sum += red[(k * kRows + f) * kProjected + (o ^ (((f >> 1) & 1) << 3))];
+      if (f >= n) sum = 0.f;
+      const uint32_t at = smem_u32(exact_x + f * kDim + rank * kProjected + o), bar = smem_u32(&sh->x_full);
+#pragma unroll
+      for (uint32_t peer = 0; peer < kCtas; ++peer) st_async_f32(map_to_cta(at, peer), sum, map_to_cta(bar, peer));
+    }
+    if (a.layers > 1) {                                        // the second codebook comes where the partial sums were
+      fence_proxy_async_smem();
+      __syncthreads();
+      if (tid == 0) load_book(1);
+    }
+    mbar_wait_cluster(&sh->x_full, 0, ctl, status, kErrWaitConsumer);
+    __syncwarp();
+  }
 #pragma unroll
   for (int i = 0; i < kMine; ++i) {
     const int f = warp + kWarps * i;
 #pragma unroll
     for (int k = 0; k < 8; ++k) x[i][k] = 0.f;
     if (f < n) {
-      const float4* p = reinterpret_cast<const float4*>(a.x + static_cast<size_t>(r0 + f) * kDim + lane * 8);
-      const float4 u = __ldcg(p), v = __ldcg(p + 1);
+      const float4* p = reinterpret_cast<const float4*>(kProject ? exact_x + f * kDim + lane * 8 : a.x + static_cast<size_t>(r0 + f) * kDim + lane * 8);
+      const float4 u = kProject ? p[0] : __ldcg(p), v = kProject ? p[1] : __ldcg(p + 1);
       x[i][0] = u.x; x[i][1] = u.y; x[i][2] = u.z; x[i][3] = u.w; x[i][4] = v.x; x[i][5] = v.y; x[i][6] = v.z; x[i][7] = v.w;
     }
   }
@@ -143,7 +227,7 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
   };
   open_layer(0);
   __syncthreads();
-  cluster_arrive_relaxed();                                    // this block runs: its shared memory may be written
+  if (!kProject) cluster_arrive_relaxed();                     // this block runs: its shared memory may be written
 
   const int g = lane >> 2, cpair = (lane & 3) * 2;
   const int mt = warp >> 1, nh = warp & 1;                     // 16 entries x half of the vectors of the products
@@ -248,7 +332,7 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
       }
     }
     __syncthreads();
-    if (l == 0) cluster_wait();
+    if (!kProject && l == 0) cluster_wait();
     if (tid < kRows * kCtas) {                                 // one of the block's best to one of 16 blocks, counted where it arrives
       const int f = tid % kRows;
       const uint32_t peer = static_cast<uint32_t>(tid / kRows);
@@ -299,11 +383,12 @@ int stack_slots() {
       return ensure_dynamic_smem(reinterpret_cast<const void*>(kern), bytes) == 0 &&
              cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
     };
-    if (!allow(rvq_stack_kernel<16>, rvqs::smem_bytes(16)) || !allow(rvq_stack_kernel<32>, rvqs::smem_bytes(32))) {
+    if (!allow(rvq_stack_kernel<16, false>, rvqs::smem_bytes(16)) || !allow(rvq_stack_kernel<32, false>, rvqs::smem_bytes(32)) ||
+        !allow(rvq_stack_kernel<16, true>, rvqs::smem_bytes(16)) || !allow(rvq_stack_kernel<32, true>, rvqs::smem_bytes(32))) {
       (void)cudaGetLastError();
       return -1;
     }
-    return resident_clusters(rvq_stack_kernel<32>, rvqs::kThreads, rvqs::smem_bytes(32), rvqs::kCtas);
+    return resident_clusters(rvq_stack_kernel<32, false>, rvqs::kThreads, rvqs::smem_bytes(32), rvqs::kCtas);
   });
   return n > 0 ? n : 0;
 }
@@ -318,15 +403,16 @@ bool rvq_stack_takes(const RvqStack* stacks, int n_stacks, long long rows, int n
   return n_codes == rvqs::kCodes && rows <= static_cast<long long>(rvqs::kMaxRows) * stack_slots();
 }
 
-int launch_rvq_stack(const RvqStack* stacks, int n_stacks, long long rows, float tau_rel, int* status, cudaStream_t st) {
+int launch_rvq_stack(const RvqStack* stacks, int n_stacks, long long rows, float tau_rel, int* status, cudaStream_t st, const RvqFrames* from) {
   using namespace rvqs;
   if (n_stacks < 1 || n_stacks > 2 || !(tau_rel >= 0.f)) return -1;
+  if (from != nullptr && (reinterpret_cast<uintptr_t>(from->x) | reinterpret_cast<uintptr_t>(from->w_hi) | reinterpret_cast<uintptr_t>(from->w_lo)) & 15u) return -3;
   RvqStackArgs a = {};
   CUtensorMap maps[2];
   const int longer = n_stacks == 2 && stacks[1].layers > stacks[0].layers ? 1 : 0;     // comes first
   for (int i = 0; i < n_stacks; ++i) {
     const RvqStack& s = stacks[i == 0 ? longer : 1 - longer];
-    if (s.residual == nullptr || s.books16 == nullptr || s.books == nullptr || s.e_sq == nullptr || s.codes == nullptr) return -1;
+    if ((s.residual == nullptr && from == nullptr) || s.books16 == nullptr || s.books == nullptr || s.e_sq == nullptr || s.codes == nullptr) return -1;
     if ((reinterpret_cast<uintptr_t>(s.residual) | reinterpret_cast<uintptr_t>(s.books) | reinterpret_cast<uintptr_t>(s.books16)) & 15u) return -3;
     RvqStackArgs::Stack& d = a.stack[i];
     d.x = s.residual;
@@ -334,6 +420,7 @@ int launch_rvq_stack(const RvqStack* stacks, int n_stacks, long long rows, float
     d.e_sq = s.e_sq;
     d.codes = s.codes;
     d.layers = s.layers;
+    d.w_row = (i == 0 ? longer : 1 - longer) * kDim;
     for (int l = 0; l < s.layers; ++l) {
       if (!(s.e_max[l] >= 0.f)) return -1;
       d.e_max[l] = s.e_max[l];
@@ -349,7 +436,13 @@ int launch_rvq_stack(const RvqStack* stacks, int n_stacks, long long rows, float
   const int few = static_cast<int>((rows + 15) / 16), slots = stack_slots();
   const bool sixteen = few <= slots && (n_stacks == 1 || 2 * few <= slots || 2 * a.stack[1].layers <= a.stack[0].layers);
   const int per = sixteen ? 16 : 32;
-  auto kern = sixteen ? rvq_stack_kernel<16> : rvq_stack_kernel<32>;
+  if (from != nullptr) {
+    a.frames = from->x;
+    a.w_hi = static_cast<const uint16_t*>(from->w_hi);
+    a.w_lo = static_cast<const uint16_t*>(from->w_lo);
+  }
+  auto kern = from != nullptr ? (sixteen ? rvq_stack_kernel<16, true> : rvq_stack_kernel<32, true>)
+                              : (sixteen ? rvq_stack_kernel<16, false> : rvq_stack_kernel<32, false>);
   return launch_kernel(kern, dim3(static_cast<unsigned>((rows + per - 1) / per) * kCtas, static_cast<unsigned>(n_stacks)), kThreads, smem_bytes(per), st, kCtas,
                        0, maps[0], maps[1], a, status);
 }

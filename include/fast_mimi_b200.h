@@ -229,6 +229,11 @@ int fm_linear_rows_f32(const float* x, const void* w_hi, const void* w_lo, float
 int fm_conv_frames_f32(const float* x, const void* w_hi, const void* w_lo, float* y, int B, int T, int C, int kernel, int stride, int n_out, int* status,
                        void* stream);
 
+/* fm_conv_frames_split into hi, lo [B * (ceil(T / stride) + kernel / stride - 1), stride * C] FP16 and the product over them, y [B, ceil(T /
+ * stride), n_out], as a chain of two launches: the form for few frames. */
+int fm_conv_parts_f32(const float* x, void* hi, void* lo, const void* w_hi, const void* w_lo, float* y, int B, int T, int C, int kernel, int stride,
+                      int n_out, int* status, void* stream);
+
 /* The stride-2 upsampling that precedes the decoder transformer (MimiModel.upsample: MimiConvTranspose1d(512, 512,
  * kernel 4, stride 2, groups 512, no bias), src/fast_mimi/model.py:2745-2753; its forward trims the last two output
  * frames): x [B, T, C] FP32 frame-major, w [C, 4] FP32 (the ConvTranspose1d weight [C, 1, 4]) -> y [B, 2T, C] FP32,
@@ -266,6 +271,12 @@ typedef struct {
   int layers;
 } fm_rvq_stack;
 int fm_rvq_encode_stacks_f32(const fm_rvq_stack* stacks, int n_stacks, void* residual16, float* tau, void* records, long long rows,
+                             int n_codes, float tau_rel, int* status, void* stream);
+
+/* fm_rvq_encode_stacks_f32 for few vectors with the stacks' input projections inside the same kernel: x [rows, k_in], w_hi and w_lo
+ * fm_split_half of [256 n_stacks, k_in], first stack first; `residual` and workspaces are not used.  -9, nothing launched: no such
+ * form for so many vectors or layers, codebooks of this size, or k_in other than 512. */
+int fm_rvq_encode_frames_f32(const float* x, int k_in, const void* w_hi, const void* w_lo, const fm_rvq_stack* stacks, int n_stacks, long long rows,
                              int n_codes, float tau_rel, int* status, void* stream);
 
 /* The form of that which many vectors take, whether or not it is the faster one for so many: one kernel, no workspaces.  At most 32

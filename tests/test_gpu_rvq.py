@@ -340,7 +340,8 @@ def test_decoding_one_code_takes_less_than_eight():
     assert time(1) < 0.55 * time(8)
 
 
-@pytest.mark.parametrize("B,T", [(1, 1), (3, 21), (2, 1100)])
+# rows: one, either side of what a cluster of 16 or 32 vectors takes, of where 16 give way to 32, of the last that one kernel takes; many
+@pytest.mark.parametrize("B,T", [(1, 1), (1, 16), (1, 17), (3, 21), (1, 65), (1, 113), (2, 112), (1, 225), (2, 1100)])
 @pytest.mark.parametrize("quantizers", [2, 8])
 def test_calls_of_the_binding_are_the_checked_ones(B, T, quantizers):
     """Convolution, search, decode and upsampling through the binding give the bits of the checked calls behind them (which a type or
