@@ -242,16 +242,21 @@ int launch_ring_append(const void* k_new, const void* v_new, void* ring_k, void*
 // T <= 8 new frames per stream over its ring (at most 256 slots), ring update included (fm_stream_attn.cu).
 int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k, void* ring_v, void* out, int S, int T,
                        int past, int slots, int window, float scale, int value_is_fp16, int* status, cudaStream_t st,
-                       int dependent = 0, const struct StreamOut* proj = nullptr);
-// With `proj` the result goes through the output projection, x1 = resid + scale * out W_o^T (rows of stream_type; no scale: one), and
-// `out` is not written: for as many streams as stream_attn_projects says.
-struct StreamOut {
-  const void *w_o, *resid;
-  void* x1;
-  ParamVec scale;
-  int stream_type;
+                       int dependent = 0);
+// LayerNorm, projection and that attention in one kernel (fm_stream_front.cu), which opens a layer's chain, for as many streams as
+// stream_front_takes says.
+struct StreamFront {
+  const void* x;                  // [S, T, 512] of stream_type
+  ParamVec ln_weight, ln_bias;
+  float eps;
+  const void* w_qkv;
+  const float *cos, *sin;
+  long long cos_bstride;
+  void *ring_k, *ring_v, *core;
+  int stream_type, value_fp16, tc_fp16;
 };
-bool stream_attn_projects(int S, int T);
+bool stream_front_takes(int S, int T, int slots);
+int launch_stream_front(const StreamFront& f, int S, int T, int past, int slots, int window, float scale, int* status, cudaStream_t st, int dependent);
 // Attention for few query tiles (fm_few_attn.cu): at most two 64-query blocks per SM.  ring_k null: clips; else T new frames
 // per stream on top of the ring, which the kernel also updates where one block has a whole (stream, head).
 bool few_attn_tiles(int S, int T);

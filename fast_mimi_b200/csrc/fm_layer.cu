@@ -72,17 +72,20 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
   const int value_fp16 = p.value_dtype & 1;
   const int tc = (p.value_dtype & 2) ? 1 : 0;                    // 16-bit type of the products' operands: 0 BF16, 1 FP16
 
+  const bool front = few && stream_front_takes(B, T, slots);    // everything up to the attention is one kernel
   const bool norm1_inside = few_rows_with_norm(rows, 1536), norm2_inside = few_rows_with_norm(rows, p.ffn);
   int rc = 0;
-  if (!norm1_inside) {
+  if (!norm1_inside && !front) {
     rc = launch_layernorm512(x, p.stream_dtype, vec(p.ln1_weight), vec(p.ln1_bias), p.ln1_eps, b.h, tc, rows, st, 1);
     if (rc != 0) return rc;
   }
   const bool one_tail = layer_tail_takes(rows, p.ffn);          // everything behind the attention is one kernel
-  const bool projected = !one_tail && few && stream_attn_projects(B, T);     // the attention kernel goes on to x1
-  const StreamOut proj = {p.w_o, x, b.x1, vec(p.attn_scale), p.stream_dtype};
   const bool few_tiles = !few && few_attn_tiles(B, T) && (!cached || slots <= 256);
-  if (whole_clip && !few_tiles && use_fused_clip(B, T)) {
+  if (front) {
+    const StreamFront f = {x, vec(p.ln1_weight), vec(p.ln1_bias), p.ln1_eps, p.w_qkv, cos, sin, cos_bstride, ring_k, ring_v, b.core, p.stream_dtype,
+                           value_fp16, tc};
+    rc = launch_stream_front(f, B, T, past, slots, p.window, p.scale, status, st, p.weights_settled);
+  } else if (whole_clip && !few_tiles && use_fused_clip(B, T)) {
     rc = launch_attn_fused_clip(b.h, p.w_qkv, cos, sin, cos_bstride, b.core, B, T, p.window, p.scale, p.value_dtype, status, st, 1);
   } else {
     QkvEpilogueArgs ep = {};
@@ -106,8 +109,7 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
     } else if (!cached) {
       rc = launch_band_attn_prefill(b.q, b.k, b.v, b.core, B, T, p.window, p.scale, value_fp16, status, st, 1);
     } else if (few) {
-      rc = launch_stream_attn(b.q, b.k, b.v, ring_k, ring_v, b.core, B, T, past, slots, p.window, p.scale, value_fp16, status, st, 1,
-                              projected ? &proj : nullptr);
+      rc = launch_stream_attn(b.q, b.k, b.v, ring_k, ring_v, b.core, B, T, past, slots, p.window, p.scale, value_fp16, status, st, 1);
     } else {
       if (delta > 0) {
         rc = launch_ring_linearize(ring_k, ring_v, b.k, b.v, b.k_lin, b.v_lin, B, T, delta, past, slots, st, 1);
@@ -126,7 +128,7 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
                          p.ln2_eps, p.stream_dtype, value_fp16, tc};
     return launch_layer_tail(t, rows, status, st, 1);
   }
-  if (!projected) rc = launch_linear_gemm(b.core, p.w_o, b.x1, vec(p.attn_scale), x, rows, 512, 512, value_fp16, p.stream_dtype, 0, status, st, 1);
+  rc = launch_linear_gemm(b.core, p.w_o, b.x1, vec(p.attn_scale), x, rows, 512, 512, value_fp16, p.stream_dtype, 0, status, st, 1);
   if (rc != 0) return rc;
   if (norm2_inside) {
     rc = launch_ln_linear_gelu(b.x1, p.stream_dtype, vec(p.ln2_weight), vec(p.ln2_bias), p.ln2_eps, p.w_fc1, b.g, rows, p.ffn, tc, status,

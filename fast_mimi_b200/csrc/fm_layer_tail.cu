@@ -73,13 +73,6 @@ __device__ __forceinline__ void copy_to_cta(uint32_t src, uint32_t dst, uint32_t
   asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(map_to_cta(dst, cta)), "r"(src), "r"(bytes), "r"(map_to_cta(smem_u32(bar), cta)) : "memory");
 }
-// c += W b for 32 values of K: lo and hi are a lane's eight of rows g and g + 8 of W, b its eight of row g of the other operand
-template <typename T>
-__device__ __forceinline__ void mma_32(float (&c)[4], const uint4& lo, const uint4& hi, const uint4& b) {
-  const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
-  mma_16x8x16<T>(c, a0, b.x, b.y);
-  mma_16x8x16<T>(c, a1, b.z, b.w);
-}
 // A value of the residual stream as it is stored: type 0 BF16, 1 FP16, 2 FP32.
 __device__ __forceinline__ float stream_load(const void* p, long long at, int type) {
   if (type == 2) return __ldcg(static_cast<const float*>(p) + at);
@@ -190,7 +183,7 @@ layer_tail_kernel(const __grid_constant__ CUtensorMap tmap_w1, const __grid_cons
       for (int mt = 0; mt < 2; ++mt) {
         d[mt][0] = d[mt][1] = d[mt][2] = d[mt][3] = 0.f;
 #pragma unroll
-        for (int j = 0; j < 2; ++j) mma_32<VT>(d[mt], w_o[mt][j][0], w_o[mt][j][1], b[t][j]);
+        for (int j = 0; j < 2; ++j) mma_16x8x32<VT>(d[mt], w_o[mt][j][0], w_o[mt][j][1], b[t][j]);
       }
 #pragma unroll
       for (int mt = 0; mt < 2; ++mt) {

@@ -78,15 +78,6 @@ struct RvqStackArgs {
   float tau_rel;
 };
 
-namespace rvqs {
-// c += W b for 32 values of K: lo and hi are a lane's eight of rows g and g + 8 of W, b its eight of row g of the other operand
-__device__ __forceinline__ void mma_32(float (&c)[4], const uint4& lo, const uint4& hi, const uint4& b) {
-  const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
-  mma_16x8x16<__half>(c, a0, b.x, b.y);
-  mma_16x8x16<__half>(c, a1, b.z, b.w);
-}
-}  // namespace rvqs
-
 template <int kRows, bool kProject>
 __global__ void __launch_bounds__(rvqs::kThreads, 1)
 rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_constant__ CUtensorMap tmap_books1,
@@ -162,9 +153,9 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
       uint4 hi, lo;
       split_half8(v[t][0], v[t][1], hi, lo);
       float small[4] = {0.f, 0.f, 0.f, 0.f}, main[4] = {0.f, 0.f, 0.f, 0.f};
-      mma_32(small, w[0][0], w[1][0], lo);
-      mma_32(small, w[0][1], w[1][1], hi);
-      mma_32(main, w[0][0], w[1][0], hi);
+      mma_16x8x32<__half>(small, w[0][0], w[1][0], lo);
+      mma_16x8x32<__half>(small, w[0][1], w[1][1], hi);
+      mma_16x8x32<__half>(main, w[0][0], w[1][0], hi);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int f = t * 8 + 2 * q + (e & 1), o = g + 8 * (e >> 1);

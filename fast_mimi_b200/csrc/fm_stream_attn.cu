@@ -23,20 +23,12 @@
 // Rows that are already in the ring do not depend on the projection, so in a chain of dependent launches the first items
 // are requested before the wait for it.  A block has an item's ring rows in shared memory before it stores that item's
 // new rows, and no other block touches its (stream, head): the ring is updated in place.
-//
-// Where fm_layer_tail.cu does not take what follows (an MLP of another size than 2048) and while the heads of every stream have blocks
-// of their own at the same time (up to 15 streams on a B200), the kernel goes on to the output projection, x1 = residual + scale * core W_o^T: the eight blocks of a stream are a cluster, hand each other their heads'
-// rows through distributed shared memory, and each multiplies them with its 64 rows of W_o, which it asked for before the wait.  As
-// a kernel of its own the projection of a few rows was 4.6 us, a launch and a first load around 0.3 us of products.  The rows are sent
-// with st.async and counted where they arrive: a barrier of the cluster is a fence besides, for every warp (0.3 to 0.5 us a layer).
-// GPU time of eight FP32 layers, a kernel of its own -> behind a barrier -> counted: 1 stream of one frame 149.9 -> 127.5 -> 125.2 us, 15 of
-// one 167.5 -> 158.0 -> 155.4, 15 of eight 197.9 -> 185.1 -> 182.1.
 #include <type_traits>
 
 #include "fm_common.cuh"
-#include "fm_device_fact.h"
 #include "fm_kernels.h"
 #include "fm_launch.h"
+#include "fm_stream_math.cuh"
 #include "fm_warp_mma.cuh"
 
 namespace fm {
@@ -57,36 +49,13 @@ struct Ctl {
   // phase cannot tell the one two before from it): it read, and gave back, a stage that was being filled.
   uint64_t full[kMaxStages * kGroups];
   uint64_t empty[kMaxStages];
-  uint64_t w_full;
-  uint64_t heads_full;     // the stream's eight heads have sent their rows
   CtaCtl ctl;
   float m[kGroups][kGroupWarps][kMaxT];
   float l[kGroups][kGroupWarps][kMaxT];
 };
-// Output projection: this block's rows of W_o (eight chunks of 64 x 64), and the eight heads' rows of the stream (8 x 64 each)
-constexpr int kOutBytes = 64 * 1024, kHeadsBytes = 8 * 1024;
-constexpr int smem_bytes(int stages, bool out_proj = false) {
-  return (out_proj ? kOutBytes + kHeadsBytes : 0) + 1024 + stages * kStageBytes + kGroups * (kNewBytes + kMergeBytes) + static_cast<int>(sizeof(Ctl));
-}
+constexpr int smem_bytes(int stages) { return 1024 + stages * kStageBytes + kGroups * (kNewBytes + kMergeBytes) + static_cast<int>(sizeof(Ctl)); }
 static_assert(smem_bytes(kMaxStages) <= 232448, "exceeds the 227 KB a block may use");
 
-// Probabilities as operands of type T without losing bits of FP32: as a sum of kParts values.  BF16 has eight significant bits
-// and the range of FP32: three parts are all 24.  FP16 has eleven, and a sign on the second part makes two of them 24 to within
-// the last bit, but nothing below 2^-24: probabilities carry a factor of 2^kShift, the sum they are divided by likewise.  (As two
-// parts each and unscaled, an FP16 result carried by probabilities of 2^-20 was off by up to 4e-3, one of BF16 by 2^-17 of its terms.)
-template <typename T> struct Parts { static constexpr int kParts = 3; static constexpr float kShift = 0.f; };
-template <> struct Parts<__half> { static constexpr int kParts = 2; static constexpr float kShift = 15.f; };
-
-template <typename T>
-__device__ __forceinline__ void split_pair(float x, float y, uint32_t (&part)[Parts<T>::kParts]) {
-#pragma unroll
-  for (int i = 0; i < Parts<T>::kParts; ++i) {
-    part[i] = Pack16<T>::pack(x, y);
-    const float2 b = Pack16<T>::unpack(part[i]);
-    x -= b.x;
-    y -= b.y;
-  }
-}
 }  // namespace stream
 
 struct StreamArgs {
@@ -98,32 +67,16 @@ struct StreamArgs {
   int stages;
   float scale_log2e;
 };
-// What the output projection needs: an argument of its kernels alone (200 bytes more cost the others 0.5 % with 64 streams).
-template <bool kOut> struct StreamOutArgs {};
-template <> struct StreamOutArgs<true> {
-  CUtensorMap w_o;
-  const void* resid;             // [S, T, 512] of stream_type
-  void* x1;
-  ParamVec scale;                // without data: one
-  int stream_type;               // 0 BF16, 1 FP16, 2 FP32
-};
-
-// kOut: a block has one item, the eight heads of a stream are a cluster, and the result goes through the output projection.
 // VT: type of the ring's values, v and the result
-template <typename VT, bool kOut>
+template <typename VT>
 __global__ void __launch_bounds__(stream::kThreads, 1)
 stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
-                   const __grid_constant__ StreamArgs a, const __grid_constant__ StreamOutArgs<kOut> out, int* status) {
+                   const __grid_constant__ StreamArgs a, int* status) {
   using namespace stream;
-  // A status set before this chain began: nothing is stored.  The blocks of a cluster write into one another's memory and
-  // stay to the end.
-  const bool skip = kOut && status != nullptr && *reinterpret_cast<volatile int*>(status) != 0;
-  if (!kOut && chain_stopped(status)) return;
+  if (chain_stopped(status)) return;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* smem_out = smem + a.stages * kStageBytes;           // kOut: W_o, then the heads
-  uint8_t* smem_heads = smem_out + kOutBytes;
-  uint8_t* smem_new = kOut ? smem_heads + kHeadsBytes : smem_out;
+  uint8_t* smem_new = smem + a.stages * kStageBytes;
   float* smem_merge = reinterpret_cast<float*>(smem_new + kGroups * kNewBytes);
   Ctl* c = reinterpret_cast<Ctl*>(smem_new + kGroups * (kNewBytes + kMergeBytes));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -133,13 +86,8 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
       mbar_init(&c->empty[i], kGroupWarps);
     }
     for (int i = 0; i < kGroups * a.stages; ++i) mbar_init(&c->full[i], 1);
-    if (kOut) {
-      mbar_init(&c->w_full, 1);
-      mbar_init(&c->heads_full, 1);
-    }
     c->ctl.abort = 0;
     fence_mbar_init();
-    if (kOut) mbar_arrive_expect_tx(&c->heads_full, 1024u * static_cast<uint32_t>(a.T));
   }
   // Slots past the loaded ones and rows past the new ones are never written: zeros, so that a probability of zero times
   // what lies there is zero.
@@ -149,21 +97,13 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
     *reinterpret_cast<uint4*>(smem + tile * kTileBytes + a.n_loaded * 128 + piece * 16) = zero;
   }
   for (int i = threadIdx.x; i < kGroups * kNewBytes / 16; i += kThreads) *reinterpret_cast<uint4*>(smem_new + i * 16) = zero;
-  if (kOut)
-    for (int i = threadIdx.x; i < kHeadsBytes / 16; i += kThreads) *reinterpret_cast<uint4*>(smem_heads + i * 16) = zero;
   fence_proxy_async_smem();
   __syncthreads();
-  if (kOut) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // this block's memory may be written
   griddep_launch();
   CtaCtl* ctl = &c->ctl;
 
   if (warp == kGroups * kGroupWarps) {
     if (lane == 0) {
-      if constexpr (kOut) {
-        mbar_arrive_expect_tx(&c->w_full, kOutBytes);
-#pragma unroll
-        for (int kc = 0; kc < 8; ++kc) tma_load_2d(smem_out + kc * 8192, &out.w_o, &c->w_full, kc * 64, static_cast<int>(blockIdx.x & 7) * 64);
-      }
       if (a.n_loaded > 0) {
         tma_prefetch_desc(&tmap_k);
         tma_prefetch_desc(&tmap_v);
@@ -242,7 +182,7 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
           if (piece < n_pieces) {
             *reinterpret_cast<uint4*>(new_k + sw128_offset(t, piece & 7)) = nk[e];
             *reinterpret_cast<uint4*>(new_v + sw128_offset(t, piece & 7)) = nv[e];
-            if (t >= a.T - a.slots && !skip) {           // of two rows for one slot the newer stays
+            if (t >= a.T - a.slots) {           // of two rows for one slot the newer stays
               const size_t at = (static_cast<size_t>(item) * a.slots + (a.past + t) % a.slots) * 64 + (piece & 7) * 8;
               *reinterpret_cast<uint4*>(a.ring_k + at) = nk[e];
               *reinterpret_cast<uint4*>(a.ring_v + at) = nv[e];
@@ -381,33 +321,6 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         }
       }
       named_bar_sync(1 + cg, kGroupWarps * 32);
-      if constexpr (kOut) {
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");            // the other heads' blocks run
-        // two values a thread, to the eight blocks of the stream
-        for (int i = gt; i < a.T * 32; i += kGroupWarps * 32) {
-          const int t = i >> 5, d = 2 * (i & 31);
-          float mx = -INFINITY;
-#pragma unroll
-          for (int w = 0; w < kGroupWarps; ++w) mx = fmaxf(mx, c->m[cg][w][t]);
-          float num[2] = {0.f, 0.f}, den = 0.f;
-#pragma unroll
-          for (int w = 0; w < kGroupWarps; ++w) {
-            const float f = ex2_approx(c->m[cg][w][t] - mx);
-            const float2 v = *reinterpret_cast<const float2*>(&merge[(w * kMaxT + t) * 64 + d]);
-            num[0] = fmaf(f, v.x, num[0]);
-            num[1] = fmaf(f, v.y, num[1]);
-            den = fmaf(f, c->l[cg][w][t], den);
-          }
-          const uint32_t pair = Pack16<VT>::pack(num[0] / den, num[1] / den);
-          const uint32_t at = smem_u32(smem_heads + h * 1024) + sw128_offset(t, d >> 3) + (d & 7) * 2;
-#pragma unroll
-          for (uint32_t peer = 0; peer < 8; ++peer)    // counted where they arrive: a barrier of the cluster would be a fence besides
-            asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
-                         ::"r"(map_to_cta(at, peer)), "r"(pair), "r"(map_to_cta(smem_u32(&c->heads_full), peer)) : "memory");
-        }
-        __syncwarp();
-        continue;                                        // the block's only item
-      }
       for (int i = gt; i < a.T * 64; i += kGroupWarps * 32) {
         const int t = i >> 6, d = i & 63;
         float mx = -INFINITY;
@@ -427,88 +340,13 @@ stream_attn_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
       named_bar_sync(1 + cg, kGroupWarps * 32);          // the merge buffer and the new rows' tiles are free again
     }
   }
-  if constexpr (kOut) {
-    __syncwarp();
-    if (warp >= kGroupWarps) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");     // the first group is past it
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // this block has sent what it had to send
-    float* red = reinterpret_cast<float*>(smem);         // the ring's stage is done with: eight partial results of 8 x 64
-    const int channel = static_cast<int>(blockIdx.x & 7) * 64 + (threadIdx.x & 63);
-    float scale = 1.f;                                   // asked for ahead of the wait (in the loop over frames: 1 % for five frames)
-    if (warp < 8 && out.scale.data != nullptr) scale = out.scale.at(channel);
-    if (warp < 8) {
-      // y^T = W_o core^T: 64 rows of W_o, the stream's frames as eight columns; warp w has K of head w
-      mbar_wait(&c->w_full, 0, ctl, status, kErrWaitTma);
-      mbar_wait_cluster(&c->heads_full, 0, ctl, status, kErrWaitConsumer);
-      __syncwarp();
-      float y[4][4];
-#pragma unroll
-      for (int mt = 0; mt < 4; ++mt) y[mt][0] = y[mt][1] = y[mt][2] = y[mt][3] = 0.f;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t b[4];
-        ldmatrix4(b, smem_u32(smem_heads + warp * 1024) + sw128_offset(lane & 7, 4 * half + (lane >> 3)));
-#pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-#pragma unroll
-          for (int mt = 0; mt < 4; ++mt) {
-            uint32_t w[4];
-            ldmatrix4(w, smem_u32(smem_out + warp * 8192) + sw128_offset(mt * 16 + (lane & 15), 4 * half + 2 * ks + (lane >> 4)));
-            mma_16x8x16<VT>(y[mt], w, b[2 * ks], b[2 * ks + 1]);
-          }
-        }
-      }
-      const int g = lane >> 2, cpair = (lane & 3) * 2;
-#pragma unroll
-      for (int mt = 0; mt < 4; ++mt) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) red[(warp * 8 + cpair + (e & 1)) * 64 + mt * 16 + g + 8 * (e >> 1)] = y[mt][e];
-      }
-    }
-    __syncthreads();
-    const long long row0 = static_cast<long long>(blockIdx.x >> 3) * a.T;
-    for (int t = static_cast<int>(threadIdx.x) >> 6; t < a.T && threadIdx.x < 256; t += 4) {
-      float v = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) v += red[(w * 8 + t) * 64 + (threadIdx.x & 63)];
-      const long long at = (row0 + t) * 512 + channel;
-      v *= scale;
-      if (out.stream_type == 2) {
-        v += __ldcg(static_cast<const float*>(out.resid) + at);
-        if (!skip) static_cast<float*>(out.x1)[at] = v;
-      } else if (out.stream_type == 1) {
-        v += __half2float(__ushort_as_half(__ldcg(static_cast<const uint16_t*>(out.resid) + at)));
-        if (!skip) static_cast<uint16_t*>(out.x1)[at] = __half_as_ushort(__float2half_rn(v));
-      } else {
-        v += __bfloat162float(__ushort_as_bfloat16(__ldcg(static_cast<const uint16_t*>(out.resid) + at)));
-        if (!skip) static_cast<uint16_t*>(out.x1)[at] = __bfloat16_as_ushort(__float2bfloat16_rn(v));
-      }
-    }
-  }
-  if constexpr (kOut) {
-    __syncwarp();
-    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");        // nobody still writes into a block that has left
-  }
   __syncthreads();
   if (ctl->abort) __nanosleep(20000);
 }
 
-// With 64 KB of W_o a block fills an SM; as many streams as the device holds clusters of eight such blocks at once (15 on a B200), since
-// one more waits for a second wave (4 us a layer, what the projection saves).  GPU time of eight FP32 layers on full rings, a kernel of
-// its own -> here: 1 stream of one frame 149.9 -> 125, 15 streams of 1, 2 and 8 frames 167.5 -> 155, 183.0 -> 160 and 197.9 -> 182.
-bool stream_attn_projects(int S, int T) {
-  static DeviceFact clusters;
-  int dev = 0;
-  if (T > stream::kMaxT || cudaGetDevice(&dev) != cudaSuccess) return false;
-  return S <= clusters.get(dev, [] {
-    const auto kern = stream_attn_kernel<__half, true>;        // the one for BF16 values takes as much
-    const int bytes = stream::smem_bytes(1, true);
-    return ensure_dynamic_smem(reinterpret_cast<const void*>(kern), bytes) == 0 ? resident_clusters(kern, stream::kThreads, bytes, 8) : -1;
-  });
-}
-
 int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k, void* ring_v, void* out, int S, int T,
                        int past, int slots, int window, float scale, int value_is_fp16, int* status,
-                       cudaStream_t st, int dependent, const StreamOut* proj) {
+                       cudaStream_t st, int dependent) {
   using namespace stream;
   if (S <= 0 || T <= 0) return (S == 0 || T == 0) ? 0 : -1;
   if (past < 0 || window <= 0 || slots < window || slots > 256 || T > kMaxT) return -1;
@@ -530,27 +368,10 @@ int launch_stream_attn(const void* q, const void* k, const void* v, void* ring_k
   const StreamArgs a = {static_cast<const uint16_t*>(q), static_cast<const uint16_t*>(k), static_cast<const uint16_t*>(v),
                   static_cast<uint16_t*>(ring_k), static_cast<uint16_t*>(ring_v), static_cast<uint16_t*>(out), n_items, T, past, delta, slots, window,
                   n_loaded, stages, scale * 1.4426950408889634f};
-  const int bytes = smem_bytes(stages, proj != nullptr), blocks = n_items < sms ? n_items : sms;
-  auto launch = [&](auto kern, const auto& then, int cluster) {
-    const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), bytes);
-    return rc != 0 ? rc : launch_kernel(kern, dim3(blocks), kThreads, bytes, st, cluster, dependent, tk, tv, a, then, status);
-  };
-  if (proj == nullptr) {
-    const StreamOutArgs<false> none = {};
-    return value_is_fp16 ? launch(stream_attn_kernel<__half, false>, none, 1) : launch(stream_attn_kernel<__nv_bfloat16, false>, none, 1);
-  }
-  if (!stream_attn_projects(S, T)) return -1;
-  if ((reinterpret_cast<uintptr_t>(proj->w_o) | reinterpret_cast<uintptr_t>(proj->resid) | reinterpret_cast<uintptr_t>(proj->x1) |
-       reinterpret_cast<uintptr_t>(proj->scale.data)) & 15u)
-    return -3;
-  StreamOutArgs<true> o = {};
-  const int rc = encode_rows_16bit(&o.w_o, proj->w_o, 512, 512, 64, 64);
-  if (rc != 0) return rc;
-  o.resid = proj->resid;
-  o.x1 = proj->x1;
-  o.scale = proj->scale;
-  o.stream_type = proj->stream_type;
-  return value_is_fp16 ? launch(stream_attn_kernel<__half, true>, o, 8) : launch(stream_attn_kernel<__nv_bfloat16, true>, o, 8);
+  const int bytes = smem_bytes(stages), blocks = n_items < sms ? n_items : sms;
+  const auto kern = value_is_fp16 ? stream_attn_kernel<__half> : stream_attn_kernel<__nv_bfloat16>;
+  const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), bytes);
+  return rc != 0 ? rc : launch_kernel(kern, dim3(blocks), kThreads, bytes, st, 1, dependent, tk, tv, a, status);
 }
 
 }  // namespace fm

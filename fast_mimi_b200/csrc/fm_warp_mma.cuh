@@ -29,6 +29,14 @@ __device__ __forceinline__ void mma_16x8x16(float (&c)[4], const uint32_t (&a)[4
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// The same over 32 values of K that lie together: lo and hi are a lane's eight (8 (lane % 4) .. of 32) of rows g and g + 8 of the first operand, b its
+// eight of row g of the second, g = lane / 4.  K is permuted alike in both, which a sum does not mind.
+template <typename T>
+__device__ __forceinline__ void mma_16x8x32(float (&c)[4], const uint4& lo, const uint4& hi, const uint4& b) {
+  const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
+  mma_16x8x16<T>(c, a0, b.x, b.y);
+  mma_16x8x16<T>(c, a1, b.z, b.w);
+}
 // Transpose of an 8 x 8 matrix of 16-bit values spread over the warp as fragments are (row lane / 4, columns 2 (lane % 4) ..).
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
   uint32_t y;

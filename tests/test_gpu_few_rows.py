@@ -236,6 +236,36 @@ def test_live_streams_against_64_bits(T, past, dtype, value_dtype):
     fm.check_status()
 
 
+# past: nothing, either side of a warp's sixteen slots, of a full ring and of its turn; 18 streams are the last that take the kernel on a B200
+@pytest.mark.parametrize("past", [0, 1, 15, 16, 17, 241, 249, 250, 257, 1000])
+@pytest.mark.parametrize("streams,T", [(1, 1), (2, 3), (18, 8)])
+@pytest.mark.parametrize("dtype,value_dtype", [(torch.float32, torch.float16), (torch.bfloat16, torch.bfloat16), (torch.float16, torch.float16)])
+def test_first_half_of_a_call_for_few_streams(streams, T, past, dtype, value_dtype):
+    """LayerNorm, projection and attention as one kernel (up to 18 streams) and as two (the same streams among 19): rings are equal bit
+    for bit, what a layer adds agrees but for the order of FP32 sums, i.e. where that flips the rounding of a 16-bit operand (bounds as
+    where the output projection's routes are compared)."""
+    import fast_mimi_b200 as fm
+    layer = fm.MimiTransformerLayerB200(value_dtype=value_dtype).cuda()
+    layer.load_state_dict(_layer_params(T + past), strict=True)
+    layer = layer.to(dtype)
+    g = torch.Generator(device="cuda").manual_seed(past + T)
+    x = torch.randn(19, T, 512, device="cuda", generator=g).to(dtype)
+    cs = fm.rope_tables(torch.randint(0, 3000, (19, T), device="cuda", generator=g))           # a table per stream
+    many, few = fm.MimiKVRing(1, 19, 250, value_dtype=value_dtype), fm.MimiKVRing(1, streams, 250, value_dtype=value_dtype)
+    for t, u in ((many.ring_k, few.ring_k), (many.ring_v, few.ring_v)):
+        t.normal_(generator=g)
+        u.copy_(t[:, :streams])
+    for ring in (many, few):
+        ring.advance(0, past)
+    want = layer(x, None, many, cs)[0][:streams].float()
+    got = layer(x[:streams], None, few, tuple(t[:streams] for t in cs))[0].float()
+    base = x[:streams].float()
+    bound = {torch.float32: 1e-3, torch.float16: 4e-3, torch.bfloat16: 2e-2}[dtype]
+    assert O.rel_l2((got - base).cpu(), (want - base).cpu()) < bound
+    assert torch.equal(few.ring_k, many.ring_k[:, :streams]) and torch.equal(few.ring_v, many.ring_v[:, :streams])
+    fm.check_status()
+
+
 # rows: one, either side of a cluster's rows (8) and of what seven clusters of 8, 16 and 24 rows hold; two clips; an MLP of another size, for
 # which there is no such kernel
 @pytest.mark.parametrize("B,T,ffn", [(1, 1, 2048), (1, 8, 2048), (1, 9, 2048), (1, 56, 2048), (1, 57, 2048), (1, 112, 2048), (1, 113, 2048), (2, 61, 2048),
@@ -244,7 +274,7 @@ def test_live_streams_against_64_bits(T, past, dtype, value_dtype):
                                                (torch.bfloat16, torch.float16), (torch.float16, torch.float16)])
 def test_layer_on_few_rows_against_64_bits(B, T, ffn, dtype, value_dtype):
     """A layer on clips of few rows in all, where everything behind the attention is one kernel, against the same in 64 bits; bars as for
-    live streams below (BF16 values: their rounding, 2^-9, in front of the output projection).  In place it is the same bit for bit."""
+    live streams below (BF16 values: their rounding, 2^-9, in front of the output projection)."""
     import fast_mimi_b200 as fm
     layer = fm.MimiTransformerLayerB200(intermediate_size=ffn, value_dtype=value_dtype).cuda()
     p = _layer_params(T)
@@ -267,10 +297,6 @@ def test_layer_on_few_rows_against_64_bits(B, T, ffn, dtype, value_dtype):
     base = xd if dtype == torch.float32 else torch.zeros_like(xd)
     bar = {torch.float32: 2e-3 if value_dtype == torch.float16 else 4e-3, torch.bfloat16: 2 ** -8, torch.float16: 2 ** -10}[dtype]
     assert O.rel_l2(y.double() - base, want - base) < bar
-    params, keep = layer._native_plan(x)
-    again = x.clone()
-    fm.ops.layer_forward(params, again, cos, sin, value_dtype=value_dtype, out=again)
-    assert torch.equal(again, y)
     fm.check_status()
 
 
