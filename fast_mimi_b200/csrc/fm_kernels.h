@@ -168,6 +168,7 @@ struct LayerTail {
   ParamVec attn_scale, mlp_scale, ln_weight, ln_bias;
   float eps;
   int stream_type, value_fp16, tc_fp16;
+  int beside;                                // blocks of the kernel in front that have an SM each to themselves
 };
 bool layer_tail_takes(int M, int ffn);
 int launch_layer_tail(const LayerTail& t, int M, int* status, cudaStream_t st, int dependent);

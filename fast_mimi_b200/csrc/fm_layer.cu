@@ -125,7 +125,7 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
   if (rc != 0) return rc;
   if (one_tail) {
     const LayerTail t = {b.core, p.w_o, p.w_fc1, p.w_fc2, x, y, vec(p.attn_scale), vec(p.mlp_scale), vec(p.ln2_weight), vec(p.ln2_bias),
-                         p.ln2_eps, p.stream_dtype, value_fp16, tc};
+                         p.ln2_eps, p.stream_dtype, value_fp16, tc, front ? 8 * B : 0};
     return launch_layer_tail(t, rows, status, st, 1);
   }
   rc = launch_linear_gemm(b.core, p.w_o, b.x1, vec(p.attn_scale), x, rows, 512, 512, value_fp16, p.stream_dtype, 0, status, st, 1);

@@ -6,7 +6,7 @@
 //
 // Latency-bound.  As three kernels (o_proj, LayerNorm + fc1 + GELU, fc2) each pays a launch (3.3 us on the host), a kernel boundary,
 // a first load and a reduction over the blocks that share K, for half a microsecond of products.  Here a cluster of 16 blocks
-// takes kRows rows through all of it: block r owns 32 channels of x1 and y and 128 of the MLP's hidden units, i.e. 288 KB of
+// takes up to 24 rows through all of it: block r owns 32 channels of x1 and y and 128 of the MLP's hidden units, i.e. 288 KB of
 // weights, all of it asked for before the wait for the kernel in front: W_o in registers, as the fragments that mma.sync wants (K is
 // permuted alike in both operands, so that a lane's share of 32 values of a row is one 16-byte load), W_1 by way of shared
 // memory in tensor memory (256 columns, the A operand of fc1), W_2 in shared memory where W_1 lay.  The rows cross the cluster
@@ -16,12 +16,12 @@
 // (hidden units would be 2048 x 2 bytes a row to every block, partial sums are 512 x 4).
 //
 // GPU time of eight FP32 layers, three kernels (for streams two: o_proj behind the attention) -> this one: a clip of 17 frames
-// 169 -> 102 us, 64 frames 170 -> 130, 112 frames 187 -> 146, 125 frames 190 -> 163, 168 frames 227 -> 173; 1 stream of one frame
-// 130 -> 96, 15 streams 160 -> 119, 64 streams of two frames 227 -> 200.  From the wait to the last block's end, us: 8 rows
-// 4.6 (x1 1.1, LayerNorm 0.75, fc1 with GELU 0.6, fc2 1.1, y 0.8), 16 rows 6.2, 24 rows 9: what grows is the two crossings, 2 KB a row into and
-// out of every block at 16 to 19 bytes a cycle.  fc1 and fc2 are tcgen05 products with weights as their 128 rows, 32 each, 19 cycles with
-// A in tensor memory and 51 with A in shared memory, whatever the columns; on mma.sync they took 16 cycles an instruction and
-// scheduler, 1024 per eight rows and product (8, 16, 24 rows: 4.9, 8, 12 us).
+// 169 -> 98 us, 64 frames 170 -> 130, 112 frames 187 -> 146, 125 frames 190 -> 161, 168 frames 227 -> 172; 64 streams of two frames 227 -> 200.
+// From the wait to the last block's end, us: 8 rows a cluster 4.4 (x1 1.1, LayerNorm 0.7, fc1 with GELU 0.6, fc2 1.1, y 0.7), 16 rows 6.2,
+// 24 rows 9: what grows is the two crossings, 2 KB a row into and out of every block at 16 to 19 bytes a cycle (one row instead of eight:
+// one stream 80 -> 72 us).  fc1 and fc2 are tcgen05 products with weights as their 128 rows, 32 each, 19 cycles with A in tensor memory and 51
+// with A in shared memory, whatever the columns; on mma.sync they took 16 cycles an instruction and scheduler, 1024 per eight rows and
+// product (8, 16, 24 rows: 4.9, 8, 12 us).
 #include <type_traits>
 
 #include "fm_common.cuh"
@@ -94,7 +94,8 @@ struct TailArgs {
   void* y;
   ParamVec attn_scale, mlp_scale, ln_weight, ln_bias;
   float eps;
-  int M, stream_type;
+  int M, rows;                           // rows of a cluster: at most kRows
+  int stream_type;
 };
 
 // VT: type of core and W_o; TOp: of the MLP's operands
@@ -104,7 +105,7 @@ layer_tail_kernel(const __grid_constant__ CUtensorMap tmap_w1, const __grid_cons
   using namespace tail;
   constexpr int kTiles = kRows / 8;                                            // columns of an mma.sync product: eight rows each
   constexpr int kElems = kRows / kGroup;                                       // of x1 and y, a thread of the first group
-  constexpr int kSlice = kRows * kCols * 4;                                    // bytes of a block's channels
+  constexpr int kSlice = kRows * kCols * 4;                                    // bytes of a block's channels, at most
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem_w = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_x = smem_w + kWBytes;
@@ -117,8 +118,9 @@ layer_tail_kernel(const __grid_constant__ CUtensorMap tmap_w1, const __grid_cons
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = static_cast<int>(threadIdx.x);
   const int g = lane >> 2, q = lane & 3;
   const int rank = static_cast<int>(cluster_cta_rank());
-  const int m0 = static_cast<int>(blockIdx.x) / kCtas * kRows;
-  const int n = a.M - m0 < kRows ? a.M - m0 : kRows;
+  const int m0 = static_cast<int>(blockIdx.x) / kCtas * a.rows;
+  const int n = a.M - m0 < a.rows ? a.M - m0 : a.rows;
+  const uint32_t slice = static_cast<uint32_t>(a.rows) * (kCols * 4);          // what a block sends another one
   // A status set before this chain began: nothing is stored.  The blocks of a cluster write into one another's memory and stay to the end.
   const bool skip = status != nullptr && *reinterpret_cast<volatile int*>(status) != 0;
   if (tid == 0) {
@@ -130,8 +132,8 @@ layer_tail_kernel(const __grid_constant__ CUtensorMap tmap_w1, const __grid_cons
     mbar_init(&c->fc_full[1], 1);
     ctl->abort = 0;
     fence_mbar_init();
-    mbar_arrive_expect_tx(&c->x1_full, (kCtas - 1) * kSlice);
-    mbar_arrive_expect_tx(&c->y_full, kCtas * kSlice);
+    mbar_arrive_expect_tx(&c->x1_full, (kCtas - 1) * slice);
+    mbar_arrive_expect_tx(&c->y_full, kCtas * slice);
     mbar_arrive_expect_tx(&c->w1_full, kWBytes);
 #pragma unroll
     for (int kc = 0; kc < kChunks; ++kc) tma_load_2d(smem_w + kc * kWBox, &tmap_w1, &c->w1_full, kc * 64, rank * kUnits);
@@ -199,6 +201,7 @@ layer_tail_kernel(const __grid_constant__ CUtensorMap tmap_w1, const __grid_cons
 #pragma unroll
     for (int i = 0; i < kElems; ++i) {
       const int row = (tid >> 5) + i * kGroup;
+      if (row >= a.rows) continue;
       float sum = 0.f;
 #pragma unroll
       for (int w = 0; w < kGroup; ++w) sum += red[(w * kRows + row) * kCols + swizzled(row, lane)];
@@ -213,7 +216,7 @@ layer_tail_kernel(const __grid_constant__ CUtensorMap tmap_w1, const __grid_cons
       for (int i = 0; i < kCtas / kGroup; ++i) {
         const int to = warp + i * kGroup;
         if (to == rank) mbar_arrive(&c->x1_full);
-        else copy_to_cta(smem_u32(x_out), smem_u32(x_out), kSlice, &c->x1_full, static_cast<uint32_t>(to));
+        else copy_to_cta(smem_u32(x_out), smem_u32(x_out), slice, &c->x1_full, static_cast<uint32_t>(to));
       }
     }
     __syncwarp();
@@ -262,7 +265,7 @@ layer_tail_kernel(const __grid_constant__ CUtensorMap tmap_w1, const __grid_cons
     float v[kMine][4][4], sum[kMine], sq[kMine];
 #pragma unroll
     for (int i = 0; i < kMine; ++i) {
-      const int row = warp + kWarps * i < kRows ? warp + kWarps * i : 0;
+      const int row = warp + kWarps * i < a.rows ? warp + kWarps * i : 0;
       sum[i] = 0.f;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {        // channels 128 j + 4 lane ..: block 4 j + lane / 8
@@ -297,7 +300,7 @@ layer_tail_kernel(const __grid_constant__ CUtensorMap tmap_w1, const __grid_cons
 #pragma unroll
     for (int i = 0; i < kMine; ++i) {
       const int row = warp + kWarps * i;
-      if (row < kRows) {
+      if (row < a.rows) {
         const float rstd = rsqrtf(sq[i] * (1.0f / kHidden) + a.eps);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -389,7 +392,7 @@ layer_tail_kernel(const __grid_constant__ CUtensorMap tmap_w1, const __grid_cons
   fence_proxy_async_smem();
   __syncwarp();
   cluster_wait();                          // no block reads x1 any more
-  if (lane == 0) copy_to_cta(smem_u32(stage), smem_u32(smem_x + rank * kSlice), kSlice, &c->y_full, static_cast<uint32_t>(warp));
+  if (lane == 0) copy_to_cta(smem_u32(stage), smem_u32(smem_x + rank * kSlice), slice, &c->y_full, static_cast<uint32_t>(warp));
   __syncwarp();
   mbar_wait_cluster(&c->y_full, 0, ctl, status, kErrWaitConsumer);
   __syncwarp();
@@ -448,30 +451,42 @@ int tail_clusters() {
   return n > 0 ? n : 0;
 }
 
-// Rows of a cluster for M rows in one wave: 8, 16 or 24, 0 where those are too few (7 clusters on a B200: 168 rows in all).  The
-// fewest that do: a row more costs every block its crossings, a cluster more nothing (56 streams 158 us at eight rows, 64 at
-// sixteen 177; without the kernel 206 and 211), though the last of seven often starts late.
-int rows_of_cluster(int M) {
-  const int clusters = tail_clusters();
-  for (int rows = 8; rows <= 24; rows += 8)
-    if (M <= rows * clusters) return rows;
-  return 0;
+// Rows of a cluster for M rows in one wave, 0 where 24 are too few (7 clusters on a B200: 168 rows in all).  Products are made for 8,
+// 16 or 24 rows: as few as the clusters that the device holds can do with.  Fewer rows than that cost every block less in its crossings, so
+// they are dealt evenly to five clusters at least: a sixth or seventh often finds no GPC with 16 free SMs until the kernel in front ends
+// (eight layers of a clip of 17 frames: 98 us on five, 102 on six, 107 on two; 40 streams 140 on five, 146 on six).  Where each block of the kernel in
+// front has an SM to itself (`beside` of them), to as many as the others hold, but three (12 streams beside 96 blocks 87 us on
+// three, 99 on four, 103 on one; 18 beside 144 109 on three, 111 on five, 142 on one).
+int rows_of_cluster(int M, int beside) {
+  const int held = tail_clusters();
+  int tile = 8;
+  while (tile < 24 && M > tile * held) tile += 8;
+  if (M > tile * held) return 0;
+  int clusters = held < 5 ? held : 5;
+  if (beside > 0) {
+    const int room = (sm_count() - beside) / tail::kCtas;
+    if (room < clusters) clusters = room < 3 ? 3 : room;
+  }
+  const int least = (M + tile - 1) / tile;
+  if (clusters < least) clusters = least;
+  return (M + clusters - 1) / clusters;
 }
 
 template <typename VT, typename TOp>
 int launch_rows(int rows, const CUtensorMap& tmap_w1, const CUtensorMap& tmap_w2, const TailArgs& a, int* status, cudaStream_t st, int dependent) {
   using namespace tail;
-  auto kern = rows == 8 ? layer_tail_kernel<VT, TOp, 8> : rows == 16 ? layer_tail_kernel<VT, TOp, 16> : layer_tail_kernel<VT, TOp, 24>;
+  const int tile = (rows + 7) / 8 * 8;
+  auto kern = tile == 8 ? layer_tail_kernel<VT, TOp, 8> : tile == 16 ? layer_tail_kernel<VT, TOp, 16> : layer_tail_kernel<VT, TOp, 24>;
   const int fmt = std::is_same<TOp, __half>::value ? 0 : 1;
-  const uint32_t idesc = umma_idesc_f16(128, rows <= 16 ? 16 : 32, fmt, fmt, 0, 0);
-  return launch_kernel(kern, dim3(kCtas * ((a.M + rows - 1) / rows)), kThreads, smem_bytes(rows), st, kCtas, dependent, tmap_w1, tmap_w2, a, idesc, status);
+  const uint32_t idesc = umma_idesc_f16(128, tile <= 16 ? 16 : 32, fmt, fmt, 0, 0);
+  return launch_kernel(kern, dim3(kCtas * ((a.M + rows - 1) / rows)), kThreads, smem_bytes(tile), st, kCtas, dependent, tmap_w1, tmap_w2, a, idesc, status);
 }
 }  // namespace
 
-bool layer_tail_takes(int M, int ffn) { return ffn == tail::kFfn && M > 0 && rows_of_cluster(M) > 0; }
+bool layer_tail_takes(int M, int ffn) { return ffn == tail::kFfn && M > 0 && rows_of_cluster(M, 0) > 0; }
 
 int launch_layer_tail(const LayerTail& t, int M, int* status, cudaStream_t st, int dependent) {
-  const int rows = M > 0 ? rows_of_cluster(M) : 0;
+  const int rows = M > 0 ? rows_of_cluster(M, t.beside) : 0;
   if (rows == 0 || t.stream_type < 0 || t.stream_type > 2) return -1;
   if ((reinterpret_cast<uintptr_t>(t.core) | reinterpret_cast<uintptr_t>(t.x) | reinterpret_cast<uintptr_t>(t.y) |
        reinterpret_cast<uintptr_t>(t.w_o) | reinterpret_cast<uintptr_t>(t.w_fc1) | reinterpret_cast<uintptr_t>(t.w_fc2) |
@@ -483,7 +498,7 @@ int launch_layer_tail(const LayerTail& t, int M, int* status, cudaStream_t st, i
   if (rc == 0) rc = encode_rows_16bit(&tmap_w2, t.w_fc2, tail::kHidden, tail::kFfn, 128, 64);
   if (rc != 0) return rc;
   const TailArgs a = {static_cast<const uint16_t*>(t.core), static_cast<const uint16_t*>(t.w_o), t.x, t.y,
-                      t.attn_scale, t.mlp_scale, t.ln_weight, t.ln_bias, t.eps, M, t.stream_type};
+                      t.attn_scale, t.mlp_scale, t.ln_weight, t.ln_bias, t.eps, M, rows, t.stream_type};
   if (t.value_fp16)
     return t.tc_fp16 ? launch_rows<__half, __half>(rows, tmap_w1, tmap_w2, a, status, st, dependent)
                      : launch_rows<__half, __nv_bfloat16>(rows, tmap_w1, tmap_w2, a, status, st, dependent);
