@@ -2,17 +2,21 @@
 // LayerNorm(x) W^T with 512 channels.  Reference: src/fast_mimi/model.py:2021-2024 with :1897-1912 and :1990-1999.
 //
 // Latency-bound: at one clip's rows a LayerNorm launch (1.5 us of memory round trip and reductions) and the product
-// behind it (2.5 us) each pay a kernel boundary.  Here a block owns `kRows` rows (16 or 32) x 64 outputs (one head):
-// its eight epilogue warps normalise the rows, one warp per row at a time, straight into the swizzled operand tile, and
-// the whole K = 512 of its weight slice (64 KB) sits in shared memory, requested before the wait for the kernel in front.
-// There is no K split, hence no cluster and no reduction.  Every block repeats the normalisation of its rows (32 or 64 KB
-// of x from L2), which is what limits the rows.
+// behind it (2.5 us) each pay a kernel boundary.  Here a block owns `kRows` rows (16, 32 or 64) x 128 outputs (two heads).  Its sixteen
+// warps bring the whole K = 512 of its weight slice (128 KB) by way of shared memory into tensor memory, where it is the A operand (256
+// columns), ahead of the wait for the kernel in front; then they normalise the rows, up to four a warp, straight into the swizzled other
+// operand.  There is no K split, hence no cluster and no reduction.  Every block repeats the normalisation of its rows (2 KB of x a row from
+// L2), which is what limits the rows.
 //
-// The tensor core multiplies 128 rows whatever kRows is; the operand tile of a K chunk is only kRows rows high, so what
-// it reads past them is the next chunk (or the weights): finite or not, those products stay in accumulator rows that
-// nobody reads.
+// With weights as the 128 rows of the product and in tensor memory an instruction takes 19 cycles for 16 columns and 32 for 64; with
+// rows as its rows, both operands in shared memory and waits between them, it took 75.  GPU time of eight layers, from the kernel that
+// did that (16 or 32 rows x 64 outputs, to 160 rows; beyond, a LayerNorm kernel and fm_linear_small.cu) to this one, us: clip of 17 frames 98 -> 92, 125 frames
+// 160 -> 158, two clips of 125 252 -> 217, four 290 -> 258, six 329 -> 310; 190 streams of one frame 347 -> 312, 384 519 -> 476; five of 50 frames 290 -> 252.
+// Tried: several row tiles one after another in a block, for more rows: 250 rows 217 -> 238, 1000 rows in two turns 331 -> 387.
 //
-// Warps 0-7: LayerNorm, then accumulator and epilogue.  Warp 8: weights.  Warp 9: MMA.
+// Warps 0-15: weights, LayerNorm, accumulator and epilogue.  Warp 0 also issues the products.
+#include <type_traits>
+
 #include "fm_launch.h"
 #include "fm_small_tile.cuh"
 
@@ -20,21 +24,20 @@ namespace fm {
 
 namespace lnlin {
 constexpr int kHidden = 512;
-constexpr int kBlockN = 64;
+constexpr int kBlockN = 128;
 constexpr int kChunks = kHidden / 64;
-constexpr int kWBytes = kBlockN * 128;          // one K chunk of the weight slice
-constexpr int kWarps = 8;
-constexpr int kThreads = (kWarps + 2) * 32;
-constexpr int kTmemCols = 64;
+constexpr int kWBox = kBlockN * 128, kWBytes = kChunks * kWBox;      // 64 of K; the weight slice
+constexpr int kWarps = 16, kThreads = kWarps * 32;
+constexpr int kTmemCols = 512, kTmemD = kHidden / 2;                 // weights | accumulator
 struct Barriers {
-  uint64_t w_full[2];                           // the two halves of the weight slice
+  uint64_t w_full;
   uint64_t acc_full;
   uint32_t tmem_base;
   CtaCtl ctl;
 };
-// The operand tile comes first: the tensor core reads up to 128 - kRows rows past its last chunk, i.e. into the weights.
-constexpr int smem_bytes(int rows) { return 1024 + kChunks * (rows * 128 + kWBytes) + rows * 256 + 64; }
-static_assert(sizeof(Barriers) <= 64, "barrier block too large");
+// Weights, later the results in FP32 | LayerNorm's result
+constexpr int smem_bytes(int rows) { return 1024 + kWBytes + kChunks * rows * 128 + static_cast<int>(sizeof(Barriers)); }
+static_assert(smem_bytes(64) <= 232448, "exceeds the 227 KB a block may use");
 }  // namespace lnlin
 
 struct LnArgs {
@@ -42,84 +45,112 @@ struct LnArgs {
   ParamVec weight;
   ParamVec bias;
   float eps;
+  int x_type;             // 0 BF16, 1 FP16, 2 FP32
   int opens_chain;        // first kernel of a chain: lets the next one start only after its own wait
 };
 
-// kIn: type of x (0 BF16, 1 FP16, 2 FP32); kTc: type of the product's operands (0 BF16, 1 FP16); kOut: kTc, or 3 = q | k | v
-template <int kIn, int kTc, int kOut, typename VT, int kRows>
-__global__ void __launch_bounds__(lnlin::kThreads)
+// kTc: type of the product's operands (0 BF16, 1 FP16); kOut: kTc, or 3 = q | k | v
+template <int kTc, int kOut, typename VT, int kRows>
+__global__ void __launch_bounds__(lnlin::kThreads, 1)
 ln_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ LnArgs ln,
                  const __grid_constant__ SmallArgs args, uint32_t idesc, int* status) {
   using namespace lnlin;
   using TOp = typename std::conditional<kTc == 1, __half, __nv_bfloat16>::type;
+  constexpr int kMine = kRows / kWarps;                  // rows of a warp
+  constexpr int kItems = (kRows * 16 + kThreads - 1) / kThreads;       // pieces of eight results of a thread
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem_h = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* smem_w = smem_h + kChunks * kRows * 128;
-  uint8_t* smem_o = smem_w + kChunks * kWBytes;
-  Barriers* bars = reinterpret_cast<Barriers*>(smem_o + kRows * 256);
+  uint8_t* smem_w = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem_h = smem_w + kWBytes;
+  float* smem_o = reinterpret_cast<float*>(smem_w);
+  Barriers* bars = reinterpret_cast<Barriers*>(smem_h + kChunks * kRows * 128);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ntile = static_cast<int>(blockIdx.x);
+  const int n0 = static_cast<int>(blockIdx.x) * kBlockN;
   const int m0 = static_cast<int>(blockIdx.y) * kRows;
   // read early: a status set before this chain began stops every kernel of it (the stores are left out)
   const bool skip = status != nullptr && *reinterpret_cast<volatile int*>(status) != 0;
   if (threadIdx.x == 0) {
-    mbar_init(&bars->w_full[0], 1);
-    mbar_init(&bars->w_full[1], 1);
+    mbar_init(&bars->w_full, 1);
     mbar_init(&bars->acc_full, 1);
     bars->ctl.abort = 0;
     fence_mbar_init();
+    mbar_arrive_expect_tx(&bars->w_full, kWBytes);
+#pragma unroll
+    for (int kc = 0; kc < kChunks; ++kc) tma_load_2d(smem_w + kc * kWBox, &tmap_w, &bars->w_full, kc * 64, n0);
   }
-  if (warp == kWarps + 1) {
+  if (warp == 1) {
     tmem_alloc(&bars->tmem_base, kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = bars->tmem_base;
-  CtaCtl* ctl = &bars->ctl;
-
-  if (warp == kWarps && lane == 0) {
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      mbar_arrive_expect_tx(&bars->w_full[half], kChunks / 2 * kWBytes);
-#pragma unroll
-      for (int kc = half * kChunks / 2; kc < (half + 1) * kChunks / 2; ++kc)
-        tma_load_2d(smem_w + kc * kWBytes, &tmap_w, &bars->w_full[half], kc * 64, ntile * kBlockN);
-    }
-  }
   if (!ln.opens_chain) griddep_launch();
-  PieceOperands ops;
+  const uint32_t tmem_base = bars->tmem_base, t_row = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+  CtaCtl* ctl = &bars->ctl;
   const int n_rows = args.M - m0 < kRows ? args.M - m0 : kRows;
-  const int n_items = skip ? 0 : n_rows * 8;
-  int item = static_cast<int>(threadIdx.x);
-  if (warp < kWarps) {
-    // this lane's channels: 4 * lane + 128 * j + (0..3)
+
+  // Weights: output 32 (warp % 4) + lane, two values of K a column
+  mbar_wait(&bars->w_full, 0, ctl, status, kErrWaitTma);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int kc = 2 * (warp >> 2) + i;
+    uint32_t r[32];
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+      const uint4 v = *reinterpret_cast<const uint4*>(smem_w + kc * kWBox + sw128_offset((warp & 3) * 32 + lane, p));
+      r[4 * p] = v.x; r[4 * p + 1] = v.y; r[4 * p + 2] = v.z; r[4 * p + 3] = v.w;
+    }
+    tmem_st32(t_row + kc * 32, r);
+  }
+  tmem_st_wait();
+  tc_fence_before_sync();                  // the products follow behind a barrier of the block
+  griddep_wait();
+  if (ln.opens_chain) griddep_launch();
+
+  // ---- LayerNorm.  This lane's channels: 4 * lane + 128 * j + (0..3)
+  {
+    float v[kMine][4][4];
     uint4 w_raw[4], b_raw[4];
-    griddep_wait();
-    if (ln.opens_chain) griddep_launch();
-    float v[kRows / kWarps][4][4];
+    auto params = [&](auto f32) {
 #pragma unroll
-    for (int i = 0; i < kRows / kWarps; ++i) {
-      const int r = i * kWarps + warp;
-      if (r < n_rows) {
+      for (int j = 0; j < 4; ++j) {
+        w_raw[j] = ln.weight.raw4<decltype(f32)::value>(128 * j + 4 * lane);
+        b_raw[j] = ln.bias.raw4<decltype(f32)::value>(128 * j + 4 * lane);
+      }
+    };
+    if (ln.x_type == 2) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) load4<kIn>(ln.x, static_cast<long long>(m0 + r) * kHidden + 128 * j + 4 * lane, v[i][j]);
-      } else {
+      for (int i = 0; i < kMine; ++i) {
+        const int r = i * kWarps + warp < n_rows ? i * kWarps + warp : 0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[i][j][0] = v[i][j][1] = v[i][j][2] = v[i][j][3] = 0.f;
+        for (int j = 0; j < 4; ++j) load4<2>(ln.x, static_cast<long long>(m0 + r) * kHidden + 128 * j + 4 * lane, v[i][j]);
+      }
+      params(std::true_type());
+    } else {
+      uint2 u[kMine][4];
+#pragma unroll
+      for (int i = 0; i < kMine; ++i) {
+        const int r = i * kWarps + warp < n_rows ? i * kWarps + warp : 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          u[i][j] = __ldcg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(ln.x) + static_cast<long long>(m0 + r) * kHidden + 128 * j + 4 * lane));
+      }
+      params(std::false_type());
+#pragma unroll
+      for (int i = 0; i < kMine; ++i) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 lo = ln.x_type == 1 ? Pack16<__half>::unpack(u[i][j].x) : Pack16<__nv_bfloat16>::unpack(u[i][j].x);
+          const float2 hi = ln.x_type == 1 ? Pack16<__half>::unpack(u[i][j].y) : Pack16<__nv_bfloat16>::unpack(u[i][j].y);
+          v[i][j][0] = lo.x; v[i][j][1] = lo.y; v[i][j][2] = hi.x; v[i][j][3] = hi.y;
+        }
       }
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      w_raw[j] = ln.weight.raw4<kIn == 2>(128 * j + 4 * lane);
-      b_raw[j] = ln.bias.raw4<kIn == 2>(128 * j + 4 * lane);
-    }
-    if (item < n_items) load_operands<kOut>(args, m0 + (item >> 3), ntile, item & 7, ops);
     // the same sums in the same order as layernorm512_kernel
-    float sum[kRows / kWarps], sq[kRows / kWarps];
+    float sum[kMine], sq[kMine];
 #pragma unroll
-    for (int i = 0; i < kRows / kWarps; ++i) {
+    for (int i = 0; i < kMine; ++i) {
       sum[i] = 0.f;
 #pragma unroll
       for (int j = 0; j < 4; ++j) sum[i] += (v[i][j][0] + v[i][j][1]) + (v[i][j][2] + v[i][j][3]);
@@ -127,10 +158,10 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
-      for (int i = 0; i < kRows / kWarps; ++i) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
+      for (int i = 0; i < kMine; ++i) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
     }
 #pragma unroll
-    for (int i = 0; i < kRows / kWarps; ++i) {
+    for (int i = 0; i < kMine; ++i) {
       const float mean = sum[i] * (1.0f / kHidden);
       sq[i] = 0.f;
 #pragma unroll
@@ -145,18 +176,18 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
-      for (int i = 0; i < kRows / kWarps; ++i) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], o);
+      for (int i = 0; i < kMine; ++i) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], o);
     }
     float w[4][4], b[4][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float4 wf = ln.weight.value4<kIn == 2>(w_raw[j]);
-      const float4 bf = ln.bias.value4<kIn == 2>(b_raw[j]);
+      const float4 wf = ln.x_type == 2 ? ln.weight.value4<true>(w_raw[j]) : ln.weight.value4(w_raw[j]);
+      const float4 bf = ln.x_type == 2 ? ln.bias.value4<true>(b_raw[j]) : ln.bias.value4(b_raw[j]);
       w[j][0] = wf.x; w[j][1] = wf.y; w[j][2] = wf.z; w[j][3] = wf.w;
       b[j][0] = bf.x; b[j][1] = bf.y; b[j][2] = bf.z; b[j][3] = bf.w;
     }
 #pragma unroll
-    for (int i = 0; i < kRows / kWarps; ++i) {
+    for (int i = 0; i < kMine; ++i) {
       const int r = i * kWarps + warp;
       const float rstd = rsqrtf(sq[i] * (1.0f / kHidden) + ln.eps);
 #pragma unroll
@@ -171,85 +202,84 @@ ln_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
     fence_proxy_async_smem();
   }
-  __syncthreads();                          // the operand tile is complete
-  if (warp == kWarps + 1) {
-    const bool one = elect_one();
+  __syncthreads();                         // the operand is complete, and the weights are in tensor memory
+
+  if (warp == 0) {
     tc_fence_after_sync();
-    const uint64_t a_desc = umma_desc_sw128(smem_u32(smem_h)), b_desc = umma_desc_sw128(smem_u32(smem_w));
+    const uint64_t h = umma_desc_sw128(smem_u32(smem_h));
+    const bool one = elect_one();
     for (int kc = 0; kc < kChunks; ++kc) {
-      if (kc % (kChunks / 2) == 0) {
-        mbar_wait(&bars->w_full[kc / (kChunks / 2)], 0, ctl, status, kErrWaitTma);
-        tc_fence_after_sync();
-      }
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks)
         if (one)
-          tc_mma_ss(tmem_base, a_desc + static_cast<uint64_t>(kc * kRows * 128 >> 4) + 2u * ks,
-                    b_desc + static_cast<uint64_t>(kc * kWBytes >> 4) + 2u * ks, idesc, (kc | ks) != 0 ? 1u : 0u);
+          tc_mma_ts(tmem_base + kTmemD, tmem_base + kc * 32 + ks * 8, h + static_cast<uint64_t>(kc * kRows * 128 >> 4) + 2u * ks, idesc,
+                    (kc | ks) != 0 ? 1u : 0u);
     }
     if (one) tc_commit(&bars->acc_full);
     __syncwarp();
   }
-  if (warp == 0) {
-    // rows 0 .. kRows - 1 sit in the first 32 lanes of tensor memory
-    mbar_wait(&bars->acc_full, 0, ctl, status, kErrWaitMma);
-    tc_fence_after_sync();
+  // item: row item / 16 of the block, head (item / 8) % 2, piece item % 8
+  const int n_items = skip ? 0 : n_rows * 16;
+  PieceOperands ops[kItems];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      uint32_t a[32];
-      tmem_ld32(tmem_base + h * 32, a);
-      tmem_ld_wait();
-      if (lane < kRows) {
+  for (int i = 0; i < kItems; ++i) {
+    const int item = static_cast<int>(threadIdx.x) + i * kThreads;
+    if (item < n_items) load_operands<kOut>(args, m0 + (item >> 4), 2 * static_cast<int>(blockIdx.x) + ((item >> 3) & 1), item & 7, ops[i]);
+  }
+  mbar_wait(&bars->acc_full, 0, ctl, status, kErrWaitMma);
+  __syncwarp();
+  tc_fence_after_sync();
+  {
+    // output 32 (warp % 4) + lane, a quarter of the rows a warp
+    constexpr int kN = kRows / 4;
+    uint32_t u[kN];
+    if constexpr (kN == 4) tmem_ld4(t_row + kTmemD + (warp >> 2) * kN, u);
+    else if constexpr (kN == 8) tmem_ld8(t_row + kTmemD + (warp >> 2) * kN, u);
+    else tmem_ld16(t_row + kTmemD + (warp >> 2) * kN, u);
+    tmem_ld_wait();
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
-          *reinterpret_cast<uint4*>(smem_o + small::red_offset(lane, h * 8 + c, lane)) =
-              make_uint4(a[4 * c], a[4 * c + 1], a[4 * c + 2], a[4 * c + 3]);
-      }
-    }
+    for (int i = 0; i < kN; ++i) smem_o[((warp >> 2) * kN + i) * kBlockN + (warp & 3) * 32 + lane] = __uint_as_float(u[i]);
     tc_fence_before_sync();
   }
   __syncthreads();
-  if (warp < kWarps && item < n_items) {    // kRows * 8 pieces, one per thread at most
-    const int local = item >> 3, j = item & 7;
-    const float4 a = *reinterpret_cast<const float4*>(smem_o + small::red_offset(local, j, local));
-    const float4 c = *reinterpret_cast<const float4*>(smem_o + small::red_offset(local, j + 8, local));
-    float lo[4] = {a.x, a.y, a.z, a.w}, hi[4] = {c.x, c.y, c.z, c.w};
-    finish_piece<kOut, VT>(args, lo, hi, ops, m0 + local, ntile, j, status);
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const int item = static_cast<int>(threadIdx.x) + i * kThreads;
+    if (item < n_items) {
+      const int local = item >> 4, sub = (item >> 3) & 1, j = item & 7;
+      const float* row = smem_o + local * kBlockN + sub * 64 + 4 * j;
+      const float4 a = *reinterpret_cast<const float4*>(row), c = *reinterpret_cast<const float4*>(row + 32);
+      float lo[4] = {a.x, a.y, a.z, a.w}, hi[4] = {c.x, c.y, c.z, c.w};
+      finish_piece<kOut, VT>(args, lo, hi, ops[i], m0 + local, 2 * static_cast<int>(blockIdx.x) + sub, j, status);
+    }
   }
   if (ctl->abort) __nanosleep(20000);
-  if (warp == kWarps + 1) {
+  if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);
   }
 }
 
 static long long blocks_for(int M, int N, int rows) { return static_cast<long long>((M + rows - 1) / rows) * (N / lnlin::kBlockN); }
-// 16 rows per block while that is at most one block per SM, else 32; beyond one block per SM of those the separate
-// LayerNorm kernel is cheaper.  More blocks than SMs do not pay: two of them leave no room on an SM for the next kernel's
-// block, which then starts (and asks for its weights) only when they have ended (125 rows: fc2 began 5 us after fc1's
-// first blocks were done instead of 2).
-static int rows_per_block(int M, int N) { return blocks_for(M, N, 16) <= sm_count() ? 16 : 32; }
+// As few rows as leave half of the SMs to the kernels in front and behind, whose blocks then bring their weights while this one runs; 64 up to
+// a block per SM (768 rows of q | k | v, 576 of an MLP of 2048).  Beyond that the separate kernels are faster (see above).
+static int rows_per_block(int M, int N) {
+  int rows = 16;
+  while (rows < 64 && 2 * blocks_for(M, N, rows) > sm_count()) rows *= 2;
+  return rows;
+}
 
-bool few_rows_with_norm(int M, int N) { return blocks_for(M, N, 32) <= sm_count(); }
+bool few_rows_with_norm(int M, int N) { return N % lnlin::kBlockN == 0 && blocks_for(M, N, 64) <= sm_count(); }
 
-template <int kIn, int kTc, int kOut, typename VT>
-static int launch_rows(const CUtensorMap& tmap_w, const LnArgs& ln, const SmallArgs& args, uint32_t idesc, int* status,
-                       cudaStream_t st, int dependent) {
+template <int kTc, int kOut, typename VT>
+static int launch_rows(const CUtensorMap& tmap_w, const LnArgs& ln, const SmallArgs& args, int* status, cudaStream_t st, int dependent) {
   using namespace lnlin;
-  const int rows = rows_per_block(args.M, args.N);
-  auto kern = rows == 16 ? ln_linear_kernel<kIn, kTc, kOut, VT, 16> : ln_linear_kernel<kIn, kTc, kOut, VT, 32>;
+  const int rows = rows_per_block(args.M, args.N), fmt = kTc == 1 ? 0 : 1;
+  auto kern = rows == 16 ? ln_linear_kernel<kTc, kOut, VT, 16> : rows == 32 ? ln_linear_kernel<kTc, kOut, VT, 32> : ln_linear_kernel<kTc, kOut, VT, 64>;
   const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes(rows));
   if (rc != 0) return rc;
   return launch_kernel(kern, dim3(args.N / kBlockN, (args.M + rows - 1) / rows), kThreads, smem_bytes(rows), st, 1, dependent,
-                       tmap_w, ln, args, idesc, status);
-}
-
-template <int kIn, int kTc>
-static int launch_typed(const CUtensorMap& tmap_w, const LnArgs& ln, const SmallArgs& args, uint32_t idesc, int qkv, int value_fp16,
-                        int* status, cudaStream_t st, int dependent) {
-  if (!qkv) return launch_rows<kIn, kTc, kTc, __half>(tmap_w, ln, args, idesc, status, st, dependent);
-  if (value_fp16) return launch_rows<kIn, kTc, 3, __half>(tmap_w, ln, args, idesc, status, st, dependent);
-  return launch_rows<kIn, kTc, 3, __nv_bfloat16>(tmap_w, ln, args, idesc, status, st, dependent);
+                       tmap_w, ln, args, umma_idesc_f16(128, rows, fmt, fmt, 0, 0), status);
 }
 
 static int launch_ln(const void* x, int x_dtype, ParamVec weight, ParamVec bias, float eps, const void* w,
@@ -262,13 +292,15 @@ static int launch_ln(const void* x, int x_dtype, ParamVec weight, ParamVec bias,
   CUtensorMap tmap_w;
   const int rc = encode_rows_16bit(&tmap_w, w, static_cast<uint64_t>(args.N), lnlin::kHidden, lnlin::kBlockN, 64);
   if (rc != 0) return rc;
-  const LnArgs ln = {x, weight, bias, eps, opens_chain};
-  const int fmt = tc_fp16 ? 0 : 1;
-  const uint32_t idesc = umma_idesc_f16(128, lnlin::kBlockN, fmt, fmt, 0, 0);
-  using Fn = int (*)(const CUtensorMap&, const LnArgs&, const SmallArgs&, uint32_t, int, int, int*, cudaStream_t, int);
-  static const Fn table[3][2] = {{launch_typed<0, 0>, launch_typed<0, 1>}, {launch_typed<1, 0>, launch_typed<1, 1>},
-                                 {launch_typed<2, 0>, launch_typed<2, 1>}};
-  return table[x_dtype][tc_fp16 ? 1 : 0](tmap_w, ln, args, idesc, qkv, value_fp16, status, st, dependent);
+  const LnArgs ln = {x, weight, bias, eps, x_dtype, opens_chain};
+  if (tc_fp16) {
+    if (!qkv) return launch_rows<1, 1, __half>(tmap_w, ln, args, status, st, dependent);
+    return value_fp16 ? launch_rows<1, 3, __half>(tmap_w, ln, args, status, st, dependent)
+                      : launch_rows<1, 3, __nv_bfloat16>(tmap_w, ln, args, status, st, dependent);
+  }
+  if (!qkv) return launch_rows<0, 0, __half>(tmap_w, ln, args, status, st, dependent);
+  return value_fp16 ? launch_rows<0, 3, __half>(tmap_w, ln, args, status, st, dependent)
+                    : launch_rows<0, 3, __nv_bfloat16>(tmap_w, ln, args, status, st, dependent);
 }
 
 int launch_ln_qkv(const void* x, int x_dtype, ParamVec weight, ParamVec bias, float eps, const void* w_qkv,

@@ -266,14 +266,15 @@ def test_first_half_of_a_call_for_few_streams(streams, T, past, dtype, value_dty
     fm.check_status()
 
 
-# rows: one, either side of a cluster's rows (8) and of what seven clusters of 8, 16 and 24 rows hold; two clips; an MLP of another size, for
-# which there is no such kernel
+# rows: one, either side of a cluster's rows (8) and of what seven clusters of 8, 16 and 24 rows hold; of where LayerNorm's products go from 16 to 32
+# and 64 rows a block (96, 192), and of the last that have LayerNorm inside (576 and 768); an MLP of another size, for which fewer kernels are there
 @pytest.mark.parametrize("B,T,ffn", [(1, 1, 2048), (1, 8, 2048), (1, 9, 2048), (1, 56, 2048), (1, 57, 2048), (1, 112, 2048), (1, 113, 2048), (2, 61, 2048),
-                                     (1, 168, 2048), (1, 169, 2048), (1, 9, 1024)])
+                                     (1, 96, 2048), (1, 97, 2048), (1, 168, 2048), (1, 169, 2048), (1, 193, 2048), (3, 192, 2048), (1, 577, 2048),
+                                     (3, 256, 2048), (1, 769, 2048), (1, 9, 1024)])
 @pytest.mark.parametrize("dtype,value_dtype", [(torch.float32, torch.float16), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16),
                                                (torch.bfloat16, torch.float16), (torch.float16, torch.float16)])
 def test_layer_on_few_rows_against_64_bits(B, T, ffn, dtype, value_dtype):
-    """A layer on clips of few rows in all, where everything behind the attention is one kernel, against the same in 64 bits; bars as for
+    """A layer on clips of few rows in all, against the same in 64 bits; bars as for
     live streams below (BF16 values: their rounding, 2^-9, in front of the output projection)."""
     import fast_mimi_b200 as fm
     layer = fm.MimiTransformerLayerB200(intermediate_size=ffn, value_dtype=value_dtype).cuda()
@@ -290,7 +291,8 @@ def test_layer_on_few_rows_against_64_bits(B, T, ffn, dtype, value_dtype):
     norm = lambda t, name: torch.nn.functional.layer_norm(t, (512,), p[name + ".weight"], p[name + ".bias"], 1e-5)
     q, k, v = ((norm(xd, "input_layernorm") @ p[f"self_attn.{n}_proj.weight"].T).view(B, T, 8, 64).transpose(1, 2) for n in "qkv")
     turn = lambda t: t * cos.double()[:, None] + O.rotate_half(t) * sin.double()[:, None]
-    hidden = torch.ones(T, T, dtype=torch.bool, device="cuda").triu(1)
+    ones = torch.ones(T, T, dtype=torch.bool, device="cuda")
+    hidden = ones.triu(1) | ones.tril(-250)
     core = torch.softmax((turn(q) @ turn(k).transpose(-1, -2) * 0.125).masked_fill(hidden, float("-inf")), -1) @ v
     x1 = xd + core.transpose(1, 2).reshape(B, T, 512) @ p["self_attn.o_proj.weight"].T * p["self_attn_layer_scale.scale"]
     want = x1 + torch.nn.functional.gelu(norm(x1, "post_attention_layernorm") @ p["mlp.fc1.weight"].T) @ p["mlp.fc2.weight"].T * p["mlp_layer_scale.scale"]
