@@ -517,6 +517,7 @@ static bool half_units(int pair_tiles, int N, int max_pairs, int k_chunks) {
   return static_cast<long long>(64 + k_chunks) * waves128 < 128ll * waves256;
 }
 
+// (What fm_linear_ws.cu takes comes first; the figures are for the other kernels alone.)
 // Half units that are one wave, for rows that two of the few-row kernel's 128 x 64 blocks on an SM would hold: those fetch half as much
 // again from L2, and the second starts when the first has gone.  With one of them to an SM they are the faster form.  Measured, few-row
 // kernel -> half units, in us: K = 2048, N = 512, FP32 2000 rows (128 blocks) 12.4 -> 13.9, 2500 (160) 13.9 -> 13.9, 3678 (232) 15.7 ->
@@ -548,6 +549,7 @@ int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, co
   if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y) |
        reinterpret_cast<uintptr_t>(scale.data) | reinterpret_cast<uintptr_t>(resid)) & 15u)
     return -3;
+  if (out_dtype != 3 && linear_ws_takes(M, N, K, dependent)) return launch_linear_ws(a, w, y, scale, resid, M, N, K, in_dtype, out_dtype, gelu, status, st, dependent);
   const int pair_tiles = ((M + kBlockM - 1) / kBlockM + 1) / 2;
   const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
   const bool one_wave = out_dtype != 3 && one_wave_of_halves(M, pair_tiles, N, max_pairs, out_dtype == 2, gelu != 0, dependent);

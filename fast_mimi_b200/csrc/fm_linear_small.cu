@@ -1,6 +1,8 @@
 // Linear layers and the QKV projection for few rows (sm_100a): y = residual + scale * act(a W^T), or q | k | v with
 // RoPE, for calls whose rows fill only a few 128-row tiles (one clip, one frame of up to a few hundred streams).
 //
+// (Linear layers of fewer rows, whose weights fit the chip's tensor memory, take fm_linear_ws.cu.)
+//
 // What bounds such a call is latency and the number of SMs that pull weights out of L2, not arithmetic: the pair
 // kernels (fm_linear_gemm.cu, fm_qkv_gemm.cu) cut the output into 256 x 256 tiles, so that 125 rows x 512 outputs at
 // K = 2048 occupied 4 of 148 SMs, each walking 32 K-chunks one after the other (with an FP32 residual 20.8 us; here 6.8 us).  Here a block owns

@@ -33,6 +33,33 @@ def test_linear_with_few_rows(rows, shape):
     fm.check_status()
 
 
+# K shared out over one, two, four and eight blocks; rows at the edges of tiles of 16, 32 and 64 and of what the kernel takes
+@pytest.mark.parametrize("rows,K,N", [(16, 512, 256), (17, 512, 512), (593, 512, 512), (1184, 512, 512), (1185, 512, 512), (2368, 512, 512), (2369, 512, 512),
+                                      (33, 1024, 1024), (500, 1024, 512), (31, 2048, 512), (33, 2048, 512), (257, 2048, 512), (512, 2048, 512),
+                                      (513, 2048, 512), (15, 4096, 512), (65, 4096, 256), (130, 4096, 512), (576, 512, 2048), (577, 512, 2048)])
+@pytest.mark.parametrize("in_dtype", [torch.float16, torch.bfloat16])
+def test_linear_with_resident_weights(rows, K, N, in_dtype):
+    """Products whose weights lie in tensor memory, against 64 bits: FP32 results to 2e-7 (partial sums of at most 128 products, 2^-24 each, and their
+    sums), 16-bit ones to their rounding; nothing behind the last row is written."""
+    import fast_mimi_b200 as fm
+    g = torch.Generator(device="cuda").manual_seed(rows + K)
+    a = torch.randn(rows, K, device="cuda", generator=g).to(in_dtype)
+    w = (torch.randn(N, K, device="cuda", generator=g) / K ** 0.5).to(in_dtype)
+    s = torch.rand(N, device="cuda", generator=g) + 0.2
+    acc = a.double() @ w.double().T
+    for out_dtype in (torch.float32, torch.float16, torch.bfloat16):
+        r = torch.randn(rows, N, device="cuda", generator=g).to(out_dtype)
+        held = torch.full((rows + 1, N), 7.0, dtype=out_dtype, device="cuda")
+        fm.ops.linear(a, w, scale=s, residual=r, out_dtype=out_dtype, out=held[:rows])
+        taken = K == 512 and (rows <= 2368 and N <= 512 or rows <= 576) or K > 512 and rows <= 512
+        bar = {torch.float32: 2e-7 if taken else 2e-6, torch.float16: 5e-4, torch.bfloat16: 4e-3}[out_dtype]
+        assert O.rel_l2(held[:rows].double(), r.double() + s * acc) < bar
+        assert (held[rows] == 7.0).all()
+        got = fm.ops.linear(a, w, activation="gelu", out_dtype=out_dtype)
+        assert O.rel_l2(got.double(), torch.nn.functional.gelu(acc)) < max(bar, 2e-6)
+    fm.check_status()
+
+
 @pytest.mark.parametrize("B,T", [(1, 1), (1, 127), (3, 43), (2, 128), (5, 100)])
 def test_projection_with_few_rows(B, T):
     import fast_mimi_b200 as fm
