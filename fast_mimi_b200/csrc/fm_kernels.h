@@ -263,7 +263,7 @@ struct StreamFront {
 bool stream_front_takes(int S, int T, int slots);
 int launch_stream_front(const StreamFront& f, int S, int T, int past, int slots, int window, float scale, int* status, cudaStream_t st, int dependent);
 // Attention for few query tiles (fm_few_attn.cu): at most two 64-query blocks per SM.  ring_k null: clips; else T new frames
-// per stream on top of the ring, which the kernel also updates where one block has a whole (stream, head).
+// per stream on top of the ring, which the kernel also updates with up to 64 of them.
 bool few_attn_tiles(int S, int T);
 bool few_attn_updates_ring(int T);
 int launch_few_attn(const void* q, const void* k, const void* v, void* ring_k, void* ring_v, void* out, int S, int T, int past,

@@ -263,6 +263,32 @@ def test_live_streams_against_64_bits(T, past, dtype, value_dtype):
     fm.check_status()
 
 
+@pytest.mark.parametrize("past", [0, 20, 249, 400])
+@pytest.mark.parametrize("T", [9, 32, 33, 64, 65])
+@pytest.mark.parametrize("dtype,value_dtype", [(torch.float32, torch.float16), (torch.bfloat16, torch.bfloat16)])
+def test_chunks_of_few_streams_in_blocks_of_32_and_64_queries(T, past, dtype, value_dtype):
+    """Five streams' chunks take blocks of 32 queries (two of them, with up to 64 frames, share a ring and update it together), forty take 64 or other
+    kernels: rings are equal bit for bit, what a layer adds agrees but for the order of FP32 sums, i.e. where that flips the rounding of a
+    16-bit operand (bounds as above)."""
+    import fast_mimi_b200 as fm
+    layer = fm.MimiTransformerLayerB200(value_dtype=value_dtype).cuda()
+    layer.load_state_dict(_layer_params(T + past), strict=True)
+    layer = layer.to(dtype)
+    g = torch.Generator(device="cuda").manual_seed(past + T)
+    x = torch.randn(40, T, 512, device="cuda", generator=g).to(dtype)
+    cs = fm.rope_tables(torch.arange(past, past + T, device="cuda")[None])
+    many, few = fm.MimiKVRing(1, 40, 250, value_dtype=value_dtype), fm.MimiKVRing(1, 5, 250, value_dtype=value_dtype)
+    for t, u in ((many.ring_k, few.ring_k), (many.ring_v, few.ring_v)):
+        t.normal_(generator=g)
+        u.copy_(t[:, :5])
+    for ring in (many, few):
+        ring.advance(0, past)
+    want, got, base = layer(x, None, many, cs)[0][:5].float(), layer(x[:5], None, few, cs)[0].float(), x[:5].float()
+    assert O.rel_l2((got - base).cpu(), (want - base).cpu()) < {torch.float32: 1e-3, torch.bfloat16: 2e-2}[dtype]
+    assert torch.equal(few.ring_k, many.ring_k[:, :5]) and torch.equal(few.ring_v, many.ring_v[:, :5])
+    fm.check_status()
+
+
 # past: nothing, either side of a warp's sixteen slots, of a full ring and of its turn; 18 streams are the last that take the kernel on a B200
 @pytest.mark.parametrize("past", [0, 1, 15, 16, 17, 241, 249, 250, 257, 1000])
 @pytest.mark.parametrize("streams,T", [(1, 1), (2, 3), (18, 8)])
