@@ -2,7 +2,7 @@
 // K = 512 .. 4096 in slices of 512.
 //
 // Latency-bound, like fm_linear_small.cu, whose blocks of 128 rows x 64 (32) outputs fetch the rows of their slice of K after the wait
-// for the kernel in front, 64 KB and more, and share K eight ways.  Here a block owns 128 outputs x 16, 32 or 64 rows and 512 of K:
+// for the kernel in front, 64 KB and more, and share K eight ways.  Here a block owns 128 outputs x 16 to 128 rows and 512 of K:
 // its weights, 128 KB, go by way of shared memory into tensor memory (the A operand, 256 columns) ahead of the wait, and what
 // it fetches behind it is kRows KB.  The blocks of a cluster share K; rows kRows / S r .. of the tile belong to cluster rank r, every block
 // sends its FP32 partial sums of an owner's rows with one bulk copy, and the owner adds them in rank order (the result does not
@@ -26,17 +26,19 @@ constexpr int kWBox = kBlockN * 128, kWBytes = kChunks * kWBox;      // 64 of K;
 constexpr int kWarps = 16, kThreads = kWarps * 32, kMaxSplit = 8;
 constexpr int kTmemCols = 512, kTmemD = kSlice / 2;                  // weights | accumulators
 constexpr int kOutRow = kBlockN * 4;                                 // bytes of a row of results
+constexpr int kQuarters = 4;                                         // of a block's rows' K, loaded and waited for one by one where a block has 128
 struct Barriers {
   uint64_t w_full;
-  uint64_t a_full;
+  uint64_t a_full[kQuarters];
   uint64_t acc_full;
   uint64_t red_full;         // the partial sums of this block's rows have arrived from every block of the cluster
   uint32_t tmem_base;
   CtaCtl ctl;
 };
-// Weights, later this block's partial sums (first half) and those that it is sent (second half) | rows
-constexpr int smem_bytes(int rows) { return 1024 + kWBytes + kChunks * rows * 128 + static_cast<int>(sizeof(Barriers)); }
-static_assert(smem_bytes(64) <= 232448 && 64 * kOutRow <= kWBytes / 2, "exceeds the 227 KB a block may use");
+// Up to 64 rows: weights, later this block's partial sums (first half) and those that it is sent (second half) | rows.  128 rows: weights, later
+// the rows, later this block's partial sums | those that it is sent
+constexpr int smem_bytes(int rows) { return 1024 + kWBytes + (rows == 128 ? 128 * kOutRow : kChunks * rows * 128) + static_cast<int>(sizeof(Barriers)); }
+static_assert(smem_bytes(64) <= 232448 && smem_bytes(128) <= 232448 && 64 * kOutRow <= kWBytes / 2, "exceeds the 227 KB a block may use");
 
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
@@ -49,13 +51,15 @@ linear_ws_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                  uint32_t idesc, int* status) {
   using namespace ws;
   constexpr int kItems = (kRows * 16 + kThreads - 1) / kThreads;       // pieces of eight results of a thread
-  // accumulators of 64 or 128 of K each, added up in FP32: in one of 512 the tensor core cuts more of the addends (3.2e-7 of the result instead of 1e-7)
-  constexpr int kSums = kRows == 16 ? 8 : 4, kPer = kChunks / kSums;
+  // accumulators of 64, 128 or 256 of K each, added up in FP32: in one of 512 the tensor core cuts more of the addends (3.2e-7 of the result instead of 1e-7)
+  constexpr int kSums = kRows == 16 ? 8 : (kRows == 128 ? 2 : 4), kPer = kChunks / kSums;
+  constexpr bool kTall = kRows == 128;
+  constexpr int kParts = kTall ? kQuarters : 1;                        // of the rows' K, a barrier each
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem_w = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* smem_a = smem_w + kWBytes;
-  uint8_t* red = smem_w + kWBytes / 2;
-  Barriers* bars = reinterpret_cast<Barriers*>(smem_a + kChunks * kRows * 128);
+  uint8_t* smem_a = kTall ? smem_w : smem_w + kWBytes;
+  uint8_t* red = kTall ? smem_w + kWBytes : smem_w + kWBytes / 2;
+  Barriers* bars = reinterpret_cast<Barriers*>(smem_w + kWBytes + (kTall ? 128 * kOutRow : kChunks * kRows * 128));
   CtaCtl* ctl = &bars->ctl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int split = args.split;
@@ -68,7 +72,7 @@ linear_ws_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const bool skip = status != nullptr && *reinterpret_cast<volatile int*>(status) != 0;
   if (threadIdx.x == 0) {
     mbar_init(&bars->w_full, 1);
-    mbar_init(&bars->a_full, 1);
+    for (int i = 0; i < kParts; ++i) mbar_init(&bars->a_full[i], 1);
     mbar_init(&bars->acc_full, 1);
     mbar_init(&bars->red_full, 1);
     ctl->abort = 0;
@@ -105,6 +109,7 @@ linear_ws_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   }
   tmem_st_wait();
   tc_fence_before_sync();
+  if (kTall) fence_proxy_async_smem();
   __syncthreads();                         // the weights are in tensor memory, and the place where they lay is free
   if (split > 1) cluster_arrive_relaxed();
   griddep_wait();
@@ -113,16 +118,26 @@ linear_ws_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     tc_fence_after_sync();
     const bool one = elect_one();
     if (one) {
-      mbar_arrive_expect_tx(&bars->a_full, kChunks * kRows * 128);
 #pragma unroll
-      for (int kc = 0; kc < kChunks; ++kc) tma_load_2d(smem_a + kc * kRows * 128, &tmap_a, &bars->a_full, rank * kSlice + kc * 64, m0);
+      for (int part = 0; part < kParts; ++part) {
+        mbar_arrive_expect_tx(&bars->a_full[part], kChunks / kParts * kRows * 128);
+#pragma unroll
+        for (int kc = part * kChunks / kParts; kc < (part + 1) * kChunks / kParts; ++kc)
+          tma_load_2d(smem_a + kc * kRows * 128, &tmap_a, &bars->a_full[part], rank * kSlice + kc * 64, m0);
+      }
     }
     __syncwarp();
-    mbar_wait(&bars->a_full, 0, ctl, status, kErrWaitTma);
-    __syncwarp();
-    tc_fence_after_sync();
     const uint64_t rows = umma_desc_sw128(smem_u32(smem_a));
+    auto arrived = [&](int part) {
+      mbar_wait(&bars->a_full[part], 0, ctl, status, kErrWaitTma);
+      __syncwarp();
+      tc_fence_after_sync();
+    };
+    if constexpr (kParts == 1) arrived(0);
     for (int kc = 0; kc < kChunks; ++kc) {
+      if constexpr (kParts > 1) {
+        if (kc % (kChunks / kParts) == 0) arrived(kc / (kChunks / kParts));
+      }
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks)
         if (one)
@@ -135,12 +150,16 @@ linear_ws_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   // item: row item / 16 of those this block owns, half (item / 8) % 2 of its columns, piece item % 8
   const int first = m0 + rank * own, n_own = args.M - first < own ? args.M - first : own;
   const int n_items = skip ? 0 : n_own * 16;
-  PieceOperands ops[kItems];
+  // what the epilogue reads besides, asked for two pieces a thread ahead
+  constexpr int kAhead = kItems < 2 ? kItems : 2;
+  PieceOperands ops[kAhead];
+  auto item_of = [&](int i) { return static_cast<int>(threadIdx.x) + i * kThreads; };
+  auto ask = [&](int i) {
+    const int item = item_of(i);
+    if (item < n_items) load_operands<kOut>(args, first + (item >> 4), 2 * ntile + ((item >> 3) & 1), item & 7, ops[i % kAhead]);
+  };
 #pragma unroll
-  for (int i = 0; i < kItems; ++i) {
-    const int item = static_cast<int>(threadIdx.x) + i * kThreads;
-    if (item < n_items) load_operands<kOut>(args, first + (item >> 4), 2 * ntile + ((item >> 3) & 1), item & 7, ops[i]);
-  }
+  for (int i = 0; i < kAhead; ++i) ask(i);
   mbar_wait(&bars->acc_full, 0, ctl, status, kErrWaitMma);
   __syncwarp();
   tc_fence_after_sync();
@@ -154,7 +173,8 @@ linear_ws_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       const uint32_t at = t_row + kTmemD + k * kRows + (warp >> 2) * kN;
       if constexpr (kN == 4) tmem_ld4(at, u);
       else if constexpr (kN == 8) tmem_ld8(at, u);
-      else tmem_ld16(at, u);
+      else if constexpr (kN == 16) tmem_ld16(at, u);
+      else tmem_ld32(at, u);
       tmem_ld_wait();
 #pragma unroll
       for (int i = 0; i < kN; ++i) sum[i] = k == 0 ? __uint_as_float(u[i]) : sum[i] + __uint_as_float(u[i]);
@@ -181,7 +201,9 @@ linear_ws_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const uint8_t* sums = split > 1 ? red : smem_w;
 #pragma unroll
   for (int i = 0; i < kItems; ++i) {
-    const int item = static_cast<int>(threadIdx.x) + i * kThreads;
+    const int item = item_of(i);
+    const PieceOperands now = ops[i % kAhead];
+    if (i + kAhead < kItems) ask(i + kAhead);
     if (item < n_items) {
       const int local = item >> 4, sub = (item >> 3) & 1, j = item & 7;
       float lo[4] = {0.f, 0.f, 0.f, 0.f}, hi[4] = {0.f, 0.f, 0.f, 0.f};
@@ -191,7 +213,7 @@ linear_ws_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         lo[0] += a.x; lo[1] += a.y; lo[2] += a.z; lo[3] += a.w;
         hi[0] += b.x; hi[1] += b.y; hi[2] += b.z; hi[3] += b.w;
       }
-      finish_piece<kOut, __half>(args, lo, hi, ops[i], first + local, 2 * ntile + sub, j, status);
+      finish_piece<kOut, __half>(args, lo, hi, now, first + local, 2 * ntile + sub, j, status);
     }
   }
   if (split > 1) {
@@ -229,13 +251,18 @@ int clusters_of(int split) {
 // blocks then bring their weights while this one runs, by itself as few as a block per SM allows; 64 up to a block per SM, as far as the
 // device holds the clusters at once (K = 2048, N = 512: 512 rows 8.0 us, 528 in two waves 12.5 where the other kernel takes 10.2; K = 4096 128 rows 10.8
 // and 8.0).  A second tile of 64 with few rows in it is not worth one (K = N = 2048, 72 rows 7.9 us, 7.6 there).
+// 128 rows, whose loads follow the weights into the same memory, by themselves are no faster than the other kernels (K = 2048, N = 512
+// 640 rows 9.9 -> 10.1 us; K = 512, N = 2048 with GELU 8.2 -> 8.9).  In a chain, where the weights come early, they are: with K shared by four or
+// more, and, without, as far as two thirds of the SMs (eight layers of five clips of 125 frames 278 -> 268 -> 260 us, of 577 BF16 frames 302 -> 291 ->
+// 279; beyond, eight clips 306 -> 314).
 static int rows_per_block(int M, int N, int K, int dependent) {
   const int split = K / ws::kSlice;
   if (M <= 0 || N % ws::kBlockN != 0 || K % ws::kSlice != 0 || split > ws::kMaxSplit || (split & (split - 1)) != 0) return 0;
   const int clusters = clusters_of(split);
-  for (int rows = 16; rows <= 64; rows *= 2) {
+  for (int rows = 16; rows <= 128; rows *= 2) {
     const long long blocks = blocks_for(M, N, K, rows), room = dependent && rows < 64 ? sm_count() / 2 : sm_count();
-    if (blocks <= room && blocks / split <= clusters) return rows == 64 && M > 64 && M <= 96 ? 0 : rows;
+    if (rows == 128 && (!dependent || (split == 1 ? 3 * blocks > 2 * sm_count() : split < 4))) return 0;
+    if (blocks <= room && blocks / split <= clusters) return rows >= 64 && M > rows && M <= rows * 3 / 2 ? 0 : rows;
   }
   return 0;
 }
@@ -261,10 +288,11 @@ int launch_linear_ws(const void* a, const void* w, void* y, ParamVec scale, cons
   if (rc == 0) rc = encode_rows_16bit(&tmap_w, w, static_cast<uint64_t>(N), static_cast<uint64_t>(K), kBlockN, 64);
   if (rc != 0) return rc;
   using Kern = void (*)(const CUtensorMap, const CUtensorMap, const SmallArgs, uint32_t, int*);
-  static const Kern table[3][3] = {{linear_ws_kernel<0, 16>, linear_ws_kernel<0, 32>, linear_ws_kernel<0, 64>},
-                                   {linear_ws_kernel<1, 16>, linear_ws_kernel<1, 32>, linear_ws_kernel<1, 64>},
-                                   {linear_ws_kernel<2, 16>, linear_ws_kernel<2, 32>, linear_ws_kernel<2, 64>}};
-  const Kern kern = table[out_dtype][rows == 16 ? 0 : rows == 32 ? 1 : 2];
+  static const Kern table[3][4] = {
+      {linear_ws_kernel<0, 16>, linear_ws_kernel<0, 32>, linear_ws_kernel<0, 64>, linear_ws_kernel<0, 128>},
+      {linear_ws_kernel<1, 16>, linear_ws_kernel<1, 32>, linear_ws_kernel<1, 64>, linear_ws_kernel<1, 128>},
+      {linear_ws_kernel<2, 16>, linear_ws_kernel<2, 32>, linear_ws_kernel<2, 64>, linear_ws_kernel<2, 128>}};
+  const Kern kern = table[out_dtype][rows == 16 ? 0 : rows == 32 ? 1 : rows == 64 ? 2 : 3];
   rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes(rows));
   if (rc != 0) return rc;
   return launch_kernel(kern, dim3(N / kBlockN * args.split, (M + rows - 1) / rows), kThreads, smem_bytes(rows), st, args.split, dependent, tmap_a, tmap_w, args,

@@ -320,10 +320,10 @@ def test_first_half_of_a_call_for_few_streams(streams, T, past, dtype, value_dty
 
 
 # rows: one, either side of a cluster's rows (8) and of what seven clusters of 8, 16 and 24 rows hold; of where LayerNorm's products go from 16 to 32
-# and 64 rows a block (96, 192), and of the last that have LayerNorm inside (576 and 768); an MLP of another size, for which fewer kernels are there
+# and 64 rows a block (96, 192), of the last that have LayerNorm inside (576 and 768) and of those whose second MLP product has blocks of 128 rows (513 .. 1024); an MLP of another size, for which fewer kernels are there
 @pytest.mark.parametrize("B,T,ffn", [(1, 1, 2048), (1, 8, 2048), (1, 9, 2048), (1, 56, 2048), (1, 57, 2048), (1, 112, 2048), (1, 113, 2048), (2, 61, 2048),
-                                     (1, 96, 2048), (1, 97, 2048), (1, 168, 2048), (1, 169, 2048), (1, 193, 2048), (3, 192, 2048), (1, 577, 2048),
-                                     (3, 256, 2048), (1, 769, 2048), (1, 9, 1024)])
+                                     (1, 96, 2048), (1, 97, 2048), (1, 168, 2048), (1, 169, 2048), (1, 193, 2048), (3, 192, 2048), (1, 513, 2048),
+                                     (1, 577, 2048), (3, 256, 2048), (1, 769, 2048), (2, 512, 2048), (1, 1025, 2048), (1, 9, 1024)])
 @pytest.mark.parametrize("dtype,value_dtype", [(torch.float32, torch.float16), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16),
                                                (torch.bfloat16, torch.float16), (torch.float16, torch.float16)])
 def test_layer_on_few_rows_against_64_bits(B, T, ffn, dtype, value_dtype):
