@@ -115,11 +115,6 @@ __device__ __forceinline__ void team_sync(int lg) {
 __device__ __forceinline__ void warp_vote() {
   asm volatile("{\n\t.reg .b32 r;\n\t.reg .pred p;\n\tsetp.eq.u32 p, 0, 0;\n\tvote.sync.ballot.b32 r, p, 0xffffffff;\n\t}" ::: "memory");
 }
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
 __device__ __forceinline__ void load_global8(const float* p, float (&v)[8]) {      // one sector; p 32-byte aligned
   asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
