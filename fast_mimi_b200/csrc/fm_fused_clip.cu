@@ -4,9 +4,9 @@
 // MimiAttention.forward before o_proj (src/fast_mimi/model.py:1897-1914 projections + _apply_rope, :1627-1688 band
 // mask, :1860-1868 SDPA); the reference's own fused front half is src/fast_mimi/_packed_qkv.py:14-131,152-202.
 //
-// Two CTAs on neighbouring SMs (cluster of 2, tcgen05 cta_group::2) own one clip at a time: CTA r holds frames
+// Two CTAs on neighbouring SMs (cluster of 2, tcgen05 cta_group::2) own heads of one clip at a time: CTA r holds frames
 // 128r .. 128r+127.  Each keeps its half of the clip's x resident in shared memory (128 KB, one TMA load per clip,
-// the next clip's chunks replacing the current ones as the last head finishes with them) and walks the 8 heads:
+// the next clip's chunks replacing the current ones as the last head finishes with them) and walks its heads:
 //
 //   projection   one pair MMA stream M = 256 frames x N = 192 (the head's q | k | v columns) x K = 512; each CTA
 //                streams HALF of the head's W slice (96 rows, 12 KB stages), so a W byte crosses L2 -> SM once per
@@ -34,6 +34,7 @@
 #include "fm_common.cuh"
 #include "fm_kernels.h"
 #include "fm_launch.h"
+#include "fm_shares.h"
 
 namespace fm {
 
@@ -137,11 +138,36 @@ __device__ __forceinline__ void pack_output_half2(uint32_t oa_addr, uint32_t ob_
 }
 }  // namespace fused
 
-template <typename VT>
+// The heads that a pair of CTAs walks.  kWhole: all of clips pair, pair + pairs, ...; else an equal share of all clips' heads in turn.
+// (The dealt form serves both, but its few instructions more, in warps that have no registers left, cost 250 -> 258 to 265 us for 512 clips.)
+template <bool kWhole>
+struct Heads {
+  int first, stride, count;
+  __device__ __forceinline__ explicit Heads(const Shares& shares) {
+    if constexpr (kWhole) {
+      first = static_cast<int>(blockIdx.x >> 1);
+      stride = static_cast<int>(gridDim.x >> 1);
+      count = 8 * ((shares.n_steps / 8 - first + stride - 1) / stride);
+    } else {
+      int clip, head;
+      shares.share(static_cast<int>(blockIdx.x >> 1), &clip, &head, &count);
+      first = 8 * clip + head;
+      stride = 0;
+    }
+  }
+  __device__ __forceinline__ int head(int g) const { return kWhole ? g & 7 : (first + g) & 7; }
+  __device__ __forceinline__ int clip(int g) const { return kWhole ? first + (g >> 3) * stride : (first + g) >> 3; }
+  __device__ __forceinline__ int nth_clip(int g) const { return kWhole ? g >> 3 : ((first + g) >> 3) - (first >> 3); }     // of this pair's
+  __device__ __forceinline__ bool opens_clip(int g) const { return head(g) == 0 || (!kWhole && g == 0); }
+  __device__ __forceinline__ int clips() const { return nth_clip(count - 1) + 1; }
+  __device__ __forceinline__ int clip_at(int n) const { return kWhole ? first + n * stride : (first >> 3) + n; }
+};
+
+template <typename VT, bool kWhole>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(fused::kThreads, 1)
 attn_fused_clip_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                        const float* __restrict__ cos_tab, const float* __restrict__ sin_tab, long long cos_bstride,
-                       uint16_t* __restrict__ out, int n_clips, int T, int window, float scale_log2e,
+                       uint16_t* __restrict__ out, const __grid_constant__ Shares shares, int T, int window, float scale_log2e,
                        uint32_t idesc_proj, int* status) {
   using namespace fused;
   using namespace attn_tile;
@@ -157,9 +183,8 @@ attn_fused_clip_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();
   const bool leader = rank == 0;
-  const int pair = static_cast<int>(blockIdx.x >> 1), n_pairs = static_cast<int>(gridDim.x >> 1);
-  const int n_local = (n_clips - pair + n_pairs - 1) / n_pairs;   // clips pair, pair + n_pairs, ...
-  const int n_heads_total = 8 * n_local;
+  const Heads<kWhole> heads(shares);
+  const int n_heads_total = heads.count;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kKChunks; ++i) {
@@ -218,7 +243,7 @@ attn_fused_clip_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
       int stage = 0;
       uint32_t phase = 0;
       for (int g = 0; g < n_heads_total; ++g) {
-        const int h = g & 7;
+        const int h = heads.head(g);
         // This CTA's 96 of the head's 192 output columns, in accumulator order q (64) | k (64) | v (64):
         // CTA 0: q 0-31, q 32-63, k 0-31;  CTA 1: k 32-63, v 0-31, v 32-63.
         const int r0 = leader ? h * 64 : 512 + h * 64 + 32;
@@ -242,8 +267,9 @@ attn_fused_clip_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
     {
       const bool one = elect_one();
       if (one) tma_prefetch_desc(&tmap_x);
+      const int n_local = heads.clips();
       for (int n = 0; n < n_local; ++n) {
-        const int clip = pair + n * n_pairs;
+        const int clip = heads.clip_at(n);
         for (int kc = 0; kc < kKChunks; ++kc) {
           if (n > 0) mbar_wait(&sh->x_empty[kc], static_cast<uint32_t>(n - 1) & 1u, ctl, status, kErrWaitMma);
           if (one) {
@@ -261,7 +287,7 @@ attn_fused_clip_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
       uint32_t phase = 0;
       int chunk = 0;                 // running count of K chunks issued
       for (int g = 0; g < n_heads_total; ++g) {
-        const int n = g >> 3, h = g & 7;
+        const int n = heads.nth_clip(g), h = heads.head(g);
         if (g >= 1) mbar_wait(&sh->acc_empty, static_cast<uint32_t>(g - 1) & 1u, ctl, status, kErrWaitConsumer);
         tc_fence_after_sync();
         for (int kc = 0; kc < kKChunks; ++kc, ++chunk) {
@@ -271,7 +297,7 @@ attn_fused_clip_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
           if (chunk >= 2)
             mbar_wait(&sh->w_empty[(chunk - 2) % kWStages], static_cast<uint32_t>((chunk - 2) / kWStages) & 1u, ctl, status,
                       kErrWaitMma);
-          if (h == 0) mbar_wait(&sh->x_full[kc], static_cast<uint32_t>(n) & 1u, ctl, status, kErrWaitTma);
+          if (heads.opens_clip(g)) mbar_wait(&sh->x_full[kc], static_cast<uint32_t>(n) & 1u, ctl, status, kErrWaitTma);
           mbar_wait(&sh->w_full[stage], phase, ctl, status, kErrWaitTma);
           tc_fence_after_sync();
           const uint64_t a_desc = umma_desc_sw128(smem_u32(smem_x + kc * kXChunkBytes));
@@ -356,7 +382,7 @@ attn_fused_clip_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
     const uint32_t vt_chunk = static_cast<uint32_t>((frame & 63) >> 3);
     for (int g = 0; g < n_heads_total; ++g) {
       const uint32_t ph = static_cast<uint32_t>(g) & 1u;
-      if ((g & 7) == 0 && cos_bstride != 0) load_tables(pair + (g >> 3) * n_pairs);
+      if (heads.opens_clip(g) && cos_bstride != 0) load_tables(heads.clip(g));
       mbar_wait(&sh->acc_full, ph, ctl, status, kErrWaitMma);
       // Q and K of the previous head must have been consumed by its score MMAs.
       if (g >= 1) mbar_wait(&sh->qk_free, ph ^ 1u, ctl, status, kErrWaitMma);
@@ -467,7 +493,7 @@ attn_fused_clip_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
       // O_B was committed after O_A by the same thread, so in CTA 1 the wait for O_B covers both.
       mbar_wait(&sh->o_full[two_parts ? 1 : 0], ph, ctl, status, kErrWaitMma);
       tc_fence_after_sync();
-      const int clip = pair + (g >> 3) * n_pairs, h = g & 7;
+      const int clip = heads.clip(g), h = heads.head(g);
       uint16_t* dst = i < T ? out + (static_cast<long long>(clip) * T + i) * 512 + h * kD : nullptr;
       if (two_parts) {
         mbar_wait(&sh->xl_full, ph, ctl, status, kErrWaitConsumer);
@@ -517,15 +543,17 @@ attn_fused_clip_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
   }
 }
 
-// One pair of CTAs owns a clip at a time, so the one-kernel form takes 36 us (+ 5) per wave of clips however full the wave
-// is and, as both 128-frame tiles are always computed, whatever T; projection kernel + attention kernel take 0.53 us per clip
-// of 250 frames (+ 8.4), about in proportion to T.  Measured, one kernel / two, in us: T = 250: 1 clip 40 / 17, 64 clips 46 / 45,
-// 90 clips 79 / 59, 148 clips 79 / 85, 180 clips 113 / 104, 222 clips 115 / 124, 512 clips 256-265 / 278; T = 200: 64 clips
-// 46 / 44, 148 clips 78 / 77, 222 clips 111 / 108, 512 clips 247 / 239; T = 140: 64 clips 42 / 36, 512 clips 243 / 192.  (At
-// T = 140 the two kernels take up to a third longer than in proportion, which moves no decision.)
+// The clips' heads are dealt to the pairs of CTAs in equal numbers, in order (a clip that two pairs share is loaded twice); whole clips in turn where that gives no
+// pair more.  A call by itself, a pair to a clip -> heads dealt, us, T = 250: 1 clip 41 -> 13.7, 10 42 -> 19, 30 43 -> 29, 64 44.1 -> 42.9, 75 76.6 -> 51.7,
+// 100 78 -> 61, 149 110 -> 88, 300 187 -> 160; 74, 148 and 512 (250) as before.  Where q, k and v may go through memory, projection kernel + attention kernel take
+// 0.53 us per clip of 250 frames (+ 8.4), about in proportion to T, so that this form is the faster one for long clips alone, and by little: a layer, one
+// kernel / two, us: T = 256 46 clips 107 / 110, 64 131.6 / 134.3, 148 268 / 278, 190 356 / 363; T = 225 64 clips 127.8 / 129.5, 92 169 / 168; T = 200 64 clips
+// 118.8 / 118.7, 148 233 / 233; T = 170 64 clips 113 / 111, 222 295 / 287.  With four heads and fewer a pair its first loads weigh more (T = 240 32 clips 83 / 81.5).
 bool use_fused_clip(int B, int T) {
-  const int pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1, waves = (B + pairs - 1) / pairs;
-  return 36.0 * waves + 5.0 <= 0.00212 * static_cast<double>(B) * T + 8.4;
+  const Shares shares(B, 8, sm_count() / 2 > 0 ? sm_count() / 2 : 1);
+  const int heads = shares.per_block;
+  if (heads <= 4) return false;
+  return (heads % 8 == 0 ? 4.5 * heads + 5.0 : 5.0 * heads + 3.0) <= 0.00212 * static_cast<double>(B) * T + 8.4;
 }
 
 int launch_attn_fused_clip(const void* x, const void* w_qkv, const float* cos, const float* sin, long long cos_bstride,
@@ -557,15 +585,18 @@ int launch_attn_fused_clip(const void* x, const void* w_qkv, const float* cos, c
     if (rc != 0) return rc;
   }
   const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
-  const int n_pairs = B < max_pairs ? B : max_pairs;
+  const Shares shares(B, 8, max_pairs);
+  const bool whole = shares.per_block % 8 == 0;
+  const int n_pairs = !whole ? shares.used() : (B < max_pairs ? B : max_pairs);
   // dtype_flags bit 0: v, P and the output are FP16 (else BF16); bit 1: x and w_qkv hold FP16 (else BF16).
   const int in_fmt = (dtype_flags & 2) ? 0 : 1;
   const uint32_t idesc_proj = umma_idesc_f16(2 * kTile, 192, in_fmt, in_fmt, 0, 0);
-  auto kern = (dtype_flags & 1) ? attn_fused_clip_kernel<__half> : attn_fused_clip_kernel<__nv_bfloat16>;
+  auto kern = (dtype_flags & 1) ? (whole ? attn_fused_clip_kernel<__half, true> : attn_fused_clip_kernel<__half, false>)
+                                : (whole ? attn_fused_clip_kernel<__nv_bfloat16, true> : attn_fused_clip_kernel<__nv_bfloat16, false>);
   const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
   if (rc != 0) return rc;
   return launch_kernel(kern, dim3(2 * n_pairs), kThreads, kSmemBytes, st, 1, dependent, tmap_x, tmap_w, cos, sin, cos_bstride,
-                       static_cast<uint16_t*>(out), B, T, window, scale * 1.4426950408889634f, idesc_proj, status);
+                       static_cast<uint16_t*>(out), shares, T, window, scale * 1.4426950408889634f, idesc_proj, status);
 }
 
 }  // namespace fm

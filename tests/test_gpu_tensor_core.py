@@ -481,6 +481,26 @@ def test_fused_kernel_when_later_keys_score_far_higher(growth):
         assert O.rel_l2(fused.float().cpu(), want) < TOL
 
 
+# one head a pair of CTAs; two and a first pair that ends inside a clip; nine, two clips of a pair; whole clips, one and two of a pair; 17 heads
+@pytest.mark.parametrize("clips", [1, 10, 75, 74, 148, 149])
+@pytest.mark.parametrize("T", [129, 256])
+def test_heads_of_whole_clips_dealt_to_pairs_of_blocks(clips, T):
+    """Which pair of blocks computes a head changes no bit: the clips, each with its own RoPE tables, in one call against
+    seven at a time, and a call of one against the two-kernel form."""
+    import fast_mimi_b200 as fm
+    g = torch.Generator(device="cuda").manual_seed(clips + T)
+    x = torch.randn(clips, T, 512, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(1536, 512, device="cuda", generator=g) * 0.03).bfloat16()
+    cos, sin = fm.rope_tables(torch.arange(T, device="cuda") + 3 * torch.arange(clips, device="cuda")[:, None])
+    out = fm.ops.attention_fused(x, w, cos, sin)
+    for at in range(0, clips, 7):
+        s = slice(at, at + 7)
+        assert torch.equal(out[s], fm.ops.attention_fused(x[s], w, cos[s].contiguous(), sin[s].contiguous()))
+    two = fm.ops.band_attention_prefill(*fm.ops.qkv_rope(x[-1:], w, cos[-1:].contiguous(), sin[-1:].contiguous()))
+    assert O.rel_l2(out[-1:].float().cpu(), two.float().cpu()) < TOL
+    fm.check_status()
+
+
 def test_decode_with_a_different_position_per_stream_across_the_wrap():
     """16 streams at positions (37 s) % 600 + step, stepped over the ring's wrap (249 -> 250 -> 251 for some of
     them), per-stream tables [S, 1, 64] and a device-side stream_pos: every stream's step against the last row of a
