@@ -161,6 +161,8 @@ int launch_linear_small(const void* a, const void* w, void* y, ParamVec scale, c
 bool linear_ws_takes(int M, int N, int K, int dependent);
 int launch_linear_ws(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N, int K, int in_dtype, int out_dtype, int gelu,
                      int* status, cudaStream_t st, int dependent);
+int launch_qkv_ws(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status, cudaStream_t st,
+                  int dependent);
 int launch_qkv_small(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status,
                      cudaStream_t st, int dependent);
 // Output projection, LayerNorm and MLP of a layer in one kernel (fm_layer_tail.cu), for as many rows as layer_tail_takes says:

@@ -44,8 +44,8 @@ __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 }  // namespace ws
 
-// kOut: 0 = BF16, 1 = FP16, 2 = FP32 output and residual
-template <int kOut, int kRows>
+// kOut: 0 = BF16, 1 = FP16, 2 = FP32 output and residual; 3 = q | k | v with RoPE (VT: type of v)
+template <int kOut, typename VT, int kRows>
 __global__ void __launch_bounds__(ws::kThreads, 1)
 linear_ws_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ SmallArgs args,
                  uint32_t idesc, int* status) {
@@ -213,7 +213,7 @@ linear_ws_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         lo[0] += a.x; lo[1] += a.y; lo[2] += a.z; lo[3] += a.w;
         hi[0] += b.x; hi[1] += b.y; hi[2] += b.z; hi[3] += b.w;
       }
-      finish_piece<kOut, __half>(args, lo, hi, now, first + local, 2 * ntile + sub, j, status);
+      finish_piece<kOut, VT>(args, lo, hi, now, first + local, 2 * ntile + sub, j, status);
     }
   }
   if (split > 1) {
@@ -239,7 +239,7 @@ int clusters_of(int split) {
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   while (1 << at < split) ++at;
   const int n = known[at].get(dev, [split] {
-    const auto kern = linear_ws_kernel<2, 64>;
+    const auto kern = linear_ws_kernel<2, __half, 64>;
     return ensure_dynamic_smem(reinterpret_cast<const void*>(kern), ws::smem_bytes(64)) == 0 ? resident_clusters(kern, ws::kThreads, ws::smem_bytes(64), split)
                                                                                              : -1;
   });
@@ -269,9 +269,26 @@ static int rows_per_block(int M, int N, int K, int dependent) {
 
 bool linear_ws_takes(int M, int N, int K, int dependent) { return rows_per_block(M, N, K, dependent) != 0; }
 
+// a [M, K] and w [N, K]: the launch of one of the kernels for 16, 32, 64 and 128 rows a block
+using Kern = void (*)(const CUtensorMap, const CUtensorMap, const SmallArgs, uint32_t, int*);
+static int launch_ws(const Kern (&kerns)[4], const void* a, const void* w, SmallArgs& args, int rows, int K, int in_dtype, int* status, cudaStream_t st,
+                     int dependent) {
+  using namespace ws;
+  args.split = K / kSlice;
+  const int fmt = in_dtype == 1 ? 0 : 1;
+  CUtensorMap tmap_a, tmap_w;
+  int rc = encode_rows_16bit(&tmap_a, a, static_cast<uint64_t>(args.M), static_cast<uint64_t>(K), static_cast<uint32_t>(rows), 64);
+  if (rc == 0) rc = encode_rows_16bit(&tmap_w, w, static_cast<uint64_t>(args.N), static_cast<uint64_t>(K), kBlockN, 64);
+  if (rc != 0) return rc;
+  const Kern kern = kerns[rows == 16 ? 0 : rows == 32 ? 1 : rows == 64 ? 2 : 3];
+  rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes(rows));
+  if (rc != 0) return rc;
+  return launch_kernel(kern, dim3(args.N / kBlockN * args.split, (args.M + rows - 1) / rows), kThreads, smem_bytes(rows), st, args.split, dependent, tmap_a,
+                       tmap_w, args, umma_idesc_f16(128, rows, fmt, fmt, 0, 0), status);
+}
+
 int launch_linear_ws(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N, int K, int in_dtype, int out_dtype, int gelu,
                      int* status, cudaStream_t st, int dependent) {
-  using namespace ws;
   const int rows = rows_per_block(M, N, K, dependent);
   if (rows == 0) return -1;
   SmallArgs args = {};
@@ -281,22 +298,25 @@ int launch_linear_ws(const void* a, const void* w, void* y, ParamVec scale, cons
   args.M = M;
   args.N = N;
   args.gelu = gelu;
-  args.split = K / kSlice;
-  const int fmt = in_dtype == 1 ? 0 : 1;
-  CUtensorMap tmap_a, tmap_w;
-  int rc = encode_rows_16bit(&tmap_a, a, static_cast<uint64_t>(M), static_cast<uint64_t>(K), static_cast<uint32_t>(rows), 64);
-  if (rc == 0) rc = encode_rows_16bit(&tmap_w, w, static_cast<uint64_t>(N), static_cast<uint64_t>(K), kBlockN, 64);
-  if (rc != 0) return rc;
-  using Kern = void (*)(const CUtensorMap, const CUtensorMap, const SmallArgs, uint32_t, int*);
   static const Kern table[3][4] = {
-      {linear_ws_kernel<0, 16>, linear_ws_kernel<0, 32>, linear_ws_kernel<0, 64>, linear_ws_kernel<0, 128>},
-      {linear_ws_kernel<1, 16>, linear_ws_kernel<1, 32>, linear_ws_kernel<1, 64>, linear_ws_kernel<1, 128>},
-      {linear_ws_kernel<2, 16>, linear_ws_kernel<2, 32>, linear_ws_kernel<2, 64>, linear_ws_kernel<2, 128>}};
-  const Kern kern = table[out_dtype][rows == 16 ? 0 : rows == 32 ? 1 : rows == 64 ? 2 : 3];
-  rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes(rows));
-  if (rc != 0) return rc;
-  return launch_kernel(kern, dim3(N / kBlockN * args.split, (M + rows - 1) / rows), kThreads, smem_bytes(rows), st, args.split, dependent, tmap_a, tmap_w, args,
-                       umma_idesc_f16(128, rows, fmt, fmt, 0, 0), status);
+      {linear_ws_kernel<0, __half, 16>, linear_ws_kernel<0, __half, 32>, linear_ws_kernel<0, __half, 64>, linear_ws_kernel<0, __half, 128>},
+      {linear_ws_kernel<1, __half, 16>, linear_ws_kernel<1, __half, 32>, linear_ws_kernel<1, __half, 64>, linear_ws_kernel<1, __half, 128>},
+      {linear_ws_kernel<2, __half, 16>, linear_ws_kernel<2, __half, 32>, linear_ws_kernel<2, __half, 64>, linear_ws_kernel<2, __half, 128>}};
+  return launch_ws(table[out_dtype], a, w, args, rows, K, in_dtype, status, st, dependent);
+}
+
+int launch_qkv_ws(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status, cudaStream_t st, int dependent) {
+  using bf16 = __nv_bfloat16;
+  const int rows = rows_per_block(M, 1536, 512, dependent);
+  if (rows == 0) return -1;
+  SmallArgs args = {};
+  args.M = M;
+  args.N = 1536;
+  args.qkv = ep;
+  static const Kern table[2][4] = {
+      {linear_ws_kernel<3, bf16, 16>, linear_ws_kernel<3, bf16, 32>, linear_ws_kernel<3, bf16, 64>, linear_ws_kernel<3, bf16, 128>},
+      {linear_ws_kernel<3, __half, 16>, linear_ws_kernel<3, __half, 32>, linear_ws_kernel<3, __half, 64>, linear_ws_kernel<3, __half, 128>}};
+  return launch_ws(table[dtype_flags & 1], x, w_qkv, args, rows, 512, (dtype_flags & 2) ? 1 : 0, status, st, dependent);
 }
 
 }  // namespace fm

@@ -416,6 +416,9 @@ int launch_qkv_rope_gemm(const void* x, const void* w_qkv, const QkvEpilogueArgs
          reinterpret_cast<uintptr_t>(ep.k) | reinterpret_cast<uintptr_t>(ep.v) | reinterpret_cast<uintptr_t>(ep.ring_k) |
          reinterpret_cast<uintptr_t>(ep.ring_v)) & 15u)
       return -3;
+    // weights resident in tensor memory, by itself to 768 rows (the few-row kernel -> that one, us: 1 row 5.4 -> 4.7, 64 5.9 -> 5.0, 125 7.0 -> 5.3, 250 7.9 -> 5.5, 768
+    // 7.9 -> 7.1), in a chain to 1024 (eight layers of 8 clips of 125 frames 307 -> 304, 4 of 250 BF16 frames 318 -> 312, 1024 live streams 912 -> 909)
+    if (linear_ws_takes(M, 1536, 512, dependent)) return launch_qkv_ws(x, w_qkv, ep, M, dtype_flags, status, st, dependent);
     return launch_qkv_small(x, w_qkv, ep, M, dtype_flags, status, st, dependent);
   }
   return launch_gemm(x, w_qkv, ep, M, dtype_flags, status, st, dependent);

@@ -714,3 +714,24 @@ def test_fp32_tensors_are_converted_where_that_is_faster(B, T, inside):
     rc = _native.load().fm_window_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), 2, strides, *(w.data_ptr() for w in ws), None, out.data_ptr(), B, T, 250,
                                             0.125, 1, None, torch.cuda.current_stream().cuda_stream)
     assert rc == 0 and all(bool((w == -7.0).all()) == inside for w in ws)
+
+
+# rows: either side of what blocks of 16, 32 and 64 hold at once, and of a last block of one row
+@pytest.mark.parametrize("rows", [1, 16, 17, 192, 193, 384, 385, 768, 769])
+@pytest.mark.parametrize("dtype,value_dtype", [(torch.float16, torch.float16), (torch.bfloat16, torch.bfloat16), (torch.float16, torch.bfloat16)])
+def test_projection_of_few_rows_against_64_bits(rows, dtype, value_dtype):
+    """q, k and v of few rows with RoPE against 64 bits.  A value is off by its rounding at most, BF16 for q and k, and by FP32 sums of
+    512 products, nothing beside it: in the mean of squares less than half a unit of the last place, 2^-9 and 2^-12."""
+    import fast_mimi_b200 as fm
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(1, rows, 512, device="cuda", generator=g).to(dtype)
+    w = (torch.randn(1536, 512, device="cuda", generator=g) * 0.03).to(dtype)
+    cos, sin = fm.rope_tables(torch.arange(rows, device="cuda")[None])
+    got = fm.ops.qkv_rope(x, w, cos, sin, value_dtype=value_dtype)
+    want = (x[0].double() @ w.double().T).view(rows, 3, 8, 64)
+    for i, (t, bar) in enumerate(zip(got, (2 ** -9, 2 ** -9, 2 ** -12 if value_dtype == torch.float16 else 2 ** -9))):
+        e = want[:, i]
+        if i < 2:
+            e = e * cos[0].double()[:, None] + O.rotate_half(e) * sin[0].double()[:, None]
+        assert O.rel_l2(t.view(rows, 8, 64).double(), e) < bar
+    fm.check_status()
