@@ -9,7 +9,7 @@
 // boundary and the way of q, k and v through memory, each of which waits for a first load.  Here a block has one head of one
 // stream: 192 rows of W_qkv, 192 KB, on the chip before the wait for the kernel in front.  k and v's are the A operand of a tcgen05 product,
 // by way of shared memory in tensor memory (256 columns; 19 cycles an instruction): the ring's new rows have the bits that the other
-// projection kernels give them.  q's are in registers, as the fragments that mma.sync wants (K permuted alike in both operands, so that
+// projection kernels of a layer's call give them, K = 512 in one accumulator.  q's are in registers, as the fragments that mma.sync wants (K permuted alike in both operands, so that
 // a lane's share of 32 values of a row is one 16-byte load), a quarter of K a warp: both go on at once.  (All three on mma.sync took 1.2 us
 // at 16 cycles an instruction and scheduler.)  The ring's rows (64 KB) come while that runs: not ahead of the wait, since the kernel that
 // opens a chain cannot know what wrote them.  Then 16 slots of the ring a warp.
@@ -278,7 +278,7 @@ stream_front_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
         return (c->q_part[0][row][at] + c->q_part[1][row][at]) + (c->q_part[2][row][at] + c->q_part[3][row][at]);
       };
       const float lo = warp < 8 ? total(lane) : c->kv[row][lane], hi = warp < 8 ? total(32 + lane) : c->kv[row][32 + lane];
-      // rounded as in the other projection kernels, whose rows this kernel's stand beside in a ring
+      // contracted and rounded as in the other projection kernels, whose rows this kernel's stand beside in a ring
       const uint32_t y = Pack16<__nv_bfloat16>::pack(__fmaf_rn(lo, cosv, -__fmul_rn(hi, sinv)), __fmaf_rn(hi, cosv, __fmul_rn(lo, sinv)));
       if (warp < 8) {
         c->q[row * kQRow + lane] = static_cast<uint16_t>(y);

@@ -289,6 +289,35 @@ def test_chunks_of_few_streams_in_blocks_of_32_and_64_queries(T, past, dtype, va
     fm.check_status()
 
 
+# rows of the larger call: 480 (LayerNorm inside the projection), 800, 1000 and 1024 (weights resident in tensor memory), 1025 and 1280 (the few-row kernel),
+# 2400 (pairs of blocks); of the smaller one: 20 to 600
+@pytest.mark.parametrize("streams,T", [(24, 20), (40, 20), (40, 25), (32, 32), (1024, 1), (1025, 1), (64, 20), (60, 40)])
+@pytest.mark.parametrize("dtype,value_dtype", [(torch.float32, torch.float16), (torch.bfloat16, torch.bfloat16)])
+def test_a_ring_does_not_depend_on_the_streams_beside_it(streams, T, dtype, value_dtype):
+    """What a layer's call writes into a stream's ring is the same bit for bit however many other streams share the call, i.e. whichever kernel
+    makes k and v: each sums K = 512 in one accumulator."""
+    import fast_mimi_b200 as fm
+    past = 300
+    layer = fm.MimiTransformerLayerB200(value_dtype=value_dtype).cuda()
+    layer.load_state_dict(_layer_params(T), strict=True)
+    layer = layer.to(dtype)
+    g = torch.Generator(device="cuda").manual_seed(streams)
+    x = torch.randn(streams, T, 512, device="cuda", generator=g).to(dtype)
+    cs = fm.rope_tables(torch.arange(past, past + T, device="cuda")[None])
+
+    def rings(n):
+        ring = fm.MimiKVRing(1, n, 250, value_dtype=value_dtype)
+        ring.advance(0, past)
+        layer(x[:n], None, ring, cs)
+        return ring.ring_k[0], ring.ring_v[0]
+
+    whole = rings(streams)
+    for n in (1, 15 if T > 8 else 600):
+        for few, many in zip(rings(n), whole):
+            assert torch.equal(few, many[:n])
+    fm.check_status()
+
+
 # past: nothing, either side of a warp's sixteen slots, of a full ring and of its turn; 18 streams are the last that take the kernel on a B200
 @pytest.mark.parametrize("past", [0, 1, 15, 16, 17, 241, 249, 250, 257, 1000])
 @pytest.mark.parametrize("streams,T", [(1, 1), (2, 3), (18, 8)])
