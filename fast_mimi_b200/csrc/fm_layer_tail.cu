@@ -40,8 +40,8 @@ constexpr int kUnits = kFfn / kCtas;                 // 128 hidden units
 constexpr int kChunks = kHidden / 64;
 constexpr int kWBox = 128 * 128;                      // 128 rows of a weight, 64 of K
 constexpr int kWBytes = kUnits * kHidden * 2;         // of W_1 and of W_2, one after the other in the same place
-constexpr int kTmemCols = 512;                       // W_1 | fc1 | fc2
-constexpr int kTmemFc1 = kHidden / 2, kTmemFc2 = kTmemFc1 + 32;
+constexpr int kTmemCols = 512;                       // W_1 | fc1, two accumulators | fc2
+constexpr int kTmemFc1 = kHidden / 2, kTmemFc2 = kTmemFc1 + 2 * 32;
 struct Ctl {
   uint64_t w1_full;
   uint64_t w2_full;
@@ -318,7 +318,8 @@ layer_tail_kernel(const __grid_constant__ CUtensorMap tmap_w1, const __grid_cons
   __syncthreads();
   cluster_arrive_relaxed();                // x1 has been read: partial sums of y may come
 
-  // ---- fc1: 128 hidden units as rows of the product.  Columns past kRows (N is a multiple of 16) are what lies behind the operand.
+  // ---- fc1: 128 hidden units as rows of the product, 256 of K in each of two accumulators (fm_ln_linear.cu).  Columns past kRows (N is a
+  // multiple of 16) are what lies behind the operand.
   if (warp == 0) {
     tc_fence_after_sync();
     const uint64_t h = umma_desc_sw128(smem_u32(smem_h));
@@ -327,8 +328,8 @@ layer_tail_kernel(const __grid_constant__ CUtensorMap tmap_w1, const __grid_cons
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks)
         if (one)
-          tc_mma_ts(tmem_base + kTmemFc1, tmem_base + kc * 32 + ks * 8, h + static_cast<uint64_t>(kc * kRows * 128 >> 4) + 2u * ks, idesc,
-                    (kc | ks) != 0 ? 1u : 0u);
+          tc_mma_ts(tmem_base + kTmemFc1 + kc / (kChunks / 2) * 32, tmem_base + kc * 32 + ks * 8, h + static_cast<uint64_t>(kc * kRows * 128 >> 4) + 2u * ks,
+                    idesc, (kc % (kChunks / 2) | ks) != 0 ? 1u : 0u);
     }
     if (one) tc_commit(&c->fc_full[0]);
     __syncwarp();
@@ -341,13 +342,18 @@ layer_tail_kernel(const __grid_constant__ CUtensorMap tmap_w1, const __grid_cons
     constexpr int kN = kRows == 24 ? 8 : 4;
     const int row0 = (warp >> 2) * kN, unit = (warp & 3) * 32 + lane;
     if (row0 < kRows) {
-      uint32_t u[kN];
-      if constexpr (kN == 8) tmem_ld8(t_row + kTmemFc1 + row0, u);
-      else tmem_ld4(t_row + kTmemFc1 + row0, u);
+      uint32_t u[kN], w[kN];
+      if constexpr (kN == 8) {
+        tmem_ld8(t_row + kTmemFc1 + row0, u);
+        tmem_ld8(t_row + kTmemFc1 + 32 + row0, w);
+      } else {
+        tmem_ld4(t_row + kTmemFc1 + row0, u);
+        tmem_ld4(t_row + kTmemFc1 + 32 + row0, w);
+      }
       tmem_ld_wait();
 #pragma unroll
       for (int i = 0; i < kN; i += 2) {
-        float v0 = __uint_as_float(u[i]), v1 = __uint_as_float(u[i + 1]);
+        float v0 = __uint_as_float(u[i]) + __uint_as_float(w[i]), v1 = __uint_as_float(u[i + 1]) + __uint_as_float(w[i + 1]);
         gelu_erf2(v0, v1);
         const uint32_t p = Pack16<TOp>::pack(v0, v1);
         uint8_t* chunk = smem_g + (unit >> 6) * (kRows * 128) + (unit & 7) * 2;

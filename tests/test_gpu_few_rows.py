@@ -384,6 +384,29 @@ def test_layer_on_few_rows_against_64_bits(B, T, ffn, dtype, value_dtype):
     fm.check_status()
 
 
+# rows of the larger call: 200 and 500 (LayerNorm inside the product), 600, 640 and 768 (weights resident in tensor memory); of the smaller one: 8 to 100, for which
+# the MLP is part of one kernel with 8, 16 or 24 rows a cluster (8 to 56, to 112, to 168 rows)
+@pytest.mark.parametrize("clips,T,few", [(2, 100, 1), (5, 100, 1), (6, 100, 1), (8, 96, 1), (96, 8, 1), (10, 60, 1), (4, 160, 1), (10, 60, 4)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_hidden_units_do_not_depend_on_the_clips_beside_them(clips, T, few, dtype):
+    """What fc1 and GELU make of a frame is the same bit for bit in every kernel that takes up to 768 rows: each sums 256 of K = 512 in an accumulator.
+    W_o = 0 and rows of the identity as W_2, so that a layer adds 512 of its hidden units, or the last 512, to its input."""
+    import fast_mimi_b200 as fm
+    layer = fm.MimiTransformerLayerB200().cuda()
+    layer.load_state_dict(_layer_params(T), strict=True)
+    with torch.no_grad():
+        layer.self_attn.o_proj.weight.zero_()
+        layer.mlp_layer_scale.scale.fill_(1.0)
+    layer = layer.to(dtype).requires_grad_(False)
+    x = torch.randn(clips, T, 512, device="cuda", generator=torch.Generator(device="cuda").manual_seed(clips)).to(dtype)
+    cs = fm.rope_tables(torch.arange(T, device="cuda")[None])
+    for unit in (0, 2048 - 512):
+        layer.mlp.fc2.weight.zero_()
+        layer.mlp.fc2.weight[:, unit:unit + 512].fill_diagonal_(1.0)
+        assert torch.equal(layer(x[:few], None, None, cs)[0], layer(x, None, None, cs)[0][:few])
+    fm.check_status()
+
+
 @pytest.mark.parametrize("T", [1, 8])
 @pytest.mark.parametrize("streams", [1, 15, 16])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
