@@ -23,6 +23,7 @@
 #include "fm_device_fact.h"
 #include "fm_kernels.h"
 #include "fm_launch.h"
+#include "fm_rvq_key.h"
 #include "fm_warp_mma.cuh"
 
 namespace fm {
@@ -34,7 +35,6 @@ constexpr int kDim = 256, kWarps = 16, kThreads = kWarps * 32;
 constexpr int kHidden = 512, kProjected = kDim / kCtas;         // channels in front of the projection; dimensions of a block
 constexpr int kBookBytes = kEntries * kDim * 2, kChunkBytes = kEntries * 128;
 constexpr int kMaxLayers = 32;
-constexpr unsigned long long kNoCandidate = 0xfffffffdull << 32;      // below every distance that is not finite, above those that are
 constexpr int kMaxRows = 32;                                   // vectors of a cluster: 32 or 16
 struct Shared {
   uint64_t full[2];
@@ -211,7 +211,7 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
       exact[1] = make_float4(x[i][4], x[i][5], x[i][6], x[i][7]);
       if (lane == 0) {
         sh->margin[f] = rvq_margin(xx, a.e_max[l], args.tau_rel);
-        sh->best_in[l & 1][f] = ~0ull;
+        sh->best_in[l & 1][f] = kRvqNoKey;
       }
     }
     if (tid == 0) sh->n_listed = 0;
@@ -280,8 +280,8 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
       const float2 margin = *reinterpret_cast<const float2*>(&sh->margin[f0 + nt * 8]);
       const float limit[2] = {m.x + margin.x, m.y + margin.y};
       if (warp == nh && g == 0) {                              // one that is not finite: no candidate in any block, whatever the others find
-        if (!(limit[0] == limit[0])) atomicMin(&sh->best_in[l & 1][f0 + nt * 8], kNoCandidate);
-        if (!(limit[1] == limit[1])) atomicMin(&sh->best_in[l & 1][f0 + nt * 8 + 1], kNoCandidate);
+        if (!(limit[0] == limit[0])) atomicMin(&sh->best_in[l & 1][f0 + nt * 8], kRvqNoCandidate);
+        if (!(limit[1] == limit[1])) atomicMin(&sh->best_in[l & 1][f0 + nt * 8 + 1], kRvqNoCandidate);
       }
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -318,7 +318,7 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         // a distance that is not finite loses to every other and leaves index 0, as where nothing is smaller than the best so far
         const unsigned long long key = acc < INFINITY ? (static_cast<unsigned long long>(__float_as_uint(acc)) << 32) | static_cast<unsigned>(j)
-                                                      : 0xfffffffeull << 32;
+                                                      : kRvqNotFinite;
         if (lane == 0 && c0 + i * kWarps < n_listed) atomicMin(&sh->best_in[l & 1][f], key);
       }
     }
@@ -329,7 +329,7 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
       const uint32_t peer = static_cast<uint32_t>(tid / kRows);
       st_async_u64(map_to_cta(smem_u32(&sh->best[l & 1][f][rank]), peer), sh->best_in[l & 1][f], map_to_cta(smem_u32(&sh->arrived[l & 1]), peer));
     }
-    mbar_wait_cluster(&sh->arrived[l & 1], static_cast<uint32_t>(l >> 1) & 1u, ctl, status, kErrWaitConsumer);
+    const bool whole = mbar_wait_cluster(&sh->arrived[l & 1], static_cast<uint32_t>(l >> 1) & 1u, ctl, status, kErrWaitConsumer);
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < kMine; ++i) {
@@ -340,9 +340,9 @@ rvq_stack_kernel(const __grid_constant__ CUtensorMap tmap_books0, const __grid_c
         const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
         best = other < best ? other : best;
       }
-      const bool none = best == ~0ull || best == kNoCandidate; // a residual that is not finite
-      const int j = none ? 0 : static_cast<int>(best & 0xffffffffu);
-      if (rank == 0 && lane == 0 && f < n && !skip) {
+      const int entry = rvq_entry_of(best, kCodes), j = entry < 0 ? 0 : entry;
+      const bool none = entry < 0;                             // a residual that is not finite
+      if (rank == 0 && lane == 0 && f < n && !skip && whole) {       // (after a wait that gave up: words of no meaning)
         a.codes[static_cast<size_t>(l) * args.rows + r0 + f] = j;
         if (none && status != nullptr) atomicMax(status, static_cast<int>(kErrNonFinite));
       }
