@@ -111,7 +111,7 @@ linear_ws_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   }
   tmem_st_wait();
   tc_fence_before_sync();
-  if (kTall) fence_proxy_async_smem();
+  if (kTall || split > 1) fence_proxy_async_smem();        // the rows, or other blocks' copies, come where the weights were read
   __syncthreads();                         // the weights are in tensor memory, and the place where they lay is free
   if (split > 1) cluster_arrive_relaxed();
   griddep_wait();

@@ -60,6 +60,20 @@ def test_linear_with_resident_weights(rows, K, N, in_dtype):
     fm.check_status()
 
 
+# K shared by two, four and eight blocks, rows of 16, 32 and 64 a block: partial sums of the other blocks come where a block's weights lay
+@pytest.mark.parametrize("rows,K,N", [(16, 1024, 1024), (300, 1024, 1024), (16, 2048, 512), (64, 2048, 512), (512, 2048, 512), (16, 4096, 256), (60, 4096, 512)])
+def test_products_whose_blocks_share_k_repeat_exactly(rows, K, N):
+    import fast_mimi_b200 as fm
+    g = torch.Generator(device="cuda").manual_seed(rows + K)
+    a = torch.randn(rows, K, device="cuda", generator=g).half()
+    w = (torch.randn(N, K, device="cuda", generator=g) / K ** 0.5).half()
+    first = fm.ops.linear(a, w, out_dtype=torch.float32)
+    assert O.rel_l2(first.double(), a.double() @ w.double().T) < 2e-6
+    for y in [fm.ops.linear(a, w, out_dtype=torch.float32) for _ in range(100)]:
+        assert torch.equal(y, first)
+    fm.check_status()
+
+
 @pytest.mark.parametrize("B,T", [(1, 1), (1, 127), (3, 43), (2, 128), (5, 100)])
 def test_projection_with_few_rows(B, T):
     import fast_mimi_b200 as fm
