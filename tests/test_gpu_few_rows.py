@@ -801,3 +801,68 @@ def test_projection_of_few_rows_against_64_bits(rows, dtype, value_dtype):
             e = e * cos[0].double()[:, None] + O.rotate_half(e) * sin[0].double()[:, None]
         assert O.rel_l2(t.view(rows, 8, 64).double(), e) < bar
     fm.check_status()
+
+
+@pytest.mark.parametrize("call", ["streams", "clip", "clips", "linear", "attention", "window", "encode", "decode", "downsample"])
+def test_a_call_may_be_its_threads_first(call):
+    """Threads that have made no CUDA call yet and whose memory comes out of the allocator's pool: no context is bound to them.  Results are those of
+    the thread that made the objects."""
+    import threading
+    import types
+    import fast_mimi_b200 as fm
+    torch.manual_seed(0)
+    cs = lambda T: fm.rope_tables(torch.arange(T, device="cuda")[None])
+    if call in ("streams", "clip", "clips"):
+        layer = fm.MimiTransformerLayerB200().cuda()
+        layer.load_state_dict(_layer_params(3))
+        S, T = {"streams": (3, 1), "clip": (1, 125), "clips": (5, 100)}[call]
+        x, tables = torch.randn(S, T, 512, device="cuda"), cs(T)
+        ring = fm.MimiKVRing(1, S, 250) if call == "streams" else None
+
+        def run():
+            if ring is not None:
+                ring.reset()
+            return layer(x, None, ring, tables)[0]
+    elif call == "linear":
+        a, w = torch.randn(200, 512, device="cuda").half(), torch.randn(512, 512, device="cuda").half()
+        run = lambda: fm.ops.linear(a, w, out_dtype=torch.float32)
+    elif call == "attention":
+        x, w, tables = torch.randn(2, 200, 512, device="cuda").bfloat16(), (torch.randn(1536, 512, device="cuda") * 0.02).bfloat16(), cs(200)
+        run = lambda: fm.ops.attention_prefill(x, w, *tables)
+    elif call == "window":
+        q, k, v = (torch.randn(1, 400, 8, 64, device="cuda").half().transpose(1, 2) for _ in range(3))
+        run = lambda: fm.native_window_attention(q, k, v, scale=0.125, window=250)
+    elif call in ("encode", "decode"):
+        branch = lambda n: fm.MimiRVQB200(torch.randn(n, 2048, 256, device="cuda"), torch.randn(256, 512, 1, device="cuda"),
+                                          torch.randn(512, 256, 1, device="cuda"))
+        split = fm.MimiSplitRVQB200(branch(1), branch(7))
+        e = torch.randn(1, 512, 1, device="cuda")               # one frame: nothing to lay out anew in front
+        codes = split.encode(e)
+        run = (lambda: split.encode(e)) if call == "encode" else (lambda: split.decode(codes))
+    else:
+        conv = torch.nn.Conv1d(512, 512, 4, 2, bias=False, device="cuda").requires_grad_(False)
+        down = fm.MimiDownsampleB200(types.SimpleNamespace(conv=conv, causal=True, pad_mode="replicate"))
+        e = torch.randn(1, 125, 512, device="cuda").transpose(1, 2)
+        run = lambda: down(e)
+    with torch.no_grad():
+        want = run()
+        run()                                                   # its result goes back to the pool
+        torch.cuda.synchronize()
+        for _ in range(2):
+            got = []
+
+            def body():
+                with torch.no_grad():
+                    try:
+                        got.append(run())
+                    except Exception as error:                  # noqa: BLE001
+                        got.append(error)
+
+            thread = threading.Thread(target=body)
+            thread.start()
+            thread.join()
+            assert isinstance(got[0], torch.Tensor), got[0]
+            torch.cuda.synchronize()
+            assert torch.equal(got[0], want)
+            got.clear()
+    fm.check_status()
