@@ -12,6 +12,14 @@ from test_gpu_layer_blocks import ROUND, _layer_params
 pytestmark = pytest.mark.gpu
 
 
+def _streams(which, T=1):
+    """Numbers of live streams either side of where a layer's call of T <= 8 frames takes other kernels: "last", each of whose heads has an SM to itself
+    (LayerNorm, projection and attention are one kernel), "next" (two), and "many", more rows than the clusters of 16 blocks could hold that take
+    up to 24 each through output projection and MLP (one kernel; for "many" three or four)."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return {"one": 1, "last": sms // 8, "next": sms // 8 + 1, "many": 24 * (sms // 16) // T + 1}[which]
+
+
 # rows: one, either side of a tile's edge, two tiles; shapes: every split (8, 4, 2, 1 blocks per cluster) that K and the
 # number of tiles lead to, a K that only divides by two, the first size past the rule's edge (two tiles per SM)
 @pytest.mark.parametrize("rows", [1, 127, 128, 129, 256, 1100])
@@ -94,9 +102,9 @@ def test_projection_with_few_rows(B, T):
 
 
 @pytest.mark.parametrize("window", [250, 100, 3])
-@pytest.mark.parametrize("streams", [1, 5])
+@pytest.mark.parametrize("streams", [1, 5, 19])
 def test_layer_on_live_streams_matches_the_oracle(streams, window):
-    """A session of calls of 1 .. 7 frames (the streaming kernel), longer ones (the tensor-core path) and one beyond the
+    """A session of calls of 1 .. 8 frames (the streaming kernels: one to 18 streams on a B200, 19 and more), longer ones (the tensor-core path) and one beyond the
     window, over rings that fill up and wrap; every call against the oracle's layer on its own cache.  Bar as for the
     layer without a cache: 2e-3 on what the layer adds to its input."""
     import fast_mimi_b200 as fm
@@ -116,16 +124,18 @@ def test_layer_on_live_streams_matches_the_oracle(streams, window):
     fm.check_status()
 
 
-# rings with spare slots, partly filled and wrapped, and one of `window` slots; T: the streaming kernel, the few-tile kernel with
-# and without the ring's update inside, the linearised path (slots > 256)
+# rings with spare slots, partly filled and wrapped, and one of `window` slots; T: the streaming kernels (two streams and one more than the first of
+# them takes), the few-tile kernel with the ring's update inside (a block or, T = 40 of two streams, two of them a stream and head) and
+# without, the linearised path (slots > 256, or T = 100 of many streams)
 @pytest.mark.parametrize("slots,past", [(256, 150), (256, 300), (250, 90), (120, 500), (100, 400), (300, 350)])
-@pytest.mark.parametrize("T", [1, 8, 20, 100])
-def test_slots_outside_the_window_do_not_show(slots, past, T):
+@pytest.mark.parametrize("T", [1, 8, 20, 40, 100])
+@pytest.mark.parametrize("streams", ["two", "next"])
+def test_slots_outside_the_window_do_not_show(streams, slots, past, T):
     """A layer call over a ring of more slots than the window, non-finite wherever a slot is empty or has left the window:
     output and new rows are those over a ring that holds the window alone.  Bar: the sums run in another order, and a flipped
     rounding of a 16-bit operand is 2^-11 of one value in many."""
     import fast_mimi_b200 as fm
-    S, window = 2, 100
+    S, window = 2 if streams == "two" else _streams(streams), 100
     layer = fm.MimiTransformerLayerB200(sliding_window=window).cuda()
     layer.load_state_dict(_layer_params(17))
     g = torch.Generator(device="cuda").manual_seed(past)
@@ -151,7 +161,8 @@ def test_slots_outside_the_window_do_not_show(slots, past, T):
 
 @pytest.mark.parametrize("value_dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("T", [1, 8])
-def test_streaming_probabilities_keep_the_bits_of_fp32(value_dtype, T):
+@pytest.mark.parametrize("streams", ["one", "next"])
+def test_streaming_probabilities_keep_the_bits_of_fp32(streams, value_dtype, T):
     """A layer whose output is the attention core of a chosen query over a chosen ring.  FP16 values: all that counts comes
     from probabilities of about 2^-20 beside one of 1 whose value is 0.  BF16 values: +1 and -1 in turn, under probabilities that
     differ by 2^-12 of themselves.  Bar: the result's own rounding; FP32 exponentials (2^-22) add 1e-3 of the BF16 result."""
@@ -177,12 +188,15 @@ def test_streaming_probabilities_keep_the_bits_of_fp32(value_dtype, T):
         k[:, at[-1], 0] = 0.0
         k[:, at[1:-1:2], 1] = -(2.0 ** -6)
         v[:, at[:-1:2]], v[:, at[1:-1:2]] = 1.0, -1.0
-    ring = fm.MimiKVRing(1, 1, 250, value_dtype=value_dtype)
-    ring.ring_k[0, 0], ring.ring_v[0, 0] = k.cuda(), v.cuda()
+    S = _streams(streams)
+    ring = fm.MimiKVRing(1, S, 250, value_dtype=value_dtype)
+    ring.ring_k[0], ring.ring_v[0] = k.cuda(), v.cuda()
     assert torch.equal(ring.ring_k[0, 0].float().cpu(), k)
     ring.advance(0, past)
     one = torch.ones(1, T, 64, device="cuda")
-    got = layer(torch.zeros(1, T, 512, device="cuda"), None, ring, (one, one * 0))[0].cpu().view(T, 8, 64)
+    every = layer(torch.zeros(S, T, 512, device="cuda"), None, ring, (one, one * 0))[0].cpu().view(S, T, 8, 64)
+    assert torch.equal(every, every[:1].expand_as(every))
+    got = every[0]
     new = torch.zeros(8, T, 64)
     kk, vv = torch.cat((k[:, at], new), dim=1).double(), torch.cat((v[:, at], new), dim=1).double()
     for t in range(T):
@@ -196,35 +210,34 @@ def test_streaming_probabilities_keep_the_bits_of_fp32(value_dtype, T):
 @pytest.mark.parametrize("T", [1, 2, 8])
 @pytest.mark.parametrize("past", [0, 3, 249, 700])
 @pytest.mark.parametrize("dtype,value_dtype", [(torch.float32, torch.float16), (torch.bfloat16, torch.bfloat16), (torch.float16, torch.float16)])
-def test_output_projection_behind_the_heads_of_a_stream(T, past, dtype, value_dtype):
-    """Up to 15 streams the attention kernel goes on to the output projection, 16 take a kernel for it: what a stream's rows come
-    to must not depend on it but for the order of FP32 sums (2^-21 of the branch) and, where that flips the rounding of an
-    operand behind it, 16-bit units (2^-9 BF16, 2^-11 FP16, over 512 terms with random signs).  Rings are equal bit for bit."""
+def test_a_stream_does_not_depend_on_those_beside_it(T, past, dtype, value_dtype):
+    """The kernels that a call takes follow from how many streams share it: what one stream's rows come to must not depend on it but for the order of
+    FP32 sums (2^-21 of the branch) and, where that flips the rounding of an operand behind it, 16-bit units (2^-9 BF16, 2^-11 FP16, over 512
+    terms with random signs).  Rings are equal bit for bit, and as long as the kernels stay the same so are the results."""
     import fast_mimi_b200 as fm
     layer = fm.MimiTransformerLayerB200(value_dtype=value_dtype).cuda()
     layer.load_state_dict(_layer_params(T + past), strict=True)
     layer = layer.to(dtype)
     g = torch.Generator(device="cuda").manual_seed(past)
-    x = torch.randn(16, T, 512, device="cuda", generator=g).to(dtype)
+    counts = [_streams(which, T) for which in ("many", "next", "last", "one")]
+    x = torch.randn(counts[0], T, 512, device="cuda", generator=g).to(dtype)
     cs = fm.rope_tables(torch.arange(past, past + T, device="cuda")[None])
-    rings = [fm.MimiKVRing(1, n, 250, value_dtype=value_dtype) for n in (16, 15, 1)]
+    rings = [fm.MimiKVRing(1, n, 250, value_dtype=value_dtype) for n in counts]
     for t in (rings[0].ring_k, rings[0].ring_v):
         t.normal_(generator=g)
+    for n, ring in zip(counts[1:], rings[1:]):
+        ring.ring_k.copy_(rings[0].ring_k[:, :n])
+        ring.ring_v.copy_(rings[0].ring_v[:, :n])
     outs = []
-    for ring in rings:
-        n = ring.num_streams
-        ring.ring_k.copy_(rings[0].ring_k[:, :n]) if ring is not rings[0] else None
-        ring.ring_v.copy_(rings[0].ring_v[:, :n]) if ring is not rings[0] else None
-    for ring in rings:
+    for n, ring in zip(counts, rings):
         ring.advance(0, past)
-        outs.append(layer(x[:ring.num_streams], None, ring, cs)[0])
-    for ring, y in zip(rings[1:], outs[1:]):
-        n = ring.num_streams
+        outs.append(layer(x[:n], None, ring, cs)[0])
+    for n, ring, y in zip(counts[1:], rings[1:], outs[1:]):
         assert torch.equal(ring.ring_k[0], rings[0].ring_k[0, :n]) and torch.equal(ring.ring_v[0], rings[0].ring_v[0, :n])
         want = outs[0][:n].float() - x[:n].float()
         bound = {torch.float32: 1e-3, torch.float16: 4e-3, torch.bfloat16: 2e-2}[dtype]
         assert O.rel_l2((y.float() - x[:n].float()).cpu(), want.cpu()) < bound
-    assert torch.equal(outs[1][:1], outs[2])
+    assert torch.equal(outs[2][:1], outs[3])
     fm.check_status()
 
 
@@ -233,34 +246,36 @@ def test_output_projection_behind_the_heads_of_a_stream(T, past, dtype, value_dt
 @pytest.mark.parametrize("dtype,value_dtype", [(torch.float32, torch.float16), (torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float16),
                                                (torch.float16, torch.float16)])
 def test_live_streams_against_64_bits(T, past, dtype, value_dtype):
-    """A layer's call for 15 streams (output projection behind the attention) and for 16 (a kernel of its own), from the parameters, the
+    """A layer's call for numbers of streams that take different kernels (``_streams``), from the parameters, the
     rings and the input as they are held, against the same in 64 bits.  FP32 streams: 2e-3 of what the layer adds, the bar of the
     layer without a cache.  16-bit streams are rounded twice on the way (2^-9 BF16, 2^-11 FP16 each at most), which covers
-    what the branches add to that.  Both routes round alike but for the order of FP32 sums: neither is 5 % further off."""
+    what the branches add to that.  All routes round alike but for the order of FP32 sums: none is 5 % further off."""
     import fast_mimi_b200 as fm
     window = slots = 250
     layer = fm.MimiTransformerLayerB200(value_dtype=value_dtype).cuda()
     layer.load_state_dict(_layer_params(90 + T + past), strict=True)
     layer = layer.to(dtype).requires_grad_(False)
     g = torch.Generator(device="cuda").manual_seed(past + T)
-    x = torch.randn(16, T, 512, device="cuda", generator=g).to(dtype)
+    counts = [_streams(which, T) for which in ("last", "next", "many")]
+    S = counts[0]                                                                    # of every call, those that are looked at
+    x = torch.randn(counts[-1], T, 512, device="cuda", generator=g).to(dtype)
     cos, sin = fm.rope_tables(torch.arange(past, past + T, device="cuda")[None])
-    first = fm.MimiKVRing(1, 16, window, value_dtype=value_dtype)
+    first = fm.MimiKVRing(1, counts[-1], window, value_dtype=value_dtype)
     for t in (first.ring_k, first.ring_v):
         t.normal_(generator=g)
-    held = [t[0].double() for t in (first.ring_k, first.ring_v)]                     # [16, 8, slots, 64]
+    held = [t[0, :S].double() for t in (first.ring_k, first.ring_v)]                 # [S, 8, slots, 64]
     got = {}
-    for n in (15, 16):
+    for n in counts:
         ring = fm.MimiKVRing(1, n, window, value_dtype=value_dtype)
         ring.ring_k.copy_(first.ring_k[:, :n])
         ring.ring_v.copy_(first.ring_v[:, :n])
         ring.advance(0, past)
-        got[n] = layer(x[:n], None, ring, (cos, sin))[0][:15].double()
+        got[n] = layer(x[:n], None, ring, (cos, sin))[0][:S].double()
     p = {k: v.double() for k, v in layer.state_dict().items()}
-    xd = x.double()
+    xd = x[:S].double()
     norm = lambda t, name: torch.nn.functional.layer_norm(t, (512,), p[name + ".weight"], p[name + ".bias"], 1e-5)
     h = norm(xd, "input_layernorm")
-    q, k, v = ((h @ p[f"self_attn.{n}_proj.weight"].T).view(16, T, 8, 64).transpose(1, 2) for n in "qkv")
+    q, k, v = ((h @ p[f"self_attn.{n}_proj.weight"].T).view(S, T, 8, 64).transpose(1, 2) for n in "qkv")
     turn = lambda t: t * cos.double()[:, None] + O.rotate_half(t) * sin.double()[:, None]
     at = torch.arange(max(0, past - window + 1), past, device="cuda")
     keys, values = torch.cat((held[0][:, :, at % slots], turn(k)), 2), torch.cat((held[1][:, :, at % slots], v), 2)
@@ -268,10 +283,10 @@ def test_live_streams_against_64_bits(T, past, dtype, value_dtype):
     new = pos[-T:, None]
     seen = (pos[None] <= new) & (pos[None] > new - window)
     core = torch.softmax((turn(q) @ keys.transpose(-1, -2) * 0.125).masked_fill(~seen, float("-inf")), -1) @ values
-    x1 = xd + core.transpose(1, 2).reshape(16, T, 512) @ p["self_attn.o_proj.weight"].T * p["self_attn_layer_scale.scale"]
+    x1 = xd + core.transpose(1, 2).reshape(S, T, 512) @ p["self_attn.o_proj.weight"].T * p["self_attn_layer_scale.scale"]
     y = x1 + torch.nn.functional.gelu(norm(x1, "post_attention_layernorm") @ p["mlp.fc1.weight"].T) @ p["mlp.fc2.weight"].T * p["mlp_layer_scale.scale"]
-    base = xd[:15] if dtype == torch.float32 else torch.zeros_like(xd[:15])
-    off = {n: O.rel_l2(got[n] - base, y[:15] - base) for n in got}
+    base = xd if dtype == torch.float32 else torch.zeros_like(xd)
+    off = {n: O.rel_l2(got[n] - base, y - base) for n in got}
     assert max(off.values()) < {torch.float32: 2e-3, torch.bfloat16: 2 ** -8, torch.float16: 2 ** -10}[dtype], off
     assert max(off.values()) < 1.05 * min(off.values()), off
     fm.check_status()
@@ -339,7 +354,7 @@ def test_a_ring_does_not_depend_on_the_streams_beside_it(streams, T, dtype, valu
 def test_first_half_of_a_call_for_few_streams(streams, T, past, dtype, value_dtype):
     """LayerNorm, projection and attention as one kernel (up to 18 streams) and as two (the same streams among 19): rings are equal bit
     for bit, what a layer adds agrees but for the order of FP32 sums, i.e. where that flips the rounding of a 16-bit operand (bounds as
-    where the output projection's routes are compared)."""
+    in ``test_a_stream_does_not_depend_on_those_beside_it``)."""
     import fast_mimi_b200 as fm
     layer = fm.MimiTransformerLayerB200(value_dtype=value_dtype).cuda()
     layer.load_state_dict(_layer_params(T + past), strict=True)
@@ -422,17 +437,18 @@ def test_hidden_units_do_not_depend_on_the_clips_beside_them(clips, T, few, dtyp
 
 
 @pytest.mark.parametrize("T", [1, 8])
-@pytest.mark.parametrize("streams", [1, 15, 16])
+@pytest.mark.parametrize("which", ["one", "last", "next", "many"])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
-def test_live_streams_without_layer_scales(streams, T, dtype):
-    """The native call takes a layer without scales (NULL) as one whose scales are one, bit for bit, whichever kernel does the
-    output projection, and refuses scales off a 16-byte boundary."""
+def test_live_streams_without_layer_scales(which, T, dtype):
+    """The native call takes a layer without scales (NULL) as one whose scales are one, bit for bit, whichever kernels apply
+    them, and refuses scales off a 16-byte boundary."""
     import fast_mimi_b200 as fm
     layer = fm.MimiTransformerLayerB200().cuda()
     layer.load_state_dict(_layer_params(31), strict=True)
     layer = layer.to(dtype).requires_grad_(False)
     layer.self_attn_layer_scale.scale.fill_(1.0)
     layer.mlp_layer_scale.scale.fill_(1.0)
+    streams = _streams(which, T)
     g = torch.Generator(device="cuda").manual_seed(streams + T)
     x = torch.randn(streams, T, 512, device="cuda", generator=g).to(dtype)
     past = 40
