@@ -386,3 +386,36 @@ def test_calls_of_the_binding_are_the_checked_ones(B, T, quantizers):
         split.encode(bad.transpose(1, 2), quantizers)
     ops.default_status(frames.device).zero_()
     assert torch.equal(split.decode(codes), y)
+
+
+# rows: one, either side of what a cluster takes, the most that all clusters take with 16 vectors each (112 on a B200) and with 32 (224), one more
+@pytest.mark.parametrize("rows", [1, 16, 17, 63, 112, 113, 160, 224, 225])
+@pytest.mark.parametrize("quantizers", [2, 8, 16, 32])
+def test_search_with_the_projections_inside_against_64_bits(rows, quantizers):
+    """Both branches from FP32 embeddings, through the binding (up to 224 vectors one kernel that projects, too) and through the calls behind it.  Every code's entry is the
+    nearest to what the codes in front of it leave of the exact projection, up to FP32: the projection is off by 1e-6 of its size at most and a
+    distance moves by 2 sqrt(d) of that, for either of two entries; sums of 256 squares are off by 2^-24 times sqrt(256), likewise."""
+    import fast_mimi_b200 as fm
+    from fast_mimi_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(rows + quantizers)
+    normal = lambda *shape: torch.randn(*shape, device="cuda", generator=g)
+    books = lambda n: normal(n, 2048, 256) * (0.6 ** torch.arange(n, device="cuda").clamp(max=7))[:, None, None]
+    branch = lambda n: fm.MimiRVQB200(books(n), normal(256, 512, 1) / 512 ** 0.5, normal(512, 256, 1) / 16)
+    split = fm.MimiSplitRVQB200(branch(1), branch(31))
+    e = normal(1, 512, rows)
+    got = split.encode(e, quantizers)
+    frames = e[0].T.contiguous()
+    x = ops._linear_rows(frames, lambda: ops.split_half(frames), split._joint_in_parts(), (rows,), None, mats=2)
+    checked = torch.empty(quantizers, rows, dtype=torch.int64, device="cuda")
+    ops._rvq_search_stacks(x, (split.semantic.books, split.acoustic.books), (checked[:1], checked[1:]), ops._status_ptr(None, x))
+    fm.check_status()
+    for codes in (got.view(quantizers, rows), checked):
+        for b, own in ((split.semantic, codes[:1]), (split.acoustic, codes[1:])):
+            r = frames.double() @ b.input_proj.double().view(256, 512).T
+            size = r.norm(dim=1)
+            for l, c in enumerate(own):
+                vectors = b.books.vectors[l].double()
+                d = torch.cdist(r, vectors, compute_mode="donot_use_mm_for_euclid_dist") ** 2
+                least, chosen = d.min(dim=1).values, d.gather(1, c[:, None])[:, 0]
+                assert (chosen - least <= 4e-6 * size * least.sqrt() + 2e-6 * least).all(), (l, float((chosen - least).max()))
+                r = r - vectors[c]
