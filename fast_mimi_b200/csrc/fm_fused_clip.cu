@@ -543,17 +543,18 @@ attn_fused_clip_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
   }
 }
 
-// The clips' heads are dealt to the pairs of CTAs in equal numbers, in order (a clip that two pairs share is loaded twice); whole clips in turn where that gives no
-// pair more.  A call by itself, a pair to a clip -> heads dealt, us, T = 250: 1 clip 41 -> 13.7, 10 42 -> 19, 30 43 -> 29, 64 44.1 -> 42.9, 75 76.6 -> 51.7,
-// 100 78 -> 61, 149 110 -> 88, 300 187 -> 160; 74, 148 and 512 (250) as before.  Where q, k and v may go through memory, projection kernel + attention kernel take
+// The clips' heads are dealt to the pairs of CTAs in equal numbers, in order (a clip that two pairs share is loaded twice), where that is worth its cost
+// (fm_shares.h); else whole clips in turn.  A call by itself, a pair to a clip -> heads dealt, us, T = 250: 1 clip 41 -> 13.7, 10 42 -> 19, 30 43 -> 29, 64 44.1 -> 42.9,
+// 75 76.6 -> 51.7, 100 78 -> 61, 149 110 -> 88, 300 187 -> 160; 74, 148 and 512 (250) as before.  Where q, k and v may go through memory, projection kernel + attention kernel take
 // 0.53 us per clip of 250 frames (+ 8.4), about in proportion to T, so that this form is the faster one for long clips alone, and by little: a layer, one
 // kernel / two, us: T = 256 46 clips 107 / 110, 64 131.6 / 134.3, 148 268 / 278, 190 356 / 363; T = 225 64 clips 127.8 / 129.5, 92 169 / 168; T = 200 64 clips
 // 118.8 / 118.7, 148 233 / 233; T = 170 64 clips 113 / 111, 222 295 / 287.  With four heads and fewer a pair its first loads weigh more (T = 240 32 clips 83 / 81.5).
 bool use_fused_clip(int B, int T) {
-  const Shares shares(B, 8, sm_count() / 2 > 0 ? sm_count() / 2 : 1);
-  const int heads = shares.per_block;
-  if (heads <= 4) return false;
-  return (heads % 8 == 0 ? 4.5 * heads + 5.0 : 5.0 * heads + 3.0) <= 0.00212 * static_cast<double>(B) * T + 8.4;
+  const int pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
+  const Shares shares(B, 8, pairs);
+  if (shares.per_block <= 4) return false;
+  const double us = dealt_heads_pay(shares, B, pairs) ? 5.0 * shares.per_block + 3.0 : 36.0 * ((B + pairs - 1) / pairs) + 5.0;
+  return us <= 0.00212 * static_cast<double>(B) * T + 8.4;
 }
 
 int launch_attn_fused_clip(const void* x, const void* w_qkv, const float* cos, const float* sin, long long cos_bstride,
@@ -586,7 +587,7 @@ int launch_attn_fused_clip(const void* x, const void* w_qkv, const float* cos, c
   }
   const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
   const Shares shares(B, 8, max_pairs);
-  const bool whole = shares.per_block % 8 == 0;
+  const bool whole = !dealt_heads_pay(shares, B, max_pairs);
   const int n_pairs = !whole ? shares.used() : (B < max_pairs ? B : max_pairs);
   // dtype_flags bit 0: v, P and the output are FP16 (else BF16); bit 1: x and w_qkv hold FP16 (else BF16).
   const int in_fmt = (dtype_flags & 2) ? 0 : 1;

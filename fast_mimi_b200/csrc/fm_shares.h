@@ -40,4 +40,14 @@ struct Shares {
   static int up(int a, int b) { return static_cast<int>((static_cast<long long>(a) + b - 1) / b); }
 };
 
+// Whether clips' heads (fm_fused_clip.cu), dealt evenly to `pairs` of blocks, are out sooner than whole clips in turn.  A dealt head costs up to a tenth
+// more: a clip that two pairs share is loaded twice, and the warps that look up whose head is next have no registers left.  Calls on new inputs,
+// whole -> dealt, us, by heads a pair:  8 -> 1 42.6 -> 19.2, 8 -> 7 44.2 -> 43.0, 16 -> 14 80.6 -> 78.9, 16 -> 15 84.1 -> 85.1, 24 -> 22 119.7 -> 120.5, 24 -> 23 126.6 -> 129.7,
+// 32 -> 29 157.5 -> 156.5, 32 -> 30 162.0 -> 163.5, 32 -> 31 163.9 -> 169.1, 40 -> 37 200.6 -> 201.6, 48 -> 45 236.9 -> 239.5, 56 -> 51 277.0 -> 274.2, 56 -> 53 285.1 -> 289.3,
+// 56 -> 55 288.1 -> 297.7 (in a captured graph, over and over on one input, dealing gains some two percent more: 24 -> 22 112.8 -> 109.0, 56 -> 53 247.9 -> 247.6).
+inline bool dealt_heads_pay(const Shares& shares, int clips, int pairs) {
+  const long long whole = 8ll * ((clips + pairs - 1ll) / pairs);
+  return 12ll * shares.per_block < 11 * whole;
+}
+
 }  // namespace fm
