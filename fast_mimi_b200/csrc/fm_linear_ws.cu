@@ -252,7 +252,9 @@ int clusters_of(int split) {
 // Rows of a block, 0: not a call for this kernel.  In a chain as few as leave half of the SMs to the kernels in front and behind, whose
 // blocks then bring their weights while this one runs, by itself as few as a block per SM allows; 64 up to a block per SM, as far as the
 // device holds the clusters at once (K = 2048, N = 512: 512 rows 8.0 us, 528 in two waves 12.5 where the other kernel takes 10.2; K = 4096 128 rows 10.8
-// and 8.0).  A second tile of 64 with few rows in it is not worth one (K = N = 2048, 72 rows 7.9 us, 7.6 there).
+// and 8.0).  A second tile of 64 with few rows in it is not worth one (K = N = 2048, 72 rows 7.9 us, 7.6 there).  Nor are two blocks that share K for 256 outputs and
+// one tile of the other kernel, where eight do (K = 1024, N = 256 1 row 4.6 to 4.8 us there, 5.1 here, 64 rows 5.0 and 5.2, 128 5.3 and 5.3, 144 5.8 and 5.3; N = 512 1 row
+// 5.4 and 5.1).
 // 128 rows, whose loads follow the weights into the same memory, by themselves are no faster than the other kernels (K = 2048, N = 512
 // 640 rows 9.9 -> 10.1 us; K = 512, N = 2048 with GELU 8.2 -> 8.9).  In a chain, where the weights come early, they are: with K shared by four or
 // more, and, without, as far as two thirds of the SMs (eight layers of five clips of 125 frames 278 -> 268 -> 260 us, of 577 BF16 frames 302 -> 291 ->
@@ -260,6 +262,7 @@ int clusters_of(int split) {
 static int rows_per_block(int M, int N, int K, int dependent) {
   const int split = K / ws::kSlice;
   if (M <= 0 || N % ws::kBlockN != 0 || K % ws::kSlice != 0 || split > ws::kMaxSplit || (split & (split - 1)) != 0) return 0;
+  if (split == 2 && N == 2 * ws::kBlockN && M <= 128) return 0;
   const int clusters = clusters_of(split);
   for (int rows = 16; rows <= 128; rows *= 2) {
     const long long blocks = blocks_for(M, N, K, rows), room = dependent && rows < 64 ? sm_count() / 2 : sm_count();

@@ -43,7 +43,7 @@ def test_linear_with_few_rows(rows, shape):
 
 # K shared out over one, two, four and eight blocks; rows at the edges of tiles of 16, 32 and 64 and of what the kernel takes
 @pytest.mark.parametrize("rows,K,N", [(16, 512, 256), (17, 512, 512), (593, 512, 512), (1184, 512, 512), (1185, 512, 512), (2368, 512, 512), (2369, 512, 512),
-                                      (33, 1024, 1024), (500, 1024, 512), (31, 2048, 512), (33, 2048, 512), (257, 2048, 512), (512, 2048, 512),
+                                      (33, 1024, 1024), (500, 1024, 512), (128, 1024, 256), (129, 1024, 256), (31, 2048, 512), (33, 2048, 512), (257, 2048, 512), (512, 2048, 512),
                                       (513, 2048, 512), (15, 4096, 512), (65, 4096, 256), (130, 4096, 512), (576, 512, 2048), (577, 512, 2048)])
 @pytest.mark.parametrize("in_dtype", [torch.float16, torch.bfloat16])
 def test_linear_with_resident_weights(rows, K, N, in_dtype):
