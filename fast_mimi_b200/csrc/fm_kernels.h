@@ -65,8 +65,7 @@ int launch_qkv_rope_gemm(const void* x, const void* w_qkv, const QkvEpilogueArgs
 int launch_out_proj_gemm(const void* a, const void* w, void* y, const float* out_scale, const void* resid, int M,
                          int dtype_flags, int* status, cudaStream_t st);
 // y[M,N] = resid + scale * act(a[M,K] * w[N,K]^T); in_dtype 0 BF16 / 1 FP16; out_dtype 0 BF16 / 1 FP16 / 2 FP32
-// (type of y and resid); gelu 1 = exact GELU.  N a multiple of 256, K a multiple of 64.  dependent 1: behind the kernel in front, in a
-// chain; 2: in a layer whose residual stream is FP32.
+// (type of y and resid); gelu 1 = exact GELU.  N a multiple of 256, K a multiple of 64.
 int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N,
                        int K, int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent = 0);
 // Split-precision product y = (a_hi + a_lo)(w_hi + w_lo)^T in FP32 grade (all four FP16; lo lo left out).  `a` is [a_rows,

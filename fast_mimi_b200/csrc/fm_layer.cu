@@ -136,7 +136,7 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
   } else {
     rc = launch_layernorm512(b.x1, p.stream_dtype, vec(p.ln2_weight), vec(p.ln2_bias), p.ln2_eps, b.h, tc, rows, st, 1);
     if (rc != 0) return rc;
-    rc = launch_linear_gemm(b.h, p.w_fc1, b.g, ParamVec(nullptr), nullptr, rows, p.ffn, 512, tc, tc, 1, status, st, p.stream_dtype == 2 ? 2 : 1);
+    rc = launch_linear_gemm(b.h, p.w_fc1, b.g, ParamVec(nullptr), nullptr, rows, p.ffn, 512, tc, tc, 1, status, st, 1);
   }
   if (rc != 0) return rc;
   return launch_linear_gemm(b.g, p.w_fc2, y, vec(p.mlp_scale), b.x1, rows, 512, p.ffn, tc, p.stream_dtype, 0, status, st, 1);

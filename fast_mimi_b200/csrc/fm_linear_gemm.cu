@@ -526,14 +526,14 @@ static bool half_units(int pair_tiles, int N, int max_pairs, int k_chunks) {
 // FP32 results of rows that hardly give any SM a second block are out sooner from the few-row kernel, whose last blocks are short where
 // their rows are few, in a call by itself: K = 2048, N = 512 2305 rows 12.9 -> 14.0, 2400 13.1 -> 13.9, K = 512, N = 512 2400 rows 7.5 -> 8.1, N = 1024
 // 1153 rows 7.3 -> 7.8, 1280 8.0 -> 7.8, N = 2048 513 rows 7.3 -> 7.8.  16-bit ones are not (K = 2048, N = 512 2400 rows 14.0 -> 14.0, K = 512 8.6 ->
-// 8.4, N = 2048, GELU 513 rows 8.3 -> 8.1), nor in a chain, whose next kernel finds an SM free the sooner (8 layers of 2313 rows 452 -> 430).  With
-// GELU that takes some rows more, and more of them in FP32 streams (8 layers, few-row kernel -> half units: FP32 560 rows 303 -> 307, 700 rows 333 -> 344,
-// 750 rows 324 -> 325, 765 rows 338 -> 332; BF16 550 rows 313 -> 315, 650 rows 333 -> 334, 700 rows 354 -> 350, 740 rows 349 -> 336; FP16 like BF16).
-static bool one_wave_of_halves(int M, int pair_tiles, int N, int max_pairs, bool fp32, bool gelu, int dependent) {
+// 8.4, N = 2048, GELU 513 rows 8.3 -> 8.1), nor in a chain, whose next kernel finds an SM free the sooner (8 layers of 2313 rows 452 -> 430).  What
+// a chain leaves to this rule of products with GELU is beyond the rows that have resident weights (8 layers, few-row kernel -> half units, FP32 and
+// BF16 streams: MLP of 2048 769 rows 315 -> 308 and 319 -> 311, 1000 331 -> 325 and 331 -> 325; of 1024 1537 rows 383 -> 373 and 393 -> 384; of 1280 1153 rows 345 -> 345 and 359 -> 355; of 2304
+// 641 307 -> 303 and 315 -> 311; of 2560 513 295 -> 291 and 304 -> 297; of 3328 385 278 -> 281 and 283 -> 283, 466 285 -> 278 and 286 -> 282; of 3840 385 286 -> 289 and 291 -> 292).
+static bool one_wave_of_halves(int M, int pair_tiles, int N, int max_pairs, bool fp32, int dependent) {
   constexpr int kBlock = lin::kBlockM * 64;
   const long long sms = sm_count(), results = static_cast<long long>(M) * N;
   if (pair_tiles * static_cast<long long>(N / 128) > max_pairs) return false;
-  if (gelu && dependent) return results > (dependent == 2 ? kBlock * 41 / 32 : kBlock * 9 / 8) * sms;
   if (fp32 && !dependent) return results > kBlock * 33 / 32 * sms;
   return static_cast<long long>((M + lin::kBlockM - 1) / lin::kBlockM) * (N / 64) > sms;
 }
@@ -552,7 +552,7 @@ int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, co
   if (out_dtype != 3 && linear_ws_takes(M, N, K, dependent)) return launch_linear_ws(a, w, y, scale, resid, M, N, K, in_dtype, out_dtype, gelu, status, st, dependent);
   const int pair_tiles = ((M + kBlockM - 1) / kBlockM + 1) / 2;
   const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
-  const bool one_wave = out_dtype != 3 && one_wave_of_halves(M, pair_tiles, N, max_pairs, out_dtype == 2, gelu != 0, dependent);
+  const bool one_wave = out_dtype != 3 && one_wave_of_halves(M, pair_tiles, N, max_pairs, out_dtype == 2, dependent);
   if (out_dtype != 3 && !one_wave && few_row_tiles(M, N))
     return launch_linear_small(a, w, y, scale, resid, M, N, K, in_dtype, out_dtype, gelu, status, st, dependent);
   // The wide shape where the epilogue carries arithmetic (GELU, candidate records) for unit after unit, the narrow one otherwise.
