@@ -1,11 +1,13 @@
 // Linear layers and the QKV projection for few rows (sm_100a): y = residual + scale * act(a W^T), or q | k | v with
 // RoPE, for calls whose rows fill only a few 128-row tiles (one clip, one frame of up to a few hundred streams).
 //
-// (Linear layers of fewer rows, whose weights fit the chip's tensor memory, take fm_linear_ws.cu.)
+// Where the weights fit the chip's tensor memory such calls take fm_linear_ws.cu.  Left to this kernel are split-precision products (the quantiser's
+// projections and convolution), q | k | v of 769 rows and more (1025 in a layer's chain), K that is not 512 times a power of two, and linear
+// layers past that kernel's lines: by themselves, FP32 with a residual, K = 2048, N = 512 600 rows 9.7 us, 1800 12.2.
 //
 // What bounds such a call is latency and the number of SMs that pull weights out of L2, not arithmetic: the pair
 // kernels (fm_linear_gemm.cu, fm_qkv_gemm.cu) cut the output into 256 x 256 tiles, so that 125 rows x 512 outputs at
-// K = 2048 occupied 4 of 148 SMs, each walking 32 K-chunks one after the other (with an FP32 residual 20.8 us; here 6.8 us).  Here a block owns
+// K = 2048 occupied 4 of 148 SMs, each walking 32 K-chunks one after the other (with an FP32 residual 20.8 us; here 6.8 us, 6.0 with resident weights).  Here a block owns
 // 128 rows x 64 outputs (one attention head; or x 32) and a SLICE of K: the blocks of a thread-block cluster share one output
 // tile and split K between them, so the same layer runs on 64 SMs with four chunks each.  The partial sums meet in
 // distributed shared memory: row r of the tile belongs to cluster rank r % S, every block sends its FP32 partials of an
@@ -257,7 +259,8 @@ linear_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 // Beyond that the blocks re-read activations and weights too often for what they save, and the 256 x 256 tiles of the
 // pair kernels are faster: at K = 512, N = 2048 1024 rows (256 tiles) take 9.1 us here and 10.9 us there, 1500 rows (384
 // tiles) 13.9 against 10.9; at K = 2048, N = 512 3678 rows (232 tiles) 17.1 against 22.1, 5000 rows (320) 27.5 against 22.5.
-// (Linear layers of more than one tile per SM take half units of the pair kernel where those are one wave: fm_linear_gemm.cu.)
+// (Those figures are of the 256 x 256 tiles alone.  Linear layers of more than one tile per SM take half units of the pair kernel where
+// those are one wave: fm_linear_gemm.cu.)
 bool few_row_tiles(int M, int N) {
   return static_cast<long long>((M + small::kBlockM - 1) / small::kBlockM) * (N / 64) <= 2ll * sm_count();
 }
