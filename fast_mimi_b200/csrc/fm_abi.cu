@@ -181,6 +181,7 @@ int fm_attention_chunk_bf16(const void* x, const void* w_qkv, const float* cos, 
   if (S < 0 || T < 0 || past < 0 || window <= 0 || ring_slots < window || value_dtype < 0 || value_dtype > 3) return -1;
   if (ring_k == nullptr || ring_v == nullptr) return -1;
   if (S == 0 || T == 0) return 0;
+  if (fm::absent(q_ws, k_ws, v_ws, out)) return -1;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int rc = fm_qkv_rope_bf16(x, w_qkv, cos, sin, cos_bstride, q_ws, k_ws, v_ws, S, T, value_dtype, status, stream);
   if (rc != 0) return rc;

@@ -340,7 +340,7 @@ int launch_ring_decode_attn(const void* q, const void* ring_k, const void* ring_
                             int value_is_fp16, int* status, cudaStream_t st) {
   using namespace dec;
   if (S <= 0) return S == 0 ? 0 : -1;
-  if (ring_slots <= 0 || ring_slots > kMaxSlots || S > (1 << 27) || pos_base < 0) return -1;
+  if (ring_slots <= 0 || ring_slots > kMaxSlots || S > (1 << 27) || pos_base < 0 || absent(q, ring_k, ring_v, out)) return -1;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(ring_k) | reinterpret_cast<uintptr_t>(ring_v)) & 15u)
     return -3;
   int dev = 0, sms = 0;

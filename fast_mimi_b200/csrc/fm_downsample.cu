@@ -45,7 +45,7 @@ conv_frames_split_kernel(const float* __restrict__ x, uint16_t* __restrict__ hi,
 
 int launch_conv_frames_split(const float* x, void* hi, void* lo, int B, int T, int C, int kernel, int stride, cudaStream_t st) {
   if (B <= 0 || T <= 0) return (B == 0 || T == 0) ? 0 : -1;
-  if (C <= 0 || C % 8 != 0 || stride <= 0 || kernel < stride || kernel % stride != 0 || kernel > 16) return -1;
+  if (C <= 0 || C % 8 != 0 || stride <= 0 || kernel < stride || kernel % stride != 0 || kernel > 16 || absent(x, hi, lo)) return -1;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 15u) return -3;
   const int T_pad = stride * ((T + stride - 1) / stride + kernel / stride - 1);
   const long long want = (static_cast<long long>(B) * T_pad * (C / 8) + 255) / 256, cap = static_cast<long long>(sm_count()) * 8;
@@ -82,7 +82,7 @@ conv_rows_split_kernel(const float* __restrict__ x, uint16_t* __restrict__ hi, u
 int launch_conv_rows_split(const float* x, void* hi, void* lo, int B, int T, int C, int kernel, int stride,
                            cudaStream_t st) {
   if (B <= 0 || T <= 0) return (B == 0 || T == 0) ? 0 : -1;
-  if (C <= 0 || C % 8 != 0 || kernel < stride || stride <= 0 || kernel > 16) return -1;
+  if (C <= 0 || C % 8 != 0 || kernel < stride || stride <= 0 || kernel > 16 || absent(x, hi, lo)) return -1;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 15u) return -3;
   const int T_out = (T + stride - 1) / stride;
   const long long total = static_cast<long long>(B) * T_out * kernel * (C / 8);
@@ -160,7 +160,7 @@ upsample2_channels_kernel(const float* __restrict__ x, const float* __restrict__
 
 int launch_upsample2_channels(const float* x, const float* w, float* y, int B, int T, int C, cudaStream_t st) {
   if (B <= 0 || T <= 0) return (B == 0 || T == 0) ? 0 : -1;
-  if (C <= 0 || C % 32 != 0 || B > 65535 || C / 32 > 65535) return -1;
+  if (C <= 0 || C % 32 != 0 || B > 65535 || C / 32 > 65535 || absent(x, w, y)) return -1;
   if ((reinterpret_cast<uintptr_t>(x) & 3u) | ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15u)) return -3;
   const dim3 grid(static_cast<unsigned>((T + 31) / 32), static_cast<unsigned>(C / 32), static_cast<unsigned>(B));
   upsample2_channels_kernel<<<grid, 256, 0, st>>>(x, w, y, T, C);
@@ -169,7 +169,7 @@ int launch_upsample2_channels(const float* x, const float* w, float* y, int B, i
 
 int launch_upsample2_depthwise(const float* x, const float* w, float* y, int B, int T, int C, cudaStream_t st) {
   if (B <= 0 || T <= 0) return (B == 0 || T == 0) ? 0 : -1;
-  if (C <= 0 || C % 4 != 0) return -1;
+  if (C <= 0 || C % 4 != 0 || absent(x, w, y)) return -1;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15u) return -3;
   const long long total = static_cast<long long>(B) * 2 * T * (C / 4);
   int dev = 0, sms = 0;

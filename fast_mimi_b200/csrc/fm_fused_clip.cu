@@ -561,7 +561,7 @@ int launch_attn_fused_clip(const void* x, const void* w_qkv, const float* cos, c
                            void* out, int B, int T, int window, float scale, int dtype_flags, int* status,
                            cudaStream_t st, int dependent) {
   using namespace fused;
-  if (T <= kTile || T > 2 * kTile || B <= 0 || window <= 0 || cos == nullptr || sin == nullptr) return -1;
+  if (T <= kTile || T > 2 * kTile || B <= 0 || window <= 0 || absent(x, w_qkv, cos, sin, out)) return -1;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w_qkv) | reinterpret_cast<uintptr_t>(out) |
        reinterpret_cast<uintptr_t>(cos) | reinterpret_cast<uintptr_t>(sin)) & 15u)
     return -3;

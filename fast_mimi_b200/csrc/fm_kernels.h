@@ -13,6 +13,11 @@
 
 namespace fm {
 
+// Whether one of a call's tensors has no memory.  A kernel would fault on it; a tensor that only stands for one (a fake one of
+// torch's) says that it lies on the device and has address 0.
+template <typename... P>
+inline bool absent(const P*... p) { return (... || (p == nullptr)); }
+
 // Where the projection epilogue puts its results.  Linear outputs are [M, 512] 16-bit tensors
 // (null = skip).  The KV ring is [clips, 8 heads, ring_slots, 64]; the frame at absolute position
 // p of a clip lands in slot p % ring_slots.

@@ -57,6 +57,7 @@ static int layer_forward(const fm_layer_params& p, const void* x, void* y, void*
   const long long rows_ll = static_cast<long long>(B) * T;
   if (B < 0 || T < 0 || rows_ll > 0x7fffffffLL || p.window <= 0 || p.ffn <= 0 || p.ffn % 256 != 0) return -1;
   if (rows_ll == 0) return 0;
+  if (absent(x, y, cos, sin) || absent(p.ln1_weight, p.ln1_bias, p.w_qkv, p.w_o, p.ln2_weight, p.ln2_bias, p.w_fc1, p.w_fc2)) return -1;
   if (!rope_tables_aligned(cos, sin, cos_bstride)) return -3;
   const bool cached = ring_k != nullptr;
   if (cached && (ring_v == nullptr || past < 0 || slots < p.window)) return -1;

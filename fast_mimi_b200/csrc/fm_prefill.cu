@@ -321,7 +321,7 @@ static int launch_general(const void* q, const void* k, const void* v, void* out
 int launch_band_attn_chunk(const void* q, const void* k, const void* v, void* out, int B, int Tq, int Tk, int window,
                            float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent) {
   if (B <= 0 || Tq <= 0) return (B == 0 || Tq == 0) ? 0 : -1;
-  if (window <= 0 || Tk < Tq) return -1;
+  if (window <= 0 || Tk < Tq || absent(q, k, v, out)) return -1;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
        reinterpret_cast<uintptr_t>(out)) & 15u)
     return -3;
@@ -333,7 +333,7 @@ int launch_band_attn_prefill(const void* q, const void* k, const void* v, void* 
                              float scale, int value_is_fp16, int* status, cudaStream_t st, int dependent) {
   using namespace fmha;
   if (B <= 0 || T <= 0) return (B == 0 || T == 0) ? 0 : -1;
-  if (window <= 0 || B > 65535) return -1;
+  if (window <= 0 || B > 65535 || absent(q, k, v, out)) return -1;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
        reinterpret_cast<uintptr_t>(out)) & 15u)
     return -3;

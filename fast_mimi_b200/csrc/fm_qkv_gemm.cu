@@ -404,7 +404,7 @@ static int launch_gemm(const void* x, const void* w_qkv, const QkvEpilogueArgs& 
 int launch_qkv_rope_gemm(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep_in, int M, int dtype_flags,
                          int* status, cudaStream_t st, int dependent) {
   if (M <= 0) return M == 0 ? 0 : -1;
-  if (ep_in.T <= 0 || ep_in.cos == nullptr || ep_in.sin == nullptr) return -1;
+  if (ep_in.T <= 0 || absent(x, w_qkv, ep_in.cos, ep_in.sin)) return -1;
   if (!rope_tables_aligned(ep_in.cos, ep_in.sin, ep_in.cos_bstride)) return -3;
   QkvEpilogueArgs ep = ep_in;
   ep.n_tiles = 6;

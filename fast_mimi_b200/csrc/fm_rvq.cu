@@ -519,6 +519,7 @@ int launch_rvq_prepare(const float* x, void* resid16, float* tau, long long rows
 int launch_rvq_to_half(const float* x, void* y, long long rows, cudaStream_t st) {
   if (rows < 0) return -1;
   if (rows == 0) return 0;
+  if (absent(x, y)) return -1;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u) return -3;
   const long long n8 = rows * (rvq::kDim / 8);
   rvq_to_half_kernel<<<grid_for((n8 + 255) / 256, 8), 256, 0, st>>>(x, static_cast<uint16_t*>(y), n8);
@@ -528,6 +529,7 @@ int launch_rvq_to_half(const float* x, void* y, long long rows, cudaStream_t st)
 int launch_split_half(const float* x, void* hi, void* lo, long long n, cudaStream_t st) {
   if (n < 0 || n % 8 != 0) return -1;
   if (n == 0) return 0;
+  if (absent(x, hi, lo)) return -1;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 15u) return -3;
   const long long n8 = n / 8;
   split_half_kernel<<<grid_for((n8 + 255) / 256, 8), 256, 0, st>>>(x, static_cast<uint16_t*>(hi), static_cast<uint16_t*>(lo), n8);

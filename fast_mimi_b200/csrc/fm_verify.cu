@@ -126,6 +126,7 @@ __global__ void band_attn_fp32_kernel(const float* __restrict__ q, const float* 
 
 int launch_linear_fp32(const float* x, const float* w, float* y, int M, int N, int K, cudaStream_t st) {
   if (M <= 0 || N <= 0 || K <= 0) return M == 0 || N == 0 ? 0 : -1;
+  if (absent(x, w, y)) return -1;
   const long long total = static_cast<long long>(M) * N;
   linear_fp32_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, st>>>(x, w, y, M, N, K);
   return static_cast<int>(cudaGetLastError());
@@ -136,6 +137,7 @@ int launch_rope_fp32(float* t, const float* cosv, const float* sinv, int B, int 
   if (D <= 0 || (D & 1)) return -1;
   const long long total = static_cast<long long>(B) * T * H * (D / 2);
   if (total == 0) return 0;
+  if (absent(t, cosv, sinv)) return -1;
   rope_fp32_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, st>>>(t, cosv, sinv, B, T, H, D,
                                                                               cos_bstride);
   return static_cast<int>(cudaGetLastError());
@@ -147,6 +149,7 @@ int launch_band_attn_fp32(const float* q, const float* k, const float* v, float*
   if (D <= 0 || D > 256 || window <= 0 || B < 0 || H <= 0 || Tq < 0 || Tk < 0) return -1;
   const long long warps = static_cast<long long>(B) * H * Tq;
   if (warps == 0) return 0;
+  if (absent(q, k, v, out)) return -1;
   const int threads = 128;
   const long long blocks = (warps * 32 + threads - 1) / threads;
   if (blocks > 0x7fffffffLL) return -2;

@@ -220,3 +220,64 @@ def test_misaligned_rotary_tables_are_refused(rows, offset):
         assert lib.fm_attention_prefill_bf16(a, a, cos, sin, 0, a, a, a, a, 1, rows, 250, 0.125, 1, n, n) == -3
         assert lib.fm_attention_chunk_bf16(a, a, cos, sin, 0, a, a, a, a, a, a, a, a, 1, rows, 300, 250, 250, 0.125, 1, n, n) == -3
         assert lib.fm_decode_step_bf16(a, a, cos, sin, 0, n, 300, a, a, a, a, 1, 250, 0.125, 1, n, n) == -3
+
+
+# Entry points and arguments of an ordinary call: P a tensor that has to be there, O one that a kernel behind the first needs or that may be left out.
+P, O, N = "P", "O", None
+CALLS = {
+    "fm_qkv_rope_bf16": [P, P, P, P, 0, O, O, O, 2, 100, 0, N, N],
+    "fm_out_proj_f16": [P, P, N, N, P, 64, 1, N, N],
+    "fm_linear_f16": [P, P, N, N, P, 64, 512, 512, 1, 2, 0, N, N],
+    "fm_layernorm_f16": [P, 2, P, P, 1e-5, P, 1, 64, N],
+    "fm_rvq_select_f32": [P, 2, P, P, P, P, P, N, 64, 2048, 1.0, 1e-3, N, N],
+    "fm_conv_rows_split": [P, P, P, 2, 50, 512, 4, 2, N],
+    "fm_conv_frames_split": [P, P, P, 2, 50, 512, 4, 2, N],
+    "fm_linear_split_f32": [P, P, 64, 512, P, P, P, 64, 1, 1, 0, 1, 512, 512, N, N],
+    "fm_linear_split_sum_f32": [P, P, P, P, P, 2, 50, 512, 512, N, N],
+    "fm_linear_rows_f32": [P, P, P, P, 64, 1, 512, 512, N, N],
+    "fm_conv_frames_f32": [P, P, P, P, 2, 50, 512, 4, 2, 512, N, N],
+    "fm_conv_parts_f32": [P, P, P, O, O, O, 2, 50, 512, 4, 2, 512, N, N],
+    "fm_upsample2_channels_f32": [P, P, P, 2, 50, 512, N],
+    "fm_upsample2_f32": [P, P, P, 2, 50, 512, N],
+    "fm_rvq_decode_split": [P, P, P, P, P, 2, 50, 8, 1, 2048, 2048, N, N],
+    "fm_split_half": [P, P, P, 64, N],
+    "fm_rvq_prepare_f32": [P, P, P, 64, 1.0, 1e-3, N],
+    "fm_rvq_candidates_f16": [P, P, P, P, P, 64, 2048, N, N],
+    "fm_rvq_select_rec_f32": [P, P, P, P, P, N, P, 64, 2048, 1.0, 1e-3, N, N],
+    "fm_rvq_to_half": [P, P, 64, N],
+    "fm_rvq_decode_f32": [P, P, P, 64, 8, 2048, N, N],
+    "fm_band_attn_prefill_bf16": [P, P, P, P, 2, 100, 250, 0.125, 1, N, N],
+    "fm_attention_prefill_bf16": [P, P, P, P, 0, P, P, P, O, 2, 100, 250, 0.125, 1, N, N],
+    "fm_band_attn_chunk_bf16": [P, P, P, P, 2, 50, 100, 250, 0.125, 1, N, N],
+    "fm_attention_fused_bf16": [P, P, P, P, 0, P, 2, 200, 250, 0.125, 1, N, N],
+    "fm_attention_chunk_bf16": [P, P, P, P, 0, P, P, P, O, O, P, P, P, 2, 50, 100, 250, 250, 0.125, 1, N, N],
+    "fm_decode_step_bf16": [P, P, P, P, 0, N, 5, P, P, P, O, 2, 250, 0.125, 1, N, N],
+    "fm_ring_attn_decode_bf16": [P, P, P, P, N, 5, 2, 250, 0.125, 1, N, N],
+    "fm_band_attn_fp32_verify": [P, P, P, P, 2, 8, 64, 50, 50, 0, 0, 250, 0.125, O, N],
+    "fm_linear_fp32_verify": [P, P, P, 4, 4, 4, N],
+    "fm_rope_fp32_verify": [P, P, P, 1, 4, 8, 64, 0, N],
+}
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="the addresses are the host's")
+def test_a_tensor_without_memory_is_refused_on_the_host():
+    """A null address where a call needs a tensor (what torch's fake tensors, which say that they lie on the device, give for theirs) is an argument that
+    the call rejects before it launches anything: -1, where a launch on this machine would be a CUDA error."""
+    from fast_mimi_b200 import _native
+    lib = _native.load()
+    memory = ctypes.create_string_buffer(1 << 16)
+    at = (ctypes.addressof(memory) + 1023) & ~1023
+    fill = lambda a: at if a in (P, O) else a
+    for name, args in CALLS.items():
+        assert len(args) == len(_native.SIGNATURES[name]), name
+        for i, a in enumerate(args):
+            if a is P:
+                assert getattr(lib, name)(*[None if j == i else fill(b) for j, b in enumerate(args)]) == -1, (name, i)
+    pointers = [n for n, t in _native.LayerParams._fields_ if t is ctypes.c_void_p]
+    params = lambda without: ctypes.byref(_native.LayerParams(*[None if n == without else at for n in pointers], 1e-5, 1e-5, 0.125, 250, 2, 3, 2048, 0, 2))
+    call = lambda p, x, y, cos, sin: lib.fm_layer_forward(p, x, y, at, 1 << 30, cos, sin, 0, 1, 20, None, None, 0, 0, None, None)
+    for n in pointers:
+        if not n.endswith("scale"):
+            assert call(params(n), at, at, at, at) == -1, n
+    for i in range(4):
+        assert call(params(None), *[None if i == j else at for j in range(4)]) == -1, i
