@@ -11,6 +11,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -450,9 +451,12 @@ PyObject* upsample_checked(PyObject* const* a, Py_ssize_t n) {
   return THPVariable_Wrap(y.transpose(1, 2));
 }
 
-// No C++ exception leaves the module (as in layer_forward); what threw did so before the first launch.
+// No C++ exception leaves the module (as in layer_forward); what threw did so before the first launch.  A call that torch.jit.trace records is left to
+// the Python side, too, whose sizes are tensors then: the search and a transposed convolution that learns refuse it, where a recording of this
+// module's calls would be one of their allocations alone.
 template <PyObject* (*kFn)(PyObject* const*, Py_ssize_t)>
 PyObject* guarded(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (at::tracer::impl::is_dispatch_enabled()) Py_RETURN_NONE;
   try {
     return kFn(a, n);
   } catch (const std::exception&) {

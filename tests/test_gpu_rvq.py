@@ -419,3 +419,19 @@ def test_search_with_the_projections_inside_against_64_bits(rows, quantizers):
                 least, chosen = d.min(dim=1).values, d.gather(1, c[:, None])[:, 0]
                 assert (chosen - least <= 4e-6 * size * least.sqrt() + 2e-6 * least).all(), (l, float((chosen - least).max()))
                 r = r - vectors[c]
+
+
+def test_calls_that_cannot_be_recorded_refuse_it():
+    """torch.jit.trace of the search and of a transposed convolution whose weight learns is an error, not a graph without their kernels."""
+    import types
+    import fast_mimi_b200 as fm
+    branch = lambda n: fm.MimiRVQB200(torch.randn(n, 2048, 256, device="cuda"), torch.randn(256, 512, 1, device="cuda"), torch.randn(512, 256, 1, device="cuda"))
+    split = fm.MimiSplitRVQB200(branch(1), branch(7))
+    up = fm.MimiUpsampleB200(types.SimpleNamespace(conv=torch.nn.ConvTranspose1d(512, 512, 4, 2, groups=512, bias=False, device="cuda"), padding_left=0, padding_right=2))
+    x = torch.randn(2, 512, 30, device="cuda")
+    for call in (split.encode, up):
+        want = call(x)
+        with pytest.raises(Exception):
+            torch.jit.trace(lambda t: call(t), (x,))
+        assert torch.equal(call(x), want)
+    fm.check_status()
