@@ -129,7 +129,7 @@ def check(rc: int, what: str) -> None:
     """Turn a non-zero native status into an exception, as the reference's launchers do
     (src/fast_mimi/_native_cutlass.py:163-164)."""
     if rc != 0:
-        kind = {-1: "rejected geometry", -2: "grid too large", -3: "misaligned pointer",
+        kind = {-1: "rejected geometry or a tensor without memory", -2: "grid too large", -3: "misaligned pointer",
                 -4: "cuTensorMapEncodeTiled unavailable",
                 -5: "more frames than the built-in workspace holds",
                 -7: "workspace too small",

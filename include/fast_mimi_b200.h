@@ -6,7 +6,8 @@
  *   - every pointer is a raw DEVICE pointer owned by the caller; nothing is allocated or freed here;
  *   - `stream` is a cudaStream_t (0 = legacy default stream); launches are asynchronous on it;
  *   - the return value is 0 on success, a positive cudaError_t / CUresult, or a negative code for a
- *     rejected geometry (-1 bad size, -3 misaligned pointer, -4 driver entry point unavailable);
+ *     rejected geometry (-1 bad size or a NULL tensor that the call needs, -3 misaligned pointer, -4 driver entry point
+ *     unavailable);
  *   - `status` (optional, may be NULL) is a caller-zeroed device int; a kernel whose bounded wait on
  *     a TMA / tensor-core completion barrier runs out writes a code >= 101 there and finishes early.
  *     Read it back with fm_read_status().
