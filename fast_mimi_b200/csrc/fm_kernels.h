@@ -162,7 +162,7 @@ int launch_ln_linear_gelu(const void* x, int x_dtype, ParamVec weight, ParamVec 
 int launch_linear_small(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N, int K,
                         int in_dtype, int out_dtype, int gelu, int* status, cudaStream_t st, int dependent);
 // The same for as few rows as one wave of blocks with their weights in tensor memory holds (fm_linear_ws.cu): K a power of two times 512.
-bool linear_ws_takes(int M, int N, int K, int dependent);
+bool linear_ws_takes(int M, int N, int K, int dependent, bool resid16 = false);      // resid16: onto a residual of 16 bits
 int launch_linear_ws(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N, int K, int in_dtype, int out_dtype, int gelu,
                      int* status, cudaStream_t st, int dependent);
 int launch_qkv_ws(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status, cudaStream_t st,

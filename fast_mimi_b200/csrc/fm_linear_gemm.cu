@@ -549,7 +549,8 @@ int launch_linear_gemm(const void* a, const void* w, void* y, ParamVec scale, co
   if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y) |
        reinterpret_cast<uintptr_t>(scale.data) | reinterpret_cast<uintptr_t>(resid)) & 15u)
     return -3;
-  if (out_dtype != 3 && linear_ws_takes(M, N, K, dependent)) return launch_linear_ws(a, w, y, scale, resid, M, N, K, in_dtype, out_dtype, gelu, status, st, dependent);
+  if (out_dtype != 3 && linear_ws_takes(M, N, K, dependent, resid != nullptr && out_dtype != 2))
+    return launch_linear_ws(a, w, y, scale, resid, M, N, K, in_dtype, out_dtype, gelu, status, st, dependent);
   const int pair_tiles = ((M + kBlockM - 1) / kBlockM + 1) / 2;
   const int max_pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
   const bool one_wave = out_dtype != 3 && one_wave_of_halves(M, pair_tiles, N, max_pairs, out_dtype == 2, dependent);

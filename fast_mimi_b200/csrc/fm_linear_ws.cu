@@ -259,21 +259,22 @@ int clusters_of(int split) {
 // 128 rows, whose loads follow the weights into the same memory, by themselves are no faster than the other kernels (K = 2048, N = 512
 // 640 rows 9.9 -> 10.1 us; K = 512, N = 2048 with GELU 8.2 -> 8.9).  In a chain, where the weights come early, they are: with K shared by four or
 // more, and, without, as far as two thirds of the SMs (eight layers of five clips of 125 frames 278 -> 268 -> 260 us, of 577 BF16 frames 302 -> 291 ->
-// 279; beyond, eight clips 306 -> 314).
-static int rows_per_block(int M, int N, int K, int dependent) {
+// 279; beyond, eight clips 306 -> 314).  Not for up to 512 outputs onto a residual of 16 bits, 2369 rows and more, where half units of the pair kernel take 48 pairs of blocks
+// at once (eight layers of 14 clips of 170 BF16 frames, there and here, 416 and 422, of 200 422 and 428; FP32 416 and 416, 422 and 421).
+static int rows_per_block(int M, int N, int K, int dependent, bool resid16) {
   const int split = K / ws::kSlice;
   if (M <= 0 || N % ws::kBlockN != 0 || K % ws::kSlice != 0 || split > ws::kMaxSplit || (split & (split - 1)) != 0) return 0;
   if (split == 2 && N == 2 * ws::kBlockN && M <= 128) return 0;
   const int clusters = clusters_of(split);
   for (int rows = 16; rows <= 128; rows *= 2) {
     const long long blocks = blocks_for(M, N, K, rows), room = dependent && rows < 64 ? sm_count() / 2 : sm_count();
-    if (rows == 128 && (!dependent || (split == 1 ? 3 * blocks > 2 * sm_count() : split < 4))) return 0;
+    if (rows == 128 && (!dependent || (split == 1 ? 3 * blocks > 2 * sm_count() || (resid16 && N <= 4 * ws::kBlockN) : split < 4))) return 0;
     if (blocks <= room && blocks / split <= clusters) return rows >= 64 && M > rows && M <= rows * 3 / 2 ? 0 : rows;
   }
   return 0;
 }
 
-bool linear_ws_takes(int M, int N, int K, int dependent) { return rows_per_block(M, N, K, dependent) != 0; }
+bool linear_ws_takes(int M, int N, int K, int dependent, bool resid16) { return rows_per_block(M, N, K, dependent, resid16) != 0; }
 
 // a [M, K] and w [N, K]: the launch of one of the kernels for 16, 32, 64 and 128 rows a block
 using Kern = void (*)(const CUtensorMap, const CUtensorMap, const SmallArgs, uint32_t, int*);
@@ -295,7 +296,7 @@ static int launch_ws(const Kern (&kerns)[4], const void* a, const void* w, Small
 
 int launch_linear_ws(const void* a, const void* w, void* y, ParamVec scale, const void* resid, int M, int N, int K, int in_dtype, int out_dtype, int gelu,
                      int* status, cudaStream_t st, int dependent) {
-  const int rows = rows_per_block(M, N, K, dependent);
+  const int rows = rows_per_block(M, N, K, dependent, resid != nullptr && out_dtype != 2);
   if (rows == 0) return -1;
   SmallArgs args = {};
   args.scale = scale;
@@ -313,7 +314,7 @@ int launch_linear_ws(const void* a, const void* w, void* y, ParamVec scale, cons
 
 int launch_qkv_ws(const void* x, const void* w_qkv, const QkvEpilogueArgs& ep, int M, int dtype_flags, int* status, cudaStream_t st, int dependent) {
   using bf16 = __nv_bfloat16;
-  const int rows = rows_per_block(M, 1536, 512, dependent);
+  const int rows = rows_per_block(M, 1536, 512, dependent, false);
   if (rows == 0) return -1;
   SmallArgs args = {};
   args.M = M;
