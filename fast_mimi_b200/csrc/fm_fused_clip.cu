@@ -546,14 +546,16 @@ attn_fused_clip_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
 // The clips' heads are dealt to the pairs of CTAs in equal numbers, in order (a clip that two pairs share is loaded twice), where that is worth its cost
 // (fm_shares.h); else whole clips in turn.  A call by itself, a pair to a clip -> heads dealt, us, T = 250: 1 clip 41 -> 13.7, 10 42 -> 19, 30 43 -> 29, 64 44.1 -> 42.9,
 // 75 76.6 -> 51.7, 100 78 -> 61, 149 110 -> 88, 300 187 -> 160; 74, 148 and 512 (250) as before.  Where q, k and v may go through memory, projection kernel + attention kernel take
-// 0.53 us per clip of 250 frames (+ 8.4), about in proportion to T, so that this form is the faster one for long clips alone, and by little: a layer, one
-// kernel / two, us: T = 256 46 clips 107 / 110, 64 131.6 / 134.3, 148 268 / 278, 190 356 / 363; T = 225 64 clips 127.8 / 129.5, 92 169 / 168; T = 200 64 clips
-// 118.8 / 118.7, 148 233 / 233; T = 170 64 clips 113 / 111, 222 295 / 287.  With four heads and fewer a pair its first loads weigh more (T = 240 32 clips 83 / 81.5).
+// 0.53 us per clip of 250 frames (+ 8.4), about in proportion to T, so that this form is the faster one for long clips alone, and by little: eight BF16 layers at the
+// full clock, two kernels -> heads dealt, us: T = 250 40 clips (5 heads a pair) 870 -> 855, 52 (6) 964 -> 957, 60 (7) 1072 -> 1063, 80 (9) 1357 -> 1349, 104 (12) 1594 -> 1619;
+// T = 225 46 clips 876 -> 860, 52 905 -> 919, 64 1061 -> 1052; T = 256 83 clips (9) 1378 -> 1374, 92 (10) 1463 -> 1476, 126 (14) 1924 -> 1943, 160 (18) 2395 -> 2432, 190 (21)
+// 2828 -> 2852 (FP32 streams alike).  With four heads and fewer a pair its first loads weigh more (T = 240 32 clips, a layer, 81.5 -> 83).
 bool use_fused_clip(int B, int T) {
   const int pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
   const Shares shares(B, 8, pairs);
-  if (shares.per_block <= 4) return false;
-  const double us = dealt_heads_pay(shares, B, pairs) ? 5.0 * shares.per_block + 3.0 : 36.0 * ((B + pairs - 1) / pairs) + 5.0;
+  const bool dealt = dealt_heads_pay(shares, B, pairs);
+  if (shares.per_block <= 4 || (dealt && shares.per_block > 9)) return false;
+  const double us = dealt ? 5.25 * shares.per_block + 2.0 : 36.0 * ((B + pairs - 1) / pairs) + 5.0;
   return us <= 0.00212 * static_cast<double>(B) * T + 8.4;
 }
 
